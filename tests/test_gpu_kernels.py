@@ -110,6 +110,20 @@ def test_linear_every_row_count_and_odd_sizes(dtype, rows, n, k):
     assert torch.allclose(got32.cpu().double(), want, atol=2e-5 if dtype == "float32" else 2e-3, rtol=1e-3)
 
 
+@pytest.mark.parametrize("rows,n,k", [(17, 5, 4097), (64, 128, 256), (65, 129, 1023), (130, 2048, 2048), (2400, 2048, 1030)])
+def test_float32_product_in_parts(rows, n, k):
+    """The many-row float32 product: edges of its tiles and parts, parts by a cluster and by one block, and the same
+    bits for a row whatever the other rows of the call are.  A sum of k products in chains has an error of at most
+    (k + parts) ulps / 2 of the sum of their magnitudes."""
+    from starter_b200 import ops
+
+    x, w = rand(rows, k, seed=rows + k), rand(n, k, seed=n + k)
+    got = ops.linear(dev(x), dev(w))
+    bound = (k + 8) * 2.0 ** -24 * (x.double().abs() @ w.double().abs().t())
+    assert bool(((got.cpu().double() - x.double() @ w.double().t()).abs() <= bound).all())
+    assert torch.equal(ops.linear(dev(x[:17]), dev(w)), got[:17])
+
+
 @pytest.mark.parametrize("dtype", list(DT))
 @pytest.mark.parametrize("rows", [1, 5, 16, 40])
 def test_gated_linear_equals_product_then_swiglu(dtype, rows):
