@@ -58,6 +58,7 @@ SOURCES = (
     "attention_sink_tc",
     "short_conv",
     "state_scan",
+    "state_scan_prompt",
 )
 
 _lock = threading.Lock()

@@ -17,6 +17,11 @@
 //   walk (forget-write, channel-decay): the decay differs by row, so a token is a step; the state's update is the whole
 //     chain, and read-outs of eight tokens are summed together.  forget-write's gates are formed beforehand
 //     (scan_gates_kernel): inside the walk every block of 16 columns would form them again.
+// Measured at 2,048 tokens of one sequence, 16 heads of 128 x 128 (state-space: 32 of 128 x 64), before -> now: state-space 577 ->
+// 164 us, gated delta 673 -> 203, forget-write 414 -> 174, channel-decay 400 -> 177; unequal sequences of 801, 712 and 623
+// tokens: 383 -> 138, 603 -> 181, 382 -> 160, 377 -> 155.  The error against 64 bits is that of the other kernel or less
+// (outputs 5.5e-7 -> 4.2e-7, 3.7e-7 -> 3.1e-7, 4.9e-8, 1.2e-7).  With one sequence a scheduler has one warp, which issues in
+// 45 % of its cycles (the rest: waits of a few cycles for the result before); DRAM and shared memory are not the bound.
 #include "common.cuh"
 
 #define SP_N 128                 // rows of the state kept (N up to this; the rest are zeros)
@@ -61,7 +66,7 @@ __device__ __forceinline__ void sp_mma(float (&c)[4], uint32_t a0, uint32_t a1, 
 }
 
 template <bool DELTA>
-__global__ void __launch_bounds__(128)
+__global__ void __launch_bounds__(128, 3)
 scan_coef_kernel(const bf16* __restrict__ q, int ldq, const bf16* __restrict__ k, int ldk, const bf16* __restrict__ a_raw,
                  int lda, const bf16* __restrict__ b_raw, int ldb, const float* __restrict__ A_log,
                  const float* __restrict__ dt_bias, const float* __restrict__ D, float* __restrict__ coef,
@@ -123,8 +128,6 @@ scan_coef_kernel(const bf16* __restrict__ q, int ldq, const bf16* __restrict__ k
   // unit norms of the block's tokens: token j's squares lie on lane (j, j / 2), entry j % 2
   float mk_t = 1.f, mq_t = 1.f, mk_i[2] = {1.f, 1.f};
   if (DELTA) {
-    const float kd = (lane & 1) == 0 ? ck[0] : ck[1], qd = (lane & 1) == 0 ? cq[2] : cq[3];
-    (void)kd; (void)qd;
     auto diag = [&](float even, float odd, int j) {
       const float e = __shfl_sync(0xffffffffu, even, 4 * j + (j >> 1)), o = __shfl_sync(0xffffffffu, odd, 4 * j + (j >> 1));
       return (j & 1) ? o : e;
@@ -228,7 +231,7 @@ __device__ __forceinline__ float sp_sums16(float (&part)[16], int p) {
 }
 
 template <bool DELTA>
-__global__ void __launch_bounds__(128)
+__global__ void __launch_bounds__(128, 3)
 scan_blocks_kernel(const bf16* __restrict__ q, int ldq, const bf16* __restrict__ k, int ldk, const bf16* __restrict__ v, int ldv,
                    const float* __restrict__ coef, float* __restrict__ state, long long slot_stride, float* __restrict__ out,
                    const int* __restrict__ seq_slot, const int* __restrict__ seq_q_start, const int* __restrict__ seq_q_len,
@@ -321,27 +324,28 @@ scan_blocks_kernel(const bf16* __restrict__ q, int ldq, const bf16* __restrict__
       const int t = p >> 1, c = p & 1;
       const float* row = st.coef[b + t];
       const float4 s = *reinterpret_cast<const float4*>(row + 16);
-      const float x = to_f<bf16>(st.v[b + t][4 * warp + 2 * half + c]);
-      float z = x, w = s.x * x;
-      if constexpr (DELTA) z = s.x * x - s.y * sp_sums16(pk, p);
-      float B[8], W[8];
+      float B[8], own = 0.f;
 #pragma unroll
-      for (int n = 0; n < 2; ++n) {
-        *reinterpret_cast<float4*>(B + 4 * n) = *reinterpret_cast<const float4*>(row + 8 + 4 * n);
-        if (DELTA) *reinterpret_cast<float4*>(W + 4 * n) = *reinterpret_cast<const float4*>(row + 4 * n);
-      }
-      if (DELTA) w = 0.f;
-      float own = 0.f;
+      for (int n = 0; n < 2; ++n) *reinterpret_cast<float4*>(B + 4 * n) = *reinterpret_cast<const float4*>(row + 8 + 4 * n);
+      if constexpr (DELTA) {
+        float W[8], w = 0.f;
 #pragma unroll
-      for (int i = 0; i < 8; ++i) {
-        const float zi = __shfl_sync(0xffffffffu, z, (lane & 16) | (2 * i + c));
-        own = fmaf(B[i], zi, own);
-        if (DELTA) w = fmaf(W[i], zi, w);
+        for (int n = 0; n < 2; ++n) *reinterpret_cast<float4*>(W + 4 * n) = *reinterpret_cast<const float4*>(row + 4 * n);
+        const float x = to_f<bf16>(st.v[b + t][4 * warp + 2 * half + c]);
+        const float z = s.x * x - s.y * sp_sums16(pk, p);
+        float zi[8];
+#pragma unroll
+        for (int i = 0; i < 8; ++i) zi[i] = __shfl_sync(0xffffffffu, z, (lane & 16) | (2 * i + c));
+#pragma unroll
+        for (int i = 0; i < 8; ++i) w = fmaf(W[i], zi[i], w);
+        written[warp][half][t][c] = w;
+#pragma unroll
+        for (int i = 0; i < 8; ++i) own = fmaf(B[i], zi[i], own);
+        __syncwarp();
+      } else {
+#pragma unroll
+        for (int i = 0; i < 8; ++i) own = fmaf(B[i], to_f<bf16>(st.v[b + i][4 * warp + 2 * half + c]), own);
       }
-      written[warp][half][t][c] = w;
-      const float done = sp_sums16(pq, p);
-      if (in && t0 + b + t < q_len) out[(size_t)(q_start + t0 + b + t) * H * V + (size_t)h * V + col + c] = fmaf(s.z, done, own);
-      __syncwarp();
       const float gone = st.coef[b][19];
       const f2 g2 = f2_make(-gone, -gone);
 #pragma unroll
@@ -352,7 +356,14 @@ scan_blocks_kernel(const bf16* __restrict__ q, int ldq, const bf16* __restrict__
       for (int tt = 0; tt < 8; ++tt) {
         const uint4 kv = *reinterpret_cast<const uint4*>(&st.k[b + tt][8 * p]);
         const f2 k2[4] = {f2_bf16(kv.x), f2_bf16(kv.y), f2_bf16(kv.z), f2_bf16(kv.w)};
-        const float2 u = *reinterpret_cast<const float2*>(written[warp][half][tt]);
+        float2 u;
+        if constexpr (DELTA) {
+          u = *reinterpret_cast<const float2*>(written[warp][half][tt]);
+        } else {
+          const uint32_t vv = *reinterpret_cast<const uint32_t*>(&st.v[b + tt][4 * warp + 2 * half]);
+          const float by = st.coef[b + tt][16];
+          u = make_float2(by * __uint_as_float(vv << 16), by * __uint_as_float(vv & 0xffff0000u));
+        }
         const f2 u0 = f2_make(u.x, u.x), u1 = f2_make(u.y, u.y);
 #pragma unroll
         for (int r = 0; r < 4; ++r) {
@@ -360,7 +371,9 @@ scan_blocks_kernel(const bf16* __restrict__ q, int ldq, const bf16* __restrict__
           S[r][1] = f2_fma(k2[r], u1, S[r][1]);
         }
       }
-      __syncwarp();
+      const float done = sp_sums16(pq, p);
+      if (in && t0 + b + t < q_len) out[(size_t)(q_start + t0 + b + t) * H * V + (size_t)h * V + col + c] = fmaf(s.z, done, own);
+      if (DELTA) __syncwarp();
     }
   }
   pdl_trigger();
@@ -417,7 +430,7 @@ template <bool FORGET> struct RowStage { typedef DecayStage type; };
 template <> struct RowStage<true> { typedef ForgetStage type; };
 
 template <bool FORGET>
-__global__ void __launch_bounds__(128)
+__global__ void __launch_bounds__(128, 3)
 scan_rows_kernel(const void* __restrict__ q, int ldq, const bf16* __restrict__ k, int ldk, const bf16* __restrict__ v, int ldv,
                  const float* __restrict__ d, float* __restrict__ state, long long slot_stride, float* __restrict__ out,
                  const int* __restrict__ seq_slot, const int* __restrict__ seq_q_start, const int* __restrict__ seq_q_len,
@@ -546,28 +559,25 @@ scan_rows_kernel(const void* __restrict__ q, int ldq, const bf16* __restrict__ k
 
 extern "C" {
 
-// Floats of scratch a step of n_tokens needs here (mode as in sb_state_scan), or -1 for what these kernels do not take:
-// q, k, v (and in mode 2 the gate's logits, in k's place) as 16-byte pieces.
-long long sb_scan_prompt_scratch(int dtype, int mode, const void* q, int ldq, const void* k, int ldk, const void* v, int ldv,
-                                 const float* row_decay, int n_tokens, int n_seqs, int H, int G, int N, int V) {
-  if (dtype != 1 || N <= 64 || N > SP_N || N % 8 || V % 8 || ldq % 8 || ldk % 8 || ldv % 8) return -1;
+// Floats of scratch a token needs here (mode as in sb_state_scan), or -1 for what these kernels do not take: q, k, v (and
+// in mode 2 the gate's logits, in k's place) as 16-byte pieces.
+int sb_scan_prompt_floats(int dtype, int mode, const void* q, int ldq, const void* k, int ldk, const void* v, int ldv,
+                          const float* row_decay, int H, int G, int N, int V) {
+  if (dtype != 1 || mode < 0 || mode > 3 || N <= 64 || N > SP_N || N % 8 || V < 8 || V % 8 || ldq % 8 || ldk % 8 || ldv % 8) return -1;
+  if (H < 1 || G < 1 || H % G || (mode >= 2 && G != H)) return -1;
   if (((uintptr_t)q | (uintptr_t)k | (uintptr_t)v | (uintptr_t)row_decay) % 16) return -1;
-  if (mode < 2) return (long long)n_tokens * H * SP_COEF;
-  return mode == 2 ? 2ll * n_tokens * H * N : 0;
+  return mode < 2 ? H * SP_COEF : mode == 2 ? 2 * H * N : 0;
 }
 
-// Arguments as sb_state_scan's; scratch: float, 16-byte aligned, of the size above (null where that is 0).
+// Arguments as sb_state_scan's; scratch: float [n_tokens, that many], 16-byte aligned (null where it is 0).
 int sb_state_scan_prompt(int mode, const void* q, int ldq, const void* k, int ldk, const void* v, int ldv,
                          const void* a_raw, int lda, const void* b_raw, int ldb, const float* A_log, const float* dt_bias,
                          const float* D, const float* row_decay, float* state, long long slot_stride, float* out,
                          const int* seq_slot, const int* seq_q_start, const int* seq_q_len, int n_tokens, int n_seqs, int H,
                          int G, int N, int V, float* scratch, cudaStream_t s) {
   if (n_seqs == 0 || n_tokens == 0) return 0;
-  if (mode < 0 || mode > 3 || H < 1 || G < 1 || H % G || (mode == 1 && !b_raw) || (mode >= 2 && G != H) ||
-      (mode == 3) != (row_decay != nullptr) || (mode < 3 && !scratch))
-    return -2;
-  if (sb_scan_prompt_scratch(1, mode, q, ldq, k, ldk, v, ldv, row_decay, n_tokens, n_seqs, H, G, N, V) < 0 ||
-      ((uintptr_t)scratch % 16))
+  if (sb_scan_prompt_floats(1, mode, q, ldq, k, ldk, v, ldv, row_decay, H, G, N, V) < 0 || (mode < 3 && !scratch) ||
+      ((uintptr_t)scratch % 16) || (mode == 1 && !b_raw) || (mode == 3) != (row_decay != nullptr))
     return -2;
   const dim3 grid(n_seqs, H, (V + SP_COLS - 1) / SP_COLS);
   if (mode < 2) {

@@ -2304,6 +2304,10 @@ def glru_scan(u, gates, r_bias, i_bias, lam, decay_scale, proj, y_col, y_bias, s
 # ---------------------------------------------------------------------------------------- recurrences with a matrix state
 
 SCAN_MODES = {"state_space": 0, "gated_delta": 1, "forget_write": 2, "channel_decay": 3}
+#: tokens a sequence on average from which a recurrence runs on the kernels for prompts.  At 16 heads of 128 x 128: 8
+#: sequences of 64 tokens take 36 to 47 us there against 60 to 79 us on the kernel for few tokens, one of 2,048 takes 164 to
+#: 203 us against 400 to 673; below, the launch that forms the coefficients or gates beforehand (5 us) is not earned back.
+SCAN_PROMPT_TOKENS = 64
 
 
 def scan_max_state() -> int:
@@ -2358,6 +2362,17 @@ def state_scan(mode, q, k, v, a_raw, b_raw, A_log, dt_bias, skip, state, state_a
         raise KernelError(f"a slot's {state.shape[1]} floats do not hold {heads} states of {n_state} x {v_dim} from {state_at}")
     n_seqs = _seq_arrays(seq_slot, seq_q_start, seq_q_len)
     out = torch.empty((n_tokens, heads * v_dim), dtype=torch.float32, device=state.device)
+    if dtype == torch.bfloat16 and n_tokens >= SCAN_PROMPT_TOKENS * n_seqs and 64 < n_state <= 128:
+        lib = _lib("state_scan_prompt")
+        floats = lib.sb_scan_prompt_floats(1, SCAN_MODES[mode], *args[:6], _ptr(decay), heads, groups, n_state, v_dim)
+        if floats >= 0:
+            scratch = torch.empty((n_tokens, floats), dtype=torch.float32, device=state.device) if floats else None
+            rc = lib.sb_state_scan_prompt(
+                SCAN_MODES[mode], *args, _ptr(A_log), _ptr(dt_bias), _ptr(skip), _ptr(decay), _at(state, state_at),
+                ctypes.c_longlong(state.shape[1]), _ptr(out), _ptr(seq_slot), _ptr(seq_q_start), _ptr(seq_q_len), n_tokens,
+                n_seqs, heads, groups, n_state, v_dim, _ptr(scratch), _stream())
+            _check(rc, "state_scan (many tokens)", 1 if mode == "channel_decay" else 2)
+            return out
     rc = _lib("state_scan").sb_state_scan(
         _code(dtype), SCAN_MODES[mode], *args, _ptr(A_log), _ptr(dt_bias), _ptr(skip), _ptr(decay), _at(state, state_at),
         ctypes.c_longlong(state.shape[1]), _ptr(out), _ptr(seq_slot), _ptr(seq_q_start), _ptr(seq_q_len), n_seqs, heads,

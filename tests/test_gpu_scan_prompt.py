@@ -1,0 +1,102 @@
+"""The matrix-state recurrences' kernels for many tokens a sequence: against the plain statements, against the kernel
+for few tokens, across the edges of their blocks of 8 and chunks of 16 tokens and of their columns, the state carried."""
+
+import pytest
+import torch
+
+import plain_bavedra as bavedra
+import plain_salulorn as salulorn
+import plain_setotar as setotar
+
+pytestmark = pytest.mark.gpu
+F = torch.float64
+BF = torch.bfloat16
+
+
+def packed(lengths, slots):
+    starts = [sum(lengths[:i]) for i in range(len(lengths))]
+    return tuple(torch.tensor(x, dtype=torch.int32).cuda() for x in (slots, starts, lengths))
+
+
+def stated(mode, q, k, v, a, b, A, bias, skip, decay, heads, groups, n, width):
+    """One sequence from an empty state, in float64."""
+    t = q.shape[0]
+    q, k, v = q.reshape(t, groups, n), k.reshape(t, groups, n), v.reshape(t, heads, width)
+    if mode == "state_space":
+        return bavedra.state_space_recurrence(v, k, q, bavedra.softplus(a + bias), A, skip)
+    if mode == "gated_delta":
+        g = torch.exp(-torch.exp(A) * bavedra.softplus(a + bias))
+        return bavedra.delta_recurrence(bavedra.unit(q) * n ** -0.5, bavedra.unit(k), v, torch.sigmoid(b), g)
+    if mode == "forget_write":
+        low = A.reshape(heads, n)
+        f = low + (1.0 - low) * torch.sigmoid(k + bias.reshape(heads, n))
+        return setotar.forget_recurrence(setotar.silu(q), f, v)
+    return salulorn.decayed_recurrence(q * n ** -0.5, k, v, 1.0 - decay.reshape(t, heads, n))
+
+
+@pytest.mark.parametrize("mode", ["state_space", "gated_delta", "forget_write", "channel_decay"])
+@pytest.mark.parametrize("heads,groups,n,width", [(2, 1, 128, 64), (4, 2, 72, 24), (10, 1, 104, 8), (3, 3, 120, 40)])
+def test_many_tokens_a_sequence(mode, heads, groups, n, width, monkeypatch):
+    from starter_b200 import ops
+
+    if mode in ("forget_write", "channel_decay"):
+        groups = heads
+    gen = torch.Generator().manual_seed(heads * n)
+    lengths, slots = [129, 64, 72, 135], [2, 0, 3, 1]
+    total = sum(lengths)
+
+    def rows(columns, scale=1.0):
+        return (torch.randn(total, columns, generator=gen, dtype=F) * scale).to(BF).cuda()
+
+    # (queries and keys as columns of one tensor, in front of them columns that are not read)
+    qk = rows(8 + 2 * groups * n, 0.7)
+    v, ab = rows(heads * width), rows(2 * heads)
+    per = heads * n if mode == "forget_write" else heads
+    A = torch.linspace(0.0, 0.95, per) if mode == "forget_write" else torch.linspace(-8.0, 0.5, per)
+    bias, skip = torch.randn(per, generator=gen) * 0.5, torch.linspace(-1.0, 2.0, heads)
+    decay = None
+    if mode == "channel_decay":
+        decay = (1.0 - torch.sigmoid(torch.randn(total, heads * n, generator=gen, dtype=F) * 3.0) ** (1 / 16)).float()
+    state = torch.zeros(4, 3 + heads * n * width, device="cuda")
+    scalars = mode in ("state_space", "gated_delta")
+
+    def run(pick, lens, sl):
+        p, vv, raw = qk[pick].contiguous(), v[pick].contiguous(), ab[pick].contiguous()
+        return ops.state_scan(
+            mode, (p, 8), (p, 8 + groups * n), (vv, 0), (raw, 0) if scalars else None, (raw, heads) if mode == "gated_delta" else None,
+            None if decay is not None else A.cuda(), None if decay is not None else bias.cuda(),
+            skip.cuda() if mode == "state_space" else None, state, 3, *packed(lens, sl), heads, groups, n, width,
+            decay=decay[pick.cpu()].cuda().contiguous() if decay is not None else None)
+
+    assert ops._lib("state_scan_prompt").sb_scan_prompt_floats(
+        1, ops.SCAN_MODES[mode], ops._at(qk, 8), qk.shape[1], ops._at(qk, 8 + groups * n), qk.shape[1], ops._ptr(v), v.shape[1],
+        ops._ptr(None), heads, groups, n, width) >= 0
+    everything = torch.arange(total).cuda()
+    got = run(everything, lengths, slots)
+    kept = state.clone()
+    want, at = [], 0
+    host = [x.double().cpu() for x in (qk[:, 8:8 + groups * n], qk[:, 8 + groups * n:], v, ab[:, :heads], ab[:, heads:])]
+    for length in lengths:
+        part = slice(at, at + length)
+        want.append(stated(mode, *(x[part] for x in host), A.double(), bias.double(), skip.double(),
+                           decay[part].double() if decay is not None else None, heads, groups, n, width))
+        at += length
+    want = torch.cat(want).reshape(total, heads * width)
+    # float arithmetic on exact inputs: sums of up to 128 products in chains over up to 135 tokens
+    assert float((got.cpu().double() - want).abs().max()) <= 2e-5 * float(want.abs().max())
+    # the same by the kernel for few tokens
+    state.zero_()
+    monkeypatch.setattr(ops, "SCAN_PROMPT_TOKENS", 1 << 30)
+    few = run(everything, lengths, slots)
+    assert float((got - few).abs().max()) <= 2e-5 * float(few.abs().max())
+    assert float((kept - state).abs().max()) <= 2e-5 * float(state.abs().max())
+    # and in two portions
+    monkeypatch.setattr(ops, "SCAN_PROMPT_TOKENS", 1)
+    state.zero_()
+    out = torch.empty_like(got)
+    starts = [sum(lengths[:i]) for i in range(4)]
+    for sizes, done in (([61, 1, 16, 130], [0, 0, 0, 0]), ([68, 63, 56, 5], [61, 1, 16, 130])):
+        pick = torch.cat([torch.arange(s + d, s + d + m) for s, d, m in zip(starts, done, sizes)]).cuda()
+        out[pick] = run(pick, sizes, slots)
+    assert float((out - got).abs().max()) <= 2e-5 * float(got.abs().max())
+    assert float((kept - state).abs().max()) <= 2e-5 * float(state.abs().max())
