@@ -73,9 +73,10 @@ __global__ void latent_prepare_kernel(const T* __restrict__ proj, int proj_width
 }
 
 // q: [tokens, heads, dim + rot]; qa: [tokens, heads, rank + rot], whose first `rank` entries per head
-// the caller fills; this files the turned last `rot` entries of q behind them.
+// the caller fills; this files the turned last `rot` entries of q behind them.  qa may be q itself (rank = dim): a pair is
+// read and written by one thread.
 template <typename T>
-__global__ void latent_rotate_q_kernel(const T* __restrict__ q, T* __restrict__ qa, const float* __restrict__ cos_t,
+__global__ void latent_rotate_q_kernel(const T* q, T* qa, const float* __restrict__ cos_t,
                                        const float* __restrict__ sin_t, int table_width,
                                        const int* __restrict__ tok_pos, int heads, int dim, int rot, int rot_dims,
                                        int rank, int split) {

@@ -1,0 +1,403 @@
+// Latent attention for prompts (bfloat16) on the fifth-generation tensor cores.
+//
+// attention_latent.cu scores the cached latents themselves: a query head of rank + rot entries, values of rank.  For a
+// step of few tokens that reads each cache row once and multiplies little.  A prompt's queries outnumber what it costs to
+// form every head's keys and values once (rows * heads * (dim + vdim) * rank products against pairs of rank + rot and
+// rank), so here they are formed: latent_gather_kernel brings the sequences' cache rows behind one another, the library's
+// product makes [k of all heads | v of all heads] of them, and this kernel attends with queries and keys of dim + rot and
+// values of vdim (192 and 128 in place of 576 and 512: 3.4 times fewer products a pair).  The rotated part of the keys
+// is the gathered rows' own, shared by the heads.
+//
+// The block is attention_prefill_tc.cu's: 256 queries of a head as two tiles of 128, S and O of both in tensor memory, TMA
+// brings the operands in 128-byte swizzle, one warp issues the products of each tile, a thread is a query row, the output
+// is rescaled only when a row's maximum has grown by more than 2^8.  Three chunks of 64 query entries leave no room for
+// steps of 128 keys (2 x 48 KB of queries, 2 x 48 of keys, 32 of values, 2 x 32 of weights): steps are 64 keys, with
+// two buffers each of keys, values and S, so that S of the next step is formed while this one's exponentials run.
+//
+// A layer of width 2048, 16 heads of 128 + 64 over a latent of 512, 2,048 tokens: 517 us a pass with the kernel that scores the latents
+// (417 of them in it, mma.sync at 0.11 of the tensor peak; two products of 11 us around it), 156 with these.  The error against
+// 64 bits is the same (0.0047: keys and values are rounded here, folded queries and summed latents there).
+//
+// Gathered rows: a sequence's keys from the first that any of its queries sees, padded to a multiple of 64 with zeros, so
+// that a step never reads another sequence's values (their weights are zero, but 0 * inf would not be).
+#include <cuda.h>
+
+#include "attention_tc.cuh"
+#include "common.cuh"
+#include "tensor_map.cuh"
+
+#define LP_BK 64
+#define LP_THREADS 352
+
+// The first key that a sequence's queries of this step see.
+__device__ __forceinline__ int lp_first_key(int kv_len, int q_len, int window) {
+  return window > 0 ? max(0, kv_len - q_len - window + 1) : 0;
+}
+__device__ __forceinline__ int lp_rows(int kv_len, int q_len, int window) {
+  return (kv_len - lp_first_key(kv_len, q_len, window) + LP_BK - 1) / LP_BK * LP_BK;
+}
+// Where sequence `seq` begins among the gathered rows (whole warp).
+__device__ __forceinline__ int lp_row0(const int* seq_kv_len, const int* seq_q_len, int seq, int window, int lane) {
+  int rows = 0;
+  for (int s = lane; s < seq; s += 32) rows += lp_rows(seq_kv_len[s], seq_q_len[s], window);
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) rows += __shfl_xor_sync(0xffffffffu, rows, o);
+  return rows;
+}
+
+// c [rows, rank] and shared [rows, rot] from the cache rows [pages, 64, rank + rot]: a warp a row, 16-byte pieces.
+__global__ void __launch_bounds__(256)
+latent_gather_kernel(const bf16* __restrict__ store, const int* __restrict__ block_table, int table_stride,
+                     const int* __restrict__ seq_slot, const int* __restrict__ seq_q_len, const int* __restrict__ seq_kv_len,
+                     bf16* __restrict__ c, bf16* __restrict__ shared, int rank, int rot, int window) {
+  pdl_wait();
+  SB_BEHIND_WAIT(store); SB_BEHIND_WAIT(block_table); SB_BEHIND_WAIT(seq_slot); SB_BEHIND_WAIT(seq_q_len); SB_BEHIND_WAIT(seq_kv_len);
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, seq = blockIdx.y;
+  const int kv_len = seq_kv_len[seq], first = lp_first_key(kv_len, seq_q_len[seq], window);
+  const int i = blockIdx.x * 8 + warp;
+  if (i >= lp_rows(kv_len, seq_q_len[seq], window)) return;
+  const size_t row = (size_t)lp_row0(seq_kv_len, seq_q_len, seq, window, lane) + i;
+  const int j = first + i;
+  const bool real = j < kv_len;
+  const int page = block_table[(size_t)seq_slot[seq] * table_stride + (real ? j : first) / SB_PAGE_TOKENS];
+  const bf16* from = store + page_row(page, 0, j % SB_PAGE_TOKENS, 1, rank + rot);
+  const int pieces = (rank + rot) / 8, own = rank / 8;
+  for (int p = lane; p < pieces; p += 32) {
+    const uint4 v = real ? *reinterpret_cast<const uint4*>(from + p * 8) : make_uint4(0u, 0u, 0u, 0u);
+    if (p < own) *reinterpret_cast<uint4*>(c + row * rank + p * 8) = v;
+    else *reinterpret_cast<uint4*>(shared + row * rot + (p - own) * 8) = v;
+  }
+}
+
+// DC: 64-entry chunks of a head's plain key, VC: of its value; the rotated part is one more chunk.
+template <int DC, int VC>
+__global__ void __launch_bounds__(LP_THREADS, 1)
+latent_prompt_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant__ CUtensorMap map_kv,
+                     const __grid_constant__ CUtensorMap map_rot, bf16* __restrict__ out, const int* __restrict__ seq_q_start,
+                     const int* __restrict__ seq_q_len, const int* __restrict__ seq_kv_len, const int* __restrict__ block_seq,
+                     const int* __restrict__ block_first, int heads, float scale_log2, int window,
+                     const float* __restrict__ sink, int* status) {
+  constexpr int QC = DC + 1;
+  constexpr int QSUB = 128 * 128, KSUB = 64 * 128;  // bytes of 128 (64) rows of 128 bytes
+  constexpr int Q_BYTES = QC * QSUB, K_BYTES = QC * KSUB, V_BYTES = VC * KSUB, P_BYTES = QSUB;
+  constexpr uint32_t TMEM_COLS = 512;               // S: 2 tiles x 2 buffers x 64; O: 2 x 128 from column 256 on
+  extern __shared__ uint8_t smem_raw[];
+  uint8_t* smem = (uint8_t*)(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
+  uint8_t* q_sm = smem;                             // 2 tiles
+  uint8_t* p_sm = q_sm + 2 * Q_BYTES;               // 2 tiles
+  uint8_t* k_sm = p_sm + 2 * P_BYTES;               // 2 buffers
+  uint8_t* v_sm = k_sm + 2 * K_BYTES;               // 2 buffers
+  __shared__ uint64_t q_full, k_full[2], k_empty[2], v_full[2], v_empty[2], s_ready[2][2], s_free[2][2], p_ready[2], o_ready[2];
+  __shared__ uint32_t tmem_holder;
+  __shared__ int abort_flag;
+
+  const int head = blockIdx.x, seq = block_seq[blockIdx.y], q_first = block_first[blockIdx.y];
+  const int q_len = seq_q_len[seq], kv_len = seq_kv_len[seq];
+  const int rows_valid = min(2 * TC_BQ, q_len - q_first);
+  const int pos0 = kv_len - q_len + q_first;
+  const int warp = __shfl_sync(0xffffffffu, threadIdx.x >> 5, 0), lane = threadIdx.x & 31;
+  // steps of 64 keys, counted from the sequence's first gathered key; this block's first step
+  const int base = lp_first_key(kv_len, q_len, window);
+  const int lo = window > 0 ? max(0, pos0 - window + 1) : 0;
+  const int step0 = (lo - base) / LP_BK;
+  int n_tile[2];
+  n_tile[0] = (pos0 + min(rows_valid, TC_BQ) - 1 - base) / LP_BK - step0 + 1;
+  n_tile[1] = rows_valid > TC_BQ ? (pos0 + rows_valid - 1 - base) / LP_BK - step0 + 1 : 0;
+  const int n_steps = max(n_tile[0], n_tile[1]);
+
+  if (threadIdx.x == 0) {
+    mbar_init(&q_full, 1);
+    for (int b = 0; b < 2; ++b) {
+      mbar_init(&k_full[b], 1);
+      mbar_init(&v_full[b], 1);
+      mbar_init(&k_empty[b], 2);
+      mbar_init(&v_empty[b], 2);
+    }
+    for (int t = 0; t < 2; ++t) {
+      for (int b = 0; b < 2; ++b) {
+        mbar_init(&s_ready[t][b], 1);
+        mbar_init(&s_free[t][b], 4);  // one arrival per softmax warp
+      }
+      mbar_init(&p_ready[t], 4);
+      mbar_init(&o_ready[t], 1);
+    }
+    abort_flag = 0;
+    asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+  }
+  pdl_trigger();
+  if (warp == 9) tmem_alloc(&tmem_holder, TMEM_COLS);
+  asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+  __syncthreads();
+  asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+  const uint32_t tmem_base = tmem_holder;
+  volatile int* abort = &abort_flag;
+
+  if (warp == 8) {
+    // ---------------- producer: the warp as a whole, one elected lane issues the copies
+    const bool elected = elect_one();
+    pdl_wait();
+    const int q_row0 = seq_q_start[seq] + q_first;
+    const int row0 = lp_row0(seq_kv_len, seq_q_len, seq, window, lane) + step0 * LP_BK;
+    const int q_tiles = n_tile[1] ? 2 : 1;
+    if (elected) mbar_expect_tx(&q_full, q_tiles * Q_BYTES);
+    for (int t = 0; t < q_tiles; ++t)
+      for (int c = 0; c < QC; ++c)
+        if (elected) tma_load_2d(q_sm + t * Q_BYTES + c * QSUB, &map_q, &q_full, head * (QC * 64) + c * 64, q_row0 + t * TC_BQ);
+    int loads[4] = {0, 0, 0, 0};                    // copies started, by buffer (keys, values)
+    bool ok = true;
+    for (int i = 0; i < n_steps && ok; ++i) {
+      const int b = i & 1, row = row0 + i * LP_BK;
+      if (i >= 2) ok = __all_sync(0xffffffffu, mbar_wait(&k_empty[b], ((i >> 1) - 1) & 1, abort));
+      if (!ok) break;
+      if (elected) mbar_expect_tx(&k_full[b], K_BYTES);
+      for (int c = 0; c < DC; ++c)
+        if (elected) tma_load_2d(k_sm + b * K_BYTES + c * KSUB, &map_kv, &k_full[b], (head * DC + c) * 64, row);
+      if (elected) tma_load_2d(k_sm + b * K_BYTES + DC * KSUB, &map_rot, &k_full[b], 0, row);
+      loads[b]++;
+      if (i >= 2) ok = __all_sync(0xffffffffu, mbar_wait(&v_empty[b], ((i >> 1) - 1) & 1, abort));
+      if (!ok) break;
+      if (elected) mbar_expect_tx(&v_full[b], V_BYTES);
+      for (int c = 0; c < VC; ++c)
+        if (elected) tma_load_2d(v_sm + b * V_BYTES + c * KSUB, &map_kv, &v_full[b], (heads * DC + head * VC + c) * 64, row);
+      loads[2 + b]++;
+    }
+    if (*abort && elected) {                        // let the copies in flight land before the block ends
+      for (int b = 0; b < 4; ++b) {
+        uint64_t* bar = b < 2 ? &k_full[b] : &v_full[b - 2];
+        const uint64_t start = now_ns();
+        while (loads[b] > 0 && !mbar_try(bar, (loads[b] - 1) & 1) && now_ns() - start < WAIT_LIMIT_NS) {}
+      }
+      const uint64_t start = now_ns();
+      while (!mbar_try(&q_full, 0) && now_ns() - start < WAIT_LIMIT_NS) {}
+    }
+  } else if (warp == 9 || warp == 10) {
+    // ---------------- MMA issuers: warp 9 for tile 0, warp 10 for tile 1
+    const int t = warp - 9, n_mine = n_tile[t], n_other = n_tile[1 - t];
+    if (n_mine > 0) {
+      const bool elected = elect_one();
+      const uint32_t idesc_s = instr_desc(LP_BK, 0), idesc_o = instr_desc(VC * 64, 1);
+      const uint32_t q_addr = smem_u32(q_sm + t * Q_BYTES), p_addr = smem_u32(p_sm + t * P_BYTES);
+      const uint32_t tmem_s = tmem_base + t * 2 * LP_BK, tmem_o = tmem_base + 4 * LP_BK + t * 128;
+      auto issue_s = [&](int b) {
+        if (elected) {
+          const uint32_t k_addr = smem_u32(k_sm + b * K_BYTES);
+#pragma unroll
+          for (int k = 0; k < QC * 4; ++k)
+            umma_bf16(tmem_s + b * LP_BK, smem_desc(q_addr + (k >> 2) * QSUB + (k & 3) * 32, 16),
+                      smem_desc(k_addr + (k >> 2) * KSUB + (k & 3) * 32, 16), idesc_s, k > 0 ? 1u : 0u);
+          umma_commit(&s_ready[t][b]);
+        }
+      };
+      // V's rows are keys (16 keys = 2048 bytes), its 64-wide chunks KSUB bytes apart
+      auto issue_pv = [&](int b, bool first) {
+        if (elected) {
+          const uint32_t v_addr = smem_u32(v_sm + b * V_BYTES);
+#pragma unroll
+          for (int k = 0; k < LP_BK / 16; ++k)
+            umma_bf16(tmem_o, smem_desc(p_addr + k * 32, 16), smem_desc(v_addr + k * 2048, KSUB), idesc_o,
+                      (first && k == 0) ? 0u : 1u);
+          umma_commit(&o_ready[t]);
+        }
+      };
+      // a buffer is free after two arrivals, one per tile; a tile that is alone in a step makes both
+      auto release = [&](uint64_t* bar, bool alone) {
+        if (elected) {
+          umma_commit(bar);
+          if (alone) umma_commit(bar);
+        }
+        __syncwarp();
+      };
+      auto wait_for = [&](uint64_t* bar, uint32_t parity) -> bool { return __all_sync(0xffffffffu, mbar_wait(bar, parity, abort)); };
+      bool ok = wait_for(&q_full, 0) && wait_for(&k_full[0], 0);
+      if (ok) {
+        asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+        issue_s(0);
+        release(&k_empty[0], n_other == 0);
+      }
+      for (int i = 0; i < n_mine && ok; ++i) {
+        const int b = i & 1;
+        if (i + 1 < n_mine) {                       // S of the next step, in the other buffer
+          const int nb = b ^ 1, use = (i + 1) >> 1;
+          ok = wait_for(&k_full[nb], use & 1);
+          if (ok && use > 0) ok = wait_for(&s_free[t][nb], (use - 1) & 1);
+          if (!ok) break;
+          asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+          issue_s(nb);
+          release(&k_empty[nb], i + 1 >= n_other);
+        }
+        ok = wait_for(&v_full[b], (i >> 1) & 1) && wait_for(&p_ready[t], i & 1);
+        if (!ok) break;
+        asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+        issue_pv(b, i == 0);
+        release(&v_empty[b], i >= n_other);
+      }
+    }
+  } else if (warp < 8) {
+    // ---------------- softmax and output: warps 0-3 own tile 0, warps 4-7 tile 1; thread = query row
+    const int t = warp >> 2, quarter = warp & 3, r = quarter * 32 + lane;
+    const int pos = pos0 + t * TC_BQ + r;
+    const uint32_t lane_addr = (uint32_t)(quarter * 32) << 16;
+    const uint32_t tmem_s = tmem_base + t * 2 * LP_BK + lane_addr, tmem_o = tmem_base + 4 * LP_BK + t * 128 + lane_addr;
+    uint8_t* p_row = p_sm + t * P_BYTES + r * 128;
+    const int n_mine = n_tile[t];
+    float m_ref = -INFINITY, l_run = 0.f;
+    if (sink) {                                     // the state a row's softmax starts from
+      m_ref = sink[head] * 1.4426950408889634f;
+      l_run = 1.f;
+    }
+    const int row_first = window > 0 ? pos - window + 1 : 0;
+    pdl_wait();
+    bool ok = true;
+    for (int i = 0; i < n_mine && ok; ++i) {
+      const int b = i & 1;
+      ok = mbar_wait(&s_ready[t][b], (i >> 1) & 1, abort);
+      if (!ok) break;
+      asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+      const int j0 = base + (step0 + i) * LP_BK;
+      float sv[64];
+      tmem_load64(tmem_s + b * LP_BK, sv);
+      asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+      __syncwarp();
+      if (lane == 0) mbar_arrive(&s_free[t][b]);    // S of this step may be overwritten
+      if (j0 + LP_BK - 1 > pos0 + t * TC_BQ || (window > 0 && j0 <= pos0 + t * TC_BQ + TC_BQ - window)) {
+#pragma unroll
+        for (int e = 0; e < 64; ++e)
+          if ((j0 + e > pos) | (j0 + e < row_first)) sv[e] = -INFINITY;
+      }
+      float mx = -INFINITY, mx2 = -INFINITY;
+#pragma unroll
+      for (int e = 0; e < 64; e += 2) {
+        mx = fmaxf(mx, sv[e]);
+        mx2 = fmaxf(mx2, sv[e + 1]);
+      }
+      mx = fmaxf(mx, mx2) * scale_log2;             // scale_log2 > 0: the maximum commutes with it
+      const bool outgrown = mx > m_ref + 8.f;       // also the first keys a row sees (m_ref = -inf)
+      if (__any_sync(0xffffffffu, outgrown)) {
+        // a new reference: rescale what has been accumulated
+        const float m_new = fmaxf(m_ref, mx);
+        const float alpha = m_ref == -INFINITY ? 1.f : fast_exp2(m_ref - m_new);
+        if (i > 0) {
+          ok = mbar_wait(&o_ready[t], (i - 1) & 1, abort);
+          if (!ok) break;
+          asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+#pragma unroll 1
+          for (int c = 0; c < VC * 64; c += 32) {
+            float ov[32];
+            tmem_load32(tmem_o + c, ov);
+#pragma unroll
+            for (int e = 0; e < 32; ++e) ov[e] *= alpha;
+            tmem_store32(tmem_o + c, ov);
+          }
+          asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
+        }
+        l_run *= alpha;
+        m_ref = m_new;
+      }
+      const float m_use = m_ref == -INFINITY ? 0.f : m_ref;
+      float rs = 0.f, rs_hi = 0.f;
+      uint32_t pk[32];
+#pragma unroll
+      for (int e = 0; e < 32; ++e) {
+        float x0, x1;
+        fma2(x0, x1, sv[2 * e], sv[2 * e + 1], scale_log2, -m_use);
+        const float p0 = fast_exp2(x0), p1 = fast_exp2(x1);
+        add2(rs, rs_hi, p0, p1);
+        __nv_bfloat162 two = __floats2bfloat162_rn(p0, p1);
+        pk[e] = *reinterpret_cast<uint32_t*>(&two);
+      }
+      // P's tile is free once PV of the step before has finished
+      if (i > 0) ok = mbar_wait(&o_ready[t], (i - 1) & 1, abort);
+      if (!ok) break;
+      // K-major A operand: 16-byte column c ^ (r % 8) of row r
+#pragma unroll
+      for (int c = 0; c < 8; ++c)
+        *reinterpret_cast<uint4*>(p_row + ((c ^ (r & 7)) << 4)) = make_uint4(pk[4 * c], pk[4 * c + 1], pk[4 * c + 2], pk[4 * c + 3]);
+      l_run += rs + rs_hi;
+      asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+      asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+      __syncwarp();
+      if (lane == 0) mbar_arrive(&p_ready[t]);
+    }
+    if (ok && n_mine > 0) ok = mbar_wait(&o_ready[t], (n_mine - 1) & 1, abort);
+    if (ok && n_mine > 0) {
+      asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+      const bool valid = t * TC_BQ + r < rows_valid;
+      const float inv = 1.f / l_run;
+      bf16* dst = out + ((size_t)seq_q_start[seq] + q_first + t * TC_BQ + r) * ((size_t)heads * (VC * 64)) + (size_t)head * (VC * 64);
+#pragma unroll 1
+      for (int c = 0; c < VC * 64; c += 32) {
+        float ov[32];
+        tmem_load32(tmem_o + c, ov);
+        if (valid) {
+#pragma unroll
+          for (int d = 0; d < 32; d += 8) {
+            uint32_t w[4];
+#pragma unroll
+            for (int e = 0; e < 4; ++e) {
+              __nv_bfloat162 two = __floats2bfloat162_rn(ov[d + 2 * e] * inv, ov[d + 2 * e + 1] * inv);
+              w[e] = *reinterpret_cast<uint32_t*>(&two);
+            }
+            *reinterpret_cast<uint4*>(dst + c + d) = make_uint4(w[0], w[1], w[2], w[3]);
+          }
+        }
+      }
+      asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+    }
+  }
+
+  asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+  __syncthreads();
+  if (warp == 9) {
+    __syncwarp();
+    tmem_free(tmem_holder, TMEM_COLS);
+  }
+  if (threadIdx.x == 0 && abort_flag && status) atomicOr(status, 16);
+}
+
+template <int DC, int VC>
+static int lp_launch(const CUtensorMap& mq, const CUtensorMap& mkv, const CUtensorMap& mr, void* out, const int* seq_q_start,
+                     const int* seq_q_len, const int* seq_kv_len, const int* block_seq, const int* block_first, int n_blocks,
+                     int heads, float scale, int window, const float* sink, int* status, cudaStream_t s) {
+  const int smem = 2 * (DC + 1) * 128 * 128 + 2 * 128 * 128 + 2 * (DC + 1 + VC) * 64 * 128 + 1024;
+  cudaError_t err = cudaFuncSetAttribute(latent_prompt_kernel<DC, VC>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+  if (err != cudaSuccess) return (int)err;
+  return launch_dependent(latent_prompt_kernel<DC, VC>, dim3(heads, n_blocks), dim3(LP_THREADS), smem, s, mq, mkv, mr, (bf16*)out,
+                          seq_q_start, seq_q_len, seq_kv_len, block_seq, block_first, heads, scale * 1.4426950408889634f, window,
+                          sink, status);
+}
+
+extern "C" {
+
+// c: [rows, rank]; shared: [rows, rot]; rows: over the sequences, the keys from the first that a query of the step sees on (all,
+// without a window), each rounded up to a multiple of 64; max_rows: the most of one sequence.
+int sb_latent_gather(const void* store, const int* block_table, int table_stride, const int* seq_slot, const int* seq_q_len,
+                     const int* seq_kv_len, int n_seqs, int max_rows, void* c, void* shared, int rank, int rot, int window,
+                     cudaStream_t s) {
+  if (n_seqs == 0 || max_rows == 0) return 0;
+  if (rank % 8 || rot % 8 || n_seqs > 65535 || (((uintptr_t)store | (uintptr_t)c | (uintptr_t)shared) & 15)) return -2;
+  return launch_dependent(latent_gather_kernel, dim3((max_rows + 7) / 8, n_seqs), dim3(256), 0, s, (const bf16*)store, block_table,
+                          table_stride, seq_slot, seq_q_len, seq_kv_len, (bf16*)c, (bf16*)shared, rank, rot, window);
+}
+
+// q: [n_tokens, heads * (dim + 64)], the last 64 entries of a head turned; kv: [rows, heads * dim + heads * vdim]; shared:
+// [rows, 64]; out: [n_tokens, heads * vdim]; block_seq / block_first: blocks of 256 queries; dim and vdim 64 or 128; scale > 0.
+int sb_latent_prompt(const void* q, const void* kv, const void* shared, void* out, const int* seq_q_start, const int* seq_q_len,
+                     const int* seq_kv_len, const int* block_seq, const int* block_first, int n_blocks, int n_tokens, int rows,
+                     int heads, int dim, int vdim, float scale, int window, const float* sink, int* status, cudaStream_t s) {
+  if (n_blocks == 0 || n_tokens == 0) return 0;
+  if ((dim != 64 && dim != 128) || (vdim != 64 && vdim != 128) || !(scale > 0.f) || n_blocks > 65535) return -2;
+  if (((uintptr_t)q | (uintptr_t)kv | (uintptr_t)shared | (uintptr_t)out) & 15) return -2;
+  CUtensorMap mq, mkv, mr;
+  int rc = sb_make_map(&mq, q, n_tokens, (long long)heads * (dim + 64), TC_BQ);
+  if (rc) return rc;
+  rc = sb_make_map(&mkv, kv, rows, (long long)heads * (dim + vdim), LP_BK);
+  if (rc) return rc;
+  rc = sb_make_map(&mr, shared, rows, 64, LP_BK);
+  if (rc) return rc;
+#define ARGS mq, mkv, mr, out, seq_q_start, seq_q_len, seq_kv_len, block_seq, block_first, n_blocks, heads, scale, window, sink, status, s
+  if (dim == 128) return vdim == 128 ? lp_launch<2, 2>(ARGS) : lp_launch<2, 1>(ARGS);
+  return vdim == 128 ? lp_launch<1, 2>(ARGS) : lp_launch<1, 1>(ARGS);
+#undef ARGS
+}
+
+}  // extern "C"

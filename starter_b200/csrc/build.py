@@ -52,6 +52,7 @@ SOURCES = (
     "residual32",
     "wkv",
     "attention_latent",
+    "attention_latent_prompt",
     "moe",
     "depth",
     "attention_sink",

@@ -1646,6 +1646,71 @@ def latent_attention_step(qa, store, block_table, ctx, heads, rank, rot, scale, 
     return latent_attention(qa, store, block_table, ctx.tok_slot, ctx.tok_pos, heads, rank, rot, scale, window, sink)
 
 
+#: tokens that every sequence of a step must bring for the latent attention to form keys and values (see
+#: ``latent_attention_prompt``), and the most cache rows it forms them for.  Forming a row costs a head 2 * 256 * 512
+#: products, a query saves it about 1,500 a row at a third of the speed: from about 25 tokens on it pays, whatever the
+#: rows; 65,536 rows bound the memory (8 KB a row with 16 heads of 128 + 128)
+LATENT_PROMPT_TOKENS, LATENT_PROMPT_ROWS = 32, 65536
+
+
+def _latent_prompt_rows(ctx, window):
+    """The rows of each sequence that ``latent_attention_prompt`` works on (numpy), as its kernels count them."""
+    q_len, kv_len = ctx.host["seq_q_len"], ctx.host["seq_kv_len"]
+    rows = kv_len
+    if window:
+        rows = kv_len - (kv_len - q_len - int(window) + 1).clip(min=0)
+    return (rows + 63) // 64 * 64
+
+
+def latent_prompt_takes(dtype, ctx, dim, rot, vdim, rank, scale, window=None) -> bool:
+    """Whether ``latent_attention_prompt`` serves this step: bfloat16, plain keys and values of 64 or 128 entries and a rotated
+    part of 64, every sequence bringing at least ``LATENT_PROMPT_TOKENS`` tokens (known on the host), and no more than
+    ``LATENT_PROMPT_ROWS`` rows to form keys and values for."""
+    if dtype != torch.bfloat16 or ctx.host is None or ctx.block_seq is None or not scale > 0:
+        return False
+    if dim not in (64, 128) or vdim not in (64, 128) or rot != 64 or rank % 16 or rank + rot > 640:
+        return False
+    return (int(ctx.host["seq_q_len"].min()) >= LATENT_PROMPT_TOKENS
+            and int(_latent_prompt_rows(ctx, window).sum()) <= LATENT_PROMPT_ROWS)
+
+
+def latent_attention_prompt(q, ukv, store, block_table, ctx, heads, dim, vdim, rank, rot, scale, window=None, sink=None):
+    """Latent attention over keys and values that are formed from the cached rows first: ``q`` ``[T, heads * (dim + rot)]``
+    (the last ``rot`` entries of a head turned), ``ukv`` ``[heads * dim + heads * vdim, rank]`` (the heads' key, then value
+    up-projections).  The sequences' rows that the step's queries see are brought behind one another, one product forms the
+    plain keys and the values of all heads, and the tcgen05 kernel attends.  Returns ``[T, heads * vdim]``: the heads'
+    outputs, already in value space."""
+    _need(q, "q", torch.bfloat16, 2)
+    _need(ukv, "ukv", q.dtype, 2)
+    n_tokens = q.shape[0]
+    if q.shape[1] != heads * (dim + rot) or tuple(ukv.shape) != (heads * (dim + vdim), rank):
+        raise KernelError(f"q {tuple(q.shape)} / ukv {tuple(ukv.shape)} do not fit {heads} heads of {dim} + {rot} / {vdim} over {rank}")
+    _need(store, "cache pages", q.dtype, 4)
+    if tuple(store.shape[1:]) != (1, PAGE_TOKENS, rank + rot):
+        raise KernelError(f"cache pages have shape {tuple(store.shape)}")
+    _need(block_table, "block_table", torch.int32, 2)
+    n_seqs = _seq_arrays(ctx.seq_slot, ctx.seq_q_start, ctx.seq_q_len)
+    for name, t in (("seq_kv_len", ctx.seq_kv_len), ("block_seq", ctx.block_seq), ("block_first", ctx.block_first)):
+        _need(t, name, torch.int32, 1)
+    each = _latent_prompt_rows(ctx, window)
+    rows = int(each.sum())
+    gathered = torch.empty((rows * (rank + rot),), dtype=q.dtype, device=q.device)
+    c, shared = gathered[:rows * rank].view(rows, rank), gathered[rows * rank:].view(rows, rot)
+    lib = _lib("attention_latent_prompt")
+    rc = lib.sb_latent_gather(_ptr(store), _ptr(block_table), block_table.shape[1], _ptr(ctx.seq_slot), _ptr(ctx.seq_q_len),
+                              _ptr(ctx.seq_kv_len), n_seqs, int(each.max()), _ptr(c), _ptr(shared), rank, rot, int(window or 0),
+                              _stream())
+    _check(rc, "latent_gather")
+    kv = linear(c, ukv, status=ctx.status)
+    out = torch.empty((n_tokens, heads * vdim), dtype=q.dtype, device=q.device)
+    rc = lib.sb_latent_prompt(
+        _ptr(q), _ptr(kv), _ptr(shared), _ptr(out), _ptr(ctx.seq_q_start), _ptr(ctx.seq_q_len), _ptr(ctx.seq_kv_len),
+        _ptr(ctx.block_seq), _ptr(ctx.block_first), ctx.block_seq.shape[0], n_tokens, rows, heads, dim, vdim,
+        ctypes.c_float(scale), int(window or 0), _latent_sink(sink, heads), _ptr(ctx.status), _stream())
+    _check(rc, "latent_attention_prompt")
+    return out
+
+
 def sigmoid_gate(a, gate, gate_col):
     """``a *= sigmoid(gate)`` in place for ``a`` ``[T, N]`` and the columns ``gate_col .. gate_col + N`` of ``gate`` ``[T, M]``."""
     _need(a, "a", None, 2)

@@ -7,8 +7,10 @@ latent and shared part in the token's cache row; the query up-projection follows
 up-projection is not applied to the cache: it is folded into the query, head by head (``q' = W_uk^T
 q_plain``), so the attention kernel scores ``q' . c + q_rot . shared`` against the cache rows as they
 are and sums the latents; the value up-projection is applied to that sum, head by head, the gate
-multiplies the heads (``ops.sigmoid_gate``) and the output projection follows.  A whole prompt, a later portion and a single token are the same code: every query
-is told its absolute position.
+multiplies the heads (``ops.sigmoid_gate``) and the output projection follows.  In a step whose sequences all bring many
+tokens the key and value up-projections are applied to the cached rows after all, once for all queries
+(``ops.latent_attention_prompt``): fewer products than scoring and summing whole latents.  A whole prompt, a later portion
+and a single token are the same code: every query is told its absolute position.
 
 A layer whose spec says ``own_kv = False`` has no key/value down-projection: the run order gives it the
 cache entry of the layer whose latent it reads (``writes_cache`` false).
@@ -74,8 +76,11 @@ class LatentAttention(Part):
         self.kv_gain = params["dkv_norm"].float().contiguous() if s.own_kv else None
         self.uq = params["uq"].contiguous()
         # per head: [dim, kv_rank] (folded into the query) and [kv_rank, vdim] (applied to the summed latents)
-        self.uk = params["uk"].contiguous().view(s.num_heads, s.head_dim, s.kv_rank)
-        self.uv = params["uv"].contiguous().view(s.num_heads, s.value_dim, s.kv_rank).transpose(1, 2)
+        # (views of one matrix whose product with a latent gives the plain keys and the values of all heads)
+        self.ukv = torch.cat([params["uk"], params["uv"]], dim=0).contiguous()
+        keys = s.num_heads * s.head_dim
+        self.uk = self.ukv[:keys].view(s.num_heads, s.head_dim, s.kv_rank)
+        self.uv = self.ukv[keys:].view(s.num_heads, s.value_dim, s.kv_rank).transpose(1, 2)
         self.o = params["o"].contiguous()
         if s.sink:
             self.sink = params["sink"].float().contiguous()
@@ -98,6 +103,14 @@ class LatentAttention(Part):
                                 write_cache=writes_cache, layout=rotation.layout, kv_col=self.kv_at)
         q = ops.linear(cq, self.uq, status=ctx.status)
         n = q.shape[0]
+        if ops.latent_prompt_takes(q.dtype, ctx, s.head_dim, s.rot_dim, s.value_dim, s.kv_rank, s.scale, s.window):
+            ops.latent_rotate_q(q, q.view(n, s.num_heads, -1), cos, sin, ctx.tok_pos, s.num_heads, s.head_dim, s.rot_dim,
+                                s.position.dims, s.head_dim, layout=rotation.layout)
+            a = ops.latent_attention_prompt(q, self.ukv, store, cache.block_table, ctx, s.num_heads, s.head_dim, s.value_dim,
+                                            s.kv_rank, s.rot_dim, s.scale, s.window, self.sink)
+            if s.output_gate:
+                ops.sigmoid_gate(a, proj, s.q_rank)
+            return ops.linear(a, self.o, status=ctx.status)
         qa = torch.empty((n, s.num_heads, self.row), dtype=q.dtype, device=q.device)
         q3 = q.view(n, s.num_heads, s.head_dim + s.rot_dim)
         torch.bmm(q3[:, :, : s.head_dim].transpose(0, 1), self.uk, out=qa[:, :, : s.kv_rank].transpose(0, 1))

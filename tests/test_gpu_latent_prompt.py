@@ -1,0 +1,106 @@
+"""Latent attention over formed keys and values: the kernel alone against float64, around the edges of its tiles of 128
+queries and steps of 64 keys, behind cached tokens, with windows and sinks; what the pages hold besides must not show; and the
+layer on it against the layer on the kernel that scores the latents themselves."""
+
+import math
+from types import SimpleNamespace
+
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+F = torch.float64
+BF = torch.bfloat16
+
+
+def context(past, new, slots):
+    from starter_b200.engine.batch import StepEntry, plan_step, upload
+
+    arrays = plan_step([StepEntry(s, [0] * n, []) for s, n in zip(slots, new)], past)
+    dev = upload(arrays, torch.device("cuda"))
+    return SimpleNamespace(host=arrays, status=torch.zeros(1, dtype=torch.int32, device="cuda"), n_seqs=len(new),
+                           max_q_len=max(new), max_kv_len=int(arrays["seq_kv_len"].max()), fenced=False, **dev)
+
+
+@pytest.mark.parametrize("dim,vdim,rank,heads,window,sink", [(128, 128, 512, 3, None, True), (128, 64, 256, 2, 100, False),
+                                                             (64, 128, 48, 5, 64, True), (64, 64, 128, 1, None, False)])
+@pytest.mark.parametrize("past,new", [([0], [257]), ([0, 63, 130], [128, 33, 64]), ([700, 5], [40, 300])])
+def test_formed_keys_and_values(dim, vdim, rank, heads, window, sink, past, new):
+    from starter_b200 import ops
+
+    gen = torch.Generator().manual_seed(dim + rank + sum(new))
+    rot, scale = 64, (dim + 64) ** -0.5
+    n, slots = len(new), [2, 0, 1][:len(new)]
+    pages = [-(-(p + m) // 64) for p, m in zip(past, new)]
+    order = torch.randperm(sum(pages) + 2, generator=gen)
+    table = torch.zeros(3, max(pages), dtype=torch.int32)
+    store = torch.full((sum(pages) + 2, 1, 64, rank + rot), math.nan, dtype=BF)       # stale rows
+    ukv = (torch.randn(heads * (dim + vdim), rank, generator=gen, dtype=F) * rank ** -0.5).to(BF)
+    q = torch.randn(sum(new), heads * (dim + rot), generator=gen, dtype=F).to(BF)
+    sinks = torch.linspace(-1.0, 2.0, heads) if sink else None
+    want, at, qat = [], 0, 0
+    for i in range(n):
+        length = past[i] + new[i]
+        rows = torch.randn(length, rank + rot, generator=gen, dtype=F).to(BF)
+        for j in range(pages[i]):
+            page = int(order[at + j])
+            table[slots[i], j] = page
+            part = rows[64 * j:64 * (j + 1)]
+            store[page, 0, :part.shape[0]] = part
+        at += pages[i]
+        r = rows.double()
+        kv = (r[:, :rank] @ ukv.double().t())
+        k = torch.cat([kv[:, :heads * dim].view(length, heads, dim), r[:, None, rank:].expand(length, heads, rot)], dim=-1)
+        v = kv[:, heads * dim:].view(length, heads, vdim)
+        qq = q[qat:qat + new[i]].double().view(new[i], heads, dim + rot)
+        qat += new[i]
+        s = torch.einsum("thd,jhd->htj", qq, k) * scale
+        i_at, j_at = torch.arange(past[i], length)[:, None], torch.arange(length)[None, :]
+        s = s.masked_fill((j_at > i_at) | ((i_at - j_at >= window) if window else (j_at > i_at)), -math.inf)
+        if sink:
+            s = torch.cat([s, sinks.double()[:, None, None].expand(heads, new[i], 1)], dim=-1)
+        want.append(torch.einsum("htj,jhd->thd", torch.softmax(s, dim=-1)[..., :length], v).flatten(1))
+    want = torch.cat(want)
+    ctx = context(past, new, slots)
+    assert ops.latent_prompt_takes(BF, ctx, dim, rot, vdim, rank, scale, window)
+    got = ops.latent_attention_prompt(q.cuda(), ukv.cuda(), store.cuda(), table.cuda(), ctx, heads, dim, vdim, rank, rot, scale,
+                                      window, sinks.cuda() if sink else None)
+    assert int(ctx.status.item()) == 0
+    # keys, values, weights and outputs are each rounded to 8 bits: a few 2^-9 of a row's size
+    off = got.cpu().double() - want
+    assert float(off.norm() / want.norm()) < 8e-3
+    assert float(off.abs().max()) < 0.05 * float(want.abs().max())
+
+
+@pytest.mark.parametrize("window,layout,gate", [(None, "interleaved", True), (90, "half_split", False)])
+def test_the_layer_on_either_kernel(window, layout, gate, monkeypatch):
+    from starter_b200 import ops
+    from starter_b200.cache import SequenceCache
+    from starter_b200.config import spec as S
+    from starter_b200.parts import lookup
+    from starter_b200.weights import random_tensor
+
+    where = (S.InterleavedRopeSpec if layout == "interleaved" else S.PartialRopeSpec)(32, 1e4)
+    spec = S.LatentAttentionSpec(256, 4, 64, 64, 128, 192, 128, 128 ** -0.5, 1e-6, where, window=window, sink=True, output_gate=gate)
+    part = lookup("mixer", spec.kind)(spec, BF, lookup("position", where.kind)(where, BF, "cuda"))
+    part.set_params({name: random_tensor(1, name, p, torch.float32 if p.role in ("gain32", "vector32") else BF, "cuda") * 3
+                     for name, p in part.param_specs().items()})
+    part.prepare(400)
+    outs = []
+    for tokens in (32, 1 << 30):
+        monkeypatch.setattr(ops, "LATENT_PROMPT_TOKENS", tokens)
+        cache = SequenceCache({0: part.kv_need()}, {}, 1024, 2, BF, "cuda")
+        slots, rows = [cache.open_sequence(), cache.open_sequence()], []
+        gen = torch.Generator(device="cuda").manual_seed(5)
+        for new in ([150, 33], [64, 130]):
+            past = [cache.lengths[s] for s in slots]
+            for s, m in zip(slots, new):
+                cache.reserve(s, cache.lengths[s] + m)
+                cache.advance(s, m)
+            cache.sync_table()
+            ctx = context(past, new, slots)
+            ctx.cache = cache
+            x = torch.randn(sum(new), 256, generator=gen, device="cuda").to(BF)
+            rows.append(part(x, ctx, 0))
+        outs.append(torch.cat(rows).double())
+    assert float((outs[0] - outs[1]).norm() / outs[1].norm()) < 1.5e-2
