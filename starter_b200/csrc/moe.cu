@@ -33,6 +33,7 @@
 #define MOE_BK 32
 #define MOE_MAX_EXPERTS 1024
 #define MOE_MAX_TOP 16
+#define MOE_STAGE_BYTES 32768
 
 // The gated expert's activation from its (rounded) gate and up products.  limit > 0: the clamped gate,
 // min(g, limit) * sigmoid(1.702 min(g, limit)) * (clamp(u, -limit, limit) + 1); limit == 0: no clamps and the
@@ -46,39 +47,116 @@ __device__ __forceinline__ float moe_gate(float g, float u, float limit) {
   return g / (1.f + expf(-g)) * u;
 }
 
-template <typename T>
-__global__ void moe_route_kernel(const T* __restrict__ h, const float* __restrict__ w, const float* __restrict__ b,
-                                 int* __restrict__ ids, float* __restrict__ weights, int width, int experts, int top,
-                                 int scoring, float weight_scale) {
-  extern __shared__ float z[];
-  pdl_wait();      // no early launch_dependents: the successor starts when this kernel's blocks have exited
-  SB_BEHIND_WAIT(h);
-  const int row = blockIdx.x;
+// The logits of TOK tokens from `row0` on (rows past `n_tokens` repeat the last one): z[token][output].  A warp takes EXP outputs
+// and all TOK tokens at a time: a piece of a router's row serves TOK tokens, a piece of a token EXP outputs (one output a warp and one token
+// a block read 128 KB of router from L2 a token with 16 experts of 2,048: 46 us for 2,048 tokens, now 17).  A sum is the
+// same whatever EXP and TOK are.
+template <typename T, int TOK, int EXP>
+__device__ __forceinline__ void moe_logits(const T* __restrict__ h, const float* __restrict__ w, const float* __restrict__ b,
+                                           float* z, int ldz, int row0, int n_tokens, int width, int outputs, int rows) {
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, warps = blockDim.x >> 5;
-  const T* hr = h + (size_t)row * width;
-  // (16-byte pieces of the router's rows when the rows allow it: a lane's loads are then all in flight together)
-  const bool wide = width % 4 == 0 && ((uintptr_t)w % 16) == 0 && ((uintptr_t)hr % 8) == 0;
-  for (int e = warp; e < experts; e += warps) {
-    const float* wr = w + (size_t)e * width;
-    float a = 0.f;
+  // (16-byte pieces of the router's rows when the rows allow it)
+  const bool wide = width % 4 == 0 && ((uintptr_t)w % 16) == 0 && ((uintptr_t)h % 8) == 0;
+  const T* ht[TOK];
+#pragma unroll
+  for (int t = 0; t < TOK; ++t) ht[t] = h + (size_t)min(row0 + t, n_tokens - 1) * width;
+  for (int e0 = warp * EXP; e0 < rows; e0 += warps * EXP) {
+    const float* wr[EXP];
+#pragma unroll
+    for (int e = 0; e < EXP; ++e) wr[e] = w + (size_t)min(e0 + e, rows - 1) * width;
+    float a[EXP][TOK];
+#pragma unroll
+    for (int e = 0; e < EXP; ++e)
+#pragma unroll
+      for (int t = 0; t < TOK; ++t) a[e][t] = 0.f;
     if (wide && sizeof(T) == 2) {
-      const float4* w4 = reinterpret_cast<const float4*>(wr);
-      const uint2* h4 = reinterpret_cast<const uint2*>(hr);
-#pragma unroll 4
-      for (int c = lane; c < width / 4; c += 32) {
-        const float4 wv = w4[c];
-        const uint2 hv = h4[c];
-        a += __uint_as_float(hv.x << 16) * wv.x + __uint_as_float(hv.x & 0xffff0000u) * wv.y +
-             __uint_as_float(hv.y << 16) * wv.z + __uint_as_float(hv.y & 0xffff0000u) * wv.w;
+      // BATCH pieces of every row in flight together (no condition between the loads and the sums, or the compiler moves each
+      // load to its use)
+      constexpr int BATCH = TOK * EXP == 1 ? 16 : 4;
+      const int pieces = width / 4;
+      auto add = [](float& sum, const uint2& hv, const float4& wv) {
+        sum += __uint_as_float(hv.x << 16) * wv.x + __uint_as_float(hv.x & 0xffff0000u) * wv.y +
+               __uint_as_float(hv.y << 16) * wv.z + __uint_as_float(hv.y & 0xffff0000u) * wv.w;
+      };
+      int c0 = 0;
+      for (; c0 + 32 * BATCH <= pieces; c0 += 32 * BATCH) {
+        float4 wv[BATCH][EXP];
+        uint2 hv[BATCH][TOK];
+#pragma unroll
+        for (int i = 0; i < BATCH; ++i) {
+#pragma unroll
+          for (int e = 0; e < EXP; ++e) wv[i][e] = reinterpret_cast<const float4*>(wr[e])[c0 + 32 * i + lane];
+#pragma unroll
+          for (int t = 0; t < TOK; ++t) hv[i][t] = reinterpret_cast<const uint2*>(ht[t])[c0 + 32 * i + lane];
+        }
+#pragma unroll
+        for (int i = 0; i < BATCH; ++i)
+#pragma unroll
+          for (int e = 0; e < EXP; ++e)
+#pragma unroll
+            for (int t = 0; t < TOK; ++t) add(a[e][t], hv[i][t], wv[i][e]);
+      }
+      for (int c = c0 + lane; c < pieces; c += 32) {
+#pragma unroll
+        for (int e = 0; e < EXP; ++e) {
+          const float4 wv = reinterpret_cast<const float4*>(wr[e])[c];
+#pragma unroll
+          for (int t = 0; t < TOK; ++t) add(a[e][t], reinterpret_cast<const uint2*>(ht[t])[c], wv);
+        }
       }
     } else {
-      for (int c = lane; c < width; c += 32) a += to_f<T>(hr[c]) * wr[c];
+      for (int c = lane; c < width; c += 32)
+#pragma unroll
+        for (int e = 0; e < EXP; ++e)
+#pragma unroll
+          for (int t = 0; t < TOK; ++t) a[e][t] += to_f<T>(ht[t][c]) * wr[e][c];
     }
-    a = warp_sum(a);
-    if (lane == 0) z[e] = a + (b ? b[e] : 0.f);
+#pragma unroll
+    for (int e = 0; e < EXP; ++e)
+#pragma unroll
+      for (int t = 0; t < TOK; ++t) {
+        const float v = warp_sum(a[e][t]);
+        if (lane == 0 && e0 + e < rows) z[t * ldz + e0 + e] = v + (b && e0 + e < outputs ? b[e0 + e] : 0.f);
+      }
   }
+}
+
+// The block's TOK rows of h into shared memory, all pieces in flight at once (a warp that reads them piece by piece beside the
+// router's rows waits for memory eight times); returns where they are, or null where they do not fit or come in no whole pieces.
+template <typename T, int TOK>
+__device__ __forceinline__ const T* moe_stage_rows(const T* __restrict__ h, unsigned char* to, int row0, int n_tokens, int width) {
+  if (TOK == 1 || (width * sizeof(T)) % 16 || ((uintptr_t)h % 16) || TOK * width * sizeof(T) > MOE_STAGE_BYTES) return nullptr;
+  const int pieces = width * (int)sizeof(T) / 16;
+#pragma unroll
+  for (int t = 0; t < TOK; ++t) {
+    const unsigned char* from = reinterpret_cast<const unsigned char*>(h + (size_t)min(row0 + t, n_tokens - 1) * width);
+    for (int c = threadIdx.x; c < pieces; c += blockDim.x) {
+      const unsigned d = (unsigned)__cvta_generic_to_shared(to + ((size_t)t * pieces + c) * 16);
+      asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(d), "l"(from + (size_t)c * 16) : "memory");
+    }
+  }
+  asm volatile("cp.async.commit_group;\n\tcp.async.wait_group 0;" ::: "memory");
   __syncthreads();
-  if (warp == 0) {
+  return reinterpret_cast<const T*>(to);
+}
+
+// TOK tokens a block; a warp chooses for a token.
+template <typename T, int TOK>
+__global__ void __launch_bounds__(512) moe_route_kernel(const T* __restrict__ h, const float* __restrict__ w, const float* __restrict__ b,
+                                 int* __restrict__ ids, float* __restrict__ weights, int n_tokens, int width, int experts, int top,
+                                 int scoring, float weight_scale) {
+  extern __shared__ __align__(16) unsigned char route_smem[];
+  float* route_z = reinterpret_cast<float*>(route_smem + (TOK > 1 ? MOE_STAGE_BYTES : 0));
+  pdl_wait();      // no early launch_dependents: the successor starts when this kernel's blocks have exited
+  SB_BEHIND_WAIT(h);
+  const int row0 = blockIdx.x * TOK;
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, warps = blockDim.x >> 5;
+  const T* staged = moe_stage_rows<T, TOK>(h, route_smem, row0, n_tokens, width);
+  moe_logits<T, TOK, TOK>(staged ? staged : h, w, b, route_z, experts, staged ? 0 : row0, staged ? TOK : n_tokens, width, experts, experts);
+  __syncthreads();
+  for (int t = warp; t < TOK && row0 + t < n_tokens; t += warps) {
+    const int row = row0 + t;
+    float* z = route_z + t * experts;
     float best[MOE_MAX_TOP];
     float top_max = 0.f;
     for (int c = 0; c < top; ++c) {
@@ -95,6 +173,7 @@ __global__ void moe_route_kernel(const T* __restrict__ h, const float* __restric
       if (at >= experts) at = 0;          // no finite logit left: keep the indices inside the table
       if (c == 0) top_max = v;
       best[c] = v;
+      __syncwarp();
       if (lane == 0) {
         ids[(size_t)row * top + c] = at;
         z[at] = -INFINITY;
@@ -120,43 +199,27 @@ __global__ void moe_route_kernel(const T* __restrict__ h, const float* __restric
 
 // The router of the softmax over all outputs (see sb_moe_route_all).  z holds outputs + 1 logits (the last one
 // the shared expert's gate, when asked for), then the scores, the choice numbers and the groups' maxima.
-template <typename T>
-__global__ void moe_route_all_kernel(const T* __restrict__ h, const float* __restrict__ w,
+template <typename T, int TOK>
+__global__ void __launch_bounds__(512) moe_route_all_kernel(const T* __restrict__ h, const float* __restrict__ w,
                                      const float* __restrict__ correction, int* __restrict__ ids,
-                                     float* __restrict__ weights, float* __restrict__ gate_out, int width, int outputs,
+                                     float* __restrict__ weights, float* __restrict__ gate_out, int n_tokens, int width, int outputs,
                                      int top, int groups, int keep, float weight_scale) {
-  extern __shared__ float z[];
+  extern __shared__ __align__(16) unsigned char route_smem[];
+  float* route_z = reinterpret_cast<float*>(route_smem + (TOK > 1 ? MOE_STAGE_BYTES : 0));
+  pdl_wait();      // no early launch_dependents: the successor starts when this kernel's blocks have exited
+  SB_BEHIND_WAIT(h);
+  const int row0 = blockIdx.x * TOK, per_token = 3 * outputs + 1 + groups;
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, warps = blockDim.x >> 5;
+  const T* staged = moe_stage_rows<T, TOK>(h, route_smem, row0, n_tokens, width);
+  moe_logits<T, TOK, TOK>(staged ? staged : h, w, nullptr, route_z, per_token, staged ? 0 : row0, staged ? TOK : n_tokens, width, outputs,
+                          outputs + (gate_out ? 1 : 0));
+  __syncthreads();
+  for (int t = warp; t < TOK && row0 + t < n_tokens; t += warps) {
+  const int row = row0 + t;
+  float* z = route_z + t * per_token;
   float* score = z + outputs + 1;
   float* choice = score + outputs;
   float* best_of = choice + outputs;
-  pdl_wait();      // no early launch_dependents: the successor starts when this kernel's blocks have exited
-  SB_BEHIND_WAIT(h);
-  const int row = blockIdx.x;
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, warps = blockDim.x >> 5;
-  const T* hr = h + (size_t)row * width;
-  const int rows = outputs + (gate_out ? 1 : 0);
-  const bool wide = width % 4 == 0 && ((uintptr_t)w % 16) == 0 && ((uintptr_t)hr % 8) == 0;
-  for (int e = warp; e < rows; e += warps) {
-    const float* wr = w + (size_t)e * width;
-    float a = 0.f;
-    if (wide && sizeof(T) == 2) {
-      const float4* w4 = reinterpret_cast<const float4*>(wr);
-      const uint2* h4 = reinterpret_cast<const uint2*>(hr);
-#pragma unroll 4
-      for (int c = lane; c < width / 4; c += 32) {
-        const float4 wv = w4[c];
-        const uint2 hv = h4[c];
-        a += __uint_as_float(hv.x << 16) * wv.x + __uint_as_float(hv.x & 0xffff0000u) * wv.y +
-             __uint_as_float(hv.y << 16) * wv.z + __uint_as_float(hv.y & 0xffff0000u) * wv.w;
-      }
-    } else {
-      for (int c = lane; c < width; c += 32) a += to_f<T>(hr[c]) * wr[c];
-    }
-    a = warp_sum(a);
-    if (lane == 0) z[e] = a;
-  }
-  __syncthreads();
-  if (warp != 0) return;
   if (gate_out && lane == 0) gate_out[row] = 1.f / (1.f + expf(-z[outputs]));
   float top_z = -INFINITY;
   for (int e = lane; e < outputs; e += 32) top_z = fmaxf(top_z, z[e]);
@@ -223,38 +286,88 @@ __global__ void moe_route_all_kernel(const T* __restrict__ h, const float* __res
     for (int c = 0; c < top; ++c) total += picked[c];
     for (int c = 0; c < top; ++c) weights[(size_t)row * top + c] = picked[c] / (total + 1e-20f) * weight_scale;
   }
+  }
+}
+
+// The lanes of the warp that hold the same number below 2^bits (a vote a bit; the hardware's own match takes a warp's time a
+// distinct number).
+__device__ __forceinline__ unsigned moe_same(int e, int bits) {
+  unsigned same = 0xffffffffu;
+  for (int b = 0; b < bits; ++b) {
+    const bool set = (e >> b) & 1;
+    const unsigned votes = __ballot_sync(0xffffffffu, set);
+    same &= set ? votes : ~votes;
+  }
+  return same;
 }
 
 // One block.  ids: [n_pairs]; sorted: [capacity] receives pair numbers or -1; tile_expert: [max_tiles].
-__global__ void moe_align_kernel(const int* __restrict__ ids, int n_pairs, int experts, int* __restrict__ sorted,
-                                 int capacity, int* __restrict__ tile_expert, int* __restrict__ n_tiles, int bm) {
-  __shared__ int count[MOE_MAX_EXPERTS], offset[MOE_MAX_EXPERTS], total;
+// The lanes of a warp that hold one expert count, and take their places, together (16 experts of 8,192 pairs would otherwise
+// queue at 16 counters: 24 us of a prompt's step, 12 now).
+__global__ void __launch_bounds__(1024)
+moe_align_kernel(const int* __restrict__ ids, int n_pairs, int experts, int* __restrict__ sorted, int capacity,
+                 int* __restrict__ tile_expert, int* __restrict__ n_tiles, int bm) {
+  __shared__ int count[MOE_MAX_EXPERTS], offset[MOE_MAX_EXPERTS];
   pdl_wait();      // no early launch_dependents: the successor starts when this kernel's blocks have exited
   SB_BEHIND_WAIT(ids);
-  for (int e = threadIdx.x; e < experts; e += blockDim.x) count[e] = 0;
+  const int tid = threadIdx.x, lane = tid & 31, threads = blockDim.x;
+  const int bits = 32 - __clz(experts);             // (numbers up to `experts`, which stands for all that have no tile)
+  for (int e = tid; e < experts; e += threads) count[e] = 0;
   __syncthreads();
   // (an id from `experts` on names an identity expert: it has no tile)
-  for (int i = threadIdx.x; i < n_pairs; i += blockDim.x)
-    if (ids[i] < experts) atomicAdd(&count[ids[i]], 1);
-  __syncthreads();
-  if (threadIdx.x == 0) {
-    int off = 0, tiles = 0;
-    for (int e = 0; e < experts; ++e) {
-      offset[e] = off;
-      const int nt = (count[e] + bm - 1) / bm;
-      for (int t = 0; t < nt; ++t) tile_expert[tiles++] = e;
-      off += nt * bm;
-      count[e] = 0;
+  for (int b0 = tid - lane; b0 < n_pairs; b0 += 8 * threads) {
+    int e[8];
+#pragma unroll
+    for (int n = 0; n < 8; ++n) e[n] = b0 + n * threads + lane < n_pairs ? min((unsigned)ids[b0 + n * threads + lane], (unsigned)experts) : experts;
+#pragma unroll
+    for (int n = 0; n < 8; ++n) {
+      if (b0 + n * threads >= n_pairs) break;
+      const unsigned same = moe_same(e[n], bits);
+      if (e[n] < experts && lane == __ffs(same) - 1) atomicAdd(&count[e[n]], __popc(same));
     }
-    n_tiles[0] = tiles;
-    total = off;
   }
   __syncthreads();
-  for (int i = threadIdx.x; i < total && i < capacity; i += blockDim.x) sorted[i] = -1;
+  // the experts' first tiles: the first warp, 32 experts at a time
+  if (tid < 32) {
+    int tiles = 0;
+    for (int e0 = 0; e0 < experts; e0 += 32) {
+      const int e = e0 + lane, mine = e < experts ? (count[e] + bm - 1) / bm : 0;
+      int upto = mine;
+#pragma unroll
+      for (int o = 1; o < 32; o <<= 1) {
+        const int v = __shfl_up_sync(0xffffffffu, upto, o);
+        if (lane >= o) upto += v;
+      }
+      if (e < experts) offset[e] = (tiles + upto - mine) * bm;
+      tiles += __shfl_sync(0xffffffffu, upto, 31);
+    }
+    if (lane == 0) n_tiles[0] = tiles;
+  }
   __syncthreads();
-  for (int i = threadIdx.x; i < n_pairs; i += blockDim.x) {
-    const int e = ids[i];
-    if (e < experts) sorted[offset[e] + atomicAdd(&count[e], 1)] = i;
+  // a warp an expert: its tiles' names, and -1 behind its pairs
+  for (int e = tid >> 5; e < experts; e += threads >> 5) {
+    const int n = count[e], first = offset[e], nt = (n + bm - 1) / bm;
+    for (int t = lane; t < nt; t += 32) tile_expert[first / bm + t] = e;
+    for (int i = first + n + lane; i < first + nt * bm && i < capacity; i += 32) sorted[i] = -1;
+  }
+  __syncthreads();
+  for (int e = tid; e < experts; e += threads) count[e] = 0;
+  __syncthreads();
+  for (int b0 = tid - lane; b0 < n_pairs; b0 += 8 * threads) {
+    int e[8];
+#pragma unroll
+    for (int n = 0; n < 8; ++n) e[n] = b0 + n * threads + lane < n_pairs ? min((unsigned)ids[b0 + n * threads + lane], (unsigned)experts) : experts;
+#pragma unroll
+    for (int n = 0; n < 8; ++n) {
+      if (b0 + n * threads >= n_pairs) break;
+      const unsigned same = moe_same(e[n], bits);
+      const int leader = __ffs(same) - 1;
+      const bool real = e[n] < experts;
+      int at = 0;
+      if (real && lane == leader) at = atomicAdd(&count[e[n]], __popc(same));
+      at = __shfl_sync(0xffffffffu, at, leader);
+      if (real) sorted[offset[e[n]] + at + __popc(same & ((1u << lane) - 1u))] = b0 + n * threads + lane;
+    }
   }
 }
 
@@ -775,9 +888,10 @@ moe_few_kernel(const bf16* __restrict__ x, const bf16* __restrict__ w, bf16* __r
 }
 
 // The rows of h in the order of `sorted` (a pair's row is h[pair / top]; zeros where a tile is padded), for a
-// product that wants its rows in place: a block a row, 16-byte pieces.  Rows behind the last tile stay unwritten.
+// product that wants its rows in place: a block MOE_GATHER rows, whose 16-byte pieces are in flight together.  Rows behind the last tile stay unwritten.
 // in_scale (float [pairs] or null) multiplies the rows.
-__global__ void moe_gather_kernel(const bf16* __restrict__ h, const int* __restrict__ sorted,
+#define MOE_GATHER 4
+__global__ void __launch_bounds__(256) moe_gather_kernel(const bf16* __restrict__ h, const int* __restrict__ sorted,
                                   const int* __restrict__ n_tiles, int tile_rows, int top, bf16* __restrict__ out,
                                   int width, const float* __restrict__ in_scale) {
   pdl_wait();      // no early launch_dependents: the successor starts when this kernel's blocks have exited
@@ -785,25 +899,29 @@ __global__ void moe_gather_kernel(const bf16* __restrict__ h, const int* __restr
   SB_BEHIND_WAIT(sorted);
   SB_BEHIND_WAIT(n_tiles);
   SB_BEHIND_WAIT(in_scale);
-  const int row = blockIdx.x;
-  if (row >= n_tiles[0] * tile_rows) return;
-  const int pair = sorted[row];
-  const uint4* from = reinterpret_cast<const uint4*>(h + (size_t)(pair >= 0 ? pair / top : 0) * width);
-  uint4* to = reinterpret_cast<uint4*>(out + (size_t)row * width);
-  if (in_scale && pair >= 0) {
-    const float by = in_scale[pair];
-    for (int c = threadIdx.x; c < width / 8; c += blockDim.x) {
-      float f[8];
-      moe_unpack8(from[c], f);
-      uint4 o;
-      __nv_bfloat162* e = reinterpret_cast<__nv_bfloat162*>(&o);
+  const int rows = n_tiles[0] * tile_rows, row0 = blockIdx.x * MOE_GATHER;
+  if (row0 >= rows) return;
+  int pair[MOE_GATHER];
 #pragma unroll
-      for (int i = 0; i < 4; ++i) e[i] = __floats2bfloat162_rn(f[2 * i] * by, f[2 * i + 1] * by);
-      to[c] = o;
+  for (int r = 0; r < MOE_GATHER; ++r) pair[r] = row0 + r < rows ? sorted[row0 + r] : -1;
+  for (int c = threadIdx.x; c < width / 8; c += blockDim.x) {
+    uint4 v[MOE_GATHER];
+#pragma unroll
+    for (int r = 0; r < MOE_GATHER; ++r)
+      v[r] = pair[r] >= 0 ? reinterpret_cast<const uint4*>(h + (size_t)(pair[r] / top) * width)[c] : make_uint4(0u, 0u, 0u, 0u);
+#pragma unroll
+    for (int r = 0; r < MOE_GATHER; ++r) {
+      if (in_scale && pair[r] >= 0) {
+        const float by = in_scale[pair[r]];
+        float f[8];
+        moe_unpack8(v[r], f);
+        __nv_bfloat162* e = reinterpret_cast<__nv_bfloat162*>(&v[r]);
+#pragma unroll
+        for (int i = 0; i < 4; ++i) e[i] = __floats2bfloat162_rn(f[2 * i] * by, f[2 * i + 1] * by);
+      }
+      if (row0 + r < rows) reinterpret_cast<uint4*>(out + (size_t)(row0 + r) * width)[c] = v[r];
     }
-    return;
   }
-  for (int c = threadIdx.x; c < width / 8; c += blockDim.x) to[c] = pair >= 0 ? from[c] : make_uint4(0u, 0u, 0u, 0u);
 }
 
 // weights null: the choices are summed as they are.  ids / h (null: every choice is a real expert): a choice from `experts` on stands for the token's own row h[t].
@@ -831,6 +949,63 @@ __global__ void moe_combine_kernel(const T* __restrict__ down, const float* __re
     if (shared) a += sg * to_f<T>(shared[(size_t)row * width + c]);
     out[(size_t)row * width + c] = from_f<T>(a);
   }
+}
+
+// The same for bfloat16 rows of 16-byte pieces: a thread a piece of a token's row, all the choices' loads in flight (a block a
+// token and two bytes a load took 16 us for 8 rows of 2,048 and 31 for 2,048, now 3 and 7).
+template <bool OWN>
+__global__ void __launch_bounds__(128)
+moe_combine_vec_kernel(const bf16* __restrict__ down, const float* __restrict__ weights, bf16* __restrict__ out, int width, int top,
+                       const int* __restrict__ ids, int experts, const bf16* __restrict__ h, const bf16* __restrict__ shared,
+                       const float* __restrict__ shared_gate) {
+  pdl_wait();      // no early launch_dependents: the successor starts when this kernel's blocks have exited
+  SB_BEHIND_WAIT(down);
+  SB_BEHIND_WAIT(weights);
+  SB_BEHIND_WAIT(ids);
+  SB_BEHIND_WAIT(h);
+  SB_BEHIND_WAIT(shared);
+  SB_BEHIND_WAIT(shared_gate);
+  const size_t row = blockIdx.x;
+  const int c = (blockIdx.y * 128 + threadIdx.x) * 8;
+  if (c >= width) return;
+  float a[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
+  auto piece = [&](int j, float& by) {
+    const size_t at = row * top + j;
+    by = weights ? weights[at] : 1.f;
+    return *reinterpret_cast<const uint4*>(OWN && ids[at] >= experts ? h + row * width + c : down + at * width + c);
+  };
+  auto add = [&](const uint4& v, float by) {
+    float f[8];
+    moe_unpack8(v, f);
+#pragma unroll
+    for (int i = 0; i < 8; ++i) a[i] += by * f[i];
+  };
+  int j = 0;
+  for (; j + 4 <= top; j += 4) {
+    uint4 v[4];
+    float by[4];
+#pragma unroll
+    for (int i = 0; i < 4; ++i) v[i] = piece(j + i, by[i]);
+#pragma unroll
+    for (int i = 0; i < 4; ++i) add(v[i], by[i]);
+  }
+  for (; j < top; ++j) {
+    float by;
+    const uint4 v = piece(j, by);
+    add(v, by);
+  }
+  if (shared) {
+    const float sg = shared_gate[row];
+    float f[8];
+    moe_unpack8(*reinterpret_cast<const uint4*>(shared + row * width + c), f);
+#pragma unroll
+    for (int i = 0; i < 8; ++i) a[i] += sg * f[i];
+  }
+  uint4 o;
+  __nv_bfloat162* e = reinterpret_cast<__nv_bfloat162*>(&o);
+#pragma unroll
+  for (int i = 0; i < 4; ++i) e[i] = __floats2bfloat162_rn(a[2 * i], a[2 * i + 1]);
+  *reinterpret_cast<uint4*>(out + row * width + c) = o;
 }
 
 // up 1: x = h [n_tokens, k_dim], w = [experts, 2 * n_out, k_dim] (gate rows, then up rows), y =
@@ -910,7 +1085,7 @@ int sb_moe_gather(const void* h, const int* sorted, const int* n_tiles, int tile
                   int width, const float* in_scale, cudaStream_t s) {
   if (capacity == 0) return 0;
   if (width % 8 || ((uintptr_t)h % 16) || ((uintptr_t)out % 16) || top < 1) return -2;
-  return launch_dependent(moe_gather_kernel, dim3(capacity), dim3(width / 8 >= 256 ? 256 : 128), 0, s, (const bf16*)h,
+  return launch_dependent(moe_gather_kernel, dim3((capacity + MOE_GATHER - 1) / MOE_GATHER), dim3(width / 8 >= 256 ? 256 : 128), 0, s, (const bf16*)h,
                           sorted, n_tiles, tile_rows, top, (bf16*)out, width, in_scale);
 }
 int sb_moe_max_experts() { return MOE_MAX_EXPERTS; }
@@ -925,20 +1100,25 @@ int sb_moe_route(int dtype, const void* h, const float* w, const float* b, int* 
   if (n_tokens == 0) return 0;
   if (experts < 1 || experts > MOE_MAX_EXPERTS || top < 1 || top > MOE_MAX_TOP || top > experts) return -2;
   if (scoring != 0 && scoring != 1 && scoring != 3) return -2;
-  const size_t smem = (size_t)experts * sizeof(float);
-  // a step of few rows leaves most SMs idle: a warp an expert (up to 16) shortens the one block a row
-  const int threads = n_tokens <= 64 ? (experts >= 16 ? 512 : experts > 4 ? 256 : 128) : 128;
-  if (dtype == 0)
-    return launch_dependent(moe_route_kernel<float>, dim3(n_tokens), dim3(threads), smem, s, (const float*)h, w, b, ids,
-                            weights, width, experts, top, scoring, weight_scale);
-  return launch_dependent(moe_route_kernel<bf16>, dim3(n_tokens), dim3(threads), smem, s, (const bf16*)h, w, b, ids,
-                          weights, width, experts, top, scoring, weight_scale);
+  // a step of few rows leaves most SMs idle: a token a block and a warp an expert (up to 16) shorten the chain; from 4 tokens
+  // an SM on, 4 tokens a block read the router once for all of them
+  const bool many = n_tokens >= 4 * 148 && experts <= 512;
+  const int threads = many ? (experts > 16 ? 256 : 128) : experts >= 16 ? 512 : experts > 4 ? 256 : 128;
+  const int blocks = many ? (n_tokens + 3) / 4 : n_tokens;
+  const size_t smem = (many ? MOE_STAGE_BYTES : 0) + (size_t)(many ? 4 : 1) * experts * sizeof(float);      // (under 48 KB)
+#define MOE_ROUTE(T, TOK)                                                                                                  \
+  return launch_dependent(moe_route_kernel<T, TOK>, dim3(blocks), dim3(threads), smem, s, (const T*)h, w, b, ids, weights, \
+                          n_tokens, width, experts, top, scoring, weight_scale)
+  if (dtype == 0) { if (many) MOE_ROUTE(float, 4); MOE_ROUTE(float, 1); }
+  if (many) MOE_ROUTE(bf16, 4);
+  MOE_ROUTE(bf16, 1);
+#undef MOE_ROUTE
 }
 
 int sb_moe_align(const int* ids, int n_pairs, int experts, int* sorted, int capacity, int* tile_expert, int* n_tiles,
                  int tile_rows, cudaStream_t s) {
   if (experts < 1 || experts > MOE_MAX_EXPERTS || tile_rows < 1) return -2;
-  return launch_dependent(moe_align_kernel, dim3(1), dim3(256), 0, s, ids, n_pairs, experts, sorted, capacity,
+  return launch_dependent(moe_align_kernel, dim3(1), dim3(n_pairs > 1024 ? 1024 : 256), 0, s, ids, n_pairs, experts, sorted, capacity,
                           tile_expert, n_tiles, tile_rows);
 }
 
@@ -959,6 +1139,12 @@ int sb_moe_combine(int dtype, const void* down, const float* weights, void* out,
                    cudaStream_t s) {
   if (n_tokens == 0) return 0;
   if ((ids != nullptr) != (h != nullptr) || (shared != nullptr) != (shared_gate != nullptr)) return -2;
+  if (dtype == 1 && width % 8 == 0 && !(((uintptr_t)down | (uintptr_t)out | (uintptr_t)h | (uintptr_t)shared) % 16)) {
+    const dim3 grid(n_tokens, (width / 8 + 127) / 128);
+    return launch_dependent(ids ? moe_combine_vec_kernel<true> : moe_combine_vec_kernel<false>, grid, dim3(128), 0, s,
+                            (const bf16*)down, weights, (bf16*)out, width, top, ids, experts, (const bf16*)h, (const bf16*)shared,
+                            shared_gate);
+  }
   const int threads = width >= 1024 ? 256 : 128;
   if (dtype == 0)
     return launch_dependent(moe_combine_kernel<float>, dim3(n_tokens), dim3(threads), 0, s, (const float*)down,
@@ -979,13 +1165,17 @@ int sb_moe_route_all(int dtype, const void* h, const float* w, const float* corr
   if (n_tokens == 0) return 0;
   if (outputs < 1 || outputs > MOE_MAX_EXPERTS || top < 1 || top > MOE_MAX_TOP) return -2;
   if (groups < 1 || outputs % groups || keep < 1 || keep > groups || top > outputs / groups * keep) return -2;
-  const size_t smem = (size_t)(3 * outputs + 1 + groups) * sizeof(float);
-  const int threads = n_tokens <= 64 ? (outputs >= 16 ? 512 : outputs > 4 ? 256 : 128) : 128;
-  if (dtype == 0)
-    return launch_dependent(moe_route_all_kernel<float>, dim3(n_tokens), dim3(threads), smem, s, (const float*)h, w,
-                            correction, ids, weights, gate_out, width, outputs, top, groups, keep, weight_scale);
-  return launch_dependent(moe_route_all_kernel<bf16>, dim3(n_tokens), dim3(threads), smem, s, (const bf16*)h, w,
-                          correction, ids, weights, gate_out, width, outputs, top, groups, keep, weight_scale);
+  const bool many = n_tokens >= 4 * 148 && outputs <= 256;          // (4 tokens a block: see sb_moe_route)
+  const int threads = many ? (outputs > 16 ? 256 : 128) : outputs >= 16 ? 512 : outputs > 4 ? 256 : 128;
+  const int blocks = many ? (n_tokens + 3) / 4 : n_tokens;
+  const size_t smem = (many ? MOE_STAGE_BYTES : 0) + (size_t)(many ? 4 : 1) * (3 * outputs + 1 + groups) * sizeof(float);      // (under 48 KB)
+#define MOE_ROUTE(T, TOK)                                                                                              \
+  return launch_dependent(moe_route_all_kernel<T, TOK>, dim3(blocks), dim3(threads), smem, s, (const T*)h, w, correction, ids, \
+                          weights, gate_out, n_tokens, width, outputs, top, groups, keep, weight_scale)
+  if (dtype == 0) { if (many) MOE_ROUTE(float, 4); MOE_ROUTE(float, 1); }
+  if (many) MOE_ROUTE(bf16, 4);
+  MOE_ROUTE(bf16, 1);
+#undef MOE_ROUTE
 }
 
 }  // extern "C"
