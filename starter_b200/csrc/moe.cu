@@ -760,14 +760,14 @@ moe_tile_big_kernel(const bf16* __restrict__ x, const bf16* __restrict__ w, bf16
     }
 }
 
-// For steps with a handful of rows an expert (single tokens): a tile is up to MOE_FEW rows of one expert, kept
-// in shared memory as floats; a block takes MOE_FEW_NB weight rows, a warp one weight row at a time, which its
-// lanes read in 16-byte pieces (several in flight) and multiply with every row of the tile; sums in float,
-// joined by shuffles.  The weights are read once per tile and nothing is multiplied for padding: the step is
-// bound by the weights' bytes, not by tiles of 64 rows of which two are real.
-#define MOE_FEW 4
-#define MOE_FEW_NB 64
-#define MOE_FEW_MAX_K 12800
+// For steps with a handful of rows an expert (single tokens): a tile is up to MOE_FEW rows of one expert, the columns of an
+// m16n8k16 product whose rows are 16 weight rows (16 gate and the matching 16 up rows).  Operands go from global memory to
+// registers in 16-byte pieces: lane 4 g + x holds the pieces x, x + 4, .. of weight rows g and g + 8 and of the tile's row g, so
+// that every product sees its k entries in one order, and a warp's next eight steps of 32 entries (four with two weight blocks) are in flight together.  Four
+// warps share the k range (their sums meet in shared memory).  The step is bound by the weights' bytes, which are read once a
+// tile: 16 experts of 2,048 x 2,048 at 8 tokens, four each: 79 us up and 33 down on the CUDA cores (160 instructions a
+// 16-byte piece, two warps a scheduler), 43 and 30 now (5.7 and 4.1 TB/s)
+#define MOE_FEW 8
 __device__ __forceinline__ void moe_unpack8(const uint4& v, float* f) {
   f[0] = __uint_as_float(v.x << 16); f[1] = __uint_as_float(v.x & 0xffff0000u);
   f[2] = __uint_as_float(v.y << 16); f[3] = __uint_as_float(v.y & 0xffff0000u);
@@ -775,15 +775,15 @@ __device__ __forceinline__ void moe_unpack8(const uint4& v, float* f) {
   f[6] = __uint_as_float(v.w << 16); f[7] = __uint_as_float(v.w & 0xffff0000u);
 }
 
+
 template <int MODE>
-__global__ void __launch_bounds__(256)
+__global__ void __launch_bounds__(128)
 moe_few_kernel(const bf16* __restrict__ x, const bf16* __restrict__ w, bf16* __restrict__ y,
                const int* __restrict__ sorted, const int* __restrict__ tile_expert, const int* __restrict__ n_tiles,
                int k_dim, int n_out, int top, float limit, const float* __restrict__ in_scale) {
   constexpr bool UP = MODE != 0;
-  constexpr int NW = MODE == 1 ? 2 : 1;
-  extern __shared__ __align__(16) float moe_xf[];       // [MOE_FEW][k_dim]
-  __shared__ int src[MOE_FEW];
+  constexpr int NW = MODE == 1 ? 2 : 1, MOE_FEW_FLY = 8 / NW;
+  __shared__ float part[4][NW * 4][32];
   pdl_wait();      // no early launch_dependents: the successor starts when this kernel's blocks have exited
   SB_BEHIND_WAIT(x);
   SB_BEHIND_WAIT(sorted);
@@ -791,99 +791,66 @@ moe_few_kernel(const bf16* __restrict__ x, const bf16* __restrict__ w, bf16* __r
   SB_BEHIND_WAIT(n_tiles);
   SB_BEHIND_WAIT(in_scale);
   const int tile = blockIdx.x;
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, g = lane >> 2, q = lane & 3;
+  // (three loads at once; a tile that is not there has garbage in its places and leaves)
+  const int expert = tile_expert[tile], own = sorted[tile * MOE_FEW + g];
   if (tile >= n_tiles[0]) return;
-  const int e = tile_expert[tile];
-  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-  if (tid < MOE_FEW) src[tid] = sorted[tile * MOE_FEW + tid];
-  __syncthreads();
-  int nr = 0;                                            // an expert's pairs fill its tiles from the front
-#pragma unroll
-  for (int r = 0; r < MOE_FEW; ++r)
-    if (src[r] >= 0) nr = r + 1;
-  const int chunks = k_dim / 8;
-  for (int r = 0; r < nr; ++r) {
-    const bf16* xr = x + (UP ? (size_t)(src[r] / top) : (size_t)tile * MOE_FEW + r) * k_dim;
-    for (int c = tid; c < chunks; c += 256) {
-      float f[8];
-      moe_unpack8(*reinterpret_cast<const uint4*>(xr + c * 8), f);
-      float4* to = reinterpret_cast<float4*>(moe_xf + (size_t)r * k_dim + c * 8);
-      to[0] = make_float4(f[0], f[1], f[2], f[3]);
-      to[1] = make_float4(f[4], f[5], f[6], f[7]);
-    }
-  }
-  __syncthreads();
-  const bf16* we = w + (size_t)e * NW * n_out * k_dim;
-  constexpr int PER_WARP = MOE_FEW_NB / 8;
-  const int n_first = blockIdx.y * MOE_FEW_NB + warp * PER_WARP;
-  if (n_first >= n_out) return;
-  // the warp walks k once: at every piece its PER_WARP weight rows' loads are in flight together, and the
-  // tile's rows of that piece are read from shared memory once for all of them
-  float acc[NW][PER_WARP][MOE_FEW];
+  const bf16* we = w + (size_t)expert * NW * n_out * k_dim;
+  const int n0 = blockIdx.y * 16;
+  // this lane's row of the tile (none: the loads are of the tile's first row, the products are not stored) and its weight rows
+  const bf16* xr = x + (UP ? (size_t)(own >= 0 ? own / top : 0) : (size_t)tile * MOE_FEW + (own >= 0 ? g : 0)) * k_dim;
+  const bf16* wr[NW][2];
 #pragma unroll
   for (int a = 0; a < NW; ++a)
 #pragma unroll
-    for (int i = 0; i < PER_WARP; ++i)
+    for (int r = 0; r < 2; ++r) wr[a][r] = we + ((size_t)a * n_out + min(n0 + g + 8 * r, n_out - 1)) * k_dim;
+  const int pieces = k_dim / 8, steps = (pieces + 3) / 4;
+  float acc[NW][4];
 #pragma unroll
-      for (int r = 0; r < MOE_FEW; ++r) acc[a][i][r] = 0.f;
-  for (int c = lane; c < chunks; c += 32) {
-    float4 xv[MOE_FEW][2];
+  for (int a = 0; a < NW; ++a) acc[a][0] = acc[a][1] = acc[a][2] = acc[a][3] = 0.f;
+  for (int s0 = warp; s0 < steps; s0 += 4 * MOE_FEW_FLY) {
+    uint4 wv[MOE_FEW_FLY][NW][2], xv[MOE_FEW_FLY];
 #pragma unroll
-    for (int r = 0; r < MOE_FEW; ++r) {
-      if (r < nr) {
-        const float4* from = reinterpret_cast<const float4*>(moe_xf + (size_t)r * k_dim + c * 8);
-        xv[r][0] = from[0];
-        xv[r][1] = from[1];
-      } else {
-        xv[r][0] = xv[r][1] = make_float4(0.f, 0.f, 0.f, 0.f);
-      }
+    for (int i = 0; i < MOE_FEW_FLY; ++i) {
+      const int piece = (s0 + 4 * i) * 4 + q;
+      const bool in = piece < pieces;
+#pragma unroll
+      for (int a = 0; a < NW; ++a)
+#pragma unroll
+        for (int r = 0; r < 2; ++r)
+          wv[i][a][r] = in ? __ldg(reinterpret_cast<const uint4*>(wr[a][r]) + piece) : make_uint4(0u, 0u, 0u, 0u);
+      xv[i] = in ? reinterpret_cast<const uint4*>(xr)[piece] : make_uint4(0u, 0u, 0u, 0u);
     }
 #pragma unroll
-    for (int a = 0; a < NW; ++a) {
-      uint4 wv[PER_WARP];
+    for (int i = 0; i < MOE_FEW_FLY; ++i)
 #pragma unroll
-      for (int i = 0; i < PER_WARP; ++i) {
-        const int n = min(n_first + i, n_out - 1);       // (a row past the end repeats the last one; it is not stored)
-        wv[i] = __ldg(reinterpret_cast<const uint4*>(we + ((size_t)a * n_out + n) * k_dim) + c);
+      for (int a = 0; a < NW; ++a) {
+        const uint4 u = wv[i][a][0], v = wv[i][a][1];
+        const uint32_t lo[4] = {u.x, v.x, u.y, v.y}, hi[4] = {u.z, v.z, u.w, v.w};
+        moe_mma(acc[a], lo, xv[i].x, xv[i].y);
+        moe_mma(acc[a], hi, xv[i].z, xv[i].w);
       }
-#pragma unroll
-      for (int i = 0; i < PER_WARP; ++i) {
-        float f[8];
-        moe_unpack8(wv[i], f);
-#pragma unroll
-        for (int r = 0; r < MOE_FEW; ++r) {
-          if (r < nr) {
-            const float4 p = xv[r][0], q = xv[r][1];
-            acc[a][i][r] += f[0] * p.x + f[1] * p.y + f[2] * p.z + f[3] * p.w + f[4] * q.x + f[5] * q.y + f[6] * q.z + f[7] * q.w;
-          }
-        }
-      }
-    }
   }
 #pragma unroll
   for (int a = 0; a < NW; ++a)
 #pragma unroll
-    for (int i = 0; i < PER_WARP; ++i)
+    for (int c = 0; c < 4; ++c) part[warp][a * 4 + c][lane] = acc[a][c];
+  __syncthreads();
+  // warp c finishes accumulator c: weight row g + 8 (c / 2), the tile's row 2 q + c % 2
+  float v[NW];
 #pragma unroll
-      for (int r = 0; r < MOE_FEW; ++r) acc[a][i][r] = warp_sum(acc[a][i][r]);
-  // lane 4 i + r files weight row i for the tile's row r
-  float v0 = 0.f, v1 = 0.f;
-#pragma unroll
-  for (int i = 0; i < PER_WARP; ++i)
-#pragma unroll
-    for (int r = 0; r < MOE_FEW; ++r)
-      if (lane == i * MOE_FEW + r) { v0 = acc[0][i][r]; v1 = acc[NW - 1][i][r]; }
-  static_assert(PER_WARP * MOE_FEW == 32, "a lane for every (weight row, tile row)");
-  const int n = n_first + lane / MOE_FEW, r = lane % MOE_FEW;
-  if (n < n_out && r < nr) {
-    const float by = UP && in_scale ? in_scale[src[r]] : 1.f;
-    if (MODE == 1) {
-      y[((size_t)tile * MOE_FEW + r) * n_out + n] = from_f<bf16>(moe_gate(rnd<bf16>(v0 * by), rnd<bf16>(v1 * by), limit));
-    } else if (MODE == 2) {
-      const float u = fmaxf(rnd<bf16>(v0 * by), 0.f);
-      y[((size_t)tile * MOE_FEW + r) * n_out + n] = from_f<bf16>(u * u);
-    } else {
-      y[(size_t)src[r] * n_out + n] = from_f<bf16>(v0);
-    }
+  for (int a = 0; a < NW; ++a) v[a] = part[0][a * 4 + warp][lane] + part[1][a * 4 + warp][lane] + part[2][a * 4 + warp][lane] + part[3][a * 4 + warp][lane];
+  const int n = n0 + g + 8 * (warp >> 1), r = 2 * q + (warp & 1);
+  const int pair = sorted[tile * MOE_FEW + r];
+  if (n >= n_out || pair < 0) return;
+  const float by = UP && in_scale ? in_scale[pair] : 1.f;
+  if (MODE == 1) {
+    y[((size_t)tile * MOE_FEW + r) * n_out + n] = from_f<bf16>(moe_gate(rnd<bf16>(v[0] * by), rnd<bf16>(v[NW - 1] * by), limit));
+  } else if (MODE == 2) {
+    const float u = fmaxf(rnd<bf16>(v[0] * by), 0.f);
+    y[((size_t)tile * MOE_FEW + r) * n_out + n] = from_f<bf16>(u * u);
+  } else {
+    y[(size_t)pair * n_out + n] = from_f<bf16>(v[0]);
   }
 }
 
@@ -1018,17 +985,9 @@ static int moe_tiles_mode(int dtype, int tile_rows, const void* x, const void* w
                           const int* tile_expert, const int* n_tiles, int max_tiles, int k_dim, int n_out, int top,
                           float limit, const float* in_scale, cudaStream_t s) {
   if (tile_rows == MOE_FEW) {
-    if (dtype != 1 || k_dim % 8 || k_dim > MOE_FEW_MAX_K || ((uintptr_t)x % 16) || ((uintptr_t)w % 16)) return -2;
-    const size_t smem = (size_t)MOE_FEW * k_dim * sizeof(float);
-    static size_t configured = 0;
-    if (smem > configured) {
-      cudaError_t err = cudaFuncSetAttribute(moe_few_kernel<MODE>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-      if (err != cudaSuccess) return (int)err;
-      configured = smem;
-    }
-    return launch_dependent(moe_few_kernel<MODE>, dim3(max_tiles, (n_out + MOE_FEW_NB - 1) / MOE_FEW_NB), dim3(256), smem, s,
-                            (const bf16*)x, (const bf16*)w, (bf16*)y, sorted, tile_expert, n_tiles, k_dim, n_out, top, limit,
-                            in_scale);
+    if (dtype != 1 || k_dim % 8 || ((uintptr_t)x % 16) || ((uintptr_t)w % 16)) return -2;
+    return launch_dependent(moe_few_kernel<MODE>, dim3(max_tiles, (n_out + 15) / 16), dim3(128), 0, s, (const bf16*)x, (const bf16*)w,
+                            (bf16*)y, sorted, tile_expert, n_tiles, k_dim, n_out, top, limit, in_scale);
   }
   if (tile_rows == MOE_BIG) {
     if (dtype != 1 || k_dim % 16 || n_out % 2 || ((uintptr_t)x % 16) || ((uintptr_t)w % 16) || ((uintptr_t)y % 4)) return -2;
@@ -1067,14 +1026,15 @@ int sb_moe_tile_rows(int dtype, int width, int inner) {
   return dtype == 1 && width % 16 == 0 && inner % 16 == 0 ? MOE_TC_BM : MOE_BM;
 }
 // The same for a step of `n_pairs` (row, expert) pairs over `experts` experts: when the tensor-core tiles take
-// the operands, 4 up to four rows an expert on average (the few-row kernel), 128 from 128 rows an expert on average (the large tiles pay for their padding from there
+// the operands, 8 up to six rows an expert on average (the few-row kernel), 128 from 128 rows an expert on average (the large tiles pay for their padding from there
 // on) and 256 from 256 (the row tiles of the grouped tcgen05 product, which runs in place of these tiles);
 // else as above.
 int sb_moe_tile_rows_for(int dtype, int width, int inner, long long n_pairs, int experts) {
   const int rows = sb_moe_tile_rows(dtype, width, inner);
   if (rows != MOE_TC_BM) return rows;
-  // 4: the few-row kernel, up to four rows an expert on average (single tokens)
-  if (n_pairs <= (long long)MOE_FEW * experts && width <= MOE_FEW_MAX_K && inner <= MOE_FEW_MAX_K) return MOE_FEW;
+  // 8: the few-row kernel, up to six rows an expert on average (single tokens; beyond, many experts take two tiles of 8, which
+  // read the weights twice)
+  if (n_pairs <= 6ll * experts) return MOE_FEW;
   // 256: the grouped tcgen05 product (its row tiles), from 256 rows an expert on average
   if (n_pairs >= 256ll * experts) return 256;
   return n_pairs >= (long long)MOE_BIG * experts ? MOE_BIG : rows;
