@@ -72,6 +72,90 @@ __global__ void latent_prepare_kernel(const T* __restrict__ proj, int proj_width
   for (int c = rot_dims + threadIdx.x; c < rot; c += blockDim.x) dst[rank + c] = shared[c];
 }
 
+// The same for bfloat16 rows in 16-byte pieces: every piece is loaded once, all at once, and kept for its norm (the kernel
+// above reads a row twice, two bytes a load, one norm after the other: 16 us for 8 rows as for 2,048, a chain of latencies; now 5
+// and 15, with cold caches).  Thread t owns pieces t, t + 256 of the query latent and piece t of the key/value latent; the shared part
+// is the last warp's.
+__global__ void __launch_bounds__(256)
+latent_prepare_vec_kernel(const bf16* __restrict__ proj, int proj_width, const float* __restrict__ qg,
+                          const float* __restrict__ kg, float eps, const float* __restrict__ cos_t,
+                          const float* __restrict__ sin_t, int table_width, const int* __restrict__ tok_pos,
+                          const int* __restrict__ tok_slot, const int* __restrict__ block_table, int table_stride,
+                          bf16* __restrict__ store, bf16* __restrict__ cq, int q_rank, int kv_col, int rank, int rot,
+                          int rot_dims, int write, int split) {
+  __shared__ float2 sums[8];
+  const int row = blockIdx.x, tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  pdl_wait();      // no early launch_dependents: the successor starts when this kernel's blocks have exited
+  SB_BEHIND_WAIT(proj);
+  SB_BEHIND_WAIT(tok_pos);
+  SB_BEHIND_WAIT(tok_slot);
+  SB_BEHIND_WAIT(block_table);
+  const bf16* pr = proj + (size_t)row * proj_width;
+  const bf16* kv = pr + kv_col;
+  const int pieces = q_rank / 8, own = write ? rank / 8 : 0;
+  uint4 q[2], k = make_uint4(0u, 0u, 0u, 0u);
+#pragma unroll
+  for (int n = 0; n < 2; ++n)
+    q[n] = tid + 256 * n < pieces ? *reinterpret_cast<const uint4*>(pr + (tid + 256 * n) * 8) : make_uint4(0u, 0u, 0u, 0u);
+  if (tid < own) k = *reinterpret_cast<const uint4*>(kv + tid * 8);
+  const int pos = tok_pos[row];
+  bf16* dst = nullptr;
+  if (write) {
+    const int page = block_table[(size_t)tok_slot[row] * table_stride + pos / SB_PAGE_TOKENS];
+    dst = store + page_row(page, 0, pos % SB_PAGE_TOKENS, 1, rank + rot);
+  }
+  if (write && warp == 7) {
+    const bf16* shared = kv + rank;
+    for (int i = lane; i < rot_dims / 2; i += 32) {
+      const int ia = split ? i : 2 * i, ib = split ? i + rot_dims / 2 : 2 * i + 1;
+      const float a = to_f<bf16>(shared[ia]), b = to_f<bf16>(shared[ib]);
+      const float c = cos_t[(size_t)pos * table_width + i], s = sin_t[(size_t)pos * table_width + i];
+      dst[rank + ia] = from_f<bf16>(a * c - b * s);
+      dst[rank + ib] = from_f<bf16>(b * c + a * s);
+    }
+    for (int c = rot_dims + lane; c < rot; c += 32) dst[rank + c] = shared[c];
+  }
+  auto unpack = [](const uint4& v, float* f) {
+    const uint32_t w[4] = {v.x, v.y, v.z, v.w};
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+      f[2 * i] = __uint_as_float(w[i] << 16);
+      f[2 * i + 1] = __uint_as_float(w[i] & 0xffff0000u);
+    }
+  };
+  float f[3][8], sq = 0.f, sk = 0.f;
+  unpack(q[0], f[0]);
+  unpack(q[1], f[1]);
+  unpack(k, f[2]);
+#pragma unroll
+  for (int e = 0; e < 8; ++e) {
+    sq += f[0][e] * f[0][e] + f[1][e] * f[1][e];
+    sk += f[2][e] * f[2][e];
+  }
+  sq = warp_sum(sq);
+  sk = warp_sum(sk);
+  if (lane == 0) sums[warp] = make_float2(sq, sk);
+  __syncthreads();
+  sq = sk = 0.f;
+#pragma unroll
+  for (int w = 0; w < 8; ++w) {
+    sq += sums[w].x;
+    sk += sums[w].y;
+  }
+  const float qi = 1.f / sqrtf(sq / (float)q_rank + eps), ki = 1.f / sqrtf(sk / (float)rank + eps);
+  auto file = [](const float* f, float inv, const float* gain, bf16* to) {
+    uint4 o;
+    __nv_bfloat162* p = reinterpret_cast<__nv_bfloat162*>(&o);
+#pragma unroll
+    for (int i = 0; i < 4; ++i) p[i] = __floats2bfloat162_rn(f[2 * i] * inv * gain[2 * i], f[2 * i + 1] * inv * gain[2 * i + 1]);
+    *reinterpret_cast<uint4*>(to) = o;
+  };
+#pragma unroll
+  for (int n = 0; n < 2; ++n)
+    if (tid + 256 * n < pieces) file(f[n], qi, qg + (tid + 256 * n) * 8, cq + (size_t)row * q_rank + (tid + 256 * n) * 8);
+  if (tid < own) file(f[2], ki, kg + tid * 8, dst + tid * 8);
+}
+
 // q: [tokens, heads, dim + rot]; qa: [tokens, heads, rank + rot], whose first `rank` entries per head
 // the caller fills; this files the turned last `rot` entries of q behind them.  qa may be q itself (rank = dim): a pair is
 // read and written by one thread.
@@ -216,6 +300,11 @@ int sb_latent_prepare(int dtype, const void* proj, int proj_width, const float* 
   if (n_tokens == 0) return 0;
   if (rot_dims % 2 || rot_dims > rot || rot_dims / 2 > table_width) return -2;
   if (kv_col < q_rank || proj_width < (write ? kv_col + rank + rot : q_rank)) return -2;
+  if (dtype == 1 && q_rank > 0 && q_rank <= 4096 && rank <= 2048 && !((q_rank | kv_col | rank | rot | proj_width) % 8) &&
+      !(((uintptr_t)proj | (uintptr_t)store | (uintptr_t)cq) % 16))
+    return launch_dependent(latent_prepare_vec_kernel, dim3(n_tokens), dim3(256), 0, s, (const bf16*)proj, proj_width, qg, kg, eps,
+                            cos_t, sin_t, table_width, tok_pos, tok_slot, block_table, table_stride, (bf16*)store, (bf16*)cq, q_rank,
+                            kv_col, rank, rot, rot_dims, write, split);
   if (dtype == 0)
     return launch_dependent(latent_prepare_kernel<float>, dim3(n_tokens), dim3(128), 0, s, (const float*)proj,
                             proj_width, qg, kg, eps, cos_t, sin_t, table_width, tok_pos, tok_slot, block_table,
@@ -542,45 +631,54 @@ latent_attention_tc_kernel(const bf16* __restrict__ qa, bf16* __restrict__ out, 
   }
 }
 
-// out[row] = sum_s acc[s][row] exp(m_s - M) / (exp(sink - M) + sum_s l_s exp(m_s - M)): a block a row.  The first warp forms
-// the parts' factors (a lane a part, up to 32 parts) and leaves them in shared memory; the sums over the
-// parts then run without a branch, their loads independent of one another.
-__global__ void latent_merge_kernel(const float* __restrict__ part_acc, const float* __restrict__ part_ml,
-                                    bf16* __restrict__ out, int n_rows, int rank, int n_splits,
-                                    const float* __restrict__ sink, int heads) {
-  __shared__ float factor[32];
+// out[row] = sum_s acc[s][row] exp(m_s - M) / (exp(sink - M) + sum_s l_s exp(m_s - M)): a block a row, a thread four columns.
+// Every warp forms the parts' factors (a lane a part, up to 32 parts) and leaves none to wait for: the first eight parts' loads are
+// in flight meanwhile, then eight at a time (128 threads with one column a load behind a barrier: 21 us for 128 rows of 18 parts, 6 now).
+__global__ void __launch_bounds__(128)
+latent_merge_kernel(const float* __restrict__ part_acc, const float* __restrict__ part_ml,
+                    bf16* __restrict__ out, int n_rows, int rank, int n_splits,
+                    const float* __restrict__ sink, int heads) {
   pdl_wait();      // no early launch_dependents: the successor starts when this kernel's blocks have exited
   SB_BEHIND_WAIT(part_acc);
   SB_BEHIND_WAIT(part_ml);
-  const int row = blockIdx.x;
-  if (threadIdx.x < 32) {
-    const int s = threadIdx.x;
-    const bool has = s < n_splits;
-    const float m = has ? part_ml[((size_t)s * n_rows + row) * 2] : -INFINITY;
-    const float l = has ? part_ml[((size_t)s * n_rows + row) * 2 + 1] : 0.f;
-    float M = m;
-    for (int o = 16; o > 0; o >>= 1) M = fmaxf(M, __shfl_xor_sync(0xffffffffu, M, o));
-    const float sk = sink ? sink[row % heads] : -INFINITY;       // (rows are token-major, then heads)
-    M = fmaxf(M, sk);
-    const float e = m == -INFINITY ? 0.f : expf(m - M);
-    float L = l * e;
-    for (int o = 16; o > 0; o >>= 1) L += __shfl_xor_sync(0xffffffffu, L, o);
-    if (sink) L += expf(sk - M);
-    factor[s] = e / L;
-  }
-  __syncthreads();
-  const float* acc = part_acc + (size_t)row * rank;
+  const int row = blockIdx.x, lane = threadIdx.x & 31, c = threadIdx.x * 4;
+  const float* acc = part_acc + (size_t)row * rank + c;
   const size_t part_stride = (size_t)n_rows * rank;
-  for (int c = threadIdx.x; c < rank; c += blockDim.x) {
-    float a = 0.f;
-#pragma unroll 8
-    for (int s = 0; s < n_splits; ++s) {
-      const float f = factor[s];
-      const float v = acc[s * part_stride + c];
-      a += f != 0.f ? v * f : 0.f;          // (a part without keys left zeros; its factor is zero)
+  const bool in = c < rank;
+  float4 v[8];
+#pragma unroll
+  for (int s = 0; s < 8; ++s)
+    v[s] = in && s < n_splits ? *reinterpret_cast<const float4*>(acc + s * part_stride) : make_float4(0.f, 0.f, 0.f, 0.f);
+  const bool has = lane < n_splits;
+  const float2 ml = has ? *reinterpret_cast<const float2*>(part_ml + ((size_t)lane * n_rows + row) * 2) : make_float2(-INFINITY, 0.f);
+  const float sk = sink ? sink[row % heads] : -INFINITY;       // (rows are token-major, then heads)
+  const float M = fmaxf(warp_max(ml.x), sk);
+  const float e = ml.x == -INFINITY ? 0.f : expf(ml.x - M);
+  float L = warp_sum(ml.y * e);
+  if (sink) L += expf(sk - M);
+  const float mine = e / L;
+  float4 a = make_float4(0.f, 0.f, 0.f, 0.f);
+  for (int s0 = 0; s0 < n_splits; s0 += 8) {
+#pragma unroll
+    for (int s = 0; s < 8; ++s) {
+      const float f = s0 + s < 32 ? __shfl_sync(0xffffffffu, mine, (s0 + s) & 31) : 0.f;
+      // (a part without keys left zeros; its factor is zero, as that of a part whose weights vanish beside the others')
+      a.x += f != 0.f ? v[s].x * f : 0.f;
+      a.y += f != 0.f ? v[s].y * f : 0.f;
+      a.z += f != 0.f ? v[s].z * f : 0.f;
+      a.w += f != 0.f ? v[s].w * f : 0.f;
     }
-    out[(size_t)row * rank + c] = from_f<bf16>(a);
+    if (s0 + 8 < n_splits) {
+#pragma unroll
+      for (int s = 0; s < 8; ++s)
+        v[s] = in && s0 + 8 + s < n_splits ? *reinterpret_cast<const float4*>(acc + (s0 + 8 + s) * part_stride) : make_float4(0.f, 0.f, 0.f, 0.f);
+    }
   }
+  if (!in) return;
+  uint2 o;
+  *reinterpret_cast<__nv_bfloat162*>(&o.x) = __floats2bfloat162_rn(a.x, a.y);
+  *reinterpret_cast<__nv_bfloat162*>(&o.y) = __floats2bfloat162_rn(a.z, a.w);
+  *reinterpret_cast<uint2*>(out + (size_t)row * rank + c) = o;
 }
 
 extern "C" {
