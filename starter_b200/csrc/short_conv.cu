@@ -98,6 +98,113 @@ short_conv_kernel(const T* __restrict__ x, int ldx, const float* __restrict__ ta
   }
 }
 
+// The same for bfloat16 channels in 8-byte pieces and up to four taps: a thread four channels and a chunk of 8 tokens, all of whose
+// loads are in flight together (no condition between them and the sums, or the compiler moves each load to its use), K
+// multiply-adds an entry (the kernel above always has eight, two bytes a load, and an exact quotient that branches for every
+// value; results are rounded to bfloat16 at once, so silu takes the fast quotient).  A sum's terms come in the
+// same order.  2,136 tokens of 4,096 channels with silu: 28 -> 20 us; 2,048 of 2,304: 18 -> 13; of 3,072 without: 20 -> 10.
+#define CONV_VEC_CHUNK 8
+__device__ __forceinline__ void conv_unpack4(const uint2& v, float* f) {
+  f[0] = __uint_as_float(v.x << 16);
+  f[1] = __uint_as_float(v.x & 0xffff0000u);
+  f[2] = __uint_as_float(v.y << 16);
+  f[3] = __uint_as_float(v.y & 0xffff0000u);
+}
+
+template <int K>
+__global__ void __launch_bounds__(128)
+short_conv_vec_kernel(const bf16* __restrict__ x, int ldx, const float* __restrict__ taps, const float* __restrict__ bias,
+                      const float* __restrict__ in_bias, bf16* __restrict__ y, int ldy, float* __restrict__ state,
+                      long long slot_stride, const int* __restrict__ seq_slot, const int* __restrict__ seq_q_start,
+                      const int* __restrict__ seq_q_len, int channels, int act, int chunks) {
+  constexpr int B = K - 1;                                   // inputs in front of the chunk
+  const int c = (blockIdx.y * 128 + threadIdx.x) * 4;
+  float tap[K][4], b[4], ib[4];                              // tap[j]: of the input j tokens back
+  if (c < channels) {                                        // (weights: ahead of the wait)
+#pragma unroll
+    for (int e = 0; e < 4; ++e) {
+      b[e] = bias ? bias[c + e] : 0.f;
+      ib[e] = in_bias ? in_bias[c + e] : 0.f;
+#pragma unroll
+      for (int j = 0; j < K; ++j) tap[j][e] = taps[(size_t)(c + e) * K + (K - 1 - j)];
+    }
+  }
+  pdl_wait();      // no early launch_dependents: the successor starts when this kernel's blocks have exited
+  SB_BEHIND_WAIT(x);
+  SB_BEHIND_WAIT(state);
+  SB_BEHIND_WAIT(seq_slot);
+  SB_BEHIND_WAIT(seq_q_start);
+  SB_BEHIND_WAIT(seq_q_len);
+  const int seq = blockIdx.x / chunks, chunk = blockIdx.x - seq * chunks;
+  const int q_len = seq_q_len[seq];
+  const int t0 = chunk * CONV_VEC_CHUNK;
+  if (c >= channels || t0 >= q_len) return;
+  const size_t q_start = seq_q_start[seq];
+  float* st = state + (size_t)seq_slot[seq] * slot_stride + c;      // row j: the input j + 1 tokens back
+  const bf16* xc = x + c;
+  uint2 raw[B + CONV_VEC_CHUNK];                             // from B tokens in front of the chunk on
+#pragma unroll
+  for (int i = 0; i < B + CONV_VEC_CHUNK; ++i) {
+    const int t = t0 + i - B;
+    raw[i] = t >= 0 && t < q_len ? *reinterpret_cast<const uint2*>(xc + (q_start + t) * ldx) : make_uint2(0u, 0u);
+  }
+  float in[B + CONV_VEC_CHUNK][4], old[B > 0 ? B : 1][4];
+#pragma unroll
+  for (int i = 0; i < B + CONV_VEC_CHUNK; ++i) {
+    conv_unpack4(raw[i], in[i]);
+#pragma unroll
+    for (int e = 0; e < 4; ++e) in[i][e] += ib[e];
+  }
+  if (chunk == 0) {                                          // what earlier steps left in front of the sequence
+#pragma unroll
+    for (int j = 0; j < B; ++j)
+#pragma unroll
+      for (int e = 0; e < 4; ++e) in[B - 1 - j][e] = old[j][e] = st[(size_t)j * channels + e];
+  }
+#pragma unroll
+  for (int i = 0; i < CONV_VEC_CHUNK; ++i) {
+    float a[4];
+#pragma unroll
+    for (int e = 0; e < 4; ++e) {
+      a[e] = b[e] + tap[0][e] * in[B + i][e];
+#pragma unroll
+      for (int j = 1; j < K; ++j) a[e] += tap[j][e] * in[B + i - j][e];
+    }
+    if (act == 1) {
+#pragma unroll
+      for (int e = 0; e < 4; ++e) a[e] = gate_act_fast(a[e], SB_ACT_SILU);
+    }
+    if (t0 + i < q_len) {
+      uint2 o;
+      *reinterpret_cast<__nv_bfloat162*>(&o.x) = __floats2bfloat162_rn(a[0], a[1]);
+      *reinterpret_cast<__nv_bfloat162*>(&o.y) = __floats2bfloat162_rn(a[2], a[3]);
+      *reinterpret_cast<uint2*>(y + (q_start + t0 + i) * ldy + c) = o;
+    }
+  }
+  if (chunk != 0) return;
+  // what the sequence's next step will find in front of it (see above)
+#pragma unroll
+  for (int j = 0; j < B; ++j) {
+    const int t = q_len - 1 - j;
+    float v[4];
+    if (t >= 0) {
+      conv_unpack4(*reinterpret_cast<const uint2*>(xc + (q_start + t) * ldx), v);
+#pragma unroll
+      for (int e = 0; e < 4; ++e) v[e] += ib[e];
+    } else {
+#pragma unroll
+      for (int e = 0; e < 4; ++e) {
+        v[e] = 0.f;
+#pragma unroll
+        for (int o = 0; o < B; ++o)
+          if (o == -t - 1) v[e] = old[o][e];
+      }
+    }
+#pragma unroll
+    for (int e = 0; e < 4; ++e) st[(size_t)j * channels + e] = v[e];
+  }
+}
+
 // ------------------------------------------------------------------------------------------ the gated unit
 
 __device__ __forceinline__ float softplus_f(float z) { return z > 20.f ? z : log1pf(expf(z)); }
@@ -216,6 +323,13 @@ int sb_short_conv(int dtype, const void* x, int ldx, const float* taps, const fl
                   const int* seq_q_len, int n_seqs, int max_q_len, int channels, int K, int act, cudaStream_t s) {
   if (n_seqs == 0 || channels == 0) return 0;
   if (K < 1 || K > CONV_MAX_TAPS || K - 1 > CONV_CHUNK || max_q_len < 1) return -2;
+  if (dtype == 1 && K <= 4 && channels % 4 == 0 && ldx % 4 == 0 && ldy % 4 == 0 && !(((uintptr_t)x | (uintptr_t)y) % 8)) {
+    const int vec_chunks = (max_q_len + CONV_VEC_CHUNK - 1) / CONV_VEC_CHUNK;
+    const dim3 vec_grid(n_seqs * vec_chunks, (channels / 4 + 127) / 128);
+    auto kernel = K == 1 ? short_conv_vec_kernel<1> : K == 2 ? short_conv_vec_kernel<2> : K == 3 ? short_conv_vec_kernel<3> : short_conv_vec_kernel<4>;
+    return launch_dependent(kernel, vec_grid, dim3(128), 0, s, (const bf16*)x, ldx, taps, bias, in_bias, (bf16*)y, ldy, state,
+                            slot_stride, seq_slot, seq_q_start, seq_q_len, channels, act, vec_chunks);
+  }
   const int chunks = (max_q_len + CONV_CHUNK - 1) / CONV_CHUNK;
   const dim3 grid(n_seqs * chunks, (channels + 127) / 128);
   if (dtype == 0)
