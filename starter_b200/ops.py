@@ -2370,8 +2370,8 @@ def glru_scan(u, gates, r_bias, i_bias, lam, decay_scale, proj, y_col, y_bias, s
 
 SCAN_MODES = {"state_space": 0, "gated_delta": 1, "forget_write": 2, "channel_decay": 3}
 #: tokens a sequence on average from which a recurrence runs on the kernels for prompts.  At 16 heads of 128 x 128: 8
-#: sequences of 64 tokens take 36 to 47 us there against 60 to 79 us on the kernel for few tokens, one of 2,048 takes 164 to
-#: 203 us against 400 to 673; below, the launch that forms the coefficients or gates beforehand (5 us) is not earned back.
+#: sequences of 64 tokens take 27 to 47 us there against 60 to 79 us on the kernel for few tokens, one of 2,048 takes 102 to
+#: 177 us against 400 to 673; below, the launch that forms the coefficients or gates beforehand (5 us) is not earned back.
 SCAN_PROMPT_TOKENS = 64
 
 

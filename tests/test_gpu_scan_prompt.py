@@ -1,5 +1,5 @@
 """The matrix-state recurrences' kernels for many tokens a sequence: against the plain statements, against the kernel
-for few tokens, across the edges of their blocks of 8 and chunks of 16 tokens and of their columns, the state carried."""
+for few tokens, across the edges of their blocks of 16 (and 8) tokens and of their columns, the state carried."""
 
 import pytest
 import torch
