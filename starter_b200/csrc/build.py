@@ -14,6 +14,7 @@ from __future__ import annotations
 import ctypes
 import hashlib
 import os
+import re
 import shutil
 import subprocess
 import sys
@@ -165,12 +166,36 @@ def library_path(name: str) -> str:
     return lib
 
 
+_ENTRY = re.compile(r"^(int|void|long long)\s+(sb_\w+)\s*\(([^)]*)\)\s*\{", re.M)
+_C_TYPES = {"int": ctypes.c_int, "long long": ctypes.c_longlong, "unsigned long long": ctypes.c_ulonglong,
+            "float": ctypes.c_float, "cudaStream_t": ctypes.c_void_p}
+
+
+def declarations(name: str) -> dict:
+    """``{entry point: (result type, argument types)}`` of ``name.cu`` as ctypes, read from its source."""
+    out = {}
+    for fname in [name + ".cu"] + _included_sources(name):
+        with open(os.path.join(HERE, fname), "r", encoding="utf-8") as handle:
+            for result, entry, params in _ENTRY.findall(handle.read()):
+                types = []
+                for param in (" ".join(p.split()) for p in params.split(",")):
+                    if param in ("", "void"):
+                        continue
+                    types.append(ctypes.c_void_p if "*" in param else _C_TYPES[param.rsplit(" ", 1)[0]])
+                out[entry] = (None if result == "void" else _C_TYPES[result], types)
+    return out
+
+
 def load(name: str) -> ctypes.CDLL:
-    """The loaded library of ``name.cu`` (built on first use)."""
+    """The loaded library of ``name.cu`` (built on first use).  Its entry points know their argument types, so callers
+    pass addresses as plain integers (a ctypes object for each cost more than the launch itself)."""
     with _lock:
         lib = _loaded.get(name)
         if lib is None:
             lib = ctypes.CDLL(library_path(name))
+            for entry, (result, types) in declarations(name).items():
+                function = getattr(lib, entry)
+                function.restype, function.argtypes = result, types
             _loaded[name] = lib
         return lib
 

@@ -39,18 +39,19 @@ class KernelError(RuntimeError):
     pass
 
 
-_checked = set()
+_libs = {}
 
 
 def _lib(name: str):
     """The kernel library of ``name.cu``; refuses one compiled for another cache page size."""
-    lib = build.load(name)
-    if name not in _checked:
+    lib = _libs.get(name)
+    if lib is None:
+        lib = build.load(name)
         compiled = lib.sb_page_tokens()
         if compiled != PAGE_TOKENS:
             raise KernelError(f"libsb_{name} was compiled for cache pages of {compiled} tokens, the cache "
                               f"uses pages of {PAGE_TOKENS}")
-        _checked.add(name)
+        _libs[name] = lib
     return lib
 
 
@@ -61,7 +62,7 @@ def _code(dtype) -> int:
 
 
 def _ptr(t):
-    return ctypes.c_void_p(t.data_ptr()) if t is not None else ctypes.c_void_p(0)
+    return t.data_ptr() if t is not None else None
 
 
 try:                                   # the raw handle of the current stream without building objects
@@ -72,10 +73,10 @@ except AttributeError:                 # pragma: no cover - older or newer torch
 
 
 def _stream():
-    """The current CUDA stream as a ``void*`` (called once per launch: it has to be cheap)."""
+    """The current CUDA stream's address (called once per launch: it has to be cheap)."""
     if _raw_stream is not None:
-        return ctypes.c_void_p(_raw_stream(_current_device()))
-    return ctypes.c_void_p(torch.cuda.current_stream().cuda_stream)
+        return _raw_stream(_current_device())
+    return torch.cuda.current_stream().cuda_stream
 
 
 def _need(t, name, dtype=None, ndim=None):
@@ -140,7 +141,7 @@ def embedding(tokens, table, status=None, fence=False):
     kernels of the step read, before their own dependent-launch wait, what earlier steps wrote."""
     _need(tokens, "tokens", torch.int32, 1)
     _need(table, "table", None, 2)
-    out = torch.empty((tokens.shape[0], table.shape[1]), dtype=table.dtype, device=table.device)
+    out = table.new_empty((tokens.shape[0], table.shape[1]))
     rc = _lib("elementwise").sb_embedding(
         _code(table.dtype), _ptr(tokens), _ptr(table), _ptr(out), tokens.shape[0], table.shape[1],
         table.shape[0], _ptr(status), int(fence), _stream())
@@ -169,7 +170,7 @@ def rmsnorm(x, gain, eps, delta=None, rows=None, out=None):
         _need(rows, "rows", torch.int32, 1)
         n_rows = rows.shape[0]
     if out is None:
-        out = torch.empty((n_rows, hidden), dtype=x.dtype, device=x.device)
+        out = x.new_empty((n_rows, hidden))
     rc = _lib("elementwise").sb_rmsnorm(
         _code(x.dtype), _gain_code(x, gain), _ptr(x), _ptr(delta), _ptr(gain), _ptr(out), _ptr(rows),
         n_rows, hidden, ctypes.c_float(eps), _stream())
@@ -203,7 +204,7 @@ def swiglu(gate_up, activation="silu"):
     if gate_up.shape[1] % 2:
         raise KernelError(f"gate_up has an odd width {gate_up.shape[1]}")
     inner = gate_up.shape[1] // 2
-    out = torch.empty((gate_up.shape[0], inner), dtype=gate_up.dtype, device=gate_up.device)
+    out = gate_up.new_empty((gate_up.shape[0], inner))
     rc = _lib("elementwise").sb_swiglu(
         _code(gate_up.dtype), _ptr(gate_up), _ptr(out), gate_up.shape[0], inner, gate_code(activation),
         _stream())
@@ -244,14 +245,14 @@ def linear(x, weight, out_float=False, gated=False, status=None, add_to=None):
         out_dtype = torch.float32 if (out_float or dt == 0) else x.dtype
         if gated and out_float and dt == 1:
             raise KernelError("a gated product cannot return float32 from bfloat16")
-        y = torch.empty((rows, n_out), dtype=out_dtype, device=x.device)
+        y = x.new_empty((rows, n_out), dtype=out_dtype)
         rc = _lib("linear_small").sb_linear_small(
             dt, int(out_float), int(gated), _ptr(x), _ptr(weight), _ptr(y), rows, n_out, k_dim,
             _stream())
         _check(rc, "linear_small")
         return y
     if dt == 0:
-        y = torch.empty((rows, n_total), dtype=torch.float32, device=x.device)
+        y = x.new_empty((rows, n_total), dtype=torch.float32)
         rc = _lib("sgemm").sb_sgemm_nt(_ptr(x), _ptr(weight), _ptr(y), rows, n_total, k_dim,
                                              _stream())
         _check(rc, "sgemm")
@@ -375,7 +376,7 @@ def linear_tensor_core(x, weight, out_float=False, gated=False, bm=None, splits=
     splits = whole_splits(-(-k_dim // 64), splits or plan[1])
     stages = stages or max(plan[2], -(-bm * 512 // (16384 + bm * 128)))
     stages = min(stages, (226 * 1024) // (16384 + bm * 128))     # a tile height other than the plan's
-    out = torch.empty((rows, n_out), dtype=torch.float32 if out_float else torch.bfloat16, device=x.device)
+    out = x.new_empty((rows, n_out), dtype=torch.float32 if out_float else torch.bfloat16)
     if withhold is not None:
         rc = _lib("gemm_tcgen05").sb_gemm_tcgen05_withheld(
             _ptr(x), _ptr(weight), _ptr(out), rows, n_out, k_dim, bm, splits, stages, int(gated),
@@ -417,7 +418,7 @@ def linear_prompt(x, weight, gated=False, bn=0, pairs=0, status=None, withhold=N
                               f"{'gated ' if gated else ''}product of shape {(rows, n_out)}")
         out = residual
     else:
-        out = torch.empty((rows, n_out), dtype=torch.bfloat16, device=x.device)
+        out = x.new_empty((rows, n_out), dtype=torch.bfloat16)
     lib = _lib("gemm_prompt_tcgen05")
     if withhold is not None:
         rc = lib.sb_gemm_prompt_withheld(_ptr(x), _ptr(weight), _ptr(out), rows, n_out, k_dim, int(bn), int(pairs),
@@ -487,7 +488,7 @@ def qk_norm_rope_store(qkv, heads, kv_heads, head_dim, q_gain, k_gain, eps, cos_
             if tuple(store.shape[1:]) != (kv_heads, PAGE_TOKENS, head_dim):
                 raise KernelError(f"cache pages have shape {tuple(store.shape)}, expected "
                                   f"[pages, {kv_heads}, {PAGE_TOKENS}, {head_dim}]")
-    q_out = torch.empty((n_tokens, heads * head_dim), dtype=qkv.dtype, device=qkv.device)
+    q_out = qkv.new_empty((n_tokens, heads * head_dim))
     rc = _lib("rope_cache").sb_qk_norm_rope_store(
         _code(qkv.dtype), gain_code, _ptr(qkv), _ptr(q_out), _ptr(q_gain), _ptr(k_gain),
         _ptr(cos_table), _ptr(sin_table), _ptr(tok_pos), _ptr(tok_slot), _ptr(block_table),
@@ -691,12 +692,12 @@ def attention_decode_qkv(qkv, k_store, v_store, block_table, row_slot, row_kv_le
             raise KernelError("rotary tables must be [positions, head_dim / 2]")
     if n_splits is None:
         n_splits = decode_splits(rows, kv_heads, heads // kv_heads, 16, kv_hint)
-    out = torch.empty((rows, heads * head_dim), dtype=qkv.dtype, device=qkv.device)
+    out = qkv.new_empty((rows, heads * head_dim))
     part_acc = part_ml = None
     in_cluster = 1 < n_splits <= DECODE_CLUSTER_SPLITS
     if n_splits > 1 and not in_cluster:
-        part_acc = torch.empty((rows * heads * n_splits * head_dim,), dtype=torch.float32, device=qkv.device)
-        part_ml = torch.empty((rows * heads * n_splits * 2,), dtype=torch.float32, device=qkv.device)
+        part_acc = qkv.new_empty((rows * heads * n_splits * head_dim,), dtype=torch.float32)
+        part_ml = qkv.new_empty((rows * heads * n_splits * 2,), dtype=torch.float32)
     rc = _lib("attention_decode_mma").sb_attention_decode_mma_fused(
         _ptr(qkv), qkv.shape[1], _ptr(out), _ptr(k_store), _ptr(v_store), _ptr(block_table),
         block_table.shape[1], _ptr(row_slot), _ptr(row_kv_len), rows, heads, kv_heads, head_dim,
@@ -742,8 +743,8 @@ def attention_decode(q, k_store, v_store, block_table, row_slot, row_kv_len, hea
     # merge through distributed shared memory; more go through scratch and a merge kernel
     in_cluster = tensor_cores and 1 < n_splits <= DECODE_CLUSTER_SPLITS
     if n_splits > 1 and not in_cluster:
-        part_acc = torch.empty((rows * heads * n_splits * head_dim,), dtype=torch.float32, device=q.device)
-        part_ml = torch.empty((rows * heads * n_splits * 2,), dtype=torch.float32, device=q.device)
+        part_acc = q.new_empty((rows * heads * n_splits * head_dim,), dtype=torch.float32)
+        part_ml = q.new_empty((rows * heads * n_splits * 2,), dtype=torch.float32)
     if tensor_cores:
         rc = _lib("attention_decode_mma").sb_attention_decode_mma(
             _ptr(q), _ptr(out), _ptr(k_store), _ptr(v_store), _ptr(block_table), block_table.shape[1],
@@ -778,7 +779,7 @@ def embedding_streams(tokens, table, streams: int, status=None, fence=False):
     residual streams of a model with hyper-connections at their start.  ``fence`` as in ``embedding``."""
     _need(tokens, "tokens", torch.int32, 1)
     _need(table, "table", None, 2)
-    out = torch.empty((tokens.shape[0], streams, table.shape[1]), dtype=torch.float32, device=table.device)
+    out = table.new_empty((tokens.shape[0], streams, table.shape[1]), dtype=torch.float32)
     rc = _lib("streams").sb_embed_streams(
         _code(table.dtype), _ptr(tokens), _ptr(table), _ptr(out), tokens.shape[0], table.shape[1],
         table.shape[0], int(streams), _ptr(status), int(fence), _stream())
@@ -830,7 +831,7 @@ def hyper_step(streams, dtype, pending=None, read=None, norm=None, rows=None):
     if rows is not None:
         _need(rows, "rows", torch.int32, 1)
         n_rows = rows.shape[0]
-    normed = torch.empty((n_rows, hidden), dtype=dtype, device=streams.device)
+    normed = streams.new_empty((n_rows, hidden), dtype=dtype)
     rc = _lib("streams").sb_hyper_step(
         _code(dtype), n_streams, _ptr(streams), _ptr(y), _ptr(bias), _ptr(scale), _ptr(mix), _ptr(out), _ptr(read),
         kind, _ptr(alpha), _ptr(weight), _ptr(shift), ctypes.c_float(eps), _ptr(normed), _ptr(rows), n_rows,
@@ -858,7 +859,7 @@ def dynamic_tanh(x, alpha, weight, bias, delta=None, rows=None):
     if rows is not None:
         _need(rows, "rows", torch.int32, 1)
         n_rows = rows.shape[0]
-    out = torch.empty((n_rows, hidden), dtype=x.dtype, device=x.device)
+    out = x.new_empty((n_rows, hidden))
     rc = _lib("streams").sb_dyt(_code(x.dtype), _ptr(x), _ptr(delta), _ptr(alpha), _ptr(weight), _ptr(bias),
                                 _ptr(out), _ptr(rows), n_rows, hidden, _stream())
     _check(rc, "dynamic_tanh")
@@ -904,7 +905,7 @@ def diff_attention_prefill(q, gate, k_store, v_store, block_table, seq_slot, seq
              and (gate is None or (gate_stride % 8 == 0 and gate.data_ptr() % 16 == 0)))
     if kernel is None:
         kernel = "tcgen05" if tc_ok and (max_q_len is None or max_q_len >= 128) else "mma"
-    out = torch.empty((q.shape[0], heads * v_dim), dtype=q.dtype, device=q.device)
+    out = q.new_empty((q.shape[0], heads * v_dim))
     if kernel == "tcgen05":
         if not tc_ok:
             raise KernelError(f"the tcgen05 differential attention takes dim 64 and v_dim 64 or 128 in bfloat16 with "
@@ -961,7 +962,7 @@ def diff_prepare(proj, bias, heads, kv_heads, dim, v_dim, gate_width, temperatur
             raise KernelError(f"cache pages have shapes {tuple(k_store.shape)} and {tuple(v_store.shape)}, expected "
                               f"[pages, {kv_heads}, {PAGE_TOKENS}, {2 * dim}] and [pages, {kv_heads}, {PAGE_TOKENS}, {v_dim}]")
     coef, every = temperature if temperature is not None else (0.0, 0)
-    q_out = torch.empty((n_tokens, q_w), dtype=proj.dtype, device=proj.device)
+    q_out = proj.new_empty((n_tokens, q_w))
     rc = _lib("attention_diff").sb_diff_prepare(
         _code(proj.dtype), _ptr(proj), proj.shape[1], _ptr(bias), _ptr(q_out), _ptr(tok_pos), _ptr(tok_slot),
         _ptr(block_table), block_table.shape[1], _ptr(k_store if write_cache else None),
@@ -1006,7 +1007,7 @@ def diff_attention(q, gate, k_store, v_store, block_table, tok_slot, tok_pos, he
     _need(tok_pos, "tok_pos", torch.int32, 1)
     if warps is None:
         warps = 1 if kv_hint <= 32 else 2 if kv_hint <= 128 else 4 if kv_hint <= 512 else 8
-    out = torch.empty((q.shape[0], heads * v_dim), dtype=q.dtype, device=q.device)
+    out = q.new_empty((q.shape[0], heads * v_dim))
     rc = _lib("attention_diff").sb_diff_attention(
         _code(q.dtype), _ptr(q), _ptr(gate), int(gate_stride), _ptr(out), _ptr(k_store), _ptr(v_store),
         _ptr(block_table), block_table.shape[1], _ptr(tok_slot), _ptr(tok_pos), q.shape[0], heads, kv_heads,
@@ -1051,10 +1052,10 @@ def diff_attention_decode(q, gate, k_store, v_store, block_table, row_slot, row_
         through_scratch = max(1, min(pages // 7, resident, 64))
         if through_scratch >= 3 * n_splits:
             n_splits = through_scratch
-    out = torch.empty((rows, heads * v_dim), dtype=q.dtype, device=q.device)
+    out = q.new_empty((rows, heads * v_dim))
     part = None
     if not cluster or n_splits > DIFF_CLUSTER_PARTS:
-        part = torch.empty((rows * heads * n_splits * 2 * (v_dim + 2),), dtype=torch.float32, device=q.device)
+        part = q.new_empty((rows * heads * n_splits * 2 * (v_dim + 2),), dtype=torch.float32)
     rc = _lib("attention_diff_prefill").sb_diff_decode(
         _ptr(q), _ptr(gate), int(gate_stride), _ptr(out), _ptr(k_store), _ptr(v_store), _ptr(block_table),
         block_table.shape[1], _ptr(row_slot), _ptr(row_kv_len), rows, heads, kv_heads, dim, v_dim,
@@ -1109,11 +1110,11 @@ def sample(logits, temperature=None, request_key=None, position=None, status=Non
         _need(request_key, "request_key", torch.int32, 1)
         _need(position, "position", torch.int32, 1)
     if out is None:
-        out = torch.empty((rows,), dtype=torch.int32, device=logits.device)
+        out = logits.new_empty((rows,), dtype=torch.int32)
     lib = _lib("sampling")
     chunks = lib.sb_sample_chunks(vocab)
-    cand_v = torch.empty((rows * chunks,), dtype=torch.float32, device=logits.device)
-    cand_i = torch.empty((rows * chunks,), dtype=torch.int32, device=logits.device)
+    cand_v = logits.new_empty((rows * chunks,), dtype=torch.float32)
+    cand_i = logits.new_empty((rows * chunks,), dtype=torch.int32)
     rc = lib.sb_sample(
         _ptr(logits), rows, vocab, ctypes.c_longlong(logits.stride(0)), _ptr(temperature),
         _ptr(request_key), _ptr(position), _ptr(out), _ptr(status),
@@ -1317,7 +1318,7 @@ def embedding32(tokens, table, scale=1.0, status=None, fence=False, out=None):
     _need(tokens, "tokens", torch.int32, 1)
     _need(table, "table", None, 2)
     if out is None:
-        out = torch.empty((tokens.shape[0], table.shape[1]), dtype=torch.float32, device=table.device)
+        out = table.new_empty((tokens.shape[0], table.shape[1]), dtype=torch.float32)
     else:
         _f32(out, "out", (tokens.shape[0], table.shape[1]))
     rc = _lib("residual32").sb_embed32(
@@ -1360,7 +1361,7 @@ def residual_norm(x, dtype, eps, pending=None, next_gain=None, rows=None):
     out = None
     if next_gain is not None:
         _f32(next_gain, "next gain", (hidden,))
-        out = torch.empty((n_rows, hidden), dtype=dtype, device=x.device)
+        out = x.new_empty((n_rows, hidden), dtype=dtype)
     rc = _lib("residual32").sb_residual_norm(
         _code(dtype), _ptr(x), _ptr(y), _ptr(y2), _ptr(bias), _ptr(post), _ptr(next_gain), _ptr(out), _ptr(rows), n_rows,
         hidden, ctypes.c_float(post_eps), ctypes.c_float(eps), _stream())
@@ -1386,7 +1387,7 @@ def residual_join(x, pending, tokens, table, scale=1.0):
             _need(t, "y", table.dtype, 2)
             if tuple(t.shape) != (n_tokens, hidden):
                 raise KernelError(f"y {tuple(t.shape)} does not match the residual stream {tuple(x.shape)}")
-    out = torch.empty((n_tokens, 2 * hidden), dtype=table.dtype, device=x.device)
+    out = x.new_empty((n_tokens, 2 * hidden), dtype=table.dtype)
     rc = _lib("residual32").sb_residual_join(
         _code(table.dtype), _ptr(x), _ptr(y), _ptr(y2), _ptr(tokens), _ptr(table), _ptr(out), n_tokens, hidden,
         table.shape[0], ctypes.c_float(scale), _stream())
@@ -1432,7 +1433,7 @@ def token_shift(h, state, mu, tok_slot):
     n_tokens, width = h.shape
     if mu.shape[1] != width or state.shape[1] < width:
         raise KernelError(f"mu {tuple(mu.shape)} / state {tuple(state.shape)} do not fit rows of {width}")
-    out = torch.empty((mu.shape[0], n_tokens, width), dtype=h.dtype, device=h.device)
+    out = h.new_empty((mu.shape[0], n_tokens, width))
     rc = _lib("wkv").sb_token_shift(_code(h.dtype), _ptr(h), _ptr(state), ctypes.c_longlong(state.shape[1]), _ptr(mu),
                                     _ptr(out), _ptr(tok_slot), n_tokens, width, mu.shape[0], _stream())
     _check(rc, "token_shift")
@@ -1472,7 +1473,7 @@ def wkv_scan(r, k, v, decay, u, g, gain, state, h, seq_slot, seq_q_start, seq_q_
         _need(t, name, torch.int32, 1)
     out = torch.empty_like(r)
     # many tokens of few sequences: scratch with which several blocks may share a head
-    o32 = torch.empty((n_tokens, hd), dtype=torch.float32, device=r.device) if n_tokens >= 4 * seq_slot.shape[0] else None
+    o32 = r.new_empty((n_tokens, hd), dtype=torch.float32) if n_tokens >= 4 * seq_slot.shape[0] else None
     rc = _lib("wkv").sb_wkv_scan(
         _code(r.dtype), _ptr(r), _ptr(k), _ptr(v), _ptr(decay), _ptr(u), _ptr(g), _ptr(gain),
         _ptr(state), ctypes.c_longlong(state.shape[1]), width, _ptr(h), width, _ptr(out), _ptr(seq_slot),
@@ -1532,7 +1533,7 @@ def latent_prepare(proj, q_gain, kv_gain, eps, cos_table, sin_table, tok_pos, to
         _need(store, "cache pages", proj.dtype, 4)
         if tuple(store.shape[1:]) != (1, PAGE_TOKENS, rank + rot):
             raise KernelError(f"cache pages have shape {tuple(store.shape)}, expected [pages, 1, {PAGE_TOKENS}, {rank + rot}]")
-    cq = torch.empty((n_tokens, q_rank), dtype=proj.dtype, device=proj.device)
+    cq = proj.new_empty((n_tokens, q_rank))
     rc = _lib("attention_latent").sb_latent_prepare(
         _code(proj.dtype), _ptr(proj), proj.shape[1], _ptr(q_gain), _ptr(kv_gain if write_cache else None),
         ctypes.c_float(eps), _ptr(cos_table), _ptr(sin_table), cos_table.shape[1], _ptr(tok_pos), _ptr(tok_slot),
@@ -1577,7 +1578,7 @@ def latent_attention(qa, store, block_table, tok_slot, tok_pos, heads, rank, rot
     _need(block_table, "block_table", torch.int32, 2)
     _need(tok_slot, "tok_slot", torch.int32, 1)
     _need(tok_pos, "tok_pos", torch.int32, 1)
-    out = torch.empty((n_tokens, heads, rank), dtype=qa.dtype, device=qa.device)
+    out = qa.new_empty((n_tokens, heads, rank))
     rc = _lib("attention_latent").sb_latent_attention(
         _code(qa.dtype), _ptr(qa), _ptr(out), _ptr(store), _ptr(block_table), block_table.shape[1], _ptr(tok_slot),
         _ptr(tok_pos), n_tokens, heads, rank, rot, ctypes.c_float(scale), int(window or 0), _latent_sink(sink, heads), _stream())
@@ -1612,12 +1613,12 @@ def latent_attention_tc(qa, store, block_table, seq_slot, seq_q_start, seq_q_len
     for name, t in (("seq_slot", seq_slot), ("seq_q_start", seq_q_start), ("seq_q_len", seq_q_len),
                     ("seq_kv_len", seq_kv_len), ("tile_seq", tile_seq), ("tile_first", tile_first)):
         _need(t, name, torch.int32, 1)
-    out = torch.empty((n_tokens, heads, rank), dtype=qa.dtype, device=qa.device)
+    out = qa.new_empty((n_tokens, heads, rank))
     part_acc = part_ml = None
     n_splits = max(1, int(n_splits))
     if n_splits > 1:
-        part_acc = torch.empty((n_splits, n_tokens * heads, rank), dtype=torch.float32, device=qa.device)
-        part_ml = torch.empty((n_splits, n_tokens * heads, 2), dtype=torch.float32, device=qa.device)
+        part_acc = qa.new_empty((n_splits, n_tokens * heads, rank), dtype=torch.float32)
+        part_ml = qa.new_empty((n_splits, n_tokens * heads, 2), dtype=torch.float32)
     rc = _lib("attention_latent").sb_latent_attention_tc(
         _ptr(qa), _ptr(out), _ptr(part_acc), _ptr(part_ml), _ptr(store), _ptr(block_table), block_table.shape[1],
         _ptr(seq_slot), _ptr(seq_q_start), _ptr(seq_q_len), _ptr(seq_kv_len), _ptr(tile_seq), _ptr(tile_first),
@@ -1694,7 +1695,7 @@ def latent_attention_prompt(q, ukv, store, block_table, ctx, heads, dim, vdim, r
         _need(t, name, torch.int32, 1)
     each = _latent_prompt_rows(ctx, window)
     rows = int(each.sum())
-    gathered = torch.empty((rows * (rank + rot),), dtype=q.dtype, device=q.device)
+    gathered = q.new_empty((rows * (rank + rot),))
     c, shared = gathered[:rows * rank].view(rows, rank), gathered[rows * rank:].view(rows, rot)
     lib = _lib("attention_latent_prompt")
     rc = lib.sb_latent_gather(_ptr(store), _ptr(block_table), block_table.shape[1], _ptr(ctx.seq_slot), _ptr(ctx.seq_q_len),
@@ -1702,7 +1703,7 @@ def latent_attention_prompt(q, ukv, store, block_table, ctx, heads, dim, vdim, r
                               _stream())
     _check(rc, "latent_gather")
     kv = linear(c, ukv, status=ctx.status)
-    out = torch.empty((n_tokens, heads * vdim), dtype=q.dtype, device=q.device)
+    out = q.new_empty((n_tokens, heads * vdim))
     rc = lib.sb_latent_prompt(
         _ptr(q), _ptr(kv), _ptr(shared), _ptr(out), _ptr(ctx.seq_q_start), _ptr(ctx.seq_q_len), _ptr(ctx.seq_kv_len),
         _ptr(ctx.block_seq), _ptr(ctx.block_first), ctx.block_seq.shape[0], n_tokens, rows, heads, dim, vdim,
@@ -1747,8 +1748,8 @@ def moe_route(h, router, router_bias, top, scoring="softmax_top", weight_scale=1
     _f32(router, "router", (experts, h.shape[1]))
     if router_bias is not None:
         _f32(router_bias, "router bias", (experts,))
-    ids = torch.empty((h.shape[0], top), dtype=torch.int32, device=h.device)
-    weights = torch.empty((h.shape[0], top), dtype=torch.float32, device=h.device)
+    ids = h.new_empty((h.shape[0], top), dtype=torch.int32)
+    weights = h.new_empty((h.shape[0], top), dtype=torch.float32)
     rc = _lib("moe").sb_moe_route(_code(h.dtype), _ptr(h), _ptr(router), _ptr(router_bias), _ptr(ids), _ptr(weights),
                                   h.shape[0], h.shape[1], experts, top, MOE_SCORINGS[scoring],
                                   ctypes.c_float(weight_scale), _stream())
@@ -1771,9 +1772,9 @@ def moe_route_all(h, router, correction, top, groups=1, keep=1, weight_scale=1.0
     _f32(router, "router", (router.shape[0], h.shape[1]))
     if correction is not None:
         _f32(correction, "correction", (outputs,))
-    ids = torch.empty((h.shape[0], top), dtype=torch.int32, device=h.device)
-    weights = torch.empty((h.shape[0], top), dtype=torch.float32, device=h.device)
-    gate = torch.empty((h.shape[0],), dtype=torch.float32, device=h.device) if shared_gate else None
+    ids = h.new_empty((h.shape[0], top), dtype=torch.int32)
+    weights = h.new_empty((h.shape[0], top), dtype=torch.float32)
+    gate = h.new_empty((h.shape[0],), dtype=torch.float32) if shared_gate else None
     rc = _lib("moe").sb_moe_route_all(_code(h.dtype), _ptr(h), _ptr(router), _ptr(correction), _ptr(ids), _ptr(weights),
                                       _ptr(gate), h.shape[0], h.shape[1], outputs, top, groups, keep,
                                       ctypes.c_float(weight_scale), _stream())
@@ -1837,16 +1838,16 @@ def moe_experts(h, ids, weights, gate_up, down, limit=0.0, expert="gated_clamped
         bm = 8 if tile_rows == 4 else int(tile_rows)
     max_tiles = -(-n_pairs // bm) + min(experts, n_pairs)
     capacity = max_tiles * bm
-    meta = torch.empty((capacity + max_tiles + 1,), dtype=torch.int32, device=h.device)
+    meta = h.new_empty((capacity + max_tiles + 1,), dtype=torch.int32)
     sorted_pairs, tile_expert, n_tiles = meta[:capacity], meta[capacity:capacity + max_tiles], meta[capacity + max_tiles:]
     rc = lib.sb_moe_align(_ptr(ids), n_pairs, experts, _ptr(sorted_pairs), capacity, _ptr(tile_expert), _ptr(n_tiles),
                           bm, _stream())
     _check(rc, "moe_align")
-    act = torch.empty((capacity, inner), dtype=h.dtype, device=h.device)
-    per_pair = torch.empty((n_pairs, width), dtype=h.dtype, device=h.device)
+    act = h.new_empty((capacity, inner))
+    per_pair = h.new_empty((n_pairs, width))
     if bm == 256:
         grouped = _lib("gemm_prompt_tcgen05").sb_gemm_prompt_grouped
-        gathered = torch.empty((capacity, width), dtype=h.dtype, device=h.device)
+        gathered = h.new_empty((capacity, width))
         rc = lib.sb_moe_gather(_ptr(h), _ptr(sorted_pairs), _ptr(n_tiles), bm, top, _ptr(gathered), capacity, width,
                                _ptr(in_scale), _stream())
         _check(rc, "moe_gather")
@@ -1922,7 +1923,7 @@ def depth_step(base, dtype, pending=None, mult=1.0, history=None, mix=None, dst=
             raise KernelError(f"no norm {name!r} here (known: {', '.join(DEPTH_NORMS)})")
         kind = DEPTH_NORMS[name]
         _f32(gain, "gain", (hidden,))
-        out = torch.empty((n_rows, hidden), dtype=dtype, device=base.device)
+        out = base.new_empty((n_rows, hidden), dtype=dtype)
     rc = _lib("depth").sb_depth_step(
         _code(dtype), _ptr(base), _ptr(pending), ctypes.c_float(mult), _ptr(history if mix is not None else None),
         ctypes.c_longlong(n_tokens * hidden), _ptr(mix), levels, _ptr(dst), _ptr(gain), _ptr(out), _ptr(rows), n_rows,
@@ -1946,7 +1947,7 @@ def gated_clamped(gate_up, limit):
     if gate_up.shape[1] % 2:
         raise KernelError(f"gate_up has an odd width {gate_up.shape[1]}")
     inner = gate_up.shape[1] // 2
-    out = torch.empty((gate_up.shape[0], inner), dtype=gate_up.dtype, device=gate_up.device)
+    out = gate_up.new_empty((gate_up.shape[0], inner))
     rc = _lib("elementwise").sb_gated_clamped(_code(gate_up.dtype), _ptr(gate_up), _ptr(out), gate_up.shape[0], inner,
                                               ctypes.c_float(limit), _stream())
     _check(rc, "gated_clamped")
@@ -1979,7 +1980,7 @@ def sink_prepare(proj, heads, kv_heads, dim, vdim, tok_pos, tok_slot, block_tabl
         if tuple(k_store.shape[1:]) != (kv_heads, PAGE_TOKENS, dim) or tuple(v_store.shape[1:]) != (kv_heads, PAGE_TOKENS, vdim):
             raise KernelError(f"cache pages have shapes {tuple(k_store.shape)} / {tuple(v_store.shape)}, expected "
                               f"[pages, {kv_heads}, {PAGE_TOKENS}, {dim}] / [.., {vdim}]")
-    gate = torch.empty((n_tokens, heads), dtype=torch.float32, device=proj.device) if gated else None
+    gate = proj.new_empty((n_tokens, heads), dtype=torch.float32) if gated else None
     rc = _lib("attention_sink").sb_sink_prepare(
         _code(proj.dtype), _ptr(proj), proj.shape[1], _ptr(tok_pos), _ptr(tok_slot), _ptr(block_table),
         block_table.shape[1], _ptr(k_store if write_cache else None), _ptr(v_store if write_cache else None),
@@ -2117,7 +2118,7 @@ def sink_attention(q, k_store, v_store, block_table, tok_slot, tok_pos, heads, k
     _need(block_table, "block_table", torch.int32, 2)
     _need(tok_slot, "tok_slot", torch.int32, 1)
     _need(tok_pos, "tok_pos", torch.int32, 1)
-    out = torch.empty((q.shape[0], heads * vdim), dtype=q.dtype, device=q.device)
+    out = q.new_empty((q.shape[0], heads * vdim))
     rc = _lib("attention_sink").sb_sink_attention(
         _code(q.dtype), _ptr(q), q.shape[1], _ptr(out), _ptr(k_store), _ptr(v_store), _ptr(block_table),
         block_table.shape[1], _ptr(tok_slot), _ptr(tok_pos), _ptr(r1), _ptr(r2), _ptr(sink), _ptr(gate), q.shape[0],
@@ -2167,12 +2168,12 @@ def sink_attention_tc(q, k_store, v_store, block_table, seq_slot, seq_q_start, s
                     ("seq_kv_len", seq_kv_len), ("tile_seq", tile_seq), ("tile_first", tile_first)):
         _need(t, name, torch.int32, 1)
     n_tokens = q.shape[0]
-    out = torch.empty((n_tokens, heads * vdim), dtype=q.dtype, device=q.device)
+    out = q.new_empty((n_tokens, heads * vdim))
     part_acc = part_ml = None
     n_splits = max(1, int(n_splits))
     if n_splits > 1:
-        part_acc = torch.empty((n_splits, n_tokens * heads, vdim), dtype=torch.float32, device=q.device)
-        part_ml = torch.empty((n_splits, n_tokens * heads, 2), dtype=torch.float32, device=q.device)
+        part_acc = q.new_empty((n_splits, n_tokens * heads, vdim), dtype=torch.float32)
+        part_ml = q.new_empty((n_splits, n_tokens * heads, 2), dtype=torch.float32)
     rc = _lib("attention_sink_tc").sb_sink_attention_tc(
         _ptr(q), q.shape[1], _ptr(out), _ptr(part_acc), _ptr(part_ml), _ptr(k_store), _ptr(v_store), _ptr(block_table),
         block_table.shape[1], _ptr(seq_slot), _ptr(seq_q_start), _ptr(seq_q_len), _ptr(seq_kv_len), _ptr(tile_seq),
@@ -2215,7 +2216,7 @@ def sink_attention_tcgen05(q, k_store, v_store, block_table, seq_slot, seq_q_sta
         for name, t in (("block_seq", blocks[0]), ("block_first", blocks[1])):
             _need(t, name, torch.int32, 1)
     list_seq, list_first = blocks if own_list else (tile_seq, tile_first)
-    out = torch.empty((q.shape[0], heads * vdim), dtype=q.dtype, device=q.device)
+    out = q.new_empty((q.shape[0], heads * vdim))
     rc = _lib("attention_prefill_tc").sb_sink_attention_tcgen05(
         _ptr(q), q.shape[1], _ptr(out), _ptr(k_store), _ptr(v_store), _ptr(block_table), block_table.shape[1],
         _ptr(seq_slot), _ptr(seq_q_start), _ptr(seq_q_len), _ptr(seq_kv_len), _ptr(list_seq), _ptr(list_first),
@@ -2263,13 +2264,13 @@ def linear_gated_clamped(x, weight, limit, status=None):
     if fused and rows <= TENSOR_CORE_MAX_ROWS:
         bm, splits, stages = gemm_plan(rows, n_out, k_dim, True)
         stages = min(max(stages, -(-bm * 512 // (16384 + bm * 128))), (226 * 1024) // (16384 + bm * 128))
-        out = torch.empty((rows, n_out), dtype=torch.bfloat16, device=x.device)
+        out = x.new_empty((rows, n_out), dtype=torch.bfloat16)
         rc = _lib("gemm_tcgen05").sb_gemm_tcgen05_clamped(_ptr(x), _ptr(weight), _ptr(out), rows, n_out, k_dim, bm, splits,
                                                           stages, ctypes.c_float(limit), _ptr(status), _stream())
         _check(rc, "gemm_tcgen05 (clamped gate)")
         return out
     if fused and rows >= PROMPT_MIN_ROWS:
-        out = torch.empty((rows, n_out), dtype=torch.bfloat16, device=x.device)
+        out = x.new_empty((rows, n_out), dtype=torch.bfloat16)
         rc = _lib("gemm_prompt_tcgen05").sb_gemm_prompt_clamped(_ptr(x), _ptr(weight), _ptr(out), rows, n_out, k_dim, 0, 0,
                                                                 ctypes.c_float(limit), _ptr(status), _stream())
         _check(rc, "gemm_prompt_tcgen05 (clamped gate)")
@@ -2281,7 +2282,7 @@ def linear_gated_clamped(x, weight, limit, status=None):
 
 def _at(t, offset: int):
     """The address of element ``offset`` of a contiguous tensor."""
-    return ctypes.c_void_p(t.data_ptr() + offset * t.element_size())
+    return t.data_ptr() + offset * t.element_size()
 
 
 def _seq_arrays(seq_slot, seq_q_start, seq_q_len):
@@ -2322,7 +2323,7 @@ def short_conv(x, col, channels, taps, bias, in_bias, state, state_at, seq_slot,
     if activation not in (None, "silu"):
         raise KernelError(f"the short convolution applies silu or nothing, not {activation!r}")
     n_seqs = _seq_arrays(seq_slot, seq_q_start, seq_q_len)
-    y = torch.empty((x.shape[0], channels), dtype=x.dtype, device=x.device)
+    y = x.new_empty((x.shape[0], channels))
     rc = _lib("short_conv").sb_short_conv(
         _code(x.dtype), _at(x, col), x.shape[1], _ptr(taps), _ptr(bias), _ptr(in_bias), _ptr(y), channels,
         _at(state, state_at) if state is not None else _ptr(None), ctypes.c_longlong(slot_floats), _ptr(seq_slot),
@@ -2405,7 +2406,7 @@ def state_scan(mode, q, k, v, a_raw, b_raw, A_log, dt_bias, skip, state, state_a
     for name, pair, width in (("q", q, groups * n_state), ("k", k, groups * n_state), ("v", v, heads * v_dim),
                               ("a_raw", a_raw, heads), ("b_raw", b_raw, heads)):
         if pair is None:
-            args += [ctypes.c_void_p(0), 0]
+            args += [None, 0]
             continue
         t, col = pair
         _need(t, name, dtype, 2)
@@ -2426,12 +2427,12 @@ def state_scan(mode, q, k, v, a_raw, b_raw, A_log, dt_bias, skip, state, state_a
     if state_at < 0 or state_at + heads * n_state * v_dim > state.shape[1]:
         raise KernelError(f"a slot's {state.shape[1]} floats do not hold {heads} states of {n_state} x {v_dim} from {state_at}")
     n_seqs = _seq_arrays(seq_slot, seq_q_start, seq_q_len)
-    out = torch.empty((n_tokens, heads * v_dim), dtype=torch.float32, device=state.device)
+    out = state.new_empty((n_tokens, heads * v_dim), dtype=torch.float32)
     if dtype == torch.bfloat16 and n_tokens >= SCAN_PROMPT_TOKENS * n_seqs and 64 < n_state <= 128:
         lib = _lib("state_scan_prompt")
         floats = lib.sb_scan_prompt_floats(1, SCAN_MODES[mode], *args[:6], _ptr(decay), heads, groups, n_state, v_dim)
         if floats >= 0:
-            scratch = torch.empty((n_tokens, floats), dtype=torch.float32, device=state.device) if floats else None
+            scratch = state.new_empty((n_tokens, floats), dtype=torch.float32) if floats else None
             rc = lib.sb_state_scan_prompt(
                 SCAN_MODES[mode], *args, _ptr(A_log), _ptr(dt_bias), _ptr(skip), _ptr(decay), _at(state, state_at),
                 ctypes.c_longlong(state.shape[1]), _ptr(out), _ptr(seq_slot), _ptr(seq_q_start), _ptr(seq_q_len), n_tokens,
@@ -2461,7 +2462,7 @@ def low_rank_decay(u, col, a2, bias, tau):
         raise KernelError(f"{rank} columns from {col} of {tuple(u.shape)} are not there")
     if not tau > 0.0:
         raise KernelError(f"tau={tau} must be positive")
-    out = torch.empty((u.shape[0], channels), dtype=torch.float32, device=u.device)
+    out = u.new_empty((u.shape[0], channels), dtype=torch.float32)
     rc = _lib("state_scan").sb_low_rank_decay(_code(u.dtype), _at(u, col), u.shape[1], _ptr(a2), _ptr(bias), _ptr(out),
                                               u.shape[0], channels, rank, ctypes.c_float(1.0 / tau), _stream())
     if rc == -2:
@@ -2486,7 +2487,7 @@ def group_norm_gate(o, z, z_col, weight, parts, eps, gate_first, dtype):
             raise KernelError(f"rows of {width} in {parts} parts with a gate from column {z_col} of {tuple(z.shape)} do not fit")
     if weight.shape[0] not in (width, width // parts):
         raise KernelError(f"a gain of {weight.shape[0]} entries fits neither the row ({width}) nor a part ({width // parts})")
-    y = torch.empty((n_tokens, width), dtype=dtype, device=o.device)
+    y = o.new_empty((n_tokens, width), dtype=dtype)
     gate, gate_width, order = (_ptr(None), 0, 2) if z is None else (_at(z, z_col), z.shape[1], 0 if gate_first else 1)
     rc = _lib("state_scan").sb_group_norm_gate(_code(dtype), _ptr(o), gate, gate_width, _ptr(weight),
                                                weight.shape[0], _ptr(y), n_tokens, parts, width // parts,

@@ -94,3 +94,22 @@ def test_decode_graph_length_classes_never_exceed_the_length():
         assert got in HINT_PAGES and got <= pages
         assert all(p > pages for p in HINT_PAGES if p > got)
     assert [hint_pages(t) for t in (1, 65, 130, 3073)] == [1, 2, 3, 48]
+
+
+def test_every_entry_point_the_operations_call_has_declared_arguments():
+    """Addresses travel as plain integers: an entry point whose arguments are not declared would cut them to 32 bits."""
+    import ctypes
+    import inspect
+    import re
+
+    from starter_b200 import ops
+    from starter_b200.csrc import build
+
+    known = {}
+    for name in build.SOURCES:
+        known.update(build.declarations(name))
+    used = set(re.findall(r"\.(sb_\w+)", inspect.getsource(ops))) - {"sb_page_tokens"}
+    assert used and not used - set(known)
+    result, types = known["sb_sgemm_nt"]
+    assert result is ctypes.c_int
+    assert types == [ctypes.c_void_p] * 3 + [ctypes.c_int] * 3 + [ctypes.c_void_p]
