@@ -1,227 +1,392 @@
-// True 32-bit y[m, n] = sum_k x[m, k] * w[n, k] for many rows: FFMA only, no reduced-precision
-// matrix mode.  This is the prompt-sized projection of the float32 path (the bfloat16 path uses
-// tensor cores instead).
+// y[m, n] = sum_k x[m, k] * w[n, k] of float32 matrices for many rows, in full 32-bit precision, on the
+// fifth-generation tensor cores.  This is the prompt-sized projection of the float32 path.
 //
-// A block makes 64 x 128 outputs with 128 threads, 8 x 8 a thread, from k-slices of 16 in two shared-memory
-// buffers (the next slice's 16-byte loads are in flight while one is multiplied).  Bound by the fma pipe: 64 fmas a
-// thread and slice entry for 16 floats from shared memory (512 bytes a warp and 16-byte load, 4 of an SM's cycles
-// whether lanes share addresses or not; with x kept twice in a row, to spare the copies into the packed fma's
-// operands, the loads were the bound: 35.7 TFLOP/s at 4096^3).  Packed fmas (two columns) halve the issue slots.
-// 46.7 TFLOP/s at 4096^3 (128 x 128 tiles, slices of 8 and 4-byte loads before: 24.2); 141 x 2048 x 2048: 47 us
-// (434 before, when 32 blocks walked all of k), 141 x 8192 x 2048: 172 us (436).
-// The k range is cut into parts whose number depends on n_out and k_dim alone.  With few output tiles the parts of a
-// tile are the blocks of one cluster, which leave their sums in their shared memory and add them, part by part; with
-// enough tiles a block walks the parts itself and adds in the same order.  The sum for one (m, n) is therefore
-// the same whatever the other rows of the call are: a chain over k in each part, the parts added in order.
-#include "common.cuh"
+// Every operand is cut into three bfloat16 pieces, a = a0 + a1 + a2 to 24 bits, and a product is
+// a0 b0 + (a0 b1 + a1 b0) + (a1 b1 + a0 b2 + a2 b0); what is left out is below 2^-26 of it.  The tensor cores truncate
+// when they add to an accumulator, so no accumulator lives long: the six products of SG_CHUNK entries of k start a fresh
+// one, the small terms first (their truncations are 2^-8 of the others'), and its sum joins the result by rounded
+// additions in registers.  Against 64 bits the error is below that of a chain of 32-bit fmas (sizes below).
+//
+// A block owns 128 rows of w (the MMA's M) and up to 160 of x (its N; equal tiles in steps of 16, so that 141 rows are
+// one tile of 144).  Eight warps read 64-entry slices of both as floats (the next slice's 16-byte loads in flight
+// while the MMAs of the one before run), cut them and file the pieces in 128-byte swizzled tiles; eight warps empty the
+// two accumulators in turn, two of which issue the MMAs.
+// Events around a launch, L2 flushed, the multiply-add kernel of 64 x 128 tiles that this replaces -> here: 141 x 2048 x 2048
+// 52 -> 29 us, 141 x 8192 x 2048 177 -> 52, 20 x 2048 x 2048 41 -> 20, 4096^3 2,942 -> 1,086 (126 TFLOP/s); nothing
+// measured between 17 x 5 x 4097 and 4096^3 is slower.  Error against 64 bits (rms, of the result's): 2.9e-7 -> 1.0e-7 at k = 2048,
+// 4.1e-7 -> 1.3e-7 at 4096.  By clock64() a slice at 144 rows is about 3,000 cycles where its MMAs alone are 1,730: issuing
+// costs some 90 cycles an MMA, and cutting 2,500 a slice.  Short k is bound by the ends: 5,000 cycles to the first
+// accumulator, 6,000 to add eight parts.
+//
+// The k range is cut into parts whose number depends on n_out and k_dim alone, the blocks of one cluster; they leave
+// their sums in shared memory and each adds its share of the tile, part by part.  So the sum for one (m, n) is the same
+// whatever the other rows of the call are.
+//
+// Infinities, NaN and values next to the largest float do not survive the cut (inf - inf), and pieces of values near the
+// smallest are cut off: a result that is not finite, or is not zero but below 2^-80, is computed again as a chain of fmas.
+#include "tcgen05.cuh"
 
-#define SG_M 64
-#define SG_N 128
-#define SG_K 16
-#define SG_XLD (SG_M + 4)
-#define SG_WLD (SG_N + 4)
+#define SG_W 128                 // rows of w a block
+#define SG_X 160                 // rows of x a block, at most (two slices of both fill the shared memory)
+#define SG_K 64                  // entries of k a slice: 128 bytes of bfloat16, one swizzle atom
+#define SG_CHUNK 32              // entries of k a fresh accumulator sums: half a slice
+#define SG_W_PLANE (SG_W * SG_K * 2)
+#define SG_CUTTERS 8             // warps that read and cut
+#define SG_DRAINERS 8            // warps that empty the accumulators: a lane quarter and every other 16 columns each
+#define SG_THREADS (32 * (SG_CUTTERS + SG_DRAINERS))
 #define SG_MAX_PARTS 8
+#define SG_MAX_STAGES 4
+#define SG_SMEM (224 * 1024)
 
-struct SgemmTiles {
-  float x[2][SG_K][SG_XLD];
-  float w[2][SG_K][SG_WLD];
-  float sum[SG_M][SG_N];           // a part's sums (cluster), or the parts so far (one block)
+struct SgemmArgs {
+  const float* x;
+  const float* w;
+  float* y;
+  int* status;
+  int rows, n_out, k_dim, tile_rows, parts, stages;
 };
 
-__device__ __forceinline__ unsigned long long sg_fma2(unsigned long long a, unsigned long long b, unsigned long long c) {
-  unsigned long long d;
-  asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(d) : "l"(a), "l"(b), "l"(c));
-  return d;
+// 16 columns of this warp's lane quarter, or twice 16 that are 32 apart.
+__device__ __forceinline__ void sg_tmem_load16(uint32_t taddr, float* v) {
+  asm volatile("tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15}, [%16];\n\t"
+               "tcgen05.wait::ld.sync.aligned;"
+               : "=f"(v[0]), "=f"(v[1]), "=f"(v[2]), "=f"(v[3]), "=f"(v[4]), "=f"(v[5]), "=f"(v[6]), "=f"(v[7]), "=f"(v[8]), "=f"(v[9]), "=f"(v[10]), "=f"(v[11]), "=f"(v[12]), "=f"(v[13]), "=f"(v[14]), "=f"(v[15])
+               : "r"(taddr) : "memory");
+}
+__device__ __forceinline__ void sg_tmem_load16x2(uint32_t taddr, float* v) {
+  asm volatile("tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15}, [%32];\n\t"
+               "tcgen05.ld.sync.aligned.32x32b.x16.b32 {%16, %17, %18, %19, %20, %21, %22, %23, %24, %25, %26, %27, %28, %29, %30, %31}, [%33];\n\t"
+               "tcgen05.wait::ld.sync.aligned;"
+               : "=f"(v[0]), "=f"(v[1]), "=f"(v[2]), "=f"(v[3]), "=f"(v[4]), "=f"(v[5]), "=f"(v[6]), "=f"(v[7]), "=f"(v[8]), "=f"(v[9]), "=f"(v[10]), "=f"(v[11]), "=f"(v[12]), "=f"(v[13]), "=f"(v[14]), "=f"(v[15]),
+                 "=f"(v[16]), "=f"(v[17]), "=f"(v[18]), "=f"(v[19]), "=f"(v[20]), "=f"(v[21]), "=f"(v[22]), "=f"(v[23]), "=f"(v[24]), "=f"(v[25]), "=f"(v[26]), "=f"(v[27]), "=f"(v[28]), "=f"(v[29]), "=f"(v[30]), "=f"(v[31])
+               : "r"(taddr), "r"(taddr + 32) : "memory");
 }
 
-__device__ __forceinline__ unsigned long long sg_twice(float v) {
-  unsigned long long d;
-  asm("mov.b64 %0, {%1, %1};" : "=l"(d) : "f"(v));
-  return d;
+// (volatile: the loads stay where they are written, ahead of the wait for a free stage)
+__device__ __forceinline__ float4 sg_load4(const float* at) {
+  float4 v;
+  asm volatile("ld.global.nc.v4.f32 {%0, %1, %2, %3}, [%4];" : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w) : "l"(at));
+  return v;
+}
+
+// Two floats as three pairs of bfloat16.
+__device__ __forceinline__ void sg_cut(float a, float b, uint32_t& hi, uint32_t& mid, uint32_t& low) {
+  const __nv_bfloat162 h = __floats2bfloat162_rn(a, b);
+  hi = *reinterpret_cast<const uint32_t*>(&h);
+  a -= __uint_as_float(hi << 16);
+  b -= __uint_as_float(hi & 0xffff0000u);
+  const __nv_bfloat162 m = __floats2bfloat162_rn(a, b);
+  mid = *reinterpret_cast<const uint32_t*>(&m);
+  a -= __uint_as_float(mid << 16);
+  b -= __uint_as_float(mid & 0xffff0000u);
+  const __nv_bfloat162 l = __floats2bfloat162_rn(a, b);
+  low = *reinterpret_cast<const uint32_t*>(&l);
+}
+
+// (addresses in shared memory are kept as such: through generic ones a store costs several times as much)
+__device__ __forceinline__ void sg_store4(uint32_t at, uint4 v) {
+  asm volatile("st.shared.v4.b32 [%0], {%1, %2, %3, %4};" ::"r"(at), "r"(v.x), "r"(v.y), "r"(v.z), "r"(v.w) : "memory");
+}
+
+__device__ __forceinline__ bool sg_again(float v) {
+  const float a = fabsf(v);
+  return !(a < INFINITY) || (a < 0x1p-80f && a != 0.f);
+}
+
+__device__ __noinline__ float sg_chain(const float* x, const float* w, int k_dim) {
+  float sum = 0.f;
+  for (int k = 0; k < k_dim; ++k) sum = fmaf(x[k], w[k], sum);
+  return sum;
 }
 
 // VEC: rows of x and w may be read in 16-byte pieces.
 template <bool VEC>
-__global__ void __launch_bounds__(128)
-sgemm_nt_kernel(const float* __restrict__ x, const float* __restrict__ w, float* __restrict__ y, int rows, int n_out,
-                int k_dim, int parts, int part_k) {
-  extern __shared__ __align__(16) unsigned char sgemm_smem[];
-  SgemmTiles& sm = *reinterpret_cast<SgemmTiles*>(sgemm_smem);
-  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-  const int tiles_n = (n_out + SG_N - 1) / SG_N;
-  const int n_base = (int)(blockIdx.x % tiles_n) * SG_N, m_base = (int)(blockIdx.x / tiles_n) * SG_M;
-  // a thread's outputs: rows m0 .. m0 + 3 and m0 + 16 .. m0 + 19, columns n0 .. n0 + 3 and n0 + 64 .. n0 + 67
-  const int m0 = 4 * (lane & 3) + 32 * (warp & 1), n0 = 4 * ((lane >> 2) + 8 * (warp >> 1));
-  const bool split = gridDim.z > 1;                  // a part a block, or all parts
-  const int p_begin = split ? blockIdx.z : 0, p_end = split ? blockIdx.z + 1 : parts;
+__global__ void __launch_bounds__(SG_THREADS, 1) sgemm_tcgen05_kernel(const SgemmArgs args) {
+  extern __shared__ uint8_t sgemm_smem[];
+  const uint32_t smem = (smem_u32(sgemm_smem) + 1023) & ~1023u;
+  __shared__ uint64_t full_bar[SG_MAX_STAGES], empty_bar[SG_MAX_STAGES], sum_full[2], sum_empty[2], done_bar;
+  __shared__ uint32_t tmem_holder;
+  __shared__ int abort_flag;
 
-  float4 px[2], pw[4];
-  auto piece = [&](const float* from, int limit, int row, int k, int k_end) {
-    float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
-    if (row < limit) {
-      const float* at = from + (size_t)row * k_dim + k;
-      if (VEC) {
-        if (k < k_end) v = *reinterpret_cast<const float4*>(at);       // (k_end is a multiple of 4 here)
-      } else {
-        if (k < k_end) v.x = at[0];
-        if (k + 1 < k_end) v.y = at[1];
-        if (k + 2 < k_end) v.z = at[2];
-        if (k + 3 < k_end) v.w = at[3];
-      }
-    }
-    return v;
-  };
-  const int lr = tid >> 2, lk = (tid & 3) * 4;       // rows lr + 32 i, entries lk .. lk + 3 of a slice
-  auto fetch = [&](int k0, int k_end) {
-#pragma unroll
-    for (int i = 0; i < 2; ++i) px[i] = piece(x, rows, m_base + lr + 32 * i, k0 + lk, k_end);
-#pragma unroll
-    for (int i = 0; i < 4; ++i) pw[i] = piece(w, n_out, n_base + lr + 32 * i, k0 + lk, k_end);
-  };
-  auto file = [&](int b) {
-#pragma unroll
-    for (int i = 0; i < 2; ++i) {
-      const float v[4] = {px[i].x, px[i].y, px[i].z, px[i].w};
-#pragma unroll
-      for (int j = 0; j < 4; ++j) sm.x[b][lk + j][lr + 32 * i] = v[j];
-    }
-#pragma unroll
-    for (int i = 0; i < 4; ++i) {
-      const float v[4] = {pw[i].x, pw[i].y, pw[i].z, pw[i].w};
-#pragma unroll
-      for (int j = 0; j < 4; ++j) sm.w[b][lk + j][lr + 32 * i] = v[j];
-    }
-  };
+  const int stages = args.stages, cols = args.tile_rows, k_dim = args.k_dim;
+  const int x_plane = cols * SG_K * 2;
+  const int stage_bytes = 3 * (SG_W_PLANE + x_plane);
+  const uint32_t buffer_cols = cols <= 128 ? 128 : 256;
+  const int warp = __shfl_sync(0xffffffffu, threadIdx.x >> 5, 0), lane = threadIdx.x & 31;
+  const int tiles = (args.n_out + SG_W - 1) / SG_W;
+  const int n_base = (int)(blockIdx.x % tiles) * SG_W, m_base = (int)(blockIdx.x / tiles) * cols, part = blockIdx.y;
+  const int kb_total = (k_dim + SG_K - 1) / SG_K;
+  const int kb_part = (kb_total + args.parts - 1) / args.parts;
+  const int kb_begin = min(part * kb_part, kb_total);
+  const int n_kb = min(kb_begin + kb_part, kb_total) - kb_begin;
+  const int rows_here = min(cols, args.rows - m_base);
 
-  for (int p = p_begin; p < p_end; ++p) {
-    const int k_begin = p * part_k, k_end = min(k_dim, k_begin + part_k);
-    unsigned long long acc[8][4];
-#pragma unroll
-    for (int i = 0; i < 8; ++i)
-#pragma unroll
-      for (int j = 0; j < 4; ++j) acc[i][j] = 0ull;
-    fetch(k_begin, k_end);
-    file(0);
-    __syncthreads();
-    int b = 0;
-    for (int k0 = k_begin; k0 < k_end; k0 += SG_K, b ^= 1) {
-      const bool more = k0 + SG_K < k_end;
-      if (more) fetch(k0 + SG_K, k_end);
-#pragma unroll
-      for (int k = 0; k < SG_K; ++k) {
-        unsigned long long a[8], c[4];
-#pragma unroll
-        for (int i = 0; i < 2; ++i) {
-          const float4 v = *reinterpret_cast<const float4*>(&sm.x[b][k][m0 + 16 * i]);
-          a[4 * i] = sg_twice(v.x);
-          a[4 * i + 1] = sg_twice(v.y);
-          a[4 * i + 2] = sg_twice(v.z);
-          a[4 * i + 3] = sg_twice(v.w);
-        }
-        const ulonglong2 w0 = *reinterpret_cast<const ulonglong2*>(&sm.w[b][k][n0]);
-        const ulonglong2 w1 = *reinterpret_cast<const ulonglong2*>(&sm.w[b][k][n0 + 64]);
-        c[0] = w0.x; c[1] = w0.y; c[2] = w1.x; c[3] = w1.y;
-#pragma unroll
-        for (int i = 0; i < 8; ++i)
-#pragma unroll
-          for (int j = 0; j < 4; ++j) acc[i][j] = sg_fma2(a[i], c[j], acc[i][j]);
-      }
-      if (more) file(b ^ 1);
-      __syncthreads();
-    }
-    // the part's sums (a thread's own places): left for the cluster, or added to the parts before
-#pragma unroll
-    for (int i = 0; i < 8; ++i)
-#pragma unroll
-      for (int j = 0; j < 4; ++j) {
-        float2* at = reinterpret_cast<float2*>(&sm.sum[m0 + 16 * (i >> 2) + (i & 3)][n0 + (j >> 1) * 64 + (j & 1) * 2]);
-        float2 v = make_float2(__uint_as_float((unsigned)acc[i][j]), __uint_as_float((unsigned)(acc[i][j] >> 32)));
-        if (p > p_begin) {
-          const float2 o = *at;
-          v.x = o.x + v.x;
-          v.y = o.y + v.y;
-        }
-        *at = v;
-      }
+  if (threadIdx.x == 0) {
+    for (int s = 0; s < stages; ++s) { mbar_init(&full_bar[s], SG_CUTTERS); mbar_init(&empty_bar[s], 2); }
+    for (int b = 0; b < 2; ++b) { mbar_init(&sum_full[b], 1); mbar_init(&sum_empty[b], SG_DRAINERS); }
+    mbar_init(&done_bar, 2);
+    abort_flag = 0;
+    asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
-  unsigned rank = 0, size = 1;
-  if (split) {
-    rank = blockIdx.z;
-    size = gridDim.z;
-    asm volatile("barrier.cluster.arrive.aligned;\n\tbarrier.cluster.wait.aligned;" ::: "memory");
+  pdl_trigger();
+  if (warp == SG_CUTTERS) tmem_alloc(&tmem_holder, 2 * buffer_cols);
+  asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+  __syncthreads();
+  asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+  const uint32_t tmem = tmem_holder;
+  volatile int* abort = &abort_flag;
+
+  if (warp < SG_CUTTERS) {
+    // ---------------- read and cut: eight lanes a row, eight entries a lane, 32 rows a step of all eight warps
+    const int row = threadIdx.x >> 3, piece = threadIdx.x & 7;
+    const int x_steps = (cols + 31) / 32;
+    float4 wv[SG_W / 32][2], xv[SG_X / 32][2];
+    auto read = [&](const float* from, int r, int limit, int k0, float4 (&v)[2]) {
+      // rows past the end read the last one: what they give is not stored
+      const float* at = from + (size_t)min(r, limit - 1) * k_dim + k0 + piece * 8;
+      if (VEC && k0 + SG_K <= k_dim) {
+        v[0] = sg_load4(at);
+        v[1] = sg_load4(at + 4);
+      } else {
+        float e[8];
+#pragma unroll
+        for (int j = 0; j < 8; ++j) e[j] = k0 + piece * 8 + j < k_dim ? at[j] : 0.f;
+        v[0] = make_float4(e[0], e[1], e[2], e[3]);
+        v[1] = make_float4(e[4], e[5], e[6], e[7]);
+      }
+    };
+    auto read_w = [&](int i) {
+#pragma unroll
+      for (int j = 0; j < SG_W / 32; ++j) read(args.w, n_base + row + 32 * j, args.n_out, (kb_begin + i) * SG_K, wv[j]);
+    };
+    auto read_x = [&](int i) {
+#pragma unroll
+      for (int j = 0; j < SG_X / 32; ++j)
+        if (j < x_steps) read(args.x, m_base + row + 32 * j, args.rows, (kb_begin + i) * SG_K, xv[j]);
+    };
+    auto file = [&](uint32_t plane, int plane_bytes, int r, const float4 (&v)[2]) {
+      uint4 hi, mid, low;
+      sg_cut(v[0].x, v[0].y, hi.x, mid.x, low.x);
+      sg_cut(v[0].z, v[0].w, hi.y, mid.y, low.y);
+      sg_cut(v[1].x, v[1].y, hi.z, mid.z, low.z);
+      sg_cut(v[1].z, v[1].w, hi.w, mid.w, low.w);
+      const uint32_t at = plane + r * 128 + ((piece ^ (r & 7)) << 4);
+      sg_store4(at, hi);
+      sg_store4(at + plane_bytes, mid);
+      sg_store4(at + 2 * plane_bytes, low);
+    };
+    pdl_wait();
+    if (n_kb > 0) {
+      read_w(0);
+      read_x(0);
+    }
+    int s = 0;
+    uint32_t parity = 1;                     // (a fresh barrier's phase before the first counts as completed)
+    for (int i = 0; i < n_kb; ++i) {
+      if (!__all_sync(0xffffffffu, mbar_wait(&empty_bar[s], parity, abort))) break;
+      const uint32_t stage = smem + s * stage_bytes;
+#pragma unroll
+      for (int j = 0; j < SG_W / 32; ++j) file(stage, SG_W_PLANE, row + 32 * j, wv[j]);
+#pragma unroll
+      for (int j = 0; j < SG_X / 32; ++j)
+        if (row + 32 * j < cols) file(stage + 3 * SG_W_PLANE, x_plane, row + 32 * j, xv[j]);
+      asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+      __syncwarp();
+      if (lane == 0) asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(smem_u32(&full_bar[s])) : "memory");
+      if (i + 1 < n_kb) {                    // (behind the fence, which would wait for them)
+        read_w(i + 1);
+        read_x(i + 1);
+      }
+      if (++s == stages) { s = 0; parity ^= 1; }
+    }
   } else {
-    __syncthreads();
-  }
-  // block `rank` of the cluster stores the tile's rows rank, rank + size, ..; a warp a row
-  for (int m = rank + size * warp; m < SG_M; m += size * 4) {
-    if (m_base + m >= rows) break;
-    const int n = 4 * lane;
-    float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
-    const unsigned at = (unsigned)__cvta_generic_to_shared(&sm.sum[m][n]);
-    for (unsigned r = 0; r < size; ++r) {
-      float4 o;
-      if (split) {
-        unsigned peer;
-        asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(peer) : "r"(at), "r"(r));
-        asm volatile("ld.shared::cluster.v4.f32 {%0, %1, %2, %3}, [%4];" : "=f"(o.x), "=f"(o.y), "=f"(o.z), "=f"(o.w) : "r"(peer) : "memory");
-      } else {
-        o = *reinterpret_cast<const float4*>(&sm.sum[m][n]);
-      }
-      if (r == 0) v = o;
-      else v = make_float4(v.x + o.x, v.y + o.y, v.z + o.z, v.w + o.w);
-    }
-    float* to = y + (size_t)(m_base + m) * n_out + n_base + n;
-    const float e[4] = {v.x, v.y, v.z, v.w};
-    if (n_out % 4 == 0) {
-      if (n_base + n < n_out) *reinterpret_cast<float4*>(to) = v;
-    } else {
+    // ---------------- add up the accumulators: a lane has one row of w, its columns are rows of x.  Two of these warps also
+    // issue the MMAs, each those of one accumulator (together, one elected lane), before they empty the other: issuing
+    // takes a warp longer than emptying (1,090 cycles of 1,800 a chunk when one warp issued all).
+    const int quarter = warp & 3, half = (warp - SG_CUTTERS) >> 2;
+    const bool issuer = quarter == 0;
+    const uint32_t idesc = instr_desc(cols);
+    const int n_chunks = n_kb * (SG_K / SG_CHUNK);
+    int s = 0;
+    uint32_t parity = 0;
+    auto issue = [&](int chunk) -> bool {
+      if (!__all_sync(0xffffffffu, mbar_wait(&full_bar[s], parity, abort))) return false;
+      if (!__all_sync(0xffffffffu, mbar_wait(&sum_empty[half], ((chunk >> 1) & 1) ^ 1, abort))) return false;
+      asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+      const uint32_t at = smem + s * stage_bytes + half * SG_CHUNK * 2;
+      const uint32_t d = tmem + half * buffer_cols;
+      // (formed by the whole warp, so that they are in uniform registers, as an MMA wants them)
+      uint64_t wd[3], xd[3];
 #pragma unroll
-      for (int j = 0; j < 4; ++j)
-        if (n_base + n + j < n_out) to[j] = e[j];
+      for (int p = 0; p < 3; ++p) {
+        wd[p] = smem_desc(at + p * SG_W_PLANE);
+        xd[p] = smem_desc(at + 3 * SG_W_PLANE + p * x_plane);
+      }
+      if (elect_one()) {
+        // the pieces of w and of x that meet, the smallest products first
+        constexpr int PW[6] = {2, 0, 1, 1, 0, 0}, PX[6] = {0, 2, 1, 0, 1, 0};
+#pragma unroll
+        for (int t = 0; t < 6; ++t)
+#pragma unroll
+          for (int k = 0; k < SG_CHUNK / 16; ++k)                     // 16 entries of k are 32 bytes: 2 units
+            umma_bf16(d, wd[PW[t]] + 2 * k, xd[PX[t]] + 2 * k, idesc, t > 0 || k > 0 ? 1u : 0u);
+        umma_commit(&sum_full[half]);
+        umma_commit(&empty_bar[s]);
+      }
+      __syncwarp();
+      if (++s == stages) { s = 0; parity ^= 1; }
+      return true;
+    };
+    const int r = quarter * 32 + lane;
+    float sum[SG_X / 32][16];
+#pragma unroll
+    for (int j = 0; j < SG_X / 32; ++j)
+#pragma unroll
+      for (int c = 0; c < 16; ++c) sum[j][c] = 0.f;
+    bool ok = !issuer || half != 0 || n_chunks == 0 || issue(0);
+#pragma unroll 1
+    for (int chunk = 0; ok && chunk < n_chunks; ++chunk) {
+      if (issuer && ((chunk + 1) & 1) == half && chunk + 1 < n_chunks && !issue(chunk + 1)) break;
+      if (!__all_sync(0xffffffffu, mbar_wait(&sum_full[chunk & 1], (chunk >> 1) & 1, abort))) break;
+      asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+      const uint32_t from = tmem + (chunk & 1) * buffer_cols + ((uint32_t)(quarter * 32) << 16);
+#pragma unroll
+      for (int j = 0; j < SG_X / 32; j += 2) {
+        const int c0 = 32 * j + 16 * half;
+        if (j + 1 < SG_X / 32 && c0 + 32 < cols) {
+          float v[32];
+          sg_tmem_load16x2(from + c0, v);
+#pragma unroll
+          for (int c = 0; c < 32; ++c) sum[j + c / 16][c % 16] += v[c];
+        } else if (c0 < cols) {
+          float v[16];
+          sg_tmem_load16(from + c0, v);
+#pragma unroll
+          for (int c = 0; c < 16; ++c) sum[j][c] += v[c];
+        }
+      }
+      asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+      __syncwarp();
+      if (lane == 0) asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(smem_u32(&sum_empty[chunk & 1])) : "memory");
+    }
+    if (issuer) {
+      // nothing this block issued is in flight when it leaves (it is not, unless a wait ran out)
+      if (elect_one()) umma_commit(&done_bar);
+      __syncwarp();
+      const uint64_t start = now_ns();
+      while (!mbar_try(&done_bar, 0) && now_ns() - start < TC_WAIT_LIMIT_NS) {}
+    }
+    pdl_wait();                              // before the first store: an earlier kernel may still read y's memory
+    const int n = n_base + r;
+    if (args.parts > 1) {
+      // (the ring is idle: every MMA that read it has been waited for)
+#pragma unroll
+      for (int j = 0; j < SG_X / 32; ++j)
+#pragma unroll
+        for (int c = 0; c < 16; ++c) {
+          const int m = 32 * j + 16 * half + c;
+          if (m < rows_here)
+            asm volatile("st.shared.f32 [%0], %1;" ::"r"(smem + (m * SG_W + r) * 4), "f"(sum[j][c]) : "memory");
+        }
+    } else if (n < args.n_out) {
+#pragma unroll
+      for (int j = 0; j < SG_X / 32; ++j)
+#pragma unroll
+        for (int c = 0; c < 16; ++c) {
+          const int m = 32 * j + 16 * half + c;
+          if (m < rows_here) args.y[(size_t)(m_base + m) * args.n_out + n] = sum[j][c];
+        }
+      bool again = false;
+#pragma unroll
+      for (int j = 0; j < SG_X / 32; ++j)
+#pragma unroll
+        for (int c = 0; c < 16; ++c) again |= 32 * j + 16 * half + c < rows_here && sg_again(sum[j][c]);
+      if (again)
+#pragma unroll 1
+        for (int m = 16 * half; m < rows_here; m += m % 16 == 15 ? 17 : 1) {
+          float* at = args.y + (size_t)(m_base + m) * args.n_out + n;
+          if (sg_again(*at)) *at = sg_chain(args.x + (size_t)(m_base + m) * k_dim, args.w + (size_t)n * k_dim, k_dim);
+        }
     }
   }
-  // no block leaves while a peer may still read its sums
-  if (split) asm volatile("barrier.cluster.arrive.aligned;\n\tbarrier.cluster.wait.aligned;" ::: "memory");
+
+  if (args.parts > 1) {
+    asm volatile("barrier.cluster.arrive.release;\n\tbarrier.cluster.wait.acquire;" ::: "memory");
+    if (!*abort) {
+      const bool vector_store = args.n_out % 4 == 0;
+      const int n_items = rows_here * (SG_W / 4);
+      uint32_t base[SG_MAX_PARTS];
+#pragma unroll
+      for (int p = 0; p < SG_MAX_PARTS; ++p) {
+        base[p] = 0;
+        if (p < args.parts) asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(base[p]) : "r"(smem), "r"(p));
+      }
+      // an item: four neighbouring results; the loads of all parts are in flight together and are added in order
+      for (int item = part * SG_THREADS + threadIdx.x; item < n_items; item += args.parts * SG_THREADS) {
+        const int m = item >> 5, c = (item & 31) * 4, n = n_base + c;
+        float4 v[SG_MAX_PARTS];
+#pragma unroll
+        for (int p = 0; p < SG_MAX_PARTS; ++p)
+          if (p < args.parts)
+            asm volatile("ld.shared::cluster.v4.f32 {%0, %1, %2, %3}, [%4];"
+                         : "=f"(v[p].x), "=f"(v[p].y), "=f"(v[p].z), "=f"(v[p].w) : "r"(base[p] + 16 * item) : "memory");
+        float e[4] = {v[0].x, v[0].y, v[0].z, v[0].w};
+#pragma unroll
+        for (int p = 1; p < SG_MAX_PARTS; ++p)
+          if (p < args.parts) { e[0] += v[p].x; e[1] += v[p].y; e[2] += v[p].z; e[3] += v[p].w; }
+#pragma unroll
+        for (int j = 0; j < 4; ++j)
+          if (sg_again(e[j]) && n + j < args.n_out)
+            e[j] = sg_chain(args.x + (size_t)(m_base + m) * k_dim, args.w + (size_t)(n + j) * k_dim, k_dim);
+        float* to = args.y + (size_t)(m_base + m) * args.n_out + n;
+        if (vector_store) {
+          if (n < args.n_out) *reinterpret_cast<float4*>(to) = make_float4(e[0], e[1], e[2], e[3]);
+        } else {
+#pragma unroll
+          for (int j = 0; j < 4; ++j)
+            if (n + j < args.n_out) to[j] = e[j];
+        }
+      }
+    }
+    // no block leaves while a neighbour may still read its sums
+    asm volatile("barrier.cluster.arrive.relaxed;\n\tbarrier.cluster.wait;" ::: "memory");
+  }
+
+  asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+  __syncthreads();
+  if (warp == SG_CUTTERS) tmem_free(tmem, 2 * buffer_cols);
+  if (threadIdx.x == 0 && abort_flag && args.status) atomicOr(args.status, 4);
 }
 
 extern "C" {
 
-// How many parts the k range of a product is cut into: enough that one row of output tiles fills the SMs about
-// twice (two to three blocks fit an SM), none shorter than 128 (eight slices: below that a block mostly fills and
-// drains its pipeline).  A cluster's blocks take the parts while all tiles' parts are at most a few waves; from four
-// waves of tiles on there is nothing to fill and the parts' sums need not travel.
-int sb_sgemm_parts(int n_out, int k_dim) {
-  const int tiles = (n_out + SG_N - 1) / SG_N;
-  int parts = 1;
-  while (parts < SG_MAX_PARTS && parts * tiles < 296 && k_dim >= 2 * parts * 128) parts *= 2;
-  return parts;
-}
-
-int sb_sgemm_nt(const float* x, const float* w, float* y, int rows, int n_out, int k_dim,
+// x [rows, k_dim] and w [n_out, k_dim] float32, y [rows, n_out].  Bit 4 of *status (if there is one) is set when a wait
+// ran out.  How many parts the k range is cut into: as many as let one row of tiles run at once, each of two slices
+// at least.  Clusters do not fill the SMs, whose groups are not multiples of them: how many of p blocks run at once is the
+// occupancy query's answer for one block an SM.  One cluster too many is a second round: 16 tiles of 8 parts took 41 us a
+// product of 141 x 2048 x 2048, of 6 parts 29.
+int sb_sgemm_nt(const float* x, const float* w, float* y, int rows, int n_out, int k_dim, int* status,
                 cudaStream_t s) {
   if (rows == 0 || n_out == 0) return 0;
-  const int parts = sb_sgemm_parts(n_out, k_dim);
-  const int part_k = ((k_dim + parts - 1) / parts + SG_K - 1) / SG_K * SG_K;
-  const int tn = (n_out + SG_N - 1) / SG_N, tm = (rows + SG_M - 1) / SG_M;
+  const int tiles = (n_out + SG_W - 1) / SG_W, slices = (k_dim + SG_K - 1) / SG_K;
+  static const int at_once[SG_MAX_PARTS + 1] = {0, 148, 74, 45, 33, 26, 22, 15, 15};
+  int parts = SG_MAX_PARTS;
+  while (parts > 1 && (at_once[parts] < tiles || 2 * parts > slices)) --parts;
+  const int row_tiles = (rows - 1) / SG_X + 1;
+  if ((long long)tiles * row_tiles > 0x7fffffffLL) return -2;
+  SgemmArgs args;
+  args.x = x; args.w = w; args.y = y; args.status = status;
+  args.rows = rows; args.n_out = n_out; args.k_dim = k_dim; args.parts = parts;
+  args.tile_rows = ((rows - 1) / row_tiles + 16) / 16 * 16;
+  const int stage_bytes = 3 * (SG_W_PLANE + args.tile_rows * SG_K * 2);
+  args.stages = (SG_SMEM - 1024) / stage_bytes;
+  if (args.stages > SG_MAX_STAGES) args.stages = SG_MAX_STAGES;
   const bool vec = k_dim % 4 == 0 && ((uintptr_t)x % 16) == 0 && ((uintptr_t)w % 16) == 0;
-  const bool split = parts > 1 && (long long)tn * tm < 4 * 148;      // (an order of work, not of sums: see above)
-  auto kernel = vec ? sgemm_nt_kernel<true> : sgemm_nt_kernel<false>;
-  cudaError_t err = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(SgemmTiles));
+  auto kernel = vec ? sgemm_tcgen05_kernel<true> : sgemm_tcgen05_kernel<false>;
+  cudaError_t err = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, SG_SMEM);
   if (err != cudaSuccess) return (int)err;
-  cudaLaunchConfig_t cfg = {};
-  cfg.gridDim = dim3((unsigned)((long long)tn * tm), 1, split ? parts : 1);
-  cfg.blockDim = dim3(128);
-  cfg.dynamicSmemBytes = sizeof(SgemmTiles);
-  cfg.stream = s;
-  cudaLaunchAttribute attr[1];
-  attr[0].id = cudaLaunchAttributeClusterDimension;
-  attr[0].val.clusterDim.x = 1;
-  attr[0].val.clusterDim.y = 1;
-  attr[0].val.clusterDim.z = split ? parts : 1;
-  cfg.attrs = attr;
-  cfg.numAttrs = 1;
-  err = cudaLaunchKernelEx(&cfg, kernel, x, w, y, rows, n_out, k_dim, parts, part_k);
-  return err == cudaSuccess ? SB_LAUNCH_RESULT() : (int)err;
+  const int smem = args.stages * stage_bytes + 1024;
+  return launch_dependent_cluster(kernel, dim3(tiles * row_tiles, parts), dim3(SG_THREADS), smem, s, dim3(1, parts, 1), args);
 }
 
 }  // extern "C"

@@ -254,7 +254,7 @@ def linear(x, weight, out_float=False, gated=False, status=None, add_to=None):
     if dt == 0:
         y = x.new_empty((rows, n_total), dtype=torch.float32)
         rc = _lib("sgemm").sb_sgemm_nt(_ptr(x), _ptr(weight), _ptr(y), rows, n_total, k_dim,
-                                             _stream())
+                                       _ptr(status), _stream())
         _check(rc, "sgemm")
     elif out_float:
         y = torch.mm(x, weight.t(), out_dtype=torch.float32)

@@ -124,6 +124,37 @@ def test_float32_product_in_parts(rows, n, k):
     assert torch.equal(ops.linear(dev(x[:17]), dev(w)), got[:17])
 
 
+@pytest.mark.parametrize("rows,n,k", [(160, 1, 33), (161, 130, 64), (321, 20, 65), (40, 6000, 640)])
+def test_float32_product_at_the_edges_of_its_tiles(rows, n, k):
+    """Tiles of up to 160 rows in steps of 16, slices of 64, one part and several: the bound of a chain of k products."""
+    from starter_b200 import ops
+
+    x, w = rand(rows, k, seed=rows), rand(n, k, seed=n)
+    got = ops.linear(dev(x), dev(w)).cpu().double()
+    bound = (k + 8) * 2.0 ** -24 * (x.double().abs() @ w.double().abs().t())
+    assert bool(((got - x.double() @ w.double().t()).abs() <= bound).all())
+
+
+@pytest.mark.parametrize("k", [100, 1024])
+def test_float32_product_of_values_that_cannot_be_cut(k):
+    """Infinities, NaN, values next to the largest float and near the smallest: as a chain of products gives them, the
+    other rows untouched."""
+    from starter_b200 import ops
+
+    x, w = rand(20, k, seed=3), rand(130, k, seed=4)
+    want = ops.linear(dev(x), dev(w)).cpu()
+    x[2, 7], x[3, k - 1], x[4, 5], x[5] = float("inf"), float("-inf"), float("nan"), 0.0
+    x[5, 9], w[:, 9] = 3.4e38, w[:, 9].clamp(-0.9, 0.9)
+    x[6] *= 1e-36
+    exact = x.double() @ w.double().t()
+    got = ops.linear(dev(x), dev(w)).cpu()
+    assert torch.equal(got[2:4].double(), exact[2:4]) and bool(got[4].isnan().all())
+    bound = (k + 8) * 2.0 ** -24 * (x.double().abs() @ w.double().abs().t()) + k * 2.0 ** -149
+    assert bool(((got.double() - exact).abs()[5:7] <= bound[5:7]).all())
+    kept = ops.linear(dev(x[7:].contiguous().repeat(2, 1)), dev(w)).cpu()
+    assert torch.equal(got[7:], kept[:13]) and want.shape == got.shape
+
+
 @pytest.mark.parametrize("dtype", list(DT))
 @pytest.mark.parametrize("rows", [1, 5, 16, 40])
 def test_gated_linear_equals_product_then_swiglu(dtype, rows):

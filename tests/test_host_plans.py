@@ -112,4 +112,4 @@ def test_every_entry_point_the_operations_call_has_declared_arguments():
     assert used and not used - set(known)
     result, types = known["sb_sgemm_nt"]
     assert result is ctypes.c_int
-    assert types == [ctypes.c_void_p] * 3 + [ctypes.c_int] * 3 + [ctypes.c_void_p]
+    assert types == [ctypes.c_void_p] * 3 + [ctypes.c_int] * 3 + [ctypes.c_void_p] * 2
