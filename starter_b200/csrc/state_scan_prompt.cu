@@ -24,6 +24,8 @@
 // channel-decay 400 -> 177; unequal sequences of 801, 712 and 623 tokens: 383 -> 72, 598 -> 100, 382 -> 160, 377 -> 155.  The
 // error against 64 bits falls or stays (outputs 5.5e-7 -> 2.2e-7, 3.7e-7 -> 2.0e-7, 4.9e-8, 1.2e-7).  With one sequence
 // an SM has four warps and the chain's latencies are the bound (about 1,500 cycles a block of sixteen), not a pipe.
+#include <type_traits>
+
 #include "common.cuh"
 
 #define SP_N 128                 // rows of the state kept (N up to this; the rest are zeros)
@@ -233,7 +235,7 @@ scan_coef_kernel(const bf16* __restrict__ q, int ldq, const bf16* __restrict__ k
       const int r = 8 * (lane >> 4) + e;
       float s = 0.f;
 #pragma unroll
-      for (int i = 0; i < SP_CT; ++i) s = fmaf(sb[warp][r][i], inv[i], s);
+      for (int i = 0; i <= 8 + e; ++i) s = fmaf(sb[warp][r][i], i <= e || (lane >> 4) ? inv[i] : 0.f, s);
       const float own = (lane >> 4) ? inv[8 + e] : inv[e];
       const float wr = __shfl_sync(0xffffffffu, wt, e), wr8 = __shfl_sync(0xffffffffu, wt, e + 8);
       if (r < ct) {
@@ -395,7 +397,13 @@ scan_blocks_kernel(const bf16* __restrict__ q, int ldq, const bf16* __restrict__
       }
       update(w);
     }
-    __syncthreads();                                // the warps' sums are there
+    const uint32_t vv = *reinterpret_cast<const uint32_t*>(&st.v[tok][c2]);
+    // Coefficients of later tokens are zero, but 0 * inf would not be: a block with a value that is not finite masks them
+    // (the test rides on a barrier that is there anyway, the masked sums stand behind the usual ones: 164 us a layer of 2,048 tokens;
+    // masking always, or a branch around the usual sums: 190)
+    bool bad = !(fabsf(__uint_as_float(vv << 16)) < INFINITY && fabsf(__uint_as_float(vv & 0xffff0000u)) < INFINITY);
+    if constexpr (DELTA) __syncthreads();           // the warps' sums are there
+    else bad = __syncthreads_or(bad);
     const float4 s4 = *reinterpret_cast<const float4*>(&st.coef[tok][S_AT]);
     float2 rq = make_float2(0.f, 0.f);
 #pragma unroll
@@ -404,7 +412,6 @@ scan_blocks_kernel(const bf16* __restrict__ q, int ldq, const bf16* __restrict__
       rq.x += p.x;
       rq.y += p.y;
     }
-    const uint32_t vv = *reinterpret_cast<const uint32_t*>(&st.v[tok][c2]);
     if constexpr (DELTA) {
       float2 rk = make_float2(0.f, 0.f);
 #pragma unroll
@@ -413,36 +420,44 @@ scan_blocks_kernel(const bf16* __restrict__ q, int ldq, const bf16* __restrict__
         rk.x += p.x;
         rk.y += p.y;
       }
-      *reinterpret_cast<float2*>(&zs[tok][c2]) =
-          make_float2(s4.x * __uint_as_float(vv << 16) - s4.y * rk.x, s4.x * __uint_as_float(vv & 0xffff0000u) - s4.y * rk.y);
-      __syncthreads();
+      const float2 z = make_float2(s4.x * __uint_as_float(vv << 16) - s4.y * rk.x, s4.x * __uint_as_float(vv & 0xffff0000u) - s4.y * rk.y);
+      *reinterpret_cast<float2*>(&zs[tok][c2]) = z;
+      bad = __syncthreads_or(!(fabsf(z.x) < INFINITY && fabsf(z.y) < INFINITY));
     }
     float2 own = make_float2(0.f, 0.f), w2 = make_float2(0.f, 0.f);
+    auto small = [&](auto masked) {
 #pragma unroll
-    for (int i = 0; i < SP_CT; i += 4) {
-      const float4 b = *reinterpret_cast<const float4*>(&st.coef[tok][B_AT + i]);
-      const float bb[4] = {b.x, b.y, b.z, b.w};
-      float ww[4] = {0.f, 0.f, 0.f, 0.f};
-      if constexpr (DELTA) {
-        const float4 w = *reinterpret_cast<const float4*>(&st.coef[tok][i]);
-        ww[0] = w.x; ww[1] = w.y; ww[2] = w.z; ww[3] = w.w;
-      }
+      for (int i = 0; i < SP_CT; i += 4) {
+        const float4 b = *reinterpret_cast<const float4*>(&st.coef[tok][B_AT + i]);
+        const float bb[4] = {b.x, b.y, b.z, b.w};
+        float ww[4] = {0.f, 0.f, 0.f, 0.f};
+        if constexpr (DELTA) {
+          const float4 w = *reinterpret_cast<const float4*>(&st.coef[tok][i]);
+          ww[0] = w.x; ww[1] = w.y; ww[2] = w.z; ww[3] = w.w;
+        }
 #pragma unroll
-      for (int e = 0; e < 4; ++e) {
-        float2 z;
-        if constexpr (DELTA) {
-          z = *reinterpret_cast<const float2*>(&zs[i + e][c2]);
-        } else {
-          const uint32_t raw = *reinterpret_cast<const uint32_t*>(&st.v[i + e][c2]);
-          z = make_float2(__uint_as_float(raw << 16), __uint_as_float(raw & 0xffff0000u));
-        }
-        own.x = fmaf(bb[e], z.x, own.x);
-        own.y = fmaf(bb[e], z.y, own.y);
-        if constexpr (DELTA) {
-          w2.x = fmaf(ww[e], z.x, w2.x);
-          w2.y = fmaf(ww[e], z.y, w2.y);
+        for (int e = 0; e < 4; ++e) {
+          float2 z;
+          if constexpr (DELTA) {
+            z = *reinterpret_cast<const float2*>(&zs[i + e][c2]);
+          } else {
+            const uint32_t raw = *reinterpret_cast<const uint32_t*>(&st.v[i + e][c2]);
+            z = make_float2(__uint_as_float(raw << 16), __uint_as_float(raw & 0xffff0000u));
+          }
+          if (decltype(masked)::value && i + e > tok) z = make_float2(0.f, 0.f);
+          own.x = fmaf(bb[e], z.x, own.x);
+          own.y = fmaf(bb[e], z.y, own.y);
+          if constexpr (DELTA) {
+            w2.x = fmaf(ww[e], z.x, w2.x);
+            w2.y = fmaf(ww[e], z.y, w2.y);
+          }
         }
       }
+    };
+    small(std::false_type{});
+    if (bad) {                                      // (behind, so that the usual way has no branch in it)
+      own = w2 = make_float2(0.f, 0.f);
+      small(std::true_type{});
     }
     if constexpr (DELTA) *reinterpret_cast<float2*>(&ws[tok][c2]) = w2;
     if (t0 + tok < q_len && col0 + c2 < V)

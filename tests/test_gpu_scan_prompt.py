@@ -100,3 +100,33 @@ def test_many_tokens_a_sequence(mode, heads, groups, n, width, monkeypatch):
         out[pick] = run(pick, sizes, slots)
     assert float((out - got).abs().max()) <= 2e-5 * float(got.abs().max())
     assert float((kept - state).abs().max()) <= 2e-5 * float(state.abs().max())
+
+
+@pytest.mark.parametrize("mode", ["state_space", "gated_delta", "forget_write", "channel_decay"])
+@pytest.mark.parametrize("which", ["q", "k", "v"])
+def test_a_token_that_is_not_finite_leaves_earlier_tokens_alone(mode, which):
+    from starter_b200 import ops
+
+    heads, n, width, tokens, bad = 2, 128, 32, 70, 37
+    gen = torch.Generator().manual_seed(heads + n)
+    ins = {name: torch.randn(tokens, heads * size, generator=gen).to(BF).cuda()
+           for name, size in (("q", n), ("k", n), ("v", width), ("ab", 2))}
+    per = heads * n if mode == "forget_write" else heads
+    A, bias, skip = torch.linspace(-2.0, -1.0, per).cuda(), torch.zeros(per).cuda(), torch.ones(heads).cuda()
+    decay = torch.full((tokens, heads * n), 0.1).cuda() if mode == "channel_decay" else None
+    scalars = mode in ("state_space", "gated_delta")
+
+    def run():
+        state = torch.zeros(1, heads * n * width, device="cuda")
+        return ops.state_scan(
+            mode, (ins["q"], 0), (ins["k"], 0), (ins["v"], 0), (ins["ab"], 0) if scalars else None,
+            (ins["ab"], heads) if mode == "gated_delta" else None, None if decay is not None else A.sigmoid(),
+            None if decay is not None else bias, skip if mode == "state_space" else None, state, 0, *packed([tokens], [0]), heads,
+            heads, n, width, decay=decay)
+
+    want = run()
+    ins[which][bad, 3] = float("inf")
+    got = run()
+    assert torch.equal(got[:bad], want[:bad])
+    # (forget-write's keys are gates: an infinite one is an open gate)
+    assert bool(got[bad].isfinite().all()) == (mode == "forget_write" and which == "k")
