@@ -215,77 +215,77 @@ __global__ void __launch_bounds__(512) moe_route_all_kernel(const T* __restrict_
                           outputs + (gate_out ? 1 : 0));
   __syncthreads();
   for (int t = warp; t < TOK && row0 + t < n_tokens; t += warps) {
-  const int row = row0 + t;
-  float* z = route_z + t * per_token;
-  float* score = z + outputs + 1;
-  float* choice = score + outputs;
-  float* best_of = choice + outputs;
-  if (gate_out && lane == 0) gate_out[row] = 1.f / (1.f + expf(-z[outputs]));
-  float top_z = -INFINITY;
-  for (int e = lane; e < outputs; e += 32) top_z = fmaxf(top_z, z[e]);
-  top_z = warp_max(top_z);
-  float sum = 0.f;
-  for (int e = lane; e < outputs; e += 32) {
-    const float v = expf(z[e] - top_z);
-    score[e] = v;
-    sum += v;
-  }
-  sum = warp_sum(sum);
-  for (int e = lane; e < outputs; e += 32) {
-    score[e] /= sum;
-    choice[e] = score[e] + (correction ? correction[e] : 0.f);
-  }
-  __syncwarp();
-  if (groups > 1) {
-    const int per = outputs / groups;
-    for (int g = lane; g < groups; g += 32) {
-      float v = -INFINITY;
-      for (int e = g * per; e < (g + 1) * per; ++e) v = fmaxf(v, choice[e]);
-      best_of[g] = v;
+    const int row = row0 + t;
+    float* z = route_z + t * per_token;
+    float* score = z + outputs + 1;
+    float* choice = score + outputs;
+    float* best_of = choice + outputs;
+    if (gate_out && lane == 0) gate_out[row] = 1.f / (1.f + expf(-z[outputs]));
+    float top_z = -INFINITY;
+    for (int e = lane; e < outputs; e += 32) top_z = fmaxf(top_z, z[e]);
+    top_z = warp_max(top_z);
+    float sum = 0.f;
+    for (int e = lane; e < outputs; e += 32) {
+      const float v = expf(z[e] - top_z);
+      score[e] = v;
+      sum += v;
+    }
+    sum = warp_sum(sum);
+    for (int e = lane; e < outputs; e += 32) {
+      score[e] /= sum;
+      choice[e] = score[e] + (correction ? correction[e] : 0.f);
     }
     __syncwarp();
-    // the `keep` best groups are marked with +inf, then every other group's outputs leave the choice
-    for (int c = 0; c < keep; ++c) {
+    if (groups > 1) {
+      const int per = outputs / groups;
+      for (int g = lane; g < groups; g += 32) {
+        float v = -INFINITY;
+        for (int e = g * per; e < (g + 1) * per; ++e) v = fmaxf(v, choice[e]);
+        best_of[g] = v;
+      }
+      __syncwarp();
+      // the `keep` best groups are marked with +inf, then every other group's outputs leave the choice
+      for (int c = 0; c < keep; ++c) {
+        float v = -INFINITY;
+        int at = 0x7fffffff;
+        for (int g = lane; g < groups; g += 32)
+          if (best_of[g] != INFINITY && (best_of[g] > v || at == 0x7fffffff)) { v = best_of[g]; at = g; }
+        for (int o = 16; o > 0; o >>= 1) {
+          const float ov = __shfl_xor_sync(0xffffffffu, v, o);
+          const int oa = __shfl_xor_sync(0xffffffffu, at, o);
+          if (oa != 0x7fffffff && (at == 0x7fffffff || ov > v || (ov == v && oa < at))) { v = ov; at = oa; }
+        }
+        if (lane == 0 && at < groups) best_of[at] = INFINITY;
+        __syncwarp();
+      }
+      for (int e = lane; e < outputs; e += 32)
+        if (best_of[e / per] != INFINITY) choice[e] = -INFINITY;
+      __syncwarp();
+    }
+    float picked[MOE_MAX_TOP];
+    for (int c = 0; c < top; ++c) {
       float v = -INFINITY;
       int at = 0x7fffffff;
-      for (int g = lane; g < groups; g += 32)
-        if (best_of[g] != INFINITY && (best_of[g] > v || at == 0x7fffffff)) { v = best_of[g]; at = g; }
+      for (int e = lane; e < outputs; e += 32)
+        if (choice[e] > v) { v = choice[e]; at = e; }
       for (int o = 16; o > 0; o >>= 1) {
         const float ov = __shfl_xor_sync(0xffffffffu, v, o);
         const int oa = __shfl_xor_sync(0xffffffffu, at, o);
-        if (oa != 0x7fffffff && (at == 0x7fffffff || ov > v || (ov == v && oa < at))) { v = ov; at = oa; }
+        if (ov > v || (ov == v && oa < at)) { v = ov; at = oa; }
       }
-      if (lane == 0 && at < groups) best_of[at] = INFINITY;
+      if (at >= outputs) at = 0;          // nothing left to choose from: keep the indices inside the table
+      picked[c] = score[at];
+      if (lane == 0) {
+        ids[(size_t)row * top + c] = at;
+        choice[at] = -INFINITY;
+      }
       __syncwarp();
     }
-    for (int e = lane; e < outputs; e += 32)
-      if (best_of[e / per] != INFINITY) choice[e] = -INFINITY;
-    __syncwarp();
-  }
-  float picked[MOE_MAX_TOP];
-  for (int c = 0; c < top; ++c) {
-    float v = -INFINITY;
-    int at = 0x7fffffff;
-    for (int e = lane; e < outputs; e += 32)
-      if (choice[e] > v) { v = choice[e]; at = e; }
-    for (int o = 16; o > 0; o >>= 1) {
-      const float ov = __shfl_xor_sync(0xffffffffu, v, o);
-      const int oa = __shfl_xor_sync(0xffffffffu, at, o);
-      if (ov > v || (ov == v && oa < at)) { v = ov; at = oa; }
-    }
-    if (at >= outputs) at = 0;          // nothing left to choose from: keep the indices inside the table
-    picked[c] = score[at];
     if (lane == 0) {
-      ids[(size_t)row * top + c] = at;
-      choice[at] = -INFINITY;
+      float total = 0.f;
+      for (int c = 0; c < top; ++c) total += picked[c];
+      for (int c = 0; c < top; ++c) weights[(size_t)row * top + c] = picked[c] / (total + 1e-20f) * weight_scale;
     }
-    __syncwarp();
-  }
-  if (lane == 0) {
-    float total = 0.f;
-    for (int c = 0; c < top; ++c) total += picked[c];
-    for (int c = 0; c < top; ++c) weights[(size_t)row * top + c] = picked[c] / (total + 1e-20f) * weight_scale;
-  }
   }
 }
 
@@ -1125,10 +1125,13 @@ int sb_moe_route_all(int dtype, const void* h, const float* w, const float* corr
   if (n_tokens == 0) return 0;
   if (outputs < 1 || outputs > MOE_MAX_EXPERTS || top < 1 || top > MOE_MAX_TOP) return -2;
   if (groups < 1 || outputs % groups || keep < 1 || keep > groups || top > outputs / groups * keep) return -2;
-  const bool many = n_tokens >= 4 * 148 && outputs <= 256;          // (4 tokens a block: see sb_moe_route)
+  // 4 tokens a block (see sb_moe_route), where their numbers fit beside the staged rows into the 48 KB of a plain launch: 256
+  // outputs in 256 groups do not
+  const size_t token_bytes = (size_t)(3 * outputs + 1 + groups) * sizeof(float);
+  const bool many = n_tokens >= 4 * 148 && MOE_STAGE_BYTES + 4 * token_bytes <= 48 * 1024;
   const int threads = many ? (outputs > 16 ? 256 : 128) : outputs >= 16 ? 512 : outputs > 4 ? 256 : 128;
   const int blocks = many ? (n_tokens + 3) / 4 : n_tokens;
-  const size_t smem = (many ? MOE_STAGE_BYTES : 0) + (size_t)(many ? 4 : 1) * (3 * outputs + 1 + groups) * sizeof(float);      // (under 48 KB)
+  const size_t smem = many ? MOE_STAGE_BYTES + 4 * token_bytes : token_bytes;
 #define MOE_ROUTE(T, TOK)                                                                                              \
   return launch_dependent(moe_route_all_kernel<T, TOK>, dim3(blocks), dim3(threads), smem, s, (const T*)h, w, correction, ids, \
                           weights, gate_out, n_tokens, width, outputs, top, groups, keep, weight_scale)
