@@ -482,15 +482,16 @@ scan_blocks_kernel(const bf16* __restrict__ q, int ldq, const bf16* __restrict__
 }
 
 // ------------------------------------------------------------------------------------------ a decay per row
-// qf = silu(q), d = (1 - lower) sigmoid(-(z + bias)): a thread eight channels of a token.
+// qf = silu(q), d = (1 - lower) sigmoid(-(z + bias)): a thread eight channels of a token (blockIdx.x: a step may bring more
+// tokens than the grid's other dimensions count to).
 __global__ void __launch_bounds__(256)
 scan_gates_kernel(const bf16* __restrict__ q, int ldq, const bf16* __restrict__ z, int ldz, const float* __restrict__ lower,
                   const float* __restrict__ bias, float* __restrict__ qf, float* __restrict__ d, int channels) {
   pdl_wait();
   SB_BEHIND_WAIT(q); SB_BEHIND_WAIT(z);
-  const int c = (blockIdx.x * 256 + threadIdx.x) * 8;
+  const int c = (blockIdx.y * 256 + threadIdx.x) * 8;
   if (c >= channels) return;
-  const size_t row = blockIdx.y;
+  const size_t row = blockIdx.x;
   const uint4 qv = *reinterpret_cast<const uint4*>(q + row * ldq + c), zv = *reinterpret_cast<const uint4*>(z + row * ldz + c);
   const uint32_t qw[4] = {qv.x, qv.y, qv.z, qv.w}, zw[4] = {zv.x, zv.y, zv.z, zv.w};
   float a[8], g[8];
@@ -696,7 +697,7 @@ int sb_state_scan_prompt(int mode, const void* q, int ldq, const void* k, int ld
     const int channels = H * N;
     float* qf = scratch;
     float* d = scratch + (size_t)n_tokens * channels;
-    int rc = launch_dependent(scan_gates_kernel, dim3((channels / 8 + 255) / 256, n_tokens), dim3(256), 0, s, (const bf16*)q, ldq,
+    int rc = launch_dependent(scan_gates_kernel, dim3(n_tokens, (channels / 8 + 255) / 256), dim3(256), 0, s, (const bf16*)q, ldq,
                               (const bf16*)k, ldk, A_log, dt_bias, qf, d, channels);
     if (rc) return rc;
     const size_t smem = SP_STAGES * sizeof(ForgetStage);

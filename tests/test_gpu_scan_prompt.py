@@ -130,3 +130,27 @@ def test_a_token_that_is_not_finite_leaves_earlier_tokens_alone(mode, which):
     assert torch.equal(got[:bad], want[:bad])
     # (forget-write's keys are gates: an infinite one is an open gate)
     assert bool(got[bad].isfinite().all()) == (mode == "forget_write" and which == "k")
+
+
+@pytest.mark.parametrize("mode", ["state_space", "gated_delta", "forget_write", "channel_decay"])
+def test_more_tokens_than_a_grid_counts_in_its_second_dimension(mode, monkeypatch):
+    from starter_b200 import ops
+
+    heads, n, width, lengths = 1, 72, 8, [33000, 32600]
+    total, gen = sum(lengths), torch.Generator().manual_seed(9)
+    q, k, v, ab = (torch.randn(total, size, generator=gen).to(BF).cuda() for size in (n, n, width, 8))
+    per = n if mode == "forget_write" else 1
+    A, bias = torch.full((per,), 0.3).cuda(), torch.zeros(per).cuda()
+    decay = torch.full((total, n), 0.1).cuda() if mode == "channel_decay" else None
+    scalars, outs = mode in ("state_space", "gated_delta"), []
+    for tokens in (64, 1 << 30):
+        monkeypatch.setattr(ops, "SCAN_PROMPT_TOKENS", tokens)
+        state = torch.zeros(2, n * width, device="cuda")
+        out = ops.state_scan(
+            mode, (q, 0), (k, 0), (v, 0), (ab, 0) if scalars else None, (ab, 1) if mode == "gated_delta" else None,
+            None if decay is not None else A, None if decay is not None else bias, bias if mode == "state_space" else None, state, 0,
+            *packed(lengths, [1, 0]), heads, heads, n, width, decay=decay)
+        outs.append((out, state))
+    for got, want in zip(*outs):
+        # (the bound of the comparison above: the state forgets within some ten tokens)
+        assert float((got - want).abs().max()) <= 2e-5 * float(want.abs().max())
