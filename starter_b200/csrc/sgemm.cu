@@ -12,7 +12,7 @@
 // while the MMAs of the one before run), cut them and file the pieces in 128-byte swizzled tiles; eight warps empty the
 // two accumulators in turn, two of which issue the MMAs.
 // Events around a launch, L2 flushed, the multiply-add kernel of 64 x 128 tiles that this replaces -> here: 141 x 2048 x 2048
-// 52 -> 29 us, 141 x 8192 x 2048 177 -> 52, 20 x 2048 x 2048 41 -> 20, 4096^3 2,942 -> 1,086 (126 TFLOP/s); nothing
+// 52 -> 30 us, 141 x 8192 x 2048 177 -> 55, 20 x 2048 x 2048 41 -> 22, 4096^3 2,942 -> 1,095 (126 TFLOP/s); nothing
 // measured between 17 x 5 x 4097 and 4096^3 is slower.  Error against 64 bits (rms, of the result's): 2.9e-7 -> 1.0e-7 at k = 2048,
 // 4.1e-7 -> 1.3e-7 at 4096.  By clock64() a slice at 144 rows is about 3,000 cycles where its MMAs alone are 1,730: issuing
 // costs some 90 cycles an MMA, and cutting 2,500 a slice.  Short k is bound by the ends: 5,000 cycles to the first
@@ -22,8 +22,15 @@
 // their sums in shared memory and each adds its share of the tile, part by part.  So the sum for one (m, n) is the same
 // whatever the other rows of the call are.
 //
-// Infinities, NaN and values next to the largest float do not survive the cut (inf - inf), and pieces of values near the
-// smallest are cut off: a result that is not finite, or is not zero but below 2^-80, is computed again as a chain of fmas.
+// What the pieces cannot hold is computed again as a chain of fmas.  Infinities, NaN and values next to the largest float do not
+// survive the cut (inf - inf): a result that is not finite is formed again.  A piece below 2^-133 is lost, which is less than
+// 2^-134 of an operand, and only of one below 2^-109: a result below 2^-80 is formed again, and so is every result whose
+// one row has such an entry and whose other row has one of 2^20 or more (where it has none, what is lost is under 2^-34 of the smallest
+// result that stays).  A product below 2^-126 may come out as zero: a zero is formed again where both rows have entries and one of them
+// has some below 2^-63.  The cutters keep the smallest magnitude they see (12 operations beside some 52 of cutting eight entries: a float32
+// layer of 141 tokens 147 -> 152 us); only a block that finds one below 2^-63 goes over its rows again and notes what each has: all
+// of k if there was one below 2^-109, else up to the first entry that is not zero (4096^3: 1,095 us, 1,180 with entries below
+// 2^-63, 2,430 with entries below 2^-109).
 #include "tcgen05.cuh"
 
 #define SG_W 128                 // rows of w a block
@@ -37,6 +44,12 @@
 #define SG_MAX_PARTS 8
 #define SG_MAX_STAGES 4
 #define SG_SMEM (224 * 1024)
+
+// What a row of an operand has in the part of k that a block cuts.
+#define SG_TINY 1                // entries below 2^-109, which are not cut exactly
+#define SG_SMALL 2               // entries below 2^-63, whose products may be below the smallest float
+#define SG_LARGE 4               // entries of 2^20 or more
+#define SG_ENTRIES 8             // entries that are not zero
 
 struct SgemmArgs {
   const float* x;
@@ -88,15 +101,45 @@ __device__ __forceinline__ void sg_store4(uint32_t at, uint4 v) {
   asm volatile("st.shared.v4.b32 [%0], {%1, %2, %3, %4};" ::"r"(at), "r"(v.x), "r"(v.y), "r"(v.z), "r"(v.w) : "memory");
 }
 
+// The smallest of `least` and the magnitudes of eight entries that are not zero, as twice its bits less one (a zero's are the largest
+// number there is).
+__device__ __forceinline__ uint32_t sg_least(uint32_t least, const float4 (&v)[2]) {
+  auto of = [](float a) { return 2u * __float_as_uint(a) - 1u; };
+  least = __vimin3_u32(least, of(v[0].x), of(v[0].y));
+  least = __vimin3_u32(least, of(v[0].z), of(v[0].w));
+  least = __vimin3_u32(least, of(v[1].x), of(v[1].y));
+  return __vimin3_u32(least, of(v[1].z), of(v[1].w));
+}
+#define SG_LEAST(e) (2u * ((127u - (e)) << 23) - 1u)      // of 2^-e
+
+// What one entry has.
+__device__ __forceinline__ uint32_t sg_note(float a) {
+  a = fabsf(a);
+  return a == 0.f ? 0u : SG_ENTRIES | (a < 0x1p-63f ? SG_SMALL : 0) | (a < 0x1p-109f ? SG_TINY : 0) | (a >= 0x1p20f ? SG_LARGE : 0);
+}
+
 __device__ __forceinline__ bool sg_again(float v) {
   const float a = fabsf(v);
   return !(a < INFINITY) || (a < 0x1p-80f && a != 0.f);
 }
+// Whether what the cut lost, or products below the smallest float, may show in a sum of rows that have `x` and `w`.
+__device__ __forceinline__ bool sg_cut_short(uint32_t x, uint32_t w) {
+  return ((x & SG_TINY) && (w & SG_LARGE)) || ((w & SG_TINY) && (x & SG_LARGE));
+}
+__device__ __forceinline__ bool sg_vanished(uint32_t x, uint32_t w) { return ((x | w) & SG_SMALL) && (x & w & SG_ENTRIES); }
 
 __device__ __noinline__ float sg_chain(const float* x, const float* w, int k_dim) {
   float sum = 0.f;
   for (int k = 0; k < k_dim; ++k) sum = fmaf(x[k], w[k], sum);
   return sum;
+}
+
+// A word of the same shared variable in block `rank` of the cluster.
+__device__ __forceinline__ uint32_t sg_remote(const void* at, int rank) {
+  uint32_t v;
+  asm volatile("{\n\t.reg .b32 a;\n\tmapa.shared::cluster.u32 a, %1, %2;\n\tld.shared::cluster.u32 %0, [a];\n\t}"
+               : "=r"(v) : "r"(smem_u32(at)), "r"(rank) : "memory");
+  return v;
 }
 
 // VEC: rows of x and w may be read in 16-byte pieces.
@@ -106,7 +149,9 @@ __global__ void __launch_bounds__(SG_THREADS, 1) sgemm_tcgen05_kernel(const Sgem
   const uint32_t smem = (smem_u32(sgemm_smem) + 1023) & ~1023u;
   __shared__ uint64_t full_bar[SG_MAX_STAGES], empty_bar[SG_MAX_STAGES], sum_full[2], sum_empty[2], done_bar;
   __shared__ uint32_t tmem_holder;
-  __shared__ int abort_flag;
+  __shared__ __align__(16) uint32_t notes[SG_W + SG_X];      // what the rows of w, then of x, have in this block's part of k
+  __shared__ uint32_t noted;                 // what any row of w has, and any of x above it (0: nothing is noted, nothing is small)
+  __shared__ int abort_flag, small_flag;
 
   const int stages = args.stages, cols = args.tile_rows, k_dim = args.k_dim;
   const int x_plane = cols * SG_K * 2;
@@ -125,7 +170,8 @@ __global__ void __launch_bounds__(SG_THREADS, 1) sgemm_tcgen05_kernel(const Sgem
     for (int s = 0; s < stages; ++s) { mbar_init(&full_bar[s], SG_CUTTERS); mbar_init(&empty_bar[s], 2); }
     for (int b = 0; b < 2; ++b) { mbar_init(&sum_full[b], 1); mbar_init(&sum_empty[b], SG_DRAINERS); }
     mbar_init(&done_bar, 2);
-    abort_flag = 0;
+    abort_flag = small_flag = 0;
+    noted = 0;
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
   pdl_trigger();
@@ -164,6 +210,7 @@ __global__ void __launch_bounds__(SG_THREADS, 1) sgemm_tcgen05_kernel(const Sgem
       for (int j = 0; j < SG_X / 32; ++j)
         if (j < x_steps) read(args.x, m_base + row + 32 * j, args.rows, (kb_begin + i) * SG_K, xv[j]);
     };
+    uint32_t least = 0xffffffffu;
     auto file = [&](uint32_t plane, int plane_bytes, int r, const float4 (&v)[2]) {
       uint4 hi, mid, low;
       sg_cut(v[0].x, v[0].y, hi.x, mid.x, low.x);
@@ -186,10 +233,16 @@ __global__ void __launch_bounds__(SG_THREADS, 1) sgemm_tcgen05_kernel(const Sgem
       if (!__all_sync(0xffffffffu, mbar_wait(&empty_bar[s], parity, abort))) break;
       const uint32_t stage = smem + s * stage_bytes;
 #pragma unroll
-      for (int j = 0; j < SG_W / 32; ++j) file(stage, SG_W_PLANE, row + 32 * j, wv[j]);
+      for (int j = 0; j < SG_W / 32; ++j) {
+        least = sg_least(least, wv[j]);
+        file(stage, SG_W_PLANE, row + 32 * j, wv[j]);
+      }
 #pragma unroll
       for (int j = 0; j < SG_X / 32; ++j)
-        if (row + 32 * j < cols) file(stage + 3 * SG_W_PLANE, x_plane, row + 32 * j, xv[j]);
+        if (row + 32 * j < cols) {
+          least = sg_least(least, xv[j]);
+          file(stage + 3 * SG_W_PLANE, x_plane, row + 32 * j, xv[j]);
+        }
       asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
       __syncwarp();
       if (lane == 0) asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(smem_u32(&full_bar[s])) : "memory");
@@ -199,6 +252,35 @@ __global__ void __launch_bounds__(SG_THREADS, 1) sgemm_tcgen05_kernel(const Sgem
       }
       if (++s == stages) { s = 0; parity ^= 1; }
     }
+    if (least < SG_LEAST(63)) atomicMax(&small_flag, least < SG_LEAST(109) ? 2 : 1);
+    asm volatile("barrier.sync 2, %0;" ::"n"(32 * SG_CUTTERS) : "memory");
+    const int small = *(volatile int*)&small_flag;
+    if (small) {
+      const int k0 = kb_begin * SG_K, k1 = min((kb_begin + n_kb) * SG_K, k_dim);
+      for (int r = row; r < SG_W + cols; r += 32) {                   // (whole warps: four rows, eight lanes each)
+        const float* at = r < SG_W ? args.w + (size_t)min(n_base + r, args.n_out - 1) * k_dim
+                                   : args.x + (size_t)min(m_base + r - SG_W, args.rows - 1) * k_dim;
+        uint32_t has = small == 1 ? SG_SMALL : 0u;                    // (which rows have them is not looked for)
+        for (int k = k0; k < k1; k += 64) {
+          float e[8];
+#pragma unroll
+          for (int j = 0; j < 8; ++j) e[j] = k + 8 * j + piece < k1 ? __ldg(at + k + 8 * j + piece) : 0.f;
+#pragma unroll
+          for (int j = 0; j < 8; ++j) has |= sg_note(e[j]);
+          if (small == 1) {
+            const uint32_t found = __ballot_sync(0xffffffffu, has & SG_ENTRIES);
+            if ((found & 0xffu) && (found & 0xff00u) && (found & 0xff0000u) && (found & 0xff000000u)) break;
+          }
+        }
+#pragma unroll
+        for (int o = 1; o < 8; o <<= 1) has |= __shfl_xor_sync(0xffffffffu, has, o);
+        if (piece == 0) {
+          notes[r] = has;
+          atomicOr(&noted, r < SG_W ? has : has << 4);
+        }
+      }
+    }
+    if (args.parts == 1) asm volatile("barrier.sync 1, %0;" ::"n"(SG_THREADS) : "memory");      // (of a cluster: below)
   } else {
     // ---------------- add up the accumulators: a lane has one row of w, its columns are rows of x.  Two of these warps also
     // issue the MMAs, each those of one accumulator (together, one elected lane), before they empty the other: issuing
@@ -276,6 +358,7 @@ __global__ void __launch_bounds__(SG_THREADS, 1) sgemm_tcgen05_kernel(const Sgem
       const uint64_t start = now_ns();
       while (!mbar_try(&done_bar, 0) && now_ns() - start < TC_WAIT_LIMIT_NS) {}
     }
+    if (args.parts == 1) asm volatile("barrier.sync 1, %0;" ::"n"(SG_THREADS) : "memory");      // the notes are there
     pdl_wait();                              // before the first store: an earlier kernel may still read y's memory
     const int n = n_base + r;
     if (args.parts > 1) {
@@ -296,7 +379,9 @@ __global__ void __launch_bounds__(SG_THREADS, 1) sgemm_tcgen05_kernel(const Sgem
           const int m = 32 * j + 16 * half + c;
           if (m < rows_here) args.y[(size_t)(m_base + m) * args.n_out + n] = sum[j][c];
         }
-      bool again = false;
+      const uint32_t any = *(volatile uint32_t*)&noted;
+      const bool lost = sg_cut_short(any >> 4, any), vanished = sg_vanished(any >> 4, any);      // (may be)
+      bool again = lost || vanished;
 #pragma unroll
       for (int j = 0; j < SG_X / 32; ++j)
 #pragma unroll
@@ -305,7 +390,9 @@ __global__ void __launch_bounds__(SG_THREADS, 1) sgemm_tcgen05_kernel(const Sgem
 #pragma unroll 1
         for (int m = 16 * half; m < rows_here; m += m % 16 == 15 ? 17 : 1) {
           float* at = args.y + (size_t)(m_base + m) * args.n_out + n;
-          if (sg_again(*at)) *at = sg_chain(args.x + (size_t)(m_base + m) * k_dim, args.w + (size_t)n * k_dim, k_dim);
+          if (sg_again(*at) || (lost && sg_cut_short(notes[SG_W + m], notes[r])) ||
+              (vanished && *at == 0.f && sg_vanished(notes[SG_W + m], notes[r])))
+            *at = sg_chain(args.x + (size_t)(m_base + m) * k_dim, args.w + (size_t)n * k_dim, k_dim);
         }
     }
   }
@@ -316,11 +403,28 @@ __global__ void __launch_bounds__(SG_THREADS, 1) sgemm_tcgen05_kernel(const Sgem
       const bool vector_store = args.n_out % 4 == 0;
       const int n_items = rows_here * (SG_W / 4);
       uint32_t base[SG_MAX_PARTS];
+      bool lost = false, vanished = false;   // (may be, in some part)
 #pragma unroll
       for (int p = 0; p < SG_MAX_PARTS; ++p) {
         base[p] = 0;
-        if (p < args.parts) asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(base[p]) : "r"(smem), "r"(p));
+        if (p < args.parts) {
+          asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(base[p]) : "r"(smem), "r"(p));
+          const uint32_t any = sg_remote(&noted, p);
+          lost |= sg_cut_short(any >> 4, any);
+          vanished |= sg_vanished(any >> 4, any);
+        }
       }
+      // the same of the result `v` of row m of x and row r of w
+      auto short_of = [&](float v, int m, int r) -> bool {
+        bool again = false;
+#pragma unroll 1
+        for (int p = 0; p < args.parts; ++p) {
+          if (sg_remote(&noted, p) == 0) continue;
+          const uint32_t x_has = sg_remote(&notes[SG_W + m], p), w_has = sg_remote(&notes[r], p);
+          again |= sg_cut_short(x_has, w_has) || (v == 0.f && sg_vanished(x_has, w_has));
+        }
+        return again;
+      };
       // an item: four neighbouring results; the loads of all parts are in flight together and are added in order
       for (int item = part * SG_THREADS + threadIdx.x; item < n_items; item += args.parts * SG_THREADS) {
         const int m = item >> 5, c = (item & 31) * 4, n = n_base + c;
@@ -336,7 +440,7 @@ __global__ void __launch_bounds__(SG_THREADS, 1) sgemm_tcgen05_kernel(const Sgem
           if (p < args.parts) { e[0] += v[p].x; e[1] += v[p].y; e[2] += v[p].z; e[3] += v[p].w; }
 #pragma unroll
         for (int j = 0; j < 4; ++j)
-          if (sg_again(e[j]) && n + j < args.n_out)
+          if (n + j < args.n_out && (sg_again(e[j]) || ((lost || (vanished && e[j] == 0.f)) && short_of(e[j], m, c + j))))
             e[j] = sg_chain(args.x + (size_t)(m_base + m) * k_dim, args.w + (size_t)(n + j) * k_dim, k_dim);
         float* to = args.y + (size_t)(m_base + m) * args.n_out + n;
         if (vector_store) {

@@ -142,7 +142,6 @@ def test_float32_product_of_values_that_cannot_be_cut(k):
     from starter_b200 import ops
 
     x, w = rand(20, k, seed=3), rand(130, k, seed=4)
-    want = ops.linear(dev(x), dev(w)).cpu()
     x[2, 7], x[3, k - 1], x[4, 5], x[5] = float("inf"), float("-inf"), float("nan"), 0.0
     x[5, 9], w[:, 9] = 3.4e38, w[:, 9].clamp(-0.9, 0.9)
     x[6] *= 1e-36
@@ -152,7 +151,25 @@ def test_float32_product_of_values_that_cannot_be_cut(k):
     bound = (k + 8) * 2.0 ** -24 * (x.double().abs() @ w.double().abs().t()) + k * 2.0 ** -149
     assert bool(((got.double() - exact).abs()[5:7] <= bound[5:7]).all())
     kept = ops.linear(dev(x[7:].contiguous().repeat(2, 1)), dev(w)).cpu()
-    assert torch.equal(got[7:], kept[:13]) and want.shape == got.shape
+    assert torch.equal(got[7:], kept[:13])
+
+
+@pytest.mark.parametrize("rows,n,k", [(40, 130, 100), (40, 130, 1030), (170, 260, 1024), (330, 5000, 128)])
+def test_float32_product_of_small_values_times_large_ones(rows, n, k):
+    """Operands whose pieces of 8 bits are below the smallest bfloat16, of either side, times ordinary and large ones, single small
+    entries among ordinary ones and products below the smallest float: the bound of a chain of k products."""
+    from starter_b200 import ops
+
+    x, w = rand(rows, k, seed=rows), rand(n, k, seed=n + 1)
+    for i, e in enumerate((-100, -110, -116, -121, -127, -136, -70, 56, 30, 19)):
+        x[i] *= 2.0 ** e
+        w[3 * i] *= 2.0 ** e
+    x[10], w[1] = 0.0, 0.0
+    x[11, 2::7], w[2, 5::7] = x[4, 2::7], w[12, 5::7]
+    x[12, k - 1], w[4] = x[4, 0], w[21]
+    got = ops.linear(dev(x), dev(w)).cpu().double()
+    bound = (k + 8) * 2.0 ** -24 * (x.double().abs() @ w.double().abs().t()) + k * 2.0 ** -149
+    assert bool(((got - x.double() @ w.double().t()).abs() <= bound).all())
 
 
 @pytest.mark.parametrize("dtype", list(DT))
