@@ -1650,8 +1650,12 @@ def latent_attention_step(qa, store, block_table, ctx, heads, rank, rot, scale, 
 #: tokens that every sequence of a step must bring for the latent attention to form keys and values (see
 #: ``latent_attention_prompt``), and the most cache rows it forms them for.  Forming a row costs a head 2 * 256 * 512
 #: products, a query saves it about 1,500 a row at a third of the speed: from about 25 tokens on it pays, whatever the
-#: rows; 65,536 rows bound the memory (8 KB a row with 16 heads of 128 + 128)
+#: rows
 LATENT_PROMPT_TOKENS, LATENT_PROMPT_ROWS = 32, 65536
+#: what the formed keys, values and gathered rows of a step may take in bytes where they take more than the folded queries and summed
+#: latents of the kernel that scores the latents (a prompt of many heads over its own tokens alone takes a quarter of those; a portion
+#: behind a long cache more): 65,536 rows of 16 heads of 128 + 128 over a latent of 512 take 612 MB
+LATENT_PROMPT_BYTES = 640 << 20
 
 
 def _latent_prompt_rows(ctx, window):
@@ -1663,16 +1667,20 @@ def _latent_prompt_rows(ctx, window):
     return (rows + 63) // 64 * 64
 
 
-def latent_prompt_takes(dtype, ctx, dim, rot, vdim, rank, scale, window=None) -> bool:
+def latent_prompt_takes(dtype, ctx, dim, rot, vdim, rank, scale, window=None, heads=1) -> bool:
     """Whether ``latent_attention_prompt`` serves this step: bfloat16, plain keys and values of 64 or 128 entries and a rotated
     part of 64, every sequence bringing at least ``LATENT_PROMPT_TOKENS`` tokens (known on the host), and no more than
-    ``LATENT_PROMPT_ROWS`` rows to form keys and values for."""
+    ``LATENT_PROMPT_ROWS`` rows to form keys and values for, which with ``heads`` heads take no more than
+    ``LATENT_PROMPT_BYTES`` or than the other kernel's buffers."""
     if dtype != torch.bfloat16 or ctx.host is None or ctx.block_seq is None or not scale > 0:
         return False
     if dim not in (64, 128) or vdim not in (64, 128) or rot != 64 or rank % 16 or rank + rot > 640:
         return False
-    return (int(ctx.host["seq_q_len"].min()) >= LATENT_PROMPT_TOKENS
-            and int(_latent_prompt_rows(ctx, window).sum()) <= LATENT_PROMPT_ROWS)
+    if int(ctx.host["seq_q_len"].min()) < LATENT_PROMPT_TOKENS:
+        return False
+    rows = int(_latent_prompt_rows(ctx, window).sum())
+    scored = 2 * int(ctx.host["seq_q_len"].sum()) * heads * (2 * rank + rot)
+    return rows <= LATENT_PROMPT_ROWS and 2 * rows * (heads * (dim + vdim) + rank + rot) <= max(LATENT_PROMPT_BYTES, scored)
 
 
 def latent_attention_prompt(q, ukv, store, block_table, ctx, heads, dim, vdim, rank, rot, scale, window=None, sink=None):

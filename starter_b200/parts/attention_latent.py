@@ -103,7 +103,8 @@ class LatentAttention(Part):
                                 write_cache=writes_cache, layout=rotation.layout, kv_col=self.kv_at)
         q = ops.linear(cq, self.uq, status=ctx.status)
         n = q.shape[0]
-        if ops.latent_prompt_takes(q.dtype, ctx, s.head_dim, s.rot_dim, s.value_dim, s.kv_rank, s.scale, s.window):
+        if ops.latent_prompt_takes(q.dtype, ctx, s.head_dim, s.rot_dim, s.value_dim, s.kv_rank, s.scale, s.window,
+                                   s.num_heads):
             ops.latent_rotate_q(q, q.view(n, s.num_heads, -1), cos, sin, ctx.tok_pos, s.num_heads, s.head_dim, s.rot_dim,
                                 s.position.dims, s.head_dim, layout=rotation.layout)
             a = ops.latent_attention_prompt(q, self.ukv, store, cache.block_table, ctx, s.num_heads, s.head_dim, s.value_dim,

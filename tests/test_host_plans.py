@@ -113,3 +113,23 @@ def test_every_entry_point_the_operations_call_has_declared_arguments():
     result, types = known["sb_sgemm_nt"]
     assert result is ctypes.c_int
     assert types == [ctypes.c_void_p] * 3 + [ctypes.c_int] * 3 + [ctypes.c_void_p] * 2
+
+
+@pytest.mark.parametrize("heads, past, new, window, takes", [
+    (16, 65000, 64, None, True), (128, 0, 10000, None, True), (128, 0, 30000, None, True), (128, 20000, 64, None, False),
+    (128, 9000, 64, None, True), (128, 65000, 64, 4096, True), (128, 65000, 15000, None, False), (128, 65000, 20000, None, False),
+    (16, 65537, 64, None, False)])
+def test_formed_keys_are_bounded_in_bytes(heads, past, new, window, takes):
+    """Beyond the fixed bound they take no more than what the kernel that scores the latents would need."""
+    from types import SimpleNamespace
+
+    import torch
+
+    from starter_b200 import ops
+
+    ctx = SimpleNamespace(host={"seq_q_len": np.array([new]), "seq_kv_len": np.array([past + new])}, block_seq=torch.zeros(1))
+    got = ops.latent_prompt_takes(torch.bfloat16, ctx, 128, 64, 128, 512, 0.1, window, heads)
+    assert got is takes
+    if got:
+        rows = min(past + new, new + (window or past) - 1) + 64
+        assert 2 * rows * (heads * 256 + 576) <= max(ops.LATENT_PROMPT_BYTES, 2 * new * heads * 1088) + 64 * 2 * (heads * 256 + 576)
