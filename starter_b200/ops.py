@@ -2382,6 +2382,9 @@ SCAN_MODES = {"state_space": 0, "gated_delta": 1, "forget_write": 2, "channel_de
 #: sequences of 64 tokens take 27 to 47 us there against 60 to 79 us on the kernel for few tokens, one of 2,048 takes 102 to
 #: 177 us against 400 to 673; below, the launch that forms the coefficients or gates beforehand (5 us) is not earned back.
 SCAN_PROMPT_TOKENS = 64
+#: the most bytes of scratch these kernels may take in a step (the kernel for few tokens needs none, and serves what would
+#: take more): 16 KB a token with 16 heads of 128 rows in the forget-write recurrence, so 65,536 tokens; 2 KB in the others
+SCAN_PROMPT_BYTES = 1 << 30
 
 
 def scan_max_state() -> int:
@@ -2439,7 +2442,7 @@ def state_scan(mode, q, k, v, a_raw, b_raw, A_log, dt_bias, skip, state, state_a
     if dtype == torch.bfloat16 and n_tokens >= SCAN_PROMPT_TOKENS * n_seqs and 64 < n_state <= 128:
         lib = _lib("state_scan_prompt")
         floats = lib.sb_scan_prompt_floats(1, SCAN_MODES[mode], *args[:6], _ptr(decay), heads, groups, n_state, v_dim)
-        if floats >= 0:
+        if 0 <= 4 * floats * n_tokens <= SCAN_PROMPT_BYTES:
             scratch = state.new_empty((n_tokens, floats), dtype=torch.float32) if floats else None
             rc = lib.sb_state_scan_prompt(
                 SCAN_MODES[mode], *args, _ptr(A_log), _ptr(dt_bias), _ptr(skip), _ptr(decay), _at(state, state_at),

@@ -154,3 +154,29 @@ def test_more_tokens_than_a_grid_counts_in_its_second_dimension(mode, monkeypatc
     for got, want in zip(*outs):
         # (the bound of the comparison above: the state forgets within some ten tokens)
         assert float((got - want).abs().max()) <= 2e-5 * float(want.abs().max())
+
+
+@pytest.mark.parametrize("mode, floats", [("state_space", 20), ("gated_delta", 36), ("forget_write", 2 * 72)])
+def test_scratch_is_bounded(mode, floats, monkeypatch):
+    """A step whose scratch would take more bytes than are allowed is served by the kernel for few tokens."""
+    from starter_b200 import ops
+
+    heads, n, width, tokens = 2, 72, 8, 70
+    gen = torch.Generator().manual_seed(4)
+    q, k, v, ab = (torch.randn(tokens, heads * size, generator=gen).to(BF).cuda() for size in (n, n, width, 2))
+    per = heads * n if mode == "forget_write" else heads
+    A, bias = torch.full((per,), 0.3).cuda(), torch.zeros(per).cuda()
+
+    def run():
+        state = torch.zeros(1, heads * n * width, device="cuda")
+        return ops.state_scan(mode, (q, 0), (k, 0), (v, 0), (ab, 0) if mode != "forget_write" else None,
+                              (ab, heads) if mode == "gated_delta" else None, A, bias, bias if mode == "state_space" else None, state, 0,
+                              *packed([tokens], [0]), heads, heads, n, width)
+
+    many = run()
+    monkeypatch.setattr(ops, "SCAN_PROMPT_BYTES", 4 * floats * heads * tokens)
+    assert torch.equal(run(), many)
+    monkeypatch.setattr(ops, "SCAN_PROMPT_BYTES", 4 * floats * heads * tokens - 1)
+    few = run()
+    monkeypatch.setattr(ops, "SCAN_PROMPT_TOKENS", 1 << 30)
+    assert torch.equal(few, run()) and not torch.equal(few, many)
