@@ -16,7 +16,9 @@
 //
 // A layer of width 2048, 16 heads of 128 + 64 over a latent of 512, 2,048 tokens: 517 us a pass with the kernel that scores the latents
 // (417 of them in it, mma.sync at 0.11 of the tensor peak; two products of 11 us around it), 156 with these.  The error against
-// 64 bits is the same (0.0047: keys and values are rounded here, folded queries and summed latents there).
+// 64 bits is no larger (keys and values are rounded here, folded queries and summed latents there): 0.00470 against 0.00473 at
+// that size, 0.00463 against 0.00464 for four sequences of up to 450 tokens, 0.00482 against 0.00489 for 300 tokens behind 900 (means of
+// three seeds; 0.00477, 0.00471 and 0.00482 while the weights were summed before their rounding and relative to the sink).
 //
 // Gathered rows: a sequence's keys from the first that any of its queries sees, padded to a multiple of 64 with zeros, so
 // that a step never reads another sequence's values (their weights are zero, but 0 * inf would not be).
@@ -241,10 +243,6 @@ latent_prompt_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_con
     uint8_t* p_row = p_sm + t * P_BYTES + r * 128;
     const int n_mine = n_tile[t];
     float m_ref = -INFINITY, l_run = 0.f;
-    if (sink) {                                     // the state a row's softmax starts from
-      m_ref = sink[head] * 1.4426950408889634f;
-      l_run = 1.f;
-    }
     const int row_first = window > 0 ? pos - window + 1 : 0;
     pdl_wait();
     bool ok = true;
@@ -300,10 +298,10 @@ latent_prompt_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_con
       for (int e = 0; e < 32; ++e) {
         float x0, x1;
         fma2(x0, x1, sv[2 * e], sv[2 * e + 1], scale_log2, -m_use);
-        const float p0 = fast_exp2(x0), p1 = fast_exp2(x1);
-        add2(rs, rs_hi, p0, p1);
-        __nv_bfloat162 two = __floats2bfloat162_rn(p0, p1);
+        __nv_bfloat162 two = __floats2bfloat162_rn(fast_exp2(x0), fast_exp2(x1));
         pk[e] = *reinterpret_cast<uint32_t*>(&two);
+        // (the sum is of the weights as they multiply the values, so that their roundings cancel where one key has most of the weight)
+        add2(rs, rs_hi, __uint_as_float(pk[e] << 16), __uint_as_float(pk[e] & 0xffff0000u));
       }
       // P's tile is free once PV of the step before has finished
       if (i > 0) ok = mbar_wait(&o_ready[t], (i - 1) & 1, abort);
@@ -322,7 +320,12 @@ latent_prompt_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_con
     if (ok && n_mine > 0) {
       asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
       const bool valid = t * TC_BQ + r < rows_valid;
-      const float inv = 1.f / l_run;
+      // the sink joins at the end, so that the weights are relative to a key's score: the largest of the first step is one exactly
+      float inv = 1.f / l_run;
+      if (sink) {
+        const float own = sink[head] * 1.4426950408889634f, top = fmaxf(m_ref, own), f = fast_exp2(m_ref - top);
+        inv = f / (l_run * f + fast_exp2(own - top));
+      }
       bf16* dst = out + ((size_t)seq_q_start[seq] + q_first + t * TC_BQ + r) * ((size_t)heads * (VC * 64)) + (size_t)head * (VC * 64);
 #pragma unroll 1
       for (int c = 0; c < VC * 64; c += 32) {

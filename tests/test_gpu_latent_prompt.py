@@ -72,6 +72,28 @@ def test_formed_keys_and_values(dim, vdim, rank, heads, window, sink, past, new)
     assert float(off.abs().max()) < 0.05 * float(want.abs().max())
 
 
+def test_a_weight_is_rounded_no_more_than_once():
+    """Each token sees itself and the sink; keys and values come out of their product unrounded.  What is left is the
+    rounding of the output: the weight's own cancels, since the weights' sum has it too."""
+    from starter_b200 import ops
+
+    heads, dim, rank, rot, tokens, gen = 2, 64, 128, 64, 300, torch.Generator().manual_seed(2)
+    pick = torch.eye(rank, dtype=BF)
+    ukv = torch.cat([pick[:dim], pick[:dim], pick[dim:], pick[dim:]])
+    rows = torch.randn(tokens, rank + rot, generator=gen).to(BF)
+    q = torch.randn(tokens, heads, dim + rot, generator=gen).to(BF)
+    store = torch.zeros(5, 1, 64, rank + rot, dtype=BF)
+    store.view(-1, rank + rot)[:tokens] = rows
+    sinks = torch.tensor([0.3, -1.7])
+    ctx = context([0], [tokens], [0])
+    got = ops.latent_attention_prompt(q.flatten(1).cuda(), ukv.cuda(), store.cuda(), torch.arange(5, dtype=torch.int32)[None].cuda(), ctx,
+                                      heads, dim, dim, rank, rot, 0.125, 1, sinks.cuda()).cpu().double().view(tokens, heads, dim)
+    r = rows.double()
+    score = torch.einsum("thd,td->th", q.double(), torch.cat([r[:, :dim], r[:, rank:]], dim=1)) * 0.125
+    want = torch.sigmoid(score - sinks.double())[:, :, None] * r[:, None, dim:rank]
+    assert bool(((got - want).abs() <= 1.01 * 2.0 ** -8 * want.abs()).all())
+
+
 @pytest.mark.parametrize("window,layout,gate", [(None, "interleaved", True), (90, "half_split", False)])
 def test_the_layer_on_either_kernel(window, layout, gate, monkeypatch):
     from starter_b200 import ops
