@@ -827,8 +827,12 @@ moe_few_kernel(const bf16* __restrict__ x, const bf16* __restrict__ w, bf16* __r
       for (int a = 0; a < NW; ++a) {
         const uint4 u = wv[i][a][0], v = wv[i][a][1];
         const uint32_t lo[4] = {u.x, v.x, u.y, v.y}, hi[4] = {u.z, v.z, u.w, v.w};
-        moe_mma(acc[a], lo, xv[i].x, xv[i].y);
-        moe_mma(acc[a], hi, xv[i].z, xv[i].w);
+        // (a step's own sum, joined by rounded additions: the tensor cores cut what they add to an accumulator)
+        float step[4] = {0.f, 0.f, 0.f, 0.f};
+        moe_mma(step, lo, xv[i].x, xv[i].y);
+        moe_mma(step, hi, xv[i].z, xv[i].w);
+#pragma unroll
+        for (int c = 0; c < 4; ++c) acc[a][c] += step[c];
       }
   }
 #pragma unroll

@@ -655,3 +655,26 @@ def test_attention_prefill_many_tokens_per_sequence(heads, kv_heads, d, window, 
                                       c["scale"], window, status=status, kernel=kernel,
                                       blocks=(ints([b[0] for b in blocks]), ints([b[1] for b in blocks])))
         assert torch.equal(again, got) and status.item() == 0
+
+
+@pytest.mark.parametrize("rows", [1, 6])
+def test_few_rows_of_an_expert_are_summed_with_rounding(rows):
+    """Entries of three quarters of the last place of a float sum of 257, which lies between two bfloat16 numbers: cut off they
+    would leave 256, rounded each counts."""
+    from starter_b200 import ops
+
+    pattern = torch.zeros(2048)
+    pattern[0], pattern[1], pattern[128::128] = 256.0, 1.0, 3 * 2.0 ** -17
+    ids, weights = dev(torch.zeros(rows, 1, dtype=torch.int32)), dev(torch.ones(rows, 1))
+
+    def run(h, up, down):
+        h, up, down = (dev(t.to(torch.bfloat16)) for t in (h, up, down))
+        return ops.moe_experts(h, ids, weights, up, down, expert="relu2", tile_rows=8).cpu().float()
+
+    first = torch.zeros(1, 2048, 64)
+    first[:, :, 0] = 1.0
+    ones = torch.zeros(rows, 64)
+    ones[:, 0] = 1.0
+    assert bool((run(ones, first, pattern.expand(1, 64, 2048)) == 258.0).all())
+    # (the square of 258 as a bfloat16 number)
+    assert bool((run(torch.ones(rows, 2048), pattern.expand(1, 64, 2048), torch.eye(2048, 64)[None])[:, :64] == 66560.0).all())
