@@ -352,7 +352,10 @@ gemm_prompt_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_const
           for (int j = 0; j < 32; ++j) {
             const float gr = rnd<bf16>(v[j]), ur = rnd<bf16>(u[j]);
             if (args.gated == SB_ACT_CLAMPED) v[j] = gate_clamped(gr, ur, args.limit);
-            else v[j] = rnd<bf16>(gate_act_fast(gr, args.gated)) * ur;
+            else if (args.gated == SB_ACT_GELU_TANH) v[j] = rnd<bf16>(gate_act_fast(gr, SB_ACT_GELU_TANH)) * ur;
+            // (both sides by a quarter: the fast quotient is zero for divisors above 2^126, which gates of -87.5 to -88.5 have; so
+            // every bfloat16 gate gives what the exact quotient gives)
+            else v[j] = rnd<bf16>(__fdividef(0.25f * gr, fmaf(0.25f, __expf(-gr), 0.25f))) * ur;
           }
         } else {
           pg_tmem_load32(acc + c * 32, v);

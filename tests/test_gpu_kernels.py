@@ -594,6 +594,21 @@ def test_linear_sends_each_row_count_to_its_kernel(monkeypatch):
         assert torch.allclose(got.cpu().double(), x.double() @ w.double().t(), atol=2e-2, rtol=2e-2)
 
 
+def test_the_prompt_product_gates_every_value():
+    """Every finite bfloat16 gate, times one: silu rounded once, down to where its exponential leaves the float range."""
+    from starter_b200 import ops
+
+    gates = torch.arange(65536, dtype=torch.int32).to(torch.int16).view(torch.bfloat16)
+    gates = torch.where(gates.isfinite(), gates, torch.zeros_like(gates)).view(1024, 64)
+    x, w = torch.zeros(1024, 128), torch.zeros(256, 128)
+    x[:, :64], x[:, 64] = gates.float(), 1.0
+    w[:64, :64], w[128:192, 64] = torch.eye(64), 1.0
+    got = ops.linear_prompt(dev(x.to(torch.bfloat16)), dev(w.to(torch.bfloat16)), gated=True)[:, :64].cpu()
+    v = gates.double()
+    want = torch.where(v < -88.6, torch.zeros_like(v), v * torch.sigmoid(v)).to(torch.bfloat16)
+    assert bool(((got == want) | (v < -88.6) & (got.double().abs() < 2e-37)).all())
+
+
 @pytest.mark.parametrize("rows,n,k,gated,kblock", [(256, 256, 512, False, 0), (600, 384, 1024, True, 3)])
 def test_a_wait_in_the_prompt_product_that_runs_out_is_reported(rows, n, k, gated, kblock):
     """One weight copy of every first CTA is left out on purpose (an entry point made for this): the
