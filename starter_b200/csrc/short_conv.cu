@@ -101,8 +101,10 @@ short_conv_kernel(const T* __restrict__ x, int ldx, const float* __restrict__ ta
 // The same for bfloat16 channels in 8-byte pieces and up to four taps: a thread four channels and a chunk of 8 tokens, all of whose
 // loads are in flight together (no condition between them and the sums, or the compiler moves each load to its use), K
 // multiply-adds an entry (the kernel above always has eight, two bytes a load, and an exact quotient that branches for every
-// value; results are rounded to bfloat16 at once, so silu takes the fast quotient).  A sum's terms come in the
-// same order.  2,136 tokens of 4,096 channels with silu: 28 -> 20 us; 2,048 of 2,304: 18 -> 13; of 3,072 without: 20 -> 10.
+// value).  A sum's terms come in the same order.  silu has the same exponential and the fast quotient, of both sides by a quarter, since
+// that is zero for divisors above 2^126: of 8.4 million results 234 are not the exact value's nearest bfloat16, 231 with the exact
+// quotient (the error of all is 0.00167215 with both), which takes 4 us more.  With caches flushed, 2,136 tokens of 4,096 channels with silu:
+// 33 -> 25 us; 2,048 of 2,304: 22 -> 18; of 3,072 without: 25 -> 14.
 #define CONV_VEC_CHUNK 8
 __device__ __forceinline__ void conv_unpack4(const uint2& v, float* f) {
   f[0] = __uint_as_float(v.x << 16);
@@ -172,7 +174,7 @@ short_conv_vec_kernel(const bf16* __restrict__ x, int ldx, const float* __restri
     }
     if (act == 1) {
 #pragma unroll
-      for (int e = 0; e < 4; ++e) a[e] = gate_act_fast(a[e], SB_ACT_SILU);
+      for (int e = 0; e < 4; ++e) a[e] = __fdividef(0.25f * a[e], fmaf(0.25f, expf(-a[e]), 0.25f));
     }
     if (t0 + i < q_len) {
       uint2 o;

@@ -693,3 +693,16 @@ def test_few_rows_of_an_expert_are_summed_with_rounding(rows):
     assert bool((run(ones, first, pattern.expand(1, 64, 2048)) == 258.0).all())
     # (the square of 258 as a bfloat16 number)
     assert bool((run(torch.ones(rows, 2048), pattern.expand(1, 64, 2048), torch.eye(2048, 64)[None])[:, :64] == 66560.0).all())
+
+
+def test_the_short_convolution_gates_every_value():
+    """Every finite bfloat16 number through one tap of one: silu rounded once, down to where its exponential leaves the float range."""
+    from starter_b200 import ops
+
+    x = torch.arange(65536, dtype=torch.int32).to(torch.int16).view(torch.bfloat16)
+    x = torch.where(x.isfinite(), x, torch.zeros_like(x)).view(1024, 64)
+    ints = [torch.tensor(v, dtype=torch.int32, device="cuda") for v in ([0], [0], [1024])]
+    got = ops.short_conv(dev(x), 0, 64, torch.ones(64, 1, device="cuda"), None, None, None, 0, *ints, 1024, "silu").cpu()
+    v = x.double()
+    want = torch.where(v < -88.6, torch.zeros_like(v), v * torch.sigmoid(v)).to(torch.bfloat16)
+    assert bool(((got == want) | (v < -88.6) & (got.double().abs() < 2e-37)).all())
