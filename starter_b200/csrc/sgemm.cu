@@ -57,6 +57,8 @@ struct SgemmArgs {
   float* y;
   int* status;
   int rows, n_out, k_dim, tile_rows, parts, stages;
+  int withhold;                    // >= 0: the first cutter does not hand over this slice (tests of the give-up path)
+  unsigned long long wait_limit_ns;
 };
 
 // 16 columns of this warp's lane quarter, or twice 16 that are 32 apart.
@@ -230,7 +232,7 @@ __global__ void __launch_bounds__(SG_THREADS, 1) sgemm_tcgen05_kernel(const Sgem
     int s = 0;
     uint32_t parity = 1;                     // (a fresh barrier's phase before the first counts as completed)
     for (int i = 0; i < n_kb; ++i) {
-      if (!__all_sync(0xffffffffu, mbar_wait(&empty_bar[s], parity, abort))) break;
+      if (!__all_sync(0xffffffffu, mbar_wait(&empty_bar[s], parity, abort, args.wait_limit_ns))) break;
       const uint32_t stage = smem + s * stage_bytes;
 #pragma unroll
       for (int j = 0; j < SG_W / 32; ++j) {
@@ -245,7 +247,8 @@ __global__ void __launch_bounds__(SG_THREADS, 1) sgemm_tcgen05_kernel(const Sgem
         }
       asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
       __syncwarp();
-      if (lane == 0) asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(smem_u32(&full_bar[s])) : "memory");
+      if (lane == 0 && (i != args.withhold || warp != 0))
+        asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(smem_u32(&full_bar[s])) : "memory");
       if (i + 1 < n_kb) {                    // (behind the fence, which would wait for them)
         read_w(i + 1);
         read_x(i + 1);
@@ -292,8 +295,8 @@ __global__ void __launch_bounds__(SG_THREADS, 1) sgemm_tcgen05_kernel(const Sgem
     int s = 0;
     uint32_t parity = 0;
     auto issue = [&](int chunk) -> bool {
-      if (!__all_sync(0xffffffffu, mbar_wait(&full_bar[s], parity, abort))) return false;
-      if (!__all_sync(0xffffffffu, mbar_wait(&sum_empty[half], ((chunk >> 1) & 1) ^ 1, abort))) return false;
+      if (!__all_sync(0xffffffffu, mbar_wait(&full_bar[s], parity, abort, args.wait_limit_ns))) return false;
+      if (!__all_sync(0xffffffffu, mbar_wait(&sum_empty[half], ((chunk >> 1) & 1) ^ 1, abort, args.wait_limit_ns))) return false;
       asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
       const uint32_t at = smem + s * stage_bytes + half * SG_CHUNK * 2;
       const uint32_t d = tmem + half * buffer_cols;
@@ -329,7 +332,7 @@ __global__ void __launch_bounds__(SG_THREADS, 1) sgemm_tcgen05_kernel(const Sgem
 #pragma unroll 1
     for (int chunk = 0; ok && chunk < n_chunks; ++chunk) {
       if (issuer && ((chunk + 1) & 1) == half && chunk + 1 < n_chunks && !issue(chunk + 1)) break;
-      if (!__all_sync(0xffffffffu, mbar_wait(&sum_full[chunk & 1], (chunk >> 1) & 1, abort))) break;
+      if (!__all_sync(0xffffffffu, mbar_wait(&sum_full[chunk & 1], (chunk >> 1) & 1, abort, args.wait_limit_ns))) break;
       asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
       const uint32_t from = tmem + (chunk & 1) * buffer_cols + ((uint32_t)(quarter * 32) << 16);
 #pragma unroll
@@ -462,15 +465,13 @@ __global__ void __launch_bounds__(SG_THREADS, 1) sgemm_tcgen05_kernel(const Sgem
   if (threadIdx.x == 0 && abort_flag && args.status) atomicOr(args.status, 4);
 }
 
-extern "C" {
-
 // x [rows, k_dim] and w [n_out, k_dim] float32, y [rows, n_out].  Bit 4 of *status (if there is one) is set when a wait
 // ran out.  How many parts the k range is cut into: as many as let one row of tiles run at once, each of two slices
 // at least.  Clusters do not fill the SMs, whose groups are not multiples of them: how many of p blocks run at once is the
 // occupancy query's answer for one block an SM.  One cluster too many is a second round: 16 tiles of 8 parts took 41 us a
 // product of 141 x 2048 x 2048, of 6 parts 29.
-int sb_sgemm_nt(const float* x, const float* w, float* y, int rows, int n_out, int k_dim, int* status,
-                cudaStream_t s) {
+static int sgemm_launch(const float* x, const float* w, float* y, int rows, int n_out, int k_dim, int* status, int withhold,
+                        unsigned long long wait_limit_ns, cudaStream_t s) {
   if (rows == 0 || n_out == 0) return 0;
   const int tiles = (n_out + SG_W - 1) / SG_W, slices = (k_dim + SG_K - 1) / SG_K;
   static const int at_once[SG_MAX_PARTS + 1] = {0, 148, 74, 45, 33, 26, 22, 15, 15};
@@ -480,6 +481,7 @@ int sb_sgemm_nt(const float* x, const float* w, float* y, int rows, int n_out, i
   if ((long long)tiles * row_tiles > 0x7fffffffLL) return -2;
   SgemmArgs args;
   args.x = x; args.w = w; args.y = y; args.status = status;
+  args.withhold = withhold; args.wait_limit_ns = wait_limit_ns;
   args.rows = rows; args.n_out = n_out; args.k_dim = k_dim; args.parts = parts;
   args.tile_rows = ((rows - 1) / row_tiles + 16) / 16 * 16;
   const int stage_bytes = 3 * (SG_W_PLANE + args.tile_rows * SG_K * 2);
@@ -491,6 +493,20 @@ int sb_sgemm_nt(const float* x, const float* w, float* y, int rows, int n_out, i
   if (err != cudaSuccess) return (int)err;
   const int smem = args.stages * stage_bytes + 1024;
   return launch_dependent_cluster(kernel, dim3(tiles * row_tiles, parts), dim3(SG_THREADS), smem, s, dim3(1, parts, 1), args);
+}
+
+extern "C" {
+
+int sb_sgemm_nt(const float* x, const float* w, float* y, int rows, int n_out, int k_dim, int* status, cudaStream_t s) {
+  return sgemm_launch(x, w, y, rows, n_out, k_dim, status, -1, TC_WAIT_LIMIT_NS, s);
+}
+
+// The same with slice `slice` (64 entries of k) of every block's part not handed over by one of its warps: the waits on it give up
+// after wait_limit_ns, the kernel returns, the status bit is set and y is undefined.  For tests.
+int sb_sgemm_nt_withheld(const float* x, const float* w, float* y, int rows, int n_out, int k_dim, int* status, int slice,
+                         unsigned long long wait_limit_ns, cudaStream_t s) {
+  if (slice < 0 || wait_limit_ns == 0) return -2;
+  return sgemm_launch(x, w, y, rows, n_out, k_dim, status, slice, wait_limit_ns, s);
 }
 
 }  // extern "C"

@@ -706,3 +706,28 @@ def test_the_short_convolution_gates_every_value():
     v = x.double()
     want = torch.where(v < -88.6, torch.zeros_like(v), v * torch.sigmoid(v)).to(torch.bfloat16)
     assert bool(((got == want) | (v < -88.6) & (got.double().abs() < 2e-37)).all())
+
+
+@pytest.mark.parametrize("rows,n,k,slice_", [(40, 130, 100, 1), (170, 260, 1024, 0), (20, 2048, 2048, 1)])
+def test_a_wait_in_the_float32_product_that_runs_out_is_reported(rows, n, k, slice_, monkeypatch):
+    """One slice of every block is never handed over (an entry point made for this): the waits on it give up after 2 ms, in blocks
+    alone and in clusters, the kernel returns and the status word says so; the same product is right afterwards."""
+    from starter_b200 import ops
+    from starter_b200.engine.runner import ModelRunner
+
+    x, w = rand(rows, k, seed=64), rand(n, k, seed=65)
+    status = torch.zeros(1, dtype=torch.int32, device="cuda")
+    lib = ops._lib("sgemm")
+    with monkeypatch.context() as m:
+        m.setattr(lib, "sb_sgemm_nt", lambda *a: lib.sb_sgemm_nt_withheld(*a[:-1], slice_, 2_000_000, a[-1]))
+        ops.linear(dev(x), dev(w), status=status)
+    torch.cuda.synchronize()
+    assert status.item() == 4
+    holder = ModelRunner.__new__(ModelRunner)
+    holder.status = status
+    with pytest.raises(RuntimeError, match="tensor-core product ran out of time"):
+        holder.check_status()
+    assert status.item() == 0
+    got = ops.linear(dev(x), dev(w), status=status).cpu().double()
+    bound = (k + 8) * 2.0 ** -24 * (x.double().abs() @ w.double().abs().t())
+    assert bool(((got - x.double() @ w.double().t()).abs() <= bound).all()) and status.item() == 0
