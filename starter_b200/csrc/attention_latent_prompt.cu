@@ -78,7 +78,7 @@ latent_prompt_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_con
                      const __grid_constant__ CUtensorMap map_rot, bf16* __restrict__ out, const int* __restrict__ seq_q_start,
                      const int* __restrict__ seq_q_len, const int* __restrict__ seq_kv_len, const int* __restrict__ block_seq,
                      const int* __restrict__ block_first, int heads, float scale_log2, int window,
-                     const float* __restrict__ sink, int* status) {
+                     const float* __restrict__ sink, int* status, int withhold) {
   constexpr int QC = DC + 1;
   constexpr int QSUB = 128 * 128, KSUB = 64 * 128;  // bytes of 128 (64) rows of 128 bytes
   constexpr int Q_BYTES = QC * QSUB, K_BYTES = QC * KSUB, V_BYTES = VC * KSUB, P_BYTES = QSUB;
@@ -159,6 +159,7 @@ latent_prompt_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_con
       if (i >= 2) ok = __all_sync(0xffffffffu, mbar_wait(&v_empty[b], ((i >> 1) - 1) & 1, abort));
       if (!ok) break;
       if (elected) mbar_expect_tx(&v_full[b], V_BYTES);
+      if (i == withhold) continue;                  // (tests: this step's values never come)
       for (int c = 0; c < VC; ++c)
         if (elected) tma_load_2d(v_sm + b * V_BYTES + c * KSUB, &map_kv, &v_full[b], (heads * DC + head * VC + c) * 64, row);
       loads[2 + b]++;
@@ -360,13 +361,33 @@ latent_prompt_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_con
 template <int DC, int VC>
 static int lp_launch(const CUtensorMap& mq, const CUtensorMap& mkv, const CUtensorMap& mr, void* out, const int* seq_q_start,
                      const int* seq_q_len, const int* seq_kv_len, const int* block_seq, const int* block_first, int n_blocks,
-                     int heads, float scale, int window, const float* sink, int* status, cudaStream_t s) {
+                     int heads, float scale, int window, const float* sink, int* status, int withhold, cudaStream_t s) {
   const int smem = 2 * (DC + 1) * 128 * 128 + 2 * 128 * 128 + 2 * (DC + 1 + VC) * 64 * 128 + 1024;
   cudaError_t err = cudaFuncSetAttribute(latent_prompt_kernel<DC, VC>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
   if (err != cudaSuccess) return (int)err;
   return launch_dependent(latent_prompt_kernel<DC, VC>, dim3(heads, n_blocks), dim3(LP_THREADS), smem, s, mq, mkv, mr, (bf16*)out,
                           seq_q_start, seq_q_len, seq_kv_len, block_seq, block_first, heads, scale * 1.4426950408889634f, window,
-                          sink, status);
+                          sink, status, withhold);
+}
+
+static int lp_run(const void* q, const void* kv, const void* shared, void* out, const int* seq_q_start, const int* seq_q_len,
+                  const int* seq_kv_len, const int* block_seq, const int* block_first, int n_blocks, int n_tokens, int rows,
+                  int heads, int dim, int vdim, float scale, int window, const float* sink, int* status, int withhold,
+                  cudaStream_t s) {
+  if (n_blocks == 0 || n_tokens == 0) return 0;
+  if ((dim != 64 && dim != 128) || (vdim != 64 && vdim != 128) || !(scale > 0.f) || n_blocks > 65535) return -2;
+  if (((uintptr_t)q | (uintptr_t)kv | (uintptr_t)shared | (uintptr_t)out) & 15) return -2;
+  CUtensorMap mq, mkv, mr;
+  int rc = sb_make_map(&mq, q, n_tokens, (long long)heads * (dim + 64), TC_BQ);
+  if (rc) return rc;
+  rc = sb_make_map(&mkv, kv, rows, (long long)heads * (dim + vdim), LP_BK);
+  if (rc) return rc;
+  rc = sb_make_map(&mr, shared, rows, 64, LP_BK);
+  if (rc) return rc;
+#define ARGS mq, mkv, mr, out, seq_q_start, seq_q_len, seq_kv_len, block_seq, block_first, n_blocks, heads, scale, window, sink, status, withhold, s
+  if (dim == 128) return vdim == 128 ? lp_launch<2, 2>(ARGS) : lp_launch<2, 1>(ARGS);
+  return vdim == 128 ? lp_launch<1, 2>(ARGS) : lp_launch<1, 1>(ARGS);
+#undef ARGS
 }
 
 extern "C" {
@@ -387,20 +408,23 @@ int sb_latent_gather(const void* store, const int* block_table, int table_stride
 int sb_latent_prompt(const void* q, const void* kv, const void* shared, void* out, const int* seq_q_start, const int* seq_q_len,
                      const int* seq_kv_len, const int* block_seq, const int* block_first, int n_blocks, int n_tokens, int rows,
                      int heads, int dim, int vdim, float scale, int window, const float* sink, int* status, cudaStream_t s) {
-  if (n_blocks == 0 || n_tokens == 0) return 0;
-  if ((dim != 64 && dim != 128) || (vdim != 64 && vdim != 128) || !(scale > 0.f) || n_blocks > 65535) return -2;
-  if (((uintptr_t)q | (uintptr_t)kv | (uintptr_t)shared | (uintptr_t)out) & 15) return -2;
-  CUtensorMap mq, mkv, mr;
-  int rc = sb_make_map(&mq, q, n_tokens, (long long)heads * (dim + 64), TC_BQ);
-  if (rc) return rc;
-  rc = sb_make_map(&mkv, kv, rows, (long long)heads * (dim + vdim), LP_BK);
-  if (rc) return rc;
-  rc = sb_make_map(&mr, shared, rows, 64, LP_BK);
-  if (rc) return rc;
-#define ARGS mq, mkv, mr, out, seq_q_start, seq_q_len, seq_kv_len, block_seq, block_first, n_blocks, heads, scale, window, sink, status, s
-  if (dim == 128) return vdim == 128 ? lp_launch<2, 2>(ARGS) : lp_launch<2, 1>(ARGS);
-  return vdim == 128 ? lp_launch<1, 2>(ARGS) : lp_launch<1, 1>(ARGS);
-#undef ARGS
+  return lp_run(q, kv, shared, out, seq_q_start, seq_q_len, seq_kv_len, block_seq, block_first, n_blocks, n_tokens, rows, heads,
+                dim, vdim, scale, window, sink, status, -1, s);
+}
+
+// The same with the values of step `step` (64 keys) of every block left out: the waits on them give up after wait_limit_ns, the
+// kernel returns, the status bit is set and out is undefined.  For tests.
+int sb_latent_prompt_withheld(const void* q, const void* kv, const void* shared, void* out, const int* seq_q_start, const int* seq_q_len,
+                              const int* seq_kv_len, const int* block_seq, const int* block_first, int n_blocks, int n_tokens, int rows,
+                              int heads, int dim, int vdim, float scale, int window, const float* sink, int* status, int step,
+                              unsigned long long wait_limit_ns, cudaStream_t s) {
+  if (step < 0 || wait_limit_ns == 0) return -2;
+  const unsigned long long usual = WAIT_LIMIT_NS;
+  cudaMemcpyToSymbolAsync(tc_wait_limit_ns, &wait_limit_ns, sizeof(usual), 0, cudaMemcpyHostToDevice, s);
+  const int rc = lp_run(q, kv, shared, out, seq_q_start, seq_q_len, seq_kv_len, block_seq, block_first, n_blocks, n_tokens, rows,
+                        heads, dim, vdim, scale, window, sink, status, step, s);
+  cudaMemcpyToSymbolAsync(tc_wait_limit_ns, &usual, sizeof(usual), 0, cudaMemcpyHostToDevice, s);
+  return rc;
 }
 
 }  // extern "C"

@@ -94,6 +94,35 @@ def test_a_weight_is_rounded_no_more_than_once():
     assert bool(((got - want).abs() <= 1.01 * 2.0 ** -8 * want.abs()).all())
 
 
+@pytest.mark.parametrize("dim,vdim,step", [(128, 128, 0), (128, 64, 3), (64, 64, 1)])
+def test_a_wait_that_runs_out_is_reported(dim, vdim, step, monkeypatch):
+    """The values of one step are left out (an entry point made for this): the waits on them give up after 2 ms, the kernel
+    returns and the status word says so; the same call is right afterwards."""
+    from starter_b200 import ops
+    from starter_b200.engine.runner import ModelRunner
+
+    heads, rank, rot, tokens, gen = 2, 128, 64, 300, torch.Generator().manual_seed(3)
+    ukv = (torch.randn(heads * (dim + vdim), rank, generator=gen) * rank ** -0.5).to(BF).cuda()
+    store = torch.randn(5, 1, 64, rank + rot, generator=gen).to(BF).cuda()
+    q = torch.randn(tokens, heads * (dim + rot), generator=gen).to(BF).cuda()
+    table, ctx = torch.arange(5, dtype=torch.int32)[None].cuda(), context([0], [tokens], [0])
+
+    def run():
+        return ops.latent_attention_prompt(q, ukv, store, table, ctx, heads, dim, vdim, rank, rot, 0.1)
+
+    want, lib = run(), ops._lib("attention_latent_prompt")
+    with monkeypatch.context() as m:
+        m.setattr(lib, "sb_latent_prompt", lambda *a: lib.sb_latent_prompt_withheld(*a[:-1], step, 2_000_000, a[-1]))
+        run()
+    torch.cuda.synchronize()
+    assert ctx.status.item() == 16
+    holder = ModelRunner.__new__(ModelRunner)
+    holder.status = ctx.status
+    with pytest.raises(RuntimeError, match="prefill attention kernel ran out of time"):
+        holder.check_status()
+    assert torch.equal(run(), want) and ctx.status.item() == 0
+
+
 @pytest.mark.parametrize("window,layout,gate", [(None, "interleaved", True), (90, "half_split", False)])
 def test_the_layer_on_either_kernel(window, layout, gate, monkeypatch):
     from starter_b200 import ops
