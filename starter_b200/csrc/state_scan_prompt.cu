@@ -13,7 +13,7 @@
 //     of such updates, Bischof and Van Loan 1987) is one 16 x 16 matrix pair a block and head, made beforehand for
 //     all blocks at once by scan_coef_kernel.  The products with S run on the tensor cores, whose other operands, keys and
 //     queries, are bfloat16 as they come: S (and the write) is cut into three pieces of 8 bits, so that nothing of its 24 is
-//     lost, and sums are float.  G is applied as S - (1 - G) S, the complement carried as such (state_scan.cu says why), and a
+//     lost (of an entry below 2^-109 less than 2^-134; S itself is kept whole), and sums are float.  G is applied as S - (1 - G) S, the complement carried as such (state_scan.cu says why), and a
 //     block's write is added to S by ordinary adds.
 //   walk (forget-write, channel-decay): the decay differs by row, so a token is a step; the state's update is the whole
 //     chain, and read-outs of eight tokens are summed together.  A thread keeps 16 entries, so that a loaded vector serves
