@@ -1648,10 +1648,13 @@ def latent_attention_step(qa, store, block_table, ctx, heads, rank, rot, scale, 
 
 
 #: tokens that every sequence of a step must bring for the latent attention to form keys and values (see
-#: ``latent_attention_prompt``), and the most cache rows it forms them for.  Forming a row costs a head 2 * 256 * 512
-#: products, a query saves it about 1,500 a row at a third of the speed: from about 25 tokens on it pays, whatever the
-#: rows
+#: ``latent_attention_prompt``), and the most cache rows it forms them for
 LATENT_PROMPT_TOKENS, LATENT_PROMPT_ROWS = 32, 65536
+#: sequences times heads from which it does not pay, for each wave of blocks (64 query rows of a sequence's tokens and heads, one an
+#: SM) that the kernel which scores the latents needs.  That kernel takes 0.1 us a key and wave, forming and attending 0.0005 us
+#: a key and head: from 47 tokens a sequence on the latter is always less.  16 heads behind 1,000 cached tokens, a layer, scored / formed: 16
+#: sequences of 32 tokens 184 / 206 us, 8 of 32 169 / 122, 16 of 48 (two waves) 303 / 214
+LATENT_PROMPT_HEADS = 200
 #: what the formed keys, values and gathered rows of a step may take in bytes where they take more than the folded queries and summed
 #: latents of the kernel that scores the latents (a prompt of many heads over its own tokens alone takes a quarter of those; a portion
 #: behind a long cache more): 65,536 rows of 16 heads of 128 + 128 over a latent of 512 take 612 MB
@@ -1671,15 +1674,20 @@ def latent_prompt_takes(dtype, ctx, dim, rot, vdim, rank, scale, window=None, he
     """Whether ``latent_attention_prompt`` serves this step: bfloat16, plain keys and values of 64 or 128 entries and a rotated
     part of 64, every sequence bringing at least ``LATENT_PROMPT_TOKENS`` tokens (known on the host), and no more than
     ``LATENT_PROMPT_ROWS`` rows to form keys and values for, which with ``heads`` heads take no more than
-    ``LATENT_PROMPT_BYTES`` or than the other kernel's buffers."""
+    ``LATENT_PROMPT_BYTES`` or than the other kernel's buffers; and no more than ``LATENT_PROMPT_HEADS`` heads of sequences for
+    each wave of the other kernel's blocks."""
     if dtype != torch.bfloat16 or ctx.host is None or ctx.block_seq is None or not scale > 0:
         return False
     if dim not in (64, 128) or vdim not in (64, 128) or rot != 64 or rank % 16 or rank + rot > 640:
         return False
-    if int(ctx.host["seq_q_len"].min()) < LATENT_PROMPT_TOKENS:
+    new = ctx.host["seq_q_len"]
+    if int(new.min()) < LATENT_PROMPT_TOKENS:
+        return False
+    waves = -(-int((-(-new * heads // 64)).sum()) // 148)
+    if new.size * heads >= LATENT_PROMPT_HEADS * waves:
         return False
     rows = int(_latent_prompt_rows(ctx, window).sum())
-    scored = 2 * int(ctx.host["seq_q_len"].sum()) * heads * (2 * rank + rot)
+    scored = 2 * int(new.sum()) * heads * (2 * rank + rot)
     return rows <= LATENT_PROMPT_ROWS and 2 * rows * (heads * (dim + vdim) + rank + rot) <= max(LATENT_PROMPT_BYTES, scored)
 
 

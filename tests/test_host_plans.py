@@ -133,3 +133,20 @@ def test_formed_keys_are_bounded_in_bytes(heads, past, new, window, takes):
     if got:
         rows = min(past + new, new + (window or past) - 1) + 64
         assert 2 * rows * (heads * 256 + 576) <= max(ops.LATENT_PROMPT_BYTES, 2 * new * heads * 1088) + 64 * 2 * (heads * 256 + 576)
+
+
+@pytest.mark.parametrize("heads, news, takes", [
+    (16, [32], True), (16, [32] * 8, True), (16, [32] * 16, False), (16, [36] * 16, False), (16, [38] * 16, True), (16, [48] * 32, True),
+    (32, [32] * 4, True), (32, [32] * 8, False), (32, [48] * 32, True), (16, [2000] + [32] * 15, True), (16, [31] * 2, False)])
+def test_keys_are_formed_where_that_is_the_shorter_way(heads, news, takes):
+    """Many sequences of few tokens fill the chip with blocks that score the latents; one block more is a second wave."""
+    from types import SimpleNamespace
+
+    import torch
+
+    from starter_b200 import ops
+
+    new = np.array(news, dtype=np.int32)
+    for past in (0, 1000):
+        ctx = SimpleNamespace(host={"seq_q_len": new, "seq_kv_len": new + past}, block_seq=torch.zeros(1))
+        assert ops.latent_prompt_takes(torch.bfloat16, ctx, 128, 64, 128, 512, 0.1, None, heads) is takes
