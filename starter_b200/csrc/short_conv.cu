@@ -325,7 +325,10 @@ int sb_short_conv(int dtype, const void* x, int ldx, const float* taps, const fl
                   const int* seq_q_len, int n_seqs, int max_q_len, int channels, int K, int act, cudaStream_t s) {
   if (n_seqs == 0 || channels == 0) return 0;
   if (K < 1 || K > CONV_MAX_TAPS || K - 1 > CONV_CHUNK || max_q_len < 1) return -2;
-  if (dtype == 1 && K <= 4 && channels % 4 == 0 && ldx % 4 == 0 && ldy % 4 == 0 && !(((uintptr_t)x | (uintptr_t)y) % 8)) {
+  // (with four taps and few tokens the general kernel's one chunk is the shorter chain: captured, 4,096 channels with silu, general /
+  // vector, 1 sequence of one token 2.7 / 3.5 us, 32 of one 3.6 / 4.7, 256 of one 18.3 / 20.0, 1 of eight 3.4 / 3.5, 128 of four 12.6 / 11.6)
+  const bool many = K <= 3 || max_q_len >= 8 || (max_q_len >= 2 && (long long)n_seqs * max_q_len >= 256);
+  if (dtype == 1 && many && K <= 4 && channels % 4 == 0 && ldx % 4 == 0 && ldy % 4 == 0 && !(((uintptr_t)x | (uintptr_t)y) % 8)) {
     const int vec_chunks = (max_q_len + CONV_VEC_CHUNK - 1) / CONV_VEC_CHUNK;
     const dim3 vec_grid(n_seqs * vec_chunks, (channels / 4 + 127) / 128);
     auto kernel = K == 1 ? short_conv_vec_kernel<1> : K == 2 ? short_conv_vec_kernel<2> : K == 3 ? short_conv_vec_kernel<3> : short_conv_vec_kernel<4>;

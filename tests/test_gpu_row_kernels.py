@@ -73,3 +73,39 @@ def test_latent_prepare_in_pieces(q_rank, rank, rot, dims, split, write):
     want[:, one], want[:, two] = shared[:, one] * c - shared[:, two] * s, shared[:, two] * c + shared[:, one] * s
     assert bool(((rows[:, rank:] - want).abs() <= HALF_STEP * want.abs() + 2.0 ** -22 * shared.abs().max()).all())
     assert int((store.float().abs().sum(dim=-1) > 0).sum()) == n
+
+
+# steps in which every sequence is listed with what it brings: whole pieces of eight tokens and rests, sequences shorter than the
+# filter beside long ones, many sequences of two tokens, single tokens
+@pytest.mark.parametrize("steps, channels", [([[150, 1, 9, 8], [7, 8, 2, 16], [1, 1, 1, 1]], 516), ([[2] * 130, [1] * 130, [3] * 130], 12)])
+@pytest.mark.parametrize("taps", [1, 2, 3, 4])
+@pytest.mark.parametrize("act", [None, "silu"])
+def test_short_convolution_in_pieces(steps, channels, taps, act):
+    from starter_b200 import ops
+
+    gen, n = torch.Generator().manual_seed(channels + taps), len(steps[0])
+    lengths = [sum(s[i] for s in steps) for i in range(n)]
+    x = [torch.randn(length, 4 + channels + 8, generator=gen).to(BF) for length in lengths]
+    w, bias, in_bias = torch.randn(channels, taps, generator=gen), torch.randn(channels, generator=gen), torch.randn(channels, generator=gen)
+    slots = list(reversed(range(n)))
+    state = torch.zeros(n, (taps - 1) * channels + 3, device="cuda") if taps > 1 else None
+    done, got = [0] * n, [[] for _ in range(n)]
+    ints = lambda v: torch.tensor(v, dtype=torch.int32, device="cuda")
+    for sizes in steps:
+        rows = torch.cat([x[i][done[i]:done[i] + m] for i, m in enumerate(sizes)]).cuda()
+        starts = [sum(sizes[:i]) for i in range(n)]
+        out = ops.short_conv(rows, 4, channels, w.cuda(), bias.cuda(), in_bias.cuda(), state, 3 if taps > 1 else 0, ints(slots), ints(starts), ints(sizes),
+                             max(sizes), act).cpu()
+        for i, m in enumerate(sizes):
+            got[i].append(out[starts[i]:starts[i] + m])
+            done[i] += m
+    for i in range(n):
+        xs = x[i][:, 4:4 + channels].double() + in_bias.double()
+        want, size = bias.double().expand_as(xs).clone(), bias.double().abs().expand_as(xs).clone()
+        for back in range(min(taps, lengths[i])):
+            want[back:] += w[:, taps - 1 - back].double() * xs[:lengths[i] - back]
+            size[back:] += (w[:, taps - 1 - back].double() * xs[:lengths[i] - back]).abs()
+        if act:
+            want = want * torch.sigmoid(want)
+        # (the slope of silu is at most 1.1)
+        assert bool(((torch.cat(got[i]).double() - want).abs() <= HALF_STEP * want.abs() + 2.0 ** -20 * size).all())
