@@ -1662,12 +1662,12 @@ LATENT_PROMPT_BYTES = 640 << 20
 
 
 def _latent_prompt_rows(ctx, window):
-    """The rows of each sequence that ``latent_attention_prompt`` works on (numpy), as its kernels count them."""
-    q_len, kv_len = ctx.host["seq_q_len"], ctx.host["seq_kv_len"]
-    rows = kv_len
+    """The rows of each sequence that ``latent_attention_prompt`` works on, as its kernels count them (plain numbers: a step's few
+    sequences cost less this way than a round of numpy calls, 15 us a layer)."""
+    rows = ctx.host["seq_kv_len"].tolist()
     if window:
-        rows = kv_len - (kv_len - q_len - int(window) + 1).clip(min=0)
-    return (rows + 63) // 64 * 64
+        rows = [kv - max(0, kv - new - int(window) + 1) for kv, new in zip(rows, ctx.host["seq_q_len"].tolist())]
+    return [(r + 63) // 64 * 64 for r in rows]
 
 
 def latent_prompt_takes(dtype, ctx, dim, rot, vdim, rank, scale, window=None, heads=1) -> bool:
@@ -1680,14 +1680,14 @@ def latent_prompt_takes(dtype, ctx, dim, rot, vdim, rank, scale, window=None, he
         return False
     if dim not in (64, 128) or vdim not in (64, 128) or rot != 64 or rank % 16 or rank + rot > 640:
         return False
-    new = ctx.host["seq_q_len"]
-    if int(new.min()) < LATENT_PROMPT_TOKENS:
+    new = ctx.host["seq_q_len"].tolist()
+    if min(new) < LATENT_PROMPT_TOKENS:
         return False
-    waves = -(-int((-(-new * heads // 64)).sum()) // 148)
-    if new.size * heads >= LATENT_PROMPT_HEADS * waves:
+    waves = -(-sum(-(-n * heads // 64) for n in new) // 148)
+    if len(new) * heads >= LATENT_PROMPT_HEADS * waves:
         return False
-    rows = int(_latent_prompt_rows(ctx, window).sum())
-    scored = 2 * int(new.sum()) * heads * (2 * rank + rot)
+    rows = sum(_latent_prompt_rows(ctx, window))
+    scored = 2 * sum(new) * heads * (2 * rank + rot)
     return rows <= LATENT_PROMPT_ROWS and 2 * rows * (heads * (dim + vdim) + rank + rot) <= max(LATENT_PROMPT_BYTES, scored)
 
 
@@ -1710,12 +1710,12 @@ def latent_attention_prompt(q, ukv, store, block_table, ctx, heads, dim, vdim, r
     for name, t in (("seq_kv_len", ctx.seq_kv_len), ("block_seq", ctx.block_seq), ("block_first", ctx.block_first)):
         _need(t, name, torch.int32, 1)
     each = _latent_prompt_rows(ctx, window)
-    rows = int(each.sum())
+    rows = sum(each)
     gathered = q.new_empty((rows * (rank + rot),))
     c, shared = gathered[:rows * rank].view(rows, rank), gathered[rows * rank:].view(rows, rot)
     lib = _lib("attention_latent_prompt")
     rc = lib.sb_latent_gather(_ptr(store), _ptr(block_table), block_table.shape[1], _ptr(ctx.seq_slot), _ptr(ctx.seq_q_len),
-                              _ptr(ctx.seq_kv_len), n_seqs, int(each.max()), _ptr(c), _ptr(shared), rank, rot, int(window or 0),
+                              _ptr(ctx.seq_kv_len), n_seqs, max(each), _ptr(c), _ptr(shared), rank, rot, int(window or 0),
                               _stream())
     _check(rc, "latent_gather")
     kv = linear(c, ukv, status=ctx.status)
