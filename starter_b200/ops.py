@@ -31,6 +31,8 @@ TENSOR_CORE_MAX_ROWS = 128
 #: (engine/engine.py:431-450).
 PROMPT_MIN_ROWS = 512
 MAX_HEAD_DIM = 256
+#: streaming multiprocessors of a B200
+SM_COUNT = 148
 
 _DT = {torch.float32: 0, torch.bfloat16: 1}
 
@@ -2399,6 +2401,20 @@ def scan_max_state() -> int:
     return _lib("state_scan").sb_scan_max_state()
 
 
+def scan_segments(n_tokens: int, n_seqs: int, blocks: int) -> int:
+    """Into how many segments the sequences of a state-space step are cut (csrc/state_scan_prompt.cu), where ``blocks`` thread
+    blocks walk a sequence's heads: as many as give every SM one block, or two where segments of 150 tokens and more remain
+    and one block an SM already means cutting (in between some SMs have twice the work of others).  Measured (us, segments):
+    2,048 tokens of 32 heads 1: 168, 4: 71, 5: 86, 8: 66; two sequences of 700 1: 68, 2: 51, 3: 56, 4: 47; of 300 1: 35,
+    2: 27, 3: 33, 4: 29; four of 500 1: 55, 2: 60.  Segments of fewer than 48 tokens gain nothing."""
+    blocks *= n_seqs
+    one, tokens = SM_COUNT // max(1, blocks), n_tokens // n_seqs
+    segs = one
+    if one > 1 and tokens >= 150 * (2 * SM_COUNT // blocks):
+        segs = 2 * SM_COUNT // blocks
+    return max(1, min(segs, tokens // 48, 16))
+
+
 def state_scan(mode, q, k, v, a_raw, b_raw, A_log, dt_bias, skip, state, state_at, seq_slot, seq_q_start, seq_q_len,
                heads, groups, n_state, v_dim, decay=None):
     """A linear recurrence with a state ``S`` ``[n_state, v_dim]`` per head over the sequences of a step.
@@ -2452,10 +2468,15 @@ def state_scan(mode, q, k, v, a_raw, b_raw, A_log, dt_bias, skip, state, state_a
         floats = lib.sb_scan_prompt_floats(1, SCAN_MODES[mode], *args[:6], _ptr(decay), heads, groups, n_state, v_dim)
         if 0 <= 4 * floats * n_tokens <= SCAN_PROMPT_BYTES:
             scratch = state.new_empty((n_tokens, floats), dtype=torch.float32) if floats else None
+            segs, carried = 1, None
+            if mode == "state_space":
+                segs = scan_segments(n_tokens, n_seqs, heads * -(-v_dim // 64))
+                if segs > 1:
+                    carried = state.new_empty((n_seqs * segs * lib.sb_scan_segment_floats(heads, v_dim),))
             rc = lib.sb_state_scan_prompt(
                 SCAN_MODES[mode], *args, _ptr(A_log), _ptr(dt_bias), _ptr(skip), _ptr(decay), _at(state, state_at),
                 ctypes.c_longlong(state.shape[1]), _ptr(out), _ptr(seq_slot), _ptr(seq_q_start), _ptr(seq_q_len), n_tokens,
-                n_seqs, heads, groups, n_state, v_dim, _ptr(scratch), _stream())
+                n_seqs, heads, groups, n_state, v_dim, _ptr(scratch), segs, _ptr(carried), _stream())
             _check(rc, "state_scan (many tokens)", 1 if mode == "channel_decay" else 2)
             return out
     rc = _lib("state_scan").sb_state_scan(

@@ -180,3 +180,38 @@ def test_scratch_is_bounded(mode, floats, monkeypatch):
     few = run()
     monkeypatch.setattr(ops, "SCAN_PROMPT_TOKENS", 1 << 30)
     assert torch.equal(few, run()) and not torch.equal(few, many)
+
+
+@pytest.mark.parametrize("segs", [2, 3, 7, 16])
+@pytest.mark.parametrize("width", [64, 72])
+def test_state_space_in_segments(segs, width, monkeypatch):
+    """Sequences cut into segments that are walked at once, some with fewer blocks of 16 tokens than segments, against one walk."""
+    from starter_b200 import ops
+
+    heads, n = 3, 72
+    gen = torch.Generator().manual_seed(segs)
+    lengths, slots = [1, 16, 17, 113, 240, 400], [5, 0, 3, 1, 2, 4]
+    total = sum(lengths)
+    qk, v, ab = (torch.randn(total, size, generator=gen).to(BF).cuda() for size in (2 * n, heads * width, heads))
+    A, bias, skip = torch.linspace(-6.0, 0.5, heads).cuda(), torch.zeros(heads).cuda(), torch.ones(heads).cuda()
+    start = torch.randn(6, heads * n * width, generator=gen).cuda()
+
+    def run(count):
+        monkeypatch.setattr(ops, "scan_segments", lambda *a: count)
+        state = start.clone()
+        out = ops.state_scan("state_space", (qk, n), (qk, 0), (v, 0), (ab, 0), None, A, bias, skip, state, 0, *packed(lengths, slots),
+                             heads, 1, n, width)
+        return out, state
+
+    (want, kept), (got, state) = run(1), run(segs)
+    # float arithmetic in another order: some hundred roundings of 2^-24 of terms that may cancel
+    assert float((got - want).abs().max()) <= 2e-5 * float(want.abs().max())
+    assert float((state - kept).abs().max()) <= 2e-5 * float(kept.abs().max())
+
+
+def test_segments_of_a_step():
+    from starter_b200 import ops
+
+    for tokens, seqs, blocks in ((64, 1, 32), (2048, 1, 32), (300, 1, 1), (5, 3, 8), (1 << 20, 4, 1), (40000, 600, 32)):
+        segs = ops.scan_segments(tokens, seqs, blocks)
+        assert 1 <= segs <= 16 and (segs == 1 or (segs * seqs * blocks <= 2 * 148 and tokens // seqs >= 48 * segs))
