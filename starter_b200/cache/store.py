@@ -55,7 +55,7 @@ class SequenceCache:
         self._stage_next = 0
 
         self.groups = plan_groups(kv_needs)
-        self._where = {}
+        self._where, self._pages = {}, {}
         self.keys, self.values = [], []
         for g, group in enumerate(self.groups):
             need: KVNeed = group.need
@@ -64,6 +64,7 @@ class SequenceCache:
             self.values.append(torch.zeros(shape[:-1] + (need.value_size,), dtype=dtype, device=self.device))
             for i, entry in enumerate(group.entries):
                 self._where[entry] = (g, i)
+                self._pages[entry] = (self.keys[g][i], self.values[g][i])
         self.state = {}
         for entry, need in state_needs.items():
             if need is None:
@@ -77,8 +78,7 @@ class SequenceCache:
     def entry_pages(self, entry: int):
         """``(keys, values)`` of one cache entry: ``[pages, kv_heads, 64, head_dim]`` and
         ``[pages, kv_heads, 64, value_dim]`` (the same shape unless the entry's need says otherwise)."""
-        g, i = self._where[entry]
-        return self.keys[g][i], self.values[g][i]
+        return self._pages[entry]
 
     def entry_need(self, entry: int) -> KVNeed:
         return self.groups[self._where[entry][0]].need

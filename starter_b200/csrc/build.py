@@ -4,8 +4,8 @@ Each ``name.cu`` becomes ``_build/libsb_name.so`` next to the sources (or, if th
 folder cannot be written, under the system temp folder), built by ``nvcc`` the
 first time a kernel of that file is needed and again whenever the source, the
 shared header or the flags change.  The libraries export plain C entry points
-and are loaded with ``ctypes``; nothing links against torch, so a build takes
-seconds.  There is no other implementation behind these entry points: if a
+and are loaded with ``ctypes``; none of them links against torch, so a build takes
+seconds (``host.cpp``, the host side of a launch, is an extension module and does).  There is no other implementation behind these entry points: if a
 library can be neither found nor built, the call fails.
 """
 
@@ -13,11 +13,13 @@ from __future__ import annotations
 
 import ctypes
 import hashlib
+import importlib.util
 import os
 import re
 import shutil
 import subprocess
 import sys
+import sysconfig
 import tempfile
 import threading
 import time
@@ -65,6 +67,7 @@ SOURCES = (
 
 _lock = threading.Lock()
 _loaded: dict = {}
+_host = None
 
 
 class KernelBuildError(RuntimeError):
@@ -186,9 +189,62 @@ def declarations(name: str) -> dict:
     return out
 
 
+def host_path() -> str:
+    """Path of the built extension module of ``host.cpp`` (the host side of a launch), compiled first if it is missing or
+    stale.  It is the one part that links against torch."""
+    import torch
+
+    root = os.path.dirname(torch.__file__)
+    compiler = os.environ.get("CXX") or shutil.which("g++") or shutil.which("c++")
+    cuda = os.path.join(os.path.dirname(os.path.dirname(os.path.realpath(_nvcc()))), "include")
+    src = os.path.join(HERE, "host.cpp")
+    flags = ["-O2", "-std=c++17", "-fPIC", "-shared", f"-D_GLIBCXX_USE_CXX11_ABI={int(torch.compiled_with_cxx11_abi())}",
+             "-I", os.path.join(root, "include"), "-I", os.path.join(root, "include", "torch", "csrc", "api", "include"),
+             "-I", cuda, "-I", sysconfig.get_paths()["include"]]
+    link = ["-L", os.path.join(root, "lib"), "-ltorch_python", "-ltorch_cuda", "-ltorch_cpu", "-ltorch", "-lc10_cuda", "-lc10",
+            "-Wl,-rpath," + os.path.join(root, "lib")]
+    lib = os.path.join(_build_dir(), "sb_host.so")
+    stamp = lib + ".stamp"
+    h = hashlib.sha256(" ".join([torch.__version__, sys.version] + flags + link).encode())
+    with open(src, "rb") as handle:
+        h.update(handle.read())
+    digest = h.hexdigest()[:16]
+    if os.path.isfile(lib) and os.path.isfile(stamp):
+        with open(stamp) as handle:
+            if handle.read().strip() == digest:
+                return lib
+    if compiler is None:
+        raise KernelBuildError("no C++ compiler was found (looked at $CXX and PATH for g++ and c++)")
+    tmp = f"{lib}.{os.getpid()}.tmp"
+    print("[starter_b200] compiling host.cpp ...", file=sys.stderr, flush=True)
+    proc = subprocess.run([compiler] + flags + ["-o", tmp, src] + link, stdout=subprocess.PIPE, stderr=subprocess.STDOUT, text=True)
+    if proc.returncode != 0:
+        if os.path.exists(tmp):
+            os.remove(tmp)
+        raise KernelBuildError(f"{compiler} failed on host.cpp:\n{proc.stdout}")
+    os.replace(tmp, lib)
+    with open(stamp, "w") as handle:
+        handle.write(digest)
+    return lib
+
+
+def load_host():
+    """The extension module of ``host.cpp`` (built on first use)."""
+    global _host
+    with _lock:
+        if _host is None:
+            import torch  # noqa: F401  (its libraries have to be there first)
+
+            spec = importlib.util.spec_from_file_location("sb_host", host_path())
+            module = importlib.util.module_from_spec(spec)
+            spec.loader.exec_module(module)
+            _host = module
+        return _host
+
+
 def load(name: str) -> ctypes.CDLL:
     """The loaded library of ``name.cu`` (built on first use).  Its entry points know their argument types, so callers
-    pass addresses as plain integers (a ctypes object for each cost more than the launch itself)."""
+    pass addresses as plain integers."""
     with _lock:
         lib = _loaded.get(name)
         if lib is None:
@@ -201,21 +257,21 @@ def load(name: str) -> ctypes.CDLL:
 
 
 def build_all(names=SOURCES) -> list:
-    """Compile every kernel source (in parallel) and return the library paths."""
+    """Compile every kernel source and the host module (in parallel) and return the library paths."""
     results = {}
     errors = []
 
     def work(n):
         try:
-            results[n] = library_path(n)
+            results[n] = host_path() if n == "host" else library_path(n)
         except Exception as exc:  # noqa: BLE001 - collected and re-raised below
             errors.append(exc)
 
-    threads = [threading.Thread(target=work, args=(n,)) for n in names]
+    threads = [threading.Thread(target=work, args=(n,)) for n in list(names) + ["host"]]
     for t in threads:
         t.start()
     for t in threads:
         t.join()
     if errors:
         raise errors[0]
-    return [results[n] for n in names]
+    return [results[n] for n in list(names) + ["host"]]

@@ -44,12 +44,26 @@ class KernelError(RuntimeError):
 _libs = {}
 
 
+class _Library:
+    """A kernel library's entry points as native callables (csrc/host.cpp): they take tensors, None, integers and floats."""
+
+    def __init__(self, name: str):
+        # (without the native part: the first call of any operation binds it)
+        host, loaded = _bind(), build.load(name)
+        self._loaded = loaded
+        for entry, (result, types) in build.declarations(name).items():
+            kinds = "".join("p" if t is ctypes.c_void_p else "f" if t is ctypes.c_float else "i" for t in types)
+            kind = "v" if result is None else "i" if result is ctypes.c_int else "l"
+            address = ctypes.cast(getattr(loaded, entry), ctypes.c_void_p).value
+            setattr(self, entry, host.Entry(address, kinds, kind))
+
+
 def _lib(name: str):
     """The kernel library of ``name.cu``; refuses one compiled for another cache page size."""
     lib = _libs.get(name)
     if lib is None:
-        lib = build.load(name)
-        compiled = lib.sb_page_tokens()
+        lib = _Library(name)
+        compiled = lib._loaded.sb_page_tokens()
         if compiled != PAGE_TOKENS:
             raise KernelError(f"libsb_{name} was compiled for cache pages of {compiled} tokens, the cache "
                               f"uses pages of {PAGE_TOKENS}")
@@ -67,35 +81,41 @@ def _ptr(t):
     return t.data_ptr() if t is not None else None
 
 
-try:                                   # the raw handle of the current stream without building objects
-    _raw_stream = torch._C._cuda_getCurrentRawStream
-    _current_device = torch._C._cuda_getDevice
-except AttributeError:                 # pragma: no cover - older or newer torch: the public way
-    _raw_stream = _current_device = None
-
-
-def _stream():
-    """The current CUDA stream's address (called once per launch: it has to be cheap)."""
-    if _raw_stream is not None:
-        return _raw_stream(_current_device())
-    return torch.cuda.current_stream().cuda_stream
-
-
-def _need(t, name, dtype=None, ndim=None):
-    # the common case first and in one expression: this runs several times per launch
-    try:
-        if (t.is_cuda and t.is_contiguous() and (dtype is None or t.dtype == dtype)
-                and (ndim is None or t.dim() == ndim)):
-            return
-    except AttributeError:
-        pass
+def _refuse(t, name, dtype=None, ndim=None):
+    """What is wrong with an operand that is no contiguous CUDA tensor of this type and number of dimensions."""
     if not isinstance(t, torch.Tensor) or not t.is_cuda:
         raise KernelError(f"{name} must be a CUDA tensor (there is no CPU implementation)")
     if not t.is_contiguous():
         raise KernelError(f"{name} must be contiguous, got strides {t.stride()} for shape {tuple(t.shape)}")
     if dtype is not None and t.dtype != dtype:
         raise KernelError(f"{name} must be {dtype}, got {t.dtype}")
-    raise KernelError(f"{name} must have {ndim} dimensions, got shape {tuple(t.shape)}")
+    if ndim is not None and t.dim() != ndim:
+        raise KernelError(f"{name} must have {ndim} dimensions, got shape {tuple(t.shape)}")
+
+
+# The check in front of every operand, an output's allocation and the current stream's address, which run several times a
+# launch, are native too (csrc/host.cpp).  The first call of any of them loads the native part and puts it in these names.
+
+def _bind():
+    global _need, _empty, _stream
+    host = build.load_host()
+    host.refuse_with(_refuse)
+    _need, _empty, _stream = host.need, host.empty, host.stream
+    return host
+
+
+def _need(t, name, dtype=None, ndim=None):
+    _refuse(t, name, dtype, ndim)          # (what is refused needs no native part)
+    _bind()
+
+
+def _empty(like, shape, dtype=None):
+    return _bind().empty(like, shape, dtype)
+
+
+def _stream():
+    """The current CUDA stream's address."""
+    return _bind().stream()
 
 
 class _Added:
@@ -143,10 +163,10 @@ def embedding(tokens, table, status=None, fence=False):
     kernels of the step read, before their own dependent-launch wait, what earlier steps wrote."""
     _need(tokens, "tokens", torch.int32, 1)
     _need(table, "table", None, 2)
-    out = table.new_empty((tokens.shape[0], table.shape[1]))
+    out = _empty(table, (tokens.shape[0], table.shape[1]))
     rc = _lib("elementwise").sb_embedding(
-        _code(table.dtype), _ptr(tokens), _ptr(table), _ptr(out), tokens.shape[0], table.shape[1],
-        table.shape[0], _ptr(status), int(fence), _stream())
+        _code(table.dtype), tokens, table, out, tokens.shape[0], table.shape[1],
+        table.shape[0], status, int(fence), _stream())
     _check(rc, "embedding")
     return out
 
@@ -172,10 +192,10 @@ def rmsnorm(x, gain, eps, delta=None, rows=None, out=None):
         _need(rows, "rows", torch.int32, 1)
         n_rows = rows.shape[0]
     if out is None:
-        out = x.new_empty((n_rows, hidden))
+        out = _empty(x, (n_rows, hidden))
     rc = _lib("elementwise").sb_rmsnorm(
-        _code(x.dtype), _gain_code(x, gain), _ptr(x), _ptr(delta), _ptr(gain), _ptr(out), _ptr(rows),
-        n_rows, hidden, ctypes.c_float(eps), _stream())
+        _code(x.dtype), _gain_code(x, gain), x, delta, gain, out, rows,
+        n_rows, hidden, eps, _stream())
     _check(rc, "rmsnorm")
     return out
 
@@ -206,9 +226,9 @@ def swiglu(gate_up, activation="silu"):
     if gate_up.shape[1] % 2:
         raise KernelError(f"gate_up has an odd width {gate_up.shape[1]}")
     inner = gate_up.shape[1] // 2
-    out = gate_up.new_empty((gate_up.shape[0], inner))
+    out = _empty(gate_up, (gate_up.shape[0], inner))
     rc = _lib("elementwise").sb_swiglu(
-        _code(gate_up.dtype), _ptr(gate_up), _ptr(out), gate_up.shape[0], inner, gate_code(activation),
+        _code(gate_up.dtype), gate_up, out, gate_up.shape[0], inner, gate_code(activation),
         _stream())
     _check(rc, "swiglu")
     return out
@@ -242,21 +262,21 @@ def linear(x, weight, out_float=False, gated=False, status=None, add_to=None):
     n_out = n_total // 2 if gated else n_total
     dt = _code(x.dtype)
     if dt == 1 and rows <= TENSOR_CORE_MAX_ROWS and tensor_core_ok(x, weight, gated, n_out):
-        return linear_tensor_core(x, weight, out_float=out_float, gated=gated, status=status)
+        return linear_tensor_core(x, weight, out_float, gated, status=status, checked=True)
     if rows <= SMALL_ROWS:
         out_dtype = torch.float32 if (out_float or dt == 0) else x.dtype
         if gated and out_float and dt == 1:
             raise KernelError("a gated product cannot return float32 from bfloat16")
-        y = x.new_empty((rows, n_out), dtype=out_dtype)
+        y = _empty(x, (rows, n_out), out_dtype)
         rc = _lib("linear_small").sb_linear_small(
-            dt, int(out_float), int(gated), _ptr(x), _ptr(weight), _ptr(y), rows, n_out, k_dim,
+            dt, int(out_float), int(gated), x, weight, y, rows, n_out, k_dim,
             _stream())
         _check(rc, "linear_small")
         return y
     if dt == 0:
-        y = x.new_empty((rows, n_total), dtype=torch.float32)
-        rc = _lib("sgemm").sb_sgemm_nt(_ptr(x), _ptr(weight), _ptr(y), rows, n_total, k_dim,
-                                       _ptr(status), _stream())
+        y = _empty(x, (rows, n_total), torch.float32)
+        rc = _lib("sgemm").sb_sgemm_nt(x, weight, y, rows, n_total, k_dim,
+                                       status, _stream())
         _check(rc, "sgemm")
     elif out_float:
         y = torch.mm(x, weight.t(), out_dtype=torch.float32)
@@ -355,41 +375,59 @@ def _gemm_plan(rows: int, n_out: int, k_dim: int, gated: bool):
     return bm, splits, stages
 
 
+@functools.lru_cache(maxsize=4096)
+def _few_rows_plan(rows: int, n_out: int, k_dim: int, gated: int):
+    """``linear_tensor_core``'s tile height, parts and stages when it is told none of them."""
+    bm, splits, stages = gemm_plan(rows, n_out, k_dim, gated)
+    stages = max(stages, -(-bm * 512 // (16384 + bm * 128)))
+    return bm, splits, min(stages, (226 * 1024) // (16384 + bm * 128))
+
+
+def _refuse_maps(rc, which):
+    if rc in (-3, -4):
+        raise KernelError(f"the TMA descriptors for the {which} product could not be made "
+                          f"(code {rc}); is the driver too old for cuTensorMapEncodeTiled?")
+
+
 def linear_tensor_core(x, weight, out_float=False, gated=False, bm=None, splits=None, stages=None,
-                       status=None, withhold=None):
+                       status=None, withhold=None, checked=False):
     """The bfloat16 product on tcgen05 tensor cores (csrc/gemm_tcgen05.cu).
 
     ``withhold = (k_block, limit_ns)`` is for tests of the kernel's give-up path: the activation copy
     of that k-block is left out, so a wait inside the kernel runs out after ``limit_ns``; the kernel
-    returns, bit 4 of ``status`` is set and the result is undefined."""
-    _need(x, "x", torch.bfloat16, 2)
-    _need(weight, "weight", torch.bfloat16, 2)
-    gated = gate_code(gated)
+    returns, bit 4 of ``status`` is set and the result is undefined.  ``checked``: the caller has looked at the operands
+    and ``gated`` is the kernels' code."""
+    if not checked:
+        _need(x, "x", torch.bfloat16, 2)
+        _need(weight, "weight", torch.bfloat16, 2)
+        gated = gate_code(gated)
     rows, k_dim = x.shape
     n_total = weight.shape[0]
     n_out = n_total // 2 if gated else n_total
-    if weight.shape[1] != k_dim:
-        raise KernelError(f"weight {tuple(weight.shape)} does not take inputs of width {k_dim}")
-    if not tensor_core_ok(x, weight, gated, n_out):
-        raise KernelError(f"the tensor-core product needs k % 8 == 0, 16-byte aligned operands and gated "
-                          f"widths in steps of 64; got k = {k_dim}, n = {n_out}")
-    plan = gemm_plan(rows, n_out, k_dim, gated)
-    bm = bm or plan[0]
-    splits = whole_splits(-(-k_dim // 64), splits or plan[1])
-    stages = stages or max(plan[2], -(-bm * 512 // (16384 + bm * 128)))
-    stages = min(stages, (226 * 1024) // (16384 + bm * 128))     # a tile height other than the plan's
-    out = x.new_empty((rows, n_out), dtype=torch.float32 if out_float else torch.bfloat16)
+    if not checked:
+        if weight.shape[1] != k_dim:
+            raise KernelError(f"weight {tuple(weight.shape)} does not take inputs of width {k_dim}")
+        if not tensor_core_ok(x, weight, gated, n_out):
+            raise KernelError(f"the tensor-core product needs k % 8 == 0, 16-byte aligned operands and gated "
+                              f"widths in steps of 64; got k = {k_dim}, n = {n_out}")
+    if bm or splits or stages:
+        plan = gemm_plan(rows, n_out, k_dim, gated)
+        bm = bm or plan[0]
+        splits = whole_splits(-(-k_dim // 64), splits or plan[1])
+        stages = stages or max(plan[2], -(-bm * 512 // (16384 + bm * 128)))
+        stages = min(stages, (226 * 1024) // (16384 + bm * 128))     # a tile height other than the plan's
+    else:
+        bm, splits, stages = _few_rows_plan(rows, n_out, k_dim, gated)
+    out = _empty(x, (rows, n_out), torch.float32 if out_float else torch.bfloat16)
     if withhold is not None:
         rc = _lib("gemm_tcgen05").sb_gemm_tcgen05_withheld(
-            _ptr(x), _ptr(weight), _ptr(out), rows, n_out, k_dim, bm, splits, stages, int(gated),
-            int(out_float), _ptr(status), ctypes.c_ulonglong(int(withhold[1])), int(withhold[0]), _stream())
+            x, weight, out, rows, n_out, k_dim, bm, splits, stages, int(gated),
+            int(out_float), status, int(withhold[1]), int(withhold[0]), _stream())
     else:
         rc = _lib("gemm_tcgen05").sb_gemm_tcgen05(
-            _ptr(x), _ptr(weight), _ptr(out), rows, n_out, k_dim, bm, splits, stages, int(gated),
-            int(out_float), _ptr(status), _stream())
-    if rc in (-3, -4):
-        raise KernelError("the TMA descriptors for the tensor-core product could not be made "
-                          f"(code {rc}); is the driver too old for cuTensorMapEncodeTiled?")
+            x, weight, out, rows, n_out, k_dim, bm, splits, stages, int(gated),
+            int(out_float), status, _stream())
+    _refuse_maps(rc, "tensor-core")
     _check(rc, "gemm_tcgen05")
     return out
 
@@ -420,18 +458,16 @@ def linear_prompt(x, weight, gated=False, bn=0, pairs=0, status=None, withhold=N
                               f"{'gated ' if gated else ''}product of shape {(rows, n_out)}")
         out = residual
     else:
-        out = x.new_empty((rows, n_out), dtype=torch.bfloat16)
+        out = _empty(x, (rows, n_out), torch.bfloat16)
     lib = _lib("gemm_prompt_tcgen05")
     if withhold is not None:
-        rc = lib.sb_gemm_prompt_withheld(_ptr(x), _ptr(weight), _ptr(out), rows, n_out, k_dim, int(bn), int(pairs),
-                                         int(gated), _ptr(status), ctypes.c_ulonglong(int(withhold[1])),
+        rc = lib.sb_gemm_prompt_withheld(x, weight, out, rows, n_out, k_dim, int(bn), int(pairs),
+                                         int(gated), status, int(withhold[1]),
                                          int(withhold[0]), _stream())
     else:
-        rc = lib.sb_gemm_prompt(_ptr(x), _ptr(weight), _ptr(out), _ptr(residual), rows, n_out, k_dim, int(bn), int(pairs),
-                                int(gated), _ptr(status), _stream())
-    if rc in (-3, -4):
-        raise KernelError("the TMA descriptors for the prompt product could not be made "
-                          f"(code {rc}); is the driver too old for cuTensorMapEncodeTiled?")
+        rc = lib.sb_gemm_prompt(x, weight, out, residual, rows, n_out, k_dim, int(bn), int(pairs),
+                                int(gated), status, _stream())
+    _refuse_maps(rc, "prompt")
     _check(rc, "gemm_prompt_tcgen05")
     return out
 
@@ -490,13 +526,13 @@ def qk_norm_rope_store(qkv, heads, kv_heads, head_dim, q_gain, k_gain, eps, cos_
             if tuple(store.shape[1:]) != (kv_heads, PAGE_TOKENS, head_dim):
                 raise KernelError(f"cache pages have shape {tuple(store.shape)}, expected "
                                   f"[pages, {kv_heads}, {PAGE_TOKENS}, {head_dim}]")
-    q_out = qkv.new_empty((n_tokens, heads * head_dim))
+    q_out = _empty(qkv, (n_tokens, heads * head_dim))
     rc = _lib("rope_cache").sb_qk_norm_rope_store(
-        _code(qkv.dtype), gain_code, _ptr(qkv), _ptr(q_out), _ptr(q_gain), _ptr(k_gain),
-        _ptr(cos_table), _ptr(sin_table), _ptr(tok_pos), _ptr(tok_slot), _ptr(block_table),
-        block_table.shape[1], _ptr(k_store if write_cache else None),
-        _ptr(v_store if write_cache else None), n_tokens, heads, kv_heads, head_dim,
-        ctypes.c_float(eps), int(write_cache), qkv.shape[1], _stream())
+        _code(qkv.dtype), gain_code, qkv, q_out, q_gain, k_gain,
+        cos_table, sin_table, tok_pos, tok_slot, block_table,
+        block_table.shape[1], k_store if write_cache else None,
+        v_store if write_cache else None, n_tokens, heads, kv_heads, head_dim,
+        eps, int(write_cache), qkv.shape[1], _stream())
     _check(rc, "qk_norm_rope_store")
     return q_out
 
@@ -518,11 +554,11 @@ def attention_rowwise(q, k_store, v_store, block_table, tok_slot, tok_pos, heads
     _need(block_table, "block_table", torch.int32, 2)
     _need(tok_slot, "tok_slot", torch.int32, 1)
     _need(tok_pos, "tok_pos", torch.int32, 1)
-    out = torch.empty_like(q)
+    out = _empty(q, q.shape)
     rc = _lib("attention_rowwise").sb_attention_rowwise(
-        _code(q.dtype), _ptr(q), _ptr(out), _ptr(k_store), _ptr(v_store), _ptr(block_table),
-        block_table.shape[1], _ptr(tok_slot), _ptr(tok_pos), q.shape[0], heads, kv_heads, head_dim,
-        ctypes.c_float(scale), int(window or 0), _stream())
+        _code(q.dtype), q, out, k_store, v_store, block_table,
+        block_table.shape[1], tok_slot, tok_pos, q.shape[0], heads, kv_heads, head_dim,
+        scale, int(window or 0), _stream())
     _check(rc, "attention_rowwise")
     return out
 
@@ -560,7 +596,7 @@ def attention_prefill(q, k_store, v_store, block_table, seq_slot, seq_q_start, s
     for name, t in (("seq_slot", seq_slot), ("seq_q_start", seq_q_start), ("seq_q_len", seq_q_len),
                     ("seq_kv_len", seq_kv_len), ("tile_seq", tile_seq), ("tile_first", tile_first)):
         _need(t, name, torch.int32, 1)
-    out = torch.empty_like(q)
+    out = _empty(q, q.shape)
     if kernel is None:
         long_enough = max_q_len is None or max_q_len > 128
         kernel = "tcgen05" if head_dim in PREFILL_TC_HEAD_DIMS and long_enough else "mma"
@@ -576,19 +612,19 @@ def attention_prefill(q, k_store, v_store, block_table, seq_slot, seq_q_start, s
         list_seq, list_first = blocks if own_list else (tile_seq, tile_first)
         if withhold is not None:
             _lib("attention_prefill_tc").sb_attention_prefill_tc_withhold(
-                int(withhold[0]), ctypes.c_ulonglong(int(withhold[1])))
+                int(withhold[0]), int(withhold[1]))
         rc = _lib("attention_prefill_tc").sb_attention_prefill_tc(
-            _ptr(q), _ptr(out), _ptr(k_store), _ptr(v_store), _ptr(block_table), block_table.shape[1],
-            _ptr(seq_slot), _ptr(seq_q_start), _ptr(seq_q_len), _ptr(seq_kv_len), _ptr(list_seq),
-            _ptr(list_first), list_seq.shape[0], q.shape[0], k_store.shape[0], heads, kv_heads, head_dim,
-            ctypes.c_float(scale), int(window or 0), _ptr(status) if status is not None else None,
+            q, out, k_store, v_store, block_table, block_table.shape[1],
+            seq_slot, seq_q_start, seq_q_len, seq_kv_len, list_seq,
+            list_first, list_seq.shape[0], q.shape[0], k_store.shape[0], heads, kv_heads, head_dim,
+            scale, int(window or 0), status if status is not None else None,
             int(own_list), _stream())
         _check(rc, "attention_prefill_tc")
         return out
     rc = _lib("attention_prefill").sb_attention_prefill(
-        _ptr(q), _ptr(out), _ptr(k_store), _ptr(v_store), _ptr(block_table), block_table.shape[1],
-        _ptr(seq_slot), _ptr(seq_q_start), _ptr(seq_q_len), _ptr(seq_kv_len), _ptr(tile_seq),
-        _ptr(tile_first), tile_seq.shape[0], heads, kv_heads, head_dim, ctypes.c_float(scale),
+        q, out, k_store, v_store, block_table, block_table.shape[1],
+        seq_slot, seq_q_start, seq_q_len, seq_kv_len, tile_seq,
+        tile_first, tile_seq.shape[0], heads, kv_heads, head_dim, scale,
         int(window or 0), _stream())
     _check(rc, "attention_prefill")
     return out
@@ -694,17 +730,17 @@ def attention_decode_qkv(qkv, k_store, v_store, block_table, row_slot, row_kv_le
             raise KernelError("rotary tables must be [positions, head_dim / 2]")
     if n_splits is None:
         n_splits = decode_splits(rows, kv_heads, heads // kv_heads, 16, kv_hint)
-    out = qkv.new_empty((rows, heads * head_dim))
+    out = _empty(qkv, (rows, heads * head_dim))
     part_acc = part_ml = None
     in_cluster = 1 < n_splits <= DECODE_CLUSTER_SPLITS
     if n_splits > 1 and not in_cluster:
-        part_acc = qkv.new_empty((rows * heads * n_splits * head_dim,), dtype=torch.float32)
-        part_ml = qkv.new_empty((rows * heads * n_splits * 2,), dtype=torch.float32)
+        part_acc = _empty(qkv, (rows * heads * n_splits * head_dim,), torch.float32)
+        part_ml = _empty(qkv, (rows * heads * n_splits * 2,), torch.float32)
     rc = _lib("attention_decode_mma").sb_attention_decode_mma_fused(
-        _ptr(qkv), qkv.shape[1], _ptr(out), _ptr(k_store), _ptr(v_store), _ptr(block_table),
-        block_table.shape[1], _ptr(row_slot), _ptr(row_kv_len), rows, heads, kv_heads, head_dim,
-        ctypes.c_float(scale), int(window or 0), n_splits, _ptr(part_acc), _ptr(part_ml), _ptr(q_gain),
-        _ptr(k_gain), gain_code, ctypes.c_float(eps), _ptr(cos_table), _ptr(sin_table), int(write_cache),
+        qkv, qkv.shape[1], out, k_store, v_store, block_table,
+        block_table.shape[1], row_slot, row_kv_len, rows, heads, kv_heads, head_dim,
+        scale, int(window or 0), n_splits, part_acc, part_ml, q_gain,
+        k_gain, gain_code, eps, cos_table, sin_table, int(write_cache),
         int(bool(early) and write_cache and EARLY_READS), _stream())
     _check(rc, "attention_decode_fused", 2 if n_splits > 1 and not in_cluster else 1)
     return out
@@ -739,27 +775,27 @@ def attention_decode(q, k_store, v_store, block_table, row_slot, row_kv_len, hea
     tensor_cores = q.dtype == torch.bfloat16 and head_dim in PREFILL_HEAD_DIMS
     if n_splits is None:
         n_splits = decode_splits(rows, kv_heads, heads // kv_heads, 16 if tensor_cores else 4, kv_hint)
-    out = torch.empty_like(q)
+    out = _empty(q, q.shape)
     part_acc = part_ml = None
     # up to DECODE_CLUSTER_SPLITS splits of the tensor-core kernel are one thread-block cluster and
     # merge through distributed shared memory; more go through scratch and a merge kernel
     in_cluster = tensor_cores and 1 < n_splits <= DECODE_CLUSTER_SPLITS
     if n_splits > 1 and not in_cluster:
-        part_acc = q.new_empty((rows * heads * n_splits * head_dim,), dtype=torch.float32)
-        part_ml = q.new_empty((rows * heads * n_splits * 2,), dtype=torch.float32)
+        part_acc = _empty(q, (rows * heads * n_splits * head_dim,), torch.float32)
+        part_ml = _empty(q, (rows * heads * n_splits * 2,), torch.float32)
     if tensor_cores:
         rc = _lib("attention_decode_mma").sb_attention_decode_mma(
-            _ptr(q), _ptr(out), _ptr(k_store), _ptr(v_store), _ptr(block_table), block_table.shape[1],
-            _ptr(row_slot), _ptr(row_kv_len), rows, heads, kv_heads, head_dim, ctypes.c_float(scale),
-            int(window or 0), n_splits, _ptr(part_acc), _ptr(part_ml), _stream())
+            q, out, k_store, v_store, block_table, block_table.shape[1],
+            row_slot, row_kv_len, rows, heads, kv_heads, head_dim, scale,
+            int(window or 0), n_splits, part_acc, part_ml, _stream())
     else:
         if withhold is not None:
-            _lib("attention_decode").sb_attention_decode_withhold(int(withhold[0]), ctypes.c_ulonglong(int(withhold[1])))
+            _lib("attention_decode").sb_attention_decode_withhold(int(withhold[0]), int(withhold[1]))
         rc = _lib("attention_decode").sb_attention_decode(
-            _code(q.dtype), _ptr(q), _ptr(out), _ptr(k_store), _ptr(v_store), _ptr(block_table),
-            block_table.shape[1], _ptr(row_slot), _ptr(row_kv_len), rows, heads, kv_heads, head_dim,
-            ctypes.c_float(scale), int(window or 0), n_splits, _ptr(part_acc), _ptr(part_ml),
-            _ptr(status), _stream())
+            _code(q.dtype), q, out, k_store, v_store, block_table,
+            block_table.shape[1], row_slot, row_kv_len, rows, heads, kv_heads, head_dim,
+            scale, int(window or 0), n_splits, part_acc, part_ml,
+            status, _stream())
     _check(rc, "attention_decode", 2 if n_splits > 1 and not in_cluster else 1)
     return out
 
@@ -781,10 +817,10 @@ def embedding_streams(tokens, table, streams: int, status=None, fence=False):
     residual streams of a model with hyper-connections at their start.  ``fence`` as in ``embedding``."""
     _need(tokens, "tokens", torch.int32, 1)
     _need(table, "table", None, 2)
-    out = table.new_empty((tokens.shape[0], streams, table.shape[1]), dtype=torch.float32)
+    out = _empty(table, (tokens.shape[0], streams, table.shape[1]), torch.float32)
     rc = _lib("streams").sb_embed_streams(
-        _code(table.dtype), _ptr(tokens), _ptr(table), _ptr(out), tokens.shape[0], table.shape[1],
-        table.shape[0], int(streams), _ptr(status), int(fence), _stream())
+        _code(table.dtype), tokens, table, out, tokens.shape[0], table.shape[1],
+        table.shape[0], int(streams), status, int(fence), _stream())
     _check(rc, "embedding_streams")
     return out
 
@@ -833,10 +869,10 @@ def hyper_step(streams, dtype, pending=None, read=None, norm=None, rows=None):
     if rows is not None:
         _need(rows, "rows", torch.int32, 1)
         n_rows = rows.shape[0]
-    normed = streams.new_empty((n_rows, hidden), dtype=dtype)
+    normed = _empty(streams, (n_rows, hidden), dtype)
     rc = _lib("streams").sb_hyper_step(
-        _code(dtype), n_streams, _ptr(streams), _ptr(y), _ptr(bias), _ptr(scale), _ptr(mix), _ptr(out), _ptr(read),
-        kind, _ptr(alpha), _ptr(weight), _ptr(shift), ctypes.c_float(eps), _ptr(normed), _ptr(rows), n_rows,
+        _code(dtype), n_streams, streams, y, bias, scale, mix, out, read,
+        kind, alpha, weight, shift, eps, normed, rows, n_rows,
         hidden, _stream())
     if rc == -2:
         raise KernelError(f"the stream kernels take 1 to {max_streams()} streams, not {n_streams} (with an RMS norm: rows "
@@ -861,9 +897,9 @@ def dynamic_tanh(x, alpha, weight, bias, delta=None, rows=None):
     if rows is not None:
         _need(rows, "rows", torch.int32, 1)
         n_rows = rows.shape[0]
-    out = x.new_empty((n_rows, hidden))
-    rc = _lib("streams").sb_dyt(_code(x.dtype), _ptr(x), _ptr(delta), _ptr(alpha), _ptr(weight), _ptr(bias),
-                                _ptr(out), _ptr(rows), n_rows, hidden, _stream())
+    out = _empty(x, (n_rows, hidden))
+    rc = _lib("streams").sb_dyt(_code(x.dtype), x, delta, alpha, weight, bias,
+                                out, rows, n_rows, hidden, _stream())
     _check(rc, "dynamic_tanh")
     return out
 
@@ -907,17 +943,17 @@ def diff_attention_prefill(q, gate, k_store, v_store, block_table, seq_slot, seq
              and (gate is None or (gate_stride % 8 == 0 and gate.data_ptr() % 16 == 0)))
     if kernel is None:
         kernel = "tcgen05" if tc_ok and (max_q_len is None or max_q_len >= 128) else "mma"
-    out = q.new_empty((q.shape[0], heads * v_dim))
+    out = _empty(q, (q.shape[0], heads * v_dim))
     if kernel == "tcgen05":
         if not tc_ok:
             raise KernelError(f"the tcgen05 differential attention takes dim 64 and v_dim 64 or 128 in bfloat16 with "
                               f"16-byte aligned rows; got dim {dim}, v_dim {v_dim}, {q.dtype}")
         rc = _lib("attention_diff_prefill_tc").sb_diff_prefill_tc(
-            _ptr(q), _ptr(gate), int(gate_stride), _ptr(out), _ptr(k_store), _ptr(v_store), _ptr(block_table),
-            block_table.shape[1], _ptr(seq_slot), _ptr(seq_q_start), _ptr(seq_q_len), _ptr(seq_kv_len),
-            _ptr(tile_seq), _ptr(tile_first), tile_seq.shape[0], q.shape[0], k_store.shape[0], heads, kv_heads, dim,
-            v_dim, ctypes.c_float(scale), int(window or 0), ctypes.c_float(lam), ctypes.c_float(out_scale),
-            ctypes.c_float(eps), _ptr(status), _stream())
+            q, gate, int(gate_stride), out, k_store, v_store, block_table,
+            block_table.shape[1], seq_slot, seq_q_start, seq_q_len, seq_kv_len,
+            tile_seq, tile_first, tile_seq.shape[0], q.shape[0], k_store.shape[0], heads, kv_heads, dim,
+            v_dim, scale, int(window or 0), lam, out_scale,
+            eps, status, _stream())
         if rc in (-3, -4):
             raise KernelError(f"the TMA descriptors for the differential attention could not be made (code {rc})")
         _check(rc, "diff_attention_prefill_tc")
@@ -927,10 +963,10 @@ def diff_attention_prefill(q, gate, k_store, v_store, block_table, seq_slot, seq
     if gate is not None and (gate_stride % 2 or gate.data_ptr() % 4):
         raise KernelError("the gate's rows must start on 4-byte boundaries")
     rc = _lib("attention_diff_prefill").sb_diff_prefill(
-        _ptr(q), _ptr(gate), int(gate_stride), _ptr(out), _ptr(k_store), _ptr(v_store), _ptr(block_table),
-        block_table.shape[1], _ptr(seq_slot), _ptr(seq_q_start), _ptr(seq_q_len), _ptr(seq_kv_len),
-        _ptr(tile_seq), _ptr(tile_first), tile_seq.shape[0], heads, kv_heads, dim, v_dim, ctypes.c_float(scale),
-        int(window or 0), ctypes.c_float(lam), ctypes.c_float(out_scale), ctypes.c_float(eps), _stream())
+        q, gate, int(gate_stride), out, k_store, v_store, block_table,
+        block_table.shape[1], seq_slot, seq_q_start, seq_q_len, seq_kv_len,
+        tile_seq, tile_first, tile_seq.shape[0], heads, kv_heads, dim, v_dim, scale,
+        int(window or 0), lam, out_scale, eps, _stream())
     _check(rc, "diff_attention_prefill")
     return out
 
@@ -964,12 +1000,12 @@ def diff_prepare(proj, bias, heads, kv_heads, dim, v_dim, gate_width, temperatur
             raise KernelError(f"cache pages have shapes {tuple(k_store.shape)} and {tuple(v_store.shape)}, expected "
                               f"[pages, {kv_heads}, {PAGE_TOKENS}, {2 * dim}] and [pages, {kv_heads}, {PAGE_TOKENS}, {v_dim}]")
     coef, every = temperature if temperature is not None else (0.0, 0)
-    q_out = proj.new_empty((n_tokens, q_w))
+    q_out = _empty(proj, (n_tokens, q_w))
     rc = _lib("attention_diff").sb_diff_prepare(
-        _code(proj.dtype), _ptr(proj), proj.shape[1], _ptr(bias), _ptr(q_out), _ptr(tok_pos), _ptr(tok_slot),
-        _ptr(block_table), block_table.shape[1], _ptr(k_store if write_cache else None),
-        _ptr(v_store if write_cache else None), n_tokens, heads, kv_heads, dim, v_dim, gate_width,
-        ctypes.c_float(coef), int(every), int(write_cache), _stream())
+        _code(proj.dtype), proj, proj.shape[1], bias, q_out, tok_pos, tok_slot,
+        block_table, block_table.shape[1], k_store if write_cache else None,
+        v_store if write_cache else None, n_tokens, heads, kv_heads, dim, v_dim, gate_width,
+        coef, int(every), int(write_cache), _stream())
     _check(rc, "diff_prepare")
     return q_out
 
@@ -1009,12 +1045,12 @@ def diff_attention(q, gate, k_store, v_store, block_table, tok_slot, tok_pos, he
     _need(tok_pos, "tok_pos", torch.int32, 1)
     if warps is None:
         warps = 1 if kv_hint <= 32 else 2 if kv_hint <= 128 else 4 if kv_hint <= 512 else 8
-    out = q.new_empty((q.shape[0], heads * v_dim))
+    out = _empty(q, (q.shape[0], heads * v_dim))
     rc = _lib("attention_diff").sb_diff_attention(
-        _code(q.dtype), _ptr(q), _ptr(gate), int(gate_stride), _ptr(out), _ptr(k_store), _ptr(v_store),
-        _ptr(block_table), block_table.shape[1], _ptr(tok_slot), _ptr(tok_pos), q.shape[0], heads, kv_heads,
-        dim, v_dim, ctypes.c_float(scale), int(window or 0), ctypes.c_float(lam), ctypes.c_float(out_scale),
-        ctypes.c_float(eps), int(warps), _stream())
+        _code(q.dtype), q, gate, int(gate_stride), out, k_store, v_store,
+        block_table, block_table.shape[1], tok_slot, tok_pos, q.shape[0], heads, kv_heads,
+        dim, v_dim, scale, int(window or 0), lam, out_scale,
+        eps, int(warps), _stream())
     _check(rc, "diff_attention")
     return out
 
@@ -1054,15 +1090,15 @@ def diff_attention_decode(q, gate, k_store, v_store, block_table, row_slot, row_
         through_scratch = max(1, min(pages // 7, resident, 64))
         if through_scratch >= 3 * n_splits:
             n_splits = through_scratch
-    out = q.new_empty((rows, heads * v_dim))
+    out = _empty(q, (rows, heads * v_dim))
     part = None
     if not cluster or n_splits > DIFF_CLUSTER_PARTS:
-        part = q.new_empty((rows * heads * n_splits * 2 * (v_dim + 2),), dtype=torch.float32)
+        part = _empty(q, (rows * heads * n_splits * 2 * (v_dim + 2),), torch.float32)
     rc = _lib("attention_diff_prefill").sb_diff_decode(
-        _ptr(q), _ptr(gate), int(gate_stride), _ptr(out), _ptr(k_store), _ptr(v_store), _ptr(block_table),
-        block_table.shape[1], _ptr(row_slot), _ptr(row_kv_len), rows, heads, kv_heads, dim, v_dim,
-        ctypes.c_float(scale), int(window or 0), ctypes.c_float(lam), ctypes.c_float(out_scale), ctypes.c_float(eps),
-        int(n_splits), _ptr(part), int(bool(early) and EARLY_READS), int(bool(cluster)), _stream())
+        q, gate, int(gate_stride), out, k_store, v_store, block_table,
+        block_table.shape[1], row_slot, row_kv_len, rows, heads, kv_heads, dim, v_dim,
+        scale, int(window or 0), lam, out_scale, eps,
+        int(n_splits), part, int(bool(early) and EARLY_READS), int(bool(cluster)), _stream())
     # 0: one launch; 1: two (walk and merge); above: a CUDA error code plus one
     _check(rc - 1 if rc > 1 else 0 if rc == 1 else rc, "diff_attention_decode", 2 if rc == 1 else 1)
     return out
@@ -1093,7 +1129,7 @@ def add_bias(y, bias):
     """``y += bias`` in place (``bias`` float32 ``[N]``, the sum rounded once to ``y``'s type)."""
     _need(y, "y", None, 2)
     _f32(bias, "bias", (y.shape[1],))
-    rc = _lib("streams").sb_add_bias(_code(y.dtype), _ptr(y), _ptr(bias), y.shape[0], y.shape[1], _stream())
+    rc = _lib("streams").sb_add_bias(_code(y.dtype), y, bias, y.shape[0], y.shape[1], _stream())
     _check(rc, "add_bias")
     return y
 
@@ -1112,16 +1148,16 @@ def sample(logits, temperature=None, request_key=None, position=None, status=Non
         _need(request_key, "request_key", torch.int32, 1)
         _need(position, "position", torch.int32, 1)
     if out is None:
-        out = logits.new_empty((rows,), dtype=torch.int32)
+        out = _empty(logits, (rows,), torch.int32)
     lib = _lib("sampling")
     chunks = lib.sb_sample_chunks(vocab)
-    cand_v = logits.new_empty((rows * chunks,), dtype=torch.float32)
-    cand_i = logits.new_empty((rows * chunks,), dtype=torch.int32)
+    cand_v = _empty(logits, (rows * chunks,), torch.float32)
+    cand_i = _empty(logits, (rows * chunks,), torch.int32)
     rc = lib.sb_sample(
-        _ptr(logits), rows, vocab, ctypes.c_longlong(logits.stride(0)), _ptr(temperature),
-        _ptr(request_key), _ptr(position), _ptr(out), _ptr(status),
-        _ptr(feed[0] if feed else None), _ptr(feed[1] if feed else None),
-        _ptr(feed[2] if feed else None), _ptr(cand_v), _ptr(cand_i), _stream())
+        logits, rows, vocab, logits.stride(0), temperature,
+        request_key, position, out, status,
+        feed[0] if feed else None, feed[1] if feed else None,
+        feed[2] if feed else None, cand_v, cand_i, _stream())
     _check(rc, "sample", 2)
     return out
 
@@ -1304,8 +1340,8 @@ class OpenChain:
             for j, v in enumerate(d):
                 desc[16 * i + j] = v
         rc = _lib("dense_chain").sb_dense_chain(
-            desc, eps, len(self.stages), self.rows, _ptr(sync), _ptr(self.status), ctypes.c_ulonglong(0),
-            _ptr(self.trace), _stream())
+            ctypes.addressof(desc), ctypes.addressof(eps), len(self.stages), self.rows, sync, self.status, 0,
+            self.trace, _stream())
         if rc in (-3, -4):
             raise KernelError(f"the TMA descriptors for a chain could not be made (code {rc})")
         _check(rc, "dense_chain")
@@ -1320,12 +1356,12 @@ def embedding32(tokens, table, scale=1.0, status=None, fence=False, out=None):
     _need(tokens, "tokens", torch.int32, 1)
     _need(table, "table", None, 2)
     if out is None:
-        out = table.new_empty((tokens.shape[0], table.shape[1]), dtype=torch.float32)
+        out = _empty(table, (tokens.shape[0], table.shape[1]), torch.float32)
     else:
         _f32(out, "out", (tokens.shape[0], table.shape[1]))
     rc = _lib("residual32").sb_embed32(
-        _code(table.dtype), _ptr(tokens), _ptr(table), _ptr(out), tokens.shape[0], table.shape[1],
-        table.shape[0], ctypes.c_float(scale), _ptr(status), int(fence), _stream())
+        _code(table.dtype), tokens, table, out, tokens.shape[0], table.shape[1],
+        table.shape[0], scale, status, int(fence), _stream())
     _check(rc, "embedding32")
     return out
 
@@ -1363,10 +1399,10 @@ def residual_norm(x, dtype, eps, pending=None, next_gain=None, rows=None):
     out = None
     if next_gain is not None:
         _f32(next_gain, "next gain", (hidden,))
-        out = x.new_empty((n_rows, hidden), dtype=dtype)
+        out = _empty(x, (n_rows, hidden), dtype)
     rc = _lib("residual32").sb_residual_norm(
-        _code(dtype), _ptr(x), _ptr(y), _ptr(y2), _ptr(bias), _ptr(post), _ptr(next_gain), _ptr(out), _ptr(rows), n_rows,
-        hidden, ctypes.c_float(post_eps), ctypes.c_float(eps), _stream())
+        _code(dtype), x, y, y2, bias, post, next_gain, out, rows, n_rows,
+        hidden, post_eps, eps, _stream())
     _check(rc, "residual_norm")
     return out
 
@@ -1389,10 +1425,10 @@ def residual_join(x, pending, tokens, table, scale=1.0):
             _need(t, "y", table.dtype, 2)
             if tuple(t.shape) != (n_tokens, hidden):
                 raise KernelError(f"y {tuple(t.shape)} does not match the residual stream {tuple(x.shape)}")
-    out = x.new_empty((n_tokens, 2 * hidden), dtype=table.dtype)
+    out = _empty(x, (n_tokens, 2 * hidden), table.dtype)
     rc = _lib("residual32").sb_residual_join(
-        _code(table.dtype), _ptr(x), _ptr(y), _ptr(y2), _ptr(tokens), _ptr(table), _ptr(out), n_tokens, hidden,
-        table.shape[0], ctypes.c_float(scale), _stream())
+        _code(table.dtype), x, y, y2, tokens, table, out, n_tokens, hidden,
+        table.shape[0], scale, _stream())
     _check(rc, "residual_join")
     return out
 
@@ -1410,8 +1446,8 @@ def bias_act(x, bias=None, activation=None):
         raise KernelError(f"no activation {activation!r} here (known: relu2, tanh)")
     if bias is not None:
         _f32(bias, "bias", (x.shape[1],))
-    out = torch.empty_like(x)
-    rc = _lib("residual32").sb_bias_act(_code(x.dtype), _ptr(x), _ptr(bias), _ptr(out), x.shape[0], x.shape[1],
+    out = _empty(x, x.shape)
+    rc = _lib("residual32").sb_bias_act(_code(x.dtype), x, bias, out, x.shape[0], x.shape[1],
                                         BIAS_ACTIVATIONS[activation], _stream())
     _check(rc, "bias_act")
     return out
@@ -1435,9 +1471,9 @@ def token_shift(h, state, mu, tok_slot):
     n_tokens, width = h.shape
     if mu.shape[1] != width or state.shape[1] < width:
         raise KernelError(f"mu {tuple(mu.shape)} / state {tuple(state.shape)} do not fit rows of {width}")
-    out = h.new_empty((mu.shape[0], n_tokens, width))
-    rc = _lib("wkv").sb_token_shift(_code(h.dtype), _ptr(h), _ptr(state), ctypes.c_longlong(state.shape[1]), _ptr(mu),
-                                    _ptr(out), _ptr(tok_slot), n_tokens, width, mu.shape[0], _stream())
+    out = _empty(h, (mu.shape[0], n_tokens, width))
+    rc = _lib("wkv").sb_token_shift(_code(h.dtype), h, state, state.shape[1], mu,
+                                    out, tok_slot, n_tokens, width, mu.shape[0], _stream())
     _check(rc, "token_shift")
     return out
 
@@ -1473,13 +1509,13 @@ def wkv_scan(r, k, v, decay, u, g, gain, state, h, seq_slot, seq_q_start, seq_q_
         raise KernelError(f"a slot's state has {state.shape[1]} floats, expected {width + heads * dim * dim}")
     for name, t in (("seq_slot", seq_slot), ("seq_q_start", seq_q_start), ("seq_q_len", seq_q_len)):
         _need(t, name, torch.int32, 1)
-    out = torch.empty_like(r)
+    out = _empty(r, r.shape)
     # many tokens of few sequences: scratch with which several blocks may share a head
-    o32 = r.new_empty((n_tokens, hd), dtype=torch.float32) if n_tokens >= 4 * seq_slot.shape[0] else None
+    o32 = _empty(r, (n_tokens, hd), torch.float32) if n_tokens >= 4 * seq_slot.shape[0] else None
     rc = _lib("wkv").sb_wkv_scan(
-        _code(r.dtype), _ptr(r), _ptr(k), _ptr(v), _ptr(decay), _ptr(u), _ptr(g), _ptr(gain),
-        _ptr(state), ctypes.c_longlong(state.shape[1]), width, _ptr(h), width, _ptr(out), _ptr(seq_slot),
-        _ptr(seq_q_start), _ptr(seq_q_len), seq_slot.shape[0], heads, dim, ctypes.c_float(eps), _ptr(o32), n_tokens,
+        _code(r.dtype), r, k, v, decay, u, g, gain,
+        state, state.shape[1], width, h, width, out, seq_slot,
+        seq_q_start, seq_q_len, seq_slot.shape[0], heads, dim, eps, o32, n_tokens,
         _stream())
     if rc == -2:
         raise KernelError(f"the recurrence kernel takes heads of 1 to {wkv_max_dim()} channels, not {dim}")
@@ -1535,11 +1571,11 @@ def latent_prepare(proj, q_gain, kv_gain, eps, cos_table, sin_table, tok_pos, to
         _need(store, "cache pages", proj.dtype, 4)
         if tuple(store.shape[1:]) != (1, PAGE_TOKENS, rank + rot):
             raise KernelError(f"cache pages have shape {tuple(store.shape)}, expected [pages, 1, {PAGE_TOKENS}, {rank + rot}]")
-    cq = proj.new_empty((n_tokens, q_rank))
+    cq = _empty(proj, (n_tokens, q_rank))
     rc = _lib("attention_latent").sb_latent_prepare(
-        _code(proj.dtype), _ptr(proj), proj.shape[1], _ptr(q_gain), _ptr(kv_gain if write_cache else None),
-        ctypes.c_float(eps), _ptr(cos_table), _ptr(sin_table), cos_table.shape[1], _ptr(tok_pos), _ptr(tok_slot),
-        _ptr(block_table), block_table.shape[1], _ptr(store if write_cache else None), _ptr(cq), n_tokens, q_rank,
+        _code(proj.dtype), proj, proj.shape[1], q_gain, kv_gain if write_cache else None,
+        eps, cos_table, sin_table, cos_table.shape[1], tok_pos, tok_slot,
+        block_table, block_table.shape[1], store if write_cache else None, cq, n_tokens, q_rank,
         kv_col, rank, rot, rot_dims, int(write_cache), LATENT_LAYOUTS[layout], _stream())
     _check(rc, "latent_prepare")
     return cq
@@ -1553,7 +1589,7 @@ def latent_rotate_q(q, qa, cos_table, sin_table, tok_pos, heads, dim, rot, rot_d
     if q.shape[1] != heads * (dim + rot) or tuple(qa.shape) != (q.shape[0], heads, rank + rot):
         raise KernelError(f"q {tuple(q.shape)} / qa {tuple(qa.shape)} do not fit {heads} heads of {dim} + {rot}")
     rc = _lib("attention_latent").sb_latent_rotate_q(
-        _code(q.dtype), _ptr(q), _ptr(qa), _ptr(cos_table), _ptr(sin_table), cos_table.shape[1], _ptr(tok_pos),
+        _code(q.dtype), q, qa, cos_table, sin_table, cos_table.shape[1], tok_pos,
         q.shape[0], heads, dim, rot, rot_dims, rank, LATENT_LAYOUTS[layout], _stream())
     _check(rc, "latent_rotate_q")
 
@@ -1561,7 +1597,7 @@ def latent_rotate_q(q, qa, cos_table, sin_table, tok_pos, heads, dim, rot, rot_d
 def _latent_sink(sink, heads):
     if sink is not None:
         _f32(sink, "sink", (heads,))
-    return _ptr(sink)
+    return sink
 
 
 def latent_attention(qa, store, block_table, tok_slot, tok_pos, heads, rank, rot, scale, window=None, sink=None):
@@ -1580,10 +1616,10 @@ def latent_attention(qa, store, block_table, tok_slot, tok_pos, heads, rank, rot
     _need(block_table, "block_table", torch.int32, 2)
     _need(tok_slot, "tok_slot", torch.int32, 1)
     _need(tok_pos, "tok_pos", torch.int32, 1)
-    out = qa.new_empty((n_tokens, heads, rank))
+    out = _empty(qa, (n_tokens, heads, rank))
     rc = _lib("attention_latent").sb_latent_attention(
-        _code(qa.dtype), _ptr(qa), _ptr(out), _ptr(store), _ptr(block_table), block_table.shape[1], _ptr(tok_slot),
-        _ptr(tok_pos), n_tokens, heads, rank, rot, ctypes.c_float(scale), int(window or 0), _latent_sink(sink, heads), _stream())
+        _code(qa.dtype), qa, out, store, block_table, block_table.shape[1], tok_slot,
+        tok_pos, n_tokens, heads, rank, rot, scale, int(window or 0), _latent_sink(sink, heads), _stream())
     _check(rc, "latent_attention")
     return out
 
@@ -1615,16 +1651,16 @@ def latent_attention_tc(qa, store, block_table, seq_slot, seq_q_start, seq_q_len
     for name, t in (("seq_slot", seq_slot), ("seq_q_start", seq_q_start), ("seq_q_len", seq_q_len),
                     ("seq_kv_len", seq_kv_len), ("tile_seq", tile_seq), ("tile_first", tile_first)):
         _need(t, name, torch.int32, 1)
-    out = qa.new_empty((n_tokens, heads, rank))
+    out = _empty(qa, (n_tokens, heads, rank))
     part_acc = part_ml = None
     n_splits = max(1, int(n_splits))
     if n_splits > 1:
-        part_acc = qa.new_empty((n_splits, n_tokens * heads, rank), dtype=torch.float32)
-        part_ml = qa.new_empty((n_splits, n_tokens * heads, 2), dtype=torch.float32)
+        part_acc = _empty(qa, (n_splits, n_tokens * heads, rank), torch.float32)
+        part_ml = _empty(qa, (n_splits, n_tokens * heads, 2), torch.float32)
     rc = _lib("attention_latent").sb_latent_attention_tc(
-        _ptr(qa), _ptr(out), _ptr(part_acc), _ptr(part_ml), _ptr(store), _ptr(block_table), block_table.shape[1],
-        _ptr(seq_slot), _ptr(seq_q_start), _ptr(seq_q_len), _ptr(seq_kv_len), _ptr(tile_seq), _ptr(tile_first),
-        tile_seq.shape[0], n_tokens, heads, rank, rot, ctypes.c_float(scale), int(window or 0), n_splits,
+        qa, out, part_acc, part_ml, store, block_table, block_table.shape[1],
+        seq_slot, seq_q_start, seq_q_len, seq_kv_len, tile_seq, tile_first,
+        tile_seq.shape[0], n_tokens, heads, rank, rot, scale, int(window or 0), n_splits,
         int(max_q_len), _latent_sink(sink, heads), _stream())
     _check(rc, "latent_attention_tc", 2 if n_splits > 1 else 1)
     return out
@@ -1713,19 +1749,19 @@ def latent_attention_prompt(q, ukv, store, block_table, ctx, heads, dim, vdim, r
         _need(t, name, torch.int32, 1)
     each = _latent_prompt_rows(ctx, window)
     rows = sum(each)
-    gathered = q.new_empty((rows * (rank + rot),))
+    gathered = _empty(q, (rows * (rank + rot),))
     c, shared = gathered[:rows * rank].view(rows, rank), gathered[rows * rank:].view(rows, rot)
     lib = _lib("attention_latent_prompt")
-    rc = lib.sb_latent_gather(_ptr(store), _ptr(block_table), block_table.shape[1], _ptr(ctx.seq_slot), _ptr(ctx.seq_q_len),
-                              _ptr(ctx.seq_kv_len), n_seqs, max(each), _ptr(c), _ptr(shared), rank, rot, int(window or 0),
+    rc = lib.sb_latent_gather(store, block_table, block_table.shape[1], ctx.seq_slot, ctx.seq_q_len,
+                              ctx.seq_kv_len, n_seqs, max(each), c, shared, rank, rot, int(window or 0),
                               _stream())
     _check(rc, "latent_gather")
     kv = linear(c, ukv, status=ctx.status)
-    out = q.new_empty((n_tokens, heads * vdim))
+    out = _empty(q, (n_tokens, heads * vdim))
     rc = lib.sb_latent_prompt(
-        _ptr(q), _ptr(kv), _ptr(shared), _ptr(out), _ptr(ctx.seq_q_start), _ptr(ctx.seq_q_len), _ptr(ctx.seq_kv_len),
-        _ptr(ctx.block_seq), _ptr(ctx.block_first), ctx.block_seq.shape[0], n_tokens, rows, heads, dim, vdim,
-        ctypes.c_float(scale), int(window or 0), _latent_sink(sink, heads), _ptr(ctx.status), _stream())
+        q, kv, shared, out, ctx.seq_q_start, ctx.seq_q_len, ctx.seq_kv_len,
+        ctx.block_seq, ctx.block_first, ctx.block_seq.shape[0], n_tokens, rows, heads, dim, vdim,
+        scale, int(window or 0), _latent_sink(sink, heads), ctx.status, _stream())
     _check(rc, "latent_attention_prompt")
     return out
 
@@ -1736,7 +1772,7 @@ def sigmoid_gate(a, gate, gate_col):
     _need(gate, "gate", a.dtype, 2)
     if gate.shape[0] != a.shape[0] or gate_col < 0 or gate_col + a.shape[1] > gate.shape[1]:
         raise KernelError(f"{a.shape[1]} columns from {gate_col} of {tuple(gate.shape)} do not gate {tuple(a.shape)}")
-    rc = _lib("elementwise").sb_sigmoid_gate(_code(a.dtype), _ptr(a), _at(gate, gate_col), gate.shape[1], a.shape[1],
+    rc = _lib("elementwise").sb_sigmoid_gate(_code(a.dtype), a, _at(gate, gate_col), gate.shape[1], a.shape[1],
                                              a.shape[0], _stream())
     _check(rc, "sigmoid_gate")
 
@@ -1766,11 +1802,11 @@ def moe_route(h, router, router_bias, top, scoring="softmax_top", weight_scale=1
     _f32(router, "router", (experts, h.shape[1]))
     if router_bias is not None:
         _f32(router_bias, "router bias", (experts,))
-    ids = h.new_empty((h.shape[0], top), dtype=torch.int32)
-    weights = h.new_empty((h.shape[0], top), dtype=torch.float32)
-    rc = _lib("moe").sb_moe_route(_code(h.dtype), _ptr(h), _ptr(router), _ptr(router_bias), _ptr(ids), _ptr(weights),
+    ids = _empty(h, (h.shape[0], top), torch.int32)
+    weights = _empty(h, (h.shape[0], top), torch.float32)
+    rc = _lib("moe").sb_moe_route(_code(h.dtype), h, router, router_bias, ids, weights,
                                   h.shape[0], h.shape[1], experts, top, MOE_SCORINGS[scoring],
-                                  ctypes.c_float(weight_scale), _stream())
+                                  weight_scale, _stream())
     if rc == -2:
         raise KernelError(f"the router takes up to {moe_limits()[0]} experts and {moe_limits()[1]} choices, not "
                           f"{experts} and {top}")
@@ -1790,12 +1826,12 @@ def moe_route_all(h, router, correction, top, groups=1, keep=1, weight_scale=1.0
     _f32(router, "router", (router.shape[0], h.shape[1]))
     if correction is not None:
         _f32(correction, "correction", (outputs,))
-    ids = h.new_empty((h.shape[0], top), dtype=torch.int32)
-    weights = h.new_empty((h.shape[0], top), dtype=torch.float32)
-    gate = h.new_empty((h.shape[0],), dtype=torch.float32) if shared_gate else None
-    rc = _lib("moe").sb_moe_route_all(_code(h.dtype), _ptr(h), _ptr(router), _ptr(correction), _ptr(ids), _ptr(weights),
-                                      _ptr(gate), h.shape[0], h.shape[1], outputs, top, groups, keep,
-                                      ctypes.c_float(weight_scale), _stream())
+    ids = _empty(h, (h.shape[0], top), torch.int32)
+    weights = _empty(h, (h.shape[0], top), torch.float32)
+    gate = _empty(h, (h.shape[0],), torch.float32) if shared_gate else None
+    rc = _lib("moe").sb_moe_route_all(_code(h.dtype), h, router, correction, ids, weights,
+                                      gate, h.shape[0], h.shape[1], outputs, top, groups, keep,
+                                      weight_scale, _stream())
     if rc == -2:
         raise KernelError(f"the router takes up to {moe_limits()[0]} outputs and {moe_limits()[1]} choices among the "
                           f"kept groups, not {outputs} outputs, {top} choices, {keep} of {groups} groups")
@@ -1834,8 +1870,8 @@ def moe_experts(h, ids, weights, gate_up, down, limit=0.0, expert="gated_clamped
         _f32(shared_gate, "shared gate", (h.shape[0],))
         if tuple(shared.shape) != tuple(h.shape):
             raise KernelError(f"the shared expert's output {tuple(shared.shape)} does not match the rows {tuple(h.shape)}")
-    extras = (_ptr(ids if identity else None), gate_up.shape[0], _ptr(h if identity else None), _ptr(shared),
-              _ptr(shared_gate if shared is not None else None))
+    extras = (ids if identity else None, gate_up.shape[0], h if identity else None, shared,
+              shared_gate if shared is not None else None)
     _need(gate_up, "gate_up", h.dtype, 3)
     _need(down, "down", h.dtype, 3)
     _need(ids, "ids", torch.int32, 2)
@@ -1849,48 +1885,48 @@ def moe_experts(h, ids, weights, gate_up, down, limit=0.0, expert="gated_clamped
     lib = _lib("moe")
     n_pairs = n_tokens * top
     # 64 and 128: tensor-core tiles (128 with many rows an expert); 32: the plain ones
-    bm = lib.sb_moe_tile_rows_for(_code(h.dtype), width, inner, ctypes.c_longlong(n_pairs), experts)
+    bm = lib.sb_moe_tile_rows_for(_code(h.dtype), width, inner, n_pairs, experts)
     if tile_rows is not None:
         if tile_rows not in (4, 8, 32, 64, 128, 256) or (tile_rows != 32 and lib.sb_moe_tile_rows(_code(h.dtype), width, inner) != 64):
             raise KernelError(f"no expert tiles of {tile_rows} rows for {h.dtype}, width {width}, inner size {inner}")
         bm = 8 if tile_rows == 4 else int(tile_rows)
     max_tiles = -(-n_pairs // bm) + min(experts, n_pairs)
     capacity = max_tiles * bm
-    meta = h.new_empty((capacity + max_tiles + 1,), dtype=torch.int32)
+    meta = _empty(h, (capacity + max_tiles + 1,), torch.int32)
     sorted_pairs, tile_expert, n_tiles = meta[:capacity], meta[capacity:capacity + max_tiles], meta[capacity + max_tiles:]
-    rc = lib.sb_moe_align(_ptr(ids), n_pairs, experts, _ptr(sorted_pairs), capacity, _ptr(tile_expert), _ptr(n_tiles),
+    rc = lib.sb_moe_align(ids, n_pairs, experts, sorted_pairs, capacity, tile_expert, n_tiles,
                           bm, _stream())
     _check(rc, "moe_align")
-    act = h.new_empty((capacity, inner))
-    per_pair = h.new_empty((n_pairs, width))
+    act = _empty(h, (capacity, inner))
+    per_pair = _empty(h, (n_pairs, width))
     if bm == 256:
         grouped = _lib("gemm_prompt_tcgen05").sb_gemm_prompt_grouped
-        gathered = h.new_empty((capacity, width))
-        rc = lib.sb_moe_gather(_ptr(h), _ptr(sorted_pairs), _ptr(n_tiles), bm, top, _ptr(gathered), capacity, width,
-                               _ptr(in_scale), _stream())
+        gathered = _empty(h, (capacity, width))
+        rc = lib.sb_moe_gather(h, sorted_pairs, n_tiles, bm, top, gathered, capacity, width,
+                               in_scale, _stream())
         _check(rc, "moe_gather")
-        rc = grouped(_ptr(gathered), _ptr(gate_up), _ptr(act), capacity, inner, width, experts, _ptr(tile_expert),
-                     _ptr(n_tiles), max_tiles, None,
+        rc = grouped(gathered, gate_up, act, capacity, inner, width, experts, tile_expert,
+                     n_tiles, max_tiles, None,
                      (GATE_CLAMPED if limit > 0.0 else ACTIVATIONS["silu"]) if up_mode == 1 else 0, 1 if up_mode == 2 else 0,
-                     ctypes.c_float(limit), _ptr(status), _stream())
+                     limit, status, _stream())
         _check(rc, "moe_up (grouped tcgen05)")
-        rc = grouped(_ptr(act), _ptr(down), _ptr(per_pair), capacity, width, inner, experts, _ptr(tile_expert),
-                     _ptr(n_tiles), max_tiles, _ptr(sorted_pairs), 0, 0, ctypes.c_float(0.0), _ptr(status), _stream())
+        rc = grouped(act, down, per_pair, capacity, width, inner, experts, tile_expert,
+                     n_tiles, max_tiles, sorted_pairs, 0, 0, 0.0, status, _stream())
         _check(rc, "moe_down (grouped tcgen05)")
-        out = torch.empty_like(h)
-        rc = lib.sb_moe_combine(_code(h.dtype), _ptr(per_pair), _ptr(out_scale), _ptr(out), n_tokens, width, top, *extras,
+        out = _empty(h, h.shape)
+        rc = lib.sb_moe_combine(_code(h.dtype), per_pair, out_scale, out, n_tokens, width, top, *extras,
                                 _stream())
         _check(rc, "moe_combine")
         return out
-    rc = lib.sb_moe_tiles(_code(h.dtype), up_mode, bm, _ptr(h), _ptr(gate_up), _ptr(act), _ptr(sorted_pairs), _ptr(tile_expert),
-                          _ptr(n_tiles), max_tiles, width, inner, top, ctypes.c_float(limit), _ptr(in_scale), _stream())
+    rc = lib.sb_moe_tiles(_code(h.dtype), up_mode, bm, h, gate_up, act, sorted_pairs, tile_expert,
+                          n_tiles, max_tiles, width, inner, top, limit, in_scale, _stream())
     _check(rc, "moe_up")
-    rc = lib.sb_moe_tiles(_code(h.dtype), 0, bm, _ptr(act), _ptr(down), _ptr(per_pair), _ptr(sorted_pairs),
-                          _ptr(tile_expert), _ptr(n_tiles), max_tiles, inner, width, top, ctypes.c_float(limit), None,
+    rc = lib.sb_moe_tiles(_code(h.dtype), 0, bm, act, down, per_pair, sorted_pairs,
+                          tile_expert, n_tiles, max_tiles, inner, width, top, limit, None,
                           _stream())
     _check(rc, "moe_down")
-    out = torch.empty_like(h)
-    rc = lib.sb_moe_combine(_code(h.dtype), _ptr(per_pair), _ptr(out_scale), _ptr(out), n_tokens, width, top, *extras,
+    out = _empty(h, h.shape)
+    rc = lib.sb_moe_combine(_code(h.dtype), per_pair, out_scale, out, n_tokens, width, top, *extras,
                                 _stream())
     _check(rc, "moe_combine")
     return out
@@ -1941,11 +1977,11 @@ def depth_step(base, dtype, pending=None, mult=1.0, history=None, mix=None, dst=
             raise KernelError(f"no norm {name!r} here (known: {', '.join(DEPTH_NORMS)})")
         kind = DEPTH_NORMS[name]
         _f32(gain, "gain", (hidden,))
-        out = base.new_empty((n_rows, hidden), dtype=dtype)
+        out = _empty(base, (n_rows, hidden), dtype)
     rc = _lib("depth").sb_depth_step(
-        _code(dtype), _ptr(base), _ptr(pending), ctypes.c_float(mult), _ptr(history if mix is not None else None),
-        ctypes.c_longlong(n_tokens * hidden), _ptr(mix), levels, _ptr(dst), _ptr(gain), _ptr(out), _ptr(rows), n_rows,
-        hidden, ctypes.c_float(eps), kind, _stream())
+        _code(dtype), base, pending, mult, history if mix is not None else None,
+        n_tokens * hidden, mix, levels, dst, gain, out, rows, n_rows,
+        hidden, eps, kind, _stream())
     _check(rc, "depth_step")
     return out
 
@@ -1953,7 +1989,7 @@ def depth_step(base, dtype, pending=None, mult=1.0, history=None, mix=None, dst=
 def softcap(logits, cap):
     """``logits <- cap * tanh(logits / cap)`` in place (float32)."""
     _need(logits, "logits", torch.float32)
-    rc = _lib("depth").sb_softcap(_ptr(logits), ctypes.c_longlong(logits.numel()), ctypes.c_float(cap), _stream())
+    rc = _lib("depth").sb_softcap(logits, logits.numel(), cap, _stream())
     _check(rc, "softcap")
     return logits
 
@@ -1965,9 +2001,9 @@ def gated_clamped(gate_up, limit):
     if gate_up.shape[1] % 2:
         raise KernelError(f"gate_up has an odd width {gate_up.shape[1]}")
     inner = gate_up.shape[1] // 2
-    out = gate_up.new_empty((gate_up.shape[0], inner))
-    rc = _lib("elementwise").sb_gated_clamped(_code(gate_up.dtype), _ptr(gate_up), _ptr(out), gate_up.shape[0], inner,
-                                              ctypes.c_float(limit), _stream())
+    out = _empty(gate_up, (gate_up.shape[0], inner))
+    rc = _lib("elementwise").sb_gated_clamped(_code(gate_up.dtype), gate_up, out, gate_up.shape[0], inner,
+                                              limit, _stream())
     _check(rc, "gated_clamped")
     return out
 
@@ -1998,11 +2034,11 @@ def sink_prepare(proj, heads, kv_heads, dim, vdim, tok_pos, tok_slot, block_tabl
         if tuple(k_store.shape[1:]) != (kv_heads, PAGE_TOKENS, dim) or tuple(v_store.shape[1:]) != (kv_heads, PAGE_TOKENS, vdim):
             raise KernelError(f"cache pages have shapes {tuple(k_store.shape)} / {tuple(v_store.shape)}, expected "
                               f"[pages, {kv_heads}, {PAGE_TOKENS}, {dim}] / [.., {vdim}]")
-    gate = proj.new_empty((n_tokens, heads), dtype=torch.float32) if gated else None
+    gate = _empty(proj, (n_tokens, heads), torch.float32) if gated else None
     rc = _lib("attention_sink").sb_sink_prepare(
-        _code(proj.dtype), _ptr(proj), proj.shape[1], _ptr(tok_pos), _ptr(tok_slot), _ptr(block_table),
-        block_table.shape[1], _ptr(k_store if write_cache else None), _ptr(v_store if write_cache else None),
-        _ptr(gate), n_tokens, heads, kv_heads, dim, vdim, int(write_cache), _stream())
+        _code(proj.dtype), proj, proj.shape[1], tok_pos, tok_slot, block_table,
+        block_table.shape[1], k_store if write_cache else None, v_store if write_cache else None,
+        gate, n_tokens, heads, kv_heads, dim, vdim, int(write_cache), _stream())
     _check(rc, "sink_prepare")
     return gate
 
@@ -2045,9 +2081,9 @@ def sink_prepare_rot(proj, heads, kv_heads, dim, vdim, tok_pos, tok_slot, block_
             raise KernelError(f"cache pages have shapes {tuple(k_store.shape)} / {tuple(v_store.shape)}, expected "
                               f"[pages, {kv_heads}, {PAGE_TOKENS}, {dim}] / [.., {vdim}]")
     rc = _lib("attention_sink").sb_sink_prepare_rot(
-        _code(proj.dtype), _ptr(proj), proj.shape[1], _ptr(tok_pos), _ptr(tok_slot), _ptr(block_table),
-        block_table.shape[1], _ptr(k_store if write_cache else None), _ptr(v_store if write_cache else None),
-        _ptr(cos_table if rot_dims else None), _ptr(sin_table if rot_dims else None), int(rot_dims), n_tokens, heads,
+        _code(proj.dtype), proj, proj.shape[1], tok_pos, tok_slot, block_table,
+        block_table.shape[1], k_store if write_cache else None, v_store if write_cache else None,
+        cos_table if rot_dims else None, sin_table if rot_dims else None, int(rot_dims), n_tokens, heads,
         kv_heads, dim, vdim, int(values_from_keys), int(write_cache), _stream())
     if rc == -2:
         raise KernelError(f"sink_prepare_rot: rot_dims={rot_dims} must be even and at most dim={dim}; values taken from "
@@ -2096,9 +2132,9 @@ def sink_prepare_norm(proj, heads, kv_heads, dim, vdim, tok_pos, tok_slot, block
             raise KernelError(f"cache pages have shapes {tuple(k_store.shape)} / {tuple(v_store.shape)}, expected "
                               f"[pages, {kv_heads}, {PAGE_TOKENS}, {dim}] / [.., {vdim}]")
     rc = _lib("attention_sink").sb_sink_prepare_norm(
-        _code(proj.dtype), _ptr(proj), proj.shape[1], _ptr(tok_pos), _ptr(tok_slot), _ptr(block_table),
-        block_table.shape[1], _ptr(k_store if write_cache else None), _ptr(v_store if write_cache else None),
-        _ptr(cos_table), _ptr(sin_table), rot, _ptr(q_gain), _ptr(k_gain), ctypes.c_float(eps), int(unit_values), n_tokens,
+        _code(proj.dtype), proj, proj.shape[1], tok_pos, tok_slot, block_table,
+        block_table.shape[1], k_store if write_cache else None, v_store if write_cache else None,
+        cos_table, sin_table, rot, q_gain, k_gain, eps, int(unit_values), n_tokens,
         heads, kv_heads, dim, vdim, int(write_cache), pairs, _stream())
     _check(rc, "sink_prepare_norm")
 
@@ -2136,12 +2172,12 @@ def sink_attention(q, k_store, v_store, block_table, tok_slot, tok_pos, heads, k
     _need(block_table, "block_table", torch.int32, 2)
     _need(tok_slot, "tok_slot", torch.int32, 1)
     _need(tok_pos, "tok_pos", torch.int32, 1)
-    out = q.new_empty((q.shape[0], heads * vdim))
+    out = _empty(q, (q.shape[0], heads * vdim))
     rc = _lib("attention_sink").sb_sink_attention(
-        _code(q.dtype), _ptr(q), q.shape[1], _ptr(out), _ptr(k_store), _ptr(v_store), _ptr(block_table),
-        block_table.shape[1], _ptr(tok_slot), _ptr(tok_pos), _ptr(r1), _ptr(r2), _ptr(sink), _ptr(gate), q.shape[0],
-        heads, kv_heads, dim, vdim, ctypes.c_float(scale), int(chunk or 0), int(window or 0), int(keep_first),
-        ctypes.c_float(softcap or 0.0), _stream())
+        _code(q.dtype), q, q.shape[1], out, k_store, v_store, block_table,
+        block_table.shape[1], tok_slot, tok_pos, r1, r2, sink, gate, q.shape[0],
+        heads, kv_heads, dim, vdim, scale, int(chunk or 0), int(window or 0), int(keep_first),
+        softcap or 0.0, _stream())
     _check(rc, "sink_attention")
     return out
 
@@ -2186,17 +2222,17 @@ def sink_attention_tc(q, k_store, v_store, block_table, seq_slot, seq_q_start, s
                     ("seq_kv_len", seq_kv_len), ("tile_seq", tile_seq), ("tile_first", tile_first)):
         _need(t, name, torch.int32, 1)
     n_tokens = q.shape[0]
-    out = q.new_empty((n_tokens, heads * vdim))
+    out = _empty(q, (n_tokens, heads * vdim))
     part_acc = part_ml = None
     n_splits = max(1, int(n_splits))
     if n_splits > 1:
-        part_acc = q.new_empty((n_splits, n_tokens * heads, vdim), dtype=torch.float32)
-        part_ml = q.new_empty((n_splits, n_tokens * heads, 2), dtype=torch.float32)
+        part_acc = _empty(q, (n_splits, n_tokens * heads, vdim), torch.float32)
+        part_ml = _empty(q, (n_splits, n_tokens * heads, 2), torch.float32)
     rc = _lib("attention_sink_tc").sb_sink_attention_tc(
-        _ptr(q), q.shape[1], _ptr(out), _ptr(part_acc), _ptr(part_ml), _ptr(k_store), _ptr(v_store), _ptr(block_table),
-        block_table.shape[1], _ptr(seq_slot), _ptr(seq_q_start), _ptr(seq_q_len), _ptr(seq_kv_len), _ptr(tile_seq),
-        _ptr(tile_first), tile_seq.shape[0], _ptr(r1), _ptr(r2), _ptr(sink), _ptr(gate), n_tokens, heads, kv_heads,
-        dim, vdim, ctypes.c_float(scale), int(chunk or 0), int(window or 0), int(keep_first), ctypes.c_float(softcap or 0.0),
+        q, q.shape[1], out, part_acc, part_ml, k_store, v_store, block_table,
+        block_table.shape[1], seq_slot, seq_q_start, seq_q_len, seq_kv_len, tile_seq,
+        tile_first, tile_seq.shape[0], r1, r2, sink, gate, n_tokens, heads, kv_heads,
+        dim, vdim, scale, int(chunk or 0), int(window or 0), int(keep_first), softcap or 0.0,
         n_splits, int(max_q_len), _stream())
     _check(rc, "sink_attention_tc", 2 if n_splits > 1 else 1)
     return out
@@ -2234,13 +2270,13 @@ def sink_attention_tcgen05(q, k_store, v_store, block_table, seq_slot, seq_q_sta
         for name, t in (("block_seq", blocks[0]), ("block_first", blocks[1])):
             _need(t, name, torch.int32, 1)
     list_seq, list_first = blocks if own_list else (tile_seq, tile_first)
-    out = q.new_empty((q.shape[0], heads * vdim))
+    out = _empty(q, (q.shape[0], heads * vdim))
     rc = _lib("attention_prefill_tc").sb_sink_attention_tcgen05(
-        _ptr(q), q.shape[1], _ptr(out), _ptr(k_store), _ptr(v_store), _ptr(block_table), block_table.shape[1],
-        _ptr(seq_slot), _ptr(seq_q_start), _ptr(seq_q_len), _ptr(seq_kv_len), _ptr(list_seq), _ptr(list_first),
-        list_seq.shape[0], q.shape[0], k_store.shape[0], heads, kv_heads, dim, vdim, ctypes.c_float(scale), _ptr(r1), _ptr(r2),
-        _ptr(sink), _ptr(gate), int(chunk or 0), int(window or 0), int(keep_first), ctypes.c_float(softcap or 0.0),
-        _ptr(status), int(own_list), _stream())
+        q, q.shape[1], out, k_store, v_store, block_table, block_table.shape[1],
+        seq_slot, seq_q_start, seq_q_len, seq_kv_len, list_seq, list_first,
+        list_seq.shape[0], q.shape[0], k_store.shape[0], heads, kv_heads, dim, vdim, scale, r1, r2,
+        sink, gate, int(chunk or 0), int(window or 0), int(keep_first), softcap or 0.0,
+        status, int(own_list), _stream())
     _check(rc, "sink_attention_tcgen05")
     return out
 
@@ -2282,15 +2318,15 @@ def linear_gated_clamped(x, weight, limit, status=None):
     if fused and rows <= TENSOR_CORE_MAX_ROWS:
         bm, splits, stages = gemm_plan(rows, n_out, k_dim, True)
         stages = min(max(stages, -(-bm * 512 // (16384 + bm * 128))), (226 * 1024) // (16384 + bm * 128))
-        out = x.new_empty((rows, n_out), dtype=torch.bfloat16)
-        rc = _lib("gemm_tcgen05").sb_gemm_tcgen05_clamped(_ptr(x), _ptr(weight), _ptr(out), rows, n_out, k_dim, bm, splits,
-                                                          stages, ctypes.c_float(limit), _ptr(status), _stream())
+        out = _empty(x, (rows, n_out), torch.bfloat16)
+        rc = _lib("gemm_tcgen05").sb_gemm_tcgen05_clamped(x, weight, out, rows, n_out, k_dim, bm, splits,
+                                                          stages, limit, status, _stream())
         _check(rc, "gemm_tcgen05 (clamped gate)")
         return out
     if fused and rows >= PROMPT_MIN_ROWS:
-        out = x.new_empty((rows, n_out), dtype=torch.bfloat16)
-        rc = _lib("gemm_prompt_tcgen05").sb_gemm_prompt_clamped(_ptr(x), _ptr(weight), _ptr(out), rows, n_out, k_dim, 0, 0,
-                                                                ctypes.c_float(limit), _ptr(status), _stream())
+        out = _empty(x, (rows, n_out), torch.bfloat16)
+        rc = _lib("gemm_prompt_tcgen05").sb_gemm_prompt_clamped(x, weight, out, rows, n_out, k_dim, 0, 0,
+                                                                limit, status, _stream())
         _check(rc, "gemm_prompt_tcgen05 (clamped gate)")
         return out
     return gated_clamped(linear(x, weight, status=status), limit)
@@ -2341,11 +2377,11 @@ def short_conv(x, col, channels, taps, bias, in_bias, state, state_at, seq_slot,
     if activation not in (None, "silu"):
         raise KernelError(f"the short convolution applies silu or nothing, not {activation!r}")
     n_seqs = _seq_arrays(seq_slot, seq_q_start, seq_q_len)
-    y = x.new_empty((x.shape[0], channels))
+    y = _empty(x, (x.shape[0], channels))
     rc = _lib("short_conv").sb_short_conv(
-        _code(x.dtype), _at(x, col), x.shape[1], _ptr(taps), _ptr(bias), _ptr(in_bias), _ptr(y), channels,
-        _at(state, state_at) if state is not None else _ptr(None), ctypes.c_longlong(slot_floats), _ptr(seq_slot),
-        _ptr(seq_q_start), _ptr(seq_q_len), n_seqs, int(max_q_len), channels, k, 1 if activation == "silu" else 0, _stream())
+        _code(x.dtype), _at(x, col), x.shape[1], taps, bias, in_bias, y, channels,
+        _at(state, state_at) if state is not None else None, slot_floats, seq_slot,
+        seq_q_start, seq_q_len, n_seqs, int(max_q_len), channels, k, 1 if activation == "silu" else 0, _stream())
     if rc == -2:
         raise KernelError(f"the short convolution takes 1 to {conv_max_taps()} taps, not {k}")
     _check(rc, "short_conv")
@@ -2375,11 +2411,11 @@ def glru_scan(u, gates, r_bias, i_bias, lam, decay_scale, proj, y_col, y_bias, s
     if proj.shape[0] != n_tokens or y_col < 0 or y_col + channels > proj.shape[1] or state_at + channels > state.shape[1]:
         raise KernelError("the gated branch or the state does not hold the channels asked for")
     n_seqs = _seq_arrays(seq_slot, seq_q_start, seq_q_len)
-    out = torch.empty_like(u)
+    out = _empty(u, u.shape)
     rc = _lib("short_conv").sb_glru_scan(
-        _code(u.dtype), _ptr(u), channels, _ptr(gates), n_tokens, channels // blocks, _ptr(r_bias), _ptr(i_bias), _ptr(lam),
-        ctypes.c_float(decay_scale), _at(proj, y_col), proj.shape[1], _ptr(y_bias), _ptr(out), _at(state, state_at),
-        ctypes.c_longlong(state.shape[1]), _ptr(seq_slot), _ptr(seq_q_start), _ptr(seq_q_len), n_seqs, int(max_q_len),
+        _code(u.dtype), u, channels, gates, n_tokens, channels // blocks, r_bias, i_bias, lam,
+        decay_scale, _at(proj, y_col), proj.shape[1], y_bias, out, _at(state, state_at),
+        state.shape[1], seq_slot, seq_q_start, seq_q_len, n_seqs, int(max_q_len),
         channels, _stream())
     _check(rc, "glru_scan")
     return out
@@ -2462,26 +2498,26 @@ def state_scan(mode, q, k, v, a_raw, b_raw, A_log, dt_bias, skip, state, state_a
     if state_at < 0 or state_at + heads * n_state * v_dim > state.shape[1]:
         raise KernelError(f"a slot's {state.shape[1]} floats do not hold {heads} states of {n_state} x {v_dim} from {state_at}")
     n_seqs = _seq_arrays(seq_slot, seq_q_start, seq_q_len)
-    out = state.new_empty((n_tokens, heads * v_dim), dtype=torch.float32)
+    out = _empty(state, (n_tokens, heads * v_dim), torch.float32)
     if dtype == torch.bfloat16 and n_tokens >= SCAN_PROMPT_TOKENS * n_seqs and 64 < n_state <= 128:
         lib = _lib("state_scan_prompt")
-        floats = lib.sb_scan_prompt_floats(1, SCAN_MODES[mode], *args[:6], _ptr(decay), heads, groups, n_state, v_dim)
+        floats = lib.sb_scan_prompt_floats(1, SCAN_MODES[mode], *args[:6], decay, heads, groups, n_state, v_dim)
         if 0 <= 4 * floats * n_tokens <= SCAN_PROMPT_BYTES:
-            scratch = state.new_empty((n_tokens, floats), dtype=torch.float32) if floats else None
+            scratch = _empty(state, (n_tokens, floats), torch.float32) if floats else None
             segs, carried = 1, None
             if mode == "state_space":
                 segs = scan_segments(n_tokens, n_seqs, heads * -(-v_dim // 64))
                 if segs > 1:
-                    carried = state.new_empty((n_seqs * segs * lib.sb_scan_segment_floats(heads, v_dim),))
+                    carried = _empty(state, (n_seqs * segs * lib.sb_scan_segment_floats(heads, v_dim),))
             rc = lib.sb_state_scan_prompt(
-                SCAN_MODES[mode], *args, _ptr(A_log), _ptr(dt_bias), _ptr(skip), _ptr(decay), _at(state, state_at),
-                ctypes.c_longlong(state.shape[1]), _ptr(out), _ptr(seq_slot), _ptr(seq_q_start), _ptr(seq_q_len), n_tokens,
-                n_seqs, heads, groups, n_state, v_dim, _ptr(scratch), segs, _ptr(carried), _stream())
+                SCAN_MODES[mode], *args, A_log, dt_bias, skip, decay, _at(state, state_at),
+                state.shape[1], out, seq_slot, seq_q_start, seq_q_len, n_tokens,
+                n_seqs, heads, groups, n_state, v_dim, scratch, segs, carried, _stream())
             _check(rc, "state_scan (many tokens)", 1 if mode == "channel_decay" else 2)
             return out
     rc = _lib("state_scan").sb_state_scan(
-        _code(dtype), SCAN_MODES[mode], *args, _ptr(A_log), _ptr(dt_bias), _ptr(skip), _ptr(decay), _at(state, state_at),
-        ctypes.c_longlong(state.shape[1]), _ptr(out), _ptr(seq_slot), _ptr(seq_q_start), _ptr(seq_q_len), n_seqs, heads,
+        _code(dtype), SCAN_MODES[mode], *args, A_log, dt_bias, skip, decay, _at(state, state_at),
+        state.shape[1], out, seq_slot, seq_q_start, seq_q_len, n_seqs, heads,
         groups, n_state, v_dim, _stream())
     if rc == -2:
         raise KernelError(f"the recurrence takes states of 1 to {scan_max_state()} rows and heads in whole groups, not "
@@ -2502,9 +2538,9 @@ def low_rank_decay(u, col, a2, bias, tau):
         raise KernelError(f"{rank} columns from {col} of {tuple(u.shape)} are not there")
     if not tau > 0.0:
         raise KernelError(f"tau={tau} must be positive")
-    out = u.new_empty((u.shape[0], channels), dtype=torch.float32)
-    rc = _lib("state_scan").sb_low_rank_decay(_code(u.dtype), _at(u, col), u.shape[1], _ptr(a2), _ptr(bias), _ptr(out),
-                                              u.shape[0], channels, rank, ctypes.c_float(1.0 / tau), _stream())
+    out = _empty(u, (u.shape[0], channels), torch.float32)
+    rc = _lib("state_scan").sb_low_rank_decay(_code(u.dtype), _at(u, col), u.shape[1], a2, bias, out,
+                                              u.shape[0], channels, rank, 1.0 / tau, _stream())
     if rc == -2:
         raise KernelError(f"the low-rank decay takes ranks of 1 to 1024, not {rank}")
     _check(rc, "low_rank_decay")
@@ -2527,11 +2563,11 @@ def group_norm_gate(o, z, z_col, weight, parts, eps, gate_first, dtype):
             raise KernelError(f"rows of {width} in {parts} parts with a gate from column {z_col} of {tuple(z.shape)} do not fit")
     if weight.shape[0] not in (width, width // parts):
         raise KernelError(f"a gain of {weight.shape[0]} entries fits neither the row ({width}) nor a part ({width // parts})")
-    y = o.new_empty((n_tokens, width), dtype=dtype)
-    gate, gate_width, order = (_ptr(None), 0, 2) if z is None else (_at(z, z_col), z.shape[1], 0 if gate_first else 1)
-    rc = _lib("state_scan").sb_group_norm_gate(_code(dtype), _ptr(o), gate, gate_width, _ptr(weight),
-                                               weight.shape[0], _ptr(y), n_tokens, parts, width // parts,
-                                               ctypes.c_float(eps), order, _stream())
+    y = _empty(o, (n_tokens, width), dtype)
+    gate, gate_width, order = (None, 0, 2) if z is None else (_at(z, z_col), z.shape[1], 0 if gate_first else 1)
+    rc = _lib("state_scan").sb_group_norm_gate(_code(dtype), o, gate, gate_width, weight,
+                                               weight.shape[0], y, n_tokens, parts, width // parts,
+                                               eps, order, _stream())
     _check(rc, "group_norm_gate")
     return y
 
@@ -2544,9 +2580,9 @@ def norm_pair_mean(a, b, gain_a, gain_b, eps):
         raise KernelError(f"rows {tuple(a.shape)} and {tuple(b.shape)} differ")
     _f32(gain_a, "gain_a", (a.shape[1],))
     _f32(gain_b, "gain_b", (a.shape[1],))
-    out = torch.empty_like(a)
-    rc = _lib("state_scan").sb_norm_pair_mean(_code(a.dtype), _ptr(a), _ptr(b), _ptr(gain_a), _ptr(gain_b), _ptr(out),
-                                              a.shape[0], a.shape[1], ctypes.c_float(eps), _stream())
+    out = _empty(a, a.shape)
+    rc = _lib("state_scan").sb_norm_pair_mean(_code(a.dtype), a, b, gain_a, gain_b, out,
+                                              a.shape[0], a.shape[1], eps, _stream())
     _check(rc, "norm_pair_mean")
     return out
 
@@ -2557,8 +2593,8 @@ def scaled_sum(a, b, weight_a, weight_b):
     _need(b, "b", a.dtype, 2)
     if tuple(a.shape) != tuple(b.shape):
         raise KernelError(f"rows {tuple(a.shape)} and {tuple(b.shape)} differ")
-    out = torch.empty_like(a)
-    rc = _lib("state_scan").sb_scaled_sum(_code(a.dtype), _ptr(a), _ptr(b), _ptr(out), ctypes.c_float(weight_a),
-                                          ctypes.c_float(weight_b), ctypes.c_longlong(a.numel()), _stream())
+    out = _empty(a, a.shape)
+    rc = _lib("state_scan").sb_scaled_sum(_code(a.dtype), a, b, out, weight_a,
+                                          weight_b, a.numel(), _stream())
     _check(rc, "scaled_sum")
     return out

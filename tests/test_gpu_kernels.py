@@ -731,3 +731,26 @@ def test_a_wait_in_the_float32_product_that_runs_out_is_reported(rows, n, k, sli
     got = ops.linear(dev(x), dev(w), status=status).cpu().double()
     bound = (k + 8) * 2.0 ** -24 * (x.double().abs() @ w.double().abs().t())
     assert bool(((got - x.double() @ w.double().t()).abs() <= bound).all()) and status.item() == 0
+
+
+def test_native_outputs_and_checks():
+    """What the native host part makes and lets pass on the device (csrc/host.cpp)."""
+    from starter_b200 import ops
+
+    x = torch.zeros(3, 4, dtype=torch.bfloat16, device="cuda")
+    for shape, dtype in (((5, 7), None), ((0, 3), torch.float32), ((2, 3, 4, 1), torch.int32), (x.shape, None), ((), torch.int64)):
+        made = ops._empty(x, shape, dtype)
+        want = x.new_empty(tuple(shape), dtype=dtype)
+        assert made.shape == want.shape and made.dtype == want.dtype and made.device == want.device and made.stride() == want.stride()
+    with torch.inference_mode():
+        assert ops._empty(x, (2,)).is_inference()
+    with pytest.raises(RuntimeError):
+        ops._empty(x, (-1, 2))
+    ops._need(x, "x", torch.bfloat16, 2)
+    for bad, why in ((x.t(), "contiguous"), (x.float(), "must be torch.bfloat16"), (x[0], "2 dimensions"), (x.cpu(), "CUDA tensor")):
+        with pytest.raises(ops.KernelError, match=why):
+            ops._need(bad, "x", torch.bfloat16, 2)
+    side = torch.cuda.Stream()
+    with torch.cuda.stream(side):
+        assert ops._stream() == side.cuda_stream
+    assert ops._stream() == torch.cuda.current_stream().cuda_stream

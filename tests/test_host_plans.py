@@ -150,3 +150,43 @@ def test_keys_are_formed_where_that_is_the_shorter_way(heads, news, takes):
     for past in (0, 1000):
         ctx = SimpleNamespace(host={"seq_q_len": new, "seq_kv_len": new + past}, block_seq=torch.zeros(1))
         assert ops.latent_prompt_takes(torch.bfloat16, ctx, 128, 64, 128, 512, 0.1, None, heads) is takes
+
+
+def test_native_entry_points_take_their_declared_arguments():
+    """Entries called natively (csrc/host.cpp) hand over what ctypes does: more arguments than registers, 64-bit results, numbers that
+    ctypes wraps; anything else is refused before the call."""
+    import ctypes
+
+    import torch
+
+    from starter_b200 import ops
+    from starter_b200.csrc import build
+
+    native, plain = ops._lib("state_scan_prompt"), build.load("state_scan_prompt")
+    assert native.sb_scan_segment_floats(40000, 64) == plain.sb_scan_segment_floats(40000, 64) > 2 ** 28
+    for args in ((1, 0, 160, 128, None, 128, 320, 64, 0, 4, 2, 128, 64), (1, 1, 160, 128, 0, 128, 320, 64, None, 4, 2, 120, 64),
+                 (1, 2, 160, 128, 0, 128, 328, 64, None, 4, 4, 128, 64), (0, 2, 160, 128, 0, 128, 328, 64, None, 4, 4, 128, 64)):
+        assert native.sb_scan_prompt_floats(*args) == plain.sb_scan_prompt_floats(*args)
+    assert native.sb_scan_segment_floats(ctypes.c_int(3), 64) == plain.sb_scan_segment_floats(3, 64)
+    x = torch.zeros(4)
+    assert native.sb_scan_prompt_floats(1, 0, x, 128, x, 128, x, 64, None, 4, 2, 128, 64) == 4 * 20
+    with pytest.raises(TypeError):
+        native.sb_scan_segment_floats(3)
+    for bad in (x, 1.5, "3", None):
+        with pytest.raises(TypeError):
+            native.sb_scan_segment_floats(3, bad)
+
+
+def test_native_checks_refuse_what_the_plain_ones_do():
+    import torch
+
+    from starter_b200 import ops
+
+    ops._bind()
+    for bad in (torch.zeros(2, 2), None, 3, [1.0]):
+        with pytest.raises(ops.KernelError, match="x must be a CUDA tensor"):
+            ops._need(bad, "x", torch.float32, 2)
+    assert ops._empty(torch.zeros(2), (3, 5), torch.int32).shape == (3, 5)
+    assert ops._empty(torch.zeros(2, dtype=torch.bfloat16), (0, 5)).dtype == torch.bfloat16
+    with pytest.raises((RuntimeError, TypeError)):
+        ops._empty(torch.zeros(2), (-3, 5))
