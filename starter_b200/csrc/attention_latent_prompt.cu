@@ -20,6 +20,9 @@
 // that size, 0.00463 against 0.00464 for four sequences of up to 450 tokens, 0.00482 against 0.00489 for 300 tokens behind 900 (means of
 // three seeds; 0.00477, 0.00471 and 0.00482 while the weights were summed before their rounding and relative to the sink).
 //
+// Few blocks over many keys: a cluster's CTAs walk a part of a block's keys each and merge (attention_tc.cuh): 700 tokens behind 1,200
+// 60.1 -> 48.6 us.
+//
 // Gathered rows: a sequence's keys from the first that any of its queries sees, padded to a multiple of 64 with zeros, so
 // that a step never reads another sequence's values (their weights are zero, but 0 * inf would not be).
 #include <cuda.h>
@@ -78,7 +81,7 @@ latent_prompt_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_con
                      const __grid_constant__ CUtensorMap map_rot, bf16* __restrict__ out, const int* __restrict__ seq_q_start,
                      const int* __restrict__ seq_q_len, const int* __restrict__ seq_kv_len, const int* __restrict__ block_seq,
                      const int* __restrict__ block_first, int heads, float scale_log2, int window,
-                     const float* __restrict__ sink, int* status, int withhold) {
+                     const float* __restrict__ sink, int* status, int withhold, int splits) {
   constexpr int QC = DC + 1;
   constexpr int QSUB = 128 * 128, KSUB = 64 * 128;  // bytes of 128 (64) rows of 128 bytes
   constexpr int Q_BYTES = QC * QSUB, K_BYTES = QC * KSUB, V_BYTES = VC * KSUB, P_BYTES = QSUB;
@@ -92,8 +95,10 @@ latent_prompt_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_con
   __shared__ uint64_t q_full, k_full[2], k_empty[2], v_full[2], v_empty[2], s_ready[2][2], s_free[2][2], p_ready[2], o_ready[2];
   __shared__ uint32_t tmem_holder;
   __shared__ int abort_flag;
+  __shared__ __align__(8) float2 ml[2 * TC_BQ];     // keys in parts: the rows' references and sums
 
-  const int head = blockIdx.x, seq = block_seq[blockIdx.y], q_first = block_first[blockIdx.y];
+  const int head = blockIdx.x / splits, part = blockIdx.x - head * splits;      // (the CTAs of a cluster share a head's block)
+  const int seq = block_seq[blockIdx.y], q_first = block_first[blockIdx.y];
   const int q_len = seq_q_len[seq], kv_len = seq_kv_len[seq];
   const int rows_valid = min(2 * TC_BQ, q_len - q_first);
   const int pos0 = kv_len - q_len + q_first;
@@ -101,11 +106,18 @@ latent_prompt_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_con
   // steps of 64 keys, counted from the sequence's first gathered key; this block's first step
   const int base = lp_first_key(kv_len, q_len, window);
   const int lo = window > 0 ? max(0, pos0 - window + 1) : 0;
-  const int step0 = (lo - base) / LP_BK;
+  int step0 = (lo - base) / LP_BK;
   int n_tile[2];
   n_tile[0] = (pos0 + min(rows_valid, TC_BQ) - 1 - base) / LP_BK - step0 + 1;
   n_tile[1] = rows_valid > TC_BQ ? (pos0 + rows_valid - 1 - base) / LP_BK - step0 + 1 : 0;
-  const int n_steps = max(n_tile[0], n_tile[1]);
+  int n_steps = max(n_tile[0], n_tile[1]);
+  if (splits > 1) {                                 // this CTA's steps
+    const int per = (n_steps + splits - 1) / splits;
+    for (int t = 0; t < 2; ++t) n_tile[t] = max(0, min(per, n_tile[t] - part * per));
+    n_steps = max(n_tile[0], n_tile[1]);
+    step0 += part * per;
+    withhold -= part * per;
+  }
 
   if (threadIdx.x == 0) {
     mbar_init(&q_full, 1);
@@ -140,8 +152,8 @@ latent_prompt_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_con
     pdl_wait();
     const int q_row0 = seq_q_start[seq] + q_first;
     const int row0 = lp_row0(seq_kv_len, seq_q_len, seq, window, lane) + step0 * LP_BK;
-    const int q_tiles = n_tile[1] ? 2 : 1;
-    if (elected) mbar_expect_tx(&q_full, q_tiles * Q_BYTES);
+    const int q_tiles = n_tile[1] ? 2 : n_steps > 0 ? 1 : 0;
+    if (elected && q_tiles) mbar_expect_tx(&q_full, q_tiles * Q_BYTES);
     for (int t = 0; t < q_tiles; ++t)
       for (int c = 0; c < QC; ++c)
         if (elected) tma_load_2d(q_sm + t * Q_BYTES + c * QSUB, &map_q, &q_full, head * (QC * 64) + c * 64, q_row0 + t * TC_BQ);
@@ -171,7 +183,7 @@ latent_prompt_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_con
         while (loads[b] > 0 && !mbar_try(bar, (loads[b] - 1) & 1) && now_ns() - start < WAIT_LIMIT_NS) {}
       }
       const uint64_t start = now_ns();
-      while (!mbar_try(&q_full, 0) && now_ns() - start < WAIT_LIMIT_NS) {}
+      while (q_tiles && !mbar_try(&q_full, 0) && now_ns() - start < WAIT_LIMIT_NS) {}
     }
   } else if (warp == 9 || warp == 10) {
     // ---------------- MMA issuers: warp 9 for tile 0, warp 10 for tile 1
@@ -318,7 +330,24 @@ latent_prompt_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_con
       if (lane == 0) mbar_arrive(&p_ready[t]);
     }
     if (ok && n_mine > 0) ok = mbar_wait(&o_ready[t], (n_mine - 1) & 1, abort);
-    if (ok && n_mine > 0) {
+    if (splits > 1) {
+      if constexpr (DC == 2 || VC == 1) {
+        ml[t * TC_BQ + r] = n_mine > 0 ? make_float2(m_ref, l_run) : make_float2(-INFINITY, 0.f);
+        if (ok && n_mine > 0) {
+          asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+#pragma unroll 1
+          for (int c = 0; c < VC * 64; c += 32) {
+            float ov[32];
+            tmem_load32(tmem_o + c, ov);
+#pragma unroll
+            for (int d = 0; d < 32; d += 4)
+              *reinterpret_cast<float4*>(part_piece<32, VC * 64>(p_sm + t * P_BYTES, q_sm + t * Q_BYTES, r, (c + d) / 4)) =
+                  make_float4(ov[d], ov[d + 1], ov[d + 2], ov[d + 3]);
+          }
+          asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+        }
+      }
+    } else if (ok && n_mine > 0) {
       asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
       const bool valid = t * TC_BQ + r < rows_valid;
       // the sink joins at the end, so that the weights are relative to a key's score: the largest of the first step is one exactly
@@ -350,6 +379,24 @@ latent_prompt_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_con
   }
 
   asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+  if constexpr (DC == 2 || VC == 1) {
+    if (splits > 1) {
+      __syncwarp();
+      cluster_barrier();
+      if (threadIdx.x < 2 * TC_BQ) {
+        const size_t stride = (size_t)heads * (VC * 64);
+        merge_parts<32, VC * 64, Q_BYTES, P_BYTES>(
+            q_sm, p_sm, ml, part, splits, rows_valid, VC * 64,
+            out + ((size_t)seq_q_start[seq] + q_first) * stride + (size_t)head * (VC * 64), stride, [&](int, float ref, float sum) {
+              if (!sink) return 1.f / sum;
+              const float own = sink[head] * 1.4426950408889634f, top = fmaxf(ref, own), f = fast_exp2(ref - top);
+              return f / (sum * f + fast_exp2(own - top));
+            });
+      }
+      __syncwarp();
+      cluster_barrier();                            // nobody leaves while others read from it
+    }
+  }
   __syncthreads();
   if (warp == 9) {
     __syncwarp();
@@ -361,19 +408,21 @@ latent_prompt_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_con
 template <int DC, int VC>
 static int lp_launch(const CUtensorMap& mq, const CUtensorMap& mkv, const CUtensorMap& mr, void* out, const int* seq_q_start,
                      const int* seq_q_len, const int* seq_kv_len, const int* block_seq, const int* block_first, int n_blocks,
-                     int heads, float scale, int window, const float* sink, int* status, int withhold, cudaStream_t s) {
+                     int heads, float scale, int window, const float* sink, int* status, int withhold, int splits,
+                     cudaStream_t s) {
   const int smem = 2 * (DC + 1) * 128 * 128 + 2 * 128 * 128 + 2 * (DC + 1 + VC) * 64 * 128 + 1024;
   cudaError_t err = cudaFuncSetAttribute(latent_prompt_kernel<DC, VC>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
   if (err != cudaSuccess) return (int)err;
-  return launch_dependent(latent_prompt_kernel<DC, VC>, dim3(heads, n_blocks), dim3(LP_THREADS), smem, s, mq, mkv, mr, (bf16*)out,
-                          seq_q_start, seq_q_len, seq_kv_len, block_seq, block_first, heads, scale * 1.4426950408889634f, window,
-                          sink, status, withhold);
+  if (splits < 1 || splits > 8 || (splits & (splits - 1)) || (DC == 1 && VC == 2)) splits = 1;
+  return launch_dependent_cluster(latent_prompt_kernel<DC, VC>, dim3(heads * splits, n_blocks), dim3(LP_THREADS), smem, s, dim3(splits),
+                                  mq, mkv, mr, (bf16*)out, seq_q_start, seq_q_len, seq_kv_len, block_seq, block_first, heads,
+                                  scale * 1.4426950408889634f, window, sink, status, withhold, splits);
 }
 
 static int lp_run(const void* q, const void* kv, const void* shared, void* out, const int* seq_q_start, const int* seq_q_len,
                   const int* seq_kv_len, const int* block_seq, const int* block_first, int n_blocks, int n_tokens, int rows,
                   int heads, int dim, int vdim, float scale, int window, const float* sink, int* status, int withhold,
-                  cudaStream_t s) {
+                  int splits, cudaStream_t s) {
   if (n_blocks == 0 || n_tokens == 0) return 0;
   if ((dim != 64 && dim != 128) || (vdim != 64 && vdim != 128) || !(scale > 0.f) || n_blocks > 65535) return -2;
   if (((uintptr_t)q | (uintptr_t)kv | (uintptr_t)shared | (uintptr_t)out) & 15) return -2;
@@ -384,7 +433,7 @@ static int lp_run(const void* q, const void* kv, const void* shared, void* out, 
   if (rc) return rc;
   rc = sb_make_map(&mr, shared, rows, 64, LP_BK);
   if (rc) return rc;
-#define ARGS mq, mkv, mr, out, seq_q_start, seq_q_len, seq_kv_len, block_seq, block_first, n_blocks, heads, scale, window, sink, status, withhold, s
+#define ARGS mq, mkv, mr, out, seq_q_start, seq_q_len, seq_kv_len, block_seq, block_first, n_blocks, heads, scale, window, sink, status, withhold, splits, s
   if (dim == 128) return vdim == 128 ? lp_launch<2, 2>(ARGS) : lp_launch<2, 1>(ARGS);
   return vdim == 128 ? lp_launch<1, 2>(ARGS) : lp_launch<1, 1>(ARGS);
 #undef ARGS
@@ -407,22 +456,23 @@ int sb_latent_gather(const void* store, const int* block_table, int table_stride
 // [rows, 64]; out: [n_tokens, heads * vdim]; block_seq / block_first: blocks of 256 queries; dim and vdim 64 or 128; scale > 0.
 int sb_latent_prompt(const void* q, const void* kv, const void* shared, void* out, const int* seq_q_start, const int* seq_q_len,
                      const int* seq_kv_len, const int* block_seq, const int* block_first, int n_blocks, int n_tokens, int rows,
-                     int heads, int dim, int vdim, float scale, int window, const float* sink, int* status, cudaStream_t s) {
+                     int heads, int dim, int vdim, float scale, int window, const float* sink, int* status, int splits,
+                     cudaStream_t s) {
   return lp_run(q, kv, shared, out, seq_q_start, seq_q_len, seq_kv_len, block_seq, block_first, n_blocks, n_tokens, rows, heads,
-                dim, vdim, scale, window, sink, status, -1, s);
+                dim, vdim, scale, window, sink, status, -1, splits, s);
 }
 
 // The same with the values of step `step` (64 keys) of every block left out: the waits on them give up after wait_limit_ns, the
 // kernel returns, the status bit is set and out is undefined.  For tests.
 int sb_latent_prompt_withheld(const void* q, const void* kv, const void* shared, void* out, const int* seq_q_start, const int* seq_q_len,
                               const int* seq_kv_len, const int* block_seq, const int* block_first, int n_blocks, int n_tokens, int rows,
-                              int heads, int dim, int vdim, float scale, int window, const float* sink, int* status, int step,
+                              int heads, int dim, int vdim, float scale, int window, const float* sink, int* status, int splits, int step,
                               unsigned long long wait_limit_ns, cudaStream_t s) {
   if (step < 0 || wait_limit_ns == 0) return -2;
   const unsigned long long usual = WAIT_LIMIT_NS;
   cudaMemcpyToSymbolAsync(tc_wait_limit_ns, &wait_limit_ns, sizeof(usual), 0, cudaMemcpyHostToDevice, s);
   const int rc = lp_run(q, kv, shared, out, seq_q_start, seq_q_len, seq_kv_len, block_seq, block_first, n_blocks, n_tokens, rows,
-                        heads, dim, vdim, scale, window, sink, status, step, s);
+                        heads, dim, vdim, scale, window, sink, status, step, splits, s);
   cudaMemcpyToSymbolAsync(tc_wait_limit_ns, &usual, sizeof(usual), 0, cudaMemcpyHostToDevice, s);
   return rc;
 }

@@ -36,6 +36,8 @@
 // behind a query's own entries (its neighbour's) out of S, and the output columns they give are not stored.
 // (Loops over the real sizes would make the one lane that issues the products form every descriptor anew.)
 //
+// Few blocks of queries over many keys: `splits` CTAs, a cluster, walk a part of a block's keys each and merge (attention_tc.cuh).
+//
 // Every wait on an mbarrier gives up after WAIT_LIMIT_NS, raises bit 16 of *status and lets the
 // block drain its copies, free its tensor memory and return.
 #include <cuda.h>
@@ -73,7 +75,7 @@ attention_prefill_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __g
                             const int* __restrict__ seq_q_len, const int* __restrict__ seq_kv_len,
                             const int* __restrict__ tile_seq, const int* __restrict__ tile_first,
                             int heads, int kv_heads, float scale_log2, int window, int* status, int list_of_blocks,
-                            TcExtras ex) {
+                            int splits, TcExtras ex) {
   // DC, VC: 64-element (128-byte) chunks of a key and of a value
   constexpr bool CAP = EXT == 2;
   const int dim = EXT ? ex.dim : DC * 64, vdim = EXT ? ex.vdim : VC * 64;
@@ -90,8 +92,10 @@ attention_prefill_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __g
   __shared__ uint64_t q_full, full[TC_RING], empty[TC_RING], s_ready[2], s_free[2], p_ready[2], o_ready[2];
   __shared__ uint32_t tmem_holder;
   __shared__ int abort_flag;
+  float2 row_state = make_float2(-INFINITY, 0.f);   // keys in parts: a row's reference and sum
 
-  const int tile = blockIdx.y, head = blockIdx.x;   // heads run fastest: the work list's order holds
+  // heads run fastest: the work list's order holds; the CTAs of a cluster share a head's block
+  const int tile = blockIdx.y, head = blockIdx.x / splits, part = blockIdx.x - head * splits;
   const int q_first = tile_first[tile];
   // the work list is either this kernel's own (one entry per block of 256 queries) or the common
   // one in tiles of 64 queries, of which every fourth starts a block
@@ -117,7 +121,13 @@ attention_prefill_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __g
   int n_tile[2];
   n_tile[0] = ((pos0 + min(rows_valid, TC_BQ) - 1) / SB_PAGE_TOKENS - page_lo + kept) / 2 + 1;
   n_tile[1] = rows_valid > TC_BQ ? (page_hi - page_lo + kept) / 2 + 1 : 0;
-  const int n_steps = max(n_tile[0], n_tile[1]);
+  int n_steps = max(n_tile[0], n_tile[1]), first_step = 0;
+  if (splits > 1) {                                 // this CTA's steps
+    const int per = (n_steps + splits - 1) / splits;
+    first_step = part * per;
+    for (int t = 0; t < 2; ++t) n_tile[t] = max(0, min(per, n_tile[t] - first_step));
+    n_steps = max(n_tile[0], n_tile[1]);
+  }
 
   if (threadIdx.x == 0) {
     mbar_init(&q_full, 1);
@@ -148,8 +158,8 @@ attention_prefill_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __g
       const bool elected = elect_one();
       pdl_wait();
       const int q_row0 = seq_q_start[seq] + q_first;
-      const int q_tiles = n_tile[1] ? 2 : 1;
-      if (elected) mbar_expect_tx(&q_full, q_tiles * Q_BYTES);
+      const int q_tiles = n_tile[1] ? 2 : n_steps > 0 ? 1 : 0;
+      if (elected && q_tiles) mbar_expect_tx(&q_full, q_tiles * Q_BYTES);
       for (int t = 0; t < q_tiles; ++t)
         for (int c = 0; c < DC; ++c)
           if (elected) tma_load_2d(q_sm + t * Q_BYTES + c * SUB, &map_q, &q_full, head * dim + c * 64, q_row0 + t * TC_BQ);
@@ -160,9 +170,9 @@ attention_prefill_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __g
         if (use > 0 && !__all_sync(0xffffffffu, mbar_wait(&empty[b], (use - 1) & 1, abort))) return false;
         const int chunks = is_v ? VC : DC;
         if (elected) mbar_expect_tx(&full[b], chunks * SUB);
-        const bool withheld = is_v && i == *(volatile int*)&tc_withhold_step;   // tests only
+        const bool withheld = is_v && first_step + i == *(volatile int*)&tc_withhold_step;   // tests only
         for (int half = 0; half < (withheld ? 1 : 2); ++half) {
-          const int page = pages[min(page_of(2 * i + half), page_hi)];
+          const int page = pages[min(page_of(2 * (first_step + i) + half), page_hi)];
           const int row = (page * kv_heads + kvh) * SB_PAGE_TOKENS;
           for (int c = 0; c < chunks; ++c)
             if (elected) tma_load_2d(ring + b * KV_BYTES + c * SUB + half * 8192, is_v ? &map_v : &map_k, &full[b], c * 64, row);
@@ -170,7 +180,7 @@ attention_prefill_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __g
         return true;
       };
       int loads[3] = {0, 0, 0};                        // per buffer: how many copies were started
-      bool ok = load(false, 0);
+      bool ok = n_steps > 0 && load(false, 0);
       if (ok) { loads[0]++; ok = load(true, 0); }
       if (ok) loads[2]++;
       if (ok && n_steps > 1) { ok = load(false, 1); if (ok) loads[1]++; }
@@ -284,7 +294,7 @@ attention_prefill_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __g
         pen1 = ex.r1[head] / scale_log2;
         pen2 = ex.r2[head];
       }
-      if (ex.sink) {
+      if (ex.sink && part == 0) {
         m_ref = ex.sink[head] * 1.4426950408889634f;
         l_run = 1.f;
       }
@@ -300,13 +310,12 @@ attention_prefill_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __g
       if (!ok) break;
       asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
       // the first keys of the step's two pages (neighbours, but for the step between the kept pages and the others)
-      const int jp[2] = {page_of(2 * i) * SB_PAGE_TOKENS, page_of(2 * i + 1) * SB_PAGE_TOKENS};
+      const int jp[2] = {page_of(2 * (first_step + i)) * SB_PAGE_TOKENS,
+                         page_of(2 * (first_step + i) + 1) * SB_PAGE_TOKENS};
       const bool edge = jp[1] + SB_PAGE_TOKENS - 1 > pos0 + t * TC_BQ ||
                         (window > 0 && jp[0] <= pos0 + t * TC_BQ + TC_BQ - window) || (EXT && jp[0] < tile_lo);
       float sv[64];
-      uint32_t pk[32];
-      float mx = -INFINITY, rs = 0.f, rs_hi = 0.f;   // the row sum in two halves (packed adds)
-      float m_use = m_ref == -INFINITY ? 0.f : m_ref;
+      float rs = 0.f, rs_hi = 0.f;                   // the row sum in two halves (packed adds)
       // half h of the row of S from tensor memory, masked where the step touches an edge
       auto load_half = [&](int h) {
         tmem_load64(tmem_s + h * 64, sv);
@@ -332,88 +341,160 @@ attention_prefill_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __g
           }
         }
       };
-      // P = exp2(S * scale - m) of 8 keys, rounded to bfloat16: one 16-byte column of the A operand
-      auto exp8 = [&](int c, uint32_t* w) {
-#pragma unroll
-        for (int e = 0; e < 4; ++e) {
-          float x0, x1;
-          fma2(x0, x1, sv[c * 8 + 2 * e], sv[c * 8 + 2 * e + 1], scale_log2, -m_use);
-          const float p0 = fast_exp2(x0), p1 = fast_exp2(x1);
-          add2(rs, rs_hi, p0, p1);
-          __nv_bfloat162 two = __floats2bfloat162_rn(p0, p1);
-          w[e] = *reinterpret_cast<uint32_t*>(&two);
-        }
-      };
-      // K-major A operand: 64-key chunk h, 16-byte column c ^ (r % 8) of row r
-      auto store8 = [&](int h, int c, const uint32_t* w) {
-        *reinterpret_cast<uint4*>(p_row + h * SUB + ((c ^ (r & 7)) << 4)) = make_uint4(w[0], w[1], w[2], w[3]);
-      };
-      auto s_consumed = [&]() {                        // S of this step may be overwritten
-        asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
-        __syncwarp();
-        if (lane == 0) mbar_arrive(&s_free[t]);
-      };
-      // One pass in the common case: the exponent's reference is the one of the step before, which
-      // is good as long as no row's maximum outgrows it by more than 2^8.
-      load_half(0);
-#pragma unroll
-      for (int e = 0; e < 64; ++e) mx = fmaxf(mx, sv[e]);
-#pragma unroll
-      for (int c = 0; c < 8; ++c) exp8(c, pk + 4 * c);
-      load_half(1);
-#pragma unroll
-      for (int e = 0; e < 64; ++e) mx = fmaxf(mx, sv[e]);
-      mx *= scale_log2;                               // scale_log2 > 0: the maximum commutes with it
-      const bool outgrown = mx > m_ref + 8.f;         // also the first keys a row sees (m_ref = -inf)
-      if (!__any_sync(0xffffffffu, outgrown)) {
-        s_consumed();
-        // P's tile and O are free once PV of the step before has finished
-        if (i > 0) ok = mbar_wait(&o_ready[t], (i - 1) & 1, abort);
-        if (!ok) break;
-#pragma unroll
-        for (int c = 0; c < 8; ++c) store8(0, c, pk + 4 * c);
-#pragma unroll
-        for (int c = 0; c < 8; ++c) {
-          uint32_t w[4];
-          exp8(c, w);
-          store8(1, c, w);
-        }
-      } else {
-        // a new reference: rescale what has been accumulated, then redo this step's P
-        const float m_new = fmaxf(m_ref, mx);
-        const float alpha = m_ref == -INFINITY ? 1.f : fast_exp2(m_ref - m_new);
-        if (i > 0) {
-          ok = mbar_wait(&o_ready[t], (i - 1) & 1, abort);
-          if (!ok) break;
-          asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+      if constexpr (CAP) {
+        // Half after half, one piece of code for both and for what is done again.  As straight code (below) the capped kernel spills
+        // 230 bytes a thread, and a block's first steps take as long to fetch as to run: 2,048 tokens of window 1,024 47.7 us against
+        // 44.5 here, 500 tokens 21.5 / 19.9, 150 tokens 13.3 / 11.8.  Without the cap the exponentials are the bound and the votes
+        // between them cost more: 2,000 tokens 35.3 us straight, 39.8 this way.
 #pragma unroll 1
-          for (int c = 0; c < vdim; c += 32) {
-            float ov[32];
-            tmem_load32(tmem_o + c, ov);
+        for (int h = 0; h < 2; ++h) {
+          load_half(h);
+          float mx = -INFINITY, mx2 = -INFINITY;
 #pragma unroll
-            for (int e = 0; e < 32; ++e) ov[e] *= alpha;
-            tmem_store32(tmem_o + c, ov);
+          for (int e = 0; e < 64; e += 2) {
+            mx = fmaxf(mx, sv[e]);
+            mx2 = fmaxf(mx2, sv[e + 1]);
           }
-          asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
-        }
-        l_run *= alpha;
-        m_ref = m_new;
-        m_use = m_ref == -INFINITY ? 0.f : m_ref;
-        rs = 0.f;
-        rs_hi = 0.f;
+          mx = fmaxf(mx, mx2) * scale_log2;             // scale_log2 > 0: the maximum commutes with it
+          const bool outgrown = mx > m_ref + 8.f;       // also the first keys a row sees (m_ref = -inf)
+          if (__any_sync(0xffffffffu, outgrown)) {
+            // a new reference: rescale what has been accumulated
+            const float m_new = fmaxf(m_ref, mx);
+            const float alpha = m_ref == -INFINITY ? 1.f : fast_exp2(m_ref - m_new);
+            if (i > 0) {
+              ok = mbar_wait(&o_ready[t], (i - 1) & 1, abort);
+              if (!ok) break;
+              asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+#pragma unroll 1
+              for (int c = 0; c < vdim; c += 32) {
+                float ov[32];
+                tmem_load32(tmem_o + c, ov);
 #pragma unroll
-        for (int c = 0; c < 8; ++c) {
-          uint32_t w[4];
-          exp8(c, w);
-          store8(1, c, w);
+                for (int e = 0; e < 32; ++e) ov[e] *= alpha;
+                tmem_store32(tmem_o + c, ov);
+              }
+              asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
+            }
+            l_run *= alpha;
+            m_ref = m_new;
+            if (h == 1) {                               // the first half again, on the new reference
+              rs = rs_hi = 0.f;
+              h = -1;
+              continue;
+            }
+          }
+          if (h == 1) {                                 // S of this step may be overwritten
+            asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+            __syncwarp();
+            if (lane == 0) mbar_arrive(&s_free[t]);
+          }
+          const float m_use = m_ref == -INFINITY ? 0.f : m_ref;
+          uint32_t pk[32];                              // P = exp2(S * scale - m), rounded to bfloat16
+#pragma unroll
+          for (int e = 0; e < 32; ++e) {
+            float x0, x1;
+            fma2(x0, x1, sv[2 * e], sv[2 * e + 1], scale_log2, -m_use);
+            const float p0 = fast_exp2(x0), p1 = fast_exp2(x1);
+            add2(rs, rs_hi, p0, p1);
+            __nv_bfloat162 two = __floats2bfloat162_rn(p0, p1);
+            pk[e] = *reinterpret_cast<uint32_t*>(&two);
+          }
+          // P's tile is free once PV of the step before has finished
+          if (h == 0 && i > 0) ok = mbar_wait(&o_ready[t], (i - 1) & 1, abort);
+          if (!ok) break;
+          // K-major A operand: 64-key chunk h, 16-byte column c ^ (r % 8) of row r
+#pragma unroll
+          for (int c = 0; c < 8; ++c)
+            *reinterpret_cast<uint4*>(p_row + h * SUB + ((c ^ (r & 7)) << 4)) =
+                make_uint4(pk[4 * c], pk[4 * c + 1], pk[4 * c + 2], pk[4 * c + 3]);
         }
+        if (!ok) break;
+      } else {
+        uint32_t pk[32];
+        float mx = -INFINITY, m_use = m_ref == -INFINITY ? 0.f : m_ref;
+        // P = exp2(S * scale - m) of 8 keys, rounded to bfloat16: one 16-byte column of the A operand
+        auto exp8 = [&](int c, uint32_t* w) {
+#pragma unroll
+          for (int e = 0; e < 4; ++e) {
+            float x0, x1;
+            fma2(x0, x1, sv[c * 8 + 2 * e], sv[c * 8 + 2 * e + 1], scale_log2, -m_use);
+            const float p0 = fast_exp2(x0), p1 = fast_exp2(x1);
+            add2(rs, rs_hi, p0, p1);
+            __nv_bfloat162 two = __floats2bfloat162_rn(p0, p1);
+            w[e] = *reinterpret_cast<uint32_t*>(&two);
+          }
+        };
+        // K-major A operand: 64-key chunk h, 16-byte column c ^ (r % 8) of row r
+        auto store8 = [&](int h, int c, const uint32_t* w) {
+          *reinterpret_cast<uint4*>(p_row + h * SUB + ((c ^ (r & 7)) << 4)) = make_uint4(w[0], w[1], w[2], w[3]);
+        };
+        auto s_consumed = [&]() {                        // S of this step may be overwritten
+          asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+          __syncwarp();
+          if (lane == 0) mbar_arrive(&s_free[t]);
+        };
+        // One pass in the common case: the exponent's reference is the one of the step before, which
+        // is good as long as no row's maximum outgrows it by more than 2^8.
         load_half(0);
-        s_consumed();
 #pragma unroll
-        for (int c = 0; c < 8; ++c) {
-          uint32_t w[4];
-          exp8(c, w);
-          store8(0, c, w);
+        for (int e = 0; e < 64; ++e) mx = fmaxf(mx, sv[e]);
+#pragma unroll
+        for (int c = 0; c < 8; ++c) exp8(c, pk + 4 * c);
+        load_half(1);
+#pragma unroll
+        for (int e = 0; e < 64; ++e) mx = fmaxf(mx, sv[e]);
+        mx *= scale_log2;                               // scale_log2 > 0: the maximum commutes with it
+        const bool outgrown = mx > m_ref + 8.f;         // also the first keys a row sees (m_ref = -inf)
+        if (!__any_sync(0xffffffffu, outgrown)) {
+          s_consumed();
+          // P's tile and O are free once PV of the step before has finished
+          if (i > 0) ok = mbar_wait(&o_ready[t], (i - 1) & 1, abort);
+          if (!ok) break;
+#pragma unroll
+          for (int c = 0; c < 8; ++c) store8(0, c, pk + 4 * c);
+#pragma unroll
+          for (int c = 0; c < 8; ++c) {
+            uint32_t w[4];
+            exp8(c, w);
+            store8(1, c, w);
+          }
+        } else {
+          // a new reference: rescale what has been accumulated, then redo this step's P
+          const float m_new = fmaxf(m_ref, mx);
+          const float alpha = m_ref == -INFINITY ? 1.f : fast_exp2(m_ref - m_new);
+          if (i > 0) {
+            ok = mbar_wait(&o_ready[t], (i - 1) & 1, abort);
+            if (!ok) break;
+            asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+#pragma unroll 1
+            for (int c = 0; c < vdim; c += 32) {
+              float ov[32];
+              tmem_load32(tmem_o + c, ov);
+#pragma unroll
+              for (int e = 0; e < 32; ++e) ov[e] *= alpha;
+              tmem_store32(tmem_o + c, ov);
+            }
+            asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
+          }
+          l_run *= alpha;
+          m_ref = m_new;
+          m_use = m_ref == -INFINITY ? 0.f : m_ref;
+          rs = 0.f;
+          rs_hi = 0.f;
+#pragma unroll
+          for (int c = 0; c < 8; ++c) {
+            uint32_t w[4];
+            exp8(c, w);
+            store8(1, c, w);
+          }
+          load_half(0);
+          s_consumed();
+#pragma unroll
+          for (int c = 0; c < 8; ++c) {
+            uint32_t w[4];
+            exp8(c, w);
+            store8(0, c, w);
+          }
         }
       }
       l_run += rs + rs_hi;
@@ -423,7 +504,24 @@ attention_prefill_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __g
       if (lane == 0) mbar_arrive(&p_ready[t]);
     }
     if (ok && n_mine > 0) ok = mbar_wait(&o_ready[t], (n_mine - 1) & 1, abort);
-    if (ok && n_mine > 0) {
+    if (splits > 1) {
+      if constexpr (DC == 2 || VC == 1) {
+        if (n_mine > 0) row_state = make_float2(m_ref, l_run);
+        if (ok && n_mine > 0) {
+          asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+#pragma unroll 1
+          for (int c = 0; c < VC * 64; c += 32) {
+            float ov[32];
+            tmem_load32(tmem_o + c, ov);
+#pragma unroll
+            for (int d = 0; d < 32; d += 4)
+              *reinterpret_cast<float4*>(part_piece<64, VC * 64>(p_sm + t * P_BYTES, q_sm + t * Q_BYTES, r, (c + d) / 4)) =
+                  make_float4(ov[d], ov[d + 1], ov[d + 2], ov[d + 3]);
+          }
+          asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+        }
+      }
+    } else if (ok && n_mine > 0) {
       asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
       const bool valid = t * TC_BQ + r < rows_valid;
       float inv = 1.f / l_run;
@@ -453,6 +551,28 @@ attention_prefill_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __g
   }
 
   asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+  if constexpr (DC == 2 || VC == 1) {
+    if (splits > 1) {
+      // (the rows' states lie where keys were: both tiles are done with them behind the block's barrier)
+      float2* ml = reinterpret_cast<float2*>(ring);
+      __syncthreads();
+      if (threadIdx.x < 2 * TC_BQ) ml[threadIdx.x] = row_state;
+      __syncwarp();
+      cluster_barrier();
+      if (threadIdx.x < 2 * TC_BQ) {
+        const size_t row0 = (size_t)seq_q_start[seq] + q_first;
+        merge_parts<64, VC * 64, Q_BYTES, P_BYTES>(
+            q_sm, p_sm, ml, part, splits, rows_valid, vdim, out + row0 * ((size_t)heads * vdim) + (size_t)head * vdim,
+            (size_t)heads * vdim, [&](int row, float, float sum) {
+              float inv = 1.f / sum;
+              if (EXT && ex.gate) inv *= ex.gate[(row0 + row) * heads + head];
+              return inv;
+            });
+      }
+      __syncwarp();
+      cluster_barrier();                            // nobody leaves while others read from it
+    }
+  }
   __syncthreads();
   if (warp == 9) {
     __syncwarp();
@@ -468,7 +588,7 @@ static int launch(const CUtensorMap& mq, const CUtensorMap& mk, const CUtensorMa
                   const int* block_table, int table_stride, const int* seq_slot, const int* seq_q_start,
                   const int* seq_q_len, const int* seq_kv_len, const int* tile_seq, const int* tile_first,
                   int n_tiles, int heads, int kv_heads, float scale, int window, int* status, int list_of_blocks,
-                  cudaStream_t s, TcExtras ex = TcExtras{nullptr, nullptr, nullptr, nullptr, 0, 0, 0.f, 0.f, DC * 64, VC * 64}) {
+                  int splits, cudaStream_t s, TcExtras ex = TcExtras{nullptr, nullptr, nullptr, nullptr, 0, 0, 0.f, 0.f, DC * 64, VC * 64}) {
   const int smem = (2 * DC + 4 + TC_RING * (DC > VC ? DC : VC)) * 128 * 128 + 1024;
   static bool configured = false;
   if (!configured) {
@@ -476,10 +596,11 @@ static int launch(const CUtensorMap& mq, const CUtensorMap& mk, const CUtensorMa
     if (e != cudaSuccess) return (int)e;
     configured = true;
   }
-  return launch_dependent(attention_prefill_tc_kernel<DC, VC, EXT>, dim3(heads, n_tiles), dim3(TC_THREADS), smem, s, mq, mk,
-                          mv, (bf16*)out, block_table, table_stride, seq_slot, seq_q_start, seq_q_len, seq_kv_len,
-                          tile_seq, tile_first, heads, kv_heads, scale * 1.4426950408889634f, window, status,
-                          list_of_blocks, ex);
+  if (splits < 1 || splits > 8 || (splits & (splits - 1)) || (DC == 1 && VC == 2)) splits = 1;
+  return launch_dependent_cluster(attention_prefill_tc_kernel<DC, VC, EXT>, dim3(heads * splits, n_tiles), dim3(TC_THREADS), smem, s,
+                                  dim3(splits), mq, mk, mv, (bf16*)out, block_table, table_stride, seq_slot, seq_q_start, seq_q_len,
+                                  seq_kv_len, tile_seq, tile_first, heads, kv_heads, scale * 1.4426950408889634f, window, status,
+                                  list_of_blocks, splits, ex);
 }
 
 static unsigned long long next_limit_ns = WAIT_LIMIT_NS;
@@ -497,14 +618,15 @@ void sb_attention_prefill_tc_withhold(int step, unsigned long long limit_ns) {
 }
 
 // Same contract as sb_attention_prefill; n_tokens rows in q/out, n_pages pages in the stores.
-// list_of_blocks: tile_seq/tile_first list blocks of 256 queries (else tiles of 64, see the kernel).
+// list_of_blocks: tile_seq/tile_first list blocks of 256 queries (else tiles of 64, see the kernel).  splits: CTAs that share a block's
+// keys (1, 2, 4 or 8; 1 where keys of up to 64 entries have values of more).
 // head_dim must be 64 or 128 (returns -2 otherwise).
 int sb_attention_prefill_tc(const void* q, void* out, const void* k_store, const void* v_store,
                             const int* block_table, int table_stride, const int* seq_slot,
                             const int* seq_q_start, const int* seq_q_len, const int* seq_kv_len,
                             const int* tile_seq, const int* tile_first, int n_tiles, int n_tokens,
                             int n_pages, int heads, int kv_heads, int head_dim, float scale, int window,
-                            int* status, int list_of_blocks, cudaStream_t s) {
+                            int* status, int list_of_blocks, int splits, cudaStream_t s) {
   if (n_tiles == 0) return 0;
   if (kv_heads <= 0 || heads % kv_heads) return -2;
   if (head_dim != 64 && head_dim != 128) return -2;
@@ -518,7 +640,7 @@ int sb_attention_prefill_tc(const void* q, void* out, const void* k_store, const
   rc = sb_make_map(&mv, v_store, kv_rows, head_dim, SB_PAGE_TOKENS);
   if (rc) return rc;
 #define ARGS mq, mk, mv, out, block_table, table_stride, seq_slot, seq_q_start, seq_q_len, seq_kv_len, \
-             tile_seq, tile_first, n_tiles, heads, kv_heads, scale, window, status, list_of_blocks, s
+             tile_seq, tile_first, n_tiles, heads, kv_heads, scale, window, status, list_of_blocks, splits, s
   const bool test_run = next_withhold_step >= 0;
   if (test_run) {
     cudaMemcpyToSymbolAsync(tc_withhold_step, &next_withhold_step, sizeof(int), 0, cudaMemcpyHostToDevice, s);
@@ -547,7 +669,7 @@ int sb_sink_attention_tcgen05(const void* q, int q_width, void* out, const void*
                               const int* seq_q_len, const int* seq_kv_len, const int* tile_seq, const int* tile_first,
                               int n_tiles, int n_tokens, int n_pages, int heads, int kv_heads, int dim, int vdim, float scale,
                               const float* r1, const float* r2, const float* sink, const float* gate, int chunk, int window,
-                              int keep, float cap, int* status, int list_of_blocks, cudaStream_t s) {
+                              int keep, float cap, int* status, int list_of_blocks, int splits, cudaStream_t s) {
   if (n_tiles == 0) return 0;
   if (kv_heads <= 0 || heads % kv_heads || !(scale > 0.f) || keep < 0) return -2;
   if (dim < 16 || dim > 128 || dim % 16 || vdim < 16 || vdim > 128 || vdim % 8) return -2;
@@ -564,7 +686,7 @@ int sb_sink_attention_tcgen05(const void* q, int q_width, void* out, const void*
   const TcExtras ex{r1, r2, sink, gate, chunk > 0 ? chunk : 0, chunk > 0 || window > 0 ? keep : 0,
                     cap > 0.f ? scale / cap : 0.f, cap > 0.f ? cap / scale : 0.f, dim, vdim};
 #define ARGS mq, mk, mv, out, block_table, table_stride, seq_slot, seq_q_start, seq_q_len, seq_kv_len, tile_seq, \
-             tile_first, n_tiles, heads, kv_heads, scale, window, status, list_of_blocks, s, ex
+             tile_first, n_tiles, heads, kv_heads, scale, window, status, list_of_blocks, splits, s, ex
   const int kind = (dim > 64) * 2 + (vdim > 64);
   if (ex.cap_out == 0.f)
     return kind == 0 ? launch<1, 1, 1>(ARGS) : kind == 1 ? launch<1, 2, 1>(ARGS) : kind == 2 ? launch<2, 1, 1>(ARGS) : launch<2, 2, 1>(ARGS);

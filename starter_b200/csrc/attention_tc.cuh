@@ -175,3 +175,73 @@ __device__ __forceinline__ uint32_t instr_desc(int n, int b_mn_major) {
   return (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)b_mn_major << 16) | ((uint32_t)(n >> 3) << 17) |
          ((uint32_t)(TC_BQ >> 4) << 24);
 }
+
+// ------------------------------------------------------------------------------------------ keys in parts
+// With few blocks of queries the CTAs of a cluster share a block: each walks a part of its keys, files its rows' reference, sum and
+// output (float, unscaled) in its own shared memory, and after the cluster's barrier every CTA merges its share of the rows, reading
+// the others' through distributed shared memory.  A tile's output lies where its own weights and queries were (nobody else
+// reads those): PC columns in P's tile, the rest in Q's, 16-byte pieces swizzled over eight.
+template <int PC, int COLS>
+__device__ __forceinline__ float* part_piece(uint8_t* p_tile, uint8_t* q_tile, int r, int piece) {
+  constexpr int QW = COLS > PC ? COLS - PC : PC;
+  return piece * 4 < PC ? reinterpret_cast<float*>(p_tile + r * (PC * 4) + ((piece ^ (r & 7)) << 4))
+                        : reinterpret_cast<float*>(q_tile + r * (QW * 4) + (((piece - PC / 4) ^ (r & 7)) << 4));
+}
+__device__ __forceinline__ void cluster_barrier() {
+  asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
+}
+__device__ __forceinline__ uint32_t peer_u32(const void* p, int rank) {
+  uint32_t a;
+  asm("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(a) : "r"(smem_u32(p)), "r"(rank));
+  return a;
+}
+__device__ __forceinline__ float4 peer_load4(uint32_t a) {
+  float4 v;
+  asm volatile("ld.shared::cluster.v4.f32 {%0, %1, %2, %3}, [%4];" : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w) : "r"(a) : "memory");
+  return v;
+}
+__device__ __forceinline__ float2 peer_load2(uint32_t a) {
+  float2 v;
+  asm volatile("ld.shared::cluster.v2.f32 {%0, %1}, [%2];" : "=f"(v.x), "=f"(v.y) : "r"(a) : "memory");
+  return v;
+}
+// The rows of this CTA's share, by its first 256 threads: 16 threads a row, eight columns each.  ml: [2 tiles][128 rows] of (reference,
+// sum); finish(t, r, reference, sum) gives the factor of the row's summed outputs; dst: output row 0 of the block, `cols` entries of a
+// head, rows `stride` apart.
+template <int PC, int COLS, int Q_BYTES, int P_BYTES, typename Finish>
+__device__ __forceinline__ void merge_parts(uint8_t* q_sm, uint8_t* p_sm, float2* ml, int rank, int splits, int rows_valid, int cols,
+                                            bf16* dst, size_t stride, Finish finish) {
+  const int share = 2 * TC_BQ / splits, c = (threadIdx.x & 15) * 8;
+  if (c >= COLS || c >= cols) return;
+  for (int n = threadIdx.x >> 4; n < share; n += 16) {
+    const int row = rank * share + n, t = row / TC_BQ, r = row % TC_BQ;
+    if (row >= rows_valid) return;
+    float top = -INFINITY;
+    float2 part[8];
+#pragma unroll
+    for (int p = 0; p < 8; ++p) {
+      part[p] = p < splits ? peer_load2(peer_u32(ml + t * TC_BQ + r, p)) : make_float2(-INFINITY, 0.f);
+      if (part[p].y > 0.f) top = fmaxf(top, part[p].x);
+    }
+    float sum = 0.f, o[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
+    const float* a = part_piece<PC, COLS>(p_sm + t * P_BYTES, q_sm + t * Q_BYTES, r, c / 4);
+    const float* b = part_piece<PC, COLS>(p_sm + t * P_BYTES, q_sm + t * Q_BYTES, r, c / 4 + 1);
+#pragma unroll
+    for (int p = 0; p < 8; ++p) {
+      if (p >= splits || !(part[p].y > 0.f)) continue;       // (a part without keys filed nothing)
+      const float w = fast_exp2(part[p].x - top);
+      sum = fmaf(w, part[p].y, sum);
+      const float4 x = peer_load4(peer_u32(a, p)), y = peer_load4(peer_u32(b, p));
+      o[0] = fmaf(w, x.x, o[0]); o[1] = fmaf(w, x.y, o[1]); o[2] = fmaf(w, x.z, o[2]); o[3] = fmaf(w, x.w, o[3]);
+      o[4] = fmaf(w, y.x, o[4]); o[5] = fmaf(w, y.y, o[5]); o[6] = fmaf(w, y.z, o[6]); o[7] = fmaf(w, y.w, o[7]);
+    }
+    const float inv = finish(row, top, sum);
+    uint32_t w[4];
+#pragma unroll
+    for (int e = 0; e < 4; ++e) {
+      const __nv_bfloat162 two = __floats2bfloat162_rn(o[2 * e] * inv, o[2 * e + 1] * inv);
+      w[e] = *reinterpret_cast<const uint32_t*>(&two);
+    }
+    *reinterpret_cast<uint4*>(dst + (size_t)row * stride + c) = make_uint4(w[0], w[1], w[2], w[3]);
+  }
+}

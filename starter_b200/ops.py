@@ -568,7 +568,7 @@ PREFILL_HEAD_DIMS = (16, 32, 64, 128)
 
 def attention_prefill(q, k_store, v_store, block_table, seq_slot, seq_q_start, seq_q_len, seq_kv_len,
                       tile_seq, tile_first, heads, kv_heads, head_dim, scale, window=None, status=None,
-                      kernel=None, max_q_len=None, blocks=None, withhold=None):
+                      kernel=None, max_q_len=None, blocks=None, withhold=None, kv_hint=0):
     """Causal attention for steps with many tokens per sequence (bfloat16, tensor cores).
 
     ``q`` ``[T, heads * head_dim]`` packed by sequence; the ``seq_*`` arrays describe each sequence
@@ -617,8 +617,8 @@ def attention_prefill(q, k_store, v_store, block_table, seq_slot, seq_q_start, s
             q, out, k_store, v_store, block_table, block_table.shape[1],
             seq_slot, seq_q_start, seq_q_len, seq_kv_len, list_seq,
             list_first, list_seq.shape[0], q.shape[0], k_store.shape[0], heads, kv_heads, head_dim,
-            scale, int(window or 0), status if status is not None else None,
-            int(own_list), _stream())
+            scale, int(window or 0), status, int(own_list),
+            prompt_splits(heads * list_first.shape[0], kv_hint, window) if own_list else 1, _stream())
         _check(rc, "attention_prefill_tc")
         return out
     rc = _lib("attention_prefill").sb_attention_prefill(
@@ -631,6 +631,22 @@ def attention_prefill(q, k_store, v_store, block_table, seq_slot, seq_q_start, s
 
 
 PREFILL_TC_HEAD_DIMS = (64, 128)
+
+
+def prompt_splits(blocks: int, keys: int, window=None, from_keys: int = 1100) -> int:
+    """How many CTAs share the keys of a block of 256 queries (one cluster, csrc/attention_tc.cuh) in a step of ``blocks`` blocks of
+    up to ``keys`` keys: 4 or 2, as long as all are resident at once, from ``from_keys`` keys that a block walks (the cluster's
+    launch, two barriers and the merge cost 3 us, a step of 128 keys saved 1.3).  Measured (us, one CTA / 2 / 4): plain attention,
+    300 tokens behind 1,000 24.6 / 22.0 / 20.9, 700 behind 1,200 33.0 / 27.2, 1,000 tokens 20.5 / 20.0, 700 tokens 16.7 / 18.0; latent
+    attention, 700 behind 1,200 60.1 / 48.6, 1,000 tokens 38.0 / 36.2, 600 tokens 27.6 / 28.8; capped scores, whose steps take three times
+    as long, 500 tokens 19.9 / 19.5 / 17.0, 1,000 tokens 31.0 / 25.8, 233 tokens twice 18.8 / 21.0 / 17.4.  Eight are slower throughout."""
+    if window:
+        keys = min(keys, window + 256)
+    if keys < from_keys:
+        return 1
+    return 4 if 4 * blocks <= SM_COUNT else 2 if 2 * blocks <= SM_COUNT else 1
+
+
 DECODE_CLUSTER_SPLITS = 8
 DECODE_HEAD_DIMS = (16, 32, 64, 128, 256)
 
@@ -1761,7 +1777,8 @@ def latent_attention_prompt(q, ukv, store, block_table, ctx, heads, dim, vdim, r
     rc = lib.sb_latent_prompt(
         q, kv, shared, out, ctx.seq_q_start, ctx.seq_q_len, ctx.seq_kv_len,
         ctx.block_seq, ctx.block_first, ctx.block_seq.shape[0], n_tokens, rows, heads, dim, vdim,
-        scale, int(window or 0), _latent_sink(sink, heads), ctx.status, _stream())
+        scale, int(window or 0), _latent_sink(sink, heads), ctx.status,
+        prompt_splits(heads * ctx.block_first.shape[0], ctx.max_kv_len, window), _stream())
     _check(rc, "latent_attention_prompt")
     return out
 
@@ -2247,7 +2264,7 @@ def sink_tcgen05_takes(q, dim, vdim) -> bool:
 
 def sink_attention_tcgen05(q, k_store, v_store, block_table, seq_slot, seq_q_start, seq_q_len, seq_kv_len, tile_seq,
                            tile_first, heads, kv_heads, dim, scale, penalty=None, sink=None, gate=None, chunk=None,
-                           window=None, status=None, blocks=None, vdim=None, keep_first=0, softcap=None):
+                           window=None, status=None, blocks=None, vdim=None, keep_first=0, softcap=None, kv_hint=0):
     """``sink_attention`` for prompts on the tcgen05 kernel of ``attention_prefill`` (256 queries of a head a
     block, S and O in tensor memory), which takes the penalty, the chunks, the sink, the gate,
     the kept keys, the cap and values of another size (``vdim``) than the keys as extras.
@@ -2276,7 +2293,8 @@ def sink_attention_tcgen05(q, k_store, v_store, block_table, seq_slot, seq_q_sta
         seq_slot, seq_q_start, seq_q_len, seq_kv_len, list_seq, list_first,
         list_seq.shape[0], q.shape[0], k_store.shape[0], heads, kv_heads, dim, vdim, scale, r1, r2,
         sink, gate, int(chunk or 0), int(window or 0), int(keep_first), softcap or 0.0,
-        status, int(own_list), _stream())
+        status, int(own_list),
+        prompt_splits(heads * list_first.shape[0], kv_hint, window, 450 if softcap else 1100) if own_list else 1, _stream())
     _check(rc, "sink_attention_tcgen05")
     return out
 
@@ -2290,7 +2308,7 @@ def sink_attention_step(q, k_store, v_store, block_table, ctx, heads, kv_heads, 
         return sink_attention_tcgen05(q, k_store, v_store, block_table, ctx.seq_slot, ctx.seq_q_start, ctx.seq_q_len,
                                       ctx.seq_kv_len, ctx.tile_seq, ctx.tile_first, heads, kv_heads, dim, scale, penalty,
                                       sink, gate, chunk, window, ctx.status, (ctx.block_seq, ctx.block_first), vdim,
-                                      keep_first, softcap)
+                                      keep_first, softcap, ctx.max_kv_len)
     if sink_tc_takes(q, heads, kv_heads, dim, vdim):
         splits = 1
         if ctx.max_q_len == 1:

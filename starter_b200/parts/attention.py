@@ -104,7 +104,7 @@ class GroupedQueryAttention(Part):
                                       ctx.seq_q_len, ctx.seq_kv_len, ctx.tile_seq, ctx.tile_first,
                                       s.num_heads, s.num_kv_heads, s.head_dim, s.scale, s.window,
                                       status=ctx.status, max_q_len=ctx.max_q_len,
-                                      blocks=(ctx.block_seq, ctx.block_first))
+                                      blocks=(ctx.block_seq, ctx.block_first), kv_hint=ctx.max_kv_len)
         else:
             a = ops.attention_rowwise(q, keys, values, cache.block_table, ctx.tok_slot, ctx.tok_pos,
                                       s.num_heads, s.num_kv_heads, s.head_dim, s.scale, s.window)

@@ -1,0 +1,98 @@
+"""Prompt attention whose blocks' keys are shared by the CTAs of a cluster, against one CTA a block: plain, with every extra, over
+formed keys; sequences of a few keys (fewer steps than parts), ragged ones, windows, chunks."""
+
+from types import SimpleNamespace
+
+import pytest
+import torch
+
+from starter_b200.engine.batch import plan_step
+
+pytestmark = pytest.mark.gpu
+BF = torch.bfloat16
+LENGTHS, PAST = [300, 1, 700, 129, 256], [0, 40, 513, 1100, 64]
+
+
+def step(n_heads_kv, dim, vdim, seed):
+    """Pages of random keys and values, and the step's arrays."""
+    pages = [-(-(p + n) // 64) for p, n in zip(PAST, LENGTHS)]
+    gen = torch.Generator().manual_seed(seed)
+    table, at = torch.zeros(len(pages), max(pages), dtype=torch.int32), 0
+    for i, n in enumerate(pages):
+        table[i, :n] = torch.randperm(n, generator=gen) + at
+        at += n
+    store = [(torch.randn(at, n_heads_kv, 64, size, generator=gen)).to(BF).cuda() for size in (dim, vdim)]
+    arrays = plan_step([SimpleNamespace(slot=i, tokens=[0] * n, want=[]) for i, n in enumerate(LENGTHS)], PAST)
+    ctx = SimpleNamespace(host=arrays, n_seqs=len(LENGTHS), max_q_len=max(LENGTHS), max_kv_len=int(arrays["seq_kv_len"].max()),
+                          status=torch.zeros(1, dtype=torch.int32).cuda(),
+                          **{k: torch.from_numpy(v).cuda() for k, v in arrays.items()})
+    return gen, table.cuda(), store, ctx
+
+
+def same(monkeypatch, run, status):
+    """Every number of parts gives what one gives, but for roundings: weights and outputs round to 2^-9 of themselves each."""
+    from starter_b200 import ops
+
+    got = {}
+    for parts in (1, 2, 4, 8):
+        monkeypatch.setattr(ops, "prompt_splits", lambda *a, **k: parts)
+        got[parts] = run().float()
+    assert int(status.item()) == 0 and bool(torch.isfinite(got[1]).all())
+    for parts in (2, 4, 8):
+        assert float((got[parts] - got[1]).abs().max()) <= 2.0 ** -7 * float(got[1].abs().max())
+        assert float((got[parts] - got[1]).norm()) <= 2.0 ** -8 * float(got[1].norm())
+        if parts > 2:
+            assert not torch.equal(got[parts], got[1])
+
+
+@pytest.mark.parametrize("dim", [64, 128])
+@pytest.mark.parametrize("window", [None, 200])
+def test_plain(dim, window, monkeypatch):
+    from starter_b200 import ops
+
+    gen, table, (keys, values), ctx = step(2, dim, dim, dim)
+    q = torch.randn(sum(LENGTHS), 4 * dim, generator=gen).to(BF).cuda()
+    same(monkeypatch, lambda: ops.attention_prefill(
+        q, keys, values, table, ctx.seq_slot, ctx.seq_q_start, ctx.seq_q_len, ctx.seq_kv_len, ctx.tile_seq, ctx.tile_first, 4, 2, dim,
+        dim ** -0.5, window, status=ctx.status, kernel="tcgen05", max_q_len=ctx.max_q_len, blocks=(ctx.block_seq, ctx.block_first),
+        kv_hint=ctx.max_kv_len), ctx.status)
+
+
+@pytest.mark.parametrize("dim,vdim,chunk,window,keep,cap,penalty,gated", [
+    (128, 128, None, 256, 0, 50.0, False, False), (48, 40, None, None, 0, 1.0, False, True), (128, 64, 300, None, 70, None, True, True),
+    (64, 64, None, 130, 5, 30.0, True, False)])
+def test_with_extras(dim, vdim, chunk, window, keep, cap, penalty, gated, monkeypatch):
+    from starter_b200 import ops
+
+    gen, table, (keys, values), ctx = step(2, dim, vdim, dim + vdim)
+    q = torch.randn(sum(LENGTHS), 4 * dim, generator=gen).to(BF).cuda()
+    slopes = tuple(torch.rand(4, generator=gen).cuda() + 0.1 for _ in range(2)) if penalty else None
+    gate = torch.rand(sum(LENGTHS), 4, generator=gen).cuda() if gated else None
+    same(monkeypatch, lambda: ops.sink_attention_tcgen05(
+        q, keys, values, table, ctx.seq_slot, ctx.seq_q_start, ctx.seq_q_len, ctx.seq_kv_len, ctx.tile_seq, ctx.tile_first, 4, 2, dim,
+        dim ** -0.5, slopes, torch.linspace(-1.0, 2.0, 4).cuda(), gate, chunk, window, ctx.status, (ctx.block_seq, ctx.block_first), vdim,
+        keep, cap, ctx.max_kv_len), ctx.status)
+
+
+@pytest.mark.parametrize("dim,vdim", [(128, 128), (64, 64), (128, 64)])
+@pytest.mark.parametrize("window,sink", [(None, True), (150, False)])
+def test_over_formed_keys(dim, vdim, window, sink, monkeypatch):
+    from starter_b200 import ops
+
+    rank, heads = 128, 3
+    gen, table, (store, _), ctx = step(1, rank + 64, 16, dim)
+    q = torch.randn(sum(LENGTHS), heads * (dim + 64), generator=gen).to(BF).cuda()
+    ukv = (torch.randn(heads * (dim + vdim), rank, generator=gen) * rank ** -0.5).to(BF).cuda()
+    same(monkeypatch, lambda: ops.latent_attention_prompt(
+        q, ukv, store, table, ctx, heads, dim, vdim, rank, 64, (dim + 64) ** -0.5, window,
+        torch.linspace(-1.0, 2.0, heads).cuda() if sink else None), ctx.status)
+
+
+def test_parts_of_a_step():
+    from starter_b200 import ops
+
+    for blocks, keys, window, least in ((1, 5000, None, 1100), (37, 1100, None, 1100), (38, 2000, None, 1100), (74, 1100, 5000, 1100),
+                                        (75, 9000, None, 1100), (10, 1099, None, 1100), (10, 5000, 512, 1100), (10, 460, 400, 450)):
+        parts = ops.prompt_splits(blocks, keys, window, least)
+        assert parts in (1, 2, 4) and (parts == 1 or parts * blocks <= 148)
+        assert (parts > 1) == (blocks <= 74 and min(keys, window + 256 if window else keys) >= least)
