@@ -141,6 +141,10 @@ struct PromptGemmArgs {
   int act;                  // without gate: 0 the product itself, 1 relu(round(product))^2
 };
 
+// An expert's plain gate: silu(gate) * up, of which only the product is rounded (as moe.cu's and gemm_tcgen05.cu's experts have it; the
+// dense feed-forward rounds the first factor too).
+#define SB_ACT_EXPERT 4
+
 // ------------------------------------------------------------------------------------------ kernel
 
 // Which tile is the t-th.  Tiles that run at the same time (one per CTA pair, consecutive t) should
@@ -355,7 +359,10 @@ gemm_prompt_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_const
             else if (args.gated == SB_ACT_GELU_TANH) v[j] = rnd<bf16>(gate_act_fast(gr, SB_ACT_GELU_TANH)) * ur;
             // (both sides by a quarter: the fast quotient is zero for divisors above 2^126, which gates of -87.5 to -88.5 have; so
             // every bfloat16 gate gives what the exact quotient gives)
-            else v[j] = rnd<bf16>(__fdividef(0.25f * gr, fmaf(0.25f, __expf(-gr), 0.25f))) * ur;
+            else {
+              const float a = __fdividef(0.25f * gr, fmaf(0.25f, __expf(-gr), 0.25f));
+              v[j] = (args.gated == SB_ACT_EXPERT ? a : rnd<bf16>(a)) * ur;
+            }
           }
         } else {
           pg_tmem_load32(acc + c * 32, v);
@@ -531,7 +538,8 @@ static int pg_entry_grouped(const void* x, const void* w, void* out, int rows, i
 
 extern "C" {
 
-// See pg_entry_grouped.  gated: 0, or the code of a gated activation (3: the clamped gate with `limit`).
+// See pg_entry_grouped.  gated: 0, or the code of a gated activation (3: the clamped gate with `limit`, 4: silu(gate) * up with the
+// first factor as it is).
 int sb_gemm_prompt_grouped(const void* x, const void* w, void* out, int rows, int n_out, int k_dim, int experts,
                            const int* tile_expert, const int* m_tiles_dev, int max_m_tiles, const int* row_map,
                            int gated, int act, float limit, int* status, cudaStream_t s) {

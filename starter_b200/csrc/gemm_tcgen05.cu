@@ -17,6 +17,11 @@
 // With `gated`, w is [gate; up] stacked ([2 * n_out, k]); a tile holds 64 gate rows and the matching
 // 64 up rows and the epilogue writes round(silu(gate)) * up (fused.py:89-112).
 //
+// Grouped (routed experts of 5 to 64 rows an expert): the rows lie in the experts' order, whole tiles of BM to an expert, and the k-th
+// tile of rows takes its expert's weights.  An expert's weights are read once, its few rows ride along; the mma.sync tiles it
+// stands in for read them at a third of that rate (16 experts of 2 x 2,048 x 2,048, four a token, a whole layer: 32 tokens 172 ->
+// 88 us, 100 tokens 176 -> 94, 200 tokens 184 -> 106; the weights alone are 61 us of copy rate).
+//
 // Every wait on an mbarrier gives up after a time limit (WAIT_LIMIT_NS unless the caller gives one),
 // raises bit 4 of *status and lets the CTA drain, free its tensor memory and return.  So that this
 // path can be exercised without a fault, the entry point sb_gemm_tcgen05_withheld leaves out one
@@ -77,10 +82,30 @@ struct GemmArgs {
   float limit;                        // the clamp of the gated activation with code 3
 };
 
-template <int BM, bool GATED>
+// What the grouped product takes besides: x holds the rows in the experts' order, BM to a tile, padded with zeros; w the experts'
+// matrices one behind the other.
+struct GroupArgs {
+  const int* tile_expert;             // the expert of every tile of rows
+  const int* n_tiles;                 // how many tiles there are (the grid has room for more)
+  const int* sorted;                  // [tiles * BM]: the pair in each row, or -1
+  const float* in_scale;              // up passes: float [pairs] that multiplies a row's products, or null
+  int up;                             // 1: gate and up, 2: squared relu, both filed by row; 0: filed by pair
+};
+
+// The gated expert's activation from its (rounded) gate and up products: with a limit the clamped gate, without the plain silu.
+__device__ __forceinline__ float expert_gate(float g, float u, float limit) {
+  if (limit > 0.f) {
+    g = fminf(g, limit);
+    u = fminf(fmaxf(u, -limit), limit);
+    return g / (1.f + expf(-1.702f * g)) * (u + 1.f);
+  }
+  return g / (1.f + expf(-g)) * u;
+}
+
+template <int BM, bool GATED, bool GROUPED>
 __global__ void __launch_bounds__(GEMM_THREADS)
 gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant__ CUtensorMap map_x,
-                    const GemmArgs args) {
+                    const GemmArgs args, const GroupArgs group) {
   constexpr int B_BYTES = BM * TILE_K * 2;
   constexpr int STAGE_BYTES = A_BYTES + B_BYTES;
   constexpr uint32_t TMEM_COLS = BM < 32 ? 32 : BM;
@@ -102,10 +127,16 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_cons
   const int kb_begin = split * kb_per;
   const int kb_end = min(kb_begin + kb_per, kb_total);
   const int n_kb = max(kb_end - kb_begin, 0);
+  int w_row0 = 0;
+  if constexpr (GROUPED) {
+    pdl_wait();                        // (which expert's weights these are is what an earlier kernel found)
+    if (mtile >= *(const volatile int*)group.n_tiles) return;        // (the whole cluster)
+    w_row0 = *(const volatile int*)(group.tile_expert + mtile) * (GATED ? 2 * args.n_out : args.n_out);
+  }
   // rows of w in the two 64-row halves of the tile
-  const int row_a = GATED ? tile * 64 : tile * TILE_N;
-  const int row_b = GATED ? args.n_out + tile * 64 : tile * TILE_N + 64;
-  const int rows_here = min(BM, args.rows - m0);
+  const int row_a = w_row0 + (GATED ? tile * 64 : tile * TILE_N);
+  const int row_b = w_row0 + (GATED ? args.n_out + tile * 64 : tile * TILE_N + 64);
+  const int rows_here = GROUPED ? BM : min(BM, args.rows - m0);
   // the result goes straight from tensor memory to global memory unless parts must be added or
   // gate and up rows (held by different threads) must meet
   const bool staged = args.splits > 1 || GATED;
@@ -124,6 +155,14 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_cons
   asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
   const uint32_t tmem = tmem_holder;
   volatile int* abort = &abort_flag;
+  const int* sorted = group.sorted;
+  if constexpr (GROUPED) SB_BEHIND_WAIT(sorted);
+  // an ungated product's value of a row
+  auto grouped_value = [&](float v, int pair) {
+    if (group.up == 0) return v;
+    const float u = fmaxf(rnd<bf16>(group.in_scale ? v * group.in_scale[pair] : v), 0.f);
+    return u * u;
+  };
 
   if (warp == 0) {
     // ---------------- producer: the warp walks the ring together, one elected lane issues the copies.
@@ -134,7 +173,7 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_cons
     const bool elected = elect_one();
     int issued = 0;
     // the weights do not depend on the kernels before this one: the first stages' weight tiles are
-    // on their way before the predecessor has finished; the activations follow after the wait
+    // on their way before the predecessor has finished; the activations follow after the wait (grouped: all behind it)
     const int early = min(n_kb, STAGES);
     for (int i = 0; i < early; ++i) {
       uint8_t* a = smem + (size_t)i * STAGE_BYTES;
@@ -221,9 +260,16 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_cons
         for (int j = 0; j < 8; ++j) {
           const int m = c + j;
           if (m < rows_here) {
-            const size_t at = (size_t)(m0 + m) * args.n_out + n;
-            if (args.out_float) ((float*)args.out)[at] = v[j];
-            else ((bf16*)args.out)[at] = __float2bfloat16_rn(v[j]);
+            if constexpr (GROUPED) {
+              const int pair = sorted[m0 + m];
+              if (pair < 0) continue;
+              const size_t row = group.up ? (size_t)(m0 + m) : (size_t)pair;
+              ((bf16*)args.out)[row * args.n_out + n] = __float2bfloat16_rn(grouped_value(v[j], pair));
+            } else {
+              const size_t at = (size_t)(m0 + m) * args.n_out + n;
+              if (args.out_float) ((float*)args.out)[at] = v[j];
+              else ((bf16*)args.out)[at] = __float2bfloat16_rn(v[j]);
+            }
           }
         }
       }
@@ -265,7 +311,20 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_cons
             if (GATED) { u[0] += uv[s].x; u[1] += uv[s].y; u[2] += uv[s].z; u[3] += uv[s].w; }
           }
         }
-        if (GATED) {
+        int pair = 0;
+        if constexpr (GROUPED) {
+          pair = sorted[m0 + m];
+          if (pair < 0) continue;
+          if constexpr (GATED) {
+            const float by = group.in_scale ? group.in_scale[pair] : 1.f;
+#pragma unroll
+            for (int j = 0; j < 4; ++j) g[j] = expert_gate(rnd<bf16>(g[j] * by), rnd<bf16>(u[j] * by), args.limit);
+          } else {
+#pragma unroll
+            for (int j = 0; j < 4; ++j) g[j] = grouped_value(g[j], pair);
+          }
+        }
+        if (GATED && !GROUPED) {
 #pragma unroll
           for (int j = 0; j < 4; ++j) {
             const float gr = rnd<bf16>(g[j]), ur = rnd<bf16>(u[j]);
@@ -274,7 +333,7 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_cons
           }
         }
         const int ncol = (GATED ? tile * 64 : tile * TILE_N) + orow;
-        const size_t at = (size_t)(m0 + m) * args.n_out + ncol;
+        const size_t at = (size_t)(GROUPED && !group.up ? pair : m0 + m) * args.n_out + ncol;
         if (vector_store && ncol + 3 < args.n_out) {
           if (args.out_float) {
             *reinterpret_cast<float4*>((float*)args.out + at) = make_float4(g[0], g[1], g[2], g[3]);
@@ -307,21 +366,21 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_cons
 
 // ------------------------------------------------------------------------------------------ host
 
-template <int BM, bool GATED>
+template <int BM, bool GATED, bool GROUPED = false>
 static int launch(const CUtensorMap& map_w, const CUtensorMap& map_x, const GemmArgs& args, int tiles,
-                  int m_tiles, cudaStream_t s) {
+                  int m_tiles, cudaStream_t s, const GroupArgs& group = GroupArgs{nullptr, nullptr, nullptr, nullptr, 0}) {
   constexpr int STAGE_BYTES = A_BYTES + BM * TILE_K * 2;
   const int smem = args.stages * STAGE_BYTES + 1024;
   if (smem > 227 * 1024 || args.stages * STAGE_BYTES < BM * TILE_N * 4) return -2;
   static int configured = 0;
   if (smem > configured) {
-    cudaError_t e = cudaFuncSetAttribute(gemm_tcgen05_kernel<BM, GATED>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+    cudaError_t e = cudaFuncSetAttribute(gemm_tcgen05_kernel<BM, GATED, GROUPED>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
     if (e != cudaSuccess) return (int)e;
     configured = smem;
   }
   dim3 grid(tiles, args.splits, m_tiles);
-  return launch_dependent_cluster(gemm_tcgen05_kernel<BM, GATED>, grid, dim3(GEMM_THREADS), smem, s,
-                                  dim3(1, args.splits, 1), map_w, map_x, args);
+  return launch_dependent_cluster(gemm_tcgen05_kernel<BM, GATED, GROUPED>, grid, dim3(GEMM_THREADS), smem, s,
+                                  dim3(1, args.splits, 1), map_w, map_x, args, group);
 }
 
 extern "C" {
@@ -364,6 +423,44 @@ static int gemm_entry(const void* x, const void* w, void* out, int rows, int n_o
   }
   // the gated epilogue is a template instance of its own: the plain product then needs fewer
   // registers, and this kernel is measurably faster the fewer it holds
+  if (gated) { BY_TILE(true) }
+  BY_TILE(false)
+#undef BY_TILE
+}
+
+// The same over experts: x [max_tiles * bm, k_dim] in the experts' order (moe.cu's align and gather), w [experts, n_out (2 * n_out
+// with up 1), k_dim]; up 1: out [max_tiles * bm, n_out] is the gated activation (limit > 0: the clamped one), up 2: the squared relu, up
+// 0: out [pairs, n_out], a row's product where its pair belongs.  n_out a multiple of 64 with up 1.
+int sb_gemm_tcgen05_grouped(const void* x, const void* w, void* out, int n_out, int k_dim, int experts, int bm, int splits, int stages,
+                            int up, float limit, const int* tile_expert, const int* n_tiles, int max_tiles, const int* sorted,
+                            const float* in_scale, int* status, cudaStream_t s) {
+  if (max_tiles == 0 || n_out == 0) return 0;
+  if (k_dim % 8 || k_dim <= 0 || splits < 1 || splits > GEMM_MAX_SPLITS || stages < 2 || stages > GEMM_MAX_STAGES) return -2;
+  if ((((uintptr_t)x | (uintptr_t)w) & 15) || up < 0 || up > 2 || (up == 1 && n_out % 64) || max_tiles > 65535) return -2;
+  if ((long long)experts * n_out * 2 > 0x7fffffffll || (long long)max_tiles * bm > 0x7fffffffll) return -2;
+  const bool gated = up == 1;
+  CUtensorMap map_w, map_x;
+  int rc = sb_make_map(&map_w, w, (long long)experts * n_out * (gated ? 2 : 1), k_dim, 64);
+  if (rc) return rc;
+  rc = sb_make_map(&map_x, x, (long long)max_tiles * bm, k_dim, bm);
+  if (rc) return rc;
+  GemmArgs args;
+  args.out = out; args.status = status;
+  args.rows = max_tiles * bm; args.n_out = n_out; args.k_dim = k_dim;
+  args.splits = splits; args.stages = stages; args.gated = gated; args.out_float = 0;
+  args.wait_limit_ns = WAIT_LIMIT_NS; args.withhold_stage = -1;
+  args.limit = limit;
+  const GroupArgs group{tile_expert, n_tiles, sorted, in_scale, up};
+  const int tiles = gated ? n_out / 64 : (n_out + TILE_N - 1) / TILE_N;
+#define BY_TILE(G)                                                                       \
+  switch (bm) {                                                                          \
+    case 16: return launch<16, G, true>(map_w, map_x, args, tiles, max_tiles, s, group);   \
+    case 32: return launch<32, G, true>(map_w, map_x, args, tiles, max_tiles, s, group);   \
+    case 64: return launch<64, G, true>(map_w, map_x, args, tiles, max_tiles, s, group);   \
+    case 128: return launch<128, G, true>(map_w, map_x, args, tiles, max_tiles, s, group); \
+    case 256: return launch<256, G, true>(map_w, map_x, args, tiles, max_tiles, s, group); \
+    default: return -2;                                                                  \
+  }
   if (gated) { BY_TILE(true) }
   BY_TILE(false)
 #undef BY_TILE

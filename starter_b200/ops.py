@@ -204,6 +204,8 @@ def rmsnorm(x, gain, eps, delta=None, rows=None, out=None):
 ACTIVATIONS = {"silu": 1, "gelu_tanh": 2}
 #: the code of the clamped gate ``min(g, L) sigmoid(1.702 min(g, L)) (clamp(u, -L, L) + 1)``, which takes its limit beside it
 GATE_CLAMPED = 3
+#: the code of an expert's plain gate ``silu(g) u``, whose first factor is not rounded by itself
+GATE_EXPERT = 4
 
 
 def gate_code(gated) -> int:
@@ -1856,6 +1858,35 @@ def moe_route_all(h, router, correction, top, groups=1, keep=1, weight_scale=1.0
     return (ids, weights, gate) if shared_gate else (ids, weights)
 
 
+def moe_group_rows(n_pairs: int, experts: int, weigh_input: bool) -> int:
+    """The rows of a tile of the experts' tcgen05 products in a step of ``n_pairs`` (row, expert) pairs: 16, 32 or 64 rows of an
+    expert as the columns of the few-row product (csrc/gemm_tcgen05.cu), 256 as the rows of the prompt product
+    (csrc/gemm_prompt_tcgen05.cu), 0: neither (the kernel for single tokens).  A layer of 16 experts of 2 x 2,048 x 2,048, four a
+    token (us; tokens: tiles of 8 / 16 / 32 / 64 / 256, and of 64 and 128 on ``mma.sync``): 8: 86 / 82; 24: 97 / 88; 32: - / 88, 172;
+    64: - / 93 / 92, 175; 100: - / 107 / 94 / 101, 176; 200: - / - / 121 / 106 / 117, 184; 300: - / - / - / 138 / 121, 306; 700: - / - / - /
+    173 / 129, 448; 1,000: - / - / - / 216 / 147, 542.  The small ones read an expert's weights once and are bound by that; where more
+    rows take several tiles, the weights come from L2 again and that is the bound, three times less of it with tiles of 256 by 256.
+    Smaller experts of few rows are faster on the kernel for single tokens, which needs no gathered rows (8 experts of 2 x 1,344 x
+    1,280, three rows each: 28.9 against 30.9; 32 of 1,280 x 1,536, two rows: 63.7 / 60.8): it serves up to four rows.
+    A weight in front of an expert multiplies the products in float; the prompt product would round the rows, so it waits for 256."""
+    rows = n_pairs / experts
+    if rows <= 4:
+        return 0
+    if rows >= (256 if weigh_input else 64):
+        return 256
+    return 16 if rows <= 13 else 32 if rows <= 28 else 64 if rows <= 64 else 128
+
+
+@functools.lru_cache(maxsize=4096)
+def _moe_group_plan(bm: int, n_out: int, k_dim: int, gated: bool, tiles: int):
+    """``(splits, stages)`` of the grouped product of few rows an expert: three blocks to an SM (16 experts of 2,048, 200 tokens in tiles of
+    64: 109 and 106 us with rings of three and four stages, 131 with one block to an SM), and the k range cut where the experts' weight
+    tiles are fewer than SMs."""
+    units = tiles * (n_out // 64 if gated else -(-n_out // 128))
+    splits = 1 if units >= SM_COUNT else 2 if 2 * units >= SM_COUNT else 4
+    return whole_splits(-(-k_dim // 64), splits), {16: 4, 32: 4, 64: 3, 128: 3}[bm]
+
+
 def moe_experts(h, ids, weights, gate_up, down, limit=0.0, expert="gated_clamped", tile_rows=None, status=None,
                 identity=False, shared=None, shared_gate=None, weigh_input=False):
     """The chosen experts of every row and their weighted sum: ``gate_up`` ``[E, 2 * F, W]`` (an expert's
@@ -1864,7 +1895,8 @@ def moe_experts(h, ids, weights, gate_up, down, limit=0.0, expert="gated_clamped
     ``"relu2"`` the experts have no gate: ``gate_up`` is ``[E, F, W]`` and an expert is
     ``down(relu(up(h))^2)``.  Returns ``[T, W]``.  ``tile_rows`` names the tile kind (32: plain; 4 or 8: the few-row kernel;
     64 and 128: ``mma.sync`` tiles; 256: the grouped tcgen05 product over rows gathered in the experts' order) instead of
-    the one the step's shape chooses: 8 up to six rows an expert on average, 128 from 128, 256 from 256.  ``status``: the
+    the one the step's shape chooses (``moe_group_rows``; the ``mma.sync`` tiles where a gated expert's inner size is no multiple of 64: 8
+    up to six rows an expert on average, 128 from 128).  ``status``: the
     device word a tcgen05 wait that ran out is noted in.
 
     ``expert`` ``"gated_silu"``: ``down(silu(gate(h)) * up(h))``, no clamps.  ``identity``: an id from ``E`` on names
@@ -1907,6 +1939,11 @@ def moe_experts(h, ids, weights, gate_up, down, limit=0.0, expert="gated_clamped
         if tile_rows not in (4, 8, 32, 64, 128, 256) or (tile_rows != 32 and lib.sb_moe_tile_rows(_code(h.dtype), width, inner) != 64):
             raise KernelError(f"no expert tiles of {tile_rows} rows for {h.dtype}, width {width}, inner size {inner}")
         bm = 8 if tile_rows == 4 else int(tile_rows)
+    few = False
+    if tile_rows is None and lib.sb_moe_tile_rows(_code(h.dtype), width, inner) == 64:
+        group = moe_group_rows(n_pairs, experts, weigh_input)
+        if group and not (up_mode == 1 and inner % 64 and group < 256) and not (gate_up.data_ptr() | down.data_ptr()) % 16:
+            bm, few = group, group < 256
     max_tiles = -(-n_pairs // bm) + min(experts, n_pairs)
     capacity = max_tiles * bm
     meta = _empty(h, (capacity + max_tiles + 1,), torch.int32)
@@ -1916,6 +1953,22 @@ def moe_experts(h, ids, weights, gate_up, down, limit=0.0, expert="gated_clamped
     _check(rc, "moe_align")
     act = _empty(h, (capacity, inner))
     per_pair = _empty(h, (n_pairs, width))
+    if few:
+        grouped = _lib("gemm_tcgen05").sb_gemm_tcgen05_grouped
+        gathered = _empty(h, (capacity, width))
+        rc = lib.sb_moe_gather(h, sorted_pairs, n_tiles, bm, top, gathered, capacity, width, None, _stream())
+        _check(rc, "moe_gather")
+        for x, w, out, n_out, k_dim, up, scale in ((gathered, gate_up, act, inner, width, up_mode, in_scale),
+                                                   (act, down, per_pair, width, inner, 0, None)):
+            splits, stages = _moe_group_plan(bm, n_out, k_dim, up == 1, min(experts, n_pairs))
+            rc = grouped(x, w, out, n_out, k_dim, experts, bm, splits, stages, up, limit, tile_expert, n_tiles, max_tiles, sorted_pairs,
+                         scale, status, _stream())
+            _refuse_maps(rc, "grouped")
+            _check(rc, "moe_up / moe_down (grouped tcgen05, few rows)")
+        out = _empty(h, h.shape)
+        rc = lib.sb_moe_combine(_code(h.dtype), per_pair, out_scale, out, n_tokens, width, top, *extras, _stream())
+        _check(rc, "moe_combine")
+        return out
     if bm == 256:
         grouped = _lib("gemm_prompt_tcgen05").sb_gemm_prompt_grouped
         gathered = _empty(h, (capacity, width))
@@ -1924,7 +1977,7 @@ def moe_experts(h, ids, weights, gate_up, down, limit=0.0, expert="gated_clamped
         _check(rc, "moe_gather")
         rc = grouped(gathered, gate_up, act, capacity, inner, width, experts, tile_expert,
                      n_tiles, max_tiles, None,
-                     (GATE_CLAMPED if limit > 0.0 else ACTIVATIONS["silu"]) if up_mode == 1 else 0, 1 if up_mode == 2 else 0,
+                     (GATE_CLAMPED if limit > 0.0 else GATE_EXPERT) if up_mode == 1 else 0, 1 if up_mode == 2 else 0,
                      limit, status, _stream())
         _check(rc, "moe_up (grouped tcgen05)")
         rc = grouped(act, down, per_pair, capacity, width, inner, experts, tile_expert,

@@ -1,0 +1,91 @@
+"""The experts' grouped tcgen05 products of few rows an expert: every tile height, at experts with no row, one row, whole tiles
+and a row more, widths that leave part of a weight tile and of a k-block, against the plain experts in float64."""
+
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+BF, F = torch.bfloat16, torch.float64
+
+
+def plain(h, ids, weights, gate_up, down, kind, limit, inner, weigh_input):
+    out = torch.zeros(h.shape[0], down.shape[1], dtype=F, device="cuda")
+    for e in range(gate_up.shape[0]):
+        row, place = torch.nonzero(ids == e, as_tuple=True)
+        if not row.numel():
+            continue
+        w, by = weights[row, place].to(F)[:, None], 1.0
+        if weigh_input:
+            by, w = w, 1.0
+        p = (h[row].to(F) @ gate_up[e].to(F).T) * by
+        p = p.to(BF).to(F)                                   # the products are rounded in front of the activation
+        if kind == "relu2":
+            a = torch.relu(p) ** 2
+        else:
+            g, u = p[:, :inner], p[:, inner:]
+            a = g * torch.sigmoid(g) * u if kind == "gated_silu" else (
+                g.clamp(max=limit) * torch.sigmoid(1.702 * g.clamp(max=limit)) * (u.clamp(-limit, limit) + 1.0))
+        out.index_add_(0, row, w * (a.to(BF).to(F) @ down[e].to(F).T).to(BF).to(F))
+    return out
+
+
+@pytest.mark.parametrize("rows", [16, 32, 64, 128, 256])
+@pytest.mark.parametrize("kind,experts,width,inner,weigh", [
+    ("gated_silu", 6, 144, 192, False), ("gated_clamped", 5, 256, 64, False), ("relu2", 7, 208, 80, False), ("gated_silu", 6, 1040, 128, True),
+    ("relu2", 40, 64, 272, True)])
+def test_experts_by_tile_height(rows, kind, experts, width, inner, weigh, monkeypatch):
+    from starter_b200 import ops
+
+    if weigh and rows == 256:
+        pytest.skip("weights in front of the experts do not go through the prompt product below 256 rows an expert")
+    gen = torch.Generator().manual_seed(rows + experts)
+    # rows of the experts in turn: none, one, a tile less one, a tile, a tile and one; then whatever is left
+    counts = ([0, 1, rows - 1, rows, rows + 1] + [3] * experts)[:experts]
+    ids = torch.tensor([e for e, n in enumerate(counts) for _ in range(n)], dtype=torch.int32)
+    ids = ids[torch.randperm(ids.numel(), generator=gen)][:, None].cuda()
+    tokens = ids.shape[0]
+    gated = kind != "relu2"
+    h = torch.randn(tokens, width, generator=gen).to(BF).cuda()
+    gate_up = (torch.randn(experts, (2 if gated else 1) * inner, width, generator=gen) * 2.0 * width ** -0.5).to(BF).cuda()
+    down = (torch.randn(experts, width, inner, generator=gen) * inner ** -0.5).to(BF).cuda()
+    weights = (torch.rand(tokens, 1, generator=gen) + 0.5).cuda()
+    status = torch.zeros(1, dtype=torch.int32, device="cuda")
+    limit = 1.25 if kind == "gated_clamped" else 0.0
+    monkeypatch.setattr(ops, "moe_group_rows", lambda *a: rows)
+    got = ops.moe_experts(h, ids, weights, gate_up, down, limit, kind, status=status, weigh_input=weigh).double()
+    want = plain(h, ids, weights, gate_up, down, kind, limit, inner, weigh)
+    # a product that falls on the other side of a rounding moves by 2^-8 of itself: a rounding of each product, of the
+    # activation and of the result
+    scale = float(want.abs().max())
+    assert int(status.item()) == 0
+    assert float((got - want).abs().max()) <= 2.0 ** -6 * scale and float((got - want).norm()) <= 2.0 ** -8 * float(want.norm())
+
+
+@pytest.mark.parametrize("splits", [1, 2, 4])
+def test_k_range_in_parts(splits, monkeypatch):
+    from starter_b200 import ops
+
+    gen = torch.Generator().manual_seed(splits)
+    experts, width, inner, tokens = 3, 520, 128, 70
+    ids = torch.randint(0, experts, (tokens, 1), generator=gen).to(torch.int32).cuda()
+    h = torch.randn(tokens, width, generator=gen).to(BF).cuda()
+    gate_up = (torch.randn(experts, 2 * inner, width, generator=gen) * 2.0 * width ** -0.5).to(BF).cuda()
+    down = (torch.randn(experts, width, inner, generator=gen) * inner ** -0.5).to(BF).cuda()
+    weights = torch.ones(tokens, 1).cuda()
+    monkeypatch.setattr(ops, "moe_group_rows", lambda *a: 32)
+    monkeypatch.setattr(ops, "_moe_group_plan", lambda bm, n_out, k, gated, tiles: (ops.whole_splits(-(-k // 64), splits), 4))
+    got = ops.moe_experts(h, ids, weights, gate_up, down, expert="gated_silu").double()
+    want = plain(h, ids, weights, gate_up, down, "gated_silu", 0.0, inner, False)
+    assert float((got - want).norm()) <= 2.0 ** -8 * float(want.norm())
+
+
+def test_tile_heights_of_a_step():
+    from starter_b200 import ops
+
+    for pairs, experts, weigh, rows in ((4, 16, False, 0), (64, 16, False, 0), (65, 16, False, 16), (208, 16, False, 16), (209, 16, False, 32),
+                                        (448, 16, False, 32), (449, 16, False, 64), (1023, 16, False, 64), (1024, 16, False, 256),
+                                        (1024, 16, True, 64), (1025, 16, True, 128), (4095, 16, True, 128), (4096, 16, True, 256)):
+        assert ops.moe_group_rows(pairs, experts, weigh) == rows
+        if 0 < rows < 256:
+            splits, stages = ops._moe_group_plan(rows, 2048, 2048, True, min(experts, pairs))
+            assert 1 <= splits <= 8 and 2 <= stages <= 8 and stages * (16384 + 128 * rows) >= 512 * rows
