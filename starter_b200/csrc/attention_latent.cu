@@ -30,7 +30,8 @@ __global__ void latent_prepare_kernel(const T* __restrict__ proj, int proj_width
                                       T* __restrict__ cq, int q_rank, int kv_col, int rank, int rot, int rot_dims,
                                       int write, int split) {
   __shared__ float scratch[33];
-  pdl_wait();      // no early launch_dependents: the successor starts when this kernel's blocks have exited
+  pdl_trigger();
+  pdl_wait();
   SB_BEHIND_WAIT(proj);
   SB_BEHIND_WAIT(tok_pos);
   SB_BEHIND_WAIT(tok_slot);
@@ -85,7 +86,8 @@ latent_prepare_vec_kernel(const bf16* __restrict__ proj, int proj_width, const f
                           int rot_dims, int write, int split) {
   __shared__ float2 sums[8];
   const int row = blockIdx.x, tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-  pdl_wait();      // no early launch_dependents: the successor starts when this kernel's blocks have exited
+  pdl_trigger();
+  pdl_wait();
   SB_BEHIND_WAIT(proj);
   SB_BEHIND_WAIT(tok_pos);
   SB_BEHIND_WAIT(tok_slot);
@@ -164,7 +166,8 @@ __global__ void latent_rotate_q_kernel(const T* q, T* qa, const float* __restric
                                        const float* __restrict__ sin_t, int table_width,
                                        const int* __restrict__ tok_pos, int heads, int dim, int rot, int rot_dims,
                                        int rank, int split) {
-  pdl_wait();      // no early launch_dependents: the successor starts when this kernel's blocks have exited
+  pdl_trigger_small();
+  pdl_wait();
   SB_BEHIND_WAIT(q);
   SB_BEHIND_WAIT(tok_pos);
   const int row = blockIdx.x;
@@ -194,7 +197,8 @@ __global__ void latent_attention_kernel(const T* __restrict__ qa, T* __restrict_
                                         const int* __restrict__ tok_slot, const int* __restrict__ tok_pos,
                                         int n_tokens, int heads, int rank, int rot, float scale, int window,
                                         const float* __restrict__ sink) {
-  pdl_wait();      // no early launch_dependents: the successor starts when this kernel's blocks have exited
+  pdl_trigger();
+  pdl_wait();
   SB_BEHIND_WAIT(qa);
   SB_BEHIND_WAIT(store);
   SB_BEHIND_WAIT(tok_slot);
@@ -638,7 +642,8 @@ __global__ void __launch_bounds__(128)
 latent_merge_kernel(const float* __restrict__ part_acc, const float* __restrict__ part_ml,
                     bf16* __restrict__ out, int n_rows, int rank, int n_splits,
                     const float* __restrict__ sink, int heads) {
-  pdl_wait();      // no early launch_dependents: the successor starts when this kernel's blocks have exited
+  pdl_trigger();
+  pdl_wait();
   SB_BEHIND_WAIT(part_acc);
   SB_BEHIND_WAIT(part_ml);
   const int row = blockIdx.x, lane = threadIdx.x & 31, c = threadIdx.x * 4;

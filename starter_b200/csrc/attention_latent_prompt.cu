@@ -55,6 +55,7 @@ __global__ void __launch_bounds__(256)
 latent_gather_kernel(const bf16* __restrict__ store, const int* __restrict__ block_table, int table_stride,
                      const int* __restrict__ seq_slot, const int* __restrict__ seq_q_len, const int* __restrict__ seq_kv_len,
                      bf16* __restrict__ c, bf16* __restrict__ shared, int rank, int rot, int window) {
+  pdl_trigger();
   pdl_wait();
   SB_BEHIND_WAIT(store); SB_BEHIND_WAIT(block_table); SB_BEHIND_WAIT(seq_slot); SB_BEHIND_WAIT(seq_q_len); SB_BEHIND_WAIT(seq_kv_len);
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, seq = blockIdx.y;

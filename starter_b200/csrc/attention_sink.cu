@@ -31,7 +31,8 @@ __global__ void sink_prepare_kernel(const T* __restrict__ proj, int proj_width, 
                                     int table_stride, T* __restrict__ k_store, T* __restrict__ v_store,
                                     float* __restrict__ gate, int heads, int kv_heads, int dim, int vdim, int write,
                                     int vec) {
-  pdl_wait();      // no early launch_dependents: the successor starts when this kernel's blocks have exited
+  pdl_trigger_small();
+  pdl_wait();
   SB_BEHIND_WAIT(proj);
   SB_BEHIND_WAIT(tok_pos);
   SB_BEHIND_WAIT(tok_slot);
@@ -88,7 +89,8 @@ __global__ void sink_prepare_rot_kernel(T* __restrict__ proj, int proj_width, co
                                         int table_stride, T* __restrict__ k_store, T* __restrict__ v_store,
                                         const float* __restrict__ cos_t, const float* __restrict__ sin_t, int rot,
                                         int heads, int kv_heads, int dim, int vdim, int v_from_k, int write) {
-  pdl_wait();      // no early launch_dependents: the successor starts when this kernel's blocks have exited
+  pdl_trigger_small();
+  pdl_wait();
   SB_BEHIND_WAIT(proj);
   SB_BEHIND_WAIT(tok_pos);
   SB_BEHIND_WAIT(tok_slot);
@@ -174,7 +176,8 @@ __global__ void sink_prepare_norm_kernel(T* __restrict__ proj, int proj_width, c
                                          const float* __restrict__ q_gain, const float* __restrict__ k_gain, float eps,
                                          int unit_v, int heads, int kv_heads, int dim, int vdim, int write) {
   __shared__ float2 shares[32];
-  pdl_wait();      // no early launch_dependents: the successor starts when this kernel's blocks have exited
+  pdl_trigger_small();
+  pdl_wait();
   SB_BEHIND_WAIT(proj);
   SB_BEHIND_WAIT(tok_pos);
   SB_BEHIND_WAIT(tok_slot);
@@ -336,7 +339,8 @@ __global__ void sink_attention_kernel(const T* __restrict__ q, int q_stride, T* 
                                       const float* __restrict__ sink, const float* __restrict__ gate, int n_tokens,
                                       int heads, int kv_heads, int dim, int vdim, float scale, int chunk, int window,
                                       int keep, float cap) {
-  pdl_wait();      // no early launch_dependents: the successor starts when this kernel's blocks have exited
+  pdl_trigger();
+  pdl_wait();
   SB_BEHIND_WAIT(q);
   SB_BEHIND_WAIT(k_store);
   SB_BEHIND_WAIT(v_store);

@@ -97,7 +97,7 @@ sink_attention_tc_kernel(const bf16* __restrict__ q, int q_stride, bf16* __restr
   float* pen_tab = reinterpret_cast<float*>(v_tiles + 2 * V_BYTES);   // [group][128], entry tok + 63 - key of the page
   float* pen_coef = pen_tab + (heads / kv_heads) * 128;               // [group][2]: r1 and r2 of the block's heads
 
-  // (no early launch_dependents: the successor starts when this kernel's blocks have exited)
+  pdl_trigger();
   pdl_wait();
   SB_BEHIND_WAIT(q);
   SB_BEHIND_WAIT(k_store);
@@ -444,7 +444,8 @@ sink_attention_tc_kernel(const bf16* __restrict__ q, int q_stride, bf16* __restr
 __global__ void sink_merge_kernel(const float* __restrict__ part_acc, const float* __restrict__ part_ml,
                                   const float* __restrict__ gate, bf16* __restrict__ out, int n_rows, int vdim,
                                   int n_splits) {
-  pdl_wait();      // no early launch_dependents: the successor starts when this kernel's blocks have exited
+  pdl_trigger();
+  pdl_wait();
   SB_BEHIND_WAIT(part_acc);
   SB_BEHIND_WAIT(part_ml);
   SB_BEHIND_WAIT(gate);

@@ -127,6 +127,12 @@ __device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;"
 // kernel reads with ordinary loads (copies issued by inline asm keep their place by themselves).
 #define SB_BEHIND_WAIT(p) asm volatile("" : "+l"(p) : : "memory")
 __device__ __forceinline__ void pdl_trigger() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+// For a kernel in front of one whose blocks are few and long (a recurrence, an attention over many keys): early only from a grid
+// on a quarter of the SMs.  Blocks that are placed while a larger grid still fills the SMs land two and three to an SM beside idle ones,
+// and stay there: a recurrence of 229 tokens took 76 us a layer in place of 37, one of 75 tokens behind a grid of 80 blocks 53 / 35.
+__device__ __forceinline__ void pdl_trigger_small() {
+  if (gridDim.x * gridDim.y * gridDim.z <= 37) pdl_trigger();
+}
 
 // The same, as thread-block clusters of `cluster` CTAs (every grid dimension a multiple of it).
 template <typename... Params, typename... Args>

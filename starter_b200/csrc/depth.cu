@@ -29,7 +29,8 @@ __global__ void depth_step_kernel(const float* __restrict__ base, const T* __res
                                   int norm_kind) {
   extern __shared__ float row[];
   __shared__ float scratch[33];
-  pdl_wait();      // no early launch_dependents: the successor starts when this kernel's blocks have exited
+  pdl_trigger();
+  pdl_wait();
   SB_BEHIND_WAIT(base);
   SB_BEHIND_WAIT(y);
   SB_BEHIND_WAIT(history);
@@ -72,7 +73,8 @@ __global__ void depth_step_kernel(const float* __restrict__ base, const T* __res
 
 // logits <- cap * tanh(logits / cap), in place, float.
 __global__ void softcap_kernel(float* __restrict__ x, size_t total, float cap) {
-  pdl_wait();      // no early launch_dependents: the successor starts when this kernel's blocks have exited
+  pdl_trigger();
+  pdl_wait();
   SB_BEHIND_WAIT(x);
   size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
   const size_t stride = (size_t)gridDim.x * blockDim.x;

@@ -372,7 +372,8 @@ __global__ void gated_clamped_kernel(const T* __restrict__ gu, T* __restrict__ a
 // a[t, c] *= sigmoid(g[t, c]), g the columns of a wider row (V = 8 / 4: 16-byte accesses; V = 1: any address).
 template <typename T, int V>
 __global__ void sigmoid_gate_kernel(T* __restrict__ a, const T* __restrict__ g, int ldg, int width, size_t pieces) {
-  pdl_wait();      // no early launch_dependents: the successor starts when this kernel's blocks have exited
+  pdl_trigger();
+  pdl_wait();
   SB_BEHIND_WAIT(a);
   SB_BEHIND_WAIT(g);
   const size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x;

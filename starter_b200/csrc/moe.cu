@@ -147,7 +147,8 @@ __global__ void __launch_bounds__(512) moe_route_kernel(const T* __restrict__ h,
                                  int scoring, float weight_scale) {
   extern __shared__ __align__(16) unsigned char route_smem[];
   float* route_z = reinterpret_cast<float*>(route_smem + (TOK > 1 ? MOE_STAGE_BYTES : 0));
-  pdl_wait();      // no early launch_dependents: the successor starts when this kernel's blocks have exited
+  pdl_trigger();
+  pdl_wait();
   SB_BEHIND_WAIT(h);
   const int row0 = blockIdx.x * TOK;
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, warps = blockDim.x >> 5;
@@ -206,7 +207,8 @@ __global__ void __launch_bounds__(512) moe_route_all_kernel(const T* __restrict_
                                      int top, int groups, int keep, float weight_scale) {
   extern __shared__ __align__(16) unsigned char route_smem[];
   float* route_z = reinterpret_cast<float*>(route_smem + (TOK > 1 ? MOE_STAGE_BYTES : 0));
-  pdl_wait();      // no early launch_dependents: the successor starts when this kernel's blocks have exited
+  pdl_trigger();
+  pdl_wait();
   SB_BEHIND_WAIT(h);
   const int row0 = blockIdx.x * TOK, per_token = 3 * outputs + 1 + groups;
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, warps = blockDim.x >> 5;
@@ -308,7 +310,8 @@ __global__ void __launch_bounds__(1024)
 moe_align_kernel(const int* __restrict__ ids, int n_pairs, int experts, int* __restrict__ sorted, int capacity,
                  int* __restrict__ tile_expert, int* __restrict__ n_tiles, int bm) {
   __shared__ int count[MOE_MAX_EXPERTS], offset[MOE_MAX_EXPERTS];
-  pdl_wait();      // no early launch_dependents: the successor starts when this kernel's blocks have exited
+  pdl_trigger();
+  pdl_wait();
   SB_BEHIND_WAIT(ids);
   const int tid = threadIdx.x, lane = tid & 31, threads = blockDim.x;
   const int bits = 32 - __clz(experts);             // (numbers up to `experts`, which stands for all that have no tile)
@@ -784,7 +787,8 @@ moe_few_kernel(const bf16* __restrict__ x, const bf16* __restrict__ w, bf16* __r
   constexpr bool UP = MODE != 0;
   constexpr int NW = MODE == 1 ? 2 : 1, MOE_FEW_FLY = 8 / NW;
   __shared__ float part[4][NW * 4][32];
-  pdl_wait();      // no early launch_dependents: the successor starts when this kernel's blocks have exited
+  pdl_trigger();
+  pdl_wait();
   SB_BEHIND_WAIT(x);
   SB_BEHIND_WAIT(sorted);
   SB_BEHIND_WAIT(tile_expert);
@@ -865,7 +869,8 @@ moe_few_kernel(const bf16* __restrict__ x, const bf16* __restrict__ w, bf16* __r
 __global__ void __launch_bounds__(256) moe_gather_kernel(const bf16* __restrict__ h, const int* __restrict__ sorted,
                                   const int* __restrict__ n_tiles, int tile_rows, int top, bf16* __restrict__ out,
                                   int width, const float* __restrict__ in_scale) {
-  pdl_wait();      // no early launch_dependents: the successor starts when this kernel's blocks have exited
+  pdl_trigger();
+  pdl_wait();
   SB_BEHIND_WAIT(h);
   SB_BEHIND_WAIT(sorted);
   SB_BEHIND_WAIT(n_tiles);
@@ -901,7 +906,8 @@ template <typename T>
 __global__ void moe_combine_kernel(const T* __restrict__ down, const float* __restrict__ weights, T* __restrict__ out,
                                    int width, int top, const int* __restrict__ ids, int experts, const T* __restrict__ h,
                                    const T* __restrict__ shared, const float* __restrict__ shared_gate) {
-  pdl_wait();      // no early launch_dependents: the successor starts when this kernel's blocks have exited
+  pdl_trigger();
+  pdl_wait();
   SB_BEHIND_WAIT(down);
   SB_BEHIND_WAIT(weights);
   SB_BEHIND_WAIT(ids);
@@ -929,7 +935,8 @@ __global__ void __launch_bounds__(128)
 moe_combine_vec_kernel(const bf16* __restrict__ down, const float* __restrict__ weights, bf16* __restrict__ out, int width, int top,
                        const int* __restrict__ ids, int experts, const bf16* __restrict__ h, const bf16* __restrict__ shared,
                        const float* __restrict__ shared_gate) {
-  pdl_wait();      // no early launch_dependents: the successor starts when this kernel's blocks have exited
+  pdl_trigger();
+  pdl_wait();
   SB_BEHIND_WAIT(down);
   SB_BEHIND_WAIT(weights);
   SB_BEHIND_WAIT(ids);

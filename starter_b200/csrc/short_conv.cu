@@ -32,7 +32,8 @@ short_conv_kernel(const T* __restrict__ x, int ldx, const float* __restrict__ ta
                   const float* __restrict__ in_bias, T* __restrict__ y, int ldy, float* __restrict__ state,
                   long long slot_stride, const int* __restrict__ seq_slot, const int* __restrict__ seq_q_start,
                   const int* __restrict__ seq_q_len, int channels, int K, int act, int chunks) {
-  pdl_wait();      // no early launch_dependents: the successor starts when this kernel's blocks have exited
+  pdl_trigger_small();
+  pdl_wait();
   SB_BEHIND_WAIT(x);
   SB_BEHIND_WAIT(state);
   SB_BEHIND_WAIT(seq_slot);
@@ -131,7 +132,8 @@ short_conv_vec_kernel(const bf16* __restrict__ x, int ldx, const float* __restri
       for (int j = 0; j < K; ++j) tap[j][e] = taps[(size_t)(c + e) * K + (K - 1 - j)];
     }
   }
-  pdl_wait();      // no early launch_dependents: the successor starts when this kernel's blocks have exited
+  pdl_trigger_small();
+  pdl_wait();
   SB_BEHIND_WAIT(x);
   SB_BEHIND_WAIT(state);
   SB_BEHIND_WAIT(seq_slot);
@@ -236,7 +238,8 @@ glru_scan_kernel(const T* __restrict__ u, int ldu, const float* __restrict__ gat
                  const int* __restrict__ seq_slot, const int* __restrict__ seq_q_start,
                  const int* __restrict__ seq_q_len, int channels) {
   __shared__ float carry_a[32][33], carry_s[32][33];
-  pdl_wait();      // no early launch_dependents: the successor starts when this kernel's blocks have exited
+  pdl_trigger();
+  pdl_wait();
   SB_BEHIND_WAIT(u);
   SB_BEHIND_WAIT(gates);
   SB_BEHIND_WAIT(ybranch);

@@ -89,6 +89,7 @@ state_scan_kernel(const T* __restrict__ q, int ldq, const T* __restrict__ k, int
   constexpr int OS_LD = SCAN_COLS + 32 / P;
   float (*os)[OS_LD] = reinterpret_cast<float (*)[OS_LD]>(scan_smem + 2 * sizeof(Buffer));
   // (launch_dependents comes at this kernel's end, not its start: a long prompt keeps its blocks for a while)
+  pdl_trigger();
   pdl_wait();
   SB_BEHIND_WAIT(q);
   SB_BEHIND_WAIT(k);
@@ -290,7 +291,8 @@ __global__ void __launch_bounds__(128)
 low_rank_decay_kernel(const T* __restrict__ u, int ldu, const float* __restrict__ a2, const float* __restrict__ bias,
                       float* __restrict__ d, int n_tokens, int channels, int rank, float inv_tau) {
   extern __shared__ float us[];                    // [rank][DECAY_TOKENS]
-  pdl_wait();      // no early launch_dependents: the successor starts when this kernel's blocks have exited
+  pdl_trigger_small();
+  pdl_wait();
   SB_BEHIND_WAIT(u);
   const int t0 = blockIdx.x * DECAY_TOKENS, nt = min(DECAY_TOKENS, n_tokens - t0);
   for (int e = threadIdx.x; e < rank * DECAY_TOKENS; e += blockDim.x) {
@@ -328,7 +330,8 @@ __global__ void group_norm_gate_kernel(const float* __restrict__ o, const T* __r
                                        const float* __restrict__ w, int wlen, T* __restrict__ y, int n_tokens,
                                        int parts, int psize, float eps, int order) {
   __shared__ float scratch[33];
-  pdl_wait();      // no early launch_dependents: the successor starts when this kernel's blocks have exited
+  pdl_trigger();
+  pdl_wait();
   SB_BEHIND_WAIT(o);
   SB_BEHIND_WAIT(z);
   const long long item = WIDE ? (long long)blockIdx.x : ((long long)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
@@ -366,7 +369,8 @@ __global__ void __launch_bounds__(256)
 group_norm_gate_vec_kernel(const float* __restrict__ o, const bf16* __restrict__ z, int ldz, const float* __restrict__ w, int wlen,
                            bf16* __restrict__ y, int n_tokens, int parts, int psize, float eps, int order) {
   __shared__ float scratch[33];
-  pdl_wait();      // no early launch_dependents: the successor starts when this kernel's blocks have exited
+  pdl_trigger();
+  pdl_wait();
   SB_BEHIND_WAIT(o);
   SB_BEHIND_WAIT(z);
   const long long item = WARP ? ((long long)blockIdx.x * blockDim.x + threadIdx.x) >> 5 : (long long)blockIdx.x;
@@ -419,7 +423,8 @@ template <typename T>
 __global__ void norm_pair_mean_kernel(const T* __restrict__ a, const T* __restrict__ b, const float* __restrict__ wa,
                                       const float* __restrict__ wb, T* __restrict__ out, int width, float eps) {
   __shared__ float scratch[33];
-  pdl_wait();      // no early launch_dependents: the successor starts when this kernel's blocks have exited
+  pdl_trigger();
+  pdl_wait();
   SB_BEHIND_WAIT(a);
   SB_BEHIND_WAIT(b);
   const T* ar = a + (size_t)blockIdx.x * width;
@@ -442,7 +447,8 @@ __global__ void norm_pair_mean_kernel(const T* __restrict__ a, const T* __restri
 template <typename T, int V>
 __global__ void scaled_sum_kernel(const T* __restrict__ a, const T* __restrict__ b, T* __restrict__ out, float wa,
                                   float wb, size_t pieces) {
-  pdl_wait();      // no early launch_dependents: the successor starts when this kernel's blocks have exited
+  pdl_trigger();
+  pdl_wait();
   SB_BEHIND_WAIT(a);
   SB_BEHIND_WAIT(b);
   const size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x;

@@ -167,7 +167,8 @@ hyper_rms_kernel(float* __restrict__ streams, const T* __restrict__ y, const flo
     outw[i] = y ? out_prev[i] : 0.f;
     inw[i] = in_next ? in_next[i] : 1.f;
   }
-  pdl_wait();      // no early launch_dependents: the successor starts when this kernel's blocks have exited
+  pdl_trigger();
+  pdl_wait();
   SB_BEHIND_WAIT(y);
   SB_BEHIND_WAIT(rows);
   const int out_row = blockIdx.x;
