@@ -726,6 +726,7 @@ int sb_latent_attention_tc(const void* qa, void* out, float* part_acc, float* pa
   else if (nt <= 16) GO(16)
   else GO(32)
 #undef GO
+  if (!out) return 0;
   return launch_dependent(latent_merge_kernel, dim3(n_tokens * heads), dim3(128), 0, s, (const float*)part_acc,
                           (const float*)part_ml, (bf16*)out, n_tokens * heads, rank, n_splits, sink, heads);
 }

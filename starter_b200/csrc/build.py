@@ -56,6 +56,7 @@ SOURCES = (
     "wkv",
     "attention_latent",
     "attention_latent_prompt",
+    "latent_heads",
     "moe",
     "depth",
     "attention_sink",

@@ -1649,12 +1649,13 @@ def latent_tc_takes(dtype, rank: int, rot: int) -> bool:
 
 
 def latent_attention_tc(qa, store, block_table, seq_slot, seq_q_start, seq_q_len, seq_kv_len, tile_seq, tile_first,
-                        heads, rank, rot, scale, window=None, n_splits=1, max_q_len=0, sink=None):
+                        heads, rank, rot, scale, window=None, n_splits=1, max_q_len=0, sink=None, join=True):
     """``latent_attention`` on tensor cores (bfloat16): a block takes the heads of consecutive tokens of a
     sequence (up to 64 query rows), which all score the same cache rows.  The ``seq_*`` arrays describe the
     sequences of the step, ``tile_seq`` / ``tile_first`` list its tiles of 64 tokens.  ``n_splits`` > 1 deals
     the keys of every block out to that many blocks, which a second kernel joins: for steps of few rows.
-    ``max_q_len``: the most tokens a sequence brings, if known (fewer idle blocks are launched)."""
+    ``max_q_len``: the most tokens a sequence brings, if known (fewer idle blocks are launched).  Without ``join`` what comes back is
+    ``(summed, part_acc, part_ml)`` for ``latent_unfold``: the parts as they are, or the sums where there is one part."""
     _need(qa, "qa", torch.bfloat16, 3)
     n_tokens = qa.shape[0]
     if tuple(qa.shape[1:]) != (heads, rank + rot):
@@ -1669,9 +1670,9 @@ def latent_attention_tc(qa, store, block_table, seq_slot, seq_q_start, seq_q_len
     for name, t in (("seq_slot", seq_slot), ("seq_q_start", seq_q_start), ("seq_q_len", seq_q_len),
                     ("seq_kv_len", seq_kv_len), ("tile_seq", tile_seq), ("tile_first", tile_first)):
         _need(t, name, torch.int32, 1)
-    out = _empty(qa, (n_tokens, heads, rank))
-    part_acc = part_ml = None
     n_splits = max(1, int(n_splits))
+    out = _empty(qa, (n_tokens, heads, rank)) if join or n_splits == 1 else None
+    part_acc = part_ml = None
     if n_splits > 1:
         part_acc = _empty(qa, (n_splits, n_tokens * heads, rank), torch.float32)
         part_ml = _empty(qa, (n_splits, n_tokens * heads, 2), torch.float32)
@@ -1680,8 +1681,8 @@ def latent_attention_tc(qa, store, block_table, seq_slot, seq_q_start, seq_q_len
         seq_slot, seq_q_start, seq_q_len, seq_kv_len, tile_seq, tile_first,
         tile_seq.shape[0], n_tokens, heads, rank, rot, scale, int(window or 0), n_splits,
         int(max_q_len), _latent_sink(sink, heads), _stream())
-    _check(rc, "latent_attention_tc", 2 if n_splits > 1 else 1)
-    return out
+    _check(rc, "latent_attention_tc", 2 if n_splits > 1 and join else 1)
+    return out if join else (out, part_acc, part_ml)
 
 
 def latent_splits(rows: int, heads: int, window, kv_hint: int) -> int:
@@ -1692,15 +1693,63 @@ def latent_splits(rows: int, heads: int, window, kv_hint: int) -> int:
     return max(1, min(32, 148 // max(1, blocks), -(-max(keys, 1) // 32)))
 
 
-def latent_attention_step(qa, store, block_table, ctx, heads, rank, rot, scale, window=None, sink=None):
+def latent_attention_step(qa, store, block_table, ctx, heads, rank, rot, scale, window=None, sink=None, join=True):
     """``latent_attention`` for the step ``ctx`` describes, on the kernel that fits its shape: tensor cores
     for bfloat16 at sizes they take, the plain kernel otherwise (float32, other sizes)."""
     if latent_tc_takes(qa.dtype, rank, rot):
         splits = latent_splits(ctx.n_seqs, heads, window, ctx.max_kv_len) if ctx.max_q_len == 1 else 1
         return latent_attention_tc(qa, store, block_table, ctx.seq_slot, ctx.seq_q_start, ctx.seq_q_len,
                                    ctx.seq_kv_len, ctx.tile_seq, ctx.tile_first, heads, rank, rot, scale, window,
-                                   splits, ctx.max_q_len, sink)
-    return latent_attention(qa, store, block_table, ctx.tok_slot, ctx.tok_pos, heads, rank, rot, scale, window, sink)
+                                   splits, ctx.max_q_len, sink, join)
+    out = latent_attention(qa, store, block_table, ctx.tok_slot, ctx.tok_pos, heads, rank, rot, scale, window, sink)
+    return out if join else (out, None, None)
+
+
+#: up to this many tokens a step's latent queries and outputs are formed by the kernels for few rows (csrc/latent_heads.cu), whose
+#: blocks read a head's matrices again for every 16 tokens; beyond, by batched library products
+LATENT_HEADS_TOKENS = 64
+
+
+def latent_heads_take(q, dim, rot, rank, vdim) -> bool:
+    return (q.dtype == torch.bfloat16 and q.shape[0] <= LATENT_HEADS_TOKENS and
+            bool(_lib("latent_heads").sb_latent_heads_take(dim, rot, rank, vdim)))
+
+
+def latent_fold(q, uk, cos_table, sin_table, tok_pos, heads, dim, rot, rot_dims, rank, layout="interleaved"):
+    """``[T, heads, rank + rot]``: the first ``dim`` entries of every head of ``q`` ``[T, heads * (dim + rot)]`` times ``uk[h]`` (the
+    contiguous ``[heads * dim, rank]``), then its last ``rot`` entries turned by the token's position as ``latent_rotate_q`` does."""
+    _need(q, "q", torch.bfloat16, 2)
+    _need(uk, "uk", q.dtype, 2)
+    if q.shape[1] != heads * (dim + rot) or tuple(uk.shape) != (heads * dim, rank):
+        raise KernelError(f"q {tuple(q.shape)} / uk {tuple(uk.shape)} do not fit {heads} heads of {dim} + {rot} over {rank}")
+    _need(tok_pos, "tok_pos", torch.int32, 1)
+    qa = _empty(q, (q.shape[0], heads, rank + rot))
+    rc = _lib("latent_heads").sb_latent_fold(q, uk, qa, cos_table, sin_table, cos_table.shape[1], tok_pos, q.shape[0], heads, dim, rot,
+                                             rot_dims, rank, LATENT_LAYOUTS[layout], _stream())
+    _check(rc, "latent_fold")
+    return qa
+
+
+def latent_unfold(parts, uv, heads, vdim, rank, sink=None, gate=None, gate_col=0):
+    """``[T, heads * vdim]`` from what ``latent_attention_step`` leaves with ``join=False``: every head's summed latents times
+    ``uv[h].T`` (the contiguous ``[heads * vdim, rank]``), then times ``sigmoid`` of the columns from ``gate_col`` on of ``gate``."""
+    summed, part_acc, part_ml = parts
+    _need(uv, "uv", torch.bfloat16, 2)
+    if tuple(uv.shape) != (heads * vdim, rank):
+        raise KernelError(f"uv {tuple(uv.shape)} does not fit {heads} heads of {vdim} over {rank}")
+    n = summed.shape[0] if summed is not None else part_acc.shape[1] // heads
+    ldg = 0
+    if gate is not None:
+        _need(gate, "gate", uv.dtype, 2)
+        if gate.shape[0] != n or gate_col < 0 or gate_col + heads * vdim > gate.shape[1]:
+            raise KernelError(f"{heads * vdim} columns from {gate_col} of {tuple(gate.shape)} do not gate {n} rows")
+        gate, ldg = _at(gate, gate_col), gate.shape[1]
+    out = _empty(uv, (n, heads * vdim))
+    rc = _lib("latent_heads").sb_latent_unfold(summed, part_acc, part_ml, part_acc.shape[0] if part_acc is not None else 1,
+                                               _latent_sink(sink, heads) if part_acc is not None else None, uv, gate, ldg, out, n, heads,
+                                               rank, vdim, _stream())
+    _check(rc, "latent_unfold")
+    return out
 
 
 #: tokens that every sequence of a step must bring for the latent attention to form keys and values (see
