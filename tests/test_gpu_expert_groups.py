@@ -1,5 +1,6 @@
 """The experts' grouped tcgen05 products of few rows an expert: every tile height, at experts with no row, one row, whole tiles
-and a row more, widths that leave part of a weight tile and of a k-block, against the plain experts in float64."""
+and a row more, widths that leave part of a weight tile and of a k-block, against the plain experts in float64; the dealing of
+pairs to tiles."""
 
 import pytest
 import torch
@@ -89,3 +90,28 @@ def test_tile_heights_of_a_step():
         if 0 < rows < 256:
             splits, stages = ops._moe_group_plan(rows, 2048, 2048, True, min(experts, pairs))
             assert 1 <= splits <= 8 and 2 <= stages <= 8 and stages * (16384 + 128 * rows) >= 512 * rows
+
+
+@pytest.mark.parametrize("pairs,experts", [(1, 1), (31, 5), (1024, 16), (1025, 16), (8191, 7), (8192, 1), (8193, 7), (20000, 130)])
+def test_pairs_are_dealt_to_tiles(pairs, experts):
+    """Every pair of an expert once, in that expert's tiles, and -1 behind them, where a thread's pairs are counted and placed in
+    one pass (up to 8 a thread, of 256 threads up to 1,024 pairs and 1,024 beyond) and where they are walked twice."""
+    from starter_b200 import ops
+
+    gen = torch.Generator().manual_seed(pairs)
+    ids = torch.randint(0, experts + 1, (pairs,), generator=gen, dtype=torch.int32)       # (`experts`: an identity expert)
+    bm = 16
+    tiles = -(-pairs // bm) + min(experts, pairs)
+    placed = torch.full((tiles * bm,), -7, dtype=torch.int32, device="cuda")
+    tile_expert = torch.full((tiles,), -7, dtype=torch.int32, device="cuda")
+    used = torch.zeros(1, dtype=torch.int32, device="cuda")
+    ops._check(ops._lib("moe").sb_moe_align(ids.cuda(), pairs, experts, placed, tiles * bm, tile_expert, used, bm, ops._stream()), "moe_align")
+    placed, names, used = placed.cpu().view(tiles, bm), tile_expert.cpu(), int(used)
+    counts = torch.bincount(ids, minlength=experts + 1)[:experts]
+    assert used == int(((counts + bm - 1) // bm).sum())
+    assert names[:used].tolist() == sorted(names[:used].tolist())
+    for expert in range(experts):
+        mine = placed[:used][names[:used] == expert].flatten()
+        n = int(counts[expert])
+        assert sorted(mine[:n].tolist()) == (ids == expert).nonzero().flatten().tolist()
+        assert (mine[n:] == -1).all()
