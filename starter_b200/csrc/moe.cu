@@ -1049,17 +1049,17 @@ extern "C" {
 int sb_moe_tile_rows(int dtype, int width, int inner) {
   return dtype == 1 && width % 16 == 0 && inner % 16 == 0 ? MOE_TC_BM : MOE_BM;
 }
-// The same for a step of `n_pairs` (row, expert) pairs over `experts` experts: when the tensor-core tiles take
-// the operands, 8 up to six rows an expert on average (the few-row kernel), 128 from 128 rows an expert on average (the large tiles pay for their padding from there
-// on) and 256 from 256 (the row tiles of the grouped tcgen05 product, which runs in place of these tiles);
-// else as above.
+// The same for a step of `n_pairs` (row, expert) pairs over `experts` experts, where the caller does not take the grouped tcgen05
+// products (more than four rows an expert on average, moe_group_rows in ops.py; it leaves gated experts of odd inner sizes and
+// misaligned weights here): 8 up to six rows an expert (the few-row kernel), 128 from 128 (the large tiles pay for their padding
+// from there on), 256 from 256 (the grouped prompt product); else as above.
 int sb_moe_tile_rows_for(int dtype, int width, int inner, long long n_pairs, int experts) {
   const int rows = sb_moe_tile_rows(dtype, width, inner);
   if (rows != MOE_TC_BM) return rows;
   // 8: the few-row kernel, up to six rows an expert on average (single tokens; beyond, many experts take two tiles of 8, which
   // read the weights twice)
   if (n_pairs <= 6ll * experts) return MOE_FEW;
-  // 256: the grouped tcgen05 product (its row tiles), from 256 rows an expert on average
+  // 256: the grouped prompt product (its row tiles), from 256 rows an expert on average
   if (n_pairs >= 256ll * experts) return 256;
   return n_pairs >= (long long)MOE_BIG * experts ? MOE_BIG : rows;
 }
