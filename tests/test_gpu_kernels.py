@@ -754,3 +754,24 @@ def test_native_outputs_and_checks():
     with torch.cuda.stream(side):
         assert ops._stream() == side.cuda_stream
     assert ops._stream() == torch.cuda.current_stream().cuda_stream
+
+
+@pytest.mark.parametrize("k", [4, 124, 128, 516, 1020, 1024, 1028, 1030, 2048, 2500, 3077])
+def test_float32_product_of_one_row(k):
+    """One row in float32: a warp's pieces of a weight row, 8 of 128 entries together (4 with a gate), around whole rounds, and
+    entry by entry where k is no multiple of 4."""
+    from starter_b200 import ops
+
+    n = 37
+    x, w = rand(1, k, dtype="float32", seed=71), rand(2 * n, k, dtype="float32", seed=72, scale=0.05)
+    exact = (x.double() @ w.double().t())[0]
+    # a lane adds up to k / 32 products and a piece more, then five sums of lanes, each rounded once
+    bound = 1.01 * (k / 32 + 4 + 5) * 2.0 ** -24 * (x.double().abs() @ w.double().abs().t())[0]
+    got = ops.linear(dev(x), dev(w)).cpu().double()[0]
+    assert ((got - exact).abs() <= bound).all()
+    gate, up = exact[:n], exact[n:]
+    silu = gate * torch.sigmoid(gate)
+    # silu's slope is at most 1.1; the exponential, the quotient and the product round a few times more
+    room = 1.1 * bound[:n] * (up.abs() + bound[n:]) + silu.abs() * bound[n:] + 2.0 ** -20 * (silu * up).abs()
+    got = ops.linear(dev(x), dev(w), gated=True).cpu().double()[0]
+    assert ((got - silu * up).abs() <= room + 1e-30).all()
