@@ -382,7 +382,6 @@ latent_prompt_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_con
   asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
   if constexpr (DC == 2 || VC == 1) {
     if (splits > 1) {
-      __syncwarp();
       cluster_barrier();
       if (threadIdx.x < 2 * TC_BQ) {
         const size_t stride = (size_t)heads * (VC * 64);
@@ -394,7 +393,6 @@ latent_prompt_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_con
               return f / (sum * f + fast_exp2(own - top));
             });
       }
-      __syncwarp();
       cluster_barrier();                            // nobody leaves while others read from it
     }
   }

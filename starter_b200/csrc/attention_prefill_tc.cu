@@ -557,7 +557,6 @@ attention_prefill_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __g
       float2* ml = reinterpret_cast<float2*>(ring);
       __syncthreads();
       if (threadIdx.x < 2 * TC_BQ) ml[threadIdx.x] = row_state;
-      __syncwarp();
       cluster_barrier();
       if (threadIdx.x < 2 * TC_BQ) {
         const size_t row0 = (size_t)seq_q_start[seq] + q_first;
@@ -569,7 +568,6 @@ attention_prefill_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __g
               return inv;
             });
       }
-      __syncwarp();
       cluster_barrier();                            // nobody leaves while others read from it
     }
   }

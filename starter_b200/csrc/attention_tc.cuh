@@ -188,6 +188,7 @@ __device__ __forceinline__ float* part_piece(uint8_t* p_tile, uint8_t* q_tile, i
                         : reinterpret_cast<float*>(q_tile + r * (QW * 4) + (((piece - PC / 4) ^ (r & 7)) << 4));
 }
 __device__ __forceinline__ void cluster_barrier() {
+  __syncwarp();                    // (.aligned: a whole warp at once)
   asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
 }
 __device__ __forceinline__ uint32_t peer_u32(const void* p, int rank) {

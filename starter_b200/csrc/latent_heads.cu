@@ -172,6 +172,7 @@ latent_unfold_kernel(const bf16* __restrict__ summed, const float* __restrict__ 
       to[1] = __floats2bfloat162_rn(a.z, a.w);
     }
     if (shares > 1) {
+      __syncwarp();                                 // (.aligned: a whole warp at once, and the loop above may leave it in two)
       asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
       for (int e = tid; e < here * pieces; e += 256) {
         const int r = e / pieces, piece = e - r * pieces, whose = piece / per;

@@ -190,3 +190,25 @@ def test_native_checks_refuse_what_the_plain_ones_do():
     assert ops._empty(torch.zeros(2, dtype=torch.bfloat16), (0, 5)).dtype == torch.bfloat16
     with pytest.raises((RuntimeError, TypeError)):
         ops._empty(torch.zeros(2), (-3, 5))
+
+
+def test_warps_are_whole_in_front_of_aligned_cluster_barriers():
+    """``barrier.cluster`` with ``.aligned`` wants all threads of a warp at it at once: in every kernel source the statement in front of
+    one makes the warp whole (a loop that lanes leave at different rounds need not)."""
+    import os
+    import re
+
+    from starter_b200.csrc import build
+
+    barriers = 0
+    for name in sorted(os.listdir(build.HERE)):
+        if not name.endswith((".cu", ".cuh")):
+            continue
+        with open(os.path.join(build.HERE, name)) as handle:
+            code = [re.sub(r"\s*//.*", "", line).strip() for line in handle]
+        code = [line for line in code if line]
+        for i, line in enumerate(code):
+            if "barrier.cluster." in line and ".aligned" in line:
+                barriers += 1
+                assert re.search(r"__sync(warp|threads)\(\);$", code[i - 1]), f"{name}: {code[i - 1]!r} in front of {line!r}"
+    assert barriers >= 4
