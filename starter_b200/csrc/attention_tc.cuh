@@ -222,14 +222,15 @@ __device__ __forceinline__ void merge_parts(uint8_t* q_sm, uint8_t* p_sm, float2
 #pragma unroll
     for (int p = 0; p < 8; ++p) {
       part[p] = p < splits ? peer_load2(peer_u32(ml + t * TC_BQ + r, p)) : make_float2(-INFINITY, 0.f);
-      if (part[p].y > 0.f) top = fmaxf(top, part[p].x);
+      if (part[p].y != 0.f) top = fmaxf(top, part[p].x);
     }
     float sum = 0.f, o[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
     const float* a = part_piece<PC, COLS>(p_sm + t * P_BYTES, q_sm + t * Q_BYTES, r, c / 4);
     const float* b = part_piece<PC, COLS>(p_sm + t * P_BYTES, q_sm + t * Q_BYTES, r, c / 4 + 1);
 #pragma unroll
     for (int p = 0; p < 8; ++p) {
-      if (p >= splits || !(part[p].y > 0.f)) continue;       // (a part without keys filed nothing)
+      // (a part without keys filed nothing; one whose sum is no number has a score that is none, which is the row's result)
+      if (p >= splits || part[p].y == 0.f) continue;
       const float w = fast_exp2(part[p].x - top);
       sum = fmaf(w, part[p].y, sum);
       const float4 x = peer_load4(peer_u32(a, p)), y = peer_load4(peer_u32(b, p));

@@ -88,6 +88,56 @@ def test_over_formed_keys(dim, vdim, window, sink, monkeypatch):
         torch.linspace(-1.0, 2.0, heads).cuda() if sink else None), ctx.status)
 
 
+@pytest.mark.parametrize("kind", ["plain", "window", "extras", "capped", "formed", "formed, sink"])
+def test_scores_that_are_no_numbers(kind, monkeypatch):
+    """A row with a score that is NaN or +infinity is no number whichever part its key lies in; every other row is what it was."""
+    from starter_b200 import ops
+
+    heads, dim, rank = 4, 128, 128
+    formed = kind.startswith("formed")
+    gen, table, (keys, values), ctx = step(1, rank + 64, 16, 5) if formed else step(2, dim, dim, 5)
+    q = torch.randn(sum(LENGTHS), heads * (dim + 64 if formed else dim), generator=gen).to(BF).cuda()
+
+    def key(seq, pos):
+        return keys[int(table[seq, pos // 64]), :, pos % 64]
+
+    key(2, 600)[:, -3] = float("nan")                  # (of a formed key's row the shared part, which is in no value)
+    key(0, 10)[:, -5] = float("inf")                   # +infinity for about half of the queries, weight 0 for the others
+    key(1, 12)[:, -1] = float("-inf")
+    q[-200] = float("nan")
+    ints = (table, ctx.seq_slot, ctx.seq_q_start, ctx.seq_q_len, ctx.seq_kv_len, ctx.tile_seq, ctx.tile_first)
+    blocks, sink = (ctx.block_seq, ctx.block_first), torch.linspace(-1.0, 2.0, heads).cuda()
+    ukv = (torch.randn(heads * 2 * dim, rank, generator=gen) * rank ** -0.5).to(BF).cuda()
+
+    def run():
+        if formed:
+            return ops.latent_attention_prompt(q, ukv, keys, table, ctx, heads, dim, dim, rank, 64, (dim + 64) ** -0.5, None,
+                                               sink if "sink" in kind else None)
+        if kind in ("plain", "window"):
+            return ops.attention_prefill(q, keys, values, *ints, heads, 2, dim, dim ** -0.5, 300 if kind == "window" else None,
+                                         status=ctx.status, kernel="tcgen05", max_q_len=ctx.max_q_len, blocks=blocks,
+                                         kv_hint=ctx.max_kv_len)
+        return ops.sink_attention_tcgen05(q, keys, values, *ints, heads, 2, dim, dim ** -0.5, None, sink, None, None, 400, ctx.status,
+                                          blocks, dim, 0, 30.0 if kind == "capped" else None, ctx.max_kv_len)
+
+    got = {}
+    for parts in (1, 2, 4):
+        monkeypatch.setattr(ops, "prompt_splits", lambda *a, **k: parts)
+        got[parts] = run().float()
+    good = got[1].isfinite()
+    # by heads: a score of +infinity is one head's (with a cap it is the cap, a number)
+    by_head = good.view(sum(LENGTHS), heads, -1)
+    assert torch.equal(by_head.all(2), by_head.any(2)) and not good[-200].any()
+    first = 87                                          # the sequence's first query that sees the key
+    last = min(LENGTHS[2], first + {"plain": 700, "window": 300}.get(kind, 700 if formed else 400))
+    lost = by_head[301 + first:301 + last]
+    assert not lost.any() and bool(by_head[301:301 + first].all()) and bool(by_head[301 + last:-385].all())
+    assert 0.2 < float(by_head[10:300].float().mean()) < 0.9 or kind == "capped"
+    for parts in (2, 4):
+        assert torch.equal(got[parts].isfinite(), good)
+        assert float((got[parts] - got[1])[good].abs().max()) <= 2.0 ** -7 * float(got[1][good].abs().max())
+
+
 def test_parts_of_a_step():
     from starter_b200 import ops
 
