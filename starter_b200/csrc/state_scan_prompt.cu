@@ -35,7 +35,7 @@
 // State-space: row B (16: the block's product of queries and keys, below the diagonal), then Gamma(last, t) dt_t, G, 1 - G of the whole
 // block, B's diagonal with D added.
 #define SP_SCOEF 20
-#define SP_COEF 36               // floats of a token's coefficients (delta rule): W row (16), B row (16), four scalars
+#define SP_COEF(DELTA) ((DELTA) ? 36 : SP_SCOEF)      // floats of a token's coefficients: W row (16, delta rule), B row (16), four scalars
 
 typedef unsigned long long f2;
 __device__ __forceinline__ f2 f2_make(float a, float b) { f2 d; asm("mov.b64 %0, {%1, %2};" : "=l"(d) : "f"(a), "f"(b)); return d; }
@@ -114,13 +114,14 @@ __device__ __forceinline__ int sp_find_block(const int* seq_q_len, int n_seqs, i
   return -1;
 }
 
+template <bool DELTA>
 __global__ void __launch_bounds__(128)
 scan_coef_kernel(const bf16* __restrict__ q, int ldq, const bf16* __restrict__ k, int ldk, const bf16* __restrict__ a_raw,
                  int lda, const bf16* __restrict__ b_raw, int ldb, const float* __restrict__ A_log,
-                 const float* __restrict__ dt_bias, float* __restrict__ coef,
+                 const float* __restrict__ dt_bias, const float* __restrict__ D, float* __restrict__ coef,
                  const int* __restrict__ seq_q_start, const int* __restrict__ seq_q_len, int n_seqs, int H, int G, int N,
                  int per_group) {
-  constexpr int COEF = SP_COEF;
+  constexpr int COEF = SP_COEF(DELTA);
   __shared__ float sa[4][16][17], sb[4][16][17];
   pdl_wait();
   SB_BEHIND_WAIT(q); SB_BEHIND_WAIT(k); SB_BEHIND_WAIT(a_raw); SB_BEHIND_WAIT(b_raw);
@@ -164,28 +165,33 @@ scan_coef_kernel(const bf16* __restrict__ q, int ldq, const bf16* __restrict__ k
     for (int n = 0; n < 2; ++n) {
       sp_mma(qk[n], qv[0].x, qv[1].x, qv[0].y, qv[1].y, kv[n].x, kv[n].y);
       sp_mma(qk[n], qv[0].z, qv[1].z, qv[0].w, qv[1].w, kv[n].z, kv[n].w);
-      sp_mma(kk[n], kv[0].x, kv[1].x, kv[0].y, kv[1].y, kv[n].x, kv[n].y);
-      sp_mma(kk[n], kv[0].z, kv[1].z, kv[0].w, kv[1].w, kv[n].z, kv[n].w);
-      sp_mma(qq[n], qv[0].x, qv[1].x, qv[0].y, qv[1].y, qv[n].x, qv[n].y);
-      sp_mma(qq[n], qv[0].z, qv[1].z, qv[0].w, qv[1].w, qv[n].z, qv[n].w);
+      if (DELTA) {
+        sp_mma(kk[n], kv[0].x, kv[1].x, kv[0].y, kv[1].y, kv[n].x, kv[n].y);
+        sp_mma(kk[n], kv[0].z, kv[1].z, kv[0].w, kv[1].w, kv[n].z, kv[n].w);
+        sp_mma(qq[n], qv[0].x, qv[1].x, qv[0].y, qv[1].y, qv[n].x, qv[n].y);
+        sp_mma(qq[n], qv[0].z, qv[1].z, qv[0].w, qv[1].w, qv[n].z, qv[n].w);
+      }
     }
   }
   // unit norms, lane t holding token t's (t < 16): its squares lie on lane 4 (t % 8) + t % 8 / 2, entry t % 2, half t / 8
-  auto diag = [&](const float (&c)[2][4]) {
-    const int j = lane & 7, from = 4 * j + (j >> 1);
-    const float a = __shfl_sync(0xffffffffu, c[0][0], from), b = __shfl_sync(0xffffffffu, c[0][1], from);
-    const float d = __shfl_sync(0xffffffffu, c[1][2], from), e = __shfl_sync(0xffffffffu, c[1][3], from);
-    return (lane & 8) ? ((j & 1) ? e : d) : ((j & 1) ? b : a);
-  };
-  const float mk = 1.f / sqrtf(diag(kk) + 1e-6f);
-  const float mq = rsqrtf((float)N) / sqrtf(diag(qq) + 1e-6f);
+  float mk = 1.f, mq = 1.f;
+  if (DELTA) {
+    auto diag = [&](const float (&c)[2][4]) {
+      const int j = lane & 7, from = 4 * j + (j >> 1);
+      const float a = __shfl_sync(0xffffffffu, c[0][0], from), b = __shfl_sync(0xffffffffu, c[0][1], from);
+      const float d = __shfl_sync(0xffffffffu, c[1][2], from), e = __shfl_sync(0xffffffffu, c[1][3], from);
+      return (lane & 8) ? ((j & 1) ? e : d) : ((j & 1) ? b : a);
+    };
+    mk = 1.f / sqrtf(diag(kk) + 1e-6f);
+    mq = rsqrtf((float)N) / sqrtf(diag(qq) + 1e-6f);
+  }
   for (int h = h0; h < h1; ++h) {
-    float d = 0.f, fac = 0.f;             // lane t < 16: token t's 1 - decay and beta
+    float d = 0.f, fac = 0.f;             // lane t < 16: token t's 1 - decay and its factor (dt, or beta)
     if (lane < ct) {
       const size_t row = (size_t)(first + lane);
       const float dt = sp_softplus(to_f<bf16>(a_raw[row * lda + h]) + dt_bias[h]);
       d = -expm1f(-expf(A_log[h]) * dt);
-      fac = 1.f / (1.f + expf(-to_f<bf16>(b_raw[row * ldb + h])));
+      fac = DELTA ? 1.f / (1.f + expf(-to_f<bf16>(b_raw[row * ldb + h]))) : dt;
     }
     float gam[2][4], all = 1.f, last = 1.f, gone = 0.f;    // Gamma(t, i); lane t: G_t, Gamma(end, t); 1 - G
 #pragma unroll
@@ -206,6 +212,24 @@ scan_coef_kernel(const bf16* __restrict__ q, int ldq, const bf16* __restrict__ k
     }
     float* rows = coef + ((size_t)first * H + h) * COEF;
     const size_t next = (size_t)H * COEF;
+    if (!DELTA) {
+      const float skip = D ? D[h] : 0.f;
+#pragma unroll
+      for (int n = 0; n < 2; ++n) {
+        const int i0 = 8 * n + 2 * x;
+        const float f0 = __shfl_sync(0xffffffffu, fac, i0), f1 = __shfl_sync(0xffffffffu, fac, i0 + 1);
+#pragma unroll
+        for (int r = 0; r < 2; ++r) {
+          const int t = g + 8 * r;
+          float2 b;
+          b.x = i0 <= t ? gam[n][2 * r] * f0 * qk[n][2 * r] + (i0 == t ? skip : 0.f) : 0.f;
+          b.y = i0 + 1 <= t ? gam[n][2 * r + 1] * f1 * qk[n][2 * r + 1] + (i0 + 1 == t ? skip : 0.f) : 0.f;
+          if (t < ct) *reinterpret_cast<float2*>(rows + t * next + i0) = b;
+        }
+      }
+      if (lane < ct) *reinterpret_cast<float4*>(rows + lane * next + SP_CT) = make_float4(last * fac, 0.f, all, gone);
+      continue;
+    }
     __syncwarp();
 #pragma unroll
     for (int r = 0; r < 2; ++r) {
@@ -256,9 +280,10 @@ scan_coef_kernel(const bf16* __restrict__ q, int ldq, const bf16* __restrict__ k
 // are exact in the tensor cores but for the float sums when the other operand is cut into three bfloat16 pieces (8 bits
 // each, 24 in all): S^T k and S^T q (the tiles as they lie are the other operand's layout), and the write S^T += w^T k.  The
 // warps' sums over their rows meet in shared memory; the two small products of the block (z to outputs and writes) are fmas.
-struct BlocksStage {
+// (State-space: where a walk in segments is not the faster one, scan_segments in ops.py.)
+template <bool DELTA> struct BlocksStage {
   bf16 k[SP_CT][SP_N + 8], q[SP_CT][SP_N + 8], v[SP_CT][SP_COLS];
-  float coef[SP_CT][SP_COEF];
+  float coef[SP_CT][SP_COEF(DELTA)];
 };
 
 __device__ __forceinline__ void sp_ldsm4(uint32_t (&r)[4], const void* p) {
@@ -271,15 +296,17 @@ __device__ __forceinline__ void sp_ldsm4_t(uint32_t (&r)[4], const void* p) {
   asm volatile("ldmatrix.sync.aligned.m8n8.x4.trans.shared.b16 {%0,%1,%2,%3}, [%4];"
                : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]) : "r"(a) : "memory");
 }
+
+template <bool DELTA>
 __global__ void __launch_bounds__(128)
 scan_blocks_kernel(const bf16* __restrict__ q, int ldq, const bf16* __restrict__ k, int ldk, const bf16* __restrict__ v, int ldv,
                    const float* __restrict__ coef, float* __restrict__ state, long long slot_stride, float* __restrict__ out,
                    const int* __restrict__ seq_slot, const int* __restrict__ seq_q_start, const int* __restrict__ seq_q_len,
                    int H, int G, int N, int V) {
-  constexpr int COEF = SP_COEF, TOKS = 2 * SP_CT;      // read-outs a block: queries, then keys
-  constexpr int B_AT = SP_CT, S_AT = COEF - 4;           // places in a row of coefficients
+  constexpr int COEF = SP_COEF(DELTA), TOKS = DELTA ? 2 * SP_CT : SP_CT;      // read-outs a block: queries (then keys)
+  constexpr int B_AT = DELTA ? SP_CT : 0, S_AT = COEF - 4;                    // places in a row of coefficients
   extern __shared__ __align__(16) unsigned char blocks_smem[];
-  BlocksStage* stages = reinterpret_cast<BlocksStage*>(blocks_smem);
+  BlocksStage<DELTA>* stages = reinterpret_cast<BlocksStage<DELTA>*>(blocks_smem);
   __shared__ __align__(16) float part[4][TOKS][SP_COLS + 2], zs[SP_CT][SP_COLS], ws[SP_CT][SP_COLS + 4];
   pdl_wait();
   SB_BEHIND_WAIT(state); SB_BEHIND_WAIT(seq_slot); SB_BEHIND_WAIT(seq_q_start); SB_BEHIND_WAIT(seq_q_len);
@@ -301,7 +328,7 @@ scan_blocks_kernel(const bf16* __restrict__ q, int ldq, const bf16* __restrict__
   const bf16* qg = q + (size_t)group * N;
   const bf16* vh = v + (size_t)h * V + col0;
   auto load = [&](int t0) {                         // a block's operands into a stage: 16-byte pieces, zeros where nothing is
-    BlocksStage& st = stages[t0 / SP_CT % SP_STAGES];
+    BlocksStage<DELTA>& st = stages[t0 / SP_CT % SP_STAGES];
 #pragma unroll
     for (int n = 0; n < 2; ++n) {
       const int e = tid + 128 * n, tt = e >> 4, c = (e & 15) * 8;
@@ -332,7 +359,7 @@ scan_blocks_kernel(const bf16* __restrict__ q, int ldq, const bf16* __restrict__
     __syncthreads();                                // the block's operands are there, and nobody reads the stage filled next
     if (t0 + 2 * SP_CT < q_len) load(t0 + 2 * SP_CT);
     sp_commit();
-    const BlocksStage& st = stages[t0 / SP_CT % SP_STAGES];
+    const BlocksStage<DELTA>& st = stages[t0 / SP_CT % SP_STAGES];
     // this warp's rows of S^T q (and S^T k): columns x tokens
     float dots[TOKS / 8][4];
 #pragma unroll
@@ -343,9 +370,9 @@ scan_blocks_kernel(const bf16* __restrict__ q, int ldq, const bf16* __restrict__
 #pragma unroll
       for (int r = 0; r < 4; ++r) sp_split(S[2 * s + (r >> 1)][2 * (r & 1)], S[2 * s + (r >> 1)][2 * (r & 1) + 1], a[r]);
       const int tt = (lane & 7) + (mi >> 1) * 8, row = 32 * warp + 16 * s + (mi & 1) * 8;
-      uint32_t b[2][4];
+      uint32_t b[DELTA ? 2 : 1][4];
       sp_ldsm4(b[0], &st.q[tt][row]);
-      sp_ldsm4(b[1], &st.k[tt][row]);
+      if constexpr (DELTA) sp_ldsm4(b[1], &st.k[tt][row]);
 #pragma unroll
       for (int p = 2; p >= 0; --p)                  // (the small pieces first)
 #pragma unroll
@@ -378,8 +405,22 @@ scan_blocks_kernel(const bf16* __restrict__ q, int ldq, const bf16* __restrict__
         }
       }
     };
+    if constexpr (!DELTA) {                         // what is written does not depend on what is read
+      float w[8];
+#pragma unroll
+      for (int n = 0; n < 8; ++n) {
+        const int t = 2 * x + (n & 1) + 8 * (n >> 2);
+        w[n] = st.coef[t][S_AT] * to_f<bf16>(st.v[t][g + 8 * ((n >> 1) & 1)]);
+      }
+      update(w);
+    }
     const uint32_t vv = *reinterpret_cast<const uint32_t*>(&st.v[tok][c2]);
-    __syncthreads();                                // the warps' sums are there
+    // Coefficients of later tokens are zero, but 0 * inf would not be: a block with a value that is not finite masks them
+    // (the test rides on a barrier that is there anyway, the masked sums stand behind the usual ones: 164 us a layer of 2,048 tokens;
+    // masking always, or a branch around the usual sums: 190)
+    bool bad = !(fabsf(__uint_as_float(vv << 16)) < INFINITY && fabsf(__uint_as_float(vv & 0xffff0000u)) < INFINITY);
+    if constexpr (DELTA) __syncthreads();           // the warps' sums are there
+    else bad = __syncthreads_or(bad);
     const float4 s4 = *reinterpret_cast<const float4*>(&st.coef[tok][S_AT]);
     float2 rq = make_float2(0.f, 0.f);
 #pragma unroll
@@ -388,35 +429,45 @@ scan_blocks_kernel(const bf16* __restrict__ q, int ldq, const bf16* __restrict__
       rq.x += p.x;
       rq.y += p.y;
     }
-    float2 rk = make_float2(0.f, 0.f);
+    if constexpr (DELTA) {
+      float2 rk = make_float2(0.f, 0.f);
 #pragma unroll
-    for (int w = 0; w < 4; ++w) {
-      const float2 p = *reinterpret_cast<const float2*>(&part[w][SP_CT + tok][c2]);
-      rk.x += p.x;
-      rk.y += p.y;
+      for (int w = 0; w < 4; ++w) {
+        const float2 p = *reinterpret_cast<const float2*>(&part[w][SP_CT + tok][c2]);
+        rk.x += p.x;
+        rk.y += p.y;
+      }
+      const float2 z = make_float2(s4.x * __uint_as_float(vv << 16) - s4.y * rk.x, s4.x * __uint_as_float(vv & 0xffff0000u) - s4.y * rk.y);
+      *reinterpret_cast<float2*>(&zs[tok][c2]) = z;
+      bad = __syncthreads_or(!(fabsf(z.x) < INFINITY && fabsf(z.y) < INFINITY));
     }
-    const float2 z = make_float2(s4.x * __uint_as_float(vv << 16) - s4.y * rk.x, s4.x * __uint_as_float(vv & 0xffff0000u) - s4.y * rk.y);
-    *reinterpret_cast<float2*>(&zs[tok][c2]) = z;
-    // Coefficients of later tokens are zero, but 0 * inf would not be: a block with a value that is not finite masks them
-    // (the test rides on a barrier that is there anyway, the masked sums stand behind the usual ones: 187 us a layer of 2,136 tokens;
-    // masking always, or a branch around the usual sums: 199 and 194)
-    const bool bad = __syncthreads_or(!(fabsf(z.x) < INFINITY && fabsf(z.y) < INFINITY));
     float2 own = make_float2(0.f, 0.f), w2 = make_float2(0.f, 0.f);
     auto small = [&](auto masked) {
 #pragma unroll
       for (int i = 0; i < SP_CT; i += 4) {
         const float4 b = *reinterpret_cast<const float4*>(&st.coef[tok][B_AT + i]);
         const float bb[4] = {b.x, b.y, b.z, b.w};
-        const float4 w = *reinterpret_cast<const float4*>(&st.coef[tok][i]);
-        const float ww[4] = {w.x, w.y, w.z, w.w};
+        float ww[4] = {0.f, 0.f, 0.f, 0.f};
+        if constexpr (DELTA) {
+          const float4 w = *reinterpret_cast<const float4*>(&st.coef[tok][i]);
+          ww[0] = w.x; ww[1] = w.y; ww[2] = w.z; ww[3] = w.w;
+        }
 #pragma unroll
         for (int e = 0; e < 4; ++e) {
-          float2 z = *reinterpret_cast<const float2*>(&zs[i + e][c2]);
+          float2 z;
+          if constexpr (DELTA) {
+            z = *reinterpret_cast<const float2*>(&zs[i + e][c2]);
+          } else {
+            const uint32_t raw = *reinterpret_cast<const uint32_t*>(&st.v[i + e][c2]);
+            z = make_float2(__uint_as_float(raw << 16), __uint_as_float(raw & 0xffff0000u));
+          }
           if (decltype(masked)::value && i + e > tok) z = make_float2(0.f, 0.f);
           own.x = fmaf(bb[e], z.x, own.x);
           own.y = fmaf(bb[e], z.y, own.y);
-          w2.x = fmaf(ww[e], z.x, w2.x);
-          w2.y = fmaf(ww[e], z.y, w2.y);
+          if constexpr (DELTA) {
+            w2.x = fmaf(ww[e], z.x, w2.x);
+            w2.y = fmaf(ww[e], z.y, w2.y);
+          }
         }
       }
     };
@@ -425,15 +476,17 @@ scan_blocks_kernel(const bf16* __restrict__ q, int ldq, const bf16* __restrict__
       own = w2 = make_float2(0.f, 0.f);
       small(std::true_type{});
     }
-    *reinterpret_cast<float2*>(&ws[tok][c2]) = w2;
+    if constexpr (DELTA) *reinterpret_cast<float2*>(&ws[tok][c2]) = w2;
     if (t0 + tok < q_len && col0 + c2 < V)
       *reinterpret_cast<float2*>(out + (size_t)(q_start + t0 + tok) * H * V + (size_t)h * V + col0 + c2) =
           make_float2(fmaf(s4.z, rq.x, own.x), fmaf(s4.z, rq.y, own.y));
-    __syncthreads();
-    float w[8];
+    if constexpr (DELTA) {
+      __syncthreads();
+      float w[8];
 #pragma unroll
-    for (int n = 0; n < 8; ++n) w[n] = ws[2 * x + (n & 1) + 8 * (n >> 2)][g + 8 * ((n >> 1) & 1)];
-    update(w);
+      for (int n = 0; n < 8; ++n) w[n] = ws[2 * x + (n & 1) + 8 * (n >> 2)][g + 8 * ((n >> 1) & 1)];
+      update(w);
+    }
   }
   pdl_trigger();
 #pragma unroll
@@ -455,9 +508,9 @@ scan_blocks_kernel(const bf16* __restrict__ q, int ldq, const bf16* __restrict__
 // of 16 columns x 8 rows.  The two halves' sums over their rows meet in shared memory one step later, behind the barrier that is
 // there anyway: each half keeps one half of the tokens.  Measured against one walk by four warps a head and 16 columns (us; segments):
 // 2,048 tokens of 32 heads 100 -> 64 (9), of 16 heads 99 -> 45 (16); 700 of 16 heads 41 -> 23 (9); four sequences of 500 tokens and 32 heads
-// 73 -> 54, eight of 400 99 -> 73 (1 each); 64 tokens of 16 heads 12.4 -> 14.4, 128 of 32 heads 15.3 -> 16.4: two kernels of longer
-// straight code.  The error against 64 bits: 1.14e-7 -> 1.16e-7, 1.13e-7 -> 1.11e-7, 1.23e-7 -> 1.17e-7, 1.39e-7 -> 1.19e-7 (2,048, 2 x 700, 333,
-// 3 x 64 tokens), the states' unchanged.  At nine segments the walk with outputs takes 31 of the 64 us: its products keep the tensor
+// 73 -> 54, eight of 400 99 -> 73 (1 each).  Few tokens or blocks that do not fill the SMs stay with one walk (64 tokens of 16 heads 9.6, here
+// 12.2: two kernels of longer straight code; scan_one_walk in ops.py).  The error against 64 bits, means of 16 seeds (outputs):
+// 2,048 tokens of 32 heads 1.87e-7 -> 1.66e-7; 2 x 700 of 16 heads 1.84e-7 -> 1.63e-7; 200 of 32 heads 1.79e-7 -> 1.59e-7.  At nine segments the walk with outputs takes 31 of the 64 us: its products keep the tensor
 // cores busy for half of that, cutting the state into pieces the issue slots for a third.
 __device__ __forceinline__ int sp_span(int q_len, int segs) {       // tokens a segment: whole blocks
   const int blocks = (q_len + SP_CT - 1) / SP_CT;
@@ -1072,6 +1125,22 @@ scan_rows_kernel(const void* __restrict__ q, int ldq, const bf16* __restrict__ k
     }
 }
 
+template <bool DELTA>
+static int scan_blocks(const bf16* q, int ldq, const bf16* k, int ldk, const bf16* v, int ldv, const bf16* a_raw, int lda, const bf16* b_raw,
+                       int ldb, const float* A_log, const float* dt_bias, const float* D, float* coef, float* state,
+                       long long slot_stride, float* out, const int* seq_slot, const int* seq_q_start, const int* seq_q_len, int n_tokens,
+                       int n_seqs, int H, int G, int N, int V, cudaStream_t s) {
+  const int per_group = (H / G + SP_HEADS - 1) / SP_HEADS;
+  const int rc = launch_dependent(scan_coef_kernel<DELTA>, dim3(n_tokens / SP_CT + n_seqs, (G * per_group + 3) / 4), dim3(128), 0, s, q, ldq, k,
+                                  ldk, a_raw, lda, b_raw, ldb, A_log, dt_bias, D, coef, seq_q_start, seq_q_len, n_seqs, H, G, N, per_group);
+  if (rc) return rc;
+  const size_t smem = SP_STAGES * sizeof(BlocksStage<DELTA>);
+  cudaError_t err = cudaFuncSetAttribute(scan_blocks_kernel<DELTA>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+  if (err != cudaSuccess) return (int)err;
+  return launch_dependent(scan_blocks_kernel<DELTA>, dim3(n_seqs, H, (V + SP_COLS - 1) / SP_COLS), dim3(128), smem, s, q, ldq, k, ldk, v, ldv,
+                          (const float*)coef, state, slot_stride, out, seq_slot, seq_q_start, seq_q_len, H, G, N, V);
+}
+
 static int scan_segments(const bf16* q, int ldq, const bf16* k, int ldk, const bf16* v, int ldv, const bf16* a_raw, int lda,
                          const float* A_log, const float* dt_bias, const float* D, float* coef, float* state, long long slot_stride,
                          float* out, const int* seq_slot, const int* seq_q_start, const int* seq_q_len, int n_tokens, int n_seqs, int H, int G, int N, int V, int segs, float* carried, cudaStream_t s) {
@@ -1102,14 +1171,15 @@ int sb_scan_prompt_floats(int dtype, int mode, const void* q, int ldq, const voi
   if (dtype != 1 || mode < 0 || mode > 3 || N <= 64 || N > SP_N || N % 8 || V < 8 || V % 8 || ldq % 8 || ldk % 8 || ldv % 8) return -1;
   if (H < 1 || G < 1 || H % G || (mode >= 2 && G != H)) return -1;
   if (((uintptr_t)q | (uintptr_t)k | (uintptr_t)v | (uintptr_t)row_decay) % 16) return -1;
-  return mode < 2 ? H * (mode == 1 ? SP_COEF : SP_SCOEF) : mode == 2 ? 2 * H * N : 0;
+  return mode < 2 ? H * SP_COEF(mode == 1) : mode == 2 ? 2 * H * N : 0;
 }
 
 // Floats of a segment's place in `carried`, per sequence: the state in whole blocks of columns, and its decay.
 long long sb_scan_segment_floats(int H, int V) { return (long long)H * ((V + SP_SCOLS - 1) / SP_SCOLS * (SP_SCOLS * SP_N) + 1); }
 
 // Arguments as sb_state_scan's; scratch: float [n_tokens, that many], 16-byte aligned (null where it is 0).  segs: segments a
-// sequence (mode 0 only; 1 otherwise), carried: float [n_seqs, segs, sb_scan_segment_floats], 16-byte aligned (null for one).
+// sequence (mode 0 only; 0: one walk, the delta rule's kernels), carried: float [n_seqs, segs, sb_scan_segment_floats], 16-byte aligned
+// (null up to one).
 int sb_state_scan_prompt(int mode, const void* q, int ldq, const void* k, int ldk, const void* v, int ldv,
                          const void* a_raw, int lda, const void* b_raw, int ldb, const float* A_log, const float* dt_bias,
                          const float* D, const float* row_decay, float* state, long long slot_stride, float* out,
@@ -1117,24 +1187,16 @@ int sb_state_scan_prompt(int mode, const void* q, int ldq, const void* k, int ld
                          int G, int N, int V, float* scratch, int segs, float* carried, cudaStream_t s) {
   if (n_seqs == 0 || n_tokens == 0) return 0;
   if (sb_scan_prompt_floats(1, mode, q, ldq, k, ldk, v, ldv, row_decay, H, G, N, V) < 0 || (mode < 3 && !scratch) ||
-      ((uintptr_t)scratch % 16) || segs < 1 || (segs > 1 && (mode != 0 || !carried || (uintptr_t)carried % 16)) || (mode == 1 && !b_raw) || (mode == 3) != (row_decay != nullptr))
+      ((uintptr_t)scratch % 16) || segs < 0 || (segs > 1 && (mode != 0 || !carried || (uintptr_t)carried % 16)) || (mode == 1 && !b_raw) ||
+      (mode == 3) != (row_decay != nullptr))
     return -2;
   const dim3 grid(n_seqs, H, (V + SP_COLS - 1) / SP_COLS);
   if (mode < 2) {
-    if (mode == 0)
-      return scan_segments((const bf16*)q, ldq, (const bf16*)k, ldk, (const bf16*)v, ldv, (const bf16*)a_raw, lda, A_log, dt_bias, D,
-                           scratch, state, slot_stride, out, seq_slot, seq_q_start, seq_q_len, n_tokens, n_seqs, H, G, N, V, segs,
-                           carried, s);
-    const int per_group = (H / G + SP_HEADS - 1) / SP_HEADS;
-    const int rc = launch_dependent(scan_coef_kernel, dim3(n_tokens / SP_CT + n_seqs, (G * per_group + 3) / 4), dim3(128), 0, s,
-                                    (const bf16*)q, ldq, (const bf16*)k, ldk, (const bf16*)a_raw, lda, (const bf16*)b_raw, ldb, A_log,
-                                    dt_bias, scratch, seq_q_start, seq_q_len, n_seqs, H, G, N, per_group);
-    if (rc) return rc;
-    const size_t smem = SP_STAGES * sizeof(BlocksStage);
-    cudaError_t err = cudaFuncSetAttribute(scan_blocks_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-    if (err != cudaSuccess) return (int)err;
-    return launch_dependent(scan_blocks_kernel, grid, dim3(128), smem, s, (const bf16*)q, ldq, (const bf16*)k, ldk, (const bf16*)v,
-                            ldv, (const float*)scratch, state, slot_stride, out, seq_slot, seq_q_start, seq_q_len, H, G, N, V);
+#define ARGS(...) (const bf16*)q, ldq, (const bf16*)k, ldk, (const bf16*)v, ldv, (const bf16*)a_raw, lda, __VA_ARGS__ A_log, dt_bias, D, scratch, \
+                  state, slot_stride, out, seq_slot, seq_q_start, seq_q_len, n_tokens, n_seqs, H, G, N, V
+    if (mode == 0 && segs > 0) return scan_segments(ARGS(), segs, carried, s);
+    return mode == 1 ? scan_blocks<true>(ARGS((const bf16*)b_raw, ldb,), s) : scan_blocks<false>(ARGS((const bf16*)b_raw, ldb,), s);
+#undef ARGS
   }
   if (mode == 2) {
     const int channels = H * N;

@@ -2571,6 +2571,16 @@ def scan_segments(n_tokens: int, n_seqs: int, blocks: int) -> int:
     return max(1, min(segs, tokens // 48, 16))
 
 
+def scan_one_walk(n_tokens: int, n_seqs: int, blocks: int) -> bool:
+    """Whether a state-space step is walked as the delta rule's are (csrc/state_scan_prompt.cu: four warps and 16 columns a block, one
+    walk) and not in segments: where its blocks, four for each of ``blocks``, are at most three to an SM and the sequences are too
+    short for many segments.  Measured (us, one walk / segments; heads x sequences, tokens each): 16 x 1, 64 9.6 / 12.2, 128 12.7 / 15.0, 176
+    14.7 / 14.4, 192 15.4 / 14.0, 300 20.3 / 15.3; 24 x 2, 128 15.0 / 15.3, 150 17.3 / 15.3; 16 x 4, 64 11.3 / 12.8, 500 38.8 / 41.1, 700 51.2 /
+    45.8; 24 x 4, 100 16.8 / 17.5, 1,000 89.3 / 93.5; 37 x 3, 200 24.2 / 24.0, 1,000 89.3 / 93.6; 28 x 4, 64 15.5 / 13.7, 1,000 127 / 94."""
+    segs, blocks = scan_segments(n_tokens, n_seqs, blocks), 4 * blocks * n_seqs
+    return blocks <= 3 * SM_COUNT and segs <= (3 if blocks <= SM_COUNT else 2)
+
+
 def state_scan(mode, q, k, v, a_raw, b_raw, A_log, dt_bias, skip, state, state_at, seq_slot, seq_q_start, seq_q_len,
                heads, groups, n_state, v_dim, decay=None):
     """A linear recurrence with a state ``S`` ``[n_state, v_dim]`` per head over the sequences of a step.
@@ -2626,7 +2636,8 @@ def state_scan(mode, q, k, v, a_raw, b_raw, A_log, dt_bias, skip, state, state_a
             scratch = _empty(state, (n_tokens, floats), torch.float32) if floats else None
             segs, carried = 1, None
             if mode == "state_space":
-                segs = scan_segments(n_tokens, n_seqs, heads * -(-v_dim // 64))
+                step = (n_tokens, n_seqs, heads * -(-v_dim // 64))
+                segs = 0 if scan_one_walk(*step) else scan_segments(*step)
                 if segs > 1:
                     carried = _empty(state, (n_seqs * segs * lib.sb_scan_segment_floats(heads, v_dim),))
             rc = lib.sb_state_scan_prompt(

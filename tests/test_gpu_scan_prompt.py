@@ -34,11 +34,24 @@ def stated(mode, q, k, v, a, b, A, bias, skip, decay, heads, groups, n, width):
     return salulorn.decayed_recurrence(q * n ** -0.5, k, v, 1.0 - decay.reshape(t, heads, n))
 
 
-@pytest.mark.parametrize("mode", ["state_space", "gated_delta", "forget_write", "channel_decay"])
+def form(mode, monkeypatch):
+    """The mode; "segments" is a state-space step that is not walked at once, whatever its size."""
+    from starter_b200 import ops
+
+    if mode == "segments":
+        monkeypatch.setattr(ops, "scan_one_walk", lambda *a: False)
+        return "state_space"
+    if mode == "state_space":
+        monkeypatch.setattr(ops, "scan_one_walk", lambda *a: True)
+    return mode
+
+
+@pytest.mark.parametrize("mode", ["state_space", "segments", "gated_delta", "forget_write", "channel_decay"])
 @pytest.mark.parametrize("heads,groups,n,width", [(2, 1, 128, 64), (4, 2, 72, 24), (10, 1, 104, 8), (3, 3, 120, 40)])
 def test_many_tokens_a_sequence(mode, heads, groups, n, width, monkeypatch):
     from starter_b200 import ops
 
+    mode = form(mode, monkeypatch)
     if mode in ("forget_write", "channel_decay"):
         groups = heads
     gen = torch.Generator().manual_seed(heads * n)
@@ -102,11 +115,12 @@ def test_many_tokens_a_sequence(mode, heads, groups, n, width, monkeypatch):
     assert float((kept - state).abs().max()) <= 2e-5 * float(state.abs().max())
 
 
-@pytest.mark.parametrize("mode", ["state_space", "gated_delta", "forget_write", "channel_decay"])
+@pytest.mark.parametrize("mode", ["state_space", "segments", "gated_delta", "forget_write", "channel_decay"])
 @pytest.mark.parametrize("which", ["q", "k", "v"])
-def test_a_token_that_is_not_finite_leaves_earlier_tokens_alone(mode, which):
+def test_a_token_that_is_not_finite_leaves_earlier_tokens_alone(mode, which, monkeypatch):
     from starter_b200 import ops
 
+    mode = form(mode, monkeypatch)
     heads, n, width, tokens, bad = 2, 128, 32, 70, 37
     gen = torch.Generator().manual_seed(heads + n)
     ins = {name: torch.randn(tokens, heads * size, generator=gen).to(BF).cuda()
@@ -132,10 +146,11 @@ def test_a_token_that_is_not_finite_leaves_earlier_tokens_alone(mode, which):
     assert bool(got[bad].isfinite().all()) == (mode == "forget_write" and which == "k")
 
 
-@pytest.mark.parametrize("mode", ["state_space", "gated_delta", "forget_write", "channel_decay"])
+@pytest.mark.parametrize("mode", ["state_space", "segments", "gated_delta", "forget_write", "channel_decay"])
 def test_more_tokens_than_a_grid_counts_in_its_second_dimension(mode, monkeypatch):
     from starter_b200 import ops
 
+    mode = form(mode, monkeypatch)
     heads, n, width, lengths = 1, 72, 8, [33000, 32600]
     total, gen = sum(lengths), torch.Generator().manual_seed(9)
     q, k, v, ab = (torch.randn(total, size, generator=gen).to(BF).cuda() for size in (n, n, width, 8))
@@ -197,16 +212,18 @@ def test_state_space_in_segments(segs, width, monkeypatch):
     start = torch.randn(6, heads * n * width, generator=gen).cuda()
 
     def run(count):
+        monkeypatch.setattr(ops, "scan_one_walk", lambda *a: count == 0)
         monkeypatch.setattr(ops, "scan_segments", lambda *a: count)
         state = start.clone()
         out = ops.state_scan("state_space", (qk, n), (qk, 0), (v, 0), (ab, 0), None, A, bias, skip, state, 0, *packed(lengths, slots),
                              heads, 1, n, width)
         return out, state
 
-    (want, kept), (got, state) = run(1), run(segs)
+    (got, state), others = run(segs), (run(0), run(1))
     # float arithmetic in another order: some hundred roundings of 2^-24 of terms that may cancel
-    assert float((got - want).abs().max()) <= 2e-5 * float(want.abs().max())
-    assert float((state - kept).abs().max()) <= 2e-5 * float(kept.abs().max())
+    for want, kept in others:
+        assert float((got - want).abs().max()) <= 2e-5 * float(want.abs().max())
+        assert float((state - kept).abs().max()) <= 2e-5 * float(kept.abs().max())
 
 
 def test_segments_of_a_step():
@@ -215,3 +232,8 @@ def test_segments_of_a_step():
     for tokens, seqs, blocks in ((64, 1, 32), (2048, 1, 32), (300, 1, 1), (5, 3, 8), (1 << 20, 4, 1), (40000, 600, 32)):
         segs = ops.scan_segments(tokens, seqs, blocks)
         assert 1 <= segs <= 16 and (segs == 1 or (segs * seqs * blocks <= 2 * 148 and tokens // seqs >= 48 * segs))
+    # one walk where sequences are short, or its blocks fill the SMs evenly and segments are few
+    for tokens, seqs, blocks, once in ((64, 1, 16, True), (191, 1, 16, True), (192, 1, 16, False), (2048, 1, 32, False), (286, 2, 24, True),
+                                       (288, 2, 24, False), (2000, 4, 16, True), (2800, 4, 16, False), (8000, 4, 24, True),
+                                       (64 * 7, 7, 16, False), (64, 1, 111, True), (64, 1, 112, False)):
+        assert ops.scan_one_walk(tokens, seqs, blocks) is once
