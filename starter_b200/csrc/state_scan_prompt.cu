@@ -499,7 +499,7 @@ scan_blocks_kernel(const bf16* __restrict__ q, int ldq, const bf16* __restrict__
 }
 
 // ------------------------------------------------------------------------------------------ segments of blocks
-// Where what a block of tokens writes does not depend on the state it finds (state-space), a segment of blocks takes S to S - gone S + L
+// Where what a block of tokens writes does not depend on the state it finds (state-space), a segment of blocks takes S to G S + L
 // with L what it writes into zeros.  So every sequence is cut into `segs` segments that are walked at once: scan_prepare_kernel
 // walks all but the last without outputs and files the state a sequence starts with (place 0), the state behind its first segment
 // (place 1) and the others' L (place of the next segment), beside the blocks' coefficients; scan_segments_kernel puts together the
@@ -509,8 +509,9 @@ scan_blocks_kernel(const bf16* __restrict__ q, int ldq, const bf16* __restrict__
 // there anyway: each half keeps one half of the tokens.  Measured against one walk by four warps a head and 16 columns (us; segments):
 // 2,048 tokens of 32 heads 100 -> 64 (9), of 16 heads 99 -> 45 (16); 700 of 16 heads 41 -> 23 (9); four sequences of 500 tokens and 32 heads
 // 73 -> 54, eight of 400 99 -> 73 (1 each).  Few tokens or blocks that do not fill the SMs stay with one walk (64 tokens of 16 heads 9.6, here
-// 12.2: two kernels of longer straight code; scan_one_walk in ops.py).  The error against 64 bits, means of 16 seeds (outputs):
-// 2,048 tokens of 32 heads 1.87e-7 -> 1.66e-7; 2 x 700 of 16 heads 1.84e-7 -> 1.63e-7; 200 of 32 heads 1.79e-7 -> 1.59e-7.  At nine segments the walk with outputs takes 31 of the 64 us: its products keep the tensor
+// 12.2: two kernels of longer straight code; scan_one_walk in ops.py).  The error against 64 bits, means of 16 seeds (outputs; states;
+// slow decays): 2,048 tokens of 32 heads 1.87e-7 -> 1.65e-7; 1.20e-7 the same; 2.54e-7 -> 1.73e-7; 2 x 700 of 16 heads 1.84e-7 -> 1.62e-7;
+// 1.16e-7 the same; 1.80e-7 -> 1.62e-7; 200 of 32 heads 1.79e-7 -> 1.58e-7; 1.14e-7 -> 1.12e-7; 1.29e-7 -> 1.19e-7.  At nine segments the walk with outputs takes 31 of the 64 us: its products keep the tensor
 // cores busy for half of that, cutting the state into pieces the issue slots for a third.
 __device__ __forceinline__ int sp_span(int q_len, int segs) {       // tokens a segment: whole blocks
   const int blocks = (q_len + SP_CT - 1) / SP_CT;
@@ -660,10 +661,11 @@ scan_prepare_kernel(const bf16* __restrict__ q, int ldq, const bf16* __restrict_
                     const float* __restrict__ D, float* __restrict__ coef, const float* __restrict__ state, long long slot_stride,
                     const int* __restrict__ seq_slot, const int* __restrict__ seq_q_start, const int* __restrict__ seq_q_len,
                     int n_seqs, int H, int G, int N, int V, int segs, int writers, float4* __restrict__ carried,
-                    float* __restrict__ gones) {
+                    float* __restrict__ keeps) {
   constexpr int T = SP_STHREADS;
   extern __shared__ __align__(16) unsigned char writes_smem[];
   WritesStage* stages = reinterpret_cast<WritesStage*>(writes_smem);
+  __shared__ float dt_of[T / 32];
   pdl_wait();
   SB_BEHIND_WAIT(q); SB_BEHIND_WAIT(k); SB_BEHIND_WAIT(a_raw); SB_BEHIND_WAIT(state);
   SB_BEHIND_WAIT(seq_slot); SB_BEHIND_WAIT(seq_q_start); SB_BEHIND_WAIT(seq_q_len);
@@ -685,7 +687,7 @@ scan_prepare_kernel(const bf16* __restrict__ q, int ldq, const bf16* __restrict_
   if (last && seg > 0) return;
   const int q_len = last ? t_first : t_first + span;
   float4* to = carried + ((((size_t)seq * H + h) * z + zi) * segs) * (SP_TILES * T) + tid;
-  float S[SP_TILES][4], gone_all = 0.f;
+  float S[SP_TILES][4], dt_mine = 0.f;
 #pragma unroll
   for (int j = 0; j < SP_TILES; ++j) S[j][0] = S[j][1] = S[j][2] = S[j][3] = 0.f;
   if (seg == 0) {
@@ -722,6 +724,7 @@ scan_prepare_kernel(const bf16* __restrict__ q, int ldq, const bf16* __restrict_
     const float behind = __shfl_down_sync(0xffffffffu, suf, 1);
     if (lane < SP_CT) st.c[lane] = dt * (lane < SP_CT - 1 ? behind : 1.f);
     if (lane == 0) st.gone = gone;
+    dt_mine += dt;
   };
   const bf16* kg = k + (size_t)group * N;
   const bf16* vh = v + (size_t)h * V + col0;
@@ -753,28 +756,38 @@ scan_prepare_kernel(const bf16* __restrict__ q, int ldq, const bf16* __restrict_
     uint32_t va[4];
     sp_values(va, st.v, cw, lane);
     if (t0 + SP_CT < q_len && warp == (t0 / SP_CT + 1) % (T / 32)) factors(t0 + SP_CT);
-    const float gone = st.gone;
-    gone_all = fmaf(-gone_all, gone, gone_all + gone);
-    sp_write<1>(S, va, st.c, gone, st.k, row0, lane);
+    if (t0 + SP_CT >= q_len) {                      // (the factors are made: their exponents' sum, beside the last products)
+      const float sum = warp_sum(dt_mine);
+      if (lane == 0) dt_of[warp] = sum;
+    }
+    sp_write<1>(S, va, st.c, st.gone, st.k, row0, lane);
   }
   pdl_trigger();
 #pragma unroll
   for (int j = 0; j < SP_TILES; ++j) to[((seg + 1) * SP_TILES + j) * T] = make_float4(S[j][0], S[j][1], S[j][2], S[j][3]);
-  if (tid == 0 && zi == 0) gones[((size_t)seq * H + h) * segs + seg] = gone_all;
+  // What the segment leaves of the state it finds, from the sum of its exponents: products of complements, which every block would round
+  // again, had the states 1.158e-7 off after 200 tokens in four segments (one walk 1.138e-7, this 1.118e-7).
+  if (zi > 0) return;
+  __syncthreads();
+  if (tid == 0) {
+    float x = 0.f;
+    for (int w = 0; w < T / 32; ++w) x += dt_of[w];
+    keeps[((size_t)seq * H + h) * segs + seg] = expf(-decay * x);
+  }
 }
 
 __global__ void __launch_bounds__(SP_STHREADS, 2)
 scan_segments_kernel(const bf16* __restrict__ q, int ldq, const bf16* __restrict__ k, int ldk, const bf16* __restrict__ v, int ldv,
                      const float* __restrict__ coef, float* __restrict__ state, long long slot_stride, float* __restrict__ out,
                      const int* __restrict__ seq_slot, const int* __restrict__ seq_q_start, const int* __restrict__ seq_q_len,
-                     int H, int G, int N, int V, int segs, const float4* __restrict__ carried, const float* __restrict__ gones) {
+                     int H, int G, int N, int V, int segs, const float4* __restrict__ carried, const float* __restrict__ keeps) {
   constexpr int T = SP_STHREADS;
   extern __shared__ __align__(16) unsigned char segments_smem[];
   SegmentStage* stages = reinterpret_cast<SegmentStage*>(segments_smem);
   __shared__ __align__(16) float4 part[2][8][32];
   pdl_wait();
   SB_BEHIND_WAIT(state); SB_BEHIND_WAIT(seq_slot); SB_BEHIND_WAIT(seq_q_start); SB_BEHIND_WAIT(seq_q_len);
-  SB_BEHIND_WAIT(carried); SB_BEHIND_WAIT(gones);
+  SB_BEHIND_WAIT(carried); SB_BEHIND_WAIT(keeps);
   const int seq = blockIdx.x / segs, seg = blockIdx.x - seq * segs, h = blockIdx.y, col0 = blockIdx.z * SP_SCOLS;
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, g = lane >> 2, x = lane & 3;
   const int cw = warp & 3, row0 = (warp >> 2) * (SP_N / 2);      // the warp's columns and rows
@@ -822,7 +835,7 @@ scan_segments_kernel(const bf16* __restrict__ q, int ldq, const bf16* __restrict
       }
   } else {
     const float4* from = carried + ((((size_t)seq * H + h) * gridDim.z + blockIdx.z) * segs) * (SP_TILES * T) + tid;
-    const float* gone = gones + ((size_t)seq * H + h) * segs;
+    const float* kept = keeps + ((size_t)seq * H + h) * segs;
     const int p0 = seg == 0 ? 0 : 1;
 #pragma unroll
     for (int j = 0; j < SP_TILES; ++j) {
@@ -830,14 +843,14 @@ scan_segments_kernel(const bf16* __restrict__ q, int ldq, const bf16* __restrict
       S[j][0] = e.x; S[j][1] = e.y; S[j][2] = e.z; S[j][3] = e.w;
     }
     for (int p = 2; p <= seg; ++p) {
-      const float d = gone[p - 1];
+      const float d = kept[p - 1];
 #pragma unroll
       for (int j = 0; j < SP_TILES; ++j) {
         const float4 e = from[(p * SP_TILES + j) * T];
-        S[j][0] = fmaf(-d, S[j][0], S[j][0]) + e.x;
-        S[j][1] = fmaf(-d, S[j][1], S[j][1]) + e.y;
-        S[j][2] = fmaf(-d, S[j][2], S[j][2]) + e.z;
-        S[j][3] = fmaf(-d, S[j][3], S[j][3]) + e.w;
+        S[j][0] = fmaf(d, S[j][0], e.x);
+        S[j][1] = fmaf(d, S[j][1], e.y);
+        S[j][2] = fmaf(d, S[j][2], e.z);
+        S[j][3] = fmaf(d, S[j][3], e.w);
       }
     }
   }
@@ -1145,7 +1158,7 @@ static int scan_segments(const bf16* q, int ldq, const bf16* k, int ldk, const b
                          const float* A_log, const float* dt_bias, const float* D, float* coef, float* state, long long slot_stride,
                          float* out, const int* seq_slot, const int* seq_q_start, const int* seq_q_len, int n_tokens, int n_seqs, int H, int G, int N, int V, int segs, float* carried, cudaStream_t s) {
   const int z = (V + SP_SCOLS - 1) / SP_SCOLS;
-  float* gones = carried ? carried + (size_t)n_seqs * segs * H * z * (SP_SCOLS * SP_N) : nullptr;
+  float* keeps = carried ? carried + (size_t)n_seqs * segs * H * z * (SP_SCOLS * SP_N) : nullptr;
   const size_t wsmem = SP_STAGES * sizeof(WritesStage), alone = 120 * 1024;
   // (blocks that all find an SM of their own ask for more than half its shared memory: two on one SM, the others idle, is up to
   // half again as slow, and happened in every third run)
@@ -1155,11 +1168,11 @@ static int scan_segments(const bf16* q, int ldq, const bf16* k, int ldk, const b
   const int writers = n_seqs * (segs - 1) * H * z, jobs = (n_tokens / SP_CT + n_seqs) * H;
   const int rc = launch_dependent(scan_prepare_kernel, dim3(writers + (jobs + 7) / 8), dim3(SP_STHREADS), wsmem, s, q, ldq, k, ldk, v,
                                   ldv, a_raw, lda, A_log, dt_bias, D, coef, (const float*)state, slot_stride, seq_slot, seq_q_start,
-                                  seq_q_len, n_seqs, H, G, N, V, segs, writers, (float4*)carried, gones);
+                                  seq_q_len, n_seqs, H, G, N, V, segs, writers, (float4*)carried, keeps);
   if (rc) return rc;
   return launch_dependent(scan_segments_kernel, dim3(n_seqs * segs, H, z), dim3(SP_STHREADS), smem, s, q, ldq, k, ldk, v, ldv, (const float*)coef,
                           state, slot_stride, out, seq_slot, seq_q_start, seq_q_len, H, G, N, V, segs, (const float4*)carried,
-                          (const float*)gones);
+                          (const float*)keeps);
 }
 
 extern "C" {

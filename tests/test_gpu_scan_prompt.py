@@ -237,3 +237,27 @@ def test_segments_of_a_step():
                                        (288, 2, 24, False), (2000, 4, 16, True), (2800, 4, 16, False), (8000, 4, 24, True),
                                        (64 * 7, 7, 16, False), (64, 1, 111, True), (64, 1, 112, False)):
         assert ops.scan_one_walk(tokens, seqs, blocks) is once
+
+
+@pytest.mark.parametrize("segs", [2, 4])
+def test_what_segments_leave_of_a_state(segs, monkeypatch):
+    """Segments that keep a ten-thousandth of what they find and write nothing: what is left is as exact as its exponent."""
+    from starter_b200 import ops
+
+    heads, n, width, tokens = 2, 72, 24, 110 * segs
+    gen = torch.Generator().manual_seed(segs)
+    qk = torch.randn(tokens, 2 * n, generator=gen).to(BF).cuda()
+    v, raw = torch.zeros(tokens, heads * width, dtype=BF).cuda(), (torch.rand(tokens, heads, generator=gen) - 2.2).to(BF).cuda()
+    A, bias = torch.tensor([-0.5, -0.6]), torch.zeros(heads)
+    start = torch.randn(1, heads * n * width, generator=gen).cuda()
+    monkeypatch.setattr(ops, "scan_one_walk", lambda *a: False)
+    monkeypatch.setattr(ops, "scan_segments", lambda *a: segs)
+    state = start.clone()
+    ops.state_scan("state_space", (qk, n), (qk, 0), (v, 0), (raw, 0), None, A.cuda(), bias.cuda(), None, state, 0, *packed([tokens], [0]),
+                   heads, 1, n, width)
+    x = A.to(F).exp() * bavedra.softplus(raw.cpu().to(F)).sum(dim=0)
+    assert 6.0 * segs < float(x.min()) < float(x.max()) < 14.0 * segs
+    left = state.cpu().to(F).view(heads, -1) / start.cpu().to(F).view(heads, -1) * x.exp()[:, None]
+    # the exponent's factors and their product round by up to 2^-23 of it each; the last segment's eight blocks, which keep a
+    # quarter, by 2^-23 of what they keep
+    assert float((left - 1.0).abs().max()) <= (3.0 * float(x.max()) + 8 * 4) * 2.0 ** -23
