@@ -56,7 +56,8 @@ bool as_word(PyObject* o, char kind, word& out) {
       }
     }
   }
-  PyObject* inner = PyObject_GetAttrString(o, "value");      // a ctypes number
+  // what stands for an integer (numpy's, a tensor of one), or a ctypes number
+  PyObject* inner = kind == 'i' && PyIndex_Check(o) ? PyNumber_Index(o) : PyObject_GetAttrString(o, "value");
   if (inner && (PyLong_Check(inner) || (kind == 'p' && inner == Py_None))) {
     const bool done = as_word(inner, kind, out);
     Py_DECREF(inner);
@@ -73,10 +74,14 @@ bool as_float(PyObject* o, double& out) {
   double v = PyFloat_AsDouble(o);
   if (v == -1.0 && PyErr_Occurred()) {
     PyErr_Clear();
-    PyObject* inner = PyObject_GetAttrString(o, "value");
+    PyObject* inner = PyObject_GetAttrString(o, "value");      // a ctypes number
     v = inner ? PyFloat_AsDouble(inner) : -1.0;
     Py_XDECREF(inner);
-    if (PyErr_Occurred()) return false;
+    if (PyErr_Occurred()) {
+      PyErr_Clear();
+      PyErr_Format(PyExc_TypeError, "a kernel's entry point takes a number here, not %s", Py_TYPE(o)->tp_name);
+      return false;
+    }
   }
   const float f = (float)v;
   word bits = 0;

@@ -177,6 +177,35 @@ def test_native_entry_points_take_their_declared_arguments():
             native.sb_scan_segment_floats(3, bad)
 
 
+def test_native_entry_points_take_what_stands_for_a_number():
+    """Sizes and factors that come as numpy's numbers, tensors of one, or objects with ``__index__``, as ctypes takes them."""
+    import ctypes
+
+    import torch
+
+    from starter_b200 import ops
+    from starter_b200.csrc import build
+
+    class Four:
+        def __index__(self):
+            return 4
+
+    native, plain = ops._lib("state_scan_prompt"), build.load("state_scan_prompt")
+    for four in (np.int64(4), np.int32(4), np.uint8(4), np.array(4), torch.tensor(4), torch.tensor([4]), Four(), True):
+        assert native.sb_scan_segment_floats(four, 64) == plain.sb_scan_segment_floats(four, 64)
+    for bad in (np.float32(4), torch.tensor(4.0), torch.tensor([1, 2]), 4.0):
+        with pytest.raises((TypeError, ctypes.ArgumentError)):
+            plain.sb_scan_segment_floats(bad, 64)
+        with pytest.raises(TypeError):
+            native.sb_scan_segment_floats(bad, 64)
+    # (no rows: the entry point returns before it looks further)
+    for eps in (np.float32(1e-6), np.float64(1e-6), torch.tensor(1e-6), 0, ctypes.c_float(1e-6)):
+        assert ops._lib("elementwise").sb_rmsnorm(0, 0, None, None, None, None, None, 0, 64, eps, None) == 0
+    for bad in (None, "1e-6", torch.zeros(2)):
+        with pytest.raises(TypeError):
+            ops._lib("elementwise").sb_rmsnorm(0, 0, None, None, None, None, None, 0, 64, bad, None)
+
+
 def test_native_checks_refuse_what_the_plain_ones_do():
     import torch
 
