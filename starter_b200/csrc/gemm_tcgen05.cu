@@ -17,7 +17,7 @@
 // With `gated`, w is [gate; up] stacked ([2 * n_out, k]); a tile holds 64 gate rows and the matching
 // 64 up rows and the epilogue writes round(silu(gate)) * up (fused.py:89-112).
 //
-// Grouped (routed experts of 5 to 64 rows an expert): the rows lie in the experts' order, whole tiles of BM to an expert, and the k-th
+// Grouped (routed experts of 7 to 63 rows an expert, to 255 with weights in front of the experts): the rows lie in the experts' order, whole tiles of BM to an expert, and the k-th
 // tile of rows takes its expert's weights.  An expert's weights are read once, its few rows ride along; the mma.sync tiles it
 // stands in for read them at a third of that rate (16 experts of 2 x 2,048 x 2,048, four a token, a whole layer: 32 tokens 172 ->
 // 88 us, 100 tokens 176 -> 94, 200 tokens 184 -> 106; the weights alone are 61 us of copy rate).

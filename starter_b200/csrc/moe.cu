@@ -1050,9 +1050,8 @@ int sb_moe_tile_rows(int dtype, int width, int inner) {
   return dtype == 1 && width % 16 == 0 && inner % 16 == 0 ? MOE_TC_BM : MOE_BM;
 }
 // The same for a step of `n_pairs` (row, expert) pairs over `experts` experts, where the caller does not take the grouped tcgen05
-// products (more than four rows an expert on average, moe_group_rows in ops.py; it leaves gated experts of odd inner sizes and
-// misaligned weights here): 8 up to six rows an expert (the few-row kernel), 128 from 128 (the large tiles pay for their padding
-// from there on), 256 from 256 (the grouped prompt product); else as above.
+// products (more than six rows an expert on average, moe_group_rows in ops.py; it leaves gated experts of odd inner sizes here):
+// 8 up to six rows an expert (the few-row kernel), 128 from 128 (the large tiles pay for their padding from there on), 256 from 256 (the grouped prompt product); else as above.
 int sb_moe_tile_rows_for(int dtype, int width, int inner, long long n_pairs, int experts) {
   const int rows = sb_moe_tile_rows(dtype, width, inner);
   if (rows != MOE_TC_BM) return rows;

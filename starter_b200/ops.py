@@ -1915,11 +1915,14 @@ def moe_group_rows(n_pairs: int, experts: int, weigh_input: bool) -> int:
     64: - / 93 / 92, 175; 100: - / 107 / 94 / 101, 176; 200: - / - / 121 / 106 / 117, 184; 300: - / - / - / 138 / 121, 306; 700: - / - / - /
     173 / 129, 448; 1,000: - / - / - / 216 / 147, 542.  The small ones read an expert's weights once and are bound by that; where more
     rows take several tiles, the weights come from L2 again and that is the bound, three times less of it with tiles of 256 by 256.
-    Smaller experts of few rows are faster on the kernel for single tokens, which needs no gathered rows (8 experts of 2 x 1,344 x
-    1,280, three rows each: 28.9 against 30.9; 32 of 1,280 x 1,536, two rows: 63.7 / 60.8): it serves up to four rows.
+    Up to six rows an expert the kernel for single tokens stays: its sums join by rounded additions every 32 entries, and through one
+    accumulator a layer of gated experts is 0.0038897 off the same in 64 bits in place of 0.0038858 (18 tokens; clamped, 20 tokens, 0.0036572 and
+    0.0036551; four seeds; beyond six rows the ``mma.sync`` tiles give the same bits as these products).  Smaller experts of few rows are
+    faster there too, because it needs no gathered rows (8 of 2 x 1,344 x 1,280, three rows each: 28.9 / 30.9; 32 of 1,280 x 1,536, two
+    rows: 63.7 / 60.8).
     A weight in front of an expert multiplies the products in float; the prompt product would round the rows, so it waits for 256."""
     rows = n_pairs / experts
-    if rows <= 4:
+    if rows <= 6:
         return 0
     if rows >= (256 if weigh_input else 64):
         return 256

@@ -83,7 +83,7 @@ def test_k_range_in_parts(splits, monkeypatch):
 def test_tile_heights_of_a_step():
     from starter_b200 import ops
 
-    for pairs, experts, weigh, rows in ((4, 16, False, 0), (64, 16, False, 0), (65, 16, False, 16), (208, 16, False, 16), (209, 16, False, 32),
+    for pairs, experts, weigh, rows in ((4, 16, False, 0), (96, 16, False, 0), (97, 16, False, 16), (208, 16, False, 16), (209, 16, False, 32),
                                         (448, 16, False, 32), (449, 16, False, 64), (1023, 16, False, 64), (1024, 16, False, 256),
                                         (1024, 16, True, 64), (1025, 16, True, 128), (4095, 16, True, 128), (4096, 16, True, 256)):
         assert ops.moe_group_rows(pairs, experts, weigh) == rows
