@@ -1706,13 +1706,23 @@ def latent_attention_step(qa, store, block_table, ctx, heads, rank, rot, scale, 
 
 
 #: up to this many tokens a step's latent queries and outputs are formed by the kernels for few rows (csrc/latent_heads.cu), whose
-#: blocks read a head's matrices again for every 16 tokens; beyond, by batched library products
+#: blocks read a head's matrices again for every 16 tokens; beyond, by batched library products.  Single tokens, whose keys are in
+#: parts that a merge kernel joins for the library products: up to 16 queries, 8 outputs
 LATENT_HEADS_TOKENS = 64
+LATENT_FOLD_SINGLE, LATENT_UNFOLD_SINGLE = 16, 8
 
 
-def latent_heads_take(q, dim, rot, rank, vdim) -> bool:
-    return (q.dtype == torch.bfloat16 and q.shape[0] <= LATENT_HEADS_TOKENS and
-            bool(_lib("latent_heads").sb_latent_heads_take(dim, rot, rank, vdim)))
+def latent_heads_take(q, dim, rot, rank, vdim, max_q_len=1) -> tuple:
+    """Whether ``latent_fold`` and ``latent_unfold`` form this step's latent queries and outputs.  Measured (us a layer of 16 heads, back to
+    back: both kernels / the first / neither): single tokens, rank 512, width 2,048: 4 sequences 35.7 / 36.9 / 40.3, 8 38.9 / 40.5 / 41.5, 10
+    43.1 / 41.0 / 43.0, 16 42.4 / 41.0 / 41.2, 17 46.7 / 43.7 / 45.1, 32 46.3 / 45.2 / 44.8, 64 58.7 / 57.3 / 57.4; rank 256, width 1,280: 8 28.7 /
+    30.8 / 32.8, 12 34.8 / 32.8 / 34.9, 17 36.9 / 35.1 / 34.9, 32 36.9 / 36.5 / 34.9; rank 512, width 1,024: 16 40.0 / 36.9 / 38.9, 20 44.2 / 43.1 /
+    41.1.  Prompts: one of 20 tokens 93.4 / 94.8 / 94.9, two of 31 79.9 / 79.9 / 80.3, rank 256 57.3 / 57.4 / 59.4."""
+    n = q.shape[0]
+    if (q.dtype != torch.bfloat16 or n > (LATENT_HEADS_TOKENS if max_q_len > 1 else LATENT_FOLD_SINGLE) or
+            not _lib("latent_heads").sb_latent_heads_take(dim, rot, rank, vdim)):
+        return False, False
+    return True, max_q_len > 1 or n <= LATENT_UNFOLD_SINGLE
 
 
 def latent_fold(q, uk, cos_table, sin_table, tok_pos, heads, dim, rot, rot_dims, rank, layout="interleaved"):

@@ -112,22 +112,23 @@ class LatentAttention(Part):
             if s.output_gate:
                 ops.sigmoid_gate(a, proj, s.q_rank)
             return ops.linear(a, self.o, status=ctx.status)
-        if ops.latent_heads_take(q, s.head_dim, s.rot_dim, s.kv_rank, s.value_dim):
-            keys = s.num_heads * s.head_dim
+        keys = s.num_heads * s.head_dim
+        fold, unfold = ops.latent_heads_take(q, s.head_dim, s.rot_dim, s.kv_rank, s.value_dim, ctx.max_q_len)
+        if fold:
             qa = ops.latent_fold(q, self.ukv[:keys], cos, sin, ctx.tok_pos, s.num_heads, s.head_dim, s.rot_dim, s.position.dims,
                                  s.kv_rank, layout=rotation.layout)
-            parts = ops.latent_attention_step(qa, store, cache.block_table, ctx, s.num_heads, s.kv_rank, s.rot_dim, s.scale, s.window,
-                                              self.sink, join=False)
-            a = ops.latent_unfold(parts, self.ukv[keys:], s.num_heads, s.value_dim, s.kv_rank, self.sink,
+        else:
+            qa = torch.empty((n, s.num_heads, self.row), dtype=q.dtype, device=q.device)
+            q3 = q.view(n, s.num_heads, s.head_dim + s.rot_dim)
+            torch.bmm(q3[:, :, : s.head_dim].transpose(0, 1), self.uk, out=qa[:, :, : s.kv_rank].transpose(0, 1))
+            ops.latent_rotate_q(q, qa, cos, sin, ctx.tok_pos, s.num_heads, s.head_dim, s.rot_dim, s.position.dims,
+                                s.kv_rank, layout=rotation.layout)
+        summed = ops.latent_attention_step(qa, store, cache.block_table, ctx, s.num_heads, s.kv_rank, s.rot_dim,
+                                           s.scale, s.window, self.sink, join=not unfold)
+        if unfold:
+            a = ops.latent_unfold(summed, self.ukv[keys:], s.num_heads, s.value_dim, s.kv_rank, self.sink,
                                   proj if s.output_gate else None, s.q_rank)
             return ops.linear(a, self.o, status=ctx.status)
-        qa = torch.empty((n, s.num_heads, self.row), dtype=q.dtype, device=q.device)
-        q3 = q.view(n, s.num_heads, s.head_dim + s.rot_dim)
-        torch.bmm(q3[:, :, : s.head_dim].transpose(0, 1), self.uk, out=qa[:, :, : s.kv_rank].transpose(0, 1))
-        ops.latent_rotate_q(q, qa, cos, sin, ctx.tok_pos, s.num_heads, s.head_dim, s.rot_dim, s.position.dims,
-                            s.kv_rank, layout=rotation.layout)
-        summed = ops.latent_attention_step(qa, store, cache.block_table, ctx, s.num_heads, s.kv_rank, s.rot_dim,
-                                           s.scale, s.window, self.sink)
         a = torch.empty((n, s.num_heads, s.value_dim), dtype=q.dtype, device=q.device)
         torch.bmm(summed.transpose(0, 1), self.uv, out=a.transpose(0, 1))
         a = a.view(n, s.num_heads * s.value_dim)

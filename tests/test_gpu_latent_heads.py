@@ -61,3 +61,44 @@ def test_unfold(n, parts, heads, rank, vdim, sink, gate):
     # the joined rows may round the other way (2^-8 of single terms), then two roundings of the result
     assert float((got - want).abs().max()) <= 2.0 ** -7 * float(want.abs().max())
     assert float((got - want).norm()) <= 2.0 ** -8 * float(want.norm())
+
+
+@pytest.mark.parametrize("seqs,new", [(3, 1), (9, 1), (17, 1), (2, 20)])
+def test_a_layer_by_either_form_of_its_products(seqs, new, monkeypatch):
+    """The head-wise kernels, each beside the library's form of the other, and neither: the same layer but for roundings."""
+    from types import SimpleNamespace
+
+    from starter_b200 import ops
+    from starter_b200.cache import SequenceCache
+    from starter_b200.config import spec as S
+    from starter_b200.engine.batch import plan_step
+    from starter_b200.parts import lookup
+
+    gen = torch.Generator().manual_seed(seqs)
+    spec = S.LatentAttentionSpec(256, 4, 64, 16, 32, 128, 128, 80 ** -0.5, 1e-6, S.InterleavedRopeSpec(16, 1e4), window=None, sink=True,
+                                 output_gate=True)
+    part = lookup("mixer", spec.kind)(spec, BF, lookup("position", spec.position.kind)(spec.position, BF, "cuda"))
+    part.set_params({name: (torch.randn(p.shape, generator=gen) * (p.shape[-1] ** -0.5 if len(p.shape) > 1 else 1.0))
+                     .to(torch.float32 if p.role != "matrix" else BF).cuda() for name, p in part.param_specs().items()})
+    cache = SequenceCache({0: part.kv_need()}, {0: None}, 128 * seqs, seqs, BF, "cuda")
+    slots = [cache.open_sequence() for _ in range(seqs)]
+    part.prepare(128)
+
+    def step(tokens):
+        arrays = plan_step([SimpleNamespace(slot=s, tokens=[0] * tokens, want=[]) for s in slots], [cache.lengths[s] for s in slots])
+        for s in slots:
+            cache.reserve(s, cache.lengths[s] + tokens)
+            cache.advance(s, tokens)
+        cache.sync_table()
+        return SimpleNamespace(host=arrays, n_seqs=seqs, max_q_len=tokens, max_kv_len=int(arrays["seq_kv_len"].max()), cache=cache,
+                               status=torch.zeros(1, dtype=torch.int32).cuda(), **{k: torch.from_numpy(v).cuda() for k, v in arrays.items()})
+
+    part(torch.randn(seqs * 70, 256, generator=gen).to(BF).cuda(), step(70), 0)
+    x, ctx, got = torch.randn(seqs * new, 256, generator=gen).to(BF).cuda(), step(new), {}
+    for form in ((False, False), (True, False), (False, True), (True, True)):
+        monkeypatch.setattr(ops, "latent_heads_take", lambda *a: form)
+        got[form] = part(x, ctx, 0).double()
+    want = got[(False, False)]
+    for form, y in got.items():
+        # a rounding of the queries, of the sums and of the outputs may fall the other way: 2^-8 of single terms each
+        assert bool(y.isfinite().all()) and float((y - want).norm()) <= 2.0 ** -7 * float(want.norm())

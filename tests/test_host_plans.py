@@ -241,3 +241,16 @@ def test_warps_are_whole_in_front_of_aligned_cluster_barriers():
                 barriers += 1
                 assert re.search(r"__sync(warp|threads)\(\);$", code[i - 1]), f"{name}: {code[i - 1]!r} in front of {line!r}"
     assert barriers >= 4
+
+
+def test_steps_whose_latent_products_are_for_few_rows():
+    """Both head-wise kernels up to 8 single tokens and 64 of prompts, the queries' alone up to 16 single tokens."""
+    import torch
+
+    from starter_b200 import ops
+
+    for n, longest, takes in ((1, 1, (True, True)), (8, 1, (True, True)), (9, 1, (True, False)), (16, 1, (True, False)), (17, 1, (False, False)),
+                              (64, 1, (False, False)), (9, 2, (True, True)), (64, 33, (True, True)), (65, 33, (False, False))):
+        assert ops.latent_heads_take(torch.empty(n, 8, dtype=torch.bfloat16), 128, 64, 512, 128, longest) == takes
+        assert ops.latent_heads_take(torch.empty(n, 8), 128, 64, 512, 128, longest) == (False, False)
+        assert ops.latent_heads_take(torch.empty(n, 8, dtype=torch.bfloat16), 120, 64, 512, 128, longest) == (False, False)
