@@ -252,12 +252,9 @@ int sb_latent_unfold(const void* summed, const float* part_acc, const float* par
   if (!sb_latent_heads_take(16, 8, rank, vdim) || n_parts < 1 || n_parts > LH_MAX_PARTS || heads > 65535) return -2;
   if (((uintptr_t)summed | (uintptr_t)part_acc | (uintptr_t)uv | (uintptr_t)out) & 15) return -2;
   const size_t smem = (size_t)((LH_OUT_COLS + LH_ROWS) * (rank + 8)) * sizeof(bf16);
-  static bool configured = false;
-  if (!configured) {
-    const cudaError_t err = cudaFuncSetAttribute(latent_unfold_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 64 * 1024);
-    if (err != cudaSuccess) return (int)err;
-    configured = true;
-  }
+  // (at every call, one limit for all sizes: the attribute is the current device's and other threads launch too)
+  const cudaError_t err = cudaFuncSetAttribute(latent_unfold_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 64 * 1024);
+  if (err != cudaSuccess) return (int)err;
   const int blocks = (vdim + LH_OUT_COLS - 1) / LH_OUT_COLS;
   const int shares = part_acc && blocks > 1 && blocks <= 8 ? blocks : 1;
   return launch_dependent_cluster(latent_unfold_kernel, dim3(blocks, heads, (n_tokens + LH_ROWS - 1) / LH_ROWS), dim3(256), smem, s,
