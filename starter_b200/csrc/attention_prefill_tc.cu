@@ -615,6 +615,28 @@ void sb_attention_prefill_tc_withhold(int step, unsigned long long limit_ns) {
   next_limit_ns = limit_ns ? limit_ns : WAIT_LIMIT_NS;
 }
 
+// How many clusters of `size` CTAs that take an SM each (the prompt attentions' blocks) the current device runs at once, or minus an
+// error.  A cluster lies inside one of the chip's processing clusters, whose SMs need not be a multiple of its size.
+int sb_prompt_clusters(int size) {
+  auto kernel = attention_prefill_tc_kernel<2, 2, 0>;
+  const int smem = (2 * 2 + 4 + TC_RING * 2) * 128 * 128 + 1024;
+  cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+  if (e != cudaSuccess) return -(int)e;
+  cudaLaunchAttribute attr[1];
+  attr[0].id = cudaLaunchAttributeClusterDimension;
+  attr[0].val.clusterDim.x = size;
+  attr[0].val.clusterDim.y = attr[0].val.clusterDim.z = 1;
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3(size);
+  cfg.blockDim = dim3(TC_THREADS);
+  cfg.dynamicSmemBytes = smem;
+  cfg.attrs = attr;
+  cfg.numAttrs = 1;
+  int n = 0;
+  e = cudaOccupancyMaxActiveClusters(&n, kernel, &cfg);
+  return e == cudaSuccess ? n : -(int)e;
+}
+
 // Same contract as sb_attention_prefill; n_tokens rows in q/out, n_pages pages in the stores.
 // list_of_blocks: tile_seq/tile_first list blocks of 256 queries (else tiles of 64, see the kernel).  splits: CTAs that share a block's
 // keys (1, 2, 4 or 8; 1 where keys of up to 64 entries have values of more).

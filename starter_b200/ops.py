@@ -635,18 +635,33 @@ def attention_prefill(q, k_store, v_store, block_table, seq_slot, seq_q_start, s
 PREFILL_TC_HEAD_DIMS = (64, 128)
 
 
+@functools.lru_cache(maxsize=None)
+def _prompt_clusters(size: int, device: int) -> int:
+    got = _lib("attention_prefill_tc").sb_prompt_clusters(size)
+    if got < 0:
+        raise KernelError(f"the device does not say how many clusters of {size} it runs at once (CUDA error {-got})")
+    return got
+
+
+def prompt_clusters(size: int) -> int:
+    """How many clusters of ``size`` CTAs of the prompt attentions, which take an SM each, the current device runs at once."""
+    return _prompt_clusters(size, torch.cuda.current_device())
+
+
 def prompt_splits(blocks: int, keys: int, window=None, from_keys: int = 1100) -> int:
     """How many CTAs share the keys of a block of 256 queries (one cluster, csrc/attention_tc.cuh) in a step of ``blocks`` blocks of
-    up to ``keys`` keys: 4 or 2, as long as all are resident at once, from ``from_keys`` keys that a block walks (the cluster's
+    up to ``keys`` keys: 4 or 2, as long as the clusters run at once, from ``from_keys`` keys that a block walks (the cluster's
     launch, two barriers and the merge cost 3 us, a step of 128 keys saved 1.3).  Measured (us, one CTA / 2 / 4): plain attention,
     300 tokens behind 1,000 24.6 / 22.0 / 20.9, 700 behind 1,200 33.0 / 27.2, 1,000 tokens 20.5 / 20.0, 700 tokens 16.7 / 18.0; latent
     attention, 700 behind 1,200 60.1 / 48.6, 1,000 tokens 38.0 / 36.2, 600 tokens 27.6 / 28.8; capped scores, whose steps take three times
-    as long, 500 tokens 19.9 / 19.5 / 17.0, 1,000 tokens 31.0 / 25.8, 233 tokens twice 18.8 / 21.0 / 17.4.  Eight are slower throughout."""
+    as long, 500 tokens 19.9 / 19.5 / 17.0, 1,000 tokens 31.0 / 25.8, 233 tokens twice 18.8 / 21.0 / 17.4.  Eight are slower throughout.
+    A B200 of 148 SMs runs 33 clusters of four, not 37: 256 queries behind 1,400 keys in 33 blocks 30.5 / 24.7 / 22.5, in 34 29.8 / 24.5 /
+    41.2, in 37 30.1 / 24.6 / 41.7, in 74 30.7 / 26.2; over formed keys 33 61.3 / 49.9 / 44.5, 34 58.8 / 47.9 / 63.0."""
     if window:
         keys = min(keys, window + 256)
-    if keys < from_keys:
+    if keys < from_keys or 2 * blocks > SM_COUNT:
         return 1
-    return 4 if 4 * blocks <= SM_COUNT else 2 if 2 * blocks <= SM_COUNT else 1
+    return next((parts for parts in (4, 2) if blocks <= prompt_clusters(parts)), 1)
 
 
 DECODE_CLUSTER_SPLITS = 8

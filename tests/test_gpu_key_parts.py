@@ -146,3 +146,16 @@ def test_parts_of_a_step():
         parts = ops.prompt_splits(blocks, keys, window, least)
         assert parts in (1, 2, 4) and (parts == 1 or parts * blocks <= 148)
         assert (parts > 1) == (blocks <= 74 and min(keys, window + 256 if window else keys) >= least)
+
+
+def test_clusters_that_share_keys_run_at_once(monkeypatch):
+    """No step gets more clusters than the device holds: those left over would walk behind the others."""
+    from starter_b200 import ops
+
+    fours, pairs = ops.prompt_clusters(4), ops.prompt_clusters(2)
+    assert 1 <= fours <= 37 and fours <= pairs <= 74
+    for blocks in range(1, 80):
+        parts = ops.prompt_splits(blocks, 5000)
+        assert parts == (4 if blocks <= fours else 2 if blocks <= pairs else 1)
+    monkeypatch.setattr(ops, "prompt_clusters", lambda size: {4: 30, 2: 70}[size])
+    assert [ops.prompt_splits(n, 5000) for n in (30, 31, 70, 71, 75)] == [4, 2, 2, 1, 1]
