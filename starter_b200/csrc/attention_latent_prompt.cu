@@ -412,7 +412,7 @@ static int lp_launch(const CUtensorMap& mq, const CUtensorMap& mkv, const CUtens
   const int smem = 2 * (DC + 1) * 128 * 128 + 2 * 128 * 128 + 2 * (DC + 1 + VC) * 64 * 128 + 1024;
   cudaError_t err = cudaFuncSetAttribute(latent_prompt_kernel<DC, VC>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
   if (err != cudaSuccess) return (int)err;
-  if (splits < 1 || splits > 8 || (splits & (splits - 1)) || (DC == 1 && VC == 2)) splits = 1;
+  splits = DC == 1 && VC == 2 ? 1 : splits >= 4 ? 4 : splits >= 2 ? 2 : 1;
   return launch_dependent_cluster(latent_prompt_kernel<DC, VC>, dim3(heads * splits, n_blocks), dim3(LP_THREADS), smem, s, dim3(splits),
                                   mq, mkv, mr, (bf16*)out, seq_q_start, seq_q_len, seq_kv_len, block_seq, block_first, heads,
                                   scale * 1.4426950408889634f, window, sink, status, withhold, splits);

@@ -594,7 +594,7 @@ static int launch(const CUtensorMap& mq, const CUtensorMap& mk, const CUtensorMa
     if (e != cudaSuccess) return (int)e;
     configured = true;
   }
-  if (splits < 1 || splits > 8 || (splits & (splits - 1)) || (DC == 1 && VC == 2)) splits = 1;
+  splits = DC == 1 && VC == 2 ? 1 : splits >= 4 ? 4 : splits >= 2 ? 2 : 1;
   return launch_dependent_cluster(attention_prefill_tc_kernel<DC, VC, EXT>, dim3(heads * splits, n_tiles), dim3(TC_THREADS), smem, s,
                                   dim3(splits), mq, mk, mv, (bf16*)out, block_table, table_stride, seq_slot, seq_q_start, seq_q_len,
                                   seq_kv_len, tile_seq, tile_first, heads, kv_heads, scale * 1.4426950408889634f, window, status,
@@ -639,7 +639,7 @@ int sb_prompt_clusters(int size) {
 
 // Same contract as sb_attention_prefill; n_tokens rows in q/out, n_pages pages in the stores.
 // list_of_blocks: tile_seq/tile_first list blocks of 256 queries (else tiles of 64, see the kernel).  splits: CTAs that share a block's
-// keys (1, 2, 4 or 8; 1 where keys of up to 64 entries have values of more).
+// keys (1, 2 or 4; 1 where keys of up to 64 entries have values of more).
 // head_dim must be 64 or 128 (returns -2 otherwise).
 int sb_attention_prefill_tc(const void* q, void* out, const void* k_store, const void* v_store,
                             const int* block_table, int table_stride, const int* seq_slot,

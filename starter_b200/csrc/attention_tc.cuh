@@ -218,9 +218,9 @@ __device__ __forceinline__ void merge_parts(uint8_t* q_sm, uint8_t* p_sm, float2
     const int row = rank * share + n, t = row / TC_BQ, r = row % TC_BQ;
     if (row >= rows_valid) return;
     float top = -INFINITY;
-    float2 part[8];
+    float2 part[4];
 #pragma unroll
-    for (int p = 0; p < 8; ++p) {
+    for (int p = 0; p < 4; ++p) {
       part[p] = p < splits ? peer_load2(peer_u32(ml + t * TC_BQ + r, p)) : make_float2(-INFINITY, 0.f);
       if (part[p].y != 0.f) top = fmaxf(top, part[p].x);
     }
@@ -228,7 +228,7 @@ __device__ __forceinline__ void merge_parts(uint8_t* q_sm, uint8_t* p_sm, float2
     const float* a = part_piece<PC, COLS>(p_sm + t * P_BYTES, q_sm + t * Q_BYTES, r, c / 4);
     const float* b = part_piece<PC, COLS>(p_sm + t * P_BYTES, q_sm + t * Q_BYTES, r, c / 4 + 1);
 #pragma unroll
-    for (int p = 0; p < 8; ++p) {
+    for (int p = 0; p < 4; ++p) {
       // (a part without keys filed nothing; one whose sum is no number has a score that is none, which is the row's result)
       if (p >= splits || part[p].y == 0.f) continue;
       const float w = fast_exp2(part[p].x - top);

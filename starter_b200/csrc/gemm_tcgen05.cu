@@ -458,7 +458,6 @@ int sb_gemm_tcgen05_grouped(const void* x, const void* w, void* out, int n_out, 
     case 32: return launch<32, G, true>(map_w, map_x, args, tiles, max_tiles, s, group);   \
     case 64: return launch<64, G, true>(map_w, map_x, args, tiles, max_tiles, s, group);   \
     case 128: return launch<128, G, true>(map_w, map_x, args, tiles, max_tiles, s, group); \
-    case 256: return launch<256, G, true>(map_w, map_x, args, tiles, max_tiles, s, group); \
     default: return -2;                                                                  \
   }
   if (gated) { BY_TILE(true) }

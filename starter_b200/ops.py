@@ -77,10 +77,6 @@ def _code(dtype) -> int:
     return _DT[dtype]
 
 
-def _ptr(t):
-    return t.data_ptr() if t is not None else None
-
-
 def _refuse(t, name, dtype=None, ndim=None):
     """What is wrong with an operand that is no contiguous CUDA tensor of this type and number of dimensions."""
     if not isinstance(t, torch.Tensor) or not t.is_cuda:

@@ -34,11 +34,11 @@ def same(monkeypatch, run, status):
     from starter_b200 import ops
 
     got = {}
-    for parts in (1, 2, 4, 8):
+    for parts in (1, 2, 4):
         monkeypatch.setattr(ops, "prompt_splits", lambda *a, **k: parts)
         got[parts] = run().float()
     assert int(status.item()) == 0 and bool(torch.isfinite(got[1]).all())
-    for parts in (2, 4, 8):
+    for parts in (2, 4):
         assert float((got[parts] - got[1]).abs().max()) <= 2.0 ** -7 * float(got[1].abs().max())
         assert float((got[parts] - got[1]).norm()) <= 2.0 ** -8 * float(got[1].norm())
         if parts > 2:

@@ -82,8 +82,8 @@ def test_many_tokens_a_sequence(mode, heads, groups, n, width, monkeypatch):
             decay=decay[pick.cpu()].cuda().contiguous() if decay is not None else None)
 
     assert ops._lib("state_scan_prompt").sb_scan_prompt_floats(
-        1, ops.SCAN_MODES[mode], ops._at(qk, 8), qk.shape[1], ops._at(qk, 8 + groups * n), qk.shape[1], ops._ptr(v), v.shape[1],
-        ops._ptr(None), heads, groups, n, width) >= 0
+        1, ops.SCAN_MODES[mode], ops._at(qk, 8), qk.shape[1], ops._at(qk, 8 + groups * n), qk.shape[1], v, v.shape[1],
+        None, heads, groups, n, width) >= 0
     everything = torch.arange(total).cuda()
     got = run(everything, lengths, slots)
     kept = state.clone()
