@@ -55,7 +55,8 @@ __device__ __forceinline__ uint32_t pack_exact_bf16(float lo, float hi) {
 __device__ __forceinline__ float gate_clamped(float g, float u, float limit) {
   g = fminf(g, limit);
   u = fminf(fmaxf(u, -limit), limit);
-  return __fdividef(g, 1.f + __expf(-1.702f * g)) * (u + 1.f);
+  // (both sides of the quotient by a quarter: the fast one is zero for divisors above 2^126, which gates of -51.4 to -52.1 have)
+  return __fdividef(0.25f * g, fmaf(0.25f, __expf(-1.702f * g), 0.25f)) * (u + 1.f);
 }
 __device__ __forceinline__ float gate_act_fast(float g, int act) {
   const float z = act == SB_ACT_GELU_TANH ? -1.5957691216057308f * (g + 0.044715f * g * g * g) : -g;

@@ -362,10 +362,13 @@ __global__ void gated_clamped_kernel(const T* __restrict__ gu, T* __restrict__ a
   for (; i < total; i += stride) {
     const size_t row = i / inner;
     const int col = (int)(i - row * inner);
-    const float g = fminf(to_f<T>(gu[row * 2 * inner + col]), limit);
-    const float u = fminf(fmaxf(to_f<T>(gu[row * 2 * inner + inner + col]), -limit), limit);
-    act[i] = from_f<T>(sizeof(T) == 2 ? __fdividef(g, 1.f + __expf(-1.702f * g)) * (u + 1.f)      // as the products' epilogue
-                                      : g / (1.f + expf(-1.702f * g)) * (u + 1.f));
+    const float g = to_f<T>(gu[row * 2 * inner + col]), u = to_f<T>(gu[row * 2 * inner + inner + col]);
+    if constexpr (sizeof(T) == 2) {
+      act[i] = from_f<T>(gate_clamped(g, u, limit));            // as the products' epilogue
+    } else {
+      const float a = fminf(g, limit);
+      act[i] = from_f<T>(a / (1.f + expf(-1.702f * a)) * (fminf(fmaxf(u, -limit), limit) + 1.f));
+    }
   }
 }
 

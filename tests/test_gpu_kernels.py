@@ -609,6 +609,30 @@ def test_the_prompt_product_gates_every_value():
     assert bool(((got == want) | (v < -88.6) & (got.double().abs() < 2e-37)).all())
 
 
+@pytest.mark.parametrize("form", ["many rows", "few rows", "by itself", "experts"])
+def test_the_clamped_gate_takes_every_value(form):
+    """Every finite bfloat16 gate, times one: min(g, 7) sigmoid(1.702 min(g, 7)) to its last place, down to where its exponential
+    leaves the float range."""
+    from starter_b200 import ops
+
+    gates = torch.arange(65536, dtype=torch.int32).to(torch.int16).view(torch.bfloat16)
+    gates = torch.where(gates.isfinite(), gates, torch.zeros_like(gates)).view(1024, 64)
+    w = torch.zeros(128, 64)
+    w[:64] = torch.eye(64)
+    if form == "by itself":
+        got = ops.gated_clamped(dev(torch.cat([gates, torch.zeros_like(gates)], dim=1)), 7.0)
+    elif form == "experts":
+        ids, one = torch.zeros(1024, 1, dtype=torch.int32), torch.ones(1024, 1)
+        got = ops.moe_experts(dev(gates), dev(ids), dev(one), dev(w[None].to(torch.bfloat16)), dev(torch.eye(64)[None].to(torch.bfloat16)), 7.0)
+    else:
+        step = 1024 if form == "many rows" else 64
+        got = torch.cat([ops.linear_gated_clamped(dev(x.contiguous()), dev(w.to(torch.bfloat16)), 7.0) for x in gates.split(step)])
+    v = gates.double().clamp(max=7.0)
+    want = v * torch.sigmoid(1.702 * v)
+    # (a value beside the middle of two may round the other way)
+    assert bool(((got.cpu().double() - want).abs() <= torch.where(v < -52.0, 2e-37, 2.0 ** -8 * want.abs() + 1e-38)).all())
+
+
 @pytest.mark.parametrize("rows,n,k,gated,kblock", [(256, 256, 512, False, 0), (600, 384, 1024, True, 3)])
 def test_a_wait_in_the_prompt_product_that_runs_out_is_reported(rows, n, k, gated, kblock):
     """One weight copy of every first CTA is left out on purpose (an entry point made for this): the
