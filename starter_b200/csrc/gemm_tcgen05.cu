@@ -431,9 +431,9 @@ static int gemm_entry(const void* x, const void* w, void* out, int rows, int n_o
 // The same over experts: x [max_tiles * bm, k_dim] in the experts' order (moe.cu's align and gather), w [experts, n_out (2 * n_out
 // with up 1), k_dim]; up 1: out [max_tiles * bm, n_out] is the gated activation (limit > 0: the clamped one), up 2: the squared relu, up
 // 0: out [pairs, n_out], a row's product where its pair belongs.  n_out a multiple of 64 with up 1.
-int sb_gemm_tcgen05_grouped(const void* x, const void* w, void* out, int n_out, int k_dim, int experts, int bm, int splits, int stages,
-                            int up, float limit, const int* tile_expert, const int* n_tiles, int max_tiles, const int* sorted,
-                            const float* in_scale, int* status, cudaStream_t s) {
+static int grouped_entry(const void* x, const void* w, void* out, int n_out, int k_dim, int experts, int bm, int splits, int stages, int up,
+                         float limit, const int* tile_expert, const int* n_tiles, int max_tiles, const int* sorted,
+                         const float* in_scale, int* status, unsigned long long wait_limit_ns, int withhold_stage, cudaStream_t s) {
   if (max_tiles == 0 || n_out == 0) return 0;
   if (k_dim % 8 || k_dim <= 0 || splits < 1 || splits > GEMM_MAX_SPLITS || stages < 2 || stages > GEMM_MAX_STAGES) return -2;
   if ((((uintptr_t)x | (uintptr_t)w) & 15) || up < 0 || up > 2 || (up == 1 && n_out % 64) || max_tiles > 65535) return -2;
@@ -448,7 +448,7 @@ int sb_gemm_tcgen05_grouped(const void* x, const void* w, void* out, int n_out, 
   args.out = out; args.status = status;
   args.rows = max_tiles * bm; args.n_out = n_out; args.k_dim = k_dim;
   args.splits = splits; args.stages = stages; args.gated = gated; args.out_float = 0;
-  args.wait_limit_ns = WAIT_LIMIT_NS; args.withhold_stage = -1;
+  args.wait_limit_ns = wait_limit_ns; args.withhold_stage = withhold_stage;
   args.limit = limit;
   const GroupArgs group{tile_expert, n_tiles, sorted, in_scale, up};
   const int tiles = gated ? n_out / 64 : (n_out + TILE_N - 1) / TILE_N;
@@ -463,6 +463,23 @@ int sb_gemm_tcgen05_grouped(const void* x, const void* w, void* out, int n_out, 
   if (gated) { BY_TILE(true) }
   BY_TILE(false)
 #undef BY_TILE
+}
+
+int sb_gemm_tcgen05_grouped(const void* x, const void* w, void* out, int n_out, int k_dim, int experts, int bm, int splits, int stages,
+                            int up, float limit, const int* tile_expert, const int* n_tiles, int max_tiles, const int* sorted,
+                            const float* in_scale, int* status, cudaStream_t s) {
+  return grouped_entry(x, w, out, n_out, k_dim, experts, bm, splits, stages, up, limit, tile_expert, n_tiles, max_tiles, sorted, in_scale,
+                       status, WAIT_LIMIT_NS, -1, s);
+}
+
+// The same with the rows of k-block `withhold_stage` of every block's range left out on purpose, for tests of the give-up path.
+int sb_gemm_tcgen05_grouped_withheld(const void* x, const void* w, void* out, int n_out, int k_dim, int experts, int bm, int splits,
+                                     int stages, int up, float limit, const int* tile_expert, const int* n_tiles, int max_tiles,
+                                     const int* sorted, const float* in_scale, int* status, unsigned long long wait_limit_ns,
+                                     int withhold_stage, cudaStream_t s) {
+  if (withhold_stage < 0 || withhold_stage >= stages || wait_limit_ns == 0) return -2;
+  return grouped_entry(x, w, out, n_out, k_dim, experts, bm, splits, stages, up, limit, tile_expert, n_tiles, max_tiles, sorted, in_scale,
+                       status, wait_limit_ns, withhold_stage, s);
 }
 
 int sb_gemm_tcgen05(const void* x, const void* w, void* out, int rows, int n_out, int k_dim, int bm,

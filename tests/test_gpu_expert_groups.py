@@ -115,3 +115,31 @@ def test_pairs_are_dealt_to_tiles(pairs, experts):
         n = int(counts[expert])
         assert sorted(mine[:n].tolist()) == (ids == expert).nonzero().flatten().tolist()
         assert (mine[n:] == -1).all()
+
+
+@pytest.mark.parametrize("rows,splits,stage", [(16, 1, 0), (32, 4, 1), (128, 2, 2)])
+def test_a_wait_in_the_grouped_product_that_runs_out_is_reported(rows, splits, stage, monkeypatch):
+    """The rows of one k-block of every block are left out on purpose (an entry point made for this): the wait on them gives up after
+    2 ms, the kernel returns, bit 4 of the status word is set; the same layer without the gap is right afterwards."""
+    from starter_b200 import ops
+
+    gen = torch.Generator().manual_seed(rows)
+    experts, width, inner, tokens = 3, 1024, 768, 70
+    ids = torch.randint(0, experts, (tokens, 1), generator=gen).to(torch.int32).cuda()
+    h = torch.randn(tokens, width, generator=gen).to(BF).cuda()
+    gate_up = (torch.randn(experts, 2 * inner, width, generator=gen) * 2.0 * width ** -0.5).to(BF).cuda()
+    down = (torch.randn(experts, width, inner, generator=gen) * inner ** -0.5).to(BF).cuda()
+    weights, status, lib = torch.ones(tokens, 1).cuda(), torch.zeros(1, dtype=torch.int32, device="cuda"), ops._lib("gemm_tcgen05")
+    monkeypatch.setattr(ops, "moe_group_rows", lambda *a: rows)
+    monkeypatch.setattr(ops, "_moe_group_plan", lambda *a: (splits, 3))
+
+    def run():
+        return ops.moe_experts(h, ids, weights, gate_up, down, expert="gated_silu", status=status).double()
+
+    with monkeypatch.context() as m:
+        m.setattr(lib, "sb_gemm_tcgen05_grouped", lambda *a: lib.sb_gemm_tcgen05_grouped_withheld(*a[:-1], 2_000_000, stage, a[-1]))
+        run()
+        assert status.item() == 4
+    status.zero_()
+    want = plain(h, ids, weights, gate_up, down, "gated_silu", 0.0, inner, False)
+    assert float((run() - want).norm()) <= 2.0 ** -8 * float(want.norm()) and status.item() == 0

@@ -159,3 +159,39 @@ def test_clusters_that_share_keys_run_at_once(monkeypatch):
         assert parts == (4 if blocks <= fours else 2 if blocks <= pairs else 1)
     monkeypatch.setattr(ops, "prompt_clusters", lambda size: {4: 30, 2: 70}[size])
     assert [ops.prompt_splits(n, 5000) for n in (30, 31, 70, 71, 75)] == [4, 2, 2, 1, 1]
+
+
+@pytest.mark.parametrize("kind", ["plain", "formed"])
+@pytest.mark.parametrize("parts,left_out", [(2, 0), (4, 0), (4, 6)])
+def test_a_wait_in_a_part_that_runs_out_is_reported(kind, parts, left_out, monkeypatch):
+    """Values of one step are left out on purpose, which one part of a block waits for: it gives up after 2 ms, meets the others at the
+    cluster's barriers, every block returns and bit 16 of the status word is set; the same call is right afterwards."""
+    from starter_b200 import ops
+
+    heads, dim, rank = 2, 128, 128
+    gen, table, (keys, values), ctx = step(1, rank + 64, 16, 9) if kind == "formed" else step(1, dim, dim, 9)
+    q = torch.randn(sum(LENGTHS), heads * (dim + 64 if kind == "formed" else dim), generator=gen).to(BF).cuda()
+    ukv = (torch.randn(heads * 2 * dim, rank, generator=gen) * rank ** -0.5).to(BF).cuda()
+
+    def run(withhold=None):
+        if kind == "formed":
+            return ops.latent_attention_prompt(q, ukv, keys, table, ctx, heads, dim, dim, rank, 64, (dim + 64) ** -0.5, None, None).float()
+        return ops.attention_prefill(q, keys, values, table, ctx.seq_slot, ctx.seq_q_start, ctx.seq_q_len, ctx.seq_kv_len, ctx.tile_seq,
+                                     ctx.tile_first, heads, 1, dim, dim ** -0.5, status=ctx.status, kernel="tcgen05",
+                                     max_q_len=ctx.max_q_len, blocks=(ctx.block_seq, ctx.block_first), withhold=withhold,
+                                     kv_hint=ctx.max_kv_len).float()
+
+    monkeypatch.setattr(ops, "prompt_splits", lambda *a, **k: 1)
+    want = run()
+    monkeypatch.setattr(ops, "prompt_splits", lambda *a, **k: parts)
+    if kind == "formed":
+        lib = ops._lib("attention_latent_prompt")
+        with monkeypatch.context() as m:
+            m.setattr(lib, "sb_latent_prompt", lambda *a: lib.sb_latent_prompt_withheld(*a[:-1], left_out, 2_000_000, a[-1]))
+            run()
+    else:
+        run((left_out, 2_000_000))
+    assert ctx.status.item() == 16
+    ctx.status.zero_()
+    got = run()
+    assert ctx.status.item() == 0 and float((got - want).abs().max()) <= 2.0 ** -7 * float(want.abs().max())
