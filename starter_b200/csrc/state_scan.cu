@@ -88,7 +88,8 @@ state_scan_kernel(const T* __restrict__ q, int ldq, const T* __restrict__ k, int
   // (rows of the output tile are padded so that the lanes of a column may file one token each without a conflict)
   constexpr int OS_LD = SCAN_COLS + 32 / P;
   float (*os)[OS_LD] = reinterpret_cast<float (*)[OS_LD]>(scan_smem + 2 * sizeof(Buffer));
-  // (launch_dependents comes at this kernel's end, not its start: a long prompt keeps its blocks for a while)
+  // (early: the norm behind it has small blocks and waits; layers in float32, two sequences of 600 tokens: 614.8 -> 612.8 us, single
+  // tokens in bfloat16 20.5 -> 18.5)
   pdl_trigger();
   pdl_wait();
   SB_BEHIND_WAIT(q);

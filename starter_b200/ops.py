@@ -1941,7 +1941,9 @@ def moe_group_rows(n_pairs: int, experts: int, weigh_input: bool) -> int:
     0.0036551; four seeds; beyond six rows the ``mma.sync`` tiles give the same bits as these products).  Smaller experts of few rows are
     faster there too, because it needs no gathered rows (8 of 2 x 1,344 x 1,280, three rows each: 28.9 / 30.9; 32 of 1,280 x 1,536, two
     rows: 63.7 / 60.8).
-    A weight in front of an expert multiplies the products in float; the prompt product would round the rows, so it waits for 256."""
+    A weight in front of an expert multiplies the products in float; the prompt product would round the rows, so it waits for 256 and
+    tiles of 128 serve from 65 (``mma.sync`` tiles / these: 66 rows 253 / 113, 128 337 / 153, 200 441 / 184, 254 539 / 230; 8 experts of
+    2 x 1,280 x 1,408 66 87 / 48, 254 167 / 95; 32 squared ones of 1,600 x 1,536 66 195 / 143, 254 331 / 281)."""
     rows = n_pairs / experts
     if rows <= 6:
         return 0
@@ -2012,10 +2014,12 @@ def moe_experts(h, ids, weights, gate_up, down, limit=0.0, expert="gated_clamped
         if tile_rows not in (4, 8, 32, 64, 128, 256) or (tile_rows != 32 and lib.sb_moe_tile_rows(_code(h.dtype), width, inner) != 64):
             raise KernelError(f"no expert tiles of {tile_rows} rows for {h.dtype}, width {width}, inner size {inner}")
         bm = 8 if tile_rows == 4 else int(tile_rows)
-    few = False
-    if tile_rows is None and lib.sb_moe_tile_rows(_code(h.dtype), width, inner) == 64:
+    few, cores = False, lib.sb_moe_tile_rows(_code(h.dtype), width, inner) == 64
+    if cores and bm != 32 and (h.data_ptr() | gate_up.data_ptr() | down.data_ptr()) % 16:
+        raise KernelError("rows and expert weights of the tensor-core tiles must be 16-byte aligned")
+    if tile_rows is None and cores:
         group = moe_group_rows(n_pairs, experts, weigh_input)
-        if group and not (up_mode == 1 and inner % 64 and group < 256) and not (gate_up.data_ptr() | down.data_ptr()) % 16:
+        if group and not (up_mode == 1 and inner % 64 and group < 256):
             bm, few = group, group < 256
     max_tiles = -(-n_pairs // bm) + min(experts, n_pairs)
     capacity = max_tiles * bm

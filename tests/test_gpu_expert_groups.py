@@ -143,3 +143,21 @@ def test_a_wait_in_the_grouped_product_that_runs_out_is_reported(rows, splits, s
     status.zero_()
     want = plain(h, ids, weights, gate_up, down, "gated_silu", 0.0, inner, False)
     assert float((run() - want).norm()) <= 2.0 ** -8 * float(want.norm()) and status.item() == 0
+
+
+@pytest.mark.parametrize("tokens", [3, 70, 200])
+@pytest.mark.parametrize("which", ["h", "gate_up", "down"])
+def test_operands_off_their_alignment_are_refused(tokens, which):
+    from starter_b200 import ops
+
+    def made(*shape, off):
+        size = 1
+        for n in shape:
+            size *= n
+        return torch.zeros(size + 8, dtype=BF, device="cuda")[int(off):int(off) + size].view(*shape)
+
+    h, gate_up, down = (made(*shape, off=which == name) for name, shape in (("h", (tokens, 64)), ("gate_up", (2, 128, 64)), ("down", (2, 64, 64))))
+    ids, weights = torch.zeros(tokens, 1, dtype=torch.int32, device="cuda"), torch.ones(tokens, 1, device="cuda")
+    with pytest.raises(ops.KernelError, match="16-byte aligned"):
+        ops.moe_experts(h, ids, weights, gate_up, down, expert="gated_silu")
+    assert bool((ops.moe_experts(h, ids, weights, gate_up, down, expert="gated_silu", tile_rows=32) == 0).all())
