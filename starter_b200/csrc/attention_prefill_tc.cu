@@ -66,7 +66,7 @@ struct TcExtras {
 };
 
 // EXT 0: plain; 1: the extras without the cap; 2: all of them.
-template <int DC, int VC, int EXT>
+template <int DC, int VC, int EXT, bool PARTS>
 __global__ void __launch_bounds__(TC_THREADS, 1)
 attention_prefill_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant__ CUtensorMap map_k,
                             const __grid_constant__ CUtensorMap map_v, bf16* __restrict__ out,
@@ -95,7 +95,7 @@ attention_prefill_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __g
   float2 row_state = make_float2(-INFINITY, 0.f);   // keys in parts: a row's reference and sum
 
   // heads run fastest: the work list's order holds; the CTAs of a cluster share a head's block
-  const int tile = blockIdx.y, head = blockIdx.x / splits, part = blockIdx.x - head * splits;
+  const int tile = blockIdx.y, head = PARTS ? blockIdx.x / splits : blockIdx.x, part = PARTS ? blockIdx.x - head * splits : 0;
   const int q_first = tile_first[tile];
   // the work list is either this kernel's own (one entry per block of 256 queries) or the common
   // one in tiles of 64 queries, of which every fourth starts a block
@@ -122,7 +122,7 @@ attention_prefill_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __g
   n_tile[0] = ((pos0 + min(rows_valid, TC_BQ) - 1) / SB_PAGE_TOKENS - page_lo + kept) / 2 + 1;
   n_tile[1] = rows_valid > TC_BQ ? (page_hi - page_lo + kept) / 2 + 1 : 0;
   int n_steps = max(n_tile[0], n_tile[1]), first_step = 0;
-  if (splits > 1) {                                 // this CTA's steps
+  if constexpr (PARTS) {                            // this CTA's steps
     const int per = (n_steps + splits - 1) / splits;
     first_step = part * per;
     for (int t = 0; t < 2; ++t) n_tile[t] = max(0, min(per, n_tile[t] - first_step));
@@ -158,7 +158,7 @@ attention_prefill_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __g
       const bool elected = elect_one();
       pdl_wait();
       const int q_row0 = seq_q_start[seq] + q_first;
-      const int q_tiles = n_tile[1] ? 2 : n_steps > 0 ? 1 : 0;
+      const int q_tiles = n_tile[1] ? 2 : !PARTS || n_steps > 0 ? 1 : 0;
       if (elected && q_tiles) mbar_expect_tx(&q_full, q_tiles * Q_BYTES);
       for (int t = 0; t < q_tiles; ++t)
         for (int c = 0; c < DC; ++c)
@@ -180,7 +180,7 @@ attention_prefill_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __g
         return true;
       };
       int loads[3] = {0, 0, 0};                        // per buffer: how many copies were started
-      bool ok = n_steps > 0 && load(false, 0);
+      bool ok = (!PARTS || n_steps > 0) && load(false, 0);
       if (ok) { loads[0]++; ok = load(true, 0); }
       if (ok) loads[2]++;
       if (ok && n_steps > 1) { ok = load(false, 1); if (ok) loads[1]++; }
@@ -504,22 +504,20 @@ attention_prefill_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __g
       if (lane == 0) mbar_arrive(&p_ready[t]);
     }
     if (ok && n_mine > 0) ok = mbar_wait(&o_ready[t], (n_mine - 1) & 1, abort);
-    if (splits > 1) {
-      if constexpr (DC == 2 || VC == 1) {
-        if (n_mine > 0) row_state = make_float2(m_ref, l_run);
-        if (ok && n_mine > 0) {
-          asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+    if constexpr (PARTS) {
+      if (n_mine > 0) row_state = make_float2(m_ref, l_run);
+      if (ok && n_mine > 0) {
+        asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
 #pragma unroll 1
-          for (int c = 0; c < VC * 64; c += 32) {
-            float ov[32];
-            tmem_load32(tmem_o + c, ov);
+        for (int c = 0; c < VC * 64; c += 32) {
+          float ov[32];
+          tmem_load32(tmem_o + c, ov);
 #pragma unroll
-            for (int d = 0; d < 32; d += 4)
-              *reinterpret_cast<float4*>(part_piece<64, VC * 64>(p_sm + t * P_BYTES, q_sm + t * Q_BYTES, r, (c + d) / 4)) =
-                  make_float4(ov[d], ov[d + 1], ov[d + 2], ov[d + 3]);
-          }
-          asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+          for (int d = 0; d < 32; d += 4)
+            *reinterpret_cast<float4*>(part_piece<64, VC * 64>(p_sm + t * P_BYTES, q_sm + t * Q_BYTES, r, (c + d) / 4)) =
+                make_float4(ov[d], ov[d + 1], ov[d + 2], ov[d + 3]);
         }
+        asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
       }
     } else if (ok && n_mine > 0) {
       asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
@@ -551,25 +549,23 @@ attention_prefill_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __g
   }
 
   asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
-  if constexpr (DC == 2 || VC == 1) {
-    if (splits > 1) {
-      // (the rows' states lie where keys were: both tiles are done with them behind the block's barrier)
-      float2* ml = reinterpret_cast<float2*>(ring);
-      __syncthreads();
-      if (threadIdx.x < 2 * TC_BQ) ml[threadIdx.x] = row_state;
-      cluster_barrier();
-      if (threadIdx.x < 2 * TC_BQ) {
-        const size_t row0 = (size_t)seq_q_start[seq] + q_first;
-        merge_parts<64, VC * 64, Q_BYTES, P_BYTES>(
-            q_sm, p_sm, ml, part, splits, rows_valid, vdim, out + row0 * ((size_t)heads * vdim) + (size_t)head * vdim,
-            (size_t)heads * vdim, [&](int row, float, float sum) {
-              float inv = 1.f / sum;
-              if (EXT && ex.gate) inv *= ex.gate[(row0 + row) * heads + head];
-              return inv;
-            });
-      }
-      cluster_barrier();                            // nobody leaves while others read from it
+  if constexpr (PARTS) {
+    // (the rows' states lie where keys were: both tiles are done with them behind the block's barrier)
+    float2* ml = reinterpret_cast<float2*>(ring);
+    __syncthreads();
+    if (threadIdx.x < 2 * TC_BQ) ml[threadIdx.x] = row_state;
+    cluster_barrier();
+    if (threadIdx.x < 2 * TC_BQ) {
+      const size_t row0 = (size_t)seq_q_start[seq] + q_first;
+      merge_parts<64, VC * 64, Q_BYTES, P_BYTES>(
+          q_sm, p_sm, ml, part, splits, rows_valid, vdim, out + row0 * ((size_t)heads * vdim) + (size_t)head * vdim,
+          (size_t)heads * vdim, [&](int row, float, float sum) {
+            float inv = 1.f / sum;
+            if (EXT && ex.gate) inv *= ex.gate[(row0 + row) * heads + head];
+            return inv;
+          });
     }
+    cluster_barrier();                            // nobody leaves while others read from it
   }
   __syncthreads();
   if (warp == 9) {
@@ -581,24 +577,43 @@ attention_prefill_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __g
 
 // ------------------------------------------------------------------------------------------ host
 
+// PARTS: keys in parts.  An instance of its own: as a question at run time it cost either form (us, then / now): one CTA a block, 2,048 tokens
+// of 16 heads of 128 35.1 / 34.4, of 64 32.1 / 30.7, 4 x 129 of 64 7.8 / 7.4; 700 behind 1,200 in two parts 28.9 / 27.6, of 64 26.3 / 24.6.
+// (The formed keys' kernel does not pay: 60.4 / 60.8, 51.7 / 52.7.)
+template <int DC, int VC, int EXT, bool PARTS>
+static int launch_as(const CUtensorMap& mq, const CUtensorMap& mk, const CUtensorMap& mv, void* out,
+                     const int* block_table, int table_stride, const int* seq_slot, const int* seq_q_start,
+                     const int* seq_q_len, const int* seq_kv_len, const int* tile_seq, const int* tile_first,
+                     int n_tiles, int heads, int kv_heads, float scale, int window, int* status, int list_of_blocks,
+                     int splits, cudaStream_t s, TcExtras ex) {
+  const int smem = (2 * DC + 4 + TC_RING * (DC > VC ? DC : VC)) * 128 * 128 + 1024;
+  auto kernel = attention_prefill_tc_kernel<DC, VC, EXT, PARTS>;
+  static bool configured = false;
+  if (!configured) {
+    cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+    if (e != cudaSuccess) return (int)e;
+    configured = true;
+  }
+#define ARGS mq, mk, mv, (bf16*)out, block_table, table_stride, seq_slot, seq_q_start, seq_q_len, seq_kv_len, tile_seq, tile_first, heads, \
+             kv_heads, scale * 1.4426950408889634f, window, status, list_of_blocks, splits, ex
+  if (PARTS)
+    return launch_dependent_cluster(kernel, dim3(heads * splits, n_tiles), dim3(TC_THREADS), smem, s, dim3(splits), ARGS);
+  return launch_dependent(kernel, dim3(heads, n_tiles), dim3(TC_THREADS), smem, s, ARGS);
+#undef ARGS
+}
+
 template <int DC, int VC, int EXT>
 static int launch(const CUtensorMap& mq, const CUtensorMap& mk, const CUtensorMap& mv, void* out,
                   const int* block_table, int table_stride, const int* seq_slot, const int* seq_q_start,
                   const int* seq_q_len, const int* seq_kv_len, const int* tile_seq, const int* tile_first,
                   int n_tiles, int heads, int kv_heads, float scale, int window, int* status, int list_of_blocks,
                   int splits, cudaStream_t s, TcExtras ex = TcExtras{nullptr, nullptr, nullptr, nullptr, 0, 0, 0.f, 0.f, DC * 64, VC * 64}) {
-  const int smem = (2 * DC + 4 + TC_RING * (DC > VC ? DC : VC)) * 128 * 128 + 1024;
-  static bool configured = false;
-  if (!configured) {
-    cudaError_t e = cudaFuncSetAttribute(attention_prefill_tc_kernel<DC, VC, EXT>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
-    if (e != cudaSuccess) return (int)e;
-    configured = true;
-  }
-  splits = DC == 1 && VC == 2 ? 1 : splits >= 4 ? 4 : splits >= 2 ? 2 : 1;
-  return launch_dependent_cluster(attention_prefill_tc_kernel<DC, VC, EXT>, dim3(heads * splits, n_tiles), dim3(TC_THREADS), smem, s,
-                                  dim3(splits), mq, mk, mv, (bf16*)out, block_table, table_stride, seq_slot, seq_q_start, seq_q_len,
-                                  seq_kv_len, tile_seq, tile_first, heads, kv_heads, scale * 1.4426950408889634f, window, status,
-                                  list_of_blocks, splits, ex);
+#define ARGS(SPLITS) mq, mk, mv, out, block_table, table_stride, seq_slot, seq_q_start, seq_q_len, seq_kv_len, tile_seq, tile_first, n_tiles, \
+                     heads, kv_heads, scale, window, status, list_of_blocks, SPLITS, s, ex
+  if constexpr (DC == 2 || VC == 1)
+    if (splits >= 2) return launch_as<DC, VC, EXT, true>(ARGS(splits >= 4 ? 4 : 2));
+  return launch_as<DC, VC, EXT, false>(ARGS(1));
+#undef ARGS
 }
 
 static unsigned long long next_limit_ns = WAIT_LIMIT_NS;
@@ -618,7 +633,7 @@ void sb_attention_prefill_tc_withhold(int step, unsigned long long limit_ns) {
 // How many clusters of `size` CTAs that take an SM each (the prompt attentions' blocks) the current device runs at once, or minus an
 // error.  A cluster lies inside one of the chip's processing clusters, whose SMs need not be a multiple of its size.
 int sb_prompt_clusters(int size) {
-  auto kernel = attention_prefill_tc_kernel<2, 2, 0>;
+  auto kernel = attention_prefill_tc_kernel<2, 2, 0, true>;
   const int smem = (2 * 2 + 4 + TC_RING * 2) * 128 * 128 + 1024;
   cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
   if (e != cudaSuccess) return -(int)e;
