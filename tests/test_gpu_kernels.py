@@ -799,3 +799,15 @@ def test_float32_product_of_one_row(k):
     room = 1.1 * bound[:n] * (up.abs() + bound[n:]) + silu.abs() * bound[n:] + 2.0 ** -20 * (silu * up).abs()
     got = ops.linear(dev(x), dev(w), gated=True).cpu().double()[0]
     assert ((got - silu * up).abs() <= room + 1e-30).all()
+
+
+@pytest.mark.parametrize("k", [36, 1024, 1030])
+@pytest.mark.parametrize("gated", [False, True])
+def test_a_row_of_the_few_row_product_depends_on_no_other(k, gated):
+    """A row alone, with up to three others and with more go through different kernels and launches: the same bits."""
+    from starter_b200 import ops
+
+    x, w = dev(rand(16, k, dtype="float32", seed=81)), dev(rand(74, k, dtype="float32", seed=82, scale=0.05))
+    whole = ops.linear(x, w, gated=gated)
+    for rows in (1, 2, 3, 4, 5, 8, 9):
+        assert torch.equal(ops.linear(x[:rows].contiguous(), w, gated=gated), whole[:rows])
