@@ -13,14 +13,14 @@
 //     of such updates, Bischof and Van Loan 1987) is one 16 x 16 matrix pair a block and head, made beforehand for
 //     all blocks at once by scan_coef_kernel.  The products with S run on the tensor cores, whose other operands, keys and
 //     queries, are bfloat16 as they come: S (and the write) is cut into three pieces of 8 bits, so that nothing of its 24 is
-//     lost (of an entry below 2^-109 less than 2^-134; S itself is kept whole), and sums are float.  G is applied as S - (1 - G) S, the complement carried as such (state_scan.cu says why), and a
-//     block's write is added to S by ordinary adds.
+//     lost (of an entry below 2^-109 less than 2^-134; S itself is kept whole), and sums are float.  A block's G is applied as
+//     S - (1 - G) S, the complement carried as such (state_scan.cu says why), and a block's write is added to S by ordinary adds.
 //   walk (forget-write, channel-decay): the decay differs by row, so a token is a step; the state's update is the whole
 //     chain, and read-outs of eight tokens are summed together.  A thread keeps 16 entries, so that a loaded vector serves
 //     four columns.  forget-write's gates are formed beforehand (scan_gates_kernel): inside the walk every block of 16
 //     columns would form them again.  32-bit multiply-adds.
 // Measured at 2,048 tokens of one sequence, 16 heads of 128 x 128 (state-space: 32 of 128 x 64), few-token kernel -> here: state-space
-// 577 -> 64 us (in one walk of four warps, as the delta rule's: 100), gated delta 673 -> 133, forget-write 414 -> 174,
+// 577 -> 63 us (in one walk of four warps, as the delta rule's: 98), gated delta 673 -> 133, forget-write 414 -> 174,
 // channel-decay 400 -> 177; unequal sequences of 801, 712 and 623 tokens: gated delta 598 -> 100, forget-write 382 -> 160,
 // channel-decay 377 -> 155.  The error against 64 bits falls or stays (outputs 5.5e-7 -> 2.2e-7, 3.7e-7 -> 2.0e-7, 4.9e-8, 1.2e-7).  With one
 // sequence of the delta rule an SM has four warps and the chain's latencies are the bound (about 2,000 cycles a block of sixteen).
