@@ -92,33 +92,56 @@ __global__ void qk_norm_rope_store_kernel(
   }
 }
 
-// Eight consecutive gains as floats, with 16-byte loads where the pointer allows it.
-__device__ __forceinline__ void load8(const float* p, float* out) {
-  if (((uintptr_t)p & 15) == 0) {
-    const float4 a = reinterpret_cast<const float4*>(p)[0], b = reinterpret_cast<const float4*>(p)[1];
-    out[0] = a.x; out[1] = a.y; out[2] = a.z; out[3] = a.w; out[4] = b.x; out[5] = b.y; out[6] = b.z; out[7] = b.w;
-  } else {
-#pragma unroll
-    for (int i = 0; i < 8; ++i) out[i] = p[i];
-  }
+// Products and sums of two bfloat16 at once.  Both have the bits of the float operation rounded to bfloat16: a product of two
+// 8-bit mantissas is exact in a float, and so is a sum unless one term is below 2^-16 of the other, where either way gives the other.
+__device__ __forceinline__ uint32_t mul2(uint32_t a, uint32_t b) {
+  const __nv_bfloat162 r = __hmul2_rn(*reinterpret_cast<__nv_bfloat162*>(&a), *reinterpret_cast<__nv_bfloat162*>(&b));
+  return *reinterpret_cast<const uint32_t*>(&r);
 }
-__device__ __forceinline__ void load8(const bf16* p, float* out) {
-  if (((uintptr_t)p & 15) == 0) {
-    const uint4 raw = *reinterpret_cast<const uint4*>(p);
-    const uint32_t w[4] = {raw.x, raw.y, raw.z, raw.w};
+__device__ __forceinline__ uint32_t add2(uint32_t a, uint32_t b) {
+  const __nv_bfloat162 r = __hadd2_rn(*reinterpret_cast<__nv_bfloat162*>(&a), *reinterpret_cast<__nv_bfloat162*>(&b));
+  return *reinterpret_cast<const uint32_t*>(&r);
+}
+__device__ __forceinline__ uint32_t pack2(float a, float b) {
+  const __nv_bfloat162 r = __floats2bfloat162_rn(a, b);
+  return *reinterpret_cast<const uint32_t*>(&r);
+}
+// Eight consecutive gains, in 16-byte loads where the pointer allows it, and two bfloat16 values times the i-th pair of them, rounded.
+struct Gains {
+  uint32_t two[4];
+  __device__ __forceinline__ void load(const bf16* p, bool wide) {
+    if (wide) {
+      const uint4 v = *reinterpret_cast<const uint4*>(p);
+      two[0] = v.x; two[1] = v.y; two[2] = v.z; two[3] = v.w;
+    } else {
 #pragma unroll
-    for (int i = 0; i < 4; ++i) {
-      out[2 * i] = __uint_as_float(w[i] << 16);
-      out[2 * i + 1] = __uint_as_float(w[i] & 0xffff0000u);
+      for (int i = 0; i < 4; ++i) two[i] = pack2(__bfloat162float(p[2 * i]), __bfloat162float(p[2 * i + 1]));
     }
-  } else {
-#pragma unroll
-    for (int i = 0; i < 8; ++i) out[i] = __bfloat162float(p[i]);
   }
-}
+  __device__ __forceinline__ uint32_t times(uint32_t x, int i) const { return mul2(x, two[i]); }
+};
+struct Gains32 {
+  float one[8];
+  __device__ __forceinline__ void load(const float* p, bool wide) {
+    if (wide) {
+      const float4 a = reinterpret_cast<const float4*>(p)[0], b = reinterpret_cast<const float4*>(p)[1];
+      one[0] = a.x; one[1] = a.y; one[2] = a.z; one[3] = a.w; one[4] = b.x; one[5] = b.y; one[6] = b.z; one[7] = b.w;
+    } else {
+#pragma unroll
+      for (int i = 0; i < 8; ++i) one[i] = p[i];
+    }
+  }
+  __device__ __forceinline__ uint32_t times(uint32_t x, int i) const {
+    return pack2(__uint_as_float(x << 16) * one[2 * i], __uint_as_float(x & 0xffff0000u) * one[2 * i + 1]);
+  }
+};
+template <typename W> struct GainsOf { typedef Gains type; };
+template <> struct GainsOf<float> { typedef Gains32 type; };
 
 // The same for bfloat16 with 16-byte accesses: L = head_dim / 16 lanes share a head row, each holding
-// 8 elements of the low half and the 8 they pair with in the high half; a warp takes 32 / L rows.
+// 8 elements of the low half and the 8 they pair with in the high half; a warp takes 32 / L rows.  What it costs is issue slots: with every
+// product and sum unpacked to floats and rounded by itself 2,400 tokens of 48 heads took 18.3 us of a pass (59 MB, 9 at the copy rate), in
+// pairs 11.5.
 template <typename W, int L>
 __global__ void qk_norm_rope_store_vec_kernel(
     const bf16* __restrict__ qkv, bf16* __restrict__ q_out, const W* __restrict__ q_gain,
@@ -161,36 +184,29 @@ __global__ void qk_norm_rope_store_vec_kernel(
     }
     // the shuffles below need every lane of a row's group; value rows fall in whole groups
   }
-  float lo[8], hi[8];
-  {
-    const uint32_t wl[4] = {raw_lo.x, raw_lo.y, raw_lo.z, raw_lo.w}, wh[4] = {raw_hi.x, raw_hi.y, raw_hi.z, raw_hi.w};
-#pragma unroll
-    for (int i = 0; i < 4; ++i) {
-      lo[2 * i] = __uint_as_float(wl[i] << 16); lo[2 * i + 1] = __uint_as_float(wl[i] & 0xffff0000u);
-      hi[2 * i] = __uint_as_float(wh[i] << 16); hi[2 * i + 1] = __uint_as_float(wh[i] & 0xffff0000u);
-    }
-  }
+  uint32_t lo[4] = {raw_lo.x, raw_lo.y, raw_lo.z, raw_lo.w}, hi[4] = {raw_hi.x, raw_hi.y, raw_hi.z, raw_hi.w};
   const W* gain = is_q ? q_gain : k_gain;
   float ss = 0.f;
 #pragma unroll
-  for (int i = 0; i < 8; ++i) ss += lo[i] * lo[i] + hi[i] * hi[i];
+  for (int i = 0; i < 4; ++i) {
+    const float l0 = __uint_as_float(lo[i] << 16), l1 = __uint_as_float(lo[i] & 0xffff0000u);
+    const float h0 = __uint_as_float(hi[i] << 16), h1 = __uint_as_float(hi[i] & 0xffff0000u);
+    ss += l0 * l0 + h0 * h0;
+    ss += l1 * l1 + h1 * h1;
+  }
 #pragma unroll
   for (int o = L / 2; o > 0; o >>= 1) ss += __shfl_xor_sync(0xffffffffu, ss, o);
   if (is_v || !live) return;
   if (gain) {
     const float inv = rsqrtf(ss / (float)D + eps);
-    float g_lo[8], g_hi[8];
-    load8(gain + part * 8, g_lo);
-    load8(gain + HALF + part * 8, g_hi);
+    const bool wide = ((uintptr_t)gain & 15) == 0;
+    typename GainsOf<W>::type g_lo, g_hi;
+    g_lo.load(gain + part * 8, wide);
+    g_hi.load(gain + HALF + part * 8, wide);
 #pragma unroll
-    for (int i = 0; i < 8; ++i) {
-      float a = lo[i] * inv, b = hi[i] * inv;
-      rnd2<bf16>(a, b);
-      a *= g_lo[i];
-      b *= g_hi[i];
-      rnd2<bf16>(a, b);
-      lo[i] = a;
-      hi[i] = b;
+    for (int i = 0; i < 4; ++i) {
+      lo[i] = g_lo.times(pack2(__uint_as_float(lo[i] << 16) * inv, __uint_as_float(lo[i] & 0xffff0000u) * inv), i);
+      hi[i] = g_hi.times(pack2(__uint_as_float(hi[i] << 16) * inv, __uint_as_float(hi[i] & 0xffff0000u) * inv), i);
     }
   }
   if (cos_table) {
@@ -198,34 +214,17 @@ __global__ void qk_norm_rope_store_vec_kernel(
     const float4* cp4 = reinterpret_cast<const float4*>(cos_table + (size_t)pos * HALF + part * 8);
     const float4* sp4 = reinterpret_cast<const float4*>(sin_table + (size_t)pos * HALF + part * 8);
     const float4 c0 = cp4[0], c1 = cp4[1], s0 = sp4[0], s1 = sp4[1];
-    const float cp[8] = {c0.x, c0.y, c0.z, c0.w, c1.x, c1.y, c1.z, c1.w};
-    const float sp[8] = {s0.x, s0.y, s0.z, s0.w, s1.x, s1.y, s1.z, s1.w};
+    const uint32_t c[4] = {pack2(c0.x, c0.y), pack2(c0.z, c0.w), pack2(c1.x, c1.y), pack2(c1.z, c1.w)};
+    const uint32_t sn[4] = {pack2(s0.x, s0.y), pack2(s0.z, s0.w), pack2(s1.x, s1.y), pack2(s1.z, s1.w)};
 #pragma unroll
-    for (int i = 0; i < 8; ++i) {
-      float c = cp[i], sn = sp[i];
-      rnd2<bf16>(c, sn);
-      float a0 = lo[i] * c, a1 = -hi[i] * sn, b0 = hi[i] * c, b1 = lo[i] * sn;
-      rnd2<bf16>(a0, a1);
-      rnd2<bf16>(b0, b1);
-      float a = a0 + a1, b = b0 + b1;
-      rnd2<bf16>(a, b);
+    for (int i = 0; i < 4; ++i) {
+      const uint32_t a = add2(mul2(lo[i], c[i]), mul2(hi[i], sn[i]) ^ 0x80008000u);
+      hi[i] = add2(mul2(hi[i], c[i]), mul2(lo[i], sn[i]));
       lo[i] = a;
-      hi[i] = b;
     }
   }
-  uint4 out_lo, out_hi;
-  {
-    uint32_t wl[4], wh[4];
-#pragma unroll
-    for (int i = 0; i < 4; ++i) {             // every value is a bfloat16 already (or came in as one)
-      wl[i] = pack_exact_bf16(lo[2 * i], lo[2 * i + 1]);
-      wh[i] = pack_exact_bf16(hi[2 * i], hi[2 * i + 1]);
-    }
-    out_lo = make_uint4(wl[0], wl[1], wl[2], wl[3]);
-    out_hi = make_uint4(wh[0], wh[1], wh[2], wh[3]);
-  }
-  *reinterpret_cast<uint4*>(dst) = out_lo;
-  *reinterpret_cast<uint4*>(dst + HALF) = out_hi;
+  *reinterpret_cast<uint4*>(dst) = make_uint4(lo[0], lo[1], lo[2], lo[3]);
+  *reinterpret_cast<uint4*>(dst + HALF) = make_uint4(hi[0], hi[1], hi[2], hi[3]);
 }
 
 template <typename W, int L>

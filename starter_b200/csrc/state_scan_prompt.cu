@@ -972,10 +972,26 @@ scan_segments_kernel(const bf16* __restrict__ q, int ldq, const bf16* __restrict
 // tokens than the grid's other dimensions count to).
 __global__ void __launch_bounds__(256)
 scan_gates_kernel(const bf16* __restrict__ q, int ldq, const bf16* __restrict__ z, int ldz, const float* __restrict__ lower,
-                  const float* __restrict__ bias, float* __restrict__ qf, float* __restrict__ d, int channels) {
+                  const float* __restrict__ bias, float* __restrict__ qf, float* __restrict__ d, int channels, int wide) {
+  const int c = (blockIdx.y * 256 + threadIdx.x) * 8;
+  alignas(16) float lo[8], bi[8];                   // (weights: ahead of the wait, in 16-byte loads where they may be)
+  if (c < channels) {
+    if (wide) {
+#pragma unroll
+      for (int i = 0; i < 8; i += 4) {
+        *reinterpret_cast<float4*>(lo + i) = *reinterpret_cast<const float4*>(lower + c + i);
+        *reinterpret_cast<float4*>(bi + i) = *reinterpret_cast<const float4*>(bias + c + i);
+      }
+    } else {
+#pragma unroll
+      for (int i = 0; i < 8; ++i) {
+        lo[i] = lower[c + i];
+        bi[i] = bias[c + i];
+      }
+    }
+  }
   pdl_wait();
   SB_BEHIND_WAIT(q); SB_BEHIND_WAIT(z);
-  const int c = (blockIdx.y * 256 + threadIdx.x) * 8;
   if (c >= channels) return;
   const size_t row = blockIdx.x;
   const uint4 qv = *reinterpret_cast<const uint4*>(q + row * ldq + c), zv = *reinterpret_cast<const uint4*>(z + row * ldz + c);
@@ -986,7 +1002,7 @@ scan_gates_kernel(const bf16* __restrict__ q, int ldq, const bf16* __restrict__ 
     const float qe = __uint_as_float(i & 1 ? qw[i / 2] & 0xffff0000u : qw[i / 2] << 16);
     const float ze = __uint_as_float(i & 1 ? zw[i / 2] & 0xffff0000u : zw[i / 2] << 16);
     a[i] = qe / (1.f + expf(-qe));
-    g[i] = (1.f - lower[c + i]) / (1.f + expf(ze + bias[c + i]));
+    g[i] = (1.f - lo[i]) / (1.f + expf(ze + bi[i]));
   }
   float4* qo = reinterpret_cast<float4*>(qf + row * channels + c);
   float4* go = reinterpret_cast<float4*>(d + row * channels + c);
@@ -1216,7 +1232,7 @@ int sb_state_scan_prompt(int mode, const void* q, int ldq, const void* k, int ld
     float* qf = scratch;
     float* d = scratch + (size_t)n_tokens * channels;
     int rc = launch_dependent(scan_gates_kernel, dim3(n_tokens, (channels / 8 + 255) / 256), dim3(256), 0, s, (const bf16*)q, ldq,
-                              (const bf16*)k, ldk, A_log, dt_bias, qf, d, channels);
+                              (const bf16*)k, ldk, A_log, dt_bias, qf, d, channels, (int)!(((uintptr_t)A_log | (uintptr_t)dt_bias) % 16));
     if (rc) return rc;
     const size_t smem = SP_STAGES * sizeof(ForgetStage);
     cudaError_t err = cudaFuncSetAttribute(scan_rows_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
