@@ -64,6 +64,7 @@ SOURCES = (
     "short_conv",
     "state_scan",
     "state_scan_prompt",
+    "state_step",
 )
 
 _lock = threading.Lock()

@@ -2609,6 +2609,36 @@ def scan_one_walk(n_tokens: int, n_seqs: int, blocks: int) -> bool:
     return blocks <= 3 * SM_COUNT and segs <= (3 if blocks <= SM_COUNT else 2)
 
 
+def _scan_operands(mode, q, k, v, a_raw, b_raw, A_log, dt_bias, skip, state, state_at, seq_slot, seq_q_start, seq_q_len, heads,
+                   groups, n_state, v_dim):
+    """The checked operands of a recurrence: ``(address, row width) * 5 of q .. b_raw, tokens, sequences``."""
+    if mode not in SCAN_MODES:
+        raise KernelError(f"no recurrence {mode!r} (known: {', '.join(SCAN_MODES)})")
+    dtype = q[0].dtype
+    n_tokens = q[0].shape[0]
+    args = []
+    for name, pair, width in (("q", q, groups * n_state), ("k", k, groups * n_state), ("v", v, heads * v_dim),
+                              ("a_raw", a_raw, heads), ("b_raw", b_raw, heads)):
+        if pair is None:
+            args += [None, 0]
+            continue
+        t, col = pair
+        _need(t, name, dtype, 2)
+        if t.shape[0] != n_tokens or col < 0 or col + width > t.shape[1]:
+            raise KernelError(f"{name}: {width} columns from {col} of {tuple(t.shape)} do not fit {n_tokens} tokens")
+        args += [_at(t, col), t.shape[1]]
+    if mode != "channel_decay":
+        per_head = heads * n_state if mode == "forget_write" else heads
+        _f32(A_log, "A_log", (per_head,))
+        _f32(dt_bias, "dt_bias", (per_head,))
+    if skip is not None:
+        _f32(skip, "skip", (heads,))
+    _need(state, "state", torch.float32, 2)
+    if state_at < 0 or state_at + heads * n_state * v_dim > state.shape[1]:
+        raise KernelError(f"a slot's {state.shape[1]} floats do not hold {heads} states of {n_state} x {v_dim} from {state_at}")
+    return args, n_tokens, _seq_arrays(seq_slot, seq_q_start, seq_q_len)
+
+
 def state_scan(mode, q, k, v, a_raw, b_raw, A_log, dt_bias, skip, state, state_at, seq_slot, seq_q_start, seq_q_len,
                heads, groups, n_state, v_dim, decay=None):
     """A linear recurrence with a state ``S`` ``[n_state, v_dim]`` per head over the sequences of a step.
@@ -2627,35 +2657,13 @@ def state_scan(mode, q, k, v, a_raw, b_raw, A_log, dt_bias, skip, state, state_a
     float32 ``[T, heads * n_state]`` holds the decays' complements ``d = 1 - alpha`` per row of the state; q times ``n_state **
     -0.5``; ``S <- diag(1 - d) S + k v^T``, ``o = S^T q``.  ``state`` float32 ``[slots, M]``: a slot's ``[heads, n_state, v_dim]`` from
     ``state_at`` on, read at the start and written at the end.  Returns float32 ``[T, heads * v_dim]``."""
-    if mode not in SCAN_MODES:
-        raise KernelError(f"no recurrence {mode!r} (known: {', '.join(SCAN_MODES)})")
-    dtype = q[0].dtype
-    n_tokens = q[0].shape[0]
-    args = []
-    for name, pair, width in (("q", q, groups * n_state), ("k", k, groups * n_state), ("v", v, heads * v_dim),
-                              ("a_raw", a_raw, heads), ("b_raw", b_raw, heads)):
-        if pair is None:
-            args += [None, 0]
-            continue
-        t, col = pair
-        _need(t, name, dtype, 2)
-        if t.shape[0] != n_tokens or col < 0 or col + width > t.shape[1]:
-            raise KernelError(f"{name}: {width} columns from {col} of {tuple(t.shape)} do not fit {n_tokens} tokens")
-        args += [_at(t, col), t.shape[1]]
+    args, n_tokens, n_seqs = _scan_operands(mode, q, k, v, a_raw, b_raw, A_log, dt_bias, skip, state, state_at, seq_slot, seq_q_start,
+                                            seq_q_len, heads, groups, n_state, v_dim)
     if (mode == "channel_decay") != (decay is not None):
         raise KernelError("decays per row of the state belong to the channel_decay recurrence")
     if decay is not None:
         _f32(decay, "decay", (n_tokens, heads * n_state))
-    else:
-        per_head = heads * n_state if mode == "forget_write" else heads
-        _f32(A_log, "A_log", (per_head,))
-        _f32(dt_bias, "dt_bias", (per_head,))
-    if skip is not None:
-        _f32(skip, "skip", (heads,))
-    _need(state, "state", torch.float32, 2)
-    if state_at < 0 or state_at + heads * n_state * v_dim > state.shape[1]:
-        raise KernelError(f"a slot's {state.shape[1]} floats do not hold {heads} states of {n_state} x {v_dim} from {state_at}")
-    n_seqs = _seq_arrays(seq_slot, seq_q_start, seq_q_len)
+    dtype = q[0].dtype
     out = _empty(state, (n_tokens, heads * v_dim), torch.float32)
     if dtype == torch.bfloat16 and n_tokens >= SCAN_PROMPT_TOKENS * n_seqs and 64 < n_state <= 128:
         lib = _lib("state_scan_prompt")
@@ -2685,25 +2693,93 @@ def state_scan(mode, q, k, v, a_raw, b_raw, A_log, dt_bias, skip, state, state_a
     return out
 
 
+@functools.lru_cache(maxsize=256)
+def _state_step_takes(mode, heads, groups, n_state, v_dim) -> bool:
+    return bool(_lib("state_step").sb_state_step_takes(SCAN_MODES[mode], heads, groups, n_state, v_dim))
+
+
+def state_scan_norm(mode, q, k, v, a_raw, b_raw, A_log, dt_bias, skip, state, state_at, seq_slot, seq_q_start, seq_q_len, max_q_len,
+                    heads, groups, n_state, v_dim, gain, parts, eps, gate=None, gate_first=False, low=None):
+    """``state_scan`` and ``group_norm_gate`` of what it reads out (``gate``: ``(tensor, first column)`` or None), in the type of
+    ``q``; with ``low = (tensor, first column, a2, bias, tau)`` the decays of a channel-decay recurrence are ``low_rank_decay``'s.
+
+    ``max_q_len``: the most tokens a sequence brings.  Where that is one, a bfloat16 step is one kernel (csrc/state_step.cu) for heads
+    that it takes, with its norm where every head is a part and the gate comes behind it; otherwise each is a kernel of its own."""
+    t, dtype = q[0], q[0].dtype
+    if max_q_len == 1 and dtype == torch.bfloat16 and mode in SCAN_MODES and _state_step_takes(mode, heads, groups, n_state, v_dim):
+        args, n_tokens, n_seqs = _scan_operands(mode, q, k, v, a_raw, b_raw, A_log, dt_bias, skip, state, state_at, seq_slot,
+                                                seq_q_start, seq_q_len, heads, groups, n_state, v_dim)
+        decays = [None, 0, None, None, 0, 0.0]
+        if (mode == "channel_decay") != (low is not None):
+            raise KernelError("decays per row of the state belong to the channel_decay recurrence")
+        if low is not None:
+            decays = list(_low_rank(*low, n_tokens, heads * n_state))
+        normed = parts == heads and not gate_first
+        gate_args = [None, 0]
+        if normed:
+            _check_gain(gain, heads * v_dim, parts)
+            if gate is not None:
+                gate_args = [_gate_at(gate, dtype, n_tokens, heads * v_dim, parts), gate[0].shape[1]]
+        out = _empty(t if normed else state, (n_tokens, heads * v_dim), dtype if normed else torch.float32)
+        rc = _lib("state_step").sb_state_step(
+            SCAN_MODES[mode], *args, A_log, dt_bias, skip, *decays, _at(state, state_at), state.shape[1], seq_slot, seq_q_start, seq_q_len,
+            n_seqs, heads, groups, n_state, v_dim, *gate_args, gain if normed else None, gain.shape[0] if normed else 0, eps,
+            None if normed else out, out if normed else None, _stream())
+        if rc != -2:                       # (an operand off its alignment: the separate kernels take any)
+            _check(rc, "state_step")
+            if normed:
+                return out
+            return group_norm_gate(out, gate[0] if gate else None, gate[1] if gate else 0, gain, parts, eps, gate_first, dtype)
+    decay = low_rank_decay(*low) if low is not None else None
+    o = state_scan(mode, q, k, v, a_raw, b_raw, A_log, dt_bias, skip, state, state_at, seq_slot, seq_q_start, seq_q_len, heads, groups,
+                   n_state, v_dim, decay=decay)
+    return group_norm_gate(o, gate[0] if gate else None, gate[1] if gate else 0, gain, parts, eps, gate_first, dtype)
+
+
+def _low_rank(u, col, a2, bias, tau, n_tokens, channels):
+    """A low-rank decay's checked operands: the entries' address and row width, ``a2``, ``bias``, the rank and ``1 / tau``."""
+    _need(u, "u", None, 2)
+    _need(a2, "a2", torch.float32, 2)
+    rank = a2.shape[0]
+    if a2.shape[1] != channels or u.shape[0] != n_tokens:
+        raise KernelError(f"a decay of {tuple(u.shape)} by {tuple(a2.shape)} is not one of {channels} rows for {n_tokens} tokens")
+    _f32(bias, "bias", (channels,))
+    if col < 0 or col + rank > u.shape[1]:
+        raise KernelError(f"{rank} columns from {col} of {tuple(u.shape)} are not there")
+    if not tau > 0.0:
+        raise KernelError(f"tau={tau} must be positive")
+    if rank < 1 or rank > 1024:
+        raise KernelError(f"the low-rank decay takes ranks of 1 to 1024, not {rank}")
+    return _at(u, col), u.shape[1], a2, bias, rank, 1.0 / tau
+
+
 def low_rank_decay(u, col, a2, bias, tau):
     """``1 - sigmoid(z) ** (1 / tau)`` with ``z = u @ a2 + bias``: how much of its row of a recurrent state every channel lets
     go of a token.  ``u``: the columns ``col .. col + R`` of a ``[T, N]`` tensor; ``a2`` float32 ``[R, C]``, ``bias`` float32
     ``[C]``.  The product, the logarithm and the exponential are float; returns float32 ``[T, C]``."""
     _need(u, "u", None, 2)
     _need(a2, "a2", torch.float32, 2)
-    rank, channels = a2.shape
-    _f32(bias, "bias", (channels,))
-    if col < 0 or col + rank > u.shape[1]:
-        raise KernelError(f"{rank} columns from {col} of {tuple(u.shape)} are not there")
-    if not tau > 0.0:
-        raise KernelError(f"tau={tau} must be positive")
+    channels = a2.shape[1]
+    at, width, _, _, rank, inv_tau = _low_rank(u, col, a2, bias, tau, u.shape[0], channels)
     out = _empty(u, (u.shape[0], channels), torch.float32)
-    rc = _lib("state_scan").sb_low_rank_decay(_code(u.dtype), _at(u, col), u.shape[1], a2, bias, out,
-                                              u.shape[0], channels, rank, 1.0 / tau, _stream())
-    if rc == -2:
-        raise KernelError(f"the low-rank decay takes ranks of 1 to 1024, not {rank}")
+    rc = _lib("state_scan").sb_low_rank_decay(_code(u.dtype), at, width, a2, bias, out, u.shape[0], channels, rank, inv_tau, _stream())
     _check(rc, "low_rank_decay")
     return out
+
+
+def _check_gain(weight, width, parts):
+    _need(weight, "weight", torch.float32, 1)
+    if weight.shape[0] not in (width, width // parts):
+        raise KernelError(f"a gain of {weight.shape[0]} entries fits neither the row ({width}) nor a part ({width // parts})")
+
+
+def _gate_at(gate, dtype, n_tokens, width, parts):
+    """The address of a gate ``(tensor, first column)`` of ``width`` entries a row."""
+    z, z_col = gate
+    _need(z, "z", dtype, 2)
+    if z.shape[0] != n_tokens or z_col < 0 or z_col + width > z.shape[1]:
+        raise KernelError(f"rows of {width} in {parts} parts with a gate from column {z_col} of {tuple(z.shape)} do not fit")
+    return _at(z, z_col)
 
 
 def group_norm_gate(o, z, z_col, weight, parts, eps, gate_first, dtype):
@@ -2713,17 +2789,12 @@ def group_norm_gate(o, z, z_col, weight, parts, eps, gate_first, dtype):
     the parts share it.  Returns ``[T, N]`` in ``dtype``."""
     _need(o, "o", torch.float32, 2)
     n_tokens, width = o.shape
-    _need(weight, "weight", torch.float32, 1)
     if parts < 1 or width % parts:
         raise KernelError(f"rows of {width} do not split into {parts} parts")
-    if z is not None:
-        _need(z, "z", dtype, 2)
-        if z.shape[0] != n_tokens or z_col < 0 or z_col + width > z.shape[1]:
-            raise KernelError(f"rows of {width} in {parts} parts with a gate from column {z_col} of {tuple(z.shape)} do not fit")
-    if weight.shape[0] not in (width, width // parts):
-        raise KernelError(f"a gain of {weight.shape[0]} entries fits neither the row ({width}) nor a part ({width // parts})")
+    at = _gate_at((z, z_col), dtype, n_tokens, width, parts) if z is not None else None
+    _check_gain(weight, width, parts)
     y = _empty(o, (n_tokens, width), dtype)
-    gate, gate_width, order = (None, 0, 2) if z is None else (_at(z, z_col), z.shape[1], 0 if gate_first else 1)
+    gate, gate_width, order = (None, 0, 2) if z is None else (at, z.shape[1], 0 if gate_first else 1)
     rc = _lib("state_scan").sb_group_norm_gate(_code(dtype), o, gate, gate_width, weight,
                                                weight.shape[0], y, n_tokens, parts, width // parts,
                                                eps, order, _stream())

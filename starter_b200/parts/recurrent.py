@@ -149,10 +149,10 @@ class StateSpaceMixer(_Recurrent):
         proj = ops.linear(x, self.w_in, status=ctx.status)
         xbc = ops.short_conv(proj, self.inner, self.convolved, self.conv, self.conv_bias, None, state, self.state_at, *seqs,
                              ctx.max_q_len, "silu")
-        y = ops.state_scan("state_space", (xbc, self.inner + self.bc), (xbc, self.inner), (xbc, 0),
-                           (proj, self.inner + self.convolved), None, self.A_log, self.dt_bias, self.D, state,
-                           self.state_at + (s.conv - 1) * self.convolved, *seqs, s.num_heads, s.groups, s.state, s.head_dim)
-        y = ops.group_norm_gate(y, proj, 0, self.gain, s.norm_groups, s.norm_eps, True, x.dtype)
+        y = ops.state_scan_norm("state_space", (xbc, self.inner + self.bc), (xbc, self.inner), (xbc, 0),
+                                (proj, self.inner + self.convolved), None, self.A_log, self.dt_bias, self.D, state,
+                                self.state_at + (s.conv - 1) * self.convolved, *seqs, ctx.max_q_len, s.num_heads, s.groups, s.state,
+                                s.head_dim, self.gain, s.norm_groups, s.norm_eps, gate=(proj, 0), gate_first=True)
         return ops.linear(y, self.o, status=ctx.status)
 
     def weight_bytes(self):
@@ -201,11 +201,10 @@ class GatedDeltaMixer(_Recurrent):
                              "silu")
         gate_at = self.convolved
         beta_at = gate_at + self.inner
-        o = ops.state_scan("gated_delta", (qkv, 0), (qkv, self.qk), (qkv, 2 * self.qk), (proj, beta_at + s.num_heads),
-                           (proj, beta_at), self.A_log, self.dt_bias, None, state,
-                           self.state_at + (s.conv - 1) * self.convolved, *seqs,
-                           s.num_heads, s.num_kv_heads, s.head_dim, s.value_dim)
-        y = ops.group_norm_gate(o, proj, gate_at, self.gain, s.num_heads, s.norm_eps, False, x.dtype)
+        y = ops.state_scan_norm("gated_delta", (qkv, 0), (qkv, self.qk), (qkv, 2 * self.qk), (proj, beta_at + s.num_heads),
+                                (proj, beta_at), self.A_log, self.dt_bias, None, state,
+                                self.state_at + (s.conv - 1) * self.convolved, *seqs, ctx.max_q_len, s.num_heads, s.num_kv_heads,
+                                s.head_dim, s.value_dim, self.gain, s.num_heads, s.norm_eps, gate=(proj, gate_at))
         return ops.linear(y, self.o, status=ctx.status)
 
     def weight_bytes(self):
@@ -241,10 +240,9 @@ class ForgetWriteMixer(_Recurrent):
         s = self.spec
         state = self._state(ctx, entry, writes_cache)
         proj = ops.linear(x, self.stacked, status=ctx.status)
-        o = ops.state_scan("forget_write", (proj, 0), (proj, self.qk), (proj, 2 * self.qk), None, None, self.lower,
-                           self.f_bias, None, state, self.state_at, ctx.seq_slot, ctx.seq_q_start, ctx.seq_q_len,
-                           s.num_heads, s.num_heads, s.head_dim, s.value_dim)
-        y = ops.group_norm_gate(o, None, 0, self.gain, s.num_heads, s.norm_eps, False, x.dtype)
+        y = ops.state_scan_norm("forget_write", (proj, 0), (proj, self.qk), (proj, 2 * self.qk), None, None, self.lower,
+                                self.f_bias, None, state, self.state_at, ctx.seq_slot, ctx.seq_q_start, ctx.seq_q_len, ctx.max_q_len,
+                                s.num_heads, s.num_heads, s.head_dim, s.value_dim, self.gain, s.num_heads, s.norm_eps)
         return ops.linear(y, self.o, status=ctx.status)
 
     def weight_bytes(self):
@@ -287,11 +285,10 @@ class GatedLinearAttention(_Recurrent):
         state = self._state(ctx, entry, writes_cache)
         gate_at = 2 * self.qk + self.inner
         proj = ops.linear(x, self.stacked, status=ctx.status)
-        decay = ops.low_rank_decay(proj, gate_at + self.inner, self.a2, self.a2_bias, s.tau)
-        o = ops.state_scan("channel_decay", (proj, 0), (proj, self.qk), (proj, 2 * self.qk), None, None, None, None, None,
-                           state, self.state_at, ctx.seq_slot, ctx.seq_q_start, ctx.seq_q_len, s.num_heads, s.num_heads,
-                           s.head_dim, s.value_dim, decay=decay)
-        y = ops.group_norm_gate(o, proj, gate_at, self.gain, s.num_heads, s.norm_eps, False, x.dtype)
+        y = ops.state_scan_norm("channel_decay", (proj, 0), (proj, self.qk), (proj, 2 * self.qk), None, None, None, None, None,
+                                state, self.state_at, ctx.seq_slot, ctx.seq_q_start, ctx.seq_q_len, ctx.max_q_len, s.num_heads,
+                                s.num_heads, s.head_dim, s.value_dim, self.gain, s.num_heads, s.norm_eps, gate=(proj, gate_at),
+                                low=(proj, gate_at + self.inner, self.a2, self.a2_bias, s.tau))
         return ops.linear(y, self.o, status=ctx.status)
 
     def weight_bytes(self):
