@@ -779,11 +779,18 @@ moe_tile_big_kernel(const bf16* __restrict__ x, const bf16* __restrict__ w, bf16
 // For steps with a handful of rows an expert (single tokens): a tile is up to MOE_FEW rows of one expert, the columns of an
 // m16n8k16 product whose rows are 16 weight rows (16 gate and the matching 16 up rows).  Operands go from global memory to
 // registers in 16-byte pieces: lane 4 g + x holds the pieces x, x + 4, .. of weight rows g and g + 8 and of the tile's row g, so
-// that every product sees its k entries in one order, and a warp's next eight steps of 32 entries (four with two weight blocks) are in flight together.  Four
-// warps share the k range (their sums meet in shared memory).  The step is bound by the weights' bytes, which are read once a
-// tile: 16 experts of 2,048 x 2,048 at 8 tokens, four each: 79 us up and 33 down on the CUDA cores (160 instructions a
-// 16-byte piece, two warps a scheduler), 43 and 30 now (5.7 and 4.1 TB/s)
+// that every product sees its k entries in one order.  The step is bound by the weights' bytes, which are read once a
+// tile, so what counts is that loads never stop: a warp keeps FLY steps of 32 entries in flight and asks for the next one as
+// soon as it has used one, and a block has as many warps (1 to 8, which share the k range; their sums meet in shared memory) as
+// bring 8 to 16 warps to every SM at once, in one round.  The weight rows of a tile run along the grid, so
+// that the warps of an SM share the tile's rows in the first cache.  A captured layer of 16 experts of 2,048 x 2,048 at 8 tokens, four each, with
+// blocks of four warps (a round and a half of them) and loads that stop between steps 84.0 us, now 77.5 (363 MB are 55); 32 experts, 11 tokens, 1,664 x
+// 1,536 90.0 -> 87.2; 8 experts, 2 tokens, three each, squared relu, 1,152 x 1,664 32.8 -> 23.6.
+// The second product may read the tiles' experts and its first weights ahead of its wait: the first one lets it start only
+// behind its own wait, when the kernel that made the tiles has completed.
 #define MOE_FEW 8
+#define MOE_FEW_WARPS 10         // warps on every SM that a grid should bring
+#define MOE_FEW_REGS 128         // (16 warps an SM; 6 and 3 steps in flight fill them.  144 registers and 8 and 4: 77.5 -> 90.0 us, 96 and 4 and 2: 88.0)
 __device__ __forceinline__ void moe_unpack8(const uint4& v, float* f) {
   f[0] = __uint_as_float(v.x << 16); f[1] = __uint_as_float(v.x & 0xffff0000u);
   f[2] = __uint_as_float(v.y << 16); f[3] = __uint_as_float(v.y & 0xffff0000u);
@@ -792,54 +799,73 @@ __device__ __forceinline__ void moe_unpack8(const uint4& v, float* f) {
 }
 
 
+__device__ __forceinline__ uint4 moe_stream16(const uint4* p) {      // (volatile: loads stay where they are asked for)
+  uint4 v;
+  asm volatile("ld.global.nc.L1::no_allocate.v4.u32 {%0, %1, %2, %3}, [%4];" : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "l"(p));
+  return v;
+}
+
 template <int MODE>
-__global__ void __launch_bounds__(128)
+__global__ void __maxnreg__(MOE_FEW_REGS)
 moe_few_kernel(const bf16* __restrict__ x, const bf16* __restrict__ w, bf16* __restrict__ y,
                const int* __restrict__ sorted, const int* __restrict__ tile_expert, const int* __restrict__ n_tiles,
                int k_dim, int n_out, int top, float limit, const float* __restrict__ in_scale) {
   constexpr bool UP = MODE != 0;
-  constexpr int NW = MODE == 1 ? 2 : 1, MOE_FEW_FLY = 8 / NW;
-  __shared__ float part[4][NW * 4][32];
-  pdl_trigger();
-  pdl_wait();
-  SB_BEHIND_WAIT(x);
+  constexpr int NW = MODE == 1 ? 2 : 1, FLY = MODE == 1 ? 3 : 6;
+  extern __shared__ float few_part[];                   // [warps][NW * 4][32], with more than one warp
+  const int warps = blockDim.x >> 5;
+  if (UP) {
+    pdl_wait();
+    pdl_trigger();
+  }
   SB_BEHIND_WAIT(sorted);
   SB_BEHIND_WAIT(tile_expert);
   SB_BEHIND_WAIT(n_tiles);
-  SB_BEHIND_WAIT(in_scale);
-  const int tile = blockIdx.x;
+  const int tile = blockIdx.y;
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, g = lane >> 2, q = lane & 3;
   // (three loads at once; a tile that is not there has garbage in its places and leaves)
   const int expert = tile_expert[tile], own = sorted[tile * MOE_FEW + g];
-  if (tile >= n_tiles[0]) return;
+  if (tile >= n_tiles[0]) {
+    if (!UP) pdl_wait();
+    return;
+  }
   const bf16* we = w + (size_t)expert * NW * n_out * k_dim;
-  const int n0 = blockIdx.y * 16;
+  const int n0 = blockIdx.x * 16;
   // this lane's row of the tile (none: the loads are of the tile's first row, the products are not stored) and its weight rows
-  const bf16* xr = x + (UP ? (size_t)(own >= 0 ? own / top : 0) : (size_t)tile * MOE_FEW + (own >= 0 ? g : 0)) * k_dim;
-  const bf16* wr[NW][2];
+  const uint4* wr[NW][2];
 #pragma unroll
   for (int a = 0; a < NW; ++a)
 #pragma unroll
-    for (int r = 0; r < 2; ++r) wr[a][r] = we + ((size_t)a * n_out + min(n0 + g + 8 * r, n_out - 1)) * k_dim;
-  const int pieces = k_dim / 8, steps = (pieces + 3) / 4;
+    for (int r = 0; r < 2; ++r)
+      wr[a][r] = reinterpret_cast<const uint4*>(we + ((size_t)a * n_out + min(n0 + g + 8 * r, n_out - 1)) * k_dim) + q;
+  const int pieces = k_dim / 8 - q;                     // (pieces from this lane's first on)
+  const int steps = (k_dim / 8 + 3) / 4;
+  uint4 wv[FLY][NW][2], xv[FLY];
+  auto load_w = [&](int i, int s) {
+    const bool in = 4 * s < pieces;
+#pragma unroll
+    for (int a = 0; a < NW; ++a)
+#pragma unroll
+      for (int r = 0; r < 2; ++r) wv[i][a][r] = in ? moe_stream16(wr[a][r] + 4 * s) : make_uint4(0u, 0u, 0u, 0u);
+  };
+#pragma unroll
+  for (int i = 0; i < FLY; ++i) load_w(i, warp + i * warps);
+  if (!UP) {
+    pdl_wait();
+    pdl_trigger();
+  }
+  SB_BEHIND_WAIT(x);
+  SB_BEHIND_WAIT(in_scale);
+  const uint4* xr = reinterpret_cast<const uint4*>(x + (UP ? (size_t)(own >= 0 ? own / top : 0) : (size_t)tile * MOE_FEW + (own >= 0 ? g : 0)) * k_dim) + q;
+  auto load_x = [&](int i, int s) { xv[i] = 4 * s < pieces ? xr[4 * s] : make_uint4(0u, 0u, 0u, 0u); };
+#pragma unroll
+  for (int i = 0; i < FLY; ++i) load_x(i, warp + i * warps);
   float acc[NW][4];
 #pragma unroll
   for (int a = 0; a < NW; ++a) acc[a][0] = acc[a][1] = acc[a][2] = acc[a][3] = 0.f;
-  for (int s0 = warp; s0 < steps; s0 += 4 * MOE_FEW_FLY) {
-    uint4 wv[MOE_FEW_FLY][NW][2], xv[MOE_FEW_FLY];
+  for (int s0 = warp; s0 < steps; s0 += FLY * warps) {
 #pragma unroll
-    for (int i = 0; i < MOE_FEW_FLY; ++i) {
-      const int piece = (s0 + 4 * i) * 4 + q;
-      const bool in = piece < pieces;
-#pragma unroll
-      for (int a = 0; a < NW; ++a)
-#pragma unroll
-        for (int r = 0; r < 2; ++r)
-          wv[i][a][r] = in ? __ldg(reinterpret_cast<const uint4*>(wr[a][r]) + piece) : make_uint4(0u, 0u, 0u, 0u);
-      xv[i] = in ? reinterpret_cast<const uint4*>(xr)[piece] : make_uint4(0u, 0u, 0u, 0u);
-    }
-#pragma unroll
-    for (int i = 0; i < MOE_FEW_FLY; ++i)
+    for (int i = 0; i < FLY; ++i) {
 #pragma unroll
       for (int a = 0; a < NW; ++a) {
         const uint4 u = wv[i][a][0], v = wv[i][a][1];
@@ -851,27 +877,43 @@ moe_few_kernel(const bf16* __restrict__ x, const bf16* __restrict__ w, bf16* __r
 #pragma unroll
         for (int c = 0; c < 4; ++c) acc[a][c] += step[c];
       }
+      const int next = s0 + (i + FLY) * warps;
+      load_w(i, next);
+      load_x(i, next);
+    }
   }
+  if (warps > 1) {
 #pragma unroll
-  for (int a = 0; a < NW; ++a)
+    for (int a = 0; a < NW; ++a)
 #pragma unroll
-    for (int c = 0; c < 4; ++c) part[warp][a * 4 + c][lane] = acc[a][c];
-  __syncthreads();
-  // warp c finishes accumulator c: weight row g + 8 (c / 2), the tile's row 2 q + c % 2
-  float v[NW];
+      for (int c = 0; c < 4; ++c) few_part[(warp * NW * 4 + a * 4 + c) * 32 + lane] = acc[a][c];
+    __syncthreads();
+  }
+  // accumulator c of a lane: weight row g + 8 (c / 2), the tile's row 2 q + c % 2; warp c finishes it
 #pragma unroll
-  for (int a = 0; a < NW; ++a) v[a] = part[0][a * 4 + warp][lane] + part[1][a * 4 + warp][lane] + part[2][a * 4 + warp][lane] + part[3][a * 4 + warp][lane];
-  const int n = n0 + g + 8 * (warp >> 1), r = 2 * q + (warp & 1);
-  const int pair = sorted[tile * MOE_FEW + r];
-  if (n >= n_out || pair < 0) return;
-  const float by = UP && in_scale ? in_scale[pair] : 1.f;
-  if (MODE == 1) {
-    y[((size_t)tile * MOE_FEW + r) * n_out + n] = from_f<bf16>(moe_gate(rnd<bf16>(v[0] * by), rnd<bf16>(v[NW - 1] * by), limit));
-  } else if (MODE == 2) {
-    const float u = fmaxf(rnd<bf16>(v[0] * by), 0.f);
-    y[((size_t)tile * MOE_FEW + r) * n_out + n] = from_f<bf16>(u * u);
-  } else {
-    y[(size_t)pair * n_out + n] = from_f<bf16>(v[0]);
+  for (int c = 0; c < 4; ++c) {
+    if (warps > 1 && c % warps != warp) continue;
+    float v[NW];
+#pragma unroll
+    for (int a = 0; a < NW; ++a) {
+      v[a] = acc[a][c];
+      if (warps > 1) {
+        v[a] = few_part[(a * 4 + c) * 32 + lane];
+        for (int p = 1; p < warps; ++p) v[a] += few_part[(p * NW * 4 + a * 4 + c) * 32 + lane];
+      }
+    }
+    const int n = n0 + g + 8 * (c >> 1), r = 2 * q + (c & 1);
+    const int pair = sorted[tile * MOE_FEW + r];
+    if (n >= n_out || pair < 0) continue;
+    const float by = UP && in_scale ? in_scale[pair] : 1.f;
+    if (MODE == 1) {
+      y[((size_t)tile * MOE_FEW + r) * n_out + n] = from_f<bf16>(moe_gate(rnd<bf16>(v[0] * by), rnd<bf16>(v[NW - 1] * by), limit));
+    } else if (MODE == 2) {
+      const float u = fmaxf(rnd<bf16>(v[0] * by), 0.f);
+      y[((size_t)tile * MOE_FEW + r) * n_out + n] = from_f<bf16>(u * u);
+    } else {
+      y[(size_t)pair * n_out + n] = from_f<bf16>(v[0]);
+    }
   }
 }
 
@@ -1010,8 +1052,13 @@ static int moe_tiles_mode(int dtype, int tile_rows, const void* x, const void* w
                           float limit, const float* in_scale, cudaStream_t s) {
   if (tile_rows == MOE_FEW) {
     if (dtype != 1 || k_dim % 8 || ((uintptr_t)x % 16) || ((uintptr_t)w % 16)) return -2;
-    return launch_dependent(moe_few_kernel<MODE>, dim3(max_tiles, (n_out + 15) / 16), dim3(128), 0, s, (const bf16*)x, (const bf16*)w,
-                            (bf16*)y, sorted, tile_expert, n_tiles, k_dim, n_out, top, limit, in_scale);
+    // warps a block: the fewest that bring MOE_FEW_WARPS to every SM (all are there at once), each with two steps and more
+    const long long items = (long long)max_tiles * ((n_out + 15) / 16);
+    int warps = 1;
+    while (warps < 8 && items * warps < 148 * MOE_FEW_WARPS && k_dim >= 32 * 4 * warps) warps *= 2;
+    const size_t smem = warps > 1 ? (size_t)warps * (MODE == 1 ? 8 : 4) * 32 * sizeof(float) : 0;
+    return launch_dependent(moe_few_kernel<MODE>, dim3((n_out + 15) / 16, max_tiles), dim3(32 * warps), smem, s, (const bf16*)x,
+                            (const bf16*)w, (bf16*)y, sorted, tile_expert, n_tiles, k_dim, n_out, top, limit, in_scale);
   }
   if (tile_rows == MOE_BIG) {
     if (dtype != 1 || k_dim % 16 || n_out % 2 || ((uintptr_t)x % 16) || ((uintptr_t)w % 16) || ((uintptr_t)y % 4)) return -2;

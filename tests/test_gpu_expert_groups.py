@@ -161,3 +161,23 @@ def test_operands_off_their_alignment_are_refused(tokens, which):
     with pytest.raises(ops.KernelError, match="16-byte aligned"):
         ops.moe_experts(h, ids, weights, gate_up, down, expert="gated_silu")
     assert bool((ops.moe_experts(h, ids, weights, gate_up, down, expert="gated_silu", tile_rows=32) == 0).all())
+
+
+# the few-row kernel: one to eight warps a block, k ranges shorter than what its warps keep in flight, weight rows that end inside a block
+@pytest.mark.parametrize("width, inner, experts, top, tokens", [(16, 16, 2, 1, 1), (48, 144, 3, 2, 5), (272, 6416, 4, 2, 3),
+                                                                (1040, 2064, 16, 4, 8), (2064, 80, 8, 3, 2)])
+@pytest.mark.parametrize("expert", ["gated_silu", "relu2", "gated_clamped"])
+def test_few_rows_an_expert(width, inner, experts, top, tokens, expert):
+    from starter_b200 import ops
+
+    gen = torch.Generator().manual_seed(width + inner)
+    wide = inner if expert == "relu2" else 2 * inner
+    h = torch.randn(tokens, width, generator=gen).to(BF).cuda()
+    up = (torch.randn(experts, wide, width, generator=gen) * width ** -0.5).to(BF).cuda()
+    down = (torch.randn(experts, width, inner, generator=gen) * inner ** -0.5).to(BF).cuda()
+    ids = torch.stack([torch.randperm(experts, generator=gen)[:top] for _ in range(tokens)]).int().cuda()
+    weights = torch.rand(tokens, top, generator=gen).cuda()
+    got = ops.moe_experts(h, ids, weights, up, down, limit=7.0, expert=expert, tile_rows=8).double()
+    want = plain(h, ids, weights, up, down, expert, 7.0, inner, False)
+    # (the result is rounded to 8 bits, a mean of 2^-10 of it, and so is what falls on the other side of a rounding before)
+    assert float((got - want).norm() / want.norm()) < 2.0 ** -8
