@@ -209,9 +209,20 @@ __device__ __forceinline__ float2 peer_load2(uint32_t a) {
 // The rows of this CTA's share, by its first 256 threads: 16 threads a row, eight columns each.  ml: [2 tiles][128 rows] of (reference,
 // sum); finish(t, r, reference, sum) gives the factor of the row's summed outputs; dst: output row 0 of the block, `cols` entries of a
 // head, rows `stride` apart.
+// gate: null, or rows (ld entries apart) of the output's columns, by whose sigmoid it is multiplied.
+__device__ __forceinline__ void gate8(float* o, const bf16* gate) {
+  const uint4 g = *reinterpret_cast<const uint4*>(gate);
+  const uint32_t w[4] = {g.x, g.y, g.z, g.w};
+#pragma unroll
+  for (int e = 0; e < 8; ++e) {
+    const float z = __uint_as_float(e & 1 ? w[e / 2] & 0xffff0000u : w[e / 2] << 16);
+    // (rounded to bfloat16 at once: the fast quotient, both sides by a quarter, since it is zero for divisors above 2^126)
+    o[e] = __fdividef(0.25f * o[e], fmaf(0.25f, __expf(-z), 0.25f));
+  }
+}
 template <int PC, int COLS, int Q_BYTES, int P_BYTES, typename Finish>
 __device__ __forceinline__ void merge_parts(uint8_t* q_sm, uint8_t* p_sm, float2* ml, int rank, int splits, int rows_valid, int cols,
-                                            bf16* dst, size_t stride, Finish finish) {
+                                            bf16* dst, size_t stride, Finish finish, const bf16* gate = nullptr, size_t gate_ld = 0) {
   const int share = 2 * TC_BQ / splits, c = (threadIdx.x & 15) * 8;
   if (c >= COLS || c >= cols) return;
   for (int n = threadIdx.x >> 4; n < share; n += 16) {
@@ -238,10 +249,13 @@ __device__ __forceinline__ void merge_parts(uint8_t* q_sm, uint8_t* p_sm, float2
       o[4] = fmaf(w, y.x, o[4]); o[5] = fmaf(w, y.y, o[5]); o[6] = fmaf(w, y.z, o[6]); o[7] = fmaf(w, y.w, o[7]);
     }
     const float inv = finish(row, top, sum);
+#pragma unroll
+    for (int e = 0; e < 8; ++e) o[e] *= inv;
+    if (gate) gate8(o, gate + (size_t)row * gate_ld + c);
     uint32_t w[4];
 #pragma unroll
     for (int e = 0; e < 4; ++e) {
-      const __nv_bfloat162 two = __floats2bfloat162_rn(o[2 * e] * inv, o[2 * e + 1] * inv);
+      const __nv_bfloat162 two = __floats2bfloat162_rn(o[2 * e], o[2 * e + 1]);
       w[e] = *reinterpret_cast<const uint32_t*>(&two);
     }
     *reinterpret_cast<uint4*>(dst + (size_t)row * stride + c) = make_uint4(w[0], w[1], w[2], w[3]);

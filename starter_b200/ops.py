@@ -1817,12 +1817,13 @@ def latent_prompt_takes(dtype, ctx, dim, rot, vdim, rank, scale, window=None, he
     return rows <= LATENT_PROMPT_ROWS and 2 * rows * (heads * (dim + vdim) + rank + rot) <= max(LATENT_PROMPT_BYTES, scored)
 
 
-def latent_attention_prompt(q, ukv, store, block_table, ctx, heads, dim, vdim, rank, rot, scale, window=None, sink=None):
+def latent_attention_prompt(q, ukv, store, block_table, ctx, heads, dim, vdim, rank, rot, scale, window=None, sink=None, turn=None, gate=None):
     """Latent attention over keys and values that are formed from the cached rows first: ``q`` ``[T, heads * (dim + rot)]``
     (the last ``rot`` entries of a head turned), ``ukv`` ``[heads * dim + heads * vdim, rank]`` (the heads' key, then value
     up-projections).  The sequences' rows that the step's queries see are brought behind one another, one product forms the
     plain keys and the values of all heads, and the tcgen05 kernel attends.  Returns ``[T, heads * vdim]``: the heads'
-    outputs, already in value space."""
+    outputs, already in value space.  With ``turn = (cos, sin, tok_pos, rot_dims, layout)`` the heads' last entries are yet to be
+    turned (``latent_rotate_q``, in place); with ``gate = (tensor, first column)`` the result is ``sigmoid_gate``'s of it."""
     _need(q, "q", torch.bfloat16, 2)
     _need(ukv, "ukv", q.dtype, 2)
     n_tokens = q.shape[0]
@@ -1840,18 +1841,36 @@ def latent_attention_prompt(q, ukv, store, block_table, ctx, heads, dim, vdim, r
     gathered = _empty(q, (rows * (rank + rot),))
     c, shared = gathered[:rows * rank].view(rows, rank), gathered[rows * rank:].view(rows, rot)
     lib = _lib("attention_latent_prompt")
+    turned = [None, None, None, 0, None, 0, 0, 0]
+    if turn is not None:
+        cos, sin, tok_pos, rot_dims, layout = turn
+        if layout == "interleaved" and rot == rot_dims == 64 and dim % 8 == 0 and cos.shape[1] % 4 == 0 and n_seqs <= 1024 and \
+                not (q.data_ptr() | cos.data_ptr() | sin.data_ptr()) % 16:
+            _need(cos, "cos table", torch.float32, 2)
+            _need(sin, "sin table", torch.float32, 2)
+            _need(tok_pos, "tok_pos", torch.int32, 1)
+            turned = [q, cos, sin, cos.shape[1], tok_pos, n_tokens, heads, dim]
+        else:
+            latent_rotate_q(q, q.view(n_tokens, heads, -1), cos, sin, tok_pos, heads, dim, rot, rot_dims, dim, layout=layout)
     rc = lib.sb_latent_gather(store, block_table, block_table.shape[1], ctx.seq_slot, ctx.seq_q_len,
                               ctx.seq_kv_len, n_seqs, max(each), c, shared, rank, rot, int(window or 0),
-                              _stream())
+                              *turned, _stream())
     _check(rc, "latent_gather")
     kv = linear(c, ukv, status=ctx.status)
     out = _empty(q, (n_tokens, heads * vdim))
+    gated = [None, 0]
+    if gate is not None:
+        at = _gate_at(gate, q.dtype, n_tokens, heads * vdim, heads)
+        if at % 16 == 0 and gate[0].shape[1] % 8 == 0:
+            gated = [at, gate[0].shape[1]]
     rc = lib.sb_latent_prompt(
         q, kv, shared, out, ctx.seq_q_start, ctx.seq_q_len, ctx.seq_kv_len,
         ctx.block_seq, ctx.block_first, ctx.block_seq.shape[0], n_tokens, rows, heads, dim, vdim,
         scale, int(window or 0), _latent_sink(sink, heads), ctx.status,
-        prompt_splits(heads * ctx.block_first.shape[0], ctx.max_kv_len, window), _stream())
+        prompt_splits(heads * ctx.block_first.shape[0], ctx.max_kv_len, window), *gated, _stream())
     _check(rc, "latent_attention_prompt")
+    if gate is not None and gated[0] is None:
+        sigmoid_gate(out, *gate)
     return out
 
 

@@ -105,12 +105,10 @@ class LatentAttention(Part):
         n = q.shape[0]
         if ops.latent_prompt_takes(q.dtype, ctx, s.head_dim, s.rot_dim, s.value_dim, s.kv_rank, s.scale, s.window,
                                    s.num_heads):
-            ops.latent_rotate_q(q, q.view(n, s.num_heads, -1), cos, sin, ctx.tok_pos, s.num_heads, s.head_dim, s.rot_dim,
-                                s.position.dims, s.head_dim, layout=rotation.layout)
             a = ops.latent_attention_prompt(q, self.ukv, store, cache.block_table, ctx, s.num_heads, s.head_dim, s.value_dim,
-                                            s.kv_rank, s.rot_dim, s.scale, s.window, self.sink)
-            if s.output_gate:
-                ops.sigmoid_gate(a, proj, s.q_rank)
+                                            s.kv_rank, s.rot_dim, s.scale, s.window, self.sink,
+                                            turn=(cos, sin, ctx.tok_pos, s.position.dims, rotation.layout),
+                                            gate=(proj, s.q_rank) if s.output_gate else None)
             return ops.linear(a, self.o, status=ctx.status)
         keys = s.num_heads * s.head_dim
         fold, unfold = ops.latent_heads_take(q, s.head_dim, s.rot_dim, s.kv_rank, s.value_dim, ctx.max_q_len)

@@ -126,3 +126,53 @@ def test_rotated_queries_in_pieces(rot, dims, dim, rank, n):
     want[..., 0:dims:2], want[..., 1:dims:2] = src[..., 0:dims:2] * c - src[..., 1:dims:2] * s, src[..., 1:dims:2] * c + src[..., 0:dims:2] * s
     assert bool(((qa[..., rank:].double() - want).abs() <= HALF_STEP * want.abs() + 2.0 ** -22 * src.abs().max()).all())
     assert not bool(qa[..., :rank].any())
+
+
+# the layer's own kernels on one side: queries turned beside the gathering and the gate in the attention's last step, with the keys of a
+# block of queries whole and in parts; on the other the turn and the gate by themselves
+@pytest.mark.parametrize("past, new, parts", [(0, 300, 1), (1200, 130, 4)])
+@pytest.mark.parametrize("sink", [True, False])
+def test_latent_prompt_turns_and_gates(past, new, parts, sink, monkeypatch):
+    from starter_b200 import ops
+    from starter_b200.cache import SequenceCache
+    from starter_b200.config import InterleavedRopeSpec
+    from starter_b200.engine import StepContext, StepEntry, plan_step
+    from starter_b200.engine.batch import upload
+    from starter_b200.cache.layout import KVNeed
+    from starter_b200.parts import InterleavedRotaryTable
+
+    heads, dim, rot, vdim, rank = 4, 128, 64, 128, 256
+    gen = torch.Generator().manual_seed(new)
+    rand = lambda *shape: torch.randn(*shape, generator=gen).cuda()
+    cache = SequenceCache({0: KVNeed(1, rank + rot, None, 0)}, {0: None}, past + new + 64, 1, BF, "cuda")
+    slot = cache.open_sequence()
+    cache.reserve(slot, past + new)
+    cache.lengths[slot] = past
+    arrays = plan_step([StepEntry(slot, [0] * new, [])], [past])
+    cache.sync_table()
+    dev = upload(arrays, torch.device("cuda:0"))
+    ctx = StepContext(n_tokens=new, n_seqs=1, max_q_len=new, max_kv_len=past + new, cache=cache, host=arrays,
+                      status=torch.zeros(1, dtype=torch.int32, device="cuda"),
+                      **{k: dev[k] for k in ("tokens", "tok_pos", "tok_slot", "seq_slot", "seq_q_start", "seq_q_len", "seq_kv_len", "want_rows",
+                                             "tile_seq", "tile_first", "block_seq", "block_first")})
+    store, _ = cache.entry_pages(0)
+    store.copy_(rand(*store.shape).to(BF))
+    tables = InterleavedRotaryTable(InterleavedRopeSpec(dims=rot, base=100.0), BF, "cuda")
+    tables.ensure(past + new)
+    cos, sin = ops.latent_tables(tables.rotation(), rot)
+    q, ukv = rand(new, heads * (dim + rot)).to(BF), (rand(heads * (dim + vdim), rank) * rank ** -0.5).to(BF)
+    wide, sinks = (rand(new, 24 + heads * vdim) * 4).to(BF), rand(heads) if sink else None
+    assert ops.prompt_splits(heads * ctx.block_first.shape[0], ctx.max_kv_len) == parts
+    other = q.clone()
+    args = (ukv, store, cache.block_table, ctx, heads, dim, vdim, rank, rot, 192 ** -0.5, None, sinks)
+    turn = (cos, sin, ctx.tok_pos, rot, "interleaved")
+    got = ops.latent_attention_prompt(q, *args, turn=turn, gate=(wide, 16)).double()
+    ops.latent_rotate_q(other, other.view(new, heads, -1), cos, sin, ctx.tok_pos, heads, dim, rot, rot, dim)
+    assert torch.equal(q, other)
+    plain = ops.latent_attention_prompt(other, *args).double()
+    want = plain * torch.sigmoid(wide[:, 16:16 + heads * vdim].double())
+    # (the plain result is rounded to 8 bits, the gated one once more)
+    assert bool(((got - want).abs() <= 2.01 * HALF_STEP * want.abs() + 1e-7).all())
+    off = ops.latent_attention_prompt(other, *args, gate=(wide, 12)).double()        # (not on 16 bytes: a kernel of its own)
+    want = plain * torch.sigmoid(wide[:, 12:12 + heads * vdim].double())
+    assert bool(((off - want).abs() <= 2.01 * HALF_STEP * want.abs() + 1e-7).all())
