@@ -62,6 +62,7 @@ SOURCES = (
     "attention_sink",
     "attention_sink_tc",
     "short_conv",
+    "sink_conv",
     "state_scan",
     "state_scan_prompt",
     "state_step",

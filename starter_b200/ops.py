@@ -2257,23 +2257,8 @@ def sink_prepare_rot(proj, heads, kv_heads, dim, vdim, tok_pos, tok_slot, block_
     _check(rc, "sink_prepare_rot")
 
 
-def sink_prepare_norm(proj, heads, kv_heads, dim, vdim, tok_pos, tok_slot, block_table, k_store, v_store, rotation=None,
-                      row_norm=None, unit_values=False, eps=0.0, write_cache=True):
-    """``sink_prepare_rot`` for rotations of either layout, with norms: ``proj`` = ``[q | k | v]`` (``[q]`` with ``write_cache``
-    false; up to 7 unused entries may follow).  ``row_norm = (q_gain, k_gain)`` (float32 ``[heads * dim]``, ``[kv_heads *
-    dim]`` or None when nothing is filed): queries and keys are RMS-normed over their whole rows first.  ``rotation`` (a
-    ``Rotation`` or None): entry ``i`` of a head's leading ``dims`` entries turns with entry ``i + dims / 2`` (half-split
-    layout), or entry ``2i`` with entry ``2i + 1`` (interleaved).
-    ``unit_values``: a head's value is RMS-normed without a gain.  Queries change in place, keys and values are
-    filed in the cache; ``eps`` stands inside every root."""
-    _need(proj, "proj", None, 2)
-    n_tokens = proj.shape[0]
-    want = heads * dim + (kv_heads * (dim + vdim) if write_cache else 0)
-    if not want <= proj.shape[1] < want + 8:
-        raise KernelError(f"proj has width {proj.shape[1]}, expected {want} (and up to 7 entries of padding)")
-    _need(tok_pos, "tok_pos", torch.int32, 1)
-    _need(tok_slot, "tok_slot", torch.int32, 1)
-    _need(block_table, "block_table", torch.int32, 2)
+def _sink_norm_operands(proj, heads, kv_heads, dim, vdim, k_store, v_store, rotation, row_norm, write_cache):
+    """The checked rotation, gains and stores of ``sink_prepare_norm``: ``(rot, cos, sin, pairs, q_gain, k_gain)``."""
     rot, cos_table, sin_table, pairs = 0, None, None, 0
     if rotation is not None:
         rot, cos_table, sin_table = rotation.rotary_dim, rotation.cos, rotation.sin
@@ -2297,12 +2282,61 @@ def sink_prepare_norm(proj, heads, kv_heads, dim, vdim, tok_pos, tok_slot, block
         if tuple(k_store.shape[1:]) != (kv_heads, PAGE_TOKENS, dim) or tuple(v_store.shape[1:]) != (kv_heads, PAGE_TOKENS, vdim):
             raise KernelError(f"cache pages have shapes {tuple(k_store.shape)} / {tuple(v_store.shape)}, expected "
                               f"[pages, {kv_heads}, {PAGE_TOKENS}, {dim}] / [.., {vdim}]")
+    return rot, cos_table, sin_table, pairs, q_gain, k_gain
+
+
+def sink_prepare_norm(proj, heads, kv_heads, dim, vdim, tok_pos, tok_slot, block_table, k_store, v_store, rotation=None,
+                      row_norm=None, unit_values=False, eps=0.0, write_cache=True):
+    """``sink_prepare_rot`` for rotations of either layout, with norms: ``proj`` = ``[q | k | v]`` (``[q]`` with ``write_cache``
+    false; up to 7 unused entries may follow).  ``row_norm = (q_gain, k_gain)`` (float32 ``[heads * dim]``, ``[kv_heads *
+    dim]`` or None when nothing is filed): queries and keys are RMS-normed over their whole rows first.  ``rotation`` (a
+    ``Rotation`` or None): entry ``i`` of a head's leading ``dims`` entries turns with entry ``i + dims / 2`` (half-split
+    layout), or entry ``2i`` with entry ``2i + 1`` (interleaved).
+    ``unit_values``: a head's value is RMS-normed without a gain.  Queries change in place, keys and values are
+    filed in the cache; ``eps`` stands inside every root."""
+    _need(proj, "proj", None, 2)
+    n_tokens = proj.shape[0]
+    want = heads * dim + (kv_heads * (dim + vdim) if write_cache else 0)
+    if not want <= proj.shape[1] < want + 8:
+        raise KernelError(f"proj has width {proj.shape[1]}, expected {want} (and up to 7 entries of padding)")
+    _need(tok_pos, "tok_pos", torch.int32, 1)
+    _need(tok_slot, "tok_slot", torch.int32, 1)
+    _need(block_table, "block_table", torch.int32, 2)
+    rot, cos_table, sin_table, pairs, q_gain, k_gain = _sink_norm_operands(proj, heads, kv_heads, dim, vdim, k_store, v_store, rotation,
+                                                                           row_norm, write_cache)
     rc = _lib("attention_sink").sb_sink_prepare_norm(
         _code(proj.dtype), proj, proj.shape[1], tok_pos, tok_slot, block_table,
         block_table.shape[1], k_store if write_cache else None, v_store if write_cache else None,
         cos_table, sin_table, rot, q_gain, k_gain, eps, int(unit_values), n_tokens,
         heads, kv_heads, dim, vdim, int(write_cache), pairs, _stream())
     _check(rc, "sink_prepare_norm")
+
+
+def sink_conv_prepare(proj, taps, in_bias, state, state_at, seq_slot, seq_q_start, seq_q_len, max_q_len, heads, kv_heads, dim, vdim,
+                      tok_pos, tok_slot, block_table, k_store, v_store, rotation=None, row_norm=None, unit_values=False, eps=0.0):
+    """``short_conv`` over the ``[q | k | v]`` of ``proj`` (no activation, no bias behind it) and ``sink_prepare_norm`` of what it gives: keys
+    and values are filed, the queries returned (the leading columns of what comes back).  One kernel (csrc/sink_conv.cu) for the
+    sizes that it takes, else those two."""
+    channels = taps.shape[0]
+    if proj.dtype == torch.bfloat16 and not unit_values and (rotation is None or rotation.layout == "interleaved") and \
+            channels == heads * dim + kv_heads * (dim + vdim):
+        _need(proj, "proj", torch.bfloat16, 2)
+        slot_floats = _conv_operands(proj, 0, channels, taps, None, in_bias, state, state_at)
+        _need(tok_pos, "tok_pos", torch.int32, 1)
+        _need(block_table, "block_table", torch.int32, 2)
+        rot, cos, sin, _, q_gain, k_gain = _sink_norm_operands(proj, heads, kv_heads, dim, vdim, k_store, v_store, rotation, row_norm, True)
+        n_seqs = _seq_arrays(seq_slot, seq_q_start, seq_q_len)
+        q = _empty(proj, (proj.shape[0], heads * dim))
+        rc = _lib("sink_conv").sb_sink_conv(
+            proj, proj.shape[1], taps, taps.shape[1], in_bias, _at(state, state_at) if state is not None else None, slot_floats, seq_slot,
+            seq_q_start, seq_q_len, n_seqs, int(max_q_len), tok_pos, block_table, block_table.shape[1], q_gain, k_gain, eps, cos, sin, rot,
+            heads, kv_heads, dim, vdim, q, k_store, v_store, _stream())
+        if rc != -2:
+            _check(rc, "sink_conv")
+            return q
+    proj = short_conv(proj, 0, channels, taps, None, in_bias, state, state_at, seq_slot, seq_q_start, seq_q_len, max_q_len)
+    sink_prepare_norm(proj, heads, kv_heads, dim, vdim, tok_pos, tok_slot, block_table, k_store, v_store, rotation, row_norm, unit_values, eps)
+    return proj
 
 
 def _sink_check(q, k_store, v_store, heads, kv_heads, dim, vdim, penalty, sink, gate):
@@ -2516,15 +2550,8 @@ def conv_max_taps() -> int:
     return _lib("short_conv").sb_conv_max_taps()
 
 
-def short_conv(x, col, channels, taps, bias, in_bias, state, state_at, seq_slot, seq_q_start, seq_q_len, max_q_len,
-               activation=None):
-    """A causal convolution over time with one filter per channel, over the sequences of a step:
-    ``y[t, c] = act(bias[c] + sum_j taps[c, K - 1 - j] * (x[t - j, col + c] + in_bias[c]))``, zeros in front of a
-    sequence.  ``x`` ``[T, N]`` (the channels are its columns ``col .. col + channels``); ``taps`` float32
-    ``[channels, K]``; ``bias``, ``in_bias`` float32 ``[channels]`` or None; ``activation`` None or ``"silu"``.
-    ``state`` float32 ``[slots, M]`` (None with one tap): a slot's last ``K - 1`` inputs (``(K - 1) * channels`` floats from
-    ``state_at`` on) stand in front of the tokens it brings and are replaced by the step's last ones.
-    ``max_q_len``: the most tokens a sequence brings.  Returns ``[T, channels]`` in the type of ``x``."""
+def _conv_operands(x, col, channels, taps, bias, in_bias, state, state_at) -> int:
+    """Checks a short convolution's operands; the floats of a slot."""
     _need(x, "x", None, 2)
     _need(taps, "taps", torch.float32, 2)
     k = taps.shape[1]
@@ -2541,6 +2568,20 @@ def short_conv(x, col, channels, taps, bias, in_bias, state, state_at, seq_slot,
     if col < 0 or col + channels > x.shape[1] or state_at < 0 or (k > 1 and state_at + (k - 1) * channels > slot_floats):
         raise KernelError(f"{channels} channels from column {col} of rows of {x.shape[1]}, or {k - 1} rows of them from "
                           f"float {state_at} of a slot's {slot_floats}, do not fit")
+    return slot_floats
+
+
+def short_conv(x, col, channels, taps, bias, in_bias, state, state_at, seq_slot, seq_q_start, seq_q_len, max_q_len,
+               activation=None):
+    """A causal convolution over time with one filter per channel, over the sequences of a step:
+    ``y[t, c] = act(bias[c] + sum_j taps[c, K - 1 - j] * (x[t - j, col + c] + in_bias[c]))``, zeros in front of a
+    sequence.  ``x`` ``[T, N]`` (the channels are its columns ``col .. col + channels``); ``taps`` float32
+    ``[channels, K]``; ``bias``, ``in_bias`` float32 ``[channels]`` or None; ``activation`` None or ``"silu"``.
+    ``state`` float32 ``[slots, M]`` (None with one tap): a slot's last ``K - 1`` inputs (``(K - 1) * channels`` floats from
+    ``state_at`` on) stand in front of the tokens it brings and are replaced by the step's last ones.
+    ``max_q_len``: the most tokens a sequence brings.  Returns ``[T, channels]`` in the type of ``x``."""
+    slot_floats = _conv_operands(x, col, channels, taps, bias, in_bias, state, state_at)
+    k = taps.shape[1]
     if activation not in (None, "silu"):
         raise KernelError(f"the short convolution applies silu or nothing, not {activation!r}")
     n_seqs = _seq_arrays(seq_slot, seq_q_start, seq_q_len)

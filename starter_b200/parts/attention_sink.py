@@ -165,15 +165,22 @@ class SinkAttention(Part):
             raise ValueError("this attention's biases and convolutions cover keys and values; it cannot only read")
         weight = self.qkvg if writes_cache else self.qg
         proj = ops.linear(x, weight, status=ctx.status)
-        if self.taps is not None:
-            proj = ops.short_conv(proj, 0, self.convolved, self.taps, None, self.biases, cache.entry_state(entry),
-                                  self.state_at, ctx.seq_slot, ctx.seq_q_start, ctx.seq_q_len, ctx.max_q_len)
+        conv = (self.taps, self.biases, cache.entry_state(entry), self.state_at, ctx.seq_slot, ctx.seq_q_start, ctx.seq_q_len,
+                ctx.max_q_len) if self.taps is not None else None
+        if conv is not None and not self.normed:
+            proj = ops.short_conv(proj, 0, self.convolved, conv[0], None, *conv[1:])
         if self.normed:
-            # queries normed and turned in place; keys normed and turned, values normed on their way into the cache
-            ops.sink_prepare_norm(proj, s.num_heads, s.num_kv_heads, s.head_dim, s.value_dim, ctx.tok_pos, ctx.tok_slot,
-                                  cache.block_table, keys, values,
-                                  self.position.rotation() if self.position is not None else None, self.row_norm,
-                                  s.unit_values, s.norm_eps, write_cache=writes_cache)
+            # queries normed and turned; keys normed and turned, values normed on their way into the cache
+            if conv is not None:
+                proj = ops.sink_conv_prepare(proj, *conv, s.num_heads, s.num_kv_heads, s.head_dim, s.value_dim, ctx.tok_pos, ctx.tok_slot,
+                                             cache.block_table, keys, values,
+                                             self.position.rotation() if self.position is not None else None, self.row_norm,
+                                             s.unit_values, s.norm_eps)
+            else:
+                ops.sink_prepare_norm(proj, s.num_heads, s.num_kv_heads, s.head_dim, s.value_dim, ctx.tok_pos, ctx.tok_slot,
+                                      cache.block_table, keys, values,
+                                      self.position.rotation() if self.position is not None else None, self.row_norm,
+                                      s.unit_values, s.norm_eps, write_cache=writes_cache)
             a = ops.sink_attention_step(proj, keys, values, cache.block_table, ctx, s.num_heads, s.num_kv_heads,
                                         s.head_dim, s.value_dim, s.scale, self.penalty, self.sink, None, s.chunk, s.window,
                                         s.keep_first, s.softcap)
