@@ -93,10 +93,10 @@ def _refuse(t, name, dtype=None, ndim=None):
 # launch, are native too (csrc/host.cpp).  The first call of any of them loads the native part and puts it in these names.
 
 def _bind():
-    global _need, _empty, _stream
+    global _need, _empty, _stream, _product
     host = build.load_host()
     host.refuse_with(_refuse)
-    _need, _empty, _stream = host.need, host.empty, host.stream
+    _need, _empty, _stream, _product = host.need, host.empty, host.stream, host.product
     return host
 
 
@@ -112,6 +112,13 @@ def _empty(like, shape, dtype=None):
 def _stream():
     """The current CUDA stream's address."""
     return _bind().stream()
+
+
+def _product(x, weight, low, high):
+    """``x @ weight.T`` by the library's product for plain bfloat16 matrices of ``low < rows < high``, or None."""
+    if isinstance(x, torch.Tensor) and x.is_cuda:
+        return _bind().product(x, weight, low, high)
+    return None
 
 
 class _Added:
@@ -248,6 +255,10 @@ def linear(x, weight, out_float=False, gated=False, status=None, add_to=None):
     returns float32 whatever the working type (used for logits).  ``status`` (int32 ``[1]``) is the
     device word in which the tensor-core kernel reports a wait that ran out.
     """
+    if not out_float:
+        y = _product(x, weight, TENSOR_CORE_MAX_ROWS, PROMPT_MIN_ROWS)
+        if y is not None and (not gated or y.shape[1] % 2 == 0):
+            return swiglu(y, gated) if gated else y
     _need(x, "x", None, 2)
     _need(weight, "weight", x.dtype, 2)
     rows, k_dim = x.shape
