@@ -730,6 +730,194 @@ latent_merge_kernel(const float* __restrict__ part_acc, const float* __restrict_
   *reinterpret_cast<uint2*>(out + (size_t)row * rank + c) = o;
 }
 
+// Single tokens of up to 16 heads: the rows of a sequence are one 16-row tile, which leaves three of the four row groups above (and six
+// of its eight warps) with nothing to do but loads.  Here a block takes a page of 64 keys at a time and all eight warps share it: a
+// warp scores eight of the keys, then, behind a barrier, sums its eighth of the latent's columns over all of them.  Pages arrive two ahead by
+// cp.async, rows behind the token as zeros.  Parts, references and sums are filed as above.  Measured (us a layer of 16 heads, captured,
+// the kernel above -> this one): rank 512, 1 sequence of 1,500 40.3 -> 36.9, 8 of up to 2,048 46.6 -> 45.2, 20 of up to 400 50.6 -> 49.1, 30 in a window
+// of 512 58.2 -> 56.9; rank 256, 4 in a window of 512 30.9 -> 29.2, 8 of up to 1,063 33.6 -> 33.4.
+#define LS_KEYS SB_PAGE_TOKENS
+#define LS_PLD (LS_KEYS + 8)
+template <int NP>   // 16-column pairs of value tiles a warp sums
+__global__ void __launch_bounds__(256, 1)
+latent_step_kernel(const bf16* __restrict__ qa, bf16* __restrict__ out, float* __restrict__ part_acc, float* __restrict__ part_ml,
+                   const bf16* __restrict__ store, const int* __restrict__ block_table, int table_stride, const int* __restrict__ seq_slot,
+                   const int* __restrict__ seq_q_start, const int* __restrict__ seq_q_len, const int* __restrict__ seq_kv_len, int heads,
+                   int rank, int rot, float scale, int window, int n_rows_total, const float* __restrict__ sink) {
+  extern __shared__ __align__(16) unsigned char latent_smem[];
+  const int Dk = rank + rot, ld = Dk + 8, pieces = Dk / 8;
+  bf16* qs = reinterpret_cast<bf16*>(latent_smem);                // [16][ld]
+  bf16* ks = qs + 16 * ld;                                        // [2][64][ld]
+  __shared__ __align__(16) bf16 ps[16 * LS_PLD];
+  __shared__ float tops[8][16], sums[8][16];
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, g = lane >> 2, tq = lane & 3;
+  const int seq = blockIdx.x, split = blockIdx.y, n_splits = gridDim.y;
+  pdl_wait();
+  SB_BEHIND_WAIT(qa); SB_BEHIND_WAIT(store); SB_BEHIND_WAIT(block_table);
+  SB_BEHIND_WAIT(seq_slot); SB_BEHIND_WAIT(seq_q_start); SB_BEHIND_WAIT(seq_q_len); SB_BEHIND_WAIT(seq_kv_len);
+  if (seq_q_len[seq] < 1) return;
+  const int last = seq_kv_len[seq] - 1;                           // the token's own position
+  const size_t row0 = (size_t)seq_q_start[seq] * heads;
+  const int* pages = block_table + (size_t)seq_slot[seq] * table_stride;
+  const int first = window > 0 ? max(0, last - window + 1) : 0;
+  const int p_lo = first / LS_KEYS, n_pages = last / LS_KEYS - p_lo + 1, per = (n_pages + n_splits - 1) / n_splits;
+  const int begin = p_lo + split * per, end = min(p_lo + n_pages, begin + per);
+  // a warp eight rows of a page, a lane pieces lane, lane + 32, ..
+  auto load_page = [&](int p) {
+    const bf16* from = store + (size_t)pages[p] * LS_KEYS * Dk;
+    bf16* to = ks + (size_t)((p - begin) & 1) * LS_KEYS * ld;
+#pragma unroll
+    for (int k = 0; k < 8; ++k) {
+      const int r = warp * 8 + k;
+      const bool real = p * LS_KEYS + r <= last;
+      for (int c = lane; c < pieces; c += 32) cp_async16(to + r * ld + c * 8, from + (real ? (size_t)r * Dk + c * 8 : 0), real);
+    }
+  };
+#pragma unroll
+  for (int k = 0; k < 2; ++k) {
+    const int r = warp * 2 + k;
+    for (int c = lane; c < pieces; c += 32) cp_async16(qs + r * ld + c * 8, qa + (row0 + (r < heads ? r : 0)) * Dk + c * 8, r < heads);
+  }
+  if (begin < end) load_page(begin);
+  cp_async_commit();
+  if (begin + 1 < end) load_page(begin + 1);
+  cp_async_commit();
+  if (gridDim.x * gridDim.y <= 148) pdl_trigger();               // (all blocks are there: what follows may take its place beside them)
+  float o[2 * NP][4];
+#pragma unroll
+  for (int n = 0; n < 2 * NP; ++n) o[n][0] = o[n][1] = o[n][2] = o[n][3] = 0.f;
+  float m_run[2] = {-INFINITY, -INFINITY}, l_run[2] = {0.f, 0.f};
+  const int n_pairs = rank / 16, mi = lane >> 3;
+  for (int p = begin; p < end; ++p) {
+    cp_async_wait<1>();
+    __syncthreads();                                // the page is there
+    const bf16* kb = ks + (size_t)((p - begin) & 1) * LS_KEYS * ld;
+    // S = Q K^T of 16 rows and the warp's eight keys, steps of 32 entries of k by turns in two sums
+    float s4[2][4];
+#pragma unroll
+    for (int n = 0; n < 2; ++n) s4[n][0] = s4[n][1] = s4[n][2] = s4[n][3] = 0.f;
+    const bf16* k_at = kb + (warp * 8 + (lane & 7)) * ld + mi * 8;
+    const bf16* q_at = qs + (lane & 15) * ld + (lane >> 4) * 8;
+    int kk = 0;
+#pragma unroll 4
+    for (; kk + 32 <= Dk; kk += 32) {
+      unsigned a[4], b[4], kf[4];
+      ldsm4(a, q_at + kk);
+      ldsm4(b, q_at + kk + 16);
+      ldsm4(kf, k_at + kk);
+      mma16816(s4[0], a, kf[0], kf[1]);
+      mma16816(s4[1], b, kf[2], kf[3]);
+    }
+    if (kk < Dk) {                                  // (a last step of 16; its second half of keys is not used)
+      unsigned a[4], kf[4];
+      ldsm4(a, q_at + kk);
+      ldsm4(kf, kb + (warp * 8 + (lane & 7)) * ld + kk + (mi & 1) * 8);
+      mma16816(s4[0], a, kf[0], kf[1]);
+    }
+    float sv[4], mx[2] = {-INFINITY, -INFINITY};
+#pragma unroll
+    for (int e = 0; e < 4; ++e) {
+      const int j = p * LS_KEYS + warp * 8 + 2 * tq + (e & 1);
+      sv[e] = j >= first && j <= last ? (s4[0][e] + s4[1][e]) * scale : -INFINITY;
+      mx[e >> 1] = fmaxf(mx[e >> 1], sv[e]);
+    }
+#pragma unroll
+    for (int i = 0; i < 2; ++i) {
+      mx[i] = fmaxf(mx[i], __shfl_xor_sync(0xffffffffu, mx[i], 1));
+      mx[i] = fmaxf(mx[i], __shfl_xor_sync(0xffffffffu, mx[i], 2));
+      if (tq == 0) tops[warp][g + 8 * i] = mx[i];
+    }
+    __syncthreads();
+    float alpha[2], m_use[2];
+#pragma unroll
+    for (int i = 0; i < 2; ++i) {
+      float top = m_run[i];
+#pragma unroll
+      for (int w = 0; w < 8; ++w) top = fmaxf(top, tops[w][g + 8 * i]);
+      m_use[i] = top == -INFINITY ? 0.f : top;
+      alpha[i] = expf(m_run[i] - m_use[i]);
+      m_run[i] = top;
+      l_run[i] *= alpha[i];
+    }
+#pragma unroll
+    for (int e = 0; e < 4; ++e) {
+      sv[e] = expf(sv[e] - m_use[e >> 1]);
+      l_run[e >> 1] += sv[e];
+    }
+#pragma unroll
+    for (int i = 0; i < 2; ++i)
+      *reinterpret_cast<unsigned*>(ps + (g + 8 * i) * LS_PLD + warp * 8 + 2 * tq) = pack_bf16(sv[2 * i], sv[2 * i + 1]);
+    __syncthreads();
+    if (__any_sync(0xffffffffu, alpha[0] != 1.f || alpha[1] != 1.f)) {
+#pragma unroll
+      for (int n = 0; n < 2 * NP; ++n) {
+        o[n][0] *= alpha[0]; o[n][1] *= alpha[0];
+        o[n][2] *= alpha[1]; o[n][3] *= alpha[1];
+      }
+    }
+#pragma unroll
+    for (int k2 = 0; k2 < LS_KEYS / 16; ++k2) {
+      unsigned pa[4];
+      ldsm4(pa, ps + (lane & 15) * LS_PLD + k2 * 16 + (lane >> 4) * 8);
+      const bf16* v_at = kb + (16 * k2 + (lane & 7) + ((lane >> 3) & 1) * 8) * ld + (lane >> 4) * 8;
+#pragma unroll
+      for (int n = 0; n < NP; ++n) {
+        const int pair = warp + 8 * n;
+        if (pair < n_pairs) {
+          unsigned vf[4];
+          ldsm4_t(vf, v_at + pair * 16);
+          mma16816(o[2 * n], pa, vf[0], vf[1]);
+          mma16816(o[2 * n + 1], pa, vf[2], vf[3]);
+        }
+      }
+    }
+    __syncthreads();                                // nobody reads the page that is filled next
+    if (p + 2 < end) load_page(p + 2);
+    cp_async_commit();
+  }
+  cp_async_wait<0>();
+  if (gridDim.x * gridDim.y > 148) pdl_trigger();
+  // the sums of the warps' own keys
+#pragma unroll
+  for (int i = 0; i < 2; ++i) {
+    l_run[i] += __shfl_xor_sync(0xffffffffu, l_run[i], 1);
+    l_run[i] += __shfl_xor_sync(0xffffffffu, l_run[i], 2);
+    if (tq == 0) sums[warp][g + 8 * i] = l_run[i];
+  }
+  __syncthreads();
+#pragma unroll
+  for (int i = 0; i < 2; ++i) {
+    const int h = g + 8 * i;
+    if (h >= heads) continue;
+    float l = 0.f;
+#pragma unroll
+    for (int w = 0; w < 8; ++w) l += sums[w][h];
+    const size_t row = row0 + h;
+    if (n_splits == 1) {
+      // the sink joins at the end (of parts: where they are merged): one more weight relative to the maximum
+      float inv = 1.f / l;
+      if (sink) {
+        const float top = fmaxf(m_run[i], sink[h]), f = expf(m_run[i] - top);
+        inv = f / (l * f + expf(sink[h] - top));
+      }
+#pragma unroll
+      for (int n = 0; n < 2 * NP; ++n) {
+        const int pair = warp + 8 * (n >> 1);
+        if (pair < n_pairs)
+          *reinterpret_cast<unsigned*>(out + row * rank + pair * 16 + (n & 1) * 8 + 2 * tq) = pack_bf16(o[n][2 * i] * inv, o[n][2 * i + 1] * inv);
+      }
+    } else {
+      float* pa = part_acc + ((size_t)split * n_rows_total + row) * rank;
+#pragma unroll
+      for (int n = 0; n < 2 * NP; ++n) {
+        const int pair = warp + 8 * (n >> 1);
+        if (pair < n_pairs) *reinterpret_cast<float2*>(pa + pair * 16 + (n & 1) * 8 + 2 * tq) = make_float2(o[n][2 * i], o[n][2 * i + 1]);
+      }
+      if (warp == 0 && tq == 0) *reinterpret_cast<float2*>(part_ml + ((size_t)split * n_rows_total + row) * 2) = make_float2(m_run[i], l);
+    }
+  }
+}
+
 extern "C" {
 
 // The bfloat16 attention on tensor cores.  seq_* describe the sequences of the step (slot, first packed
@@ -745,6 +933,26 @@ int sb_latent_attention_tc(const void* qa, void* out, float* part_acc, float* pa
                            int max_q_len, const float* sink, cudaStream_t s) {
   if (n_tiles == 0 || n_tokens == 0) return 0;
   if (rank % 16 || rot % 16 || rank < 16 || rank > 512 || rank + rot > 640 || n_splits < 1 || n_splits > 32) return -2;
+  if (max_q_len == 1 && heads <= 16) {             // n_tiles: the sequences, one token each
+    const int rows = rank + rot + 8, smem = (16 + 2 * LS_KEYS) * rows * (int)sizeof(bf16);
+    const int each = (rank / 16 + 7) / 8;
+#define STEP(NP)                                                                                                                      \
+    {                                                                                                                                 \
+      cudaError_t e = cudaFuncSetAttribute(latent_step_kernel<NP>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);                \
+      if (e != cudaSuccess) return (int)e;                                                                                            \
+      const int rc = launch_dependent(latent_step_kernel<NP>, dim3(n_tiles, n_splits), dim3(256), smem, s, (const bf16*)qa,           \
+                                      (bf16*)out, part_acc, part_ml, (const bf16*)store, block_table, table_stride, seq_slot,         \
+                                      seq_q_start, seq_q_len, seq_kv_len, heads, rank, rot, scale, window, n_tokens * heads, sink);   \
+      if (rc != 0 || n_splits == 1) return rc;                                                                                        \
+    }
+    if (each <= 1) STEP(1)
+    else if (each <= 2) STEP(2)
+    else STEP(4)
+#undef STEP
+    if (!out) return 0;
+    return launch_dependent(latent_merge_kernel, dim3(n_tokens * heads), dim3(128), 0, s, (const float*)part_acc,
+                            (const float*)part_ml, (bf16*)out, n_tokens * heads, rank, n_splits, sink, heads);
+  }
   const int heads_per_block = heads < 64 ? heads : 64;
   const int tokens_per_block = 64 / heads_per_block;
   const int head_chunks = (heads + heads_per_block - 1) / heads_per_block;

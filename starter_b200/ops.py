@@ -1702,17 +1702,23 @@ def latent_attention_tc(qa, store, block_table, seq_slot, seq_q_start, seq_q_len
         qa, out, part_acc, part_ml, store, block_table, block_table.shape[1],
         seq_slot, seq_q_start, seq_q_len, seq_kv_len, tile_seq, tile_first,
         tile_seq.shape[0], n_tokens, heads, rank, rot, scale, int(window or 0), n_splits,
-        int(max_q_len), _latent_sink(sink, heads), _stream())
+        # (one token a sequence: the kernel for that takes the sequences in their order, so the list has to be all of them)
+        int(max_q_len) if max_q_len != 1 or tile_seq.shape[0] == seq_slot.shape[0] else 2, _latent_sink(sink, heads), _stream())
     _check(rc, "latent_attention_tc", 2 if n_splits > 1 and join else 1)
     return out if join else (out, part_acc, part_ml)
 
 
 def latent_splits(rows: int, heads: int, window, kv_hint: int) -> int:
-    """Into how many parts the keys of a single-token step are cut: enough blocks to fill the SMs, no part
-    shorter than a block of 32 keys, at most 32."""
+    """Into how many parts the keys of a single-token step are cut: enough blocks to fill the SMs, at most 32, no part shorter than a block
+    of 32 keys; up to 16 heads, whose kernel takes whole pages, as many as leave no part empty."""
     blocks = rows * -(-heads // 64)
-    keys = kv_hint if not window else min(window, max(kv_hint, 1))
-    return max(1, min(32, 148 // max(1, blocks), -(-max(keys, 1) // 32)))
+    keys = max(1, kv_hint if not window else min(window, max(kv_hint, 1)))
+    most = min(32, SM_COUNT // max(1, blocks))
+    if heads > 16:
+        return max(1, min(most, -(-keys // 32)))
+    pages = -(-keys // PAGE_TOKENS) + (1 if window and keys < kv_hint else 0)       # (a window begins and ends inside a page)
+    each = -(-pages // max(1, most))
+    return -(-pages // each)
 
 
 def latent_attention_step(qa, store, block_table, ctx, heads, rank, rot, scale, window=None, sink=None, join=True):
