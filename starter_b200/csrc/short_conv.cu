@@ -149,10 +149,17 @@ short_conv_vec_kernel(const bf16* __restrict__ x, int ldx, const float* __restri
   float* st = state + (size_t)seq_slot[seq] * slot_stride + c;      // row j: the input j + 1 tokens back
   const bf16* xc = x + c;
   uint2 raw[B + CHUNK];                                      // from B tokens in front of the chunk on
+  const bf16* from = xc + (long long)(q_start + t0 - B) * ldx;
+  const bool whole = t0 >= B && t0 + CHUNK <= q_len;         // (most chunks of a prompt: no token is asked whether it is there)
+  if (whole) {
 #pragma unroll
-  for (int i = 0; i < B + CHUNK; ++i) {
-    const int t = t0 + i - B;
-    raw[i] = t >= 0 && t < q_len ? *reinterpret_cast<const uint2*>(xc + (q_start + t) * ldx) : make_uint2(0u, 0u);
+    for (int i = 0; i < B + CHUNK; ++i) raw[i] = *reinterpret_cast<const uint2*>(from + (long long)i * ldx);
+  } else {
+#pragma unroll
+    for (int i = 0; i < B + CHUNK; ++i) {
+      const int t = t0 + i - B;
+      raw[i] = t >= 0 && t < q_len ? *reinterpret_cast<const uint2*>(from + (long long)i * ldx) : make_uint2(0u, 0u);
+    }
   }
   float in[K][4], old[B > 0 ? B : 1][4];                     // in[i % K]: token t0 + i - B
 #pragma unroll
@@ -167,6 +174,7 @@ short_conv_vec_kernel(const bf16* __restrict__ x, int ldx, const float* __restri
 #pragma unroll
       for (int e = 0; e < 4; ++e) in[B - 1 - j][e] = old[j][e] = st[(size_t)j * channels + e];
   }
+  bf16* to = y + (q_start + t0) * ldy + c;
 #pragma unroll
   for (int i = 0; i < CHUNK; ++i) {
     float a[4], *now = in[(B + i) % K];
@@ -182,11 +190,11 @@ short_conv_vec_kernel(const bf16* __restrict__ x, int ldx, const float* __restri
 #pragma unroll
       for (int e = 0; e < 4; ++e) a[e] = __fdividef(0.25f * a[e], fmaf(0.25f, expf(-a[e]), 0.25f));
     }
-    if (t0 + i < q_len) {
+    if (whole || t0 + i < q_len) {
       uint2 o;
       *reinterpret_cast<__nv_bfloat162*>(&o.x) = __floats2bfloat162_rn(a[0], a[1]);
       *reinterpret_cast<__nv_bfloat162*>(&o.y) = __floats2bfloat162_rn(a[2], a[3]);
-      *reinterpret_cast<uint2*>(y + (q_start + t0 + i) * ldy + c) = o;
+      *reinterpret_cast<uint2*>(to + (long long)i * ldy) = o;
     }
   }
   if (chunk != 0) return;
