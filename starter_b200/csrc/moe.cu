@@ -49,7 +49,7 @@ __device__ __forceinline__ float moe_gate(float g, float u, float limit) {
 
 // The logits of TOK tokens from `row0` on (rows past `n_tokens` repeat the last one): z[token][output].  A warp takes EXP outputs
 // and all TOK tokens at a time: a piece of a router's row serves TOK tokens, a piece of a token EXP outputs (one output a warp and one token
-// a block read 128 KB of router from L2 a token with 16 experts of 2,048: 46 us for 2,048 tokens, now 17).  A sum is the
+// a block read 128 KB of router from L2 a token with 16 experts of 2,048: 46 us for 2,048 tokens, 18 with four; moe_route_many_kernel 12).  A sum is the
 // same whatever EXP and TOK are.
 template <typename T, int TOK, int EXP>
 __device__ __forceinline__ void moe_logits(const T* __restrict__ h, const float* __restrict__ w, const float* __restrict__ b,
@@ -194,6 +194,170 @@ __global__ void __launch_bounds__(512) moe_route_kernel(const T* __restrict__ h,
       } else {
         for (int c = 0; c < top; ++c) weights[(size_t)row * top + c] = best[c] / sum;
       }
+    }
+  }
+}
+
+// ROUTE_TOKENS tokens a block, bfloat16 rows in whole 16-byte pieces, up to ROUTE_EXPERTS experts.  What bounds the router is the way from
+// L2: a block of four tokens brings all router rows for those four (512 blocks times 128 KB with 16 experts of 2,048: 64 MB), a block of
+// sixteen a quarter of that; rows and tokens pass through shared memory, 512 entries of each a stage, two stages ahead.  A warp
+// keeps the sums of TPW tokens and eight experts (a piece of a router's row serves TPW tokens, a piece of a token eight experts), and
+// each sum has the terms and the order that moe_logits gives it: the same bits.  The choice keeps a token's logits in the lanes'
+// registers and finds the largest by the warp's integer maximum.
+// Measured, four tokens a block / here, us: 16 experts of 2,048 600 tokens 9.8 / 8.9, 2,048 11.3 / 9.2 (behind other kernels, whose
+// weights have emptied the caches, 18.0 / 12.4), 4,096 21.1 / 17.6; 8 of 1,024 600 7.4 / 5.1; 32 of 1,536 1,000 9.7 / 12.5, 2,048 18.1 /
+// 12.9; 64 of 2,048 1,000 17.7 / 27.9, 2,048 33.5 / 28.5: a block's passes over 16 experts are a chain, which more than sixteen want 1,184
+// tokens for.  Stages of 256 entries, four: 13.2 (2,048 tokens of 16 experts).
+#define ROUTE_TOKENS 16
+#define ROUTE_EXPERTS 64
+#define ROUTE_STAGES 3
+#define ROUTE_K 512
+template <int GROUPS>
+__global__ void __launch_bounds__(256) moe_route_many_kernel(const bf16* __restrict__ h, const float* __restrict__ w, const float* __restrict__ b,
+                                 int* __restrict__ ids, float* __restrict__ weights, int n_tokens, int width, int experts, int top,
+                                 int scoring, float weight_scale) {
+  // GROUPS of eight experts at a time, eight warps: 8 / GROUPS warps of TPW tokens each
+  constexpr int TPW = ROUTE_TOKENS * GROUPS / 8, EPP = 8 * GROUPS;
+  constexpr int W_BYTES = EPP * ROUTE_K * 4, STAGE = W_BYTES + ROUTE_TOKENS * ROUTE_K * 2;
+  extern __shared__ __align__(16) unsigned char route_smem[];
+  __shared__ float z[ROUTE_TOKENS][ROUTE_EXPERTS];
+  pdl_trigger();
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, row0 = blockIdx.x * ROUTE_TOKENS;
+  const int group = warp % GROUPS, t0 = warp / GROUPS * TPW;
+  const int stages = (width + ROUTE_K - 1) / ROUTE_K, all = stages * ((experts + EPP - 1) / EPP);
+  const unsigned smem = (unsigned)__cvta_generic_to_shared(route_smem);
+  // a stage: the pass's router rows and the block's tokens, zeros behind the width
+  auto bring_router = [&](int e0, int k0, int slot) {
+#pragma unroll
+    for (int i = 0; i < EPP * (ROUTE_K / 4) / 256; ++i) {
+      const int c = threadIdx.x + 256 * i, e = min(e0 + c / (ROUTE_K / 4), experts - 1), k = k0 + c % (ROUTE_K / 4) * 4;
+      asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(smem + slot * STAGE + c * 16),
+                   "l"(w + (size_t)e * width + min(k, width - 4)), "r"(k < width ? 16 : 0) : "memory");
+    }
+  };
+  auto bring_tokens = [&](int k0, int slot) {
+#pragma unroll
+    for (int i = 0; i < ROUTE_TOKENS * (ROUTE_K / 8) / 256; ++i) {
+      const int c = threadIdx.x + 256 * i, t = min(row0 + c / (ROUTE_K / 8), n_tokens - 1), k = k0 + c % (ROUTE_K / 8) * 8;
+      asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(smem + slot * STAGE + W_BYTES + c * 16),
+                   "l"(h + (size_t)t * width + min(k, width - 8)), "r"(k < width ? 16 : 0) : "memory");
+    }
+  };
+  // (the router's rows are weights: the first stages' are asked for in front of the wait)
+  int e_ahead = 0, k_ahead = 0;                    // the next stage to ask for
+  auto next = [&] {
+    if ((k_ahead += ROUTE_K) >= width) { k_ahead = 0; e_ahead += EPP; }
+  };
+  for (int i = 0; i < ROUTE_STAGES - 1 && i < all; ++i, next()) bring_router(e_ahead, k_ahead, i);
+  pdl_wait();
+  SB_BEHIND_WAIT(h);
+  for (int i = 0, k = 0; i < ROUTE_STAGES - 1; ++i) {
+    if (i < all) bring_tokens(k, i);
+    asm volatile("cp.async.commit_group;" ::: "memory");
+    if ((k += ROUTE_K) >= width) k = 0;
+  }
+  float a[8][TPW];
+  int slot = 0, free_slot = ROUTE_STAGES - 1, left = stages, pass_e = 0;
+#pragma unroll 1
+  for (int at = 0; at < all; ++at) {
+    if (left == stages)
+#pragma unroll
+      for (int e = 0; e < 8; ++e)
+#pragma unroll
+        for (int t = 0; t < TPW; ++t) a[e][t] = 0.f;
+    asm volatile("cp.async.wait_group %0;" ::"n"(ROUTE_STAGES - 2) : "memory");
+    __syncthreads();          // stage `at` is there for all, and nobody reads the stage before any more
+    if (at + ROUTE_STAGES - 1 < all) {
+      bring_router(e_ahead, k_ahead, free_slot);
+      bring_tokens(k_ahead, free_slot);
+      next();
+    }
+    asm volatile("cp.async.commit_group;" ::: "memory");
+    const unsigned char* stage = route_smem + slot * STAGE;
+    slot = slot == ROUTE_STAGES - 1 ? 0 : slot + 1;
+    free_slot = free_slot == ROUTE_STAGES - 1 ? 0 : free_slot + 1;
+#pragma unroll
+    for (int piece = 0; piece < ROUTE_K / 128; ++piece) {
+      float hv[TPW][4];
+#pragma unroll
+      for (int t = 0; t < TPW; ++t) {
+        const uint2 v = reinterpret_cast<const uint2*>(stage + W_BYTES + (t0 + t) * ROUTE_K * 2)[piece * 32 + lane];
+        hv[t][0] = __uint_as_float(v.x << 16);
+        hv[t][1] = __uint_as_float(v.x & 0xffff0000u);
+        hv[t][2] = __uint_as_float(v.y << 16);
+        hv[t][3] = __uint_as_float(v.y & 0xffff0000u);
+      }
+#pragma unroll
+      for (int e = 0; e < 8; ++e) {
+        const float4 wv = reinterpret_cast<const float4*>(stage + (group * 8 + e) * ROUTE_K * 4)[piece * 32 + lane];
+#pragma unroll
+        for (int t = 0; t < TPW; ++t) a[e][t] += hv[t][0] * wv.x + hv[t][1] * wv.y + hv[t][2] * wv.z + hv[t][3] * wv.w;
+      }
+    }
+    if (--left == 0) {
+      // the lanes' sums, a token's eight at a time: each step hands half of the values over and leaves the same tree as warp_sum's
+      const int e0 = pass_e + group * 8;
+      left = stages;
+      pass_e += EPP;
+#pragma unroll
+      for (int t = 0; t < TPW; ++t) {
+        float v[8];
+#pragma unroll
+        for (int e = 0; e < 8; ++e) v[e] = a[e][t];
+#pragma unroll
+        for (int e = 0; e < 4; ++e) {
+          const bool up = lane & 16;
+          const float got = __shfl_xor_sync(0xffffffffu, up ? v[e] : v[e + 4], 16);
+          v[e] = (up ? v[e + 4] : v[e]) + got;
+        }
+#pragma unroll
+        for (int e = 0; e < 2; ++e) {
+          const bool up = lane & 8;
+          const float got = __shfl_xor_sync(0xffffffffu, up ? v[e] : v[e + 2], 8);
+          v[e] = (up ? v[e + 2] : v[e]) + got;
+        }
+        const bool up = lane & 4;
+        const float got = __shfl_xor_sync(0xffffffffu, up ? v[0] : v[1], 4);
+        float sum = (up ? v[1] : v[0]) + got;
+        sum += __shfl_xor_sync(0xffffffffu, sum, 2);
+        sum += __shfl_xor_sync(0xffffffffu, sum, 1);
+        const int e = e0 + (lane >> 4) * 4 + (lane >> 3 & 1) * 2 + (lane >> 2 & 1);
+        if ((lane & 3) == 0 && e < experts) z[t0 + t][e] = sum + (b ? b[e] : 0.f);
+      }
+    }
+  }
+  asm volatile("cp.async.wait_group 0;" ::: "memory");
+  __syncthreads();
+  // a float as an integer of the same order; INT_MIN: nothing to choose (no number, or minus infinity)
+  auto key = [](float v) {
+    const int i = __float_as_int(v + 0.f);
+    return v > -INFINITY ? i ^ (i >> 31 & 0x7fffffff) : (int)0x80000000;
+  };
+#pragma unroll 1
+  for (int t = warp; t < ROUTE_TOKENS && row0 + t < n_tokens; t += 8) {
+    const float z0 = lane < experts ? z[t][lane] : -INFINITY, z1 = lane + 32 < experts ? z[t][lane + 32] : -INFINITY;
+    int k0 = key(z0), k1 = key(z1), chosen = 0;
+    float best = 0.f, first = 0.f;
+#pragma unroll 1
+    for (int c = 0; c < top; ++c) {
+      // the largest logit left, the lowest index among equals; none left: index 0, to keep inside the table
+      const int most = __reduce_max_sync(0xffffffffu, max(k0, k1));
+      const unsigned low = __ballot_sync(0xffffffffu, k0 == most), high = __ballot_sync(0xffffffffu, k1 == most);
+      int at = low ? __ffs(low) - 1 : 31 + __ffs(high);
+      float v = __shfl_sync(0xffffffffu, at < 32 ? z0 : z1, at & 31);
+      if (most == (int)0x80000000) { at = 0; v = -INFINITY; }
+      if (c == 0) first = v;
+      if (lane == c) { best = v; chosen = at; }
+      if (lane == (at & 31)) (at < 32 ? k0 : k1) = (int)0x80000000;
+    }
+    if (lane < top) best = scoring != 0 ? 1.f / (1.f + expf(-best)) : expf(best - first);
+    float sum = 0.f;
+#pragma unroll 1
+    for (int c = 0; c < top; ++c) sum += __shfl_sync(0xffffffffu, best, c);
+    if (lane < top) {
+      const size_t to = (size_t)(row0 + t) * top + lane;
+      ids[to] = chosen;
+      weights[to] = scoring == 3 ? best * weight_scale : scoring == 1 ? best / (sum + 1e-20f) * weight_scale : best / sum;
     }
   }
 }
@@ -1130,8 +1294,21 @@ int sb_moe_route(int dtype, const void* h, const float* w, const float* b, int* 
   if (n_tokens == 0) return 0;
   if (experts < 1 || experts > MOE_MAX_EXPERTS || top < 1 || top > MOE_MAX_TOP || top > experts) return -2;
   if (scoring != 0 && scoring != 1 && scoring != 3) return -2;
+  if (dtype == 1 && n_tokens >= (experts > 16 ? 8 : 4) * 148 && experts <= ROUTE_EXPERTS && width % 8 == 0 && !(((uintptr_t)h | (uintptr_t)w) % 16)) {
+    const int groups = experts > 8 ? 2 : 1;
+    const int smem = ROUTE_STAGES * (groups * 8 * ROUTE_K * 4 + ROUTE_TOKENS * ROUTE_K * 2);
+    const auto kernel = groups == 2 ? moe_route_many_kernel<2> : moe_route_many_kernel<1>;
+    static bool configured[2];
+    if (!configured[groups - 1]) {
+      const cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+      if (e != cudaSuccess) return (int)e;
+      configured[groups - 1] = true;
+    }
+    return launch_dependent(kernel, dim3((n_tokens + ROUTE_TOKENS - 1) / ROUTE_TOKENS), dim3(256), smem, s, (const bf16*)h, w, b, ids, weights,
+                            n_tokens, width, experts, top, scoring, weight_scale);
+  }
   // a step of few rows leaves most SMs idle: a token a block and a warp an expert (up to 16) shorten the chain; from 4 tokens
-  // an SM on, 4 tokens a block read the router once for all of them
+  // an SM on, 4 tokens a block read the router once for all of them (what moe_route_many_kernel does not take)
   const bool many = n_tokens >= 4 * 148 && experts <= 512;
   const int threads = many ? (experts > 16 ? 256 : 128) : experts >= 16 ? 512 : experts > 4 ? 256 : 128;
   const int blocks = many ? (n_tokens + 3) / 4 : n_tokens;
