@@ -181,3 +181,27 @@ def test_few_rows_an_expert(width, inner, experts, top, tokens, expert):
     want = plain(h, ids, weights, up, down, expert, 7.0, inner, False)
     # (the result is rounded to 8 bits, a mean of 2^-10 of it, and so is what falls on the other side of a rounding before)
     assert float((got - want).norm() / want.norm()) < 2.0 ** -8
+
+
+# by a cluster: its smallest steps, all its experts, the last pairs that its threads keep and the first that they walk twice
+@pytest.mark.parametrize("pairs,experts", [(512, 64), (513, 1), (513, 64), (2049, 33), (2049, 65), (16383, 16), (16384, 64), (16385, 16), (40000, 63)])
+def test_pairs_are_dealt_to_tiles_by_eight_blocks(pairs, experts):
+    from starter_b200 import ops
+
+    gen = torch.Generator().manual_seed(pairs)
+    ids = torch.randint(0, experts + 1, (pairs,), generator=gen, dtype=torch.int32)       # (`experts`: an identity expert)
+    bm = 16
+    tiles = -(-pairs // bm) + min(experts, pairs)
+    placed = torch.full((tiles * bm,), -7, dtype=torch.int32, device="cuda")
+    tile_expert = torch.full((tiles,), -7, dtype=torch.int32, device="cuda")
+    used = torch.zeros(1, dtype=torch.int32, device="cuda")
+    ops._check(ops._lib("moe").sb_moe_align(ids.cuda(), pairs, experts, placed, tiles * bm, tile_expert, used, bm, ops._stream()), "moe_align")
+    placed, names, used = placed.cpu().view(tiles, bm), tile_expert.cpu(), int(used)
+    counts = torch.bincount(ids, minlength=experts + 1)[:experts]
+    assert used == int(((counts + bm - 1) // bm).sum())
+    assert names[:used].tolist() == sorted(names[:used].tolist())
+    for expert in range(experts):
+        mine = placed[:used][names[:used] == expert].flatten()
+        n = int(counts[expert])
+        assert sorted(mine[:n].tolist()) == (ids == expert).nonzero().flatten().tolist()
+        assert (mine[n:] == -1).all()
