@@ -116,9 +116,7 @@ def _stream():
 
 def _product(x, weight, low, high):
     """``x @ weight.T`` by the library's product for plain bfloat16 matrices of ``low < rows < high``, or None."""
-    if isinstance(x, torch.Tensor) and x.is_cuda:
-        return _bind().product(x, weight, low, high)
-    return None
+    return _bind().product(x, weight, low, high)
 
 
 class _Added:
@@ -255,13 +253,13 @@ def linear(x, weight, out_float=False, gated=False, status=None, add_to=None):
     returns float32 whatever the working type (used for logits).  ``status`` (int32 ``[1]``) is the
     device word in which the tensor-core kernel reports a wait that ran out.
     """
-    if not out_float:
+    _need(x, "x", None, 2)
+    rows, k_dim = x.shape
+    if TENSOR_CORE_MAX_ROWS < rows < PROMPT_MIN_ROWS and not out_float:
         y = _product(x, weight, TENSOR_CORE_MAX_ROWS, PROMPT_MIN_ROWS)
         if y is not None and (not gated or y.shape[1] % 2 == 0):
             return swiglu(y, gated) if gated else y
-    _need(x, "x", None, 2)
     _need(weight, "weight", x.dtype, 2)
-    rows, k_dim = x.shape
     if weight.shape[1] != k_dim:
         raise KernelError(f"weight {tuple(weight.shape)} does not take inputs of width {k_dim}")
     n_total = weight.shape[0]
@@ -2686,9 +2684,42 @@ def scan_one_walk(n_tokens: int, n_seqs: int, blocks: int) -> bool:
     return blocks <= 3 * SM_COUNT and segs <= (3 if blocks <= SM_COUNT else 2)
 
 
-def _scan_operands(mode, q, k, v, a_raw, b_raw, A_log, dt_bias, skip, state, state_at, seq_slot, seq_q_start, seq_q_len, heads,
-                   groups, n_state, v_dim):
-    """The checked operands of a recurrence: ``(address, row width) * 5 of q .. b_raw, tokens, sequences``."""
+def state_scan(mode, q, k, v, a_raw, b_raw, A_log, dt_bias, skip, state, state_at, seq_slot, seq_q_start, seq_q_len,
+               heads, groups, n_state, v_dim, decay=None):
+    """A linear recurrence with a state ``S`` ``[n_state, v_dim]`` per head over the sequences of a step.
+
+    ``q, k, v, a_raw, b_raw`` are ``(tensor [T, N], first column)`` pairs of the working type: ``groups`` heads of
+    ``n_state`` queries and keys (head ``h`` reads ``h // (heads // groups)``), ``heads`` heads of ``v_dim`` values,
+    ``heads`` entries each of ``a_raw`` and ``b_raw``.  ``A_log``, ``dt_bias`` (and ``skip`` or None) float32 ``[heads]``.
+
+    ``"state_space"``: ``dt = softplus(a_raw + dt_bias)``, ``S <- exp(-exp(A_log) dt) S + k (dt v)^T``, ``o = S^T q +
+    skip * v`` (``b_raw`` None).  ``"gated_delta"``: q and k made unit vectors (``x / sqrt(sum x^2 + 1e-6)``), q times
+    ``n_state ** -0.5``; ``S <- exp(-exp(A_log) softplus(a_raw + dt_bias)) S``, ``u = sigmoid(b_raw) (v - S^T k)``, ``S
+    <- S + k u^T``, ``o = S^T q``.  ``"forget_write"`` (``groups`` = ``heads``; ``a_raw``, ``b_raw`` None): ``q <- silu(q)``,
+    ``k`` holds the logits of a forget gate ``f = A_log + (1 - A_log) sigmoid(k + dt_bias)`` per row of the state, with
+    lower bounds in ``A_log`` and biases in ``dt_bias`` (float32 ``[heads * n_state]`` each); ``S <- diag(f) S + (1 - f)
+    v^T``, ``o = S^T q``.  ``"channel_decay"`` (``groups`` = ``heads``; ``a_raw``, ``b_raw``, ``A_log``, ``dt_bias`` None): ``decay``
+    float32 ``[T, heads * n_state]`` holds the decays' complements ``d = 1 - alpha`` per row of the state; q times ``n_state **
+    -0.5``; ``S <- diag(1 - d) S + k v^T``, ``o = S^T q``.  ``state`` float32 ``[slots, M]``: a slot's ``[heads, n_state, v_dim]`` from
+    ``state_at`` on, read at the start and written at the end.  Returns float32 ``[T, heads * v_dim]``."""
+    return state_scan_norm(mode, q, k, v, a_raw, b_raw, A_log, dt_bias, skip, state, state_at, seq_slot, seq_q_start, seq_q_len, 0, heads,
+                           groups, n_state, v_dim, decay=decay)
+
+
+@functools.lru_cache(maxsize=256)
+def _state_step_takes(mode, heads, groups, n_state, v_dim) -> bool:
+    return bool(_lib("state_step").sb_state_step_takes(SCAN_MODES[mode], heads, groups, n_state, v_dim))
+
+
+def state_scan_norm(mode, q, k, v, a_raw, b_raw, A_log, dt_bias, skip, state, state_at, seq_slot, seq_q_start, seq_q_len, max_q_len,
+                    heads, groups, n_state, v_dim, gain=None, parts=0, eps=0.0, gate=None, gate_first=False, low=None, decay=None):
+    """``state_scan`` and ``group_norm_gate`` of what it reads out (``gate``: ``(tensor, first column)`` or None), in the type of
+    ``q``; without ``gain`` the recurrence alone.  With ``low = (tensor, first column, a2, bias, tau)`` the decays of a channel-decay
+    recurrence are ``low_rank_decay``'s.
+
+    ``max_q_len``: the most tokens a sequence brings.  Where that is one, a bfloat16 step is one kernel (csrc/state_step.cu) for heads
+    that it takes, with its norm where every head is a part and the gate comes behind it; otherwise each is a kernel of its own.  (The
+    checks stand here and once: prompts of few tokens are bound by the host.)"""
     if mode not in SCAN_MODES:
         raise KernelError(f"no recurrence {mode!r} (known: {', '.join(SCAN_MODES)})")
     dtype = q[0].dtype
@@ -2713,34 +2744,33 @@ def _scan_operands(mode, q, k, v, a_raw, b_raw, A_log, dt_bias, skip, state, sta
     _need(state, "state", torch.float32, 2)
     if state_at < 0 or state_at + heads * n_state * v_dim > state.shape[1]:
         raise KernelError(f"a slot's {state.shape[1]} floats do not hold {heads} states of {n_state} x {v_dim} from {state_at}")
-    return args, n_tokens, _seq_arrays(seq_slot, seq_q_start, seq_q_len)
-
-
-def state_scan(mode, q, k, v, a_raw, b_raw, A_log, dt_bias, skip, state, state_at, seq_slot, seq_q_start, seq_q_len,
-               heads, groups, n_state, v_dim, decay=None):
-    """A linear recurrence with a state ``S`` ``[n_state, v_dim]`` per head over the sequences of a step.
-
-    ``q, k, v, a_raw, b_raw`` are ``(tensor [T, N], first column)`` pairs of the working type: ``groups`` heads of
-    ``n_state`` queries and keys (head ``h`` reads ``h // (heads // groups)``), ``heads`` heads of ``v_dim`` values,
-    ``heads`` entries each of ``a_raw`` and ``b_raw``.  ``A_log``, ``dt_bias`` (and ``skip`` or None) float32 ``[heads]``.
-
-    ``"state_space"``: ``dt = softplus(a_raw + dt_bias)``, ``S <- exp(-exp(A_log) dt) S + k (dt v)^T``, ``o = S^T q +
-    skip * v`` (``b_raw`` None).  ``"gated_delta"``: q and k made unit vectors (``x / sqrt(sum x^2 + 1e-6)``), q times
-    ``n_state ** -0.5``; ``S <- exp(-exp(A_log) softplus(a_raw + dt_bias)) S``, ``u = sigmoid(b_raw) (v - S^T k)``, ``S
-    <- S + k u^T``, ``o = S^T q``.  ``"forget_write"`` (``groups`` = ``heads``; ``a_raw``, ``b_raw`` None): ``q <- silu(q)``,
-    ``k`` holds the logits of a forget gate ``f = A_log + (1 - A_log) sigmoid(k + dt_bias)`` per row of the state, with
-    lower bounds in ``A_log`` and biases in ``dt_bias`` (float32 ``[heads * n_state]`` each); ``S <- diag(f) S + (1 - f)
-    v^T``, ``o = S^T q``.  ``"channel_decay"`` (``groups`` = ``heads``; ``a_raw``, ``b_raw``, ``A_log``, ``dt_bias`` None): ``decay``
-    float32 ``[T, heads * n_state]`` holds the decays' complements ``d = 1 - alpha`` per row of the state; q times ``n_state **
-    -0.5``; ``S <- diag(1 - d) S + k v^T``, ``o = S^T q``.  ``state`` float32 ``[slots, M]``: a slot's ``[heads, n_state, v_dim]`` from
-    ``state_at`` on, read at the start and written at the end.  Returns float32 ``[T, heads * v_dim]``."""
-    args, n_tokens, n_seqs = _scan_operands(mode, q, k, v, a_raw, b_raw, A_log, dt_bias, skip, state, state_at, seq_slot, seq_q_start,
-                                            seq_q_len, heads, groups, n_state, v_dim)
-    if (mode == "channel_decay") != (decay is not None):
+    n_seqs = _seq_arrays(seq_slot, seq_q_start, seq_q_len)
+    if (mode == "channel_decay") != (decay is not None or low is not None):
         raise KernelError("decays per row of the state belong to the channel_decay recurrence")
+    if max_q_len == 1 and gain is not None and dtype == torch.bfloat16 and _state_step_takes(mode, heads, groups, n_state, v_dim):
+        decays = [None, 0, None, None, 0, 0.0]
+        if low is not None:
+            decays = list(_low_rank(*low, n_tokens, heads * n_state))
+        normed = parts == heads and not gate_first
+        gate_args = [None, 0]
+        if normed:
+            _check_gain(gain, heads * v_dim, parts)
+            if gate is not None:
+                gate_args = [_gate_at(gate, dtype, n_tokens, heads * v_dim, parts), gate[0].shape[1]]
+        out = _empty(q[0] if normed else state, (n_tokens, heads * v_dim), dtype if normed else torch.float32)
+        rc = _lib("state_step").sb_state_step(
+            SCAN_MODES[mode], *args, A_log, dt_bias, skip, *decays, _at(state, state_at), state.shape[1], seq_slot, seq_q_start, seq_q_len,
+            n_seqs, heads, groups, n_state, v_dim, *gate_args, gain if normed else None, gain.shape[0] if normed else 0, eps,
+            None if normed else out, out if normed else None, _stream())
+        if rc != -2:                       # (an operand off its alignment: the separate kernels take any)
+            _check(rc, "state_step")
+            if normed:
+                return out
+            return group_norm_gate(out, *gate or (None, 0), gain, parts, eps, gate_first, dtype)
+    if low is not None:
+        decay = low_rank_decay(*low)
     if decay is not None:
         _f32(decay, "decay", (n_tokens, heads * n_state))
-    dtype = q[0].dtype
     out = _empty(state, (n_tokens, heads * v_dim), torch.float32)
     if dtype == torch.bfloat16 and n_tokens >= SCAN_PROMPT_TOKENS * n_seqs and 64 < n_state <= 128:
         lib = _lib("state_scan_prompt")
@@ -2758,7 +2788,7 @@ def state_scan(mode, q, k, v, a_raw, b_raw, A_log, dt_bias, skip, state, state_a
                 state.shape[1], out, seq_slot, seq_q_start, seq_q_len, n_tokens,
                 n_seqs, heads, groups, n_state, v_dim, scratch, segs, carried, _stream())
             _check(rc, "state_scan (many tokens)", 1 if mode == "channel_decay" else 2)
-            return out
+            return out if gain is None else group_norm_gate(out, *gate or (None, 0), gain, parts, eps, gate_first, dtype)
     rc = _lib("state_scan").sb_state_scan(
         _code(dtype), SCAN_MODES[mode], *args, A_log, dt_bias, skip, decay, _at(state, state_at),
         state.shape[1], out, seq_slot, seq_q_start, seq_q_len, n_seqs, heads,
@@ -2767,58 +2797,17 @@ def state_scan(mode, q, k, v, a_raw, b_raw, A_log, dt_bias, skip, state, state_a
         raise KernelError(f"the recurrence takes states of 1 to {scan_max_state()} rows and heads in whole groups, not "
                           f"{n_state} rows, {heads} heads, {groups} groups")
     _check(rc, "state_scan")
-    return out
+    return out if gain is None else group_norm_gate(out, *gate or (None, 0), gain, parts, eps, gate_first, dtype)
 
 
-@functools.lru_cache(maxsize=256)
-def _state_step_takes(mode, heads, groups, n_state, v_dim) -> bool:
-    return bool(_lib("state_step").sb_state_step_takes(SCAN_MODES[mode], heads, groups, n_state, v_dim))
-
-
-def state_scan_norm(mode, q, k, v, a_raw, b_raw, A_log, dt_bias, skip, state, state_at, seq_slot, seq_q_start, seq_q_len, max_q_len,
-                    heads, groups, n_state, v_dim, gain, parts, eps, gate=None, gate_first=False, low=None):
-    """``state_scan`` and ``group_norm_gate`` of what it reads out (``gate``: ``(tensor, first column)`` or None), in the type of
-    ``q``; with ``low = (tensor, first column, a2, bias, tau)`` the decays of a channel-decay recurrence are ``low_rank_decay``'s.
-
-    ``max_q_len``: the most tokens a sequence brings.  Where that is one, a bfloat16 step is one kernel (csrc/state_step.cu) for heads
-    that it takes, with its norm where every head is a part and the gate comes behind it; otherwise each is a kernel of its own."""
-    t, dtype = q[0], q[0].dtype
-    if max_q_len == 1 and dtype == torch.bfloat16 and mode in SCAN_MODES and _state_step_takes(mode, heads, groups, n_state, v_dim):
-        args, n_tokens, n_seqs = _scan_operands(mode, q, k, v, a_raw, b_raw, A_log, dt_bias, skip, state, state_at, seq_slot,
-                                                seq_q_start, seq_q_len, heads, groups, n_state, v_dim)
-        decays = [None, 0, None, None, 0, 0.0]
-        if (mode == "channel_decay") != (low is not None):
-            raise KernelError("decays per row of the state belong to the channel_decay recurrence")
-        if low is not None:
-            decays = list(_low_rank(*low, n_tokens, heads * n_state))
-        normed = parts == heads and not gate_first
-        gate_args = [None, 0]
-        if normed:
-            _check_gain(gain, heads * v_dim, parts)
-            if gate is not None:
-                gate_args = [_gate_at(gate, dtype, n_tokens, heads * v_dim, parts), gate[0].shape[1]]
-        out = _empty(t if normed else state, (n_tokens, heads * v_dim), dtype if normed else torch.float32)
-        rc = _lib("state_step").sb_state_step(
-            SCAN_MODES[mode], *args, A_log, dt_bias, skip, *decays, _at(state, state_at), state.shape[1], seq_slot, seq_q_start, seq_q_len,
-            n_seqs, heads, groups, n_state, v_dim, *gate_args, gain if normed else None, gain.shape[0] if normed else 0, eps,
-            None if normed else out, out if normed else None, _stream())
-        if rc != -2:                       # (an operand off its alignment: the separate kernels take any)
-            _check(rc, "state_step")
-            if normed:
-                return out
-            return group_norm_gate(out, gate[0] if gate else None, gate[1] if gate else 0, gain, parts, eps, gate_first, dtype)
-    decay = low_rank_decay(*low) if low is not None else None
-    o = state_scan(mode, q, k, v, a_raw, b_raw, A_log, dt_bias, skip, state, state_at, seq_slot, seq_q_start, seq_q_len, heads, groups,
-                   n_state, v_dim, decay=decay)
-    return group_norm_gate(o, gate[0] if gate else None, gate[1] if gate else 0, gain, parts, eps, gate_first, dtype)
-
-
-def _low_rank(u, col, a2, bias, tau, n_tokens, channels):
+def _low_rank(u, col, a2, bias, tau, n_tokens=None, channels=None):
     """A low-rank decay's checked operands: the entries' address and row width, ``a2``, ``bias``, the rank and ``1 / tau``."""
     _need(u, "u", None, 2)
     _need(a2, "a2", torch.float32, 2)
     rank = a2.shape[0]
-    if a2.shape[1] != channels or u.shape[0] != n_tokens:
+    if channels is None:
+        channels = a2.shape[1]
+    elif a2.shape[1] != channels or u.shape[0] != n_tokens:
         raise KernelError(f"a decay of {tuple(u.shape)} by {tuple(a2.shape)} is not one of {channels} rows for {n_tokens} tokens")
     _f32(bias, "bias", (channels,))
     if col < 0 or col + rank > u.shape[1]:
@@ -2834,12 +2823,10 @@ def low_rank_decay(u, col, a2, bias, tau):
     """``1 - sigmoid(z) ** (1 / tau)`` with ``z = u @ a2 + bias``: how much of its row of a recurrent state every channel lets
     go of a token.  ``u``: the columns ``col .. col + R`` of a ``[T, N]`` tensor; ``a2`` float32 ``[R, C]``, ``bias`` float32
     ``[C]``.  The product, the logarithm and the exponential are float; returns float32 ``[T, C]``."""
-    _need(u, "u", None, 2)
-    _need(a2, "a2", torch.float32, 2)
-    channels = a2.shape[1]
-    at, width, _, _, rank, inv_tau = _low_rank(u, col, a2, bias, tau, u.shape[0], channels)
-    out = _empty(u, (u.shape[0], channels), torch.float32)
-    rc = _lib("state_scan").sb_low_rank_decay(_code(u.dtype), at, width, a2, bias, out, u.shape[0], channels, rank, inv_tau, _stream())
+    operands = _low_rank(u, col, a2, bias, tau)
+    n_tokens, channels = u.shape[0], a2.shape[1]
+    out = _empty(u, (n_tokens, channels), torch.float32)
+    rc = _lib("state_scan").sb_low_rank_decay(_code(u.dtype), *operands[:4], out, n_tokens, channels, *operands[4:], _stream())
     _check(rc, "low_rank_decay")
     return out
 
