@@ -1413,11 +1413,14 @@ int sb_moe_route(int dtype, const void* h, const float* w, const float* b, int* 
     const int groups = experts > 8 ? 2 : 1;
     const int smem = ROUTE_STAGES * (groups * 8 * ROUTE_K * 4 + ROUTE_TOKENS * ROUTE_K * 2);
     const auto kernel = groups == 2 ? moe_route_many_kernel<2> : moe_route_many_kernel<1>;
-    static bool configured[2];
-    if (!configured[groups - 1]) {
+    // (a device's own setting)
+    static bool configured[64][2];
+    int dev = 0;
+    cudaGetDevice(&dev);
+    if (dev >= 64 || !configured[dev][groups - 1]) {
       const cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
       if (e != cudaSuccess) return (int)e;
-      configured[groups - 1] = true;
+      if (dev < 64) configured[dev][groups - 1] = true;
     }
     return launch_dependent(kernel, dim3((n_tokens + ROUTE_TOKENS - 1) / ROUTE_TOKENS), dim3(256), smem, s, (const bf16*)h, w, b, ids, weights,
                             n_tokens, width, experts, top, scoring, weight_scale);
