@@ -1,4 +1,5 @@
-// Causal grouped-query attention over the paged cache, one warp per (query token, query head).
+// Causal grouped-query attention over the paged cache: a block of four warps for the query heads of a group and a token, or (heads of more
+// than 128 entries or no multiple of 4) one warp per (query token, query head).
 //
 // This is the plain kernel: it serves the whole 32-bit path (prompts and single tokens alike) and any
 // shape the faster bfloat16 kernels refuse.  A query at absolute position p of the sequence in `slot`
@@ -92,10 +93,9 @@ __global__ void attention_rowwise_kernel(const T* __restrict__ q, T* __restrict_
   }
 }
 
-// The same for heads of up to 128 entries, a multiple of 4, in 16- or 8-byte pieces: a lane holds four entries of a row, and 16
-// keys and their values are asked for together (four keys a round, each round a chain of page number, keys, sums, exponential and
-// values: 75 us for 141 tokens of 16 heads over up to 77 keys, 18 now).  The sums of 16 scores share their shuffles: lane l
-// ends with key l / 2.
+// Heads of up to 128 entries, a multiple of 4, in 16- or 8-byte pieces: a lane holds four entries of a row, and 16 keys, then their
+// values, are asked for together (four keys a round, each round a chain of page number, keys, sums, exponential and values: 75 us for
+// 141 tokens of 16 heads over up to 77 keys).  The sums of 16 scores share their shuffles: lane l ends with key l / 2.
 #define ROW_KEYS 16
 template <typename T> struct RowPiece;
 template <> struct RowPiece<float> {
@@ -112,79 +112,142 @@ template <> struct RowPiece<bf16> {
   static __device__ __forceinline__ uint2 zero() { return make_uint2(0u, 0u); }
 };
 
-template <typename T>
-__global__ void __launch_bounds__(128)
-attention_rowwise_vec_kernel(const T* __restrict__ q, T* __restrict__ out, const T* __restrict__ k_store,
-                             const T* __restrict__ v_store, const int* __restrict__ block_table, int table_stride,
-                             const int* __restrict__ tok_slot, const int* __restrict__ tok_pos, int n_tokens, int heads,
-                             int kv_heads, int head_dim, float scale, int window) {
+// A block of four warps has HB query heads of one key/value head and a token: a warp takes every fourth sixteen keys, which serve all HB
+// heads, and the warps' sums meet in shared memory.  What bounds a prompt here is the chain of rounds a warp walks: a quarter of those
+// that a warp a head and token has, and a key is asked for once in place of once a head.  A warp a head -> here, us a float32 layer:
+// 40 tokens behind 150, 16 heads of 8, 113.5 -> 105.2; 150 tokens, 16 of 4, 133.0 -> 125.4; 17 + 17 behind 60 78.1 -> 74.8; 77 + 64
+// tokens 151.2 -> 150.3 (the attention 13.8 -> 11.3).  Three blocks an SM in place of four (no spills): 151.9, 103.4, 129.2, 75.5.
+template <typename T, int HB>
+__global__ void __launch_bounds__(128, 4)
+attention_rowwise_group_kernel(const T* __restrict__ q, T* __restrict__ out, const T* __restrict__ k_store,
+                               const T* __restrict__ v_store, const int* __restrict__ block_table, int table_stride,
+                               const int* __restrict__ tok_slot, const int* __restrict__ tok_pos, int heads,
+                               int kv_heads, int head_dim, float scale, int window) {
   typedef RowPiece<T> Piece;
   typedef typename Piece::type Raw;
-  const long long warp = ((long long)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-  const int lane = threadIdx.x & 31;
-  if (warp >= (long long)n_tokens * heads) return;
-  const int token = (int)(warp / heads);
-  const int h = (int)(warp - (long long)token * heads);
-  const int kvh = h / (heads / kv_heads);
+  __shared__ __align__(16) float sums[4][HB][128];
+  __shared__ float most[4][HB], total[4][HB];
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const int group = heads / kv_heads, shares = (group + HB - 1) / HB;
+  const int token = blockIdx.x / (kv_heads * shares), rest = blockIdx.x - token * (kv_heads * shares);
+  const int kvh = rest / shares, h0 = kvh * group + (rest - kvh * shares) * HB, here = min(HB, (kvh + 1) * group - h0);
   const int pos = tok_pos[token];
   const int* pages = block_table + (size_t)tok_slot[token] * table_stride;
   const int d = 4 * lane;
   const bool in = d < head_dim;
-  const size_t own = ((size_t)token * heads + h) * head_dim + d;
-  float4 qv = in ? Piece::open(*reinterpret_cast<const Raw*>(q + own)) : make_float4(0.f, 0.f, 0.f, 0.f);
-  qv.x *= scale; qv.y *= scale; qv.z *= scale; qv.w *= scale;
-  float4 acc = make_float4(0.f, 0.f, 0.f, 0.f);
-  float m = -INFINITY, l = 0.f;                     // l: this lane's own keys' weights
+  const T* own = q + ((size_t)token * heads + h0) * head_dim + d;
+  float4 qv[HB], acc[HB];
+  float m[HB], l[HB];                               // l: this lane's own keys' weights
+#pragma unroll
+  for (int i = 0; i < HB; ++i) {
+    qv[i] = in && i < here ? Piece::open(*reinterpret_cast<const Raw*>(own + (size_t)i * head_dim)) : make_float4(0.f, 0.f, 0.f, 0.f);
+    qv[i].x *= scale; qv[i].y *= scale; qv[i].z *= scale; qv[i].w *= scale;
+    acc[i] = make_float4(0.f, 0.f, 0.f, 0.f);
+    m[i] = -INFINITY;
+    l[i] = 0.f;
+  }
   int first = 0;
   if (window > 0 && pos - window + 1 > 0) first = pos - window + 1;
-  for (int j0 = first; j0 <= pos; j0 += ROW_KEYS) {
+#pragma unroll 1
+  for (int j0 = first + warp * ROW_KEYS; j0 <= pos; j0 += 4 * ROW_KEYS) {
     // a lane a key looks up its page
     const int mine = min(j0 + (lane & (ROW_KEYS - 1)), pos);
     const long long at = (long long)page_row(pages[mine / SB_PAGE_TOKENS], kvh, mine % SB_PAGE_TOKENS, kv_heads, head_dim);
-    Raw kr[ROW_KEYS], vr[ROW_KEYS];
+    Raw raw[ROW_KEYS];
 #pragma unroll
     for (int u = 0; u < ROW_KEYS; ++u) {
       const long long row = __shfl_sync(0xffffffffu, at, u) + d;
-      kr[u] = in ? *reinterpret_cast<const Raw*>(k_store + row) : Piece::zero();
-      vr[u] = in && j0 + u <= pos ? *reinterpret_cast<const Raw*>(v_store + row) : Piece::zero();
+      raw[u] = in ? *reinterpret_cast<const Raw*>(k_store + row) : Piece::zero();
     }
-    float s[ROW_KEYS];
+    const bool seen = j0 + (lane >> 1) <= pos;
+    float p[HB];
+#pragma unroll
+    for (int i = 0; i < HB; ++i) {
+      float s[ROW_KEYS];
+#pragma unroll
+      for (int u = 0; u < ROW_KEYS; ++u) {
+        const float4 k = Piece::open(raw[u]);
+        s[u] = qv[i].x * k.x + qv[i].y * k.y + qv[i].z * k.z + qv[i].w * k.w;
+      }
+      if (i == HB - 1) {
+        // the keys are used: their values take their place
+#pragma unroll
+        for (int u = 0; u < ROW_KEYS; ++u) {
+          const long long row = __shfl_sync(0xffffffffu, at, u) + d;
+          raw[u] = in && j0 + u <= pos ? *reinterpret_cast<const Raw*>(v_store + row) : Piece::zero();
+        }
+      }
+#pragma unroll
+      for (int w = ROW_KEYS / 2; w >= 1; w >>= 1) {
+        const bool upper = (lane & (2 * w)) != 0;
+#pragma unroll
+        for (int c = 0; c < w; ++c) {
+          const float send = upper ? s[c] : s[c + w], keep = upper ? s[c + w] : s[c];
+          s[c] = keep + __shfl_xor_sync(0xffffffffu, send, 2 * w);
+        }
+      }
+      s[0] += __shfl_xor_sync(0xffffffffu, s[0], 1);
+      const float m_new = fmaxf(m[i], warp_max(seen ? s[0] : -INFINITY));
+      const float alpha = expf(m[i] - m_new);
+      p[i] = seen ? expf(s[0] - m_new) : 0.f;
+      l[i] = l[i] * alpha + p[i];
+      acc[i].x *= alpha; acc[i].y *= alpha; acc[i].z *= alpha; acc[i].w *= alpha;
+      m[i] = m_new;
+    }
 #pragma unroll
     for (int u = 0; u < ROW_KEYS; ++u) {
-      const float4 k = Piece::open(kr[u]);
-      s[u] = qv.x * k.x + qv.y * k.y + qv.z * k.z + qv.w * k.w;
-    }
+      const float4 v = Piece::open(raw[u]);          // (zeros past the last key)
 #pragma unroll
-    for (int w = ROW_KEYS / 2; w >= 1; w >>= 1) {
-      const bool upper = (lane & (2 * w)) != 0;
-#pragma unroll
-      for (int i = 0; i < w; ++i) {
-        const float send = upper ? s[i] : s[i + w], keep = upper ? s[i + w] : s[i];
-        s[i] = keep + __shfl_xor_sync(0xffffffffu, send, 2 * w);
+      for (int i = 0; i < HB; ++i) {
+        const float pu = __shfl_sync(0xffffffffu, p[i], 2 * u);
+        acc[i].x += pu * v.x; acc[i].y += pu * v.y; acc[i].z += pu * v.z; acc[i].w += pu * v.w;
       }
     }
-    s[0] += __shfl_xor_sync(0xffffffffu, s[0], 1);
-    const bool seen = j0 + (lane >> 1) <= pos;
-    const float m_new = fmaxf(m, warp_max(seen ? s[0] : -INFINITY));
-    const float alpha = expf(m - m_new), p = seen ? expf(s[0] - m_new) : 0.f;
-    l = l * alpha + p;
-    acc.x *= alpha; acc.y *= alpha; acc.z *= alpha; acc.w *= alpha;
-#pragma unroll
-    for (int u = 0; u < ROW_KEYS; ++u) {
-      const float pu = __shfl_sync(0xffffffffu, p, 2 * u);
-      const float4 v = Piece::open(vr[u]);          // (zeros past the last key)
-      acc.x += pu * v.x; acc.y += pu * v.y; acc.z += pu * v.z; acc.w += pu * v.w;
-    }
-    m = m_new;
   }
-  l = warp_sum((lane & 1) ? 0.f : l);
-  if (!in) return;
-  const float inv = 1.f / l;
-  T* o = out + own;
-  o[0] = from_f<T>(acc.x * inv);
-  o[1] = from_f<T>(acc.y * inv);
-  o[2] = from_f<T>(acc.z * inv);
-  o[3] = from_f<T>(acc.w * inv);
+#pragma unroll
+  for (int i = 0; i < HB; ++i) {
+    const float sum = warp_sum((lane & 1) ? 0.f : l[i]);
+    *reinterpret_cast<float4*>(&sums[warp][i][d]) = acc[i];
+    if (lane == 0) {
+      most[warp][i] = m[i];
+      total[warp][i] = sum;
+    }
+  }
+  __syncthreads();
+  for (int i = warp; i < here; i += 4) {
+    // (a warp without keys has minus infinity and zeros)
+    const float top = fmaxf(fmaxf(most[0][i], most[1][i]), fmaxf(most[2][i], most[3][i]));
+    float4 o = make_float4(0.f, 0.f, 0.f, 0.f);
+    float sum = 0.f;
+#pragma unroll
+    for (int w = 0; w < 4; ++w) {
+      const float by = expf(most[w][i] - top);
+      const float4 a = *reinterpret_cast<const float4*>(&sums[w][i][d]);
+      sum += by * total[w][i];
+      o.x += by * a.x; o.y += by * a.y; o.z += by * a.z; o.w += by * a.w;
+    }
+    if (in) {
+      const float inv = 1.f / sum;
+      T* to = out + ((size_t)token * heads + h0 + i) * head_dim + d;
+      to[0] = from_f<T>(o.x * inv);
+      to[1] = from_f<T>(o.y * inv);
+      to[2] = from_f<T>(o.z * inv);
+      to[3] = from_f<T>(o.w * inv);
+    }
+  }
+}
+
+template <typename T>
+static int rowwise_group(const void* q, void* out, const void* k_store, const void* v_store, const int* block_table, int table_stride,
+                         const int* tok_slot, const int* tok_pos, int n_tokens, int heads, int kv_heads, int head_dim, float scale,
+                         int window, cudaStream_t s) {
+  const int group = heads / kv_heads, each = group == 1 ? 1 : group == 2 ? 2 : 4;
+  const long long blocks = (long long)n_tokens * kv_heads * ((group + each - 1) / each);
+  const auto kernel = each == 1 ? attention_rowwise_group_kernel<T, 1> : each == 2 ? attention_rowwise_group_kernel<T, 2>
+                                                                                   : attention_rowwise_group_kernel<T, 4>;
+  kernel<<<(unsigned)blocks, 128, 0, s>>>((const T*)q, (T*)out, (const T*)k_store, (const T*)v_store, block_table, table_stride, tok_slot,
+                                          tok_pos, heads, kv_heads, head_dim, scale, window);
+  return SB_LAUNCH_RESULT();
 }
 
 extern "C" {
@@ -200,15 +263,10 @@ int sb_attention_rowwise(int dtype, const void* q, void* out, const void* k_stor
   const int threads = 128;
   const long long blocks = (warps * 32 + threads - 1) / threads;
   if (head_dim <= 128 && head_dim % 4 == 0 && !(((uintptr_t)q | (uintptr_t)k_store | (uintptr_t)v_store) % 16)) {
-    if (dtype == 0)
-      attention_rowwise_vec_kernel<float><<<(unsigned)blocks, threads, 0, s>>>(
-          (const float*)q, (float*)out, (const float*)k_store, (const float*)v_store, block_table, table_stride, tok_slot,
-          tok_pos, n_tokens, heads, kv_heads, head_dim, scale, window);
-    else
-      attention_rowwise_vec_kernel<bf16><<<(unsigned)blocks, threads, 0, s>>>(
-          (const bf16*)q, (bf16*)out, (const bf16*)k_store, (const bf16*)v_store, block_table, table_stride, tok_slot, tok_pos,
-          n_tokens, heads, kv_heads, head_dim, scale, window);
-    return SB_LAUNCH_RESULT();
+    return dtype == 0 ? rowwise_group<float>(q, out, k_store, v_store, block_table, table_stride, tok_slot, tok_pos, n_tokens, heads,
+                                             kv_heads, head_dim, scale, window, s)
+                      : rowwise_group<bf16>(q, out, k_store, v_store, block_table, table_stride, tok_slot, tok_pos, n_tokens, heads,
+                                            kv_heads, head_dim, scale, window, s);
   }
   if (dtype == 0)
     attention_rowwise_kernel<float><<<(unsigned)blocks, threads, 0, s>>>(

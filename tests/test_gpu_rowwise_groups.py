@@ -1,0 +1,36 @@
+"""The plain attention's blocks of four warps for the query heads of one key/value head: groups of all sizes, contexts that end before,
+at and behind a warp's sixteen keys and a round of sixty-four, windows, head sizes, against float64."""
+
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+F = torch.float64
+
+
+@pytest.mark.parametrize("heads,kv_heads,dim,window", [(3, 3, 128, 0), (4, 2, 64, 0), (6, 2, 100, 0), (8, 2, 128, 0), (5, 1, 36, 0), (16, 2, 128, 0),
+                                                       (4, 1, 4, 0), (8, 2, 128, 1), (8, 2, 64, 40), (3, 1, 128, 17)])
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+def test_groups_of_heads(heads, kv_heads, dim, window, dtype):
+    from starter_b200 import ops
+
+    gen = torch.Generator().manual_seed(heads * dim + window)
+    pages, page, table = 12, ops.PAGE_TOKENS, 6
+    longest = min(table * page, 200)
+    store = [(torch.randn(pages, kv_heads, page, dim, generator=gen) * (2.0 if n else 1.0)).to(dtype).cuda() for n in (0, 1)]
+    order = torch.randperm(pages, generator=gen)[:2 * table].view(2, table).to(torch.int32)
+    pos = sorted({p for p in (0, 1, 14, 15, 16, 17, 62, 63, 64, 65, 79, 80, 127, 128, longest - 1) if p < longest})
+    tok_pos = torch.tensor(pos * 2, dtype=torch.int32)
+    tok_slot = torch.tensor([0] * len(pos) + [1] * len(pos), dtype=torch.int32)
+    q = torch.randn(len(tok_pos), heads * dim, generator=gen).to(dtype).cuda()
+    scale = dim ** -0.5
+    got = ops.attention_rowwise(q, *store, order.cuda(), tok_slot.cuda(), tok_pos.cuda(), heads, kv_heads, dim, scale, window or None)
+    want = torch.empty(len(tok_pos), heads, dim, dtype=F)
+    for t, (slot, p) in enumerate(zip(tok_slot.tolist(), tok_pos.tolist())):
+        first = max(0, p - window + 1) if window else 0
+        k, v = (s.cpu().to(F)[order[slot].long()].transpose(0, 1).reshape(kv_heads, table * page, dim)[:, first:p + 1] for s in store)
+        w = torch.softmax(torch.einsum("ghd,gkd->ghk", q[t].cpu().to(F).view(kv_heads, heads // kv_heads, dim) * scale, k), dim=-1)
+        want[t] = torch.einsum("ghk,gkd->ghd", w, v).reshape(heads, dim)
+    off = (got.cpu().to(F).view_as(want) - want).abs().max()
+    # float sums of up to 200 products of unit size, exponentials of 2 ulp; a rounding to bfloat16 is 2^-9 of the result
+    assert float(off) <= (2e-6 if dtype == torch.float32 else 2.0 ** -8) * float(want.abs().max())
