@@ -21,7 +21,9 @@
 // three seeds; 0.00477, 0.00471 and 0.00482 while the weights were summed before their rounding and relative to the sink).
 //
 // Few blocks over many keys: a cluster's CTAs walk a part of a block's keys each and merge (attention_tc.cuh): 700 tokens behind 1,200
-// 60.1 -> 48.6 us.
+// 60.1 -> 48.6 us.  Up to a block an SM, of unequal lengths: blocks from `split_from` steps on are shared by the two CTAs of a cluster,
+// in front of shorter ones the two take a head's block each; a causal prompt's longest chain gets shorter while short blocks fill the
+// SMs (2,048 tokens a layer 147 -> 137 us, 1,300 114 -> 106, 1,200 behind 1,200 136 -> 120; latent_mixed_splits in ops.py).
 //
 // Gathered rows: a sequence's keys from the first that any of its queries sees, padded to a multiple of 64 with zeros, so
 // that a step never reads another sequence's values (their weights are zero, but 0 * inf would not be).
@@ -119,7 +121,8 @@ latent_prompt_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_con
                      const __grid_constant__ CUtensorMap map_rot, bf16* __restrict__ out, const int* __restrict__ seq_q_start,
                      const int* __restrict__ seq_q_len, const int* __restrict__ seq_kv_len, const int* __restrict__ block_seq,
                      const int* __restrict__ block_first, int heads, float scale_log2, int window,
-                     const float* __restrict__ sink, int* status, int withhold, int splits, const bf16* __restrict__ gate, int gate_ld) {
+                     const float* __restrict__ sink, int* status, int withhold, int splits, int split_from, const bf16* __restrict__ gate,
+                     int gate_ld) {
   constexpr int QC = DC + 1;
   constexpr int QSUB = 128 * 128, KSUB = 64 * 128;  // bytes of 128 (64) rows of 128 bytes
   constexpr int Q_BYTES = QC * QSUB, K_BYTES = QC * KSUB, V_BYTES = VC * KSUB, P_BYTES = QSUB;
@@ -135,7 +138,6 @@ latent_prompt_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_con
   __shared__ int abort_flag;
   __shared__ __align__(8) float2 ml[2 * TC_BQ];     // keys in parts: the rows' references and sums
 
-  const int head = blockIdx.x / splits, part = blockIdx.x - head * splits;      // (the CTAs of a cluster share a head's block)
   const int seq = block_seq[blockIdx.y], q_first = block_first[blockIdx.y];
   const int q_len = seq_q_len[seq], kv_len = seq_kv_len[seq];
   const int rows_valid = min(2 * TC_BQ, q_len - q_first);
@@ -149,6 +151,10 @@ latent_prompt_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_con
   n_tile[0] = (pos0 + min(rows_valid, TC_BQ) - 1 - base) / LP_BK - step0 + 1;
   n_tile[1] = rows_valid > TC_BQ ? (pos0 + rows_valid - 1 - base) / LP_BK - step0 + 1 : 0;
   int n_steps = max(n_tile[0], n_tile[1]);
+  // the CTAs of a cluster share a head's block, or, of fewer steps than split_from, take one each
+  if (n_steps < split_from) splits = 1;
+  const int head = blockIdx.x / splits, part = blockIdx.x - head * splits;
+  if (head >= heads) return;
   if (splits > 1) {                                 // this CTA's steps
     const int per = (n_steps + splits - 1) / splits;
     for (int t = 0; t < 2; ++t) n_tile[t] = max(0, min(per, n_tile[t] - part * per));
@@ -449,15 +455,15 @@ latent_prompt_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_con
 template <int DC, int VC>
 static int lp_launch(const CUtensorMap& mq, const CUtensorMap& mkv, const CUtensorMap& mr, void* out, const int* seq_q_start,
                      const int* seq_q_len, const int* seq_kv_len, const int* block_seq, const int* block_first, int n_blocks,
-                     int heads, float scale, int window, const float* sink, int* status, int withhold, int splits,
+                     int heads, float scale, int window, const float* sink, int* status, int withhold, int split,
                      const bf16* gate, int gate_ld, cudaStream_t s) {
   const int smem = 2 * (DC + 1) * 128 * 128 + 2 * 128 * 128 + 2 * (DC + 1 + VC) * 64 * 128 + 1024;
   cudaError_t err = cudaFuncSetAttribute(latent_prompt_kernel<DC, VC>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
   if (err != cudaSuccess) return (int)err;
-  splits = DC == 1 && VC == 2 ? 1 : splits >= 4 ? 4 : splits >= 2 ? 2 : 1;
+  const int parts = split & 255, splits = DC == 1 && VC == 2 ? 1 : parts >= 4 ? 4 : parts >= 2 ? 2 : 1, split_from = split >> 8;
   return launch_dependent_cluster(latent_prompt_kernel<DC, VC>, dim3(heads * splits, n_blocks), dim3(LP_THREADS), smem, s, dim3(splits),
                                   mq, mkv, mr, (bf16*)out, seq_q_start, seq_q_len, seq_kv_len, block_seq, block_first, heads,
-                                  scale * 1.4426950408889634f, window, sink, status, withhold, splits, gate, gate_ld);
+                                  scale * 1.4426950408889634f, window, sink, status, withhold, splits, split_from, gate, gate_ld);
 }
 
 static int lp_run(const void* q, const void* kv, const void* shared, void* out, const int* seq_q_start, const int* seq_q_len,
@@ -506,7 +512,8 @@ int sb_latent_gather(const void* store, const int* block_table, int table_stride
 
 // q: [n_tokens, heads * (dim + 64)], the last 64 entries of a head turned; kv: [rows, heads * dim + heads * vdim]; shared:
 // [rows, 64]; out: [n_tokens, heads * vdim], with a gate (rows of gate_ld entries, those of a head's values in out's order; null: none)
-// times its sigmoid; block_seq / block_first: blocks of 256 queries; dim and vdim 64 or 128; scale > 0.
+// times its sigmoid; block_seq / block_first: blocks of 256 queries; dim and vdim 64 or 128; scale > 0.  splits: 1, 2 or 4 CTAs that share
+// a block's keys, in its higher bytes the least steps of 64 keys of a block that they share (shorter ones go to one CTA).
 int sb_latent_prompt(const void* q, const void* kv, const void* shared, void* out, const int* seq_q_start, const int* seq_q_len,
                      const int* seq_kv_len, const int* block_seq, const int* block_first, int n_blocks, int n_tokens, int rows,
                      int heads, int dim, int vdim, float scale, int window, const float* sink, int* status, int splits,

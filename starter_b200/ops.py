@@ -1832,6 +1832,41 @@ def latent_prompt_takes(dtype, ctx, dim, rot, vdim, rank, scale, window=None, he
     return rows <= LATENT_PROMPT_ROWS and 2 * rows * (heads * (dim + vdim) + rank + rot) <= max(LATENT_PROMPT_BYTES, scored)
 
 
+def latent_block_steps(kv_lens, q_lens, window) -> tuple:
+    """The steps of 64 keys that the blocks of 256 queries walk, the longest first, as csrc/attention_latent_prompt.cu counts them."""
+    steps = []
+    for kv, new in zip(kv_lens, q_lens):
+        base = max(0, kv - new - int(window) + 1) if window else 0
+        for first in range(0, new, 256):
+            low = max(0, kv - new + first - int(window) + 1) if window else 0
+            steps.append((kv - new + min(first + 256, new) - 1 - base) // 64 - (low - base) // 64 + 1)
+    return tuple(sorted(steps, reverse=True))
+
+
+def latent_mixed_splits(steps: tuple, heads: int) -> int:
+    """``splits`` of ``sb_latent_prompt`` for blocks of ``steps`` steps of 64 keys (the longest first), ``heads`` heads each, that leave SMs
+    idle but are too many for two CTAs each: 1, or 2 with the steps from which a block is shared by two CTAs in its second byte
+    on.  A causal prompt's last blocks walk many times the keys of its first, and their chain is the kernel's time.
+
+    That with the least time on the busiest SM by this estimate, in steps (1.5 us): a block alone takes its steps and 3, half a block its
+    steps and 9 (the cluster's launch, two barriers, the merge), and a CTA beyond one an SM starts 10 behind the end of a short one,
+    because the two of a cluster want two SMs at once.  Measured (us a layer of 16 heads, one CTA a block / two from 16, 20, 24, 28
+    steps on): 2,048 tokens 147 / 151, 152, 146, 137; 1,600 133 / 136, 129, 126, 133; 1,300 114 / 106, 109, 114; 1,300 behind 700 132 / 137,
+    137, 122, 127; 1,200 behind 1,200 136 / 142, 142, 120, 126; 2 x 1,000 126 / 129; a window of 1,024 over 2,000 134 / 150."""
+    def time(split_from):
+        jobs = sorted((job for s in steps for job in (2 * [-(-s // 2) + 9] if s >= split_from else [s + 3]) * heads), reverse=True)
+        behind = [jobs[SM_COUNT - 1 - i] + jobs[SM_COUNT + i] + 10 for i in range(min(SM_COUNT, len(jobs) - SM_COUNT))]
+        return max([jobs[0]] + behind), split_from
+
+    most, split_from = min(time(s) for s in set(steps))
+    return 2 | split_from << 8 if most <= 0.93 * (steps[0] + 3) else 1
+
+
+@functools.lru_cache(maxsize=1024)
+def _latent_mixed(kv_lens, q_lens, window, heads) -> int:
+    return latent_mixed_splits(latent_block_steps(kv_lens, q_lens, window), heads)
+
+
 def latent_attention_prompt(q, ukv, store, block_table, ctx, heads, dim, vdim, rank, rot, scale, window=None, sink=None, turn=None, gate=None):
     """Latent attention over keys and values that are formed from the cached rows first: ``q`` ``[T, heads * (dim + rot)]``
     (the last ``rot`` entries of a head turned), ``ukv`` ``[heads * dim + heads * vdim, rank]`` (the heads' key, then value
@@ -1878,11 +1913,14 @@ def latent_attention_prompt(q, ukv, store, block_table, ctx, heads, dim, vdim, r
         at = _gate_at(gate, q.dtype, n_tokens, heads * vdim, heads)
         if at % 16 == 0 and gate[0].shape[1] % 8 == 0:
             gated = [at, gate[0].shape[1]]
+    splits = prompt_splits(heads * ctx.block_first.shape[0], ctx.max_kv_len, window)
+    if splits == 1 and SM_COUNT < 2 * heads * ctx.block_first.shape[0] <= 2 * SM_COUNT:
+        splits = _latent_mixed(tuple(ctx.host["seq_kv_len"].tolist()), tuple(ctx.host["seq_q_len"].tolist()), window, heads)
     rc = lib.sb_latent_prompt(
         q, kv, shared, out, ctx.seq_q_start, ctx.seq_q_len, ctx.seq_kv_len,
         ctx.block_seq, ctx.block_first, ctx.block_seq.shape[0], n_tokens, rows, heads, dim, vdim,
         scale, int(window or 0), _latent_sink(sink, heads), ctx.status,
-        prompt_splits(heads * ctx.block_first.shape[0], ctx.max_kv_len, window), *gated, _stream())
+        splits, *gated, _stream())
     _check(rc, "latent_attention_prompt")
     if gate is not None and gated[0] is None:
         sigmoid_gate(out, *gate)

@@ -1,0 +1,65 @@
+"""Latent prompts whose longer blocks are shared by two CTAs of a cluster while the shorter ones go to one each: the kernel against a CTA a
+block, and the rule that says from how many steps on."""
+
+import pytest
+import torch
+
+BF = torch.bfloat16
+
+
+# (sequences of 301, 700 and 385 tokens and one more, blocks of 1 to 11 steps; an odd number of heads leaves a CTA of a cluster idle)
+@pytest.mark.gpu
+@pytest.mark.parametrize("heads", [1, 3, 4])
+@pytest.mark.parametrize("dim,vdim,window,gated", [(128, 128, None, True), (64, 64, 150, False), (128, 64, None, False), (64, 128, None, False)])
+def test_long_blocks_in_two_parts_short_ones_whole(heads, dim, vdim, window, gated, monkeypatch):
+    from starter_b200 import ops
+    from test_gpu_key_parts import LENGTHS, step
+
+    rank = 128
+    gen, table, (rows, _), ctx = step(1, rank + 64, 16, heads)
+    q = torch.randn(sum(LENGTHS), heads * (dim + 64), generator=gen).to(BF).cuda()
+    ukv = (torch.randn(heads * (dim + vdim), rank, generator=gen) * rank ** -0.5).to(BF).cuda()
+    gate = (torch.randn(sum(LENGTHS), heads * vdim, generator=gen).to(BF).cuda(), 0) if gated else None
+    sink = torch.linspace(-1.0, 2.0, heads).cuda()
+
+    def run(splits):
+        monkeypatch.setattr(ops, "prompt_splits", lambda *a, **k: splits)
+        return ops.latent_attention_prompt(q, ukv, rows, table, ctx, heads, dim, vdim, rank, 64, (dim + 64) ** -0.5, window, sink, gate=gate)
+
+    whole = run(1)
+    for split_from in (1, 2, 4, 5, 8, 11, 12):
+        got = run(2 | split_from << 8)
+        # (the parts' sums join in another order: a rounding to 8 bits that falls on the other side)
+        assert float((got.float() - whole.float()).abs().max()) <= 2.0 ** -7 * float(whole.float().abs().max())
+    assert torch.equal(run(2 | 1000 << 8), whole)
+    assert int(ctx.status.item()) == 0
+
+
+@pytest.mark.parametrize("window", [None, 1, 64, 300])
+def test_steps_of_blocks(window):
+    from starter_b200 import ops
+
+    kv, new = [700, 257, 64, 1500], [700, 1, 64, 513]
+    want = []
+    for k, n in zip(kv, new):
+        sees = [range(max(0, p - window + 1) if window else 0, p + 1) for p in range(k - n, k)]
+        for first in range(0, n, 256):
+            keys = {key for s in sees[first:first + 256] for key in s}
+            want.append(len({(key - sees[0][0]) // 64 for key in keys}))
+    assert ops.latent_block_steps(kv, new, window) == tuple(sorted(want, reverse=True))
+
+
+def test_which_blocks_are_shared():
+    from starter_b200 import ops
+
+    # a causal prompt's last blocks; blocks of one length, and one that two CTAs could not end before: none
+    assert ops.latent_mixed_splits((32, 28, 24, 20, 16, 12, 8, 4), 16) == 2 | 28 << 8
+    assert ops.latent_mixed_splits((25, 24, 20, 16, 12, 8, 4), 16) == 2 | 24 << 8
+    assert ops.latent_mixed_splits((38, 35, 31, 27, 23), 16) == 2 | 27 << 8
+    assert ops.latent_mixed_splits((20, 20, 20, 20, 16, 12, 8, 4), 16) == 1
+    assert ops.latent_mixed_splits((16, 16, 12, 12, 8, 8, 4, 4), 16) == 1
+    assert ops.latent_mixed_splits((10,), 100) == 1
+    for heads in (1, 2, 40, 75, 148):
+        for steps in ((1,), (500,), (60, 3), (60, 60)):
+            got = ops.latent_mixed_splits(steps, heads)
+            assert got == 1 or (got & 255 == 2 and 1 <= got >> 8 <= steps[0])
