@@ -117,6 +117,8 @@ __device__ __forceinline__ size_t page_row(int page, int head, int offset, int k
 // earlier kernel of the stream may have written and before its first write to global memory (a
 // buffer may be recycled memory that an earlier kernel still reads).  Because a kernel cannot
 // complete before its own pdl_wait() returns, completion is transitive along the stream.
+// (One exception, moe_few_kernel<0>: it reads in front of its wait what was complete before the kernel directly in front of it passed its
+// own, and that kernel triggers behind its wait.  One entry point launches the two.)
 __device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 // A load through a `const T* __restrict__` parameter counts as invariant (nothing in the kernel can
 // change what it reads), so the compiler is free to move it up, across volatile asm and its memory

@@ -1065,8 +1065,8 @@ moe_tile_big_kernel(const bf16* __restrict__ x, const bf16* __restrict__ w, bf16
 // that the warps of an SM share the tile's rows in the first cache.  A captured layer of 16 experts of 2,048 x 2,048 at 8 tokens, four each, with
 // blocks of four warps (a round and a half of them) and loads that stop between steps 84.0 us, now 77.5 (363 MB are 55); 32 experts, 11 tokens, 1,664 x
 // 1,536 90.0 -> 87.2; 8 experts, 2 tokens, three each, squared relu, 1,152 x 1,664 32.8 -> 23.6.
-// The second product may read the tiles' experts and its first weights ahead of its wait: the first one lets it start only
-// behind its own wait, when the kernel that made the tiles has completed.
+// The second product reads the tiles' experts and its first weights ahead of its wait.  It may because it stands directly behind the first
+// one (sb_moe_few launches both), which lets it start only behind its own wait, when the kernel that made the tiles has completed.
 #define MOE_FEW 8
 #define MOE_FEW_WARPS 10         // warps on every SM that a grid should bring
 #define MOE_FEW_REGS 128         // (16 warps an SM; 6 and 3 steps in flight fill them.  144 registers and 8 and 4: 77.5 -> 90.0 us, 96 and 4 and 2: 88.0)
@@ -1325,20 +1325,11 @@ moe_combine_vec_kernel(const bf16* __restrict__ down, const float* __restrict__ 
 // [experts, n_out, k_dim] and the squared relu.  up 0: x = that y [capacity, k_dim], w = [experts,
 // n_out, k_dim], y = [n_pairs, n_out] by pair.  in_scale (up passes): float [n_pairs] that multiplies the products ahead
 // of the activation, or null.
+// (tiles of MOE_FEW rows: sb_moe_few)
 template <int MODE>
 static int moe_tiles_mode(int dtype, int tile_rows, const void* x, const void* w, void* y, const int* sorted,
                           const int* tile_expert, const int* n_tiles, int max_tiles, int k_dim, int n_out, int top,
                           float limit, const float* in_scale, cudaStream_t s) {
-  if (tile_rows == MOE_FEW) {
-    if (dtype != 1 || k_dim % 8 || ((uintptr_t)x % 16) || ((uintptr_t)w % 16)) return -2;
-    // warps a block: the fewest that bring MOE_FEW_WARPS to every SM (all are there at once), each with two steps and more
-    const long long items = (long long)max_tiles * ((n_out + 15) / 16);
-    int warps = 1;
-    while (warps < 8 && items * warps < 148 * MOE_FEW_WARPS && k_dim >= 32 * 4 * warps) warps *= 2;
-    const size_t smem = warps > 1 ? (size_t)warps * (MODE == 1 ? 8 : 4) * 32 * sizeof(float) : 0;
-    return launch_dependent(moe_few_kernel<MODE>, dim3((n_out + 15) / 16, max_tiles), dim3(32 * warps), smem, s, (const bf16*)x,
-                            (const bf16*)w, (bf16*)y, sorted, tile_expert, n_tiles, k_dim, n_out, top, limit, in_scale);
-  }
   if (tile_rows == MOE_BIG) {
     if (dtype != 1 || k_dim % 16 || n_out % 2 || ((uintptr_t)x % 16) || ((uintptr_t)w % 16) || ((uintptr_t)y % 4)) return -2;
     constexpr int NW = MODE == 1 ? 2 : 1, LD = (NW == 1 ? 64 : 32) + 8;
@@ -1366,6 +1357,19 @@ static int moe_tiles_mode(int dtype, int tile_rows, const void* x, const void* w
   return launch_dependent(moe_tile_kernel<bf16, MODE>, grid, dim3(256), 0, s, (const bf16*)x, (const bf16*)w,
                           (bf16*)y, sorted, tile_expert, n_tiles, k_dim, n_out, top, limit,
                             in_scale);
+}
+
+// A product of the few-row kernel, bfloat16, k_dim a multiple of 8.
+template <int MODE>
+static int moe_few(const void* x, const void* w, void* y, const int* sorted, const int* tile_expert, const int* n_tiles, int max_tiles,
+                   int k_dim, int n_out, int top, float limit, const float* in_scale, cudaStream_t s) {
+  // warps a block: the fewest that bring MOE_FEW_WARPS to every SM (all are there at once), each with two steps and more
+  const long long items = (long long)max_tiles * ((n_out + 15) / 16);
+  int warps = 1;
+  while (warps < 8 && items * warps < 148 * MOE_FEW_WARPS && k_dim >= 32 * 4 * warps) warps *= 2;
+  const size_t smem = warps > 1 ? (size_t)warps * (MODE == 1 ? 8 : 4) * 32 * sizeof(float) : 0;
+  return launch_dependent(moe_few_kernel<MODE>, dim3((n_out + 15) / 16, max_tiles), dim3(32 * warps), smem, s, (const bf16*)x,
+                          (const bf16*)w, (bf16*)y, sorted, tile_expert, n_tiles, k_dim, n_out, top, limit, in_scale);
 }
 
 extern "C" {
@@ -1460,6 +1464,20 @@ int sb_moe_tiles(int dtype, int up, int tile_rows, const void* x, const void* w,
   if (up == 2) return moe_tiles_mode<2>(MOE_ARGS);
 #undef MOE_ARGS
   return -2;
+}
+
+// Both products over tiles of MOE_FEW rows, bfloat16: `up` (1 or 2) of h [.., width] and w [experts, (2 *) inner, width] into act [capacity,
+// inner], then down [experts, width, inner] into per_pair [n_pairs, width].  They are one entry because the second reads the tiles in front of
+// its wait: nothing may stand between the two.
+int sb_moe_few(int up, const void* h, const void* w, void* act, const void* down, void* per_pair, const int* sorted,
+               const int* tile_expert, const int* n_tiles, int max_tiles, int width, int inner, int top, float limit,
+               const float* in_scale, cudaStream_t s) {
+  if (max_tiles == 0) return 0;
+  if (up < 1 || up > 2 || top < 1 || width % 8 || inner % 8 || (((uintptr_t)h | (uintptr_t)w | (uintptr_t)act | (uintptr_t)down) % 16)) return -2;
+  const int rc = up == 1 ? moe_few<1>(h, w, act, sorted, tile_expert, n_tiles, max_tiles, width, inner, top, limit, in_scale, s)
+                         : moe_few<2>(h, w, act, sorted, tile_expert, n_tiles, max_tiles, width, inner, top, limit, in_scale, s);
+  if (rc) return rc;
+  return moe_few<0>(act, down, per_pair, sorted, tile_expert, n_tiles, max_tiles, inner, width, top, limit, nullptr, s);
 }
 
 int sb_moe_combine(int dtype, const void* down, const float* weights, void* out, int n_tokens, int width, int top,

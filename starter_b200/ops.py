@@ -2137,13 +2137,18 @@ def moe_experts(h, ids, weights, gate_up, down, limit=0.0, expert="gated_clamped
                                 _stream())
         _check(rc, "moe_combine")
         return out
-    rc = lib.sb_moe_tiles(_code(h.dtype), up_mode, bm, h, gate_up, act, sorted_pairs, tile_expert,
-                          n_tiles, max_tiles, width, inner, top, limit, in_scale, _stream())
-    _check(rc, "moe_up")
-    rc = lib.sb_moe_tiles(_code(h.dtype), 0, bm, act, down, per_pair, sorted_pairs,
-                          tile_expert, n_tiles, max_tiles, inner, width, top, limit, None,
-                          _stream())
-    _check(rc, "moe_down")
+    if bm == 8:
+        rc = lib.sb_moe_few(up_mode, h, gate_up, act, down, per_pair, sorted_pairs, tile_expert, n_tiles, max_tiles, width, inner, top,
+                            limit, in_scale, _stream())
+        _check(rc, "moe_up / moe_down (few rows)", 2)
+    else:
+        rc = lib.sb_moe_tiles(_code(h.dtype), up_mode, bm, h, gate_up, act, sorted_pairs, tile_expert,
+                              n_tiles, max_tiles, width, inner, top, limit, in_scale, _stream())
+        _check(rc, "moe_up")
+        rc = lib.sb_moe_tiles(_code(h.dtype), 0, bm, act, down, per_pair, sorted_pairs,
+                              tile_expert, n_tiles, max_tiles, inner, width, top, limit, None,
+                              _stream())
+        _check(rc, "moe_down")
     out = _empty(h, h.shape)
     rc = lib.sb_moe_combine(_code(h.dtype), per_pair, out_scale, out, n_tokens, width, top, *extras,
                                 _stream())

@@ -254,3 +254,16 @@ def test_steps_whose_latent_products_are_for_few_rows():
         assert ops.latent_heads_take(torch.empty(n, 8, dtype=torch.bfloat16), 128, 64, 512, 128, longest) == takes
         assert ops.latent_heads_take(torch.empty(n, 8), 128, 64, 512, 128, longest) == (False, False)
         assert ops.latent_heads_take(torch.empty(n, 8, dtype=torch.bfloat16), 120, 64, 512, 128, longest) == (False, False)
+
+
+@pytest.mark.parametrize("up", [0, 1, 2])
+def test_products_over_tiles_of_eight_rows_come_in_pairs(up):
+    """The down product of few rows reads its tiles in front of its wait, so neither of the two has an entry of its own."""
+    from starter_b200.csrc import build
+
+    entry = build.load("moe").sb_moe_tiles
+    result, types = build.declarations("moe")["sb_moe_tiles"]
+    entry.restype, entry.argtypes = result, types
+    tile_rows = 8
+    # (refused in front of any launch, so no address is looked at)
+    assert entry(1, up, tile_rows, None, None, None, None, None, None, 1, 64, 64, 1, 0.0, None, None) == -2
