@@ -733,7 +733,7 @@ latent_merge_kernel(const float* __restrict__ part_acc, const float* __restrict_
 // Single tokens of up to 16 heads: the rows of a sequence are one 16-row tile, which leaves three of the four row groups above (and six
 // of its eight warps) with nothing to do but loads.  Here a block takes a page of 64 keys at a time and all eight warps share it: a
 // warp scores eight of the keys, then, behind a barrier, sums its eighth of the latent's columns over all of them.  Pages arrive two ahead by
-// cp.async, rows behind the token as zeros.  Parts, references and sums are filed as above.  Measured (us a layer of 16 heads, captured,
+// cp.async, rows behind the token and in front of the window as zeros (their weights are zero, but 0 * inf would not be).  Parts, references and sums are filed as above.  Measured (us a layer of 16 heads, captured,
 // the kernel above -> this one): rank 512, 1 sequence of 1,500 40.3 -> 36.9, 8 of up to 2,048 46.6 -> 45.2, 20 of up to 400 50.6 -> 49.1, 30 in a window
 // of 512 58.2 -> 56.9; rank 256, 4 in a window of 512 30.9 -> 29.2, 8 of up to 1,063 33.6 -> 33.4.
 #define LS_KEYS SB_PAGE_TOKENS
@@ -769,7 +769,7 @@ latent_step_kernel(const bf16* __restrict__ qa, bf16* __restrict__ out, float* _
 #pragma unroll
     for (int k = 0; k < 8; ++k) {
       const int r = warp * 8 + k;
-      const bool real = p * LS_KEYS + r <= last;
+      const bool real = (unsigned)(p * LS_KEYS + r - first) <= (unsigned)(last - first);
       for (int c = lane; c < pieces; c += 32) cp_async16(to + r * ld + c * 8, from + (real ? (size_t)r * Dk + c * 8 : 0), real);
     }
   };

@@ -43,6 +43,28 @@ def test_single_tokens(heads, rank, rot, window, sink):
         assert float((got - want).norm()) <= 1.05 * float((old - want).norm()) + 1e-6 * float(want.norm())
 
 
+@pytest.mark.parametrize("window", [1, 70, 128])
+@pytest.mark.parametrize("splits", [1, 3])
+def test_rows_in_front_of_the_window_do_not_count(window, splits):
+    from starter_b200 import ops
+
+    gen = torch.Generator().manual_seed(window)
+    heads, rank, rot, lengths, per = 16, 256, 64, [1, 65, 129, 191, 192, 700], 11
+    n, width = len(lengths), rank + rot
+    ints = lambda v: torch.tensor(v, dtype=torch.int32, device="cuda")
+    table = torch.randperm(n * per, generator=gen).int().view(n, per).cuda()
+    store = torch.randn(n * per, 1, 64, width, generator=gen).to(BF).cuda()
+    qa = torch.randn(n, heads, width, generator=gen).to(BF).cuda()
+    seqs = (ints(list(range(n))), ints(list(range(n))), ints([1] * n), ints(lengths), ints(list(range(n))), ints([0] * n))
+    run = lambda: ops.latent_attention_tc(qa, store, table, *seqs, heads, rank, rot, width ** -0.5, window, splits, 1)
+    want = run()
+    assert bool(torch.isfinite(want).all())
+    for slot, length in enumerate(lengths):
+        for at in range(max(0, length - window)):
+            store[int(table[slot, at // 64]), 0, at % 64] = (float("nan"), float("inf"), -float("inf"))[at % 3]
+    assert torch.equal(run(), want)
+
+
 def test_parts_of_whole_pages():
     from starter_b200 import ops
 
