@@ -188,8 +188,9 @@ attention_rowwise_group_kernel(const T* __restrict__ q, T* __restrict__ out, con
       }
       s[0] += __shfl_xor_sync(0xffffffffu, s[0], 1);
       const float m_new = fmaxf(m[i], warp_max(seen ? s[0] : -INFINITY));
-      const float alpha = expf(m[i] - m_new);
-      p[i] = seen ? expf(s[0] - m_new) : 0.f;
+      // (scores of minus infinity alone, so far: they weigh nothing, whatever the other warps have)
+      const float m_use = m_new == -INFINITY ? 0.f : m_new, alpha = expf(m[i] - m_use);
+      p[i] = seen ? expf(s[0] - m_use) : 0.f;
       l[i] = l[i] * alpha + p[i];
       acc[i].x *= alpha; acc[i].y *= alpha; acc[i].z *= alpha; acc[i].w *= alpha;
       m[i] = m_new;

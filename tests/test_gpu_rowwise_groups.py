@@ -34,3 +34,25 @@ def test_groups_of_heads(heads, kv_heads, dim, window, dtype):
     off = (got.cpu().to(F).view_as(want) - want).abs().max()
     # float sums of up to 200 products of unit size, exponentials of 2 ulp; a rounding to bfloat16 is 2^-9 of the result
     assert float(off) <= (2e-6 if dtype == torch.float32 else 2.0 ** -8) * float(want.abs().max())
+
+
+# keys whose scores are minus infinity: the only key of a warp, all of a warp's first sixteen, all but the last
+@pytest.mark.parametrize("heads,kv_heads", [(3, 3), (4, 2), (8, 2)])
+@pytest.mark.parametrize("pos,gone", [(16, [16]), (32, [32]), (48, [48]), (100, list(range(16, 32)) + list(range(80, 96))), (77, list(range(77)))])
+def test_scores_of_minus_infinity_weigh_nothing(heads, kv_heads, pos, gone):
+    from starter_b200 import ops
+
+    dim, page = 64, ops.PAGE_TOKENS
+    gen = torch.Generator().manual_seed(pos)
+    store = [torch.randn(2, kv_heads, page, dim, generator=gen).cuda() for _ in range(2)]
+    q = torch.rand(1, heads * dim, generator=gen).cuda() + 0.5
+    rows = [store[0][j // page, :, j % page] for j in range(pos + 1)]
+    for j in gone:
+        rows[j][:, 3] = -float("inf")
+    zero = torch.zeros(1, dtype=torch.int32, device="cuda")
+    got = ops.attention_rowwise(q, *store, torch.tensor([[0, 1]], dtype=torch.int32).cuda(), zero, zero + pos, heads, kv_heads, dim, 0.125)
+    left = [j for j in range(pos + 1) if j not in gone]
+    k, v = (torch.stack([s[j // page, :, j % page] for j in left]).to(F) for s in store)
+    s = torch.einsum("hgd,khd->hgk", q.view(kv_heads, heads // kv_heads, dim).to(F) * 0.125, k)
+    want = torch.einsum("hgk,khd->hgd", torch.softmax(s, dim=-1), v).reshape(1, -1)
+    assert float((got.to(F) - want).abs().max()) <= 2e-6 * float(want.abs().max())
