@@ -15,6 +15,7 @@
 #include <ATen/autocast_mode.h>
 #include <ATen/cuda/EmptyTensor.h>
 #include <ATen/core/LegacyTypeDispatch.h>
+#include <ATen/record_function.h>
 #include <ATen/ops/mm_cuda_dispatch.h>
 #include <c10/core/GradMode.h>
 #include <c10/core/impl/LocalDispatchKeySet.h>
@@ -201,15 +202,16 @@ PyObject* empty(PyObject*, PyObject* const* args, Py_ssize_t n) {
 bool plain(const at::Tensor& t) {
   static const c10::DispatchKeySet usual =
       c10::DispatchKeySet({c10::DispatchKey::CUDA, c10::DispatchKey::ADInplaceOrView, c10::DispatchKey::AutogradCUDA, c10::DispatchKey::AutocastCUDA});
-  return t.is_cuda() && t.layout() == at::kStrided && !(t.key_set().raw_repr() & ~usual.raw_repr()) && !(t.requires_grad() && c10::GradMode::is_enabled());
+  return t.is_cuda() && t.layout() == at::kStrided && !(t.key_set().raw_repr() & ~usual.raw_repr()) && !(t.requires_grad() && c10::GradMode::is_enabled()) &&
+         !t._fw_grad(0).defined();           // (a dual number's tangent shows in neither: torch's one level of them)
 }
 bool plain_thread() {
   return !(c10::impl::tls_local_dispatch_key_set().included_.raw_repr() & ~c10::default_included_set.raw_repr()) && !at::autocast::is_autocast_enabled(at::kCUDA) &&
-         !at::impl::torch_function_mode_enabled();
+         !at::impl::torch_function_mode_enabled() && !at::hasCallbacks();      // (a profiler sees the operation at the dispatcher)
 }
 
 // product(x, w, low, high): x @ w.T by the library for contiguous bfloat16 matrices of low < rows < high on one device, as torch.mm(x, w.t()) calls
-// it (the dispatcher and the Python bindings of a view and a product less: a product of 300 rows keeps the host busy for 9.8 us in place of 12.9).  None where it is
+// it (the dispatcher and the Python bindings of a view and a product less: a product of 300 rows keeps the host busy for 9.7 us in place of 10.9).  None where it is
 // not that plain a call, or fails: torch.mm does it then, or says why not.
 PyObject* product(PyObject*, PyObject* const* args, Py_ssize_t n) {
   if (n == 4 && THPVariable_CheckExact(args[0]) && THPVariable_CheckExact(args[1]) && PyLong_Check(args[2]) && PyLong_Check(args[3])) {

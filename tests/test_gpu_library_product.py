@@ -49,3 +49,29 @@ def test_what_is_no_plain_product_goes_the_general_way():
         ops.linear(x, w, gated="no such activation")
     with pytest.raises(ops.KernelError):
         ops.linear(x, torch.randn(48, 32).to(BF).cuda())
+
+
+@pytest.mark.parametrize("which", ["x", "w", "both"])
+def test_tangents_are_carried(which):
+    from torch.autograd import forward_ad
+
+    from starter_b200 import ops
+
+    x, w, dx, dw = (torch.randn(*shape).to(BF).cuda() for shape in ((200, 64), (48, 64), (200, 64), (48, 64)))
+    with forward_ad.dual_level():
+        a = forward_ad.make_dual(x, dx) if which != "w" else x
+        b = forward_ad.make_dual(w, dw) if which != "x" else w
+        assert ops._product(a, b, 128, 512) is None
+        got, want = (forward_ad.unpack_dual(y) for y in (ops.linear(a, b), torch.mm(a, b.t())))
+        assert torch.equal(got.primal, want.primal) and torch.equal(got.tangent, want.tangent)
+    assert torch.equal(ops._product(x, w, 128, 512), torch.mm(x, w.t()))
+
+
+def test_a_profiler_sees_the_product():
+    from starter_b200 import ops
+
+    x, w = torch.randn(200, 64).to(BF).cuda(), torch.randn(48, 64).to(BF).cuda()
+    ops.linear(x, w)
+    with torch.profiler.profile(activities=[torch.profiler.ProfilerActivity.CPU]) as seen:
+        ops.linear(x, w)
+    assert "aten::mm" in {e.key for e in seen.key_averages()}
