@@ -2790,7 +2790,8 @@ def state_scan_norm(mode, q, k, v, a_raw, b_raw, A_log, dt_bias, skip, state, st
     n_seqs = _seq_arrays(seq_slot, seq_q_start, seq_q_len)
     if (mode == "channel_decay") != (decay is not None or low is not None):
         raise KernelError("decays per row of the state belong to the channel_decay recurrence")
-    if max_q_len == 1 and gain is not None and dtype == torch.bfloat16 and _state_step_takes(mode, heads, groups, n_state, v_dim):
+    if max_q_len == 1 and gain is not None and dtype == torch.bfloat16 and (low is None or low[0].dtype == dtype) and \
+            _state_step_takes(mode, heads, groups, n_state, v_dim):
         decays = [None, 0, None, None, 0, 0.0]
         if low is not None:
             decays = list(_low_rank(*low, n_tokens, heads * n_state))
@@ -2810,7 +2811,7 @@ def state_scan_norm(mode, q, k, v, a_raw, b_raw, A_log, dt_bias, skip, state, st
             if normed:
                 return out
             return group_norm_gate(out, *gate or (None, 0), gain, parts, eps, gate_first, dtype)
-    if low is not None:
+    if low is not None:                    # (of any type)
         decay = low_rank_decay(*low)
     if decay is not None:
         _f32(decay, "decay", (n_tokens, heads * n_state))

@@ -93,3 +93,25 @@ def test_one_token_steps(mode, heads, groups, N, V, aligned):
     bound = 2.0 ** -18 * (S.abs() + before[here, 4:].view(3, heads, N, V).to(F).abs() + S.abs().amax(-2, keepdim=True))
     assert bool(((left - S).abs() <= bound).all())
     assert torch.equal(state[[2, 3]], before[[2, 3]]) and torch.equal(state[:, :4], before[:, :4])
+
+
+@pytest.mark.parametrize("dtype", [BF, torch.float32])
+def test_low_rank_entries_of_either_type(dtype):
+    from starter_b200 import ops
+
+    gen = torch.Generator().manual_seed(5)
+    n, heads, N, V, rank = 3, 2, 64, 64, 12
+    rand = lambda *shape: torch.randn(*shape, generator=gen).cuda()
+    x, low, a2, bias, gain = rand(n, 4 * heads * N).to(BF), rand(n, rank).to(dtype), rand(rank, heads * N), rand(heads * N) + 2, rand(V)
+    ints = lambda t: torch.tensor(t, dtype=torch.int32, device="cuda")
+    at, w = heads * N, {"a2": a2, "a2_bias": bias, "gain": gain}
+    state = rand(n, heads * N * V)
+    before = state.clone().view(n, heads, N, V).to(F)
+    got = ops.state_scan_norm("channel_decay", (x, 0), (x, at), (x, 2 * at), None, None, None, None, None, state, 0, ints([0, 1, 2]),
+                              ints([0, 1, 2]), ints([1, 1, 1]), 1, heads, heads, N, V, gain, heads, 1e-6, gate=(x, 3 * at),
+                              low=(low, 0, a2, bias, 16.0))
+    cols = {"q": 0, "k": at, "v": 2 * at, "g": 3 * at, "low": 4 * at}
+    want, size, S = step("channel_decay", torch.cat([x.to(F), low.to(F)], dim=1), cols, w, before, heads, heads, N, V, True, gain, heads, False)
+    assert bool(((got.to(F) - want).abs() <= HALF_STEP * want.abs() + 2.0 ** -17 * size).all())
+    left = state.view(n, heads, N, V).to(F)
+    assert bool(((left - S).abs() <= 2.0 ** -18 * (S.abs() + before.abs() + S.abs().amax(-2, keepdim=True))).all())
