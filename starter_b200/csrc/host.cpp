@@ -24,7 +24,11 @@
 #include <torch/csrc/Dtype.h>
 #include <torch/csrc/autograd/python_variable.h>
 
+#include <algorithm>
 #include <cstring>
+#include <functional>
+#include <utility>
+#include <vector>
 
 namespace {
 
@@ -239,6 +243,82 @@ PyObject* product(PyObject*, PyObject* const* args, Py_ssize_t n) {
   Py_RETURN_NONE;
 }
 
+// A sequence of integers; false with an exception set.
+bool integers(PyObject* o, std::vector<long long>& out) {
+  PyObject* fast = PySequence_Fast(o, "a sequence of integers is wanted here");
+  if (!fast) return false;
+  const Py_ssize_t n = PySequence_Fast_GET_SIZE(fast);
+  out.resize(n);
+  for (Py_ssize_t i = 0; i < n; ++i) out[i] = PyLong_AsLongLong(PySequence_Fast_GET_ITEM(fast, i));
+  Py_DECREF(fast);
+  return !PyErr_Occurred();
+}
+
+// block_steps(kv lengths, new tokens, window): see latent_block_steps in ops.py.
+PyObject* block_steps(PyObject*, PyObject* const* args, Py_ssize_t n) {
+  std::vector<long long> kv, q, steps;
+  if (n != 3 || !integers(args[0], kv) || !integers(args[1], q)) {
+    if (!PyErr_Occurred()) PyErr_SetString(PyExc_TypeError, "block_steps(kv lengths, new tokens, window)");
+    return nullptr;
+  }
+  const long long window = PyLong_AsLongLong(args[2]);
+  if (PyErr_Occurred()) return nullptr;
+  for (size_t i = 0; i < kv.size() && i < q.size(); ++i) {
+    const long long past = kv[i] - q[i], base = window ? std::max(0ll, past - window + 1) : 0;
+    for (long long first = 0; first < q[i]; first += 256) {
+      const long long low = window ? std::max(0ll, past + first - window + 1) : 0;
+      steps.push_back((past + std::min(first + 256, q[i]) - 1 - base) / 64 - (low - base) / 64 + 1);
+    }
+  }
+  std::sort(steps.begin(), steps.end(), std::greater<long long>());
+  PyObject* out = PyTuple_New((Py_ssize_t)steps.size());
+  for (size_t i = 0; out && i < steps.size(); ++i) PyTuple_SET_ITEM(out, i, PyLong_FromLongLong(steps[i]));
+  return out;
+}
+
+// mixed_splits(steps, heads, SMs): see latent_mixed_splits in ops.py.  At most sixteen of the lengths are tried: 2 us with 16 heads, 21 with one (148 blocks).
+PyObject* mixed_splits(PyObject*, PyObject* const* args, Py_ssize_t n) {
+  std::vector<long long> steps;
+  if (n != 3 || !integers(args[0], steps)) {
+    if (!PyErr_Occurred()) PyErr_SetString(PyExc_TypeError, "mixed_splits(steps, heads, SMs)");
+    return nullptr;
+  }
+  const long long heads = PyLong_AsLongLong(args[1]), sms = PyLong_AsLongLong(args[2]);
+  if (PyErr_Occurred()) return nullptr;
+  if (steps.empty() || heads < 1 || sms < 1) return PyLong_FromLong(1);
+  std::sort(steps.begin(), steps.end(), std::greater<long long>());
+  std::vector<std::pair<long long, long long>> runs;         // (steps, blocks of all heads)
+  for (long long s : steps) {
+    if (runs.empty() || runs.back().first != s) runs.push_back({s, 0});
+    runs.back().second += heads;
+  }
+  const size_t apart = (runs.size() + 15) / 16;
+  long long best = 0, from = 0;
+  std::vector<long long> jobs;
+  for (size_t last = (runs.size() - 1) / apart * apart;; last -= apart) {      // blocks of runs[.. last] in two, the shortest such first
+    // the jobs, the longest first, as many as the estimate looks at
+    long long all = 0;
+    for (size_t k = 0; k < runs.size(); ++k) all += (k <= last ? 2 : 1) * runs[k].second;
+    jobs.clear();
+    size_t a = 0, b = last + 1;
+    while ((long long)jobs.size() < std::min(all, 2 * sms)) {
+      const long long half = a <= last ? (runs[a].first + 1) / 2 + 9 : -1, whole = b < runs.size() ? runs[b].first + 3 : -1;
+      const bool split = half >= whole;
+      const long long many = split ? 2 * runs[a].second : runs[b].second;
+      jobs.insert(jobs.end(), (size_t)std::min(many, 2 * sms - (long long)jobs.size()), split ? half : whole);
+      ++(split ? a : b);
+    }
+    long long time = jobs[0];
+    for (long long i = 0; i < std::min(sms, all - sms); ++i) time = std::max(time, jobs[sms - 1 - i] + jobs[sms + i] + 10);
+    if (!from || time < best) {
+      best = time;
+      from = runs[last].first;
+    }
+    if (!last) break;
+  }
+  return PyLong_FromLongLong((double)best <= 0.93 * (double)(steps[0] + 3) ? 2 | from << 8 : 1);
+}
+
 // stream(): the current CUDA stream's address.
 PyObject* stream(PyObject*, PyObject*) {
   try {
@@ -259,6 +339,8 @@ PyMethodDef methods[] = {
     {"need", (PyCFunction)(void (*)(void))need, METH_FASTCALL, nullptr},
     {"empty", (PyCFunction)(void (*)(void))empty, METH_FASTCALL, nullptr},
     {"product", (PyCFunction)(void (*)(void))product, METH_FASTCALL, nullptr},
+    {"block_steps", (PyCFunction)(void (*)(void))block_steps, METH_FASTCALL, nullptr},
+    {"mixed_splits", (PyCFunction)(void (*)(void))mixed_splits, METH_FASTCALL, nullptr},
     {"stream", stream, METH_NOARGS, nullptr},
     {"refuse_with", refuse_with, METH_O, nullptr},
     {nullptr, nullptr, 0, nullptr}};

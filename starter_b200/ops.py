@@ -93,10 +93,11 @@ def _refuse(t, name, dtype=None, ndim=None):
 # launch, are native too (csrc/host.cpp).  The first call of any of them loads the native part and puts it in these names.
 
 def _bind():
-    global _need, _empty, _stream, _product
+    global _need, _empty, _stream, _product, _block_steps, _mixed_splits
     host = build.load_host()
     host.refuse_with(_refuse)
     _need, _empty, _stream, _product = host.need, host.empty, host.stream, host.product
+    _block_steps, _mixed_splits = host.block_steps, host.mixed_splits
     return host
 
 
@@ -117,6 +118,14 @@ def _stream():
 def _product(x, weight, low, high):
     """``x @ weight.T`` by the library's product for plain bfloat16 matrices of ``low < rows < high``, or None."""
     return _bind().product(x, weight, low, high)
+
+
+def _block_steps(kv_lens, q_lens, window):
+    return _bind().block_steps(kv_lens, q_lens, window)
+
+
+def _mixed_splits(steps, heads, sms):
+    return _bind().mixed_splits(steps, heads, sms)
 
 
 class _Added:
@@ -1834,37 +1843,25 @@ def latent_prompt_takes(dtype, ctx, dim, rot, vdim, rank, scale, window=None, he
 
 def latent_block_steps(kv_lens, q_lens, window) -> tuple:
     """The steps of 64 keys that the blocks of 256 queries walk, the longest first, as csrc/attention_latent_prompt.cu counts them."""
-    steps = []
-    for kv, new in zip(kv_lens, q_lens):
-        base = max(0, kv - new - int(window) + 1) if window else 0
-        for first in range(0, new, 256):
-            low = max(0, kv - new + first - int(window) + 1) if window else 0
-            steps.append((kv - new + min(first + 256, new) - 1 - base) // 64 - (low - base) // 64 + 1)
-    return tuple(sorted(steps, reverse=True))
+    return _block_steps(kv_lens, q_lens, int(window or 0))
 
 
 def latent_mixed_splits(steps: tuple, heads: int) -> int:
-    """``splits`` of ``sb_latent_prompt`` for blocks of ``steps`` steps of 64 keys (the longest first), ``heads`` heads each, that leave SMs
+    """``splits`` of ``sb_latent_prompt`` for blocks of ``steps`` steps of 64 keys, ``heads`` heads each, that leave SMs
     idle but are too many for two CTAs each: 1, or 2 with the steps from which a block is shared by two CTAs in its second byte
     on.  A causal prompt's last blocks walk many times the keys of its first, and their chain is the kernel's time.
 
     That with the least time on the busiest SM by this estimate, in steps (1.5 us): a block alone takes its steps and 3, half a block its
     steps and 9 (the cluster's launch, two barriers, the merge), and a CTA beyond one an SM starts 10 behind the end of a short one,
-    because the two of a cluster want two SMs at once.  Measured (us a layer of 16 heads, one CTA a block / two from 16, 20, 24, 28
-    steps on): 2,048 tokens 147 / 151, 152, 146, 137; 1,600 133 / 136, 129, 126, 133; 1,300 114 / 106, 109, 114; 1,300 behind 700 132 / 137,
-    137, 122, 127; 1,200 behind 1,200 136 / 142, 142, 120, 126; 2 x 1,000 126 / 129; a window of 1,024 over 2,000 134 / 150."""
-    def time(split_from):
-        jobs = sorted((job for s in steps for job in (2 * [-(-s // 2) + 9] if s >= split_from else [s + 3]) * heads), reverse=True)
-        behind = [jobs[SM_COUNT - 1 - i] + jobs[SM_COUNT + i] + 10 for i in range(min(SM_COUNT, len(jobs) - SM_COUNT))]
-        return max([jobs[0]] + behind), split_from
+    because the two of a cluster want two SMs at once.  Up to sixteen lengths, evenly among those that there are, are tried.  It is formed
+    for every layer anew, natively (csrc/host.cpp): prompts in service hardly repeat their lengths.
 
-    most, split_from = min(time(s) for s in set(steps))
-    return 2 | split_from << 8 if most <= 0.93 * (steps[0] + 3) else 1
-
-
-@functools.lru_cache(maxsize=1024)
-def _latent_mixed(kv_lens, q_lens, window, heads) -> int:
-    return latent_mixed_splits(latent_block_steps(kv_lens, q_lens, window), heads)
+    Measured (us a layer, one CTA a block / as chosen here): 16 heads, 2,048 tokens 146 / 137, 1,300 behind 700 129 / 120; 12 heads, 2,048
+    140 / 125, 2,300 150 / 135; 8 heads, 3,200 166 / 144; 4, 6,400 267 / 212; 2, 12,800 460 / 347; 1, 20,000 680 / 498.  Where the line
+    lies, 16 heads, whole / from 16, 20, 24, 28 steps on: 2,048 tokens 147 / 151, 152, 146, 137; 1,600 133 / 136, 129, 126, 133; 1,300 114 / 106,
+    109, 114; 1,300 behind 700 132 / 137, 137, 122, 127; 1,200 behind 1,200 136 / 142, 142, 120, 126; 2 x 1,000 126 / 129; a window of 1,024 over
+    2,000 134 / 150."""
+    return _mixed_splits(steps, heads, SM_COUNT)
 
 
 def latent_attention_prompt(q, ukv, store, block_table, ctx, heads, dim, vdim, rank, rot, scale, window=None, sink=None, turn=None, gate=None):
@@ -1914,8 +1911,9 @@ def latent_attention_prompt(q, ukv, store, block_table, ctx, heads, dim, vdim, r
         if at % 16 == 0 and gate[0].shape[1] % 8 == 0:
             gated = [at, gate[0].shape[1]]
     splits = prompt_splits(heads * ctx.block_first.shape[0], ctx.max_kv_len, window)
-    if splits == 1 and SM_COUNT < 2 * heads * ctx.block_first.shape[0] <= 2 * SM_COUNT:
-        splits = _latent_mixed(tuple(ctx.host["seq_kv_len"].tolist()), tuple(ctx.host["seq_q_len"].tolist()), window, heads)
+    if splits == 1 and SM_COUNT < 2 * heads * ctx.block_first.shape[0] <= 2 * SM_COUNT and (dim, vdim) != (64, 128):
+        # (64 and 128: a CTA a block always)
+        splits = latent_mixed_splits(latent_block_steps(ctx.host["seq_kv_len"].tolist(), ctx.host["seq_q_len"].tolist(), window), heads)
     rc = lib.sb_latent_prompt(
         q, kv, shared, out, ctx.seq_q_start, ctx.seq_q_len, ctx.seq_kv_len,
         ctx.block_seq, ctx.block_first, ctx.block_seq.shape[0], n_tokens, rows, heads, dim, vdim,

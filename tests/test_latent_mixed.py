@@ -1,6 +1,9 @@
 """Latent prompts whose longer blocks are shared by two CTAs of a cluster while the shorter ones go to one each: the kernel against a CTA a
 block, and the rule that says from how many steps on."""
 
+import random
+import time
+
 import pytest
 import torch
 
@@ -63,3 +66,39 @@ def test_which_blocks_are_shared():
         for steps in ((1,), (500,), (60, 3), (60, 60)):
             got = ops.latent_mixed_splits(steps, heads)
             assert got == 1 or (got & 255 == 2 and 1 <= got >> 8 <= steps[0])
+
+
+def test_the_plan_is_the_estimates_least():
+    from starter_b200 import ops
+
+    def plain(steps, heads):
+        def cost(split_from):
+            jobs = sorted((job for s in steps for job in (2 * [-(-s // 2) + 9] if s >= split_from else [s + 3]) * heads), reverse=True)
+            behind = [jobs[147 - i] + jobs[148 + i] + 10 for i in range(min(148, len(jobs) - 148))]
+            return max([jobs[0]] + behind), split_from
+        most, split_from = min(cost(s) for s in set(steps))
+        return 2 | split_from << 8 if most <= 0.93 * (max(steps) + 3) else 1
+
+    rng, shared = random.Random(1), 0
+    for _ in range(400):
+        heads = rng.choice((1, 2, 5, 12, 16))
+        lengths = [rng.randint(1, 80) for _ in range(rng.randint(1, 16))]
+        steps = tuple(sorted((rng.choice(lengths) for _ in range(rng.randint(75 // heads + 1, 148 // heads))), reverse=True))
+        shared += plain(steps, heads) > 1
+        assert ops.latent_mixed_splits(steps, heads) == plain(steps, heads)
+    assert 50 < shared < 350
+    with pytest.raises(TypeError):
+        ops.latent_mixed_splits(("a",), 4)
+
+
+@pytest.mark.parametrize("heads,tokens", [(16, 2048), (4, 7000), (1, 36000)])
+def test_a_plan_for_new_lengths_costs_little(heads, tokens):
+    """(It stands in front of the launches of a step's first latent layer, whose gain is some 10 us.)"""
+    from starter_b200 import ops
+
+    took = []
+    for i in range(7):
+        began = time.perf_counter()
+        ops.latent_mixed_splits(ops.latent_block_steps([tokens + i], [tokens + i], None), heads)
+        took.append(time.perf_counter() - began)
+    assert min(took[1:]) < 1e-4
