@@ -204,10 +204,13 @@ __global__ void __launch_bounds__(512) moe_route_kernel(const T* __restrict__ h,
 // keeps the sums of TPW tokens and eight experts (a piece of a router's row serves TPW tokens, a piece of a token eight experts), and
 // each sum has the terms and the order that moe_logits gives it: the same bits.  The choice keeps a token's logits in the lanes'
 // registers and finds the largest by the warp's integer maximum.
-// Measured, four tokens a block / here, us: 16 experts of 2,048 600 tokens 9.8 / 8.9, 2,048 11.3 / 9.2 (behind other kernels, whose
-// weights have emptied the caches, 18.0 / 12.4), 4,096 21.1 / 17.6; 8 of 1,024 600 7.4 / 5.1; 32 of 1,536 1,000 9.7 / 12.5, 2,048 18.1 /
-// 12.9; 64 of 2,048 1,000 17.7 / 27.9, 2,048 33.5 / 28.5: a block's passes over 16 experts are a chain, which more than sixteen want 1,184
-// tokens for.  Stages of 256 entries, four: 13.2 (2,048 tokens of 16 experts).
+// Both kinds run in waves: 1,184 tokens (more than 16 experts) or 2,368 (up to 16) of four a block, 2,368 of sixteen a block; and a block's
+// passes over 16 experts are a chain.  So more than 16 experts want more than a wave of the other kind.  Measured, four tokens a block /
+// here, us, width 2,048, in a row (and with the caches emptied in front, as behind other layers): 8 experts 592 tokens 8.6 / 6.6 (18.4 / 12.3);
+// 16 592 8.7 / 8.4 (18.4 / 14.3), 2,368 13.1 / 10.9 (20.5 / 16.4), 5,000 31.7 / 27.2 (41 / 33); 32 1,184 10.3 / 14.8 (20.4 / 20.7), 1,400 19.1 /
+// 14.8 (30.7 / 22.5), 2,600 28.3 / 28.5 (39 / 35); 48 1,184 15.2 / 20.9 (30.7 / 28.7), 1,400 28.7 / 21.0 (45 / 29), 2,600 42.7 / 40.7 (59 / 49); 64
+// 1,184 16.2 / 27.0 (30.7 / 34.8), 1,400 30.8 / 27.3 (45 / 35), 2,600 45.8 / 52.9 (61.4 / 59.4), 8,192 112 / 109 (127 / 115).  Stages of 256 entries,
+// four: 13.2 for 12.4 (2,048 tokens of 16 experts).
 #define ROUTE_TOKENS 16
 #define ROUTE_EXPERTS 64
 #define ROUTE_STAGES 3
@@ -1404,6 +1407,11 @@ int sb_moe_gather(const void* h, const int* sorted, const int* n_tiles, int tile
 int sb_moe_max_experts() { return MOE_MAX_EXPERTS; }
 int sb_moe_max_top() { return MOE_MAX_TOP; }
 
+// From how many tokens on a block of the router takes sixteen of them (moe_route_many_kernel).
+int sb_moe_route_many_from(int experts) {
+  return experts > 16 ? 8 * 148 + 1 : 4 * 148;
+}
+
 // h: [n_tokens, width]; w: float [experts, width]; b: float [experts] or null; ids: int [n_tokens, top];
 // weights: float [n_tokens, top].
 // scoring 0: softmax over the chosen logits; 1: sigmoid scores divided by their sum, times weight_scale; 3: plain
@@ -1413,7 +1421,7 @@ int sb_moe_route(int dtype, const void* h, const float* w, const float* b, int* 
   if (n_tokens == 0) return 0;
   if (experts < 1 || experts > MOE_MAX_EXPERTS || top < 1 || top > MOE_MAX_TOP || top > experts) return -2;
   if (scoring != 0 && scoring != 1 && scoring != 3) return -2;
-  if (dtype == 1 && n_tokens >= (experts > 16 ? 8 : 4) * 148 && experts <= ROUTE_EXPERTS && width % 8 == 0 && !(((uintptr_t)h | (uintptr_t)w) % 16)) {
+  if (dtype == 1 && n_tokens >= sb_moe_route_many_from(experts) && experts <= ROUTE_EXPERTS && width % 8 == 0 && !(((uintptr_t)h | (uintptr_t)w) % 16)) {
     const int groups = experts > 8 ? 2 : 1;
     const int smem = ROUTE_STAGES * (groups * 8 * ROUTE_K * 4 + ROUTE_TOKENS * ROUTE_K * 2);
     const auto kernel = groups == 2 ? moe_route_many_kernel<2> : moe_route_many_kernel<1>;

@@ -267,3 +267,11 @@ def test_products_over_tiles_of_eight_rows_come_in_pairs(up):
     tile_rows = 8
     # (refused in front of any launch, so no address is looked at)
     assert entry(1, up, tile_rows, None, None, None, None, None, None, 1, 64, 64, 1, 0.0, None, None) == -2
+
+
+def test_the_router_takes_sixteen_tokens_a_block_behind_a_wave_of_four_a_block():
+    from starter_b200.csrc import build
+
+    entry = build.load("moe").sb_moe_route_many_from
+    # (two blocks of four an SM with more than 16 experts: 1,184 tokens of 64 experts 16 us, in sixteens 27)
+    assert [entry(n) for n in (1, 16, 17, 64)] == [592, 592, 1185, 1185]
