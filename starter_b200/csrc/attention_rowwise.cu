@@ -1,5 +1,5 @@
-// Causal grouped-query attention over the paged cache: a block of four warps for the query heads of a group and a token, or (heads of more
-// than 128 entries or no multiple of 4) one warp per (query token, query head).
+// Causal grouped-query attention over the paged cache: two warps a query head and token or four warps up to four heads of a group, or (heads
+// of more than 128 entries or no multiple of 4) one warp per (query token, query head).
 //
 // This is the plain kernel: it serves the whole 32-bit path (prompts and single tokens alike) and any
 // shape the faster bfloat16 kernels refuse.  A query at absolute position p of the sequence in `slot`
@@ -112,24 +112,34 @@ template <> struct RowPiece<bf16> {
   static __device__ __forceinline__ uint2 zero() { return make_uint2(0u, 0u); }
 };
 
-// A block of four warps has HB query heads of one key/value head and a token: a warp takes every fourth sixteen keys, which serve all HB
-// heads, and the warps' sums meet in shared memory.  What bounds a prompt here is the chain of rounds a warp walks: a quarter of those
-// that a warp a head and token has, and a key is asked for once in place of once a head.  A warp a head -> here, us a float32 layer:
-// 40 tokens behind 150, 16 heads of 8, 113.5 -> 105.2; 150 tokens, 16 of 4, 133.0 -> 125.4; 17 + 17 behind 60 78.1 -> 74.8; 77 + 64
-// tokens 151.2 -> 150.3 (the attention 13.8 -> 11.3).  Three blocks an SM in place of four (no spills): 151.9, 103.4, 129.2, 75.5.
+// W warps have HB query heads of one key/value head and a token (a unit): a warp takes every W-th sixteen keys, which serve all HB heads,
+// and the warps' sums meet in shared memory.  What bounds a step of few tokens here is the chain of rounds a warp walks, one of many its
+// issue slots and the keys' way from L2.  HB 1, W 2, two units a block: half the rounds of a warp a head and token, three blocks an SM (145
+// registers, no spills; four an SM spill 52 bytes).  HB 4, W 4: keys and values are asked for once for four heads, four blocks an SM (spills of
+// 192 bytes; three an SM are slower: 154 tokens 151.9 for 150.3), from 1,184 heads of tokens on, when its blocks fill half the SMs' places.
+// Measured, a float32 layer, us, a warp a head / HB 1 / HB 4, groups of four (16 heads): 20 tokens 77.4 / 76.0 / 79.2, 40 behind 150 113.7 / 94.2 /
+// 96.5, 100 108.6 / 106.5 / 104.2, 120 behind 100 144.0 / 131.8 / 119.0, 2 x 77 126.2 / 125.4 / 125.5, 2 x 150 244.8 / 241.5 / 231.7; of six (12
+// heads) 100 100.6 / 94.4 / 96.0, 2 x 77 113.4 / 113.1 / 115.6, 2 x 110 183.2 / 182.3 / 180.9; of eight 20 76.1 / 74.8 / 78.2, 100 106.6 / 104.3 /
+// 102.5, 2 x 110 196.0 / 195.4 / 189.2.  Smaller groups, a warp a head / HB 1 / four warps up to four heads: of one 2 x 77 152.0 / 151.3 / 154.6,
+// 40 behind 150 129.4 / 111.1 / 114.3; of two 2 x 77 129.0 / 129.4 / 133.7, 40 behind 150 116.6 / 98.2 / 104.1, 2 x 150 251.5 / 250.8 / 253.0; of three
+// 2 x 77 114.9 / 115.0 / 117.6, 40 behind 150 101.2 / 87.7 / 90.4, 2 x 150 224.0 / 221.3 / 219.2.
+#define ROW_UNIT_WARPS(HB) ((HB) == 1 ? 2 : 4)
 template <typename T, int HB>
-__global__ void __launch_bounds__(128, 4)
+__global__ void __launch_bounds__(128, HB == 1 ? 3 : 4)
 attention_rowwise_group_kernel(const T* __restrict__ q, T* __restrict__ out, const T* __restrict__ k_store,
                                const T* __restrict__ v_store, const int* __restrict__ block_table, int table_stride,
                                const int* __restrict__ tok_slot, const int* __restrict__ tok_pos, int heads,
-                               int kv_heads, int head_dim, float scale, int window) {
+                               int kv_heads, int head_dim, float scale, int window, unsigned units) {
   typedef RowPiece<T> Piece;
   typedef typename Piece::type Raw;
+  constexpr int W = ROW_UNIT_WARPS(HB);
   __shared__ __align__(16) float sums[4][HB][128];
   __shared__ float most[4][HB], total[4][HB];
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const int group = heads / kv_heads, shares = (group + HB - 1) / HB;
-  const int token = blockIdx.x / (kv_heads * shares), rest = blockIdx.x - token * (kv_heads * shares);
+  const int turn = warp % W;
+  const unsigned unit = min(blockIdx.x * (4 / W) + warp / W, units - 1);           // (an odd last one is done twice)
+  const int token = unit / (unsigned)(kv_heads * shares), rest = unit - token * (unsigned)(kv_heads * shares);
   const int kvh = rest / shares, h0 = kvh * group + (rest - kvh * shares) * HB, here = min(HB, (kvh + 1) * group - h0);
   const int pos = tok_pos[token];
   const int* pages = block_table + (size_t)tok_slot[token] * table_stride;
@@ -149,7 +159,7 @@ attention_rowwise_group_kernel(const T* __restrict__ q, T* __restrict__ out, con
   int first = 0;
   if (window > 0 && pos - window + 1 > 0) first = pos - window + 1;
 #pragma unroll 1
-  for (int j0 = first + warp * ROW_KEYS; j0 <= pos; j0 += 4 * ROW_KEYS) {
+  for (int j0 = first + turn * ROW_KEYS; j0 <= pos; j0 += W * ROW_KEYS) {
     // a lane a key looks up its page
     const int mine = min(j0 + (lane & (ROW_KEYS - 1)), pos);
     const long long at = (long long)page_row(pages[mine / SB_PAGE_TOKENS], kvh, mine % SB_PAGE_TOKENS, kv_heads, head_dim);
@@ -215,16 +225,19 @@ attention_rowwise_group_kernel(const T* __restrict__ q, T* __restrict__ out, con
     }
   }
   __syncthreads();
-  for (int i = warp; i < here; i += 4) {
+  const int w0 = warp - turn;
+  for (int i = turn; i < here; i += W) {
     // (a warp without keys has minus infinity and zeros)
-    const float top = fmaxf(fmaxf(most[0][i], most[1][i]), fmaxf(most[2][i], most[3][i]));
+    float top = most[w0][i];
+#pragma unroll
+    for (int w = 1; w < W; ++w) top = fmaxf(top, most[w0 + w][i]);
     float4 o = make_float4(0.f, 0.f, 0.f, 0.f);
     float sum = 0.f;
 #pragma unroll
-    for (int w = 0; w < 4; ++w) {
-      const float by = expf(most[w][i] - top);
-      const float4 a = *reinterpret_cast<const float4*>(&sums[w][i][d]);
-      sum += by * total[w][i];
+    for (int w = 0; w < W; ++w) {
+      const float by = expf(most[w0 + w][i] - top);
+      const float4 a = *reinterpret_cast<const float4*>(&sums[w0 + w][i][d]);
+      sum += by * total[w0 + w][i];
       o.x += by * a.x; o.y += by * a.y; o.z += by * a.z; o.w += by * a.w;
     }
     if (in) {
@@ -242,12 +255,16 @@ template <typename T>
 static int rowwise_group(const void* q, void* out, const void* k_store, const void* v_store, const int* block_table, int table_stride,
                          const int* tok_slot, const int* tok_pos, int n_tokens, int heads, int kv_heads, int head_dim, float scale,
                          int window, cudaStream_t s) {
-  const int group = heads / kv_heads, each = group == 1 ? 1 : group == 2 ? 2 : 4;
-  const long long blocks = (long long)n_tokens * kv_heads * ((group + each - 1) / each);
-  const auto kernel = each == 1 ? attention_rowwise_group_kernel<T, 1> : each == 2 ? attention_rowwise_group_kernel<T, 2>
-                                                                                   : attention_rowwise_group_kernel<T, 4>;
-  kernel<<<(unsigned)blocks, 128, 0, s>>>((const T*)q, (T*)out, (const T*)k_store, (const T*)v_store, block_table, table_stride, tok_slot,
-                                          tok_pos, heads, kv_heads, head_dim, scale, window);
+  const int group = heads / kv_heads;
+  const long long fours = (long long)n_tokens * kv_heads * ((group + 3) / 4), ones = (long long)n_tokens * heads;
+  if (group >= 4 && ones >= 8 * 148)
+    attention_rowwise_group_kernel<T, 4><<<(unsigned)fours, 128, 0, s>>>(
+        (const T*)q, (T*)out, (const T*)k_store, (const T*)v_store, block_table, table_stride, tok_slot, tok_pos, heads, kv_heads, head_dim,
+        scale, window, (unsigned)fours);
+  else
+    attention_rowwise_group_kernel<T, 1><<<(unsigned)((ones + 1) / 2), 128, 0, s>>>(
+        (const T*)q, (T*)out, (const T*)k_store, (const T*)v_store, block_table, table_stride, tok_slot, tok_pos, heads, kv_heads, head_dim,
+        scale, window, (unsigned)ones);
   return SB_LAUNCH_RESULT();
 }
 

@@ -1,5 +1,5 @@
-"""The plain attention's blocks of four warps for the query heads of one key/value head: groups of all sizes, contexts that end before,
-at and behind a warp's sixteen keys and a round of sixty-four, windows, head sizes, against float64."""
+"""The plain attention's two warps a query head, and its four warps up to four heads of a group in steps of many tokens: groups of all
+sizes, contexts that end before, at and behind a warp's sixteen keys and a round of sixty-four, windows, head sizes, against float64."""
 
 import pytest
 import torch
@@ -12,6 +12,17 @@ F = torch.float64
                                                        (4, 1, 4, 0), (8, 2, 128, 1), (8, 2, 64, 40), (3, 1, 128, 17)])
 @pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
 def test_groups_of_heads(heads, kv_heads, dim, window, dtype):
+    against_float64(heads, kv_heads, dim, window, dtype, 1)
+
+
+# (four heads a block from 1,184 heads of tokens on; groups that leave a block with one to four heads)
+@pytest.mark.parametrize("heads,kv_heads,dim,window", [(4, 1, 128, 0), (5, 1, 36, 0), (6, 1, 64, 17), (16, 2, 128, 0), (12, 3, 4, 40), (11, 1, 100, 1)])
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+def test_four_heads_a_block(heads, kv_heads, dim, window, dtype):
+    against_float64(heads, kv_heads, dim, window, dtype, 1 + 1184 // (26 * heads))
+
+
+def against_float64(heads, kv_heads, dim, window, dtype, copies):
     from starter_b200 import ops
 
     gen = torch.Generator().manual_seed(heads * dim + window)
@@ -24,7 +35,13 @@ def test_groups_of_heads(heads, kv_heads, dim, window, dtype):
     tok_slot = torch.tensor([0] * len(pos) + [1] * len(pos), dtype=torch.int32)
     q = torch.randn(len(tok_pos), heads * dim, generator=gen).to(dtype).cuda()
     scale = dim ** -0.5
-    got = ops.attention_rowwise(q, *store, order.cuda(), tok_slot.cuda(), tok_pos.cuda(), heads, kv_heads, dim, scale, window or None)
+    if copies > 1:
+        assert copies * len(tok_pos) * heads >= 1184
+    got = ops.attention_rowwise(q.repeat(copies, 1), *store, order.cuda(), tok_slot.repeat(copies).cuda(), tok_pos.repeat(copies).cuda(), heads,
+                                kv_heads, dim, scale, window or None)
+    got = got.view(copies, len(tok_pos), -1)
+    assert torch.equal(got, got[:1].expand_as(got))
+    got = got[0]
     want = torch.empty(len(tok_pos), heads, dim, dtype=F)
     for t, (slot, p) in enumerate(zip(tok_slot.tolist(), tok_pos.tolist())):
         first = max(0, p - window + 1) if window else 0
@@ -38,8 +55,9 @@ def test_groups_of_heads(heads, kv_heads, dim, window, dtype):
 
 # keys whose scores are minus infinity: the only key of a warp, all of a warp's first sixteen, all but the last
 @pytest.mark.parametrize("heads,kv_heads", [(3, 3), (4, 2), (8, 2)])
+@pytest.mark.parametrize("copies", [1, 500])
 @pytest.mark.parametrize("pos,gone", [(16, [16]), (32, [32]), (48, [48]), (100, list(range(16, 32)) + list(range(80, 96))), (77, list(range(77)))])
-def test_scores_of_minus_infinity_weigh_nothing(heads, kv_heads, pos, gone):
+def test_scores_of_minus_infinity_weigh_nothing(heads, kv_heads, pos, gone, copies):
     from starter_b200 import ops
 
     dim, page = 64, ops.PAGE_TOKENS
@@ -49,8 +67,9 @@ def test_scores_of_minus_infinity_weigh_nothing(heads, kv_heads, pos, gone):
     rows = [store[0][j // page, :, j % page] for j in range(pos + 1)]
     for j in gone:
         rows[j][:, 3] = -float("inf")
-    zero = torch.zeros(1, dtype=torch.int32, device="cuda")
-    got = ops.attention_rowwise(q, *store, torch.tensor([[0, 1]], dtype=torch.int32).cuda(), zero, zero + pos, heads, kv_heads, dim, 0.125)
+    zero = torch.zeros(copies, dtype=torch.int32, device="cuda")
+    got = ops.attention_rowwise(q.repeat(copies, 1), *store, torch.tensor([[0, 1]], dtype=torch.int32).cuda(), zero, zero + pos, heads, kv_heads, dim,
+                                0.125)
     left = [j for j in range(pos + 1) if j not in gone]
     k, v = (torch.stack([s[j // page, :, j % page] for j in left]).to(F) for s in store)
     s = torch.einsum("hgd,khd->hgk", q.view(kv_heads, heads // kv_heads, dim).to(F) * 0.125, k)
