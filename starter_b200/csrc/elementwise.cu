@@ -206,8 +206,12 @@ __global__ void rmsnorm_vec_kernel(T* __restrict__ x, const T* __restrict__ delt
 // whose chain (load, block reduction with two barriers, store) is latency, in two waves: 10 us for
 // 21 MB.  A warp per row needs no barrier, 64 rows are in flight on an SM and all rows at once.  NV > 0: a lane keeps the
 // NV pieces of its row as they came (rows of up to NV * 32 pieces), so that all of a row is asked for at once and read once; 0: any
-// row, read twice (the second time from L1/L2, where this lane's own writes of the sum are).  2,400 rows of 2,560 behind a product, in a
-// pass: 17.7 us read twice, 11.1 kept (25 MB, 3.8 at the copy rate).
+// row, read twice (the second time from L1/L2, where this lane's own writes of the sum are).  Registers leave two blocks of the kept kind an
+// SM (2,368 rows at once), three of the other: kept up to two such waves, of sixteen pieces up to one.  With an addition sixteen pieces are
+// twice the registers (4,096 wide 13.5 -> 18.6 us at 1,800 rows): read twice.  Between two products, us a layer read twice / kept: 2,560 wide
+// with an addition 1,184 rows 59.1 / 48.6, 2,368 87.8 / 73.2, 2,400 88.3 / 77.8, 4,736 136.5 / 130.5, 6,000 177.7 / 178.6, 8,192 226.5 / 235.3;
+// 2,048 without 2,048 60.7 / 55.5, 4,736 113.9 / 111.6, 8,192 173.3 / 177.9; 4,096 without 1,500 85.8 / 79.6, 2,400 111.7 / 111.1, 3,552 150.8 /
+// 158.2, 8,192 338 / 368.
 template <typename T, typename W, bool ADD, int NV>
 __global__ void rmsnorm_warp_kernel(T* __restrict__ x, const T* __restrict__ delta,
                                     const W* __restrict__ gain, T* __restrict__ y, int n_rows,
@@ -310,7 +314,8 @@ static int launch_rmsnorm(void* x, const void* delta, const void* gain, void* y,
   if (aligned && !rows && n_rows > 256 && x != y) {
     const int threads_w = 256;                       // 8 rows a block
     const int blocks = (n_rows + 7) / 8;
-    const int pieces = (hidden / N + 31) / 32;       // of a lane
+    int pieces = (hidden / N + 31) / 32;             // of a lane
+    if (pieces > (blocks <= 2 * 148 ? 16 : blocks <= 4 * 148 ? 12 : 0)) pieces = 17;      // (read twice)
 #define WARP_LAUNCH(A, NV) launch_dependent(rmsnorm_warp_kernel<T, W, A, NV>, dim3(blocks), dim3(threads_w), 0, s, xp, dp, gp, yp, n_rows, hidden, eps)
     if (delta) return pieces <= 8 ? WARP_LAUNCH(true, 8) : pieces <= 12 ? WARP_LAUNCH(true, 12) : WARP_LAUNCH(true, 0);
     return pieces <= 8 ? WARP_LAUNCH(false, 8) : pieces <= 12 ? WARP_LAUNCH(false, 12) : pieces <= 16 ? WARP_LAUNCH(false, 16) : WARP_LAUNCH(false, 0);

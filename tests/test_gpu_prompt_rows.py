@@ -33,6 +33,20 @@ def test_norms_of_many_rows(dtype, hidden, add):
     assert bool(((got - want).abs() <= bound * want.abs()).all())
 
 
+@pytest.mark.parametrize("dtype,hidden,rows", [(torch.bfloat16, 4096, 2369), (torch.bfloat16, 3072, 4737), (torch.float32, 512, 4737), (torch.float32, 2048, 2369)])
+@pytest.mark.parametrize("add", [False, True])
+def test_norms_of_more_rows_than_are_kept_have_the_same_bits(dtype, hidden, rows, add):
+    from starter_b200 import ops
+
+    gen = torch.Generator().manual_seed(rows)
+    x, d = (torch.randn(rows, hidden, generator=gen).to(dtype).cuda() for _ in range(2))
+    gain = torch.rand(hidden, generator=gen).to(dtype).cuda() + 0.5
+    few, many = x[1:].clone(), x.clone()
+    want = ops.rmsnorm(few, gain, 1e-6, delta=d[1:] if add else None)         # a row less: the last step whose rows are kept
+    assert torch.equal(ops.rmsnorm(many, gain, 1e-6, delta=d if add else None)[1:], want)
+    assert torch.equal(many[1:], few)
+
+
 @pytest.mark.parametrize("d", [32, 128])
 def test_rotation_has_the_bits_of_rounded_float_products(d):
     """Without a norm every step is a product or a sum of two bfloat16 values: equal to float operations rounded one by one, for
