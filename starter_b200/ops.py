@@ -2842,14 +2842,14 @@ def state_scan_norm(mode, q, k, v, a_raw, b_raw, A_log, dt_bias, skip, state, st
     return out if gain is None else group_norm_gate(out, *gate or (None, 0), gain, parts, eps, gate_first, dtype)
 
 
-def _low_rank(u, col, a2, bias, tau, n_tokens=None, channels=None):
-    """A low-rank decay's checked operands: the entries' address and row width, ``a2``, ``bias``, the rank and ``1 / tau``."""
+def _low_rank(u, col, a2, bias, tau, n_tokens, channels):
+    """A low-rank decay's checked operands: the entries' address and row width, ``a2``, ``bias``, the rank and ``1 / tau``.  (What
+    ``low_rank_decay`` checks, which stands by itself as ``group_norm_gate`` does: a short prompt is bound by the host, 33 us a layer, of which
+    shared helpers took one.)"""
     _need(u, "u", None, 2)
     _need(a2, "a2", torch.float32, 2)
     rank = a2.shape[0]
-    if channels is None:
-        channels = a2.shape[1]
-    elif a2.shape[1] != channels or u.shape[0] != n_tokens:
+    if a2.shape[1] != channels or u.shape[0] != n_tokens:
         raise KernelError(f"a decay of {tuple(u.shape)} by {tuple(a2.shape)} is not one of {channels} rows for {n_tokens} tokens")
     _f32(bias, "bias", (channels,))
     if col < 0 or col + rank > u.shape[1]:
@@ -2865,10 +2865,19 @@ def low_rank_decay(u, col, a2, bias, tau):
     """``1 - sigmoid(z) ** (1 / tau)`` with ``z = u @ a2 + bias``: how much of its row of a recurrent state every channel lets
     go of a token.  ``u``: the columns ``col .. col + R`` of a ``[T, N]`` tensor; ``a2`` float32 ``[R, C]``, ``bias`` float32
     ``[C]``.  The product, the logarithm and the exponential are float; returns float32 ``[T, C]``."""
-    operands = _low_rank(u, col, a2, bias, tau)
-    n_tokens, channels = u.shape[0], a2.shape[1]
-    out = _empty(u, (n_tokens, channels), torch.float32)
-    rc = _lib("state_scan").sb_low_rank_decay(_code(u.dtype), *operands[:4], out, n_tokens, channels, *operands[4:], _stream())
+    _need(u, "u", None, 2)
+    _need(a2, "a2", torch.float32, 2)
+    rank, channels = a2.shape
+    _f32(bias, "bias", (channels,))
+    if col < 0 or col + rank > u.shape[1]:
+        raise KernelError(f"{rank} columns from {col} of {tuple(u.shape)} are not there")
+    if not tau > 0.0:
+        raise KernelError(f"tau={tau} must be positive")
+    out = _empty(u, (u.shape[0], channels), torch.float32)
+    rc = _lib("state_scan").sb_low_rank_decay(_code(u.dtype), _at(u, col), u.shape[1], a2, bias, out,
+                                              u.shape[0], channels, rank, 1.0 / tau, _stream())
+    if rc == -2:
+        raise KernelError(f"the low-rank decay takes ranks of 1 to 1024, not {rank}")
     _check(rc, "low_rank_decay")
     return out
 
@@ -2895,12 +2904,17 @@ def group_norm_gate(o, z, z_col, weight, parts, eps, gate_first, dtype):
     the parts share it.  Returns ``[T, N]`` in ``dtype``."""
     _need(o, "o", torch.float32, 2)
     n_tokens, width = o.shape
+    _need(weight, "weight", torch.float32, 1)
     if parts < 1 or width % parts:
         raise KernelError(f"rows of {width} do not split into {parts} parts")
-    at = _gate_at((z, z_col), dtype, n_tokens, width, parts) if z is not None else None
-    _check_gain(weight, width, parts)
+    if z is not None:
+        _need(z, "z", dtype, 2)
+        if z.shape[0] != n_tokens or z_col < 0 or z_col + width > z.shape[1]:
+            raise KernelError(f"rows of {width} in {parts} parts with a gate from column {z_col} of {tuple(z.shape)} do not fit")
+    if weight.shape[0] not in (width, width // parts):
+        raise KernelError(f"a gain of {weight.shape[0]} entries fits neither the row ({width}) nor a part ({width // parts})")
     y = _empty(o, (n_tokens, width), dtype)
-    gate, gate_width, order = (None, 0, 2) if z is None else (at, z.shape[1], 0 if gate_first else 1)
+    gate, gate_width, order = (None, 0, 2) if z is None else (_at(z, z_col), z.shape[1], 0 if gate_first else 1)
     rc = _lib("state_scan").sb_group_norm_gate(_code(dtype), o, gate, gate_width, weight,
                                                weight.shape[0], y, n_tokens, parts, width // parts,
                                                eps, order, _stream())
