@@ -1091,7 +1091,7 @@ template <int MODE>
 __global__ void __maxnreg__(MOE_FEW_REGS)
 moe_few_kernel(const bf16* __restrict__ x, const bf16* __restrict__ w, bf16* __restrict__ y,
                const int* __restrict__ sorted, const int* __restrict__ tile_expert, const int* __restrict__ n_tiles,
-               int k_dim, int n_out, int top, float limit, const float* __restrict__ in_scale) {
+               int max_tiles, int k_dim, int n_out, int top, float limit, const float* __restrict__ in_scale) {
   constexpr bool UP = MODE != 0;
   constexpr int NW = MODE == 1 ? 2 : 1, FLY = MODE == 1 ? 3 : 6;
   extern __shared__ float few_part[];                   // [warps][NW * 4][32], with more than one warp
@@ -1103,7 +1103,11 @@ moe_few_kernel(const bf16* __restrict__ x, const bf16* __restrict__ w, bf16* __r
   SB_BEHIND_WAIT(sorted);
   SB_BEHIND_WAIT(tile_expert);
   SB_BEHIND_WAIT(n_tiles);
-  const int tile = blockIdx.y;
+  const int tile = blockIdx.z * gridDim.y + blockIdx.y;
+  if (tile >= max_tiles) {                               // (more tiles than a grid's dimension counts to)
+    if (!UP) pdl_wait();
+    return;
+  }
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, g = lane >> 2, q = lane & 3;
   // (three loads at once; a tile that is not there has garbage in its places and leaves)
   const int expert = tile_expert[tile], own = sorted[tile * MOE_FEW + g];
@@ -1371,8 +1375,9 @@ static int moe_few(const void* x, const void* w, void* y, const int* sorted, con
   int warps = 1;
   while (warps < 8 && items * warps < 148 * MOE_FEW_WARPS && k_dim >= 32 * 4 * warps) warps *= 2;
   const size_t smem = warps > 1 ? (size_t)warps * (MODE == 1 ? 8 : 4) * 32 * sizeof(float) : 0;
-  return launch_dependent(moe_few_kernel<MODE>, dim3((n_out + 15) / 16, max_tiles), dim3(32 * warps), smem, s, (const bf16*)x,
-                          (const bf16*)w, (bf16*)y, sorted, tile_expert, n_tiles, k_dim, n_out, top, limit, in_scale);
+  const int layers = (max_tiles + 65534) / 65535;
+  return launch_dependent(moe_few_kernel<MODE>, dim3((n_out + 15) / 16, (max_tiles + layers - 1) / layers, layers), dim3(32 * warps), smem, s,
+                          (const bf16*)x, (const bf16*)w, (bf16*)y, sorted, tile_expert, n_tiles, max_tiles, k_dim, n_out, top, limit, in_scale);
 }
 
 extern "C" {

@@ -183,6 +183,21 @@ def test_few_rows_an_expert(width, inner, experts, top, tokens, expert):
     assert float((got - want).norm() / want.norm()) < 2.0 ** -8
 
 
+def test_more_tiles_of_few_rows_than_a_grids_dimension_counts():
+    from starter_b200 import ops
+
+    gen = torch.Generator().manual_seed(8)
+    tokens, top, experts, size = 131100, 4, 5, 16
+    h = torch.randn(tokens, size, generator=gen).to(BF).cuda()
+    up, down = (torch.randn(experts, size, size, generator=gen).to(BF).cuda() for _ in range(2))
+    ids = torch.stack([(torch.arange(tokens) + i) % experts for i in range(top)], dim=1).int().cuda()
+    weights = torch.rand(tokens, top, generator=gen).cuda()
+    got, want = (ops.moe_experts(h, ids, weights, up, down, expert="relu2", tile_rows=rows).double() for rows in (8, 32))
+    assert float((got - want).norm() / want.norm()) < 2.0 ** -8
+    for part in (slice(0, 1000), slice(-1000, None)):
+        assert float((got[part] - want[part]).norm() / want[part].norm()) < 2.0 ** -8
+
+
 # by a cluster: its smallest steps, all its experts, the last pairs that its threads keep and the first that they walk twice
 @pytest.mark.parametrize("pairs,experts", [(512, 64), (513, 1), (513, 64), (2049, 33), (2049, 65), (16383, 16), (16384, 64), (16385, 16), (40000, 63)])
 def test_pairs_are_dealt_to_tiles_by_eight_blocks(pairs, experts):
