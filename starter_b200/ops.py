@@ -1864,6 +1864,11 @@ def latent_mixed_splits(steps: tuple, heads: int) -> int:
     return _mixed_splits(steps, heads, SM_COUNT)
 
 
+def latent_turn_rows(n_tokens: int, heads: int, n_seqs: int, max_rows: int) -> int:
+    """The rows of the gathering's grid when it turns the queries too (``sb_latent_gather``): one a sequence, and the turning blocks."""
+    return n_seqs + -(-(-(-n_tokens * heads * 8 // 256)) // -(-max_rows // 8))
+
+
 def latent_attention_prompt(q, ukv, store, block_table, ctx, heads, dim, vdim, rank, rot, scale, window=None, sink=None, turn=None, gate=None):
     """Latent attention over keys and values that are formed from the cached rows first: ``q`` ``[T, heads * (dim + rot)]``
     (the last ``rot`` entries of a head turned), ``ukv`` ``[heads * dim + heads * vdim, rank]`` (the heads' key, then value
@@ -1891,7 +1896,8 @@ def latent_attention_prompt(q, ukv, store, block_table, ctx, heads, dim, vdim, r
     turned = [None, None, None, 0, None, 0, 0, 0]
     if turn is not None:
         cos, sin, tok_pos, rot_dims, layout = turn
-        if layout == "interleaved" and rot == rot_dims == 64 and dim % 8 == 0 and cos.shape[1] % 4 == 0 and n_seqs <= 1024 and \
+        if layout == "interleaved" and rot == rot_dims == 64 and dim % 8 == 0 and cos.shape[1] % 4 == 0 and \
+                latent_turn_rows(n_tokens, heads, n_seqs, max(each)) <= 65535 and \
                 not (q.data_ptr() | cos.data_ptr() | sin.data_ptr()) % 16:
             _need(cos, "cos table", torch.float32, 2)
             _need(sin, "sin table", torch.float32, 2)

@@ -275,3 +275,17 @@ def test_the_router_takes_sixteen_tokens_a_block_behind_a_wave_of_four_a_block()
     entry = build.load("moe").sb_moe_route_many_from
     # (two blocks of four an SM with more than 16 experts: 1,184 tokens of 64 experts 16 us, in sixteens 27)
     assert [entry(n) for n in (1, 16, 17, 64)] == [592, 592, 1185, 1185]
+
+
+def test_queries_are_turned_beside_the_gathering_where_its_grid_holds_them():
+    from starter_b200.csrc import build
+    from starter_b200.ops import latent_turn_rows
+
+    assert latent_turn_rows(2048, 16, 1, 2048) == 1 + 4 and latent_turn_rows(33, 3, 2, 64) == 2 + 1
+    # (252 heads and 1,024 sequences of 64 tokens, which the path takes: a row too many for one grid)
+    assert latent_turn_rows(65536, 251, 1024, 64) <= 65535 < latent_turn_rows(65536, 252, 1024, 64)
+    entry = build.load("attention_latent_prompt").sb_latent_gather
+    result, types = build.declarations("attention_latent_prompt")["sb_latent_gather"]
+    entry.restype, entry.argtypes = result, types
+    at = 4096              # (no address is looked at: the entry refuses in front of its launch)
+    assert entry(at, at, 1, at, at, at, 1024, 64, at, at, 64, 64, 0, at, at, at, 32, at, 65536, 252, 128, None) == -2
