@@ -10,15 +10,18 @@ import torch
 BF = torch.bfloat16
 
 
-# (sequences of 301, 700 and 385 tokens and one more, blocks of 1 to 11 steps; an odd number of heads leaves a CTA of a cluster idle)
+# (blocks of 1 to 20 steps, 1 to 7 in the window: every line between them, and one behind the longest; an odd number of heads leaves a CTA of a
+# cluster idle; keys of 64 with values of 128 take a CTA a block whatever is asked for)
 @pytest.mark.gpu
 @pytest.mark.parametrize("heads", [1, 3, 4])
 @pytest.mark.parametrize("dim,vdim,window,gated", [(128, 128, None, True), (64, 64, 150, False), (128, 64, None, False), (64, 128, None, False)])
 def test_long_blocks_in_two_parts_short_ones_whole(heads, dim, vdim, window, gated, monkeypatch):
     from starter_b200 import ops
-    from test_gpu_key_parts import LENGTHS, step
+    from test_gpu_key_parts import LENGTHS, PAST, step
 
     rank = 128
+    steps = ops.latent_block_steps([p + n for p, n in zip(PAST, LENGTHS)], LENGTHS, window)
+    assert len(set(steps)) > 4
     gen, table, (rows, _), ctx = step(1, rank + 64, 16, heads)
     q = torch.randn(sum(LENGTHS), heads * (dim + 64), generator=gen).to(BF).cuda()
     ukv = (torch.randn(heads * (dim + vdim), rank, generator=gen) * rank ** -0.5).to(BF).cuda()
@@ -30,12 +33,35 @@ def test_long_blocks_in_two_parts_short_ones_whole(heads, dim, vdim, window, gat
         return ops.latent_attention_prompt(q, ukv, rows, table, ctx, heads, dim, vdim, rank, 64, (dim + 64) ** -0.5, window, sink, gate=gate)
 
     whole = run(1)
-    for split_from in (1, 2, 4, 5, 8, 11, 12):
+    for split_from in sorted(set(steps)) + [steps[0] + 1]:
         got = run(2 | split_from << 8)
+        assert torch.equal(got, whole) == (split_from > steps[0] or (dim, vdim) == (64, 128))
         # (the parts' sums join in another order: a rounding to 8 bits that falls on the other side)
         assert float((got.float() - whole.float()).abs().max()) <= 2.0 ** -7 * float(whole.float().abs().max())
-    assert torch.equal(run(2 | 1000 << 8), whole)
     assert int(ctx.status.item()) == 0
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("heads,new,past,window,split_from", [(16, [1300], [0], None, 16), (16, [1300], [700], 1500, 25), (5, [2048, 1700], [0, 0], None, 8)])
+def test_a_steps_own_plan_reaches_the_kernel(heads, new, past, window, split_from, monkeypatch):
+    import test_gpu_key_parts as parts
+    from starter_b200 import ops
+
+    monkeypatch.setattr(parts, "LENGTHS", new)
+    monkeypatch.setattr(parts, "PAST", past)
+    rank, dim = 64, 128
+    gen, table, (rows, _), ctx = parts.step(1, rank + 64, 16, heads)
+    q = torch.randn(sum(new), heads * (dim + 64), generator=gen).to(BF).cuda()
+    ukv = (torch.randn(heads * 2 * dim, rank, generator=gen) * rank ** -0.5).to(BF).cuda()
+    lib, asked = ops._lib("attention_latent_prompt"), []
+    entry = lib.sb_latent_prompt
+    monkeypatch.setattr(lib, "sb_latent_prompt", lambda *a: (asked.append(a[-4]), entry(*a))[1])
+    run = lambda: ops.latent_attention_prompt(q, ukv, rows, table, ctx, heads, dim, dim, rank, 64, 192 ** -0.5, window)
+    got = run().float()
+    monkeypatch.setattr(ops, "latent_mixed_splits", lambda *a: 1)
+    whole = run().float()
+    assert asked == [2 | split_from << 8, 1] and int(ctx.status.item()) == 0
+    assert float((got - whole).abs().max()) <= 2.0 ** -7 * float(whole.abs().max()) and not torch.equal(got, whole)
 
 
 @pytest.mark.parametrize("window", [None, 1, 64, 300])
