@@ -198,7 +198,7 @@ extern "C" {
 // x: [n_tokens, ldx] bfloat16, a row = [q (heads * dim) | k (kv_heads * dim) | v (kv_heads * vdim) | ..]; taps float [channels, K] and
 // in_bias float [channels] or null over those channels; state: float, a slot's K - 1 rows of them start at the pointer (as sb_short_conv's,
 // no activation); gains, tables and stores as sb_sink_prepare_norm's (pairs of neighbours; keys and values are filed); q: [n_tokens,
-// heads * dim].  -2: not taken (the separate kernels take anything): whole warps of queries, keys and values, up to 2,048 channels of queries
+// heads * dim].  tok_pos: a sequence's positions follow each other (the first of every chunk of tokens is read).  -2: not taken (the separate kernels take anything): whole warps of queries, keys and values, up to 2,048 channels of queries
 // and of keys and values, 1 to 4 taps, everything on 16 bytes.
 int sb_sink_conv(const void* x, int ldx, const float* taps, int K, const float* in_bias, float* state, long long slot_stride,
                  const int* seq_slot, const int* seq_q_start, const int* seq_q_len, int n_seqs, int max_q_len, const int* tok_pos,

@@ -2378,13 +2378,16 @@ def sink_conv_prepare(proj, taps, in_bias, state, state_at, seq_slot, seq_q_star
                       tok_pos, tok_slot, block_table, k_store, v_store, rotation=None, row_norm=None, unit_values=False, eps=0.0):
     """``short_conv`` over the ``[q | k | v]`` of ``proj`` (no activation, no bias behind it) and ``sink_prepare_norm`` of what it gives: keys
     and values are filed, the queries returned (the leading columns of what comes back).  One kernel (csrc/sink_conv.cu) for the
-    sizes that it takes, else those two."""
+    sizes that it takes, else those two.  A sequence's tokens stand at positions that follow each other, in its slot, as in every step of the
+    engine (the attention behind this counts them so too): the one kernel reads the position of every second or eighth token and the
+    sequences' slots."""
     channels = taps.shape[0]
     if proj.dtype == torch.bfloat16 and not unit_values and (rotation is None or rotation.layout == "interleaved") and \
             channels == heads * dim + kv_heads * (dim + vdim):
         _need(proj, "proj", torch.bfloat16, 2)
         slot_floats = _conv_operands(proj, 0, channels, taps, None, in_bias, state, state_at)
         _need(tok_pos, "tok_pos", torch.int32, 1)
+        _need(tok_slot, "tok_slot", torch.int32, 1)
         _need(block_table, "block_table", torch.int32, 2)
         rot, cos, sin, _, q_gain, k_gain = _sink_norm_operands(proj, heads, kv_heads, dim, vdim, k_store, v_store, rotation, row_norm, True)
         n_seqs = _seq_arrays(seq_slot, seq_q_start, seq_q_len)

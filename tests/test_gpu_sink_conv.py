@@ -51,3 +51,17 @@ def test_one_kernel_gives_what_two_give(heads, kv, dim, vdim, rot, width, taps, 
         assert float((got != ref).double().mean()) < 1e-3
     assert torch.equal(stores[1], other[1])
     assert state is None or torch.equal(state, kept)
+
+
+@pytest.mark.parametrize("which", ["tok_pos", "tok_slot"])
+def test_places_of_another_type_are_refused(which):
+    from starter_b200 import ops
+
+    ints = lambda v: torch.tensor(v, dtype=torch.int32, device="cuda")
+    heads, kv, dim = 2, 1, 128
+    channels, places = heads * dim + 2 * kv * dim, {"tok_pos": ints([0, 1]), "tok_slot": ints([0, 0])}
+    places[which] = places[which].long()
+    stores = [torch.zeros(1, kv, 64, dim, dtype=BF, device="cuda") for _ in range(2)]
+    with pytest.raises(ops.KernelError, match=which):
+        ops.sink_conv_prepare(torch.zeros(2, channels, dtype=BF, device="cuda"), torch.zeros(channels, 1, device="cuda"), None, None, 0, ints([0]),
+                              ints([0]), ints([2]), 2, heads, kv, dim, dim, places["tok_pos"], places["tok_slot"], ints([[0]]), *stores, eps=1e-6)
