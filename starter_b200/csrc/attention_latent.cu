@@ -733,9 +733,11 @@ latent_merge_kernel(const float* __restrict__ part_acc, const float* __restrict_
 // Single tokens of up to 16 heads: the rows of a sequence are one 16-row tile, which leaves three of the four row groups above (and six
 // of its eight warps) with nothing to do but loads.  Here a block takes a page of 64 keys at a time and all eight warps share it: a
 // warp scores eight of the keys, then, behind a barrier, sums its eighth of the latent's columns over all of them.  Pages arrive two ahead by
-// cp.async, rows behind the token and in front of the window as zeros (their weights are zero, but 0 * inf would not be).  Parts, references and sums are filed as above.  Measured (us a layer of 16 heads, captured,
-// the kernel above -> this one): rank 512, 1 sequence of 1,500 40.3 -> 36.9, 8 of up to 2,048 46.6 -> 45.2, 20 of up to 400 50.6 -> 49.1, 30 in a window
-// of 512 58.2 -> 56.9; rank 256, 4 in a window of 512 30.9 -> 29.2, 8 of up to 1,063 33.6 -> 33.4.
+// cp.async, rows behind the token and in front of the window as zeros (their weights are zero, but 0 * inf would not be).  Parts,
+// references and sums are filed as above.  Measured (us a captured layer of rank 512, the kernel above -> this one): 16 heads, 1 sequence of 2,048
+// 37.2 -> 35.0, 8 42.4 -> 42.3 (49.2 for 51.2 with the caches emptied), 32 of 1,000 59.4 -> 54.8, of 4,000 108 -> 94, in a window of 1,024
+// 62 -> 58, 100 of 2,000 174 -> 146, 148 of 1,000 110 -> 94; 8 heads 37.1 -> 33.0, 39.2 -> 37.1, 51.5 -> 47.4, 103 -> 89, 174 -> 147 (the same
+// without the window); 1 head 33.0 -> 30.9, 37.0 -> 32.9, 51.4 -> 46.7, 103 -> 88, 168 -> 140; rank 256, 32 of 4,000, 16 heads 90 -> 82, 4 78 -> 70.
 #define LS_KEYS SB_PAGE_TOKENS
 #define LS_PLD (LS_KEYS + 8)
 template <int NP>   // 16-column pairs of value tiles a warp sums

@@ -206,10 +206,7 @@ __device__ __forceinline__ float2 peer_load2(uint32_t a) {
   asm volatile("ld.shared::cluster.v2.f32 {%0, %1}, [%2];" : "=f"(v.x), "=f"(v.y) : "r"(a) : "memory");
   return v;
 }
-// The rows of this CTA's share, by its first 256 threads: 16 threads a row, eight columns each.  ml: [2 tiles][128 rows] of (reference,
-// sum); finish(t, r, reference, sum) gives the factor of the row's summed outputs; dst: output row 0 of the block, `cols` entries of a
-// head, rows `stride` apart.
-// gate: null, or rows (ld entries apart) of the output's columns, by whose sigmoid it is multiplied.
+// Eight outputs times the sigmoid of their gates.
 __device__ __forceinline__ void gate8(float* o, const bf16* gate) {
   const uint4 g = *reinterpret_cast<const uint4*>(gate);
   const uint32_t w[4] = {g.x, g.y, g.z, g.w};
@@ -220,6 +217,10 @@ __device__ __forceinline__ void gate8(float* o, const bf16* gate) {
     o[e] = __fdividef(0.25f * o[e], fmaf(0.25f, __expf(-z), 0.25f));
   }
 }
+// The rows of this CTA's share, by its first 256 threads: 16 threads a row, eight columns each.  ml: [2 tiles][128 rows] of (reference,
+// sum); finish(t, r, reference, sum) gives the factor of the row's summed outputs; dst: output row 0 of the block, `cols` entries of a
+// head, rows `stride` apart.  gate: null, or rows
+// (gate_ld entries apart) of the output's columns, by whose sigmoid it is multiplied.
 template <int PC, int COLS, int Q_BYTES, int P_BYTES, typename Finish>
 __device__ __forceinline__ void merge_parts(uint8_t* q_sm, uint8_t* p_sm, float2* ml, int rank, int splits, int rows_valid, int cols,
                                             bf16* dst, size_t stride, Finish finish, const bf16* gate = nullptr, size_t gate_ld = 0) {

@@ -1063,15 +1063,21 @@ moe_tile_big_kernel(const bf16* __restrict__ x, const bf16* __restrict__ w, bf16
 // registers in 16-byte pieces: lane 4 g + x holds the pieces x, x + 4, .. of weight rows g and g + 8 and of the tile's row g, so
 // that every product sees its k entries in one order.  The step is bound by the weights' bytes, which are read once a
 // tile, so what counts is that loads never stop: a warp keeps FLY steps of 32 entries in flight and asks for the next one as
-// soon as it has used one, and a block has as many warps (1 to 8, which share the k range; their sums meet in shared memory) as
-// bring 8 to 16 warps to every SM at once, in one round.  The weight rows of a tile run along the grid, so
-// that the warps of an SM share the tile's rows in the first cache.  A captured layer of 16 experts of 2,048 x 2,048 at 8 tokens, four each, with
-// blocks of four warps (a round and a half of them) and loads that stop between steps 84.0 us, now 77.5 (363 MB are 55); 32 experts, 11 tokens, 1,664 x
-// 1,536 90.0 -> 87.2; 8 experts, 2 tokens, three each, squared relu, 1,152 x 1,664 32.8 -> 23.6.
+// soon as it has used one, and a block has as many warps (1, 2, 4 or 8, which share the k range; their sums meet in shared memory) as
+// bring ten and more to every SM: 1,480 to 2,958 warps over the grid from 185 to 1,479 blocks, eight a block and fewer warps in all below, one a
+// block above.  (16 fit an SM.  An end at those 16, one round for all, is slower where it bites: 1,296 blocks, gated, 45.3 us a layer -> 49.4, squared
+// relu 35.3 -> 37.1; four always 43.3 -> 46.4 and 35.0 -> 37.0 at 1,152.)  The number of warps, and with it the order in which the parts of
+// a sum over k join, follows from the step's tiles: a row's last bits depend on how many other rows a step has.
+// The weight rows of a tile run along the grid, so that the warps of an SM share the tile's rows in the first cache, in which the
+// weights take no place: from memory, where a model's layers are, 16 experts of 2,048 x 2,048, 8 tokens 96 -> 88 us and of 1,024 x 1,024, 4 tokens
+// 38.9 -> 36.9; a layer called in a row whose weights stay in L2 loses by it (the latter 25.0 -> 29.7).
+// A captured layer of 16 experts of 2,048 x 2,048 at 8 tokens, four each, with blocks of four warps (a round and a half of them) and loads that
+// stop between steps 82, now 74 (363 MB are 55); with the caches emptied in front 98 -> 88, one token 57 -> 41, 16 tokens of 1,536 x 1,536 78 -> 66,
+// squared relu 70 -> 49.
 // The second product reads the tiles' experts and its first weights ahead of its wait.  It may because it stands directly behind the first
 // one (sb_moe_few launches both), which lets it start only behind its own wait, when the kernel that made the tiles has completed.
 #define MOE_FEW 8
-#define MOE_FEW_WARPS 10         // warps on every SM that a grid should bring
+#define MOE_FEW_WARPS 10         // the fewest warps an SM that a grid should bring
 #define MOE_FEW_REGS 128         // (16 warps an SM; 6 and 3 steps in flight fill them.  144 registers and 8 and 4: 77.5 -> 90.0 us, 96 and 4 and 2: 88.0)
 __device__ __forceinline__ void moe_unpack8(const uint4& v, float* f) {
   f[0] = __uint_as_float(v.x << 16); f[1] = __uint_as_float(v.x & 0xffff0000u);
@@ -1370,7 +1376,7 @@ static int moe_tiles_mode(int dtype, int tile_rows, const void* x, const void* w
 template <int MODE>
 static int moe_few(const void* x, const void* w, void* y, const int* sorted, const int* tile_expert, const int* n_tiles, int max_tiles,
                    int k_dim, int n_out, int top, float limit, const float* in_scale, cudaStream_t s) {
-  // warps a block: the fewest that bring MOE_FEW_WARPS to every SM (all are there at once), each with two steps and more
+  // warps a block: the fewest that bring MOE_FEW_WARPS to every SM, each with two steps and more
   const long long items = (long long)max_tiles * ((n_out + 15) / 16);
   int warps = 1;
   while (warps < 8 && items * warps < 148 * MOE_FEW_WARPS && k_dim >= 32 * 4 * warps) warps *= 2;

@@ -7,8 +7,11 @@
 // separate kernels would have filed, and the rows' squares of all CH tokens meet behind one barrier, with the angles and pages on their way.
 // Queries and the keys and values are blocks of their own, so that two of them share an SM and one's loads run beside the other's sums (a
 // block of all 3,072 channels: 22 us of a pass).  In two kernels 2,048 tokens of 24 heads of 128 spend 7 and 15 us, most of it issue slots
-// for indexes, partners and small loads; here 14.  A layer, two kernels -> one (us): 2,048 tokens 107.4 -> 104.6, 256 captured 39.0 -> 32.8,
-// twice 200 behind 300 captured 41.9 -> 37.3, captured single tokens of 1, 8 and 30 sequences 27.9 -> 24.3, 39.7 -> 36.2, 38.2 -> 33.4.
+// for indexes, partners and small loads; here 14.  At the 64 registers that two blocks of 512 threads leave, eight tokens a thread spill 52 to
+// 100 bytes of stores and as many to 164 of loads (three taps 80 and 144), two tokens none.
+// A layer, two kernels / two tokens a thread / eight (us): captured, single tokens of 1 sequence 27.8 / 26.8 / 29.4, of 30 43.3 / 39.2 / 41.3, 256
+// tokens 35.0 / 30.9 / 33.8, 600 55.1 / 52.0 / 52.8; 900 66.9 / 63.2 / 61.8, 1,184 85.3 / 83.6 / 80.7, 2 x 700 77.2 / 75.4 / 76.6, 1,500 93.4 / 90.8 /
+// 91.3, 2,048 104.9 / 104.0 / 101.5.
 #include "common.cuh"
 
 struct SinkConvArgs {
@@ -214,7 +217,8 @@ int sb_sink_conv(const void* x, int ldx, const float* taps, int K, const float* 
   if (ldx % 8 || ldx < channels || slot_stride % 4) return -2;
   if (((uintptr_t)x | (uintptr_t)taps | (uintptr_t)in_bias | (uintptr_t)state | (uintptr_t)q_gain | (uintptr_t)k_gain | (uintptr_t)cos_t |
        (uintptr_t)sin_t | (uintptr_t)q | (uintptr_t)k_store | (uintptr_t)v_store) % 16) return -2;
-  // eight tokens a thread once that gives every SM a block, else two (which have to reach over the taps)
+  // eight tokens a thread once that gives every SM a block, else two (which have to reach over the taps): measured above, within 4 %
+  // of each other from 600 to 1,500 tokens
   const bool many = K > 3 || (long long)n_seqs * ((max_q_len + 7) / 8) >= 148;
   const int chunk = many ? 8 : 2, chunks = (max_q_len + chunk - 1) / chunk;
   const int kv_size = kv_heads * (dim + vdim), threads = (heads * dim > kv_size ? heads * dim : kv_size) / 4;

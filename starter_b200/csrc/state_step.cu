@@ -11,6 +11,8 @@
 //   state-space, gated delta: both read-outs are taken of the state as it is found (state_scan.cu), the delta rule's warps each add all
 //     warps' S^T k behind the barrier and then write; forget-write, channel-decay: the state moves first.
 // The state-space norm spans the heads, so that mode ends with float read-outs.
+// (At the 64 registers that two blocks of 512 threads leave, channel-decay spills 52 bytes of stores and 36 of loads, state-space up to 44,
+// the others 12 at most.)
 // Measured captured, a whole layer, in separate kernels -> here (us): channel-decay, width 2,048, 16 heads, 1 sequence 27.5 -> 21.5, 32 sequences
 // 70.8 -> 41.1 (67 MB of states are 10.5 at the copy rate); gated delta, 1,536, 12 heads, 4 sequences 25.8 -> 20.6, 2,048, 16 heads, 32 71.8 -> 50.1;
 // forget-write, 1,536, 12 heads, 4 22.6 -> 16.5; state-space, heads of 128 x 64, 32 of them, 1 20.6 -> 18.6, 24, 16 33.6 -> 24.8, 32,
