@@ -219,8 +219,7 @@ __device__ __forceinline__ void gate8(float* o, const bf16* gate) {
 }
 // The rows of this CTA's share, by its first 256 threads: 16 threads a row, eight columns each.  ml: [2 tiles][128 rows] of (reference,
 // sum); finish(t, r, reference, sum) gives the factor of the row's summed outputs; dst: output row 0 of the block, `cols` entries of a
-// head, rows `stride` apart.  gate: null, or rows
-// (gate_ld entries apart) of the output's columns, by whose sigmoid it is multiplied.
+// head, rows `stride` apart.  gate: null, or rows (gate_ld entries apart) of the output's columns, by whose sigmoid it is multiplied.
 template <int PC, int COLS, int Q_BYTES, int P_BYTES, typename Finish>
 __device__ __forceinline__ void merge_parts(uint8_t* q_sm, uint8_t* p_sm, float2* ml, int rank, int splits, int rows_valid, int cols,
                                             bf16* dst, size_t stride, Finish finish, const bf16* gate = nullptr, size_t gate_ld = 0) {
