@@ -255,7 +255,7 @@ bool integers(PyObject* o, std::vector<long long>& out) {
 }
 
 // block_steps(kv lengths, new tokens, window): see latent_block_steps in ops.py.
-PyObject* block_steps(PyObject*, PyObject* const* args, Py_ssize_t n) {
+PyObject* block_steps(PyObject*, PyObject* const* args, Py_ssize_t n) try {
   std::vector<long long> kv, q, steps;
   if (n != 3 || !integers(args[0], kv) || !integers(args[1], q)) {
     if (!PyErr_Occurred()) PyErr_SetString(PyExc_TypeError, "block_steps(kv lengths, new tokens, window)");
@@ -274,10 +274,13 @@ PyObject* block_steps(PyObject*, PyObject* const* args, Py_ssize_t n) {
   PyObject* out = PyTuple_New((Py_ssize_t)steps.size());
   for (size_t i = 0; out && i < steps.size(); ++i) PyTuple_SET_ITEM(out, i, PyLong_FromLongLong(steps[i]));
   return out;
+} catch (const std::exception& e) {
+  PyErr_SetString(PyExc_RuntimeError, e.what());
+  return nullptr;
 }
 
 // mixed_splits(steps, heads, SMs): see latent_mixed_splits in ops.py.  At most sixteen of the lengths are tried: 2 us with 16 heads, 21 with one (148 blocks).
-PyObject* mixed_splits(PyObject*, PyObject* const* args, Py_ssize_t n) {
+PyObject* mixed_splits(PyObject*, PyObject* const* args, Py_ssize_t n) try {
   std::vector<long long> steps;
   if (n != 3 || !integers(args[0], steps)) {
     if (!PyErr_Occurred()) PyErr_SetString(PyExc_TypeError, "mixed_splits(steps, heads, SMs)");
@@ -285,7 +288,7 @@ PyObject* mixed_splits(PyObject*, PyObject* const* args, Py_ssize_t n) {
   }
   const long long heads = PyLong_AsLongLong(args[1]), sms = PyLong_AsLongLong(args[2]);
   if (PyErr_Occurred()) return nullptr;
-  if (steps.empty() || heads < 1 || sms < 1) return PyLong_FromLong(1);
+  if (steps.empty() || heads < 1 || sms < 1 || *std::min_element(steps.begin(), steps.end()) < 1) return PyLong_FromLong(1);
   std::sort(steps.begin(), steps.end(), std::greater<long long>());
   std::vector<std::pair<long long, long long>> runs;         // (steps, blocks of all heads)
   for (long long s : steps) {
@@ -317,6 +320,9 @@ PyObject* mixed_splits(PyObject*, PyObject* const* args, Py_ssize_t n) {
     if (!last) break;
   }
   return PyLong_FromLongLong((double)best <= 0.93 * (double)(steps[0] + 3) ? 2 | from << 8 : 1);
+} catch (const std::exception& e) {
+  PyErr_SetString(PyExc_RuntimeError, e.what());
+  return nullptr;
 }
 
 // stream(): the current CUDA stream's address.

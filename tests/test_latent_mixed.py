@@ -113,6 +113,7 @@ def test_the_plan_is_the_estimates_least():
         shared += plain(steps, heads) > 1
         assert ops.latent_mixed_splits(steps, heads) == plain(steps, heads)
     assert 50 < shared < 350
+    assert ops.latent_mixed_splits((), 4) == ops.latent_mixed_splits((5, 0), 4) == ops.latent_mixed_splits((5, -2, -7), 100) == 1
     with pytest.raises(TypeError):
         ops.latent_mixed_splits(("a",), 4)
 
